@@ -388,9 +388,11 @@ int sweep_fused(const g2d_sweep_desc *d, cudaStream_t stream, LaunchTimer *timer
     a.forced = (const F *)d->forced_z;
     a.y_pre = (F *)d->y_pre;
     a.qmin = (F)d->qmin; a.qmax = (F)d->qmax;
+    a.small_integer_bounds = d->qmin == rint(d->qmin) && d->qmax == rint(d->qmax) && fabs(d->qmin) <= 4194304.0 && fabs(d->qmax) <= 4194304.0;
     a.kind = d->quant_kind;
     a.batch = d->batch; a.m = d->m; a.n = d->n;
     a.nI = (int)ceil_div(d->m, TILE); a.nJ = (int)ceil_div(d->n, TILE);
+    a.ld = d->n; a.ldl = d->m; a.ldu = d->n; a.ldm = d->m;
     if (cudaMemsetAsync(a.c, 0, sizeof(F) * (size_t)count, stream) != cudaSuccess) return G2D_ERR_CUDA;
 
     BandArgs<F> b;

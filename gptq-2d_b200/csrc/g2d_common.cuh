@@ -57,9 +57,39 @@ __device__ __forceinline__ float affine_value_rcp(float y, float scale, float zp
     t = t > qmax ? qmax : t;
     return __fmul_rn(__fsub_rn(t, zp), scale);
 }
-__device__ __forceinline__ double affine_value_rcp(double y, double scale, double zp, double, double qmin, double qmax) {
-    return affine_value(y, scale, zp, qmin, qmax);
+// The same for bounds that are integers below 2^22 in size: then clamping and rounding commute, and a clamped value is
+// rounded half to even by adding and subtracting 1.5 * 2^23, eight cycles instead of the conversion unit's twenty-odd.
+// NaN stays NaN as with the comparisons above.
+__device__ __forceinline__ float affine_value_fast(float y, float scale, float zp, float rc, float qmin, float qmax) {
+    const float q0 = y * rc;
+    float t = __fadd_rn(fmaf(fmaf(-q0, scale, y), rc, q0), zp);
+    asm("min.NaN.f32 %0, %0, %1;" : "+f"(t) : "f"(qmax));
+    asm("max.NaN.f32 %0, %0, %1;" : "+f"(t) : "f"(qmin));
+    t = __fsub_rn(__fadd_rn(t, 12582912.f), 12582912.f);
+    return __fmul_rn(__fsub_rn(t, zp), scale);
 }
+__device__ __forceinline__ double affine_value_fast(double y, double, double, double, double, double) { return y; }  // not used: see the dispatch
+// double: `rc` is the correctly rounded reciprocal; two residual corrections make the quotient correctly rounded (the
+// first brings it within an ulp, and Markstein's theorem then gives RN(q + r rc) = RN(y / s)).  Same bits as
+// affine_value, without the division's hundred-odd cycles on the critical path of every stage.
+__device__ __forceinline__ double affine_value_rcp(double y, double scale, double zp, double rc, double qmin, double qmax) {
+    double q = y * rc;
+    q = fma(fma(-q, scale, y), rc, q);
+    q = fma(fma(-q, scale, y), rc, q);
+    double t = rint(__dadd_rn(q, zp));
+    t = t < qmin ? qmin : t;
+    t = t > qmax ? qmax : t;
+    return __dmul_rn(__dsub_rn(t, zp), scale);
+}
+// The reciprocal that affine_value_rcp takes, and the scales for which neither form leaves the range of normal numbers.
+__device__ __forceinline__ float rounding_reciprocal(float s) {
+    float v;
+    asm("rcp.approx.f32 %0, %1;" : "=f"(v) : "f"(s));
+    return fmaf(fmaf(-s, v, 1.f), v, v);  // one Newton step: the reciprocal to within half an ulp
+}
+__device__ __forceinline__ double rounding_reciprocal(double s) { return __drcp_rn(s); }
+__device__ __forceinline__ bool reciprocal_is_safe(float s) { return fabsf(s) > 1e-18f && fabsf(s) < 1e18f; }
+__device__ __forceinline__ bool reciprocal_is_safe(double s) { return fabs(s) > 1e-150 && fabs(s) < 1e150; }
 
 // float -> fp16 / bf16 -> float, round to nearest even (denormals kept).
 __device__ __forceinline__ float round_to_half(float f, int half_kind) {
@@ -113,9 +143,11 @@ struct SweepArgs {
     const F *forced;
     F *y_pre;
     F qmin, qmax;
+    int small_integer_bounds = 0;  // qmin and qmax are integers of at most 2^22 in size
     int kind;
     int64_t batch, m, n;
     int nI, nJ;  // tiles per column / per row
+    int64_t ld, ldl, ldu, ldm;  // row strides of Y, C, E and the planes; of L; of U; of the transposed planes
     // float, single matrix, tensor-core updates only (else null): tf32 hi / lo copies of the finished tiles,
     // E transposed ([n, m]) and the completed C ([m, n]), operands of the macro updates
     float *et_hi = nullptr, *et_lo = nullptr, *c_hi = nullptr, *c_lo = nullptr;

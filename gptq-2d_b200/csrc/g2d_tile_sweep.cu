@@ -9,18 +9,16 @@
 //   * the host launches one grid per tile anti-diagonal; the tiles of one anti-diagonal are
 //     independent, all feedback from earlier tiles is already in Y (right) and C (down);
 //   * inside the CTA the tile lives in shared memory; the 16 x 16 sub-tiles are taken on a sub-tile wavefront: the
-//     up to four sub-tiles of one sub-tile anti-diagonal are swept in registers by the four half-warps of warps 0 and 1.
-//     These two warps are the critical path of the whole sweep and do nothing but the rounding stages: four helper
-//     warps, one per sub-tile row, carry everything else while a sub-tile anti-diagonal is swept (the quantizer
-//     parameters of the next one, the feedback of finished sub-tiles into sub-tiles two or more anti-diagonals ahead,
-//     the feedback of the neighbour tiles) and, between two sweeps, the one product pair per sub-tile that cannot
-//     be formed earlier: the feedback of the anti-diagonal just swept into the next one;
-//   * inside a sub-tile lane k of the half-warp owns column k (the down feedback, "C") and row k (the right feedback,
-//     "Y"), both skewed so that the entries of anti-diagonal s sit in register s mod 16 of every lane: the stage loop
-//     runs in groups of ROLL stages that index registers statically, and the registers are renamed by moving them
-//     after every group; two shuffles per stage exchange the row accumulator and the completed C with the partner
-//     lane.  The feedback coefficients of a sub-tile come from zero-padded copies of the diagonal blocks of L and
-//     U^T, so the pushes need no bounds predicates: out-of-range pushes multiply by zero;
+//     up to four sub-tiles of one sub-tile anti-diagonal are swept in registers by four warps.  These are the critical
+//     path of the whole sweep and do little but the rounding stages: four helper warps carry the rest while a sub-tile
+//     anti-diagonal is swept (the quantizer parameters of the next one, the feedback of finished sub-tiles into sub-tiles
+//     two or more anti-diagonals ahead, the feedback for the neighbour tiles); between two sweeps both form the one
+//     product pair per sub-tile that cannot be formed earlier, from the anti-diagonal just swept into the next one;
+//   * inside a sub-tile half of a warp's lanes own the columns (the down feedback, "C"), the other half the rows (the right
+//     feedback, "Y"), skewed so that the entries of an anti-diagonal sit in register 0 of every lane when their stage
+//     comes: a push moves the accumulators down by one register.  One shuffle per stage exchanges the two sums of an
+//     entry.  The feedback coefficients of a sub-tile come from zero-padded copies of the diagonal blocks of L and U^T,
+//     so the pushes need no bounds predicates: out-of-range pushes multiply by zero;
 //   * pipelined schedule: a tile also adds the far-feedback planes as it loads, and the feedback between neighbour
 //     tiles of consecutive tile anti-diagonals travels as a push: the helper warps of tile (I, J) form, from the
 //     errors and the completed C in shared memory,  L[I + 1, I] E[I, J]  and  C[I, J] U[J, J + 1]  while the tile is
@@ -36,13 +34,13 @@ namespace g2d {
 // the value of source p to the receiver dd places further (L[p + dd][p] or U[p][p + dd]), zero for dd = 0 and past the
 // block's end.  A lane fetches its row with four 16-byte loads; a row stride of 20 keeps eight lanes on distinct banks.
 constexpr int DLD = SUB + 4;            // row stride
-constexpr int DBLK = SUB * DLD;         // elements per block
 constexpr int ROLL = 4;                 // rounding stages per iteration of the stage loop
-constexpr int SWEEPERS = NSUB / 2;      // warps that sweep: one half-warp per sub-tile row
+constexpr int DROWS = (2 * NSUB + 1) * SUB + SUB + 1;  // rows of all eight blocks with 16 zero rows before and 17 behind them
+constexpr int SWEEPERS = NSUB;          // warps that sweep: one per sub-tile row
 constexpr int HELPERS = NSUB;           // warps that feed them: one per sub-tile row
 constexpr int TTH = (SWEEPERS + HELPERS) * 32;  // threads per CTA
-constexpr int LANES = SWEEPERS * 32;    // sweeping lanes
-constexpr int ZLD = SUB;                // row stride of the staging blocks of the rounded values (the walk down an anti-diagonal moves 15 words: no conflicts)
+constexpr int PLD = SUB + 2;            // entries per row of a sub-tile's quantizer parameters (the walk along an anti-diagonal moves 17 entries: no conflicts)
+constexpr int PPAD = (SUB + 1) * PLD;   // entries behind the parameters that lanes past their last entry may read (and ignore)
 
 template <typename F>
 __device__ __forceinline__ void load4(const F *p, F (&v)[4]);
@@ -68,302 +66,281 @@ __device__ __forceinline__ void store4<double>(double *p, const double (&v)[4]) 
     *reinterpret_cast<double2 *>(p + 2) = make_double2(v[2], v[3]);
 }
 
-template <typename F>
+// Sixteen bytes from global to shared memory without passing through registers; zeros when `in` is false.
+__device__ __forceinline__ void async16(void *dst, const void *src, bool in) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src), "r"(in ? 16 : 0) : "memory");
+}
+__device__ __forceinline__ uint32_t shared_address(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
+// Loads of the stage loop: volatile, so that they stay where they are written (one stage ahead of their use, behind the shuffle).
+__device__ __forceinline__ void load4_here(uint32_t at, float (&v)[4]) {
+    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]) : "r"(at));
+}
+__device__ __forceinline__ void load4_here(uint32_t at, double (&v)[4]) {
+    asm volatile("ld.shared.v2.f64 {%0, %1}, [%2];" : "=d"(v[0]), "=d"(v[1]) : "r"(at));
+    asm volatile("ld.shared.v2.f64 {%0, %1}, [%2];" : "=d"(v[2]), "=d"(v[3]) : "r"(at + 16));
+}
+// A predicated store instead of a branch around a store
+__device__ __forceinline__ void store_shared_if(uint32_t at, float v, bool on) {
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %2, 0;\n\t@p st.shared.f32 [%0], %1;\n\t}" ::"r"(at), "f"(v), "r"((uint32_t)on));
+}
+__device__ __forceinline__ void store_shared_if(uint32_t at, double v, bool on) {
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %2, 0;\n\t@p st.shared.f64 [%0], %1;\n\t}" ::"r"(at), "d"(v), "r"((uint32_t)on));
+}
+
+// D += A B with 16 inner terms, all in shared memory with row stride LD; one warp.  The row and column counts of D are 16 x 16,
+// 16 x 64 (WIDE) or 64 x 16 (TALL): the strips give a lane 4 x 8 or 8 x 4 outputs and need half the operand loads per
+// multiply-add of the small block (2 x 4 outputs per lane), and shared-memory loads are what these products are short of.
+enum Shape { SMALL, WIDE, TALL };
+template <int SHAPE, typename F>
 __device__ __forceinline__ void mm16(F *__restrict__ D, const F *__restrict__ A, const F *__restrict__ B, int lane) {
-    // D[16x16] += A[16x16] * B[16x16], all in shared memory with row stride LD; one warp, 2 x 4 outputs per lane
-    const int r = (lane >> 2) * 2, c = (lane & 3) * 4;
-    F d0[4], d1[4];
-    load4(D + r * LD + c, d0);
-    load4(D + (r + 1) * LD + c, d1);
+    constexpr int NR = SHAPE == SMALL ? 2 : SHAPE == WIDE ? 4 : 8, NC = SHAPE == WIDE ? 2 : 1;  // rows and groups of four columns per lane
+    const int r = SHAPE == WIDE ? (lane >> 3) * 4 : SHAPE == TALL ? lane >> 2 : (lane >> 2) * 2, rs = SHAPE == TALL ? 8 : 1;
+    const int c = SHAPE == WIDE ? (lane & 7) * 4 : (lane & 3) * 4;
+    constexpr int CS = 32;  // distance of a lane's column groups
+    F d[NR][NC][4];
 #pragma unroll
-    for (int k = 0; k < SUB; k += 4) {
-        F a0[4], a1[4];
-        load4(A + r * LD + k, a0);
-        load4(A + (r + 1) * LD + k, a1);
+    for (int i = 0; i < NR; ++i)
 #pragma unroll
-        for (int kk = 0; kk < 4; ++kk) {
-            F b[4];
-            load4(B + (k + kk) * LD + c, b);
-#pragma unroll
-            for (int y = 0; y < 4; ++y) {
-                d0[y] += a0[kk] * b[y];
-                d1[y] += a1[kk] * b[y];
-            }
-        }
-    }
-    store4(D + r * LD + c, d0);
-    store4(D + (r + 1) * LD + c, d1);
-}
-
-// The one or two products that carry finished sub-tiles into sub-tile (ap, bp): the errors of (as, bp) down through
-// L[ap, as] into C, then the completed C of (ap, bs) right through U[bs, bp] into Y; a source index outside 0 .. NSUB - 1
-// means there is no such source.  One warp; a loop, so that the product's code exists once per call site.
-template <typename F>
-__device__ __forceinline__ void carry_into(F *Ys, F *Cs, const F *LUs, int ap, int bp, int as, int bs, int lane) {
+        for (int g = 0; g < NC; ++g) load4(D + (r + i * rs) * LD + c + g * CS, d[i][g]);
+    constexpr int KU = SHAPE == SMALL ? SUB : 4;  // inner terms per trip: the small product entirely unrolled, the strips in four trips
 #pragma unroll 1
-    for (int prod = 0; prod < 2; ++prod) {
-        const int src = prod == 0 ? as : bs;
-        if (src < 0 || src >= NSUB) continue;
-        F *D = (prod == 0 ? Cs : Ys) + ap * SUB * LD + bp * SUB;
-        const F *A = prod == 0 ? LUs + ap * SUB * LD + src * SUB : Cs + ap * SUB * LD + src * SUB;
-        const F *B = prod == 0 ? Ys + src * SUB * LD + bp * SUB : LUs + src * SUB * LD + bp * SUB;
-        mm16(D, A, B, lane);
-    }
-}
-
-// The products of the neighbour push: the 2 x 4 outputs of a lane stay in registers.  d += A B with A and B in shared
-// memory (row stride LD), and the same with the lane's two rows of A held in registers.
-template <typename F>
-__device__ __forceinline__ void mm16_acc(F (&d0)[4], F (&d1)[4], const F *__restrict__ A, const F *__restrict__ B, int lane) {
-    const int r = (lane >> 2) * 2, c = (lane & 3) * 4;
+    for (int k0 = 0; k0 < SUB; k0 += KU) {
+        F a[NR][KU], b[KU][NC][4];
 #pragma unroll
-    for (int k = 0; k < SUB; k += 4) {
-        F a0[4], a1[4];
-        load4(A + r * LD + k, a0);
-        load4(A + (r + 1) * LD + k, a1);
+        for (int k = 0; k < KU; k += 4) {
 #pragma unroll
-        for (int kk = 0; kk < 4; ++kk) {
-            F b[4];
-            load4(B + (k + kk) * LD + c, b);
+            for (int i = 0; i < NR; ++i) {
+                F t[4];
+                load4(A + (r + i * rs) * LD + k0 + k, t);
 #pragma unroll
-            for (int y = 0; y < 4; ++y) {
-                d0[y] += a0[kk] * b[y];
-                d1[y] += a1[kk] * b[y];
+                for (int x = 0; x < 4; ++x) a[i][k + x] = t[x];
             }
         }
-    }
-}
-template <typename F>
-__device__ __forceinline__ void mm16_areg(F (&d0)[4], F (&d1)[4], const F *a0, const F *a1, const F *__restrict__ B, int lane) {
-    // a0 / a1: this lane's quarter of its two rows of A (columns 4 (lane % 4) .. + 3); the four lanes that share the
-    // rows hand each other their quarters by shuffle
-    const int c = (lane & 3) * 4;
 #pragma unroll
-    for (int k = 0; k < SUB; ++k) {
-        F b[4];
-        load4(B + k * LD + c, b);
-        const F v0 = __shfl_sync(0xffffffffu, a0[k & 3], k >> 2, 4), v1 = __shfl_sync(0xffffffffu, a1[k & 3], k >> 2, 4);
+        for (int k = 0; k < KU; ++k)
 #pragma unroll
-        for (int y = 0; y < 4; ++y) {
-            d0[y] += v0 * b[y];
-            d1[y] += v1 * b[y];
-        }
-    }
-}
-// Stores a lane's 2 x 4 outputs of a 16 x 16 block at `dst` (row stride ld); rows / columns from rows_left / cols_left on lie
-// outside the matrix.  `vec`: rows are 16-byte aligned and columns come in whole groups of four.
-template <typename F>
-__device__ __forceinline__ void store_block(F *dst, int64_t ld, const F (&d0)[4], const F (&d1)[4], int lane, int64_t rows_left, int64_t cols_left, bool vec) {
-    const int r = (lane >> 2) * 2, c = (lane & 3) * 4;
-    if (vec) {
-        if (c < cols_left) {
-            if (r < rows_left) store4(dst + r * ld + c, d0);
-            if (r + 1 < rows_left) store4(dst + (r + 1) * ld + c, d1);
-        }
-    } else {
+            for (int g = 0; g < NC; ++g) load4(B + (k0 + k) * LD + c + g * CS, b[k][g]);
 #pragma unroll
-        for (int y = 0; y < 4; ++y) {
-            if (c + y < cols_left) {
-                if (r < rows_left) dst[r * ld + c + y] = d0[y];
-                if (r + 1 < rows_left) dst[(r + 1) * ld + c + y] = d1[y];
-            }
-        }
+        for (int k = 0; k < KU; ++k)
+#pragma unroll
+            for (int i = 0; i < NR; ++i)
+#pragma unroll
+                for (int g = 0; g < NC; ++g)
+#pragma unroll
+                    for (int y = 0; y < 4; ++y) d[i][g][y] += a[i][k] * b[k][g][y];
     }
+#pragma unroll
+    for (int i = 0; i < NR; ++i)
+#pragma unroll
+        for (int g = 0; g < NC; ++g) store4(D + (r + i * rs) * LD + c + g * CS, d[i][g]);
 }
 
 template <typename F, int KIND>
-__global__ void __launch_bounds__(TTH) tile_sweep_kernel(SweepArgs<F> P, int S, int i_first, int i_step) {
+__global__ void __launch_bounds__(TTH, 1) tile_sweep_kernel(SweepArgs<F> P, int S, int i_first, int i_step) {
     extern __shared__ __align__(16) unsigned char g2d_smem[];
     F *Ys = reinterpret_cast<F *>(g2d_smem);  // X + right feedback; the errors E once a sub-tile is swept
     F *Cs = Ys + TILE * LD;                   // down feedback; the completed C once a sub-tile is swept
     F *LUs = Cs + TILE * LD;                  // strict lower part: L[I, I]; strict upper part: U[J, J]
-    F *Dg = LUs + TILE * LD;                  // [2][NSUB] zero-padded diagonal blocks: L[a, a] and U[b, b]^T, strictly lower
-    F *Ubs = Dg + 2 * NSUB * DBLK;            // pipelined schedule: U[J, J + 1], the right neighbour's coupling block
-    F *Ps = Ubs + TILE * LD;                   // [3][SUB][LANES]: quantizer parameters of the sweeping lanes, by register number
-    F *Zst = Ps + 3 * SUB * LANES;            // [NSUB][SUB][ZLD]: rounded values of the sub-tiles being swept, written out by the helpers after the sweep
-    unsigned *Pv = reinterpret_cast<unsigned *>(Zst + NSUB * SUB * ZLD);  // [2][LANES] registers holding entries inside the matrix, one word per half of the registers; [2][SWEEPERS] reciprocal division allowed
+    F *Dg = LUs + TILE * LD;                  // zero-padded diagonal blocks L[a, a] and U[b, b]^T, strictly lower, between rows of zeros
+    F *Par = Dg + DROWS * DLD;                // [NSUB][SUB][PLD][4]: scale, zero point, reciprocal, rounded value of the entries of the sub-tiles being swept
+    F *Ubs = Par + NSUB * SUB * PLD * 4;      // float only, pipelined schedule: U[J, J + 1], the right neighbour's coupling block
+    F *Lbs = Ubs + TILE * LD;                 // the same: L[I + 1, I], the lower neighbour's
+    F *Yns = Lbs + TILE * LD;                 // the same: the feedback for the right neighbour, C[I, J] U[J, J + 1], growing sub-tile by sub-tile
+    F *Cns = Yns + TILE * LD;                 // and for the lower one, L[I + 1, I] E[I, J]
+    __shared__ unsigned fast_div[NSUB];       // every scale of the sub-tile allows the division by reciprocal
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int k = lane & 15, half = lane >> 4;
+    const int k = lane & 15, role = lane >> 4;
     const int I = i_first + i_step * (int)blockIdx.x, J = S - I;  // tiles of the anti-diagonal S, every one or every second
     const int64_t i0 = (int64_t)I * TILE, j0 = (int64_t)J * TILE;
     const int64_t m = P.m, n = P.n;
     const bool full = i0 + TILE <= m && j0 + TILE <= n;
-    const bool sweeper = warp < SWEEPERS;
-    const int helper = warp - SWEEPERS;  // 0 .. HELPERS - 1 for the helper warps: the sub-tile row the warp feeds
+    // Warps w and w + 4 share one of the SM's four schedulers.  The sweeping warps take two of them (rows 0 and 2, rows 1 and 3)
+    // and the helpers the other two: a helper's product beside it costs a sweeping warp more than its neighbour does.
+    static_assert(SWEEPERS == 4 && HELPERS == 4, "warps are dealt out to the schedulers in twos");
+    const bool sweeper = (warp & 2) == 0;
+    const int number = (warp & 1) + (warp >> 2) * 2;  // of the warp among those of its kind
+    const int helper = number;                        // the sub-tile row whose parameters a helper prepares
+    const int rows_in = (int)(m - i0 < TILE ? m - i0 : TILE), cols_in = (int)(n - j0 < TILE ? n - j0 : TILE);  // of this tile
 
     for (int64_t batch = blockIdx.y; batch < P.batch; batch += gridDim.y) {
-        F *yg = P.y + batch * m * n, *cg = P.c + batch * m * n, *eg = P.e + batch * m * n;
+        // Y, C, E and the planes have rows of ld values (n, or n rounded up to a multiple of 4), L and U rows of ldl and ldu
+        const int64_t ld = P.ld, ldl = P.ldl, ldu = P.ldu;
+        F *yg = P.y + batch * m * ld, *cg = P.c + batch * m * ld, *eg = P.e + batch * m * ld;
         const F *lg = P.l + (P.l_off ? P.l_off[batch] : 0);
         const F *ug = P.u + (P.u_off ? P.u_off[batch] : 0);
         const F *sg = KIND == G2D_Q_AFFINE ? P.scale + (P.scale_off ? P.scale_off[batch] : 0) : nullptr;
         const F *zg = KIND == G2D_Q_AFFINE ? P.zero + (P.zero_off ? P.zero_off[batch] : 0) : nullptr;
         const F *fg = KIND == G2D_Q_FORCED ? P.forced + batch * m * n : nullptr;
         F *pre = P.y_pre ? P.y_pre + batch * m * n : nullptr;
-        const F *yfg = P.yf ? P.yf + batch * m * n : nullptr, *cfg = P.yf ? P.cf + batch * m * n : nullptr;
+        const F *yfg = P.yf, *cfg = P.cf;
         // neighbour push (pipelined schedule): what this tile receives and what it owes
-        F *yng = P.yn ? P.yn + batch * m * n : nullptr, *cng = P.yn ? P.cn + batch * m * n : nullptr;
+        F *yng = P.yn, *cng = P.cn;  // these planes exist for a single matrix only
         const bool gets_right = yng != nullptr && J > 0, gets_down = yng != nullptr && I > 0;
         const bool owes_right = yng != nullptr && J + 1 < P.nJ, owes_down = yng != nullptr && I + 1 < P.nI;
 
         // ---- quantizer parameters, prepared by the helper warps ----
-        // Helper warp h prepares, for the sweeping lane of its own lane number in sweeping warp h mod SWEEPERS, half
-        // h / SWEEPERS of that lane's registers: register r holds entry ((r - k) mod 16, k) of the lane's sub-tile.
-        // Scale, zero point and, for the float affine quantizer, the refined reciprocal of the scale (see
-        // affine_value_rcp) wait in shared memory by register number, with the bits that say which registers hold
-        // entries inside the matrix and the warp-wide decision whether every scale is in the range where the reciprocal
-        // form of the division is safe.  The loads are issued one sub-tile anti-diagonal ahead and travel while the
-        // helper does its other work.
-        constexpr int PR = SUB / (HELPERS / SWEEPERS);  // registers per helper lane
+        // Helper warp h prepares the parameters of the sub-tile that sweeping warp h takes next: a lane has the entries
+        // (2 x + lane / 16, lane % 16).  Scale, zero point and, for the affine quantizer, the reciprocal of the scale wait
+        // in shared memory by entry, with the warp-wide decision whether every scale is in the range where the reciprocal
+        // form of the division is safe.  The loads are issued one sub-tile anti-diagonal ahead and travel while the helper
+        // does its other work.
+        constexpr int PR = SUB * SUB / 32;  // entries per helper lane
         F sc[PR], zp[PR], rc[PR];
         bool pfast = true;
-        unsigned pvalid = 0;
-        const int p_warp = helper & (SWEEPERS - 1), p_part = helper / SWEEPERS;  // helpers only
-        const int p_lane = p_warp * 32 + lane;
-        const int p_a = 2 * p_warp + half;  // sub-tile row of the lane prepared for
+        unsigned pvalid = 0;  // entries inside the matrix
         auto fetch_params = [&](int w_next) {
-            const int b_raw = w_next - p_a;
-            const int b = b_raw >= 0 && b_raw < NSUB ? b_raw : 0;  // a half-warp without a sub-tile gets valid dummies and stays masked
-            const int r0 = p_a * SUB, c0 = b * SUB;
-            unsigned bits = 0;
+            const int b = w_next - helper;
+            if (b < 0 || b >= NSUB || KIND == G2D_Q_ROUND) return;
+            const int r = helper * SUB + role, c = b * SUB + k;  // first entry; the others follow two rows apart
+            // entries outside the matrix load a value from inside it (no select waits on the load here) and get their
+            // neutral parameters in finish_params
+            const int rc_ = min(r, rows_in - 1), cc = min(c, cols_in - 1);
+            pvalid = 0;
 #pragma unroll
-            for (int x = 0; x < PR; ++x) {
-                const int r = p_part * PR + x, o = (r - k) & (SUB - 1);
-                const int64_t gi = i0 + r0 + o, gj = j0 + c0 + k;
-                const bool in = full || (gi < m && gj < n);
-                bits |= in ? (1u << r) : 0u;
-                // entries outside the matrix load a value from inside it (no select waits on the load here) and get
-                // their neutral parameters in finish_params
-                const int64_t ci = gi < m ? gi : m - 1, cj = gj < n ? gj : n - 1;
-                if (KIND == G2D_Q_AFFINE) {
-                    sc[x] = sg[ci * P.srs + cj * P.scs];
-                    zp[x] = zg[ci * P.zrs + cj * P.zcs];
-                } else if (KIND == G2D_Q_FORCED) {
-                    sc[x] = fg[ci * n + cj];
+            for (int x = 0; x < PR; ++x) pvalid |= (r + 2 * x < rows_in && c < cols_in) ? (1u << x) : 0u;
+            if (KIND == G2D_Q_AFFINE) {
+                const F *ps = sg + (i0 + rc_) * P.srs + (j0 + cc) * P.scs, *pz = zg + (i0 + rc_) * P.zrs + (j0 + cc) * P.zcs;
+                const int64_t ss = 2 * P.srs, zs = 2 * P.zrs;
+#pragma unroll
+                for (int x = 0; x < PR; ++x) {
+                    sc[x] = *ps;
+                    zp[x] = *pz;
+                    if (r + 2 * x + 2 < rows_in) {
+                        ps += ss;
+                        pz += zs;
+                    }
+                }
+            } else {
+                const F *pf = fg + (i0 + rc_) * n + j0 + cc;
+#pragma unroll
+                for (int x = 0; x < PR; ++x) {
+                    sc[x] = *pf;
+                    if (r + 2 * x + 2 < rows_in) pf += 2 * n;
                 }
             }
-            pvalid = bits;
         };
-        auto finish_params = [&]() {
+        auto finish_params = [&](int w_next) {
+            if (w_next - helper < 0 || w_next - helper >= NSUB) return;
+            bool normal = true;
 #pragma unroll
             for (int x = 0; x < PR; ++x) {
-                const bool in = (pvalid >> (p_part * PR + x)) & 1u;
+                const bool in = (pvalid >> x) & 1u;
                 if (KIND == G2D_Q_AFFINE) {
                     sc[x] = in ? sc[x] : (F)1;
                     zp[x] = in ? zp[x] : (F)0;
+                    normal = normal && reciprocal_is_safe(sc[x]);
+                    rc[x] = rounding_reciprocal(sc[x]);
                 } else if (KIND == G2D_Q_FORCED) {
                     sc[x] = in ? sc[x] : (F)0;
                 }
             }
-            if (KIND == G2D_Q_AFFINE && sizeof(F) == sizeof(float)) {
-                bool normal = true;
-#pragma unroll
-                for (int x = 0; x < PR; ++x) {
-                    const float sv = (float)sc[x], av = fabsf(sv);
-                    normal = normal && av > 1e-18f && av < 1e18f;
-                    float v = __frcp_rn(sv);
-                    v = fmaf(fmaf(-sv, v, 1.f), v, v);  // one Newton step: the reciprocal to within half an ulp
-                    rc[x] = (F)v;
-                }
-                pfast = __all_sync(0xffffffffu, normal);
-            }
+            pfast = __all_sync(0xffffffffu, normal);
         };
-        auto store_params = [&]() {
+        auto store_params = [&](int w_next) {
+            if (w_next - helper < 0 || w_next - helper >= NSUB) return;
+            F *dst = Par + ((helper * SUB + role) * PLD + k) * 4;
 #pragma unroll
             for (int x = 0; x < PR; ++x) {
-                const int r = p_part * PR + x;
-                if (KIND != G2D_Q_ROUND) Ps[(0 * SUB + r) * LANES + p_lane] = sc[x];
                 if (KIND == G2D_Q_AFFINE) {
-                    Ps[(1 * SUB + r) * LANES + p_lane] = zp[x];
-                    Ps[(2 * SUB + r) * LANES + p_lane] = rc[x];
+                    const F v[4] = {sc[x], zp[x], rc[x], (F)0};
+                    store4(dst + 2 * x * PLD * 4, v);
+                } else if (KIND == G2D_Q_FORCED) {
+                    dst[2 * x * PLD * 4] = sc[x];
                 }
             }
-            Pv[p_part * LANES + p_lane] = pvalid;
-            if (lane == 0) Pv[2 * LANES + p_part * SWEEPERS + p_warp] = pfast ? 1u : 0u;
+            if (lane == 0) fast_div[helper] = pfast ? 1u : 0u;
         };
         if (!sweeper) fetch_params(0);
 
         constexpr bool PUSH = sizeof(F) == sizeof(float);  // the neighbour push exists for float (pipelined schedule) only
 
-        // ---- load the tile; all global loads of a pass are issued before its shared-memory stores ----
-        const bool vec = full && (n % 4 == 0) && (m % 4 == 0) &&
+        // ---- load the tile ----
+        const bool vec = full && ((ld | ldl | ldu) % 4 == 0) &&
                          ((reinterpret_cast<uintptr_t>(yg) | reinterpret_cast<uintptr_t>(cg) | reinterpret_cast<uintptr_t>(eg) |
                            reinterpret_cast<uintptr_t>(lg) | reinterpret_cast<uintptr_t>(ug)) % (4 * sizeof(F)) == 0);
-        if (vec) {
-            constexpr int VECS = TILE * TILE / 4;              // vectors per array
-            constexpr int PER = (VECS + TTH - 1) / TTH;        // per thread, the last one partly
-#pragma unroll
-            for (int pass = 0; pass < 2; ++pass) {
-                F va[PER][4], vb[PER][4];
+        bool have_diagonal = false;
+        if constexpr (PUSH) {
+            if (owes_right || owes_down)
+                for (int idx = tid; idx < 2 * TILE * LD / 4; idx += TTH) {
+                    const F zero[4] = {(F)0, (F)0, (F)0, (F)0};
+                    store4(Yns + idx * 4, zero);
+                }
+            if (vec) {
+                // One wait on global memory: the off-diagonal blocks of L[I, I] and U[J, J] and the two coupling blocks
+                // travel to shared memory on their own (cp.async), the diagonal blocks and the six planes that make up Y and
+                // C through registers, and all of them are issued before the first is used.
+                have_diagonal = true;
+                for (int c = tid; c < 12 * SUB * 4; c += TTH) {
+                    const int blk = c / (SUB * 4), ba = blk / 3, bb = blk % 3 + (blk % 3 >= ba ? 1 : 0), row = ba * SUB + c / 4 % SUB, col = bb * SUB + c % 4 * 4;
+                    async16(LUs + row * LD + col, ba > bb ? lg + (i0 + row) * ldl + i0 + col : ug + (j0 + row) * ldu + j0 + col, true);
+                }
+                if (owes_right)
+                    for (int c = tid; c < TILE * TILE / 4; c += TTH) {
+                        const int row = c / (TILE / 4), col = c % (TILE / 4) * 4;
+                        const bool in = j0 + TILE + col < n;  // n is not always a multiple of 4, the row stride is: the tail is zero there
+                        async16(Ubs + row * LD + col, ug + (j0 + row) * ldu + (in ? j0 + TILE + col : 0), in);
+                    }
+                if (owes_down)
+                    for (int c = tid; c < TILE * TILE / 4; c += TTH) {
+                        const int row = c / (TILE / 4), col = c % (TILE / 4) * 4;
+                        const bool in = i0 + TILE + row < m;
+                        async16(Lbs + row * LD + col, lg + (in ? i0 + TILE + row : 0) * ldl + i0 + col, in);
+                    }
+                asm volatile("cp.async.commit_group;" ::: "memory");
+                constexpr int PER = TILE * TILE / 4 / TTH;  // vectors per thread and array
+                F vy[PER][4], vc[PER][4], fy[PER][4], fc[PER][4], ny[PER][4], nc[PER][4], dv[2][4];
 #pragma unroll
                 for (int t = 0; t < PER; ++t) {
                     const int idx = t * TTH + tid, r = idx / (TILE / 4), c = (idx % (TILE / 4)) * 4;
-                    if (idx >= VECS) continue;
-                    if (pass == 0) {
-                        load4(yg + (i0 + r) * n + j0 + c, va[t]);
-                        load4(cg + (i0 + r) * n + j0 + c, vb[t]);
-                    } else {
-                        load4(lg + (i0 + r) * m + i0 + c, va[t]);
-                        load4(ug + (j0 + r) * n + j0 + c, vb[t]);
+                    const int64_t at = (i0 + r) * ld + j0 + c;
+                    load4(yg + at, vy[t]);
+                    load4(cg + at, vc[t]);
+#pragma unroll
+                    for (int x = 0; x < 4; ++x) fy[t][x] = fc[t][x] = ny[t][x] = nc[t][x] = (F)0;
+                    if (yfg != nullptr) {
+                        load4(yfg + at, fy[t]);
+                        load4(cfg + at, fc[t]);
                     }
+                    if (gets_right) load4(yng + at, ny[t]);
+                    if (gets_down) load4(cng + at, nc[t]);
                 }
-                if (pass == 0 && yfg != nullptr) {
-                    // the far planes and what the left and the upper neighbour pushed one launch ago: all loads are
-                    // issued before the first addition, so that the tile waits for global memory once
-                    F fa[PER][4], fb[PER][4], na[PER][4], nb[PER][4];
 #pragma unroll
-                    for (int t = 0; t < PER; ++t) {
-                        const int idx = t * TTH + tid, r = idx / (TILE / 4), c = (idx % (TILE / 4)) * 4;
-                        if (idx >= VECS) continue;
-                        load4(yfg + (i0 + r) * n + j0 + c, fa[t]);
-                        load4(cfg + (i0 + r) * n + j0 + c, fb[t]);
-                        if constexpr (PUSH) {
-#pragma unroll
-                            for (int x = 0; x < 4; ++x) na[t][x] = nb[t][x] = (F)0;
-                            if (gets_right) load4(yng + (i0 + r) * n + j0 + c, na[t]);
-                            if (gets_down) load4(cng + (i0 + r) * n + j0 + c, nb[t]);
-                        }
-                    }
-#pragma unroll
-                    for (int t = 0; t < PER; ++t) {
-                        if (t * TTH + tid >= VECS) continue;
-#pragma unroll
-                        for (int x = 0; x < 4; ++x) {
-                            va[t][x] += fa[t][x];
-                            vb[t][x] += fb[t][x];
-                            if constexpr (PUSH) {
-                                va[t][x] += na[t][x];
-                                vb[t][x] += nb[t][x];
-                            }
-                        }
-                    }
+                for (int t = 0; t < 2; ++t) {  // the eight diagonal blocks, 64 vectors each
+                    const int idx = t * TTH + tid, blk = idx / 64, r = idx / 4 % SUB, c = idx % 4 * 4, o = (blk % NSUB) * SUB;
+                    load4(blk < NSUB ? lg + (i0 + o + r) * ldl + i0 + o + c : ug + (j0 + o + r) * ldu + j0 + o + c, dv[t]);
                 }
-                if (pass == 1 && owes_right) {
-#pragma unroll
-                    for (int t = 0; t < PER; ++t) {
-                        const int idx = t * TTH + tid, r = idx / (TILE / 4), c = (idx % (TILE / 4)) * 4;
-                        if (idx >= VECS) continue;
-                        F uv[4] = {(F)0, (F)0, (F)0, (F)0};
-                        if (j0 + TILE + c < n) load4(ug + (j0 + r) * n + j0 + TILE + c, uv);
-                        store4(Ubs + r * LD + c, uv);
-                    }
+                for (int idx = tid; idx < DROWS * DLD / 4; idx += TTH) {
+                    const F zero[4] = {(F)0, (F)0, (F)0, (F)0};
+                    store4(Dg + idx * 4, zero);
                 }
+                __syncthreads();
 #pragma unroll
                 for (int t = 0; t < PER; ++t) {
                     const int idx = t * TTH + tid, r = idx / (TILE / 4), c = (idx % (TILE / 4)) * 4;
-                    if (idx >= VECS) continue;
-                    if (pass == 0) {
-                        store4(Ys + r * LD + c, va[t]);
-                        store4(Cs + r * LD + c, vb[t]);
-                    } else {
-                        F lu[4];
 #pragma unroll
-                        for (int x = 0; x < 4; ++x) lu[x] = r > c + x ? va[t][x] : (r < c + x ? vb[t][x] : (F)0);
-                        store4(LUs + r * LD + c, lu);
+                    for (int x = 0; x < 4; ++x) {
+                        vy[t][x] += fy[t][x];
+                        vc[t][x] += fc[t][x];
+                        vy[t][x] += ny[t][x];
+                        vc[t][x] += nc[t][x];
+                    }
+                    store4(Ys + r * LD + c, vy[t]);
+                    store4(Cs + r * LD + c, vc[t]);
+                }
+#pragma unroll
+                for (int t = 0; t < 2; ++t) {
+                    const int idx = t * TTH + tid, blk = idx / 64, r = idx / 4 % SUB, c = idx % 4 * 4;
+#pragma unroll
+                    for (int x = 0; x < 4; ++x) {
+                        const int p = blk < NSUB ? c + x : r, q = blk < NSUB ? r : c + x;  // source and receiver
+                        if (q > p) Dg[(SUB + blk * SUB + p) * DLD + q - p] = dv[t][x];
                     }
                 }
+                asm volatile("cp.async.wait_all;" ::: "memory");
             }
-        } else {
+        }
+        if (!have_diagonal) {
             constexpr int UN = 8;
             for (int base = 0; base < TILE * TILE; base += TTH * UN) {
                 F vy[UN], vc[UN], vl[UN];
@@ -371,279 +348,267 @@ __global__ void __launch_bounds__(TTH) tile_sweep_kernel(SweepArgs<F> P, int S, 
                 for (int t = 0; t < UN; ++t) {
                     const int idx = base + t * TTH + tid, r = idx / TILE, c = idx % TILE;
                     const int64_t gi = i0 + r, gj = j0 + c;
-                    const bool in = idx < TILE * TILE && gi < m && gj < n;
-                    vy[t] = in ? yg[gi * n + gj] : (F)0;
-                    vc[t] = in ? cg[gi * n + gj] : (F)0;
+                    const bool in = gi < m && gj < n;
+                    vy[t] = in ? yg[gi * ld + gj] : (F)0;
+                    vc[t] = in ? cg[gi * ld + gj] : (F)0;
                     if (in && yfg != nullptr) {
-                        vy[t] += yfg[gi * n + gj];
-                        vc[t] += cfg[gi * n + gj];
-                        if (gets_right) vy[t] += yng[gi * n + gj];
-                        if (gets_down) vc[t] += cng[gi * n + gj];
+                        vy[t] += yfg[gi * ld + gj];
+                        vc[t] += cfg[gi * ld + gj];
+                        if (gets_right) vy[t] += yng[gi * ld + gj];
+                        if (gets_down) vc[t] += cng[gi * ld + gj];
                     }
                     vl[t] = (F)0;
-                    if (idx < TILE * TILE) {
-                        if (r > c) {
-                            if (gi < m) vl[t] = lg[gi * m + i0 + c];
-                        } else if (r < c) {
-                            if (gj < n) vl[t] = ug[(j0 + r) * n + gj];
-                        }
+                    if (r > c) {
+                        if (gi < m) vl[t] = lg[gi * ldl + i0 + c];
+                    } else if (r < c) {
+                        if (gj < n) vl[t] = ug[(j0 + r) * ldu + gj];
                     }
                 }
 #pragma unroll
                 for (int t = 0; t < UN; ++t) {
                     const int idx = base + t * TTH + tid, r = idx / TILE, c = idx % TILE;
-                    if (idx >= TILE * TILE) continue;
                     Ys[r * LD + c] = vy[t];
                     Cs[r * LD + c] = vc[t];
                     LUs[r * LD + c] = vl[t];
                 }
             }
-            if (owes_right)
-                for (int idx = tid; idx < TILE * TILE; idx += TTH) {
-                    const int r = idx / TILE, c = idx % TILE;
-                    Ubs[r * LD + c] = (j0 + r < n && j0 + TILE + c < n) ? ug[(j0 + r) * n + j0 + TILE + c] : (F)0;
+            if constexpr (PUSH) {
+                if (owes_right)
+                    for (int idx = tid; idx < TILE * TILE; idx += TTH) {
+                        const int r = idx / TILE, c = idx % TILE;
+                        Ubs[r * LD + c] = (j0 + r < n && j0 + TILE + c < n) ? ug[(j0 + r) * ldu + j0 + TILE + c] : (F)0;
+                    }
+                if (owes_down)
+                    for (int idx = tid; idx < TILE * TILE; idx += TTH) {
+                        const int r = idx / TILE, c = idx % TILE;
+                        Lbs[r * LD + c] = (i0 + TILE + r < m && i0 + c < m) ? lg[(i0 + TILE + r) * ldl + i0 + c] : (F)0;
+                    }
+            }
+            __syncthreads();
+            for (int idx = tid; idx < DROWS * DLD; idx += TTH) {
+                const int row = idx / DLD - SUB, dd = idx % DLD, blk = row / SUB, p = row % SUB;
+                F v = (F)0;
+                if (row >= 0 && blk < 2 * NSUB && dd >= 1 && dd < SUB && p + dd < SUB) {
+                    const int at = (blk % NSUB) * SUB + p;
+                    v = blk < NSUB ? LUs[(at + dd) * LD + at] : LUs[at * LD + at + dd];
                 }
-        }
-        __syncthreads();
-        for (int idx = tid; idx < 2 * NSUB * DBLK; idx += TTH) {
-            const int which = idx / (NSUB * DBLK), blk = idx / DBLK % NSUB, p = idx % DBLK / DLD, dd = idx % DLD;
-            F v = (F)0;
-            if (dd >= 1 && dd < SUB && p + dd < SUB)
-                v = which == 0 ? LUs[(blk * SUB + p + dd) * LD + blk * SUB + p] : LUs[(blk * SUB + p) * LD + blk * SUB + p + dd];
-            Dg[idx] = v;
+                Dg[idx] = v;
+            }
         }
         if (!sweeper) {
-            finish_params();
-            store_params();
+            finish_params(0);
+            store_params(0);
         }
         __syncthreads();
-
-        // Sweep of the sub-tiles.  A half-warp (16 lanes) sweeps one sub-tile, so warps 0 and 1 hold the up to four
-        // sub-tiles of a sub-tile anti-diagonal: half-warp h of warp w2 takes sub-tile row a = 2 w2 + h.  Lane k owns
-        // column k (down feedback, "C") and row k (right feedback, "Y") of its sub-tile, both skewed so that the entries of
-        // anti-diagonal s sit in register s mod 16.  At stage s lane k rounds its column's entry (p, k), p = s - k; the
-        // lane that owns row p is lane p, and lane p in turn rounds (k, p), the entry of this lane's row: the two lanes
-        // exchange the row accumulator before rounding and the completed C after it.
+        // Sweep of the sub-tiles: sweeping warp a takes the sub-tiles of row a, one per sub-tile anti-diagonal.  Lane k of the
+        // warp's first half owns column k of the sub-tile (down feedback, "C"), lane k of the second half row k (right
+        // feedback, "Y"), both skewed so that the entry of stage s sits in register 0 when the stage comes.  At stage s the
+        // column lane k and the row lane p = s - k hold the two summands of entry (p, k): one shuffle exchanges them and
+        // both lanes round the entry (the sum commutes, so they get the same bits).  The column lane pushes the error down,
+        // the row lane, which received the C accumulator with the same shuffle, the completed C to the right: one shuffle
+        // and fifteen multiply-adds per lane and stage.  (Half a warp per sub-tile with both feedbacks in one lane takes
+        // two shuffles and thirty multiply-adds: 208 cycles per stage against about 100.)
+        // What bounds a stage is the chain from one rounding to the next (multiply-add, shuffle, the quantizer's dozen dependent
+        // operations: about 95 cycles); everything else has to fit into its gaps.  So every address of a stage is a lane's base
+        // plus a constant stride (lanes before their first or past their last entry read zero rows or values that they
+        // ignore, and store nothing), the operands of a stage are loaded one stage ahead, and there is no branch inside the
+        // four unrolled stages (one branch per stage costs 40 cycles): about 120 cycles per stage for one warp on its
+        // scheduler, 150 for two, against 168 with wrapped addresses and selects.
         // The two roles run the same sequence of barriers from loops of their own, so that neither holds the other's registers.
         if (sweeper) {
+            const int sub_a = number, r0 = sub_a * SUB;
+            const int par0 = (sub_a * SUB * PLD + (role ? k * PLD - k : k - k * PLD)) * 4, par_step = (role ? 1 : PLD) * 4;
             for (int w = 0; w < 2 * NSUB - 1; ++w) {
-                const int sub_a = 2 * warp + half;
-                const int b_raw = w - sub_a;
-                const bool tile_ok = b_raw >= 0 && b_raw < NSUB;  // a half-warp without a sub-tile runs along with everything masked
-                const int b = tile_ok ? b_raw : 0;
-                const int r0 = sub_a * SUB, c0 = b * SUB;
-                const unsigned valid_bits = Pv[tid] | Pv[LANES + tid];
-                const bool fast_division = (Pv[2 * LANES + warp] & Pv[2 * LANES + SWEEPERS + warp]) != 0u;
-                F cacc[SUB], yacc[SUB];
+                const int b = w - sub_a;
+                if (b >= 0 && b < NSUB) {
+                    const int c0 = b * SUB;
+                    // entries of this lane inside the matrix: the first `count` of its column or row
+                    const int rows_left = rows_in - r0, cols_left = cols_in - c0;
+                    const int along = role ? cols_left : rows_left, count = k < (role ? rows_left : cols_left) ? max(0, min(along, SUB)) : 0;
+                    const int step = role ? 1 : LD;
+                    F acc[SUB];
+                    {
+                        const F *const src = role ? Ys + (r0 + k) * LD + c0 : Cs + r0 * LD + c0 + k;
 #pragma unroll
-                for (int r = 0; r < SUB; ++r) {
-                    const int o = (r - k) & (SUB - 1);
-                    cacc[r] = Cs[(r0 + o) * LD + c0 + k];
-                    yacc[r] = Ys[(r0 + k) * LD + c0 + o];
-                }
-                // entry (s - k, k) of the sub-tile: a lane-constant address plus s rows
-                const int entry0 = (r0 - k) * LD + c0 + k;
-                F *pre_ptr = pre ? pre + (i0 + r0 - k) * n + j0 + c0 + k : nullptr;
-                const int zst0 = (r0 - k) * ZLD + k;
-                const F *const dgl = Dg + sub_a * DBLK, *const dgu = Dg + (NSUB + b) * DBLK;
-                // The 32 stages in groups of ROLL: inside a group the registers are indexed statically, after it they are
-                // renamed by moving them ROLL places, so that the loop body is ROLL stages long (the fully unrolled form
-                // is 25 KB of straight-line code per pass that no instruction cache level close to the scheduler holds).
-                auto stages = [&](auto fast_tag) {
-                    constexpr bool FASTDIV = decltype(fast_tag)::value;
-#pragma unroll 1
-                    for (int group = 0; group < 2 * SUB / ROLL; ++group) {
-                        const int s_first = group * ROLL;
-#pragma unroll
-                        for (int j = 0; j < ROLL; ++j) {
-                            const int s = s_first + j, r = s & (SUB - 1);
-                            const int p = s - k;  // row of this lane's column entry = column of its row entry = partner lane
-                            const bool active = tile_ok && p >= 0 && p < SUB;
-                            const int pw = p & (SUB - 1);
-                            const F yrow = __shfl_sync(0xffffffffu, yacc[j], pw, SUB);  // Y accumulator of (p, k) from the owner of row p
-                            const F yv = yrow + cacc[j];
-                            const bool ok = active && ((valid_bits >> r) & 1u);
-                            F z;
-                            if (KIND == G2D_Q_AFFINE) {
-                                const F scv = Ps[(0 * SUB + r) * LANES + tid], zpv = Ps[(1 * SUB + r) * LANES + tid];
-                                z = FASTDIV ? affine_value_rcp(yv, scv, zpv, Ps[(2 * SUB + r) * LANES + tid], P.qmin, P.qmax) : affine_value(yv, scv, zpv, P.qmin, P.qmax);
-                            } else if (KIND == G2D_Q_FORCED) {
-                                z = Ps[(0 * SUB + r) * LANES + tid];
-                            } else {
-                                z = rint_even(yv);
-                            }
-                            const F ev = ok ? z - yv : (F)0;
-                            const F cc = cacc[j] + ev;
-                            const F ccrow = __shfl_sync(0xffffffffu, cc, pw, SUB);  // completed C of (k, p), rounded by lane p
-                            if (active) {
-                                Ys[entry0 + s * LD] = ev;
-                                Cs[entry0 + s * LD] = cc;
-                                Zst[zst0 + s * ZLD] = z;
-                            }
-                            if (ok && pre_ptr) pre_ptr[(int64_t)s * n] = yv;
-                            // pushes: the error down column k through L, the completed C of (k, p) right along row k through U;
-                            // rows past the block's end read the zero padding, inactive lanes push zero
-                            const F vcol = active ? ev : (F)0, vrow = active ? ccrow : (F)0;
-                            F kl[SUB], ku[SUB];
+                        for (int r = 0; r < SUB; ++r) acc[r] = src[((r - k) & (SUB - 1)) * step];
+                    }
+                    F *const pre_ptr = pre + (i0 + r0) * n + j0 + c0 + k;  // the caller's array: rows of n
+                    const int partner0 = ((role ^ 1) << 4) - k;
+                    auto stages = [&](auto divide_tag, auto record_tag) {
+                        constexpr int DIVIDE = decltype(divide_tag)::value;
+                        constexpr bool RECORD = decltype(record_tag)::value;
+                        uint32_t dg = shared_address(Dg) + (uint32_t)((SUB + ((role ? NSUB + b : sub_a)) * SUB - k) * DLD * (int)sizeof(F));
+                        uint32_t par = shared_address(Par) + (uint32_t)(par0 * (int)sizeof(F));
+                        const uint32_t par_bytes = (uint32_t)(par_step * (int)sizeof(F));
+                        uint32_t own = shared_address(role ? Cs + (r0 + k) * LD + c0 : Ys + r0 * LD + c0 + k) - (uint32_t)(k * step * (int)sizeof(F));
+                        F kc[SUB], pa[4];
+                        auto fetch = [&](uint32_t d, uint32_t q, F (&co)[SUB], F (&pq)[4]) {
+                            if (KIND != G2D_Q_ROUND) load4_here(q, pq);
 #pragma unroll
                             for (int v4 = 0; v4 < SUB; v4 += 4) {
                                 F t[4];
-                                load4(dgl + pw * DLD + v4, t);
+                                load4_here(d + (uint32_t)(v4 * (int)sizeof(F)), t);
 #pragma unroll
-                                for (int x = 0; x < 4; ++x) kl[v4 + x] = t[x];
-                                load4(dgu + pw * DLD + v4, t);
-#pragma unroll
-                                for (int x = 0; x < 4; ++x) ku[v4 + x] = t[x];
+                                for (int x = 0; x < 4; ++x) co[v4 + x] = t[x];
                             }
+                        };
+                        fetch(dg, par, kc, pa);
+                        int p = -k;  // place of this lane's entry in its column or row
+#pragma unroll 1
+                        for (int s_first = 0; s_first < 2 * SUB; s_first += ROLL) {
 #pragma unroll
-                            for (int dd = 1; dd < SUB; ++dd) {
-                                cacc[(j + dd) & (SUB - 1)] += kl[dd] * vcol;
-                                yacc[(j + dd) & (SUB - 1)] += ku[dd] * vrow;
+                            for (int j = 0; j < ROLL; ++j) {
+                                const bool ok = (unsigned)p < (unsigned)count;
+                                const F other = __shfl_sync(0xffffffffu, acc[0], partner0 + s_first + j);
+                                F kc_next[SUB], pa_next[4];
+                                fetch(dg + (uint32_t)((j + 1) * DLD * (int)sizeof(F)), par + par_bytes, kc_next, pa_next);
+                                const F carry = role ? other : (F)0;
+                                const F yv = acc[0] + other;
+                                F z;
+                                if (KIND == G2D_Q_AFFINE) {
+                                    z = DIVIDE == 2   ? affine_value(yv, pa[0], pa[1], P.qmin, P.qmax)
+                                        : DIVIDE == 1 ? affine_value_rcp(yv, pa[0], pa[1], pa[2], P.qmin, P.qmax)
+                                                      : affine_value_fast(yv, pa[0], pa[1], pa[2], P.qmin, P.qmax);
+                                } else if (KIND == G2D_Q_FORCED) {
+                                    z = pa[0];
+                                } else {
+                                    z = rint_even(yv);
+                                }
+                                const F carried = (z - yv) + carry;  // completed C (row lanes) or error (column lanes)
+                                const F v = ok ? carried : (F)0;     // lanes without an entry push zero
+#pragma unroll
+                                // the push moves every accumulator down by one register on the way
+                                const F last = acc[0];
+#pragma unroll
+                                for (int dd = 1; dd < SUB; ++dd) acc[dd - 1] = acc[dd] + kc[dd] * v;
+                                acc[SUB - 1] = last;
+                                store_shared_if(own, carried, ok);
+                                store_shared_if(par + 3 * (uint32_t)sizeof(F), z, ok);  // both lanes of an entry store the same value
+                                if (RECORD && ok && !role) pre_ptr[(int64_t)p * n] = yv;
+                                own += (uint32_t)(step * (int)sizeof(F));
+                                par += par_bytes;
+                                ++p;
+#pragma unroll
+                                for (int x = 0; x < SUB; ++x) kc[x] = kc_next[x];
+#pragma unroll
+                                for (int x = 0; x < 4; ++x) pa[x] = pa_next[x];
                             }
+                            dg += (uint32_t)(ROLL * DLD * (int)sizeof(F));
                         }
-                        // rename: what was register i + ROLL is register i from here on
-                        F keep_c[ROLL], keep_y[ROLL];
-#pragma unroll
-                        for (int i = 0; i < ROLL; ++i) { keep_c[i] = cacc[i]; keep_y[i] = yacc[i]; }
-#pragma unroll
-                        for (int i = 0; i < SUB - ROLL; ++i) { cacc[i] = cacc[i + ROLL]; yacc[i] = yacc[i + ROLL]; }
-#pragma unroll
-                        for (int i = 0; i < ROLL; ++i) { cacc[SUB - ROLL + i] = keep_c[i]; yacc[SUB - ROLL + i] = keep_y[i]; }
-                    }
-                };
-                if (fast_division) stages(std::true_type{});
-                else stages(std::false_type{});
+                    };
+                    using std::integral_constant;
+                    // 0 and 1 for the common case, without a branch in the stages; recording the pre-rounding values is a matter of tests
+                    const bool exact = !fast_div[sub_a];
+                    if (pre != nullptr) {
+                        if (exact) stages(integral_constant<int, 2>{}, std::true_type{});
+                        else stages(integral_constant<int, 1>{}, std::true_type{});
+                    } else if (exact) stages(integral_constant<int, 2>{}, std::false_type{});
+                    else if (sizeof(F) != sizeof(float) || !P.small_integer_bounds) stages(integral_constant<int, 1>{}, std::false_type{});
+                    else stages(integral_constant<int, 0>{}, std::false_type{});
+                }
                 __syncthreads();
-                if (w + 1 < 2 * NSUB - 1) __syncthreads();  // the helpers carry the anti-diagonal just swept into the next one
+                if (w + 1 < 2 * NSUB - 1) {
+                    // the anti-diagonal just swept, carried into the next one: the right product here, the down product by the helper
+                    const int bn = w + 1 - sub_a;
+                    if (bn >= 1 && bn < NSUB)
+                        mm16<SMALL>(Ys + r0 * LD + bn * SUB, Cs + r0 * LD + (bn - 1) * SUB, LUs + (bn - 1) * SUB * LD + bn * SUB, lane);
+                    __syncthreads();
+                }
             }
         } else {
-            // ---- neighbour push: registers of the helper warps (float, pipelined schedule) ----
-            // Helper warp h keeps, in the layout of mm16 (rows 2 (lane / 4) and the next one), its two rows of the strip
-            // L[I + 1, I](rows 16 h ..) for the down push (of each block of 16 columns the four that belong to lane % 4:
-            // the four lanes of a row pair share them by shuffle), the running sums of the right push of sub-tile row h (four blocks;
-            // not for the last row, whose four blocks are spread over the four helpers so that the work left after the
-            // last sweep is one product each), and the last column's down push up to its last term.
-            F lb0[PUSH ? TILE / 4 : 1], lb1[PUSH ? TILE / 4 : 1];
-            F yn0[PUSH ? NSUB : 1][4], yn1[PUSH ? NSUB : 1][4], y30[4], y31[4], c30[4], c31[4];
-            if constexpr (PUSH) {
-#pragma unroll
-                for (int y = 0; y < 4; ++y) {
-#pragma unroll
-                    for (int cb = 0; cb < NSUB; ++cb) yn0[cb][y] = yn1[cb][y] = (F)0;
-                    y30[y] = y31[y] = c30[y] = c31[y] = (F)0;
-                }
-            }
             for (int w = 0; w < 2 * NSUB - 1; ++w) {
                 const bool more = w + 1 < 2 * NSUB - 1;
-                // Helper warp of sub-tile row ap, while sub-tile anti-diagonal w is swept.  Everything written here goes
-                // to sub-tiles of row ap on later anti-diagonals, which no other warp touches before the barrier.
                 const int ap = helper;
                 if (more) fetch_params(w + 1);
-                if (w >= 1) {
-                    // the sub-tiles swept one anti-diagonal ago, carried into the sub-tiles two or more ahead of them
-                    const int first = w + 1 - ap > 0 ? w + 1 - ap : 0;
-                    for (int bp = first; bp < NSUB; ++bp) carry_into(Ys, Cs, LUs, ap, bp, w - 1 - bp, w - 1 - ap, lane);
-                    __syncwarp();
+                // While sub-tile anti-diagonal w is swept: the products of the sub-tiles (a, b) swept one anti-diagonal ago, i.e.
+                // the row strip of each in the push to the right neighbour, the column strip in the push to the lower one
+                // (dealt out to the helpers in turn), and the feedback to the sub-tiles two or more places down (helpers 0
+                // and 1) and to the right (2 and 3).  All these products have targets of their own, none of them on w.
+                const int a_lo = max(0, w - NSUB), a_hi = min(NSUB, w);
+#pragma unroll 1
+                for (int a = a_lo; a < a_hi; ++a) {
+                    const int b = w - 1 - a, to = helper < 2 ? a + 2 + helper : b + helper;
+                    if (to >= NSUB) continue;
+                    if (helper < 2) mm16<SMALL>(Cs + to * SUB * LD + b * SUB, LUs + to * SUB * LD + a * SUB, Ys + a * SUB * LD + b * SUB, lane);
+                    else mm16<SMALL>(Ys + a * SUB * LD + to * SUB, Cs + a * SUB * LD + b * SUB, LUs + b * SUB * LD + to * SUB, lane);
                 }
                 if constexpr (PUSH) {
-                    const bool pvec = n % 4 == 0 && reinterpret_cast<uintptr_t>(yng) % (4 * sizeof(F)) == 0;
-                    if (owes_down && w == 1) {  // the strip of L[I + 1, I]: first used three anti-diagonals from here
-                        const int64_t gi = i0 + TILE + ap * SUB + (lane >> 2) * 2;
-                        const bool lvec = m % 4 == 0 && reinterpret_cast<uintptr_t>(lg) % (4 * sizeof(F)) == 0;
-#pragma unroll
-                        for (int as = 0; as < NSUB; ++as) {
-                            const int64_t col = i0 + as * SUB + (lane & 3) * 4;
-                            F t0[4] = {(F)0, (F)0, (F)0, (F)0}, t1[4] = {(F)0, (F)0, (F)0, (F)0};
-                            if (lvec) {
-                                if (gi < m) load4(lg + gi * m + col, t0);
-                                if (gi + 1 < m) load4(lg + (gi + 1) * m + col, t1);
-                            } else {
-#pragma unroll
-                                for (int x = 0; x < 4; ++x) {
-                                    if (gi < m) t0[x] = lg[gi * m + col + x];
-                                    if (gi + 1 < m) t1[x] = lg[(gi + 1) * m + col + x];
-                                }
-                            }
-#pragma unroll
-                            for (int x = 0; x < 4; ++x) { lb0[as * 4 + x] = t0[x]; lb1[as * 4 + x] = t1[x]; }
-                        }
-                    }
-                    if (owes_right && w >= 1) {
-                        // right push: the completed C of the row's sub-tile swept one anti-diagonal ago times its block
-                        // row of U[J, J + 1]; a row is stored once its last sub-tile has gone in
-                        const int b = w - 1 - ap;
-                        if (ap < NSUB - 1 && b >= 0 && b < NSUB) {
-#pragma unroll
-                            for (int cb = 0; cb < NSUB; ++cb) mm16_acc(yn0[cb], yn1[cb], Cs + ap * SUB * LD + b * SUB, Ubs + b * SUB * LD + cb * SUB, lane);
-                            if (b == NSUB - 1) {
-#pragma unroll
-                                for (int cb = 0; cb < NSUB; ++cb)
-                                    store_block(yng + (i0 + ap * SUB) * n + j0 + TILE + cb * SUB, n, yn0[cb], yn1[cb], lane, m - (i0 + ap * SUB), n - (j0 + TILE + cb * SUB), pvec);
-                            }
-                        }
-                        const int b3 = w - NSUB;  // the last row's sub-tile swept one anti-diagonal ago: this helper's column block of it
-                        if (b3 >= 0 && b3 < NSUB) mm16_acc(y30, y31, Cs + (NSUB - 1) * SUB * LD + b3 * SUB, Ubs + b3 * SUB * LD + ap * SUB, lane);
-                    }
-                    if (owes_down) {
-                        // down push: a column of sub-tiles is complete three anti-diagonals after its first; this helper's
-                        // row strip of L[I + 1, I] times the column's errors, stored at once
-                        const int b = w - NSUB;
-                        if (b >= 0) {
-                            F d0[4] = {(F)0, (F)0, (F)0, (F)0}, d1[4] = {(F)0, (F)0, (F)0, (F)0};
-#pragma unroll
-                            for (int as = 0; as < NSUB; ++as) mm16_areg(d0, d1, lb0 + as * 4, lb1 + as * 4, Ys + as * SUB * LD + b * SUB, lane);
-                            store_block(cng + (i0 + TILE + ap * SUB) * n + j0 + b * SUB, n, d0, d1, lane, m - (i0 + TILE + ap * SUB), n - (j0 + b * SUB), pvec);
-                        }
-                        if (!more) {  // the last column, up to the term of the sub-tile being swept now
-#pragma unroll
-                            for (int as = 0; as < NSUB - 1; ++as) mm16_areg(c30, c31, lb0 + as * 4, lb1 + as * 4, Ys + as * SUB * LD + (NSUB - 1) * SUB, lane);
+#pragma unroll 1
+                    for (int job = helper; job < 2 * (a_hi - a_lo); job += HELPERS) {
+                        const int a = a_lo + (job >> 1), b = w - 1 - a;
+                        if (job & 1) {
+                            if (owes_down) mm16<TALL>(Cns + b * SUB, Lbs + a * SUB, Ys + a * SUB * LD + b * SUB, lane);
+                        } else {
+                            if (owes_right) mm16<WIDE>(Yns + a * SUB * LD, Cs + a * SUB * LD + b * SUB, Ubs + b * SUB * LD, lane);
                         }
                     }
                 }
-                if (more) finish_params();
+                if (more) finish_params(w + 1);
                 __syncthreads();
                 {   // the rounded values of the sub-tiles just swept: helper warp ap writes out the block of its row
                     const int bz = w - ap;
                     if (bz >= 0 && bz < NSUB) {
-                        const bool zvec = n % 4 == 0 && reinterpret_cast<uintptr_t>(yg) % (4 * sizeof(F)) == 0;
+                        const bool zvec = ld % 4 == 0 && reinterpret_cast<uintptr_t>(yg) % (4 * sizeof(F)) == 0;
 #pragma unroll
                         for (int q = 0; q < 2; ++q) {
                             const int e = lane * 2 + q, row = e >> 2, c4 = (e & 3) * 4;
                             const int64_t gi = i0 + ap * SUB + row, gj = j0 + bz * SUB + c4;
                             F v[4];
-                            load4(Zst + (ap * SUB + row) * ZLD + c4, v);
+#pragma unroll
+                            for (int x = 0; x < 4; ++x) v[x] = Par[((ap * SUB + row) * PLD + c4 + x) * 4 + 3];
                             if (gi < m) {
                                 if (zvec) {
-                                    if (gj < n) store4(yg + gi * n + gj, v);
+                                    if (gj < n) store4(yg + gi * ld + gj, v);
                                 } else {
 #pragma unroll
                                     for (int x = 0; x < 4; ++x)
-                                        if (gj + x < n) yg[gi * n + gj + x] = v[x];
+                                        if (gj + x < n) yg[gi * ld + gj + x] = v[x];
                                 }
                             }
                         }
+                        __syncwarp();  // the next parameters overwrite them
                     }
                 }
                 // ---- between two sweeps: the anti-diagonal just swept, carried into the next one; the next parameters ----
                 if (more) {
-                    store_params();
+                    store_params(w + 1);
                     const int bn = w + 1 - ap;
-                    if (bn >= 0 && bn < NSUB) carry_into(Ys, Cs, LUs, ap, bn, ap - 1, bn - 1, lane);
+                    if (ap >= 1 && bn >= 0 && bn < NSUB)  // the right product is the sweeping warp's
+                        mm16<SMALL>(Cs + ap * SUB * LD + bn * SUB, LUs + ap * SUB * LD + (ap - 1) * SUB, Ys + (ap - 1) * SUB * LD + bn * SUB, lane);
                     __syncthreads();
                 }
             }
-            // ---- neighbour push: the last sub-tile's terms, one product per helper and plane ----
-            if constexpr (PUSH) {
-                {
-                    const bool pvec = n % 4 == 0 && reinterpret_cast<uintptr_t>(yng) % (4 * sizeof(F)) == 0;
-                    const int x = helper, last = NSUB - 1;
-                    if (owes_right) {
-                        mm16_acc(y30, y31, Cs + last * SUB * LD + last * SUB, Ubs + last * SUB * LD + x * SUB, lane);
-                        store_block(yng + (i0 + last * SUB) * n + j0 + TILE + x * SUB, n, y30, y31, lane, m - (i0 + last * SUB), n - (j0 + TILE + x * SUB), pvec);
+        }
+        // ---- neighbour push: the last sub-tile's terms, one product per warp, then out to the planes of the neighbours ----
+        if constexpr (PUSH) {
+            if (owes_right || owes_down) {
+                constexpr int last = NSUB - 1;
+                const int x = warp & 3;
+                F *const D = warp < 4 ? Yns + last * SUB * LD + x * SUB : Cns + x * SUB * LD + last * SUB;
+                const F *const A = warp < 4 ? Cs + last * SUB * LD + last * SUB : Lbs + x * SUB * LD + last * SUB;
+                const F *const B = warp < 4 ? Ubs + last * SUB * LD + x * SUB : Ys + last * SUB * LD + last * SUB;
+                if (warp < 4 ? owes_right : owes_down) mm16<SMALL>(D, A, B, lane);
+                __syncthreads();
+                // rows and columns past the matrix are not stored; a row's last group of four may reach into its padding
+                const bool pvec = ld % 4 == 0 && reinterpret_cast<uintptr_t>(yng) % (4 * sizeof(F)) == 0;
+                for (int idx = tid; idx < TILE * TILE / 4; idx += TTH) {
+                    const int r = idx / (TILE / 4), c = (idx % (TILE / 4)) * 4;
+                    F v[4];
+                    if (owes_right && i0 + r < m && j0 + TILE + c < n) {
+                        load4(Yns + r * LD + c, v);
+                        F *dst = yng + (i0 + r) * ld + j0 + TILE + c;
+                        if (pvec) store4(dst, v);
+                        else
+                            for (int x4 = 0; x4 < 4; ++x4)
+                                if (j0 + TILE + c + x4 < n) dst[x4] = v[x4];
                     }
-                    if (owes_down) {
-                        mm16_areg(c30, c31, lb0 + last * 4, lb1 + last * 4, Ys + last * SUB * LD + last * SUB, lane);
-                        store_block(cng + (i0 + TILE + x * SUB) * n + j0 + last * SUB, n, c30, c31, lane, m - (i0 + TILE + x * SUB), n - (j0 + last * SUB), pvec);
+                    if (owes_down && i0 + TILE + r < m && j0 + c < n) {
+                        load4(Cns + r * LD + c, v);
+                        F *dst = cng + (i0 + TILE + r) * ld + j0 + c;
+                        if (pvec) store4(dst, v);
+                        else
+                            for (int x4 = 0; x4 < 4; ++x4)
+                                if (j0 + c + x4 < n) dst[x4] = v[x4];
                     }
                 }
             }
@@ -670,8 +635,8 @@ __global__ void __launch_bounds__(TTH) tile_sweep_kernel(SweepArgs<F> P, int S, 
                             float v[4], hi[4], lo[4];
                             load4(reinterpret_cast<const float *>(Cs) + r * LD + c, v);
                             split4(v, hi, lo);
-                            store4(P.c_hi + (i0 + r) * n + j0 + c, hi);
-                            store4(P.c_lo + (i0 + r) * n + j0 + c, lo);
+                            store4(P.c_hi + (i0 + r) * ld + j0 + c, hi);
+                            store4(P.c_lo + (i0 + r) * ld + j0 + c, lo);
                         }
                         {
                             const int c = idx % TILE, r = (idx / TILE) * 4;
@@ -679,8 +644,8 @@ __global__ void __launch_bounds__(TTH) tile_sweep_kernel(SweepArgs<F> P, int S, 
 #pragma unroll
                             for (int x = 0; x < 4; ++x) v[x] = (float)Ys[(r + x) * LD + c];
                             split4(v, hi, lo);
-                            store4(P.et_hi + (j0 + c) * m + i0 + r, hi);
-                            store4(P.et_lo + (j0 + c) * m + i0 + r, lo);
+                            store4(P.et_hi + (j0 + c) * P.ldm + i0 + r, hi);
+                            store4(P.et_lo + (j0 + c) * P.ldm + i0 + r, lo);
                         }
                     }
                 } else {
@@ -692,8 +657,8 @@ __global__ void __launch_bounds__(TTH) tile_sweep_kernel(SweepArgs<F> P, int S, 
                                 const float v = (float)Cs[r * LD + c];
                                 uint32_t h;
                                 asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(h) : "f"(v));
-                                P.c_hi[gi * n + gj] = __uint_as_float(h);
-                                P.c_lo[gi * n + gj] = v - __uint_as_float(h);
+                                P.c_hi[gi * ld + gj] = __uint_as_float(h);
+                                P.c_lo[gi * ld + gj] = v - __uint_as_float(h);
                             }
                         }
                         {   // E^T[j][i], consecutive threads along i
@@ -703,31 +668,32 @@ __global__ void __launch_bounds__(TTH) tile_sweep_kernel(SweepArgs<F> P, int S, 
                                 const float v = (float)Ys[r * LD + c];
                                 uint32_t h;
                                 asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(h) : "f"(v));
-                                P.et_hi[gj * m + gi] = __uint_as_float(h);
-                                P.et_lo[gj * m + gi] = v - __uint_as_float(h);
+                                P.et_hi[gj * P.ldm + gi] = __uint_as_float(h);
+                                P.et_lo[gj * P.ldm + gi] = v - __uint_as_float(h);
                             }
                         }
                     }
                 }
             }
         }
-        // ---- store the errors and the completed C of the tile ----
-        if (vec) {
+        // ---- store the errors and the completed C of the tile, unless only their operand planes are read from here on ----
+        if (yng != nullptr) {
+        } else if (vec) {
             for (int idx = tid; idx < TILE * TILE / 4; idx += TTH) {
                 const int r = idx / (TILE / 4), c = (idx % (TILE / 4)) * 4;
                 F ve[4], vc[4];
                 load4(Ys + r * LD + c, ve);
                 load4(Cs + r * LD + c, vc);
-                store4(eg + (i0 + r) * n + j0 + c, ve);
-                store4(cg + (i0 + r) * n + j0 + c, vc);
+                store4(eg + (i0 + r) * ld + j0 + c, ve);
+                store4(cg + (i0 + r) * ld + j0 + c, vc);
             }
         } else {
             for (int idx = tid; idx < TILE * TILE; idx += TTH) {
                 const int r = idx / TILE, c = idx % TILE;
                 const int64_t gi = i0 + r, gj = j0 + c;
                 if (gi < m && gj < n) {
-                    eg[gi * n + gj] = Ys[r * LD + c];
-                    cg[gi * n + gj] = Cs[r * LD + c];
+                    eg[gi * ld + gj] = Ys[r * LD + c];
+                    cg[gi * ld + gj] = Cs[r * LD + c];
                 }
             }
         }
@@ -739,7 +705,7 @@ template <typename F, int KIND>
 static int launch_kind(const SweepArgs<F> &args, int S, int parity, cudaStream_t stream) {
     // the opt-in to more than 48 KB of dynamic shared memory is per device
     static PerDeviceOnce configured;
-    const size_t smem = sizeof(F) * (4 * TILE * LD + 2 * NSUB * DBLK + 3 * SUB * LANES + NSUB * SUB * ZLD) + sizeof(unsigned) * (2 * LANES + 2 * SWEEPERS);
+    const size_t smem = sizeof(F) * (3 * TILE * LD + DROWS * DLD + NSUB * SUB * PLD * 4 + (sizeof(F) == sizeof(float) ? 4 * TILE * LD : PPAD * 4));
     // and the largest shared-memory carve-out, like the update kernels that run on the neighbouring SMs
     if (configured.run([&] {
             return cudaFuncSetAttribute(tile_sweep_kernel<F, KIND>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) == cudaSuccess &&
