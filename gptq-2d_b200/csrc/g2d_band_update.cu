@@ -5,12 +5,11 @@
 //
 // with stage(i, j) = i / P + j / Q.  This is the work of _repack_errors_kernel + _flush_down_kernel +
 // _flush_right_kernel of the reference (gptq_2d.py:632-1057).  The errors stay in their natural
-// [m, n] layout and the band is selected by masks while the operands are staged in shared memory, so
-// there is no repacking pass.  In tile mode (P = Q = TILE, used by the fused sweep) stages are tile
-// anti-diagonals, every operand block is either wholly inside or wholly outside the band and the
-// k range of a target tile is exact; the plain (P = Q = 1) and general modes serve the generic path.
+// [m, n] layout and there is no repacking pass.  In tile mode (P = Q = TILE, used by the fused sweep) stages are tile
+// anti-diagonals, every operand block is either wholly inside or wholly outside the band and the k range of a target
+// tile is exact; the plain (P = Q = 1) and general modes serve the generic path with masks (second kernel).
 //
-// One CTA of 64 threads owns one 64 x 64 target tile; each thread accumulates 8 x 8 outputs in
+// Tile mode: one CTA of 64 threads owns one 64 x 64 target tile; each thread accumulates 8 x 8 outputs in
 // registers, operands are staged 16 k at a time.
 #include "g2d_common.cuh"
 
@@ -25,42 +24,20 @@ constexpr int BLD = BT + 4;  // shared row stride of the staged operands
 // so that its shared-memory reads are two 16-byte vectors that never collide with its neighbours'.
 __device__ __forceinline__ int own(int t, int x) { return x < 4 ? t * 4 + x : 32 + t * 4 + (x - 4); }
 
-template <typename F, int MODE>
-struct BandGeom {
-    int P, Q;
-    int64_t s0, s1, s_end;
-    __device__ __forceinline__ int64_t stage(int64_t i, int64_t j) const {
-        if (MODE == BAND_TILE) return (i / TILE) + (j / TILE);
-        if (MODE == BAND_PLAIN) return i + j;
-        return i / P + j / Q;
-    }
-    __device__ __forceinline__ int64_t brow(int64_t i) const { return MODE == BAND_TILE ? i / TILE : (MODE == BAND_PLAIN ? i : i / P); }
-    __device__ __forceinline__ int64_t bcol(int64_t j) const { return MODE == BAND_TILE ? j / TILE : (MODE == BAND_PLAIN ? j : j / Q); }
-};
-
-// acc[8][8] += A[i0.., k_lo..k_hi) * B[k_lo..k_hi), j0..) with element masks:
-//   DOWN : A = L[i, k] where brow(k) < brow(i);       B = E[k, j] where stage(k, j) in [s0, s1)
-//   RIGHT: A = C[i, k] where stage(i, k) in [s0, s1);  B = U[k, j] where bcol(k) < bcol(j)
-template <typename F, int MODE, bool DOWN>
-__device__ __forceinline__ void band_product(F (&acc)[8][8], const F *__restrict__ A, int64_t lda, const F *__restrict__ B,
-                                             int64_t ldb, int64_t i0, int64_t j0, int64_t rows, int64_t cols,
-                                             int64_t k_lo, int64_t k_hi, const BandGeom<F, MODE> &g, F *As, F *Bs) {
+// Edge tiles in tile mode: acc[8][8] += A[i0.., k_lo..k_hi) * B[k_lo..k_hi), j0..) with zeros outside the matrix.
+template <typename F>
+__device__ __forceinline__ void band_product(F (&acc)[8][8], const F *__restrict__ A, int64_t lda, const F *__restrict__ B, int64_t ldb,
+                                             int64_t i0, int64_t j0, int64_t rows, int64_t cols, int64_t k_lo, int64_t k_hi, F *As, F *Bs) {
     const int tid = threadIdx.x, ty = tid >> 3, tx = tid & 7;
     for (int64_t k0 = k_lo; k0 < k_hi; k0 += BK) {
         // stage A transposed (As[kk][row]) and B (Bs[kk][col])
         for (int idx = tid; idx < BT * BK; idx += BTH) {
             const int row = idx / BK, kk = idx % BK;
-            const int64_t i = i0 + row, k = k0 + kk;
-            bool ok = i < rows && k < k_hi;
-            if (MODE != BAND_TILE && ok) ok = DOWN ? g.brow(k) < g.brow(i) : (g.stage(i, k) >= g.s0 && g.stage(i, k) < g.s1);
-            As[kk * BLD + row] = ok ? A[i * lda + k] : (F)0;
+            As[kk * BLD + row] = i0 + row < rows && k0 + kk < k_hi ? A[(i0 + row) * lda + k0 + kk] : (F)0;
         }
         for (int idx = tid; idx < BT * BK; idx += BTH) {
             const int kk = idx / BT, col = idx % BT;
-            const int64_t k = k0 + kk, j = j0 + col;
-            bool ok = j < cols && k < k_hi;
-            if (MODE != BAND_TILE && ok) ok = DOWN ? (g.stage(k, j) >= g.s0 && g.stage(k, j) < g.s1) : g.bcol(k) < g.bcol(j);
-            Bs[kk * BLD + col] = ok ? B[k * ldb + j] : (F)0;
+            Bs[kk * BLD + col] = j0 + col < cols && k0 + kk < k_hi ? B[(k0 + kk) * ldb + j0 + col] : (F)0;
         }
         __syncthreads();
 #pragma unroll
@@ -166,7 +143,7 @@ __device__ __forceinline__ void band_product_fast(F (&acc)[8][8], const F *__res
     }
 }
 
-template <typename F, int MODE>
+template <typename F>
 __global__ void __launch_bounds__(BTH) band_update_kernel(BandArgs<F> P, int nTI, int nTJ, int a_lo) {
     __shared__ __align__(16) F As[2 * BK * BLD];
     __shared__ __align__(16) F Bs[2 * BK * BLD];
@@ -178,109 +155,192 @@ __global__ void __launch_bounds__(BTH) band_update_kernel(BandArgs<F> P, int nTI
     const int TJ = A - TI;
     const int64_t m = P.m, n = P.n;
     const int64_t i0 = (int64_t)TI * BT, j0 = (int64_t)TJ * BT;
-    const int64_t i1 = min(i0 + BT, m) - 1, j1 = min(j0 + BT, n) - 1;  // last row / column of the tile
     const int tid = threadIdx.x, ty = tid >> 3, tx = tid & 7;
+    // the k ranges of the tile's sources: whole tiles above it (down) and to its left (right)
+    int64_t dk_lo = max((P.s0 - TJ) * BT, (int64_t)0), dk_hi = min(min((P.s1 - TJ) * BT, m), (int64_t)TI * BT);
+    int64_t rk_lo = max((P.s0 - TI) * BT, (int64_t)0), rk_hi = min(min((P.s1 - TI) * BT, n), (int64_t)TJ * BT);
+    if (P.filter == 2 && !((TI & 1) && (TJ & 1))) return;
+    if (P.filter == 1) {
+        // single-stage use: the down source is tile (dk_lo / 64, TJ), the right source tile (TI, rk_lo / 64)
+        if ((TJ & 1) || ((dk_lo / BT) & 1)) dk_hi = dk_lo;
+        if ((TI & 1) || ((rk_lo / BT) & 1)) rk_hi = rk_lo;
+    }
 
     for (int64_t batch = blockIdx.z; batch < P.batch; batch += gridDim.z) {
-        // the band of this batch: the same for every batch unless the batches are the skewed slabs of an N-factor sweep
-        const int64_t behind = (MODE == BAND_GENERAL && P.skew != nullptr) ? P.skew[batch] : 0;
-        const int64_t s0 = P.s0 - behind, s1 = P.s1 - behind, s_end = P.s_end - behind;
-        BandGeom<F, MODE> g{P.P, P.Q, s0, s1, s_end};
-        // does the tile hold any target?
-        if (g.stage(i1, j1) < s1 || g.stage(i0, j0) >= s_end) continue;
-        // k ranges: block rows (down) / block columns (right) that hold sources for this tile
-        const int64_t PP = MODE == BAND_TILE ? TILE : (MODE == BAND_PLAIN ? 1 : P.P);
-        const int64_t QQ = MODE == BAND_TILE ? TILE : (MODE == BAND_PLAIN ? 1 : P.Q);
-        int64_t dk_lo = (s0 - g.bcol(j1)) * PP, dk_hi = (s1 - g.bcol(j0)) * PP;
-        dk_lo = max(dk_lo, (int64_t)0);
-        dk_hi = min(min(dk_hi, m), g.brow(i1) * PP);  // sources lie in block rows above the targets
-        int64_t rk_lo = (s0 - g.brow(i1)) * QQ, rk_hi = (s1 - g.brow(i0)) * QQ;
-        rk_lo = max(rk_lo, (int64_t)0);
-        rk_hi = min(min(rk_hi, n), g.bcol(j1) * QQ);
-        if (MODE == BAND_TILE && P.filter == 2 && !((TI & 1) && (TJ & 1))) continue;
-        if (MODE == BAND_TILE && P.filter == 1) {
-            // single-stage use: the down source is tile (dk_lo / 64, TJ), the right source tile (TI, rk_lo / 64)
-            if ((TJ & 1) || ((dk_lo / TILE) & 1)) dk_hi = dk_lo;
-            if ((TI & 1) || ((rk_lo / TILE) & 1)) rk_hi = rk_lo;
-        }
         F *yg = P.y + batch * m * n, *cg = P.c + batch * m * n;
         const F *eg = P.e + batch * m * n;
         const F *lg = P.l + (P.l_off ? P.l_off[batch] : 0);
         const F *ug = P.u + (P.u_off ? P.u_off[batch] : 0);
-        // interior tiles of the fused sweep take the vectorised, double-buffered product
-        const bool fast = MODE == BAND_TILE && i0 + BT <= m && j0 + BT <= n && m % 4 == 0 && n % 4 == 0 &&
+        // interior tiles take the vectorised, double-buffered product
+        const bool fast = i0 + BT <= m && j0 + BT <= n && m % 4 == 0 && n % 4 == 0 &&
                           ((reinterpret_cast<uintptr_t>(yg) | reinterpret_cast<uintptr_t>(cg) | reinterpret_cast<uintptr_t>(eg) |
                             reinterpret_cast<uintptr_t>(lg) | reinterpret_cast<uintptr_t>(ug)) % (4 * sizeof(F)) == 0);
-        F acc[8][8];
-        if (dk_lo < dk_hi) {
+        for (int right = 0; right < 2; ++right) {
+            // the right product reads C only on sources of the band, which no CTA of this launch writes
+            const int64_t k_lo = right ? rk_lo : dk_lo, k_hi = right ? rk_hi : dk_hi;
+            if (k_lo >= k_hi) continue;
+            F acc[8][8];
 #pragma unroll
             for (int x = 0; x < 8; ++x)
 #pragma unroll
                 for (int y = 0; y < 8; ++y) acc[x][y] = (F)0;
-            if (fast) band_product_fast<F>(acc, lg, m, eg, n, i0, j0, dk_lo, dk_hi, As, Bs);
-            else band_product<F, MODE, true>(acc, lg, m, eg, n, i0, j0, m, n, dk_lo, dk_hi, g, As, Bs);
+            const F *a = right ? cg : lg, *b = right ? ug : eg;
+            const int64_t lda = right ? n : m;
+            if (fast) band_product_fast<F>(acc, a, lda, b, n, i0, j0, k_lo, k_hi, As, Bs);
+            else band_product<F>(acc, a, lda, b, n, i0, j0, m, n, k_lo, k_hi, As, Bs);
+            F *out = right ? yg : cg;
 #pragma unroll
             for (int x = 0; x < 8; ++x) {
                 const int64_t i = i0 + own(ty, x);
 #pragma unroll
                 for (int y = 0; y < 8; ++y) {
                     const int64_t j = j0 + own(tx, y);
-                    if (i < m && j < n) {
-                        const int64_t st = g.stage(i, j);
-                        if (st >= s1 && st < s_end) {
-                            cg[i * n + j] += acc[x][y];
-                            if (P.down_into_y) yg[i * n + j] += acc[x][y];
-                        }
-                    }
-                }
-            }
-        }
-        if (rk_lo < rk_hi) {
-            // reads C only on sources of the band, which no CTA of this launch writes
-#pragma unroll
-            for (int x = 0; x < 8; ++x)
-#pragma unroll
-                for (int y = 0; y < 8; ++y) acc[x][y] = (F)0;
-            if (fast) band_product_fast<F>(acc, cg, n, ug, n, i0, j0, rk_lo, rk_hi, As, Bs);
-            else band_product<F, MODE, false>(acc, cg, n, ug, n, i0, j0, m, n, rk_lo, rk_hi, g, As, Bs);
-#pragma unroll
-            for (int x = 0; x < 8; ++x) {
-                const int64_t i = i0 + own(ty, x);
-#pragma unroll
-                for (int y = 0; y < 8; ++y) {
-                    const int64_t j = j0 + own(tx, y);
-                    if (i < m && j < n) {
-                        const int64_t st = g.stage(i, j);
-                        if (st >= s1 && st < s_end) yg[i * n + j] += acc[x][y];
-                    }
+                    if (i < m && j < n) out[i * n + j] += acc[x][y];
                 }
             }
         }
     }
 }
 
+// Band update with element masks (P x Q super-entries, any stages): the flushes of the stage-by-stage engines.
+//
+// The sources of a target are a window of k that moves with its super-entry column (down) or row (right), so a tile of
+// targets takes the union of its windows and zeros outside each: the wider the tile against the band, the more of the union is
+// zeros.  Bands of few stages therefore use tiles of 16 rows, wide ones tiles of 64; 256 threads, k in chunks staged in
+// shared memory with the next chunk on its way, masks from bounds that a thread computes once for the rows and columns
+// it stages (in place of divisions per element: 1 ms per flush before, 10 to 100 us now at 512 x 2048 under 1 x 32
+// super-entries).  The terms of a sum keep their order, ascending in k, and the down sum is added before the right one.
+constexpr int MTH = 256;
+template <typename F, int BM>
+__global__ void __launch_bounds__(MTH) band_masked_kernel(BandArgs<F> P) {
+    constexpr int CK = sizeof(F) == sizeof(float) ? 32 : 16;  // k per chunk
+    constexpr int NR = BM / 16;                               // rows per thread; 4 columns
+    constexpr int LA = BM * CK / MTH, LB = 64 * CK / MTH;     // elements of A and B staged per thread
+    constexpr int ALD = BM + 1, BLD2 = 64 + 4;
+    __shared__ __align__(16) F As[2][CK * ALD];
+    __shared__ __align__(16) F Bs[2][CK * BLD2];
+    const int tid = threadIdx.x, ty = tid >> 4, tx = tid & 15;
+    const int64_t m = P.m, n = P.n;
+    const int64_t i0 = (int64_t)blockIdx.y * BM, i1 = min(i0 + BM, m) - 1;
+    for (int64_t batch = blockIdx.z; batch < P.batch; batch += gridDim.z) {
+        const int64_t behind = P.skew != nullptr ? P.skew[batch] : 0;
+        const int64_t s0 = P.s0 - behind, s1 = P.s1 - behind, s_end = P.s_end - behind;
+        // tile columns that can hold targets of these rows start at column block s1 - (last row block)
+        const int64_t first = max((int64_t)0, s1 - i1 / P.P) * P.Q / 64;
+        const int64_t j0 = (first + blockIdx.x) * 64, j1 = min(j0 + 64, n) - 1;
+        if (j0 >= n || i0 / P.P + j0 / P.Q >= s_end || i1 / P.P + j1 / P.Q < s1) continue;
+        F *yg = P.y + batch * m * n, *cg = P.c + batch * m * n;
+        const F *eg = P.e + batch * m * n;
+        const F *lg = P.l + (P.l_off ? P.l_off[batch] : 0);
+        const F *ug = P.u + (P.u_off ? P.u_off[batch] : 0);
+        bool target[NR][4];
+#pragma unroll
+        for (int r = 0; r < NR; ++r)
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                const int64_t i = i0 + ty * NR + r, j = j0 + tx * 4 + c, st = i / P.P + j / P.Q;
+                target[r][c] = i < m && j < n && st >= s1 && st < s_end;
+            }
+        for (int right = 0; right < 2; ++right) {
+            // union of the windows; sources lie in super-entry rows above / columns left of the targets
+            const int64_t near_hi = right ? (s1 - i0 / P.P) * P.Q : (s1 - j0 / P.Q) * P.P, far_lo = right ? (s0 - i1 / P.P) * P.Q : (s0 - j1 / P.Q) * P.P;
+            const int64_t k_lo = max(far_lo, (int64_t)0), k_hi = right ? min(min(near_hi, n), j1 / P.Q * P.Q) : min(min(near_hi, m), i1 / P.P * P.P);
+            if (k_lo >= k_hi) continue;
+            // bounds of k for the rows of A and the columns of B that this thread stages
+            int64_t a_lo[LA], a_hi[LA], b_lo, b_hi;
+            const F *pa[LA];
+#pragma unroll
+            for (int t = 0; t < LA; ++t) {
+                const int64_t i = i0 + (t * MTH + tid) / CK;
+                pa[t] = right ? cg + i * n : lg + i * m;
+                a_lo[t] = right ? (s0 - i / P.P) * P.Q : 0;
+                a_hi[t] = i >= m ? 0 : right ? (s1 - i / P.P) * P.Q : i / P.P * P.P;
+            }
+            const int64_t jb = j0 + (tid & 63);
+            b_lo = right ? 0 : (s0 - jb / P.Q) * P.P;
+            b_hi = jb >= n ? 0 : right ? jb / P.Q * P.Q : (s1 - jb / P.Q) * P.P;
+            const F *pb = (right ? ug : eg) + jb;
+            F ra[LA], rb[LB];
+            auto fetch = [&](int64_t k0) {
+#pragma unroll
+                for (int t = 0; t < LA; ++t) {
+                    const int64_t k = k0 + (tid & (CK - 1));
+                    ra[t] = k < k_hi && k >= a_lo[t] && k < a_hi[t] ? pa[t][k] : (F)0;
+                }
+#pragma unroll
+                for (int t = 0; t < LB; ++t) {
+                    const int64_t k = k0 + t * (MTH / 64) + (tid >> 6);
+                    rb[t] = k < k_hi && k >= b_lo && k < b_hi ? pb[k * n] : (F)0;
+                }
+            };
+            auto stash = [&](int buf) {
+#pragma unroll
+                for (int t = 0; t < LA; ++t) As[buf][(tid & (CK - 1)) * ALD + (t * MTH + tid) / CK] = ra[t];
+#pragma unroll
+                for (int t = 0; t < LB; ++t) Bs[buf][(t * (MTH / 64) + (tid >> 6)) * BLD2 + (tid & 63)] = rb[t];
+            };
+            F acc[NR][4];
+#pragma unroll
+            for (int r = 0; r < NR; ++r)
+#pragma unroll
+                for (int c = 0; c < 4; ++c) acc[r][c] = (F)0;
+            fetch(k_lo);
+            stash(0);
+            __syncthreads();
+            int buf = 0;
+            for (int64_t k0 = k_lo; k0 < k_hi; k0 += CK) {
+                const bool more = k0 + CK < k_hi;
+                if (more) fetch(k0 + CK);
+#pragma unroll
+                for (int kk = 0; kk < CK; ++kk) {
+                    F av[NR], bv[4];
+#pragma unroll
+                    for (int r = 0; r < NR; ++r) av[r] = As[buf][kk * ALD + ty * NR + r];
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) bv[c] = Bs[buf][kk * BLD2 + tx * 4 + c];
+#pragma unroll
+                    for (int r = 0; r < NR; ++r)
+#pragma unroll
+                        for (int c = 0; c < 4; ++c) acc[r][c] += av[r] * bv[c];
+                }
+                if (more) stash(buf ^ 1);
+                __syncthreads();
+                buf ^= 1;
+            }
+#pragma unroll
+            for (int r = 0; r < NR; ++r)
+#pragma unroll
+                for (int c = 0; c < 4; ++c)
+                    if (target[r][c]) {
+                        const int64_t at = (i0 + ty * NR + r) * n + j0 + tx * 4 + c;
+                        if (!right) cg[at] += acc[r][c];
+                        if (right || P.down_into_y) yg[at] += acc[r][c];
+                    }
+        }
+    }
+}
+
 template <typename F>
 int launch_band_update(const BandArgs<F> &args, cudaStream_t stream) {
-    const int nTI = (int)ceil_div(args.m, BT), nTJ = (int)ceil_div(args.n, BT);
-    int a_lo = 0, a_hi = nTI + nTJ - 2;  // target tile anti-diagonals (inclusive)
+    const unsigned batches = (unsigned)(args.batch < 65535 ? args.batch : 65535);
     if (args.mode == BAND_TILE) {
-        a_lo = (int)args.s1;
-        a_hi = (int)args.s_end - 1;
-    } else if (args.mode == BAND_PLAIN) {
-        // a tile on anti-diagonal A holds the entry stages 64 A .. 64 A + 126
-        const int64_t lo = (args.s1 - 2 * (BT - 1)) / BT;
-        a_lo = (int)(lo > 0 ? lo : 0);
-        const int64_t hi = (args.s_end - 1) / BT;
-        a_hi = (int)(hi < a_hi ? hi : a_hi);
+        const int nTI = (int)ceil_div(args.m, BT), nTJ = (int)ceil_div(args.n, BT);
+        if (args.s_end <= args.s1) return G2D_OK;
+        dim3 grid((unsigned)(nTI < nTJ ? nTI : nTJ), (unsigned)(args.s_end - args.s1), batches);
+        band_update_kernel<F><<<grid, BTH, 0, stream>>>(args, nTI, nTJ, (int)args.s1);
+        return check_launch();
     }
-    if (a_hi < a_lo) return G2D_OK;
-    const int max_len = nTI < nTJ ? nTI : nTJ;
-    dim3 grid((unsigned)max_len, (unsigned)(a_hi - a_lo + 1), (unsigned)(args.batch < 65535 ? args.batch : 65535));
-    switch (args.mode) {
-    case BAND_TILE: band_update_kernel<F, BAND_TILE><<<grid, BTH, 0, stream>>>(args, nTI, nTJ, a_lo); break;
-    case BAND_PLAIN: band_update_kernel<F, BAND_PLAIN><<<grid, BTH, 0, stream>>>(args, nTI, nTJ, a_lo); break;
-    default: band_update_kernel<F, BAND_GENERAL><<<grid, BTH, 0, stream>>>(args, nTI, nTJ, a_lo); break;
-    }
+    // 64-row tiles when the band's windows are at least as wide as what a tile of that many rows adds to them
+    BandArgs<F> a = args;
+    if (a.mode == BAND_PLAIN) a.P = a.Q = 1;
+    const int BM = (a.s1 - a.s0) * a.P >= 64 || a.m > 16 * 65535 ? 64 : 16;
+    int64_t across = ceil_div((a.s_end - a.s1 + BM / a.P + 2) * a.Q, 64) + 2;  // tile columns that the targets of a tile row can touch
+    const int64_t all = ceil_div(a.n, 64), down = ceil_div(a.m, BM);
+    if (across > all) across = all;
+    if (down > 65535) return G2D_ERR_TOO_LARGE;
+    dim3 grid((unsigned)across, (unsigned)down, batches);
+    if (BM == 64) band_masked_kernel<F, 64><<<grid, MTH, 0, stream>>>(a);
+    else band_masked_kernel<F, 16><<<grid, MTH, 0, stream>>>(a);
     return check_launch();
 }
 

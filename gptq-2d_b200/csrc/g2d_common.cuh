@@ -7,6 +7,7 @@
 #include <stdint.h>
 
 #include <atomic>
+#include <functional>
 #include <mutex>
 
 #include "../../include/gptq2d_b200.h"
@@ -90,6 +91,15 @@ __device__ __forceinline__ float rounding_reciprocal(float s) {
 __device__ __forceinline__ double rounding_reciprocal(double s) { return __drcp_rn(s); }
 __device__ __forceinline__ bool reciprocal_is_safe(float s) { return fabsf(s) > 1e-18f && fabsf(s) < 1e18f; }
 __device__ __forceinline__ bool reciprocal_is_safe(double s) { return fabs(s) > 1e-150 && fabs(s) < 1e150; }
+
+// Largest value over a warp, in every lane.  Non-negative floats order like their bit patterns, so float takes one reduction
+// instruction; NaN counts as the smallest, as fmax has it.
+__device__ __forceinline__ float warp_max(float v) { return __uint_as_float(__reduce_max_sync(0xffffffffu, v == v ? __float_as_uint(v) : 0u)); }
+__device__ __forceinline__ double warp_max(double v) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
+    return v;
+}
 
 // float -> fp16 / bf16 -> float, round to nearest even (denormals kept).
 __device__ __forceinline__ float round_to_half(float f, int half_kind) {
@@ -272,10 +282,34 @@ struct BandArgs {
 template <typename F>
 int launch_band_update(const BandArgs<F> &args, cudaStream_t stream);
 
+// Feedback between tiles of TR x TC entries (see g2d_block_update.cu): sources the tile anti-diagonals s0..s1-1, targets
+// t0..t1-1 (t0 >= s1); `y` and `c` receive the sums, `c_from` holds the completed C of the sources.
+template <typename F>
+struct BlockUpdateArgs {
+    F *y, *c;
+    const F *e, *c_from, *l, *u;
+    const int64_t *l_off, *u_off;
+    int64_t batch, m, n;
+    int TR, TC;
+    int s0, s1, t0, t1;
+};
+template <typename F>
+int launch_block_update(const BlockUpdateArgs<F> &args, cudaStream_t stream);
+
+// Overlapped schedule: tile launches on the critical path, everything else beside them (see g2d_api.cu).
+// tiles(s, stream) sweeps tile anti-diagonal s; update(s0, s1, t0, t1, far, stream) carries the sources s0..s1-1 into the
+// targets t0..t1-1, into the far planes or into Y and C.  `pushes`: a tile hands the feedback for its two neighbours on itself.
+typedef std::function<int(int, cudaStream_t)> TileLauncher;
+typedef std::function<int(int, int, int, int, bool, cudaStream_t)> UpdateLauncher;
+int sweep_overlapped(int waves, bool pushes, cudaStream_t caller, const TileLauncher &tiles, const UpdateLauncher &update);
+
 // skew (device, one int per batch, may be null): batch b works at stage s - skew[b] (slabs of an N-factor sweep);
 // z_stride: values of z per batch (0: exactly the stage's d p q)
 template <typename F>
 int launch_stage_push(const g2d_stage_desc &d, const F *z, int64_t s, int64_t s1, cudaStream_t stream, const int32_t *skew = nullptr,
                       int64_t z_stride = 0);
+// Its first half alone: errors, completed C and rounded values of stage s.
+template <typename F>
+int launch_stage_commit(const g2d_stage_desc &d, const F *z, int64_t s, cudaStream_t stream, const int32_t *skew = nullptr, int64_t z_stride = 0);
 
 }  // namespace g2d

@@ -106,7 +106,7 @@ __global__ void stage_push_kernel(StageArgs<F> A) {
 }
 
 template <typename F>
-int launch_stage_push(const g2d_stage_desc &d, const F *z, int64_t s, int64_t s1, cudaStream_t stream, const int32_t *skew, int64_t z_stride) {
+static StageArgs<F> stage_args(const g2d_stage_desc &d, const F *z, int64_t s, int64_t s1, const int32_t *skew, int64_t z_stride) {
     StageArgs<F> A;
     A.skew = skew; A.z_stride = z_stride;
     A.y = (F *)d.y; A.c = (F *)d.c; A.e = (F *)d.e;
@@ -114,20 +114,30 @@ int launch_stage_push(const g2d_stage_desc &d, const F *z, int64_t s, int64_t s1
     A.l_off = d.l_offsets; A.u_off = d.u_offsets;
     A.batch = d.batch; A.m = d.m; A.n = d.n; A.s = s; A.s1 = s1;
     A.p = d.p; A.q = d.q;
+    return A;
+}
+
+template <typename F>
+int launch_stage_commit(const g2d_stage_desc &d, const F *z, int64_t s, cudaStream_t stream, const int32_t *skew, int64_t z_stride) {
+    const int64_t mbar = d.m / d.p, nbar = d.n / d.q;
+    const int64_t i_lo = s - nbar + 1 > 0 ? s - nbar + 1 : 0, i_hi = s + 1 < mbar ? s + 1 : mbar;
+    const int64_t total = skew != nullptr ? z_stride * d.batch : (i_hi - i_lo) * d.p * d.q * d.batch;
+    if (total <= 0) return G2D_OK;
+    const int threads = 128;
+    int64_t blocks = ceil_div(total, threads);
+    if (blocks > 65535 * 16) blocks = 65535 * 16;
+    stage_error_kernel<F><<<(unsigned)blocks, threads, 0, stream>>>(stage_args<F>(d, z, s, s + 1, skew, z_stride));
+    return check_launch();
+}
+
+template <typename F>
+int launch_stage_push(const g2d_stage_desc &d, const F *z, int64_t s, int64_t s1, cudaStream_t stream, const int32_t *skew, int64_t z_stride) {
     const int64_t mbar = d.m / d.p, nbar = d.n / d.q, stages = mbar + nbar - 1;
     if (skew == nullptr && (s < 0 || s >= stages)) return G2D_ERR_BAD_ARGUMENT;
     if (s1 <= s) return G2D_ERR_BAD_ARGUMENT;
     if (skew == nullptr && s1 > stages) s1 = stages;
-    const int64_t i_lo = s - nbar + 1 > 0 ? s - nbar + 1 : 0, i_hi = s + 1 < mbar ? s + 1 : mbar;
-    const int64_t total = skew != nullptr ? z_stride * d.batch : (i_hi - i_lo) * d.p * d.q * d.batch;
-    if (total <= 0) return G2D_OK;
-    {
-        const int threads = 128;
-        int64_t blocks = ceil_div(total, threads);
-        if (blocks > 65535 * 16) blocks = 65535 * 16;
-        stage_error_kernel<F><<<(unsigned)blocks, threads, 0, stream>>>(A);
-        if (check_launch() != G2D_OK) return G2D_ERR_CUDA;
-    }
+    const int status = launch_stage_commit<F>(d, z, s, stream, skew, z_stride);
+    if (status != G2D_OK) return status;
     const int64_t pushes = s1 - s - 1;
     if (pushes > 0) {
         const int64_t lanes = mbar < nbar ? mbar : nbar;
@@ -136,12 +146,14 @@ int launch_stage_push(const g2d_stage_desc &d, const F *z, int64_t s, int64_t s1
         if (bx > 4096) bx = 4096;
         dim3 grid((unsigned)bx, (unsigned)pushes, (unsigned)(d.batch < 65535 ? d.batch : 65535));
         if (pushes > 65535) return G2D_ERR_TOO_LARGE;
-        stage_push_kernel<F><<<grid, threads, 0, stream>>>(A);
+        stage_push_kernel<F><<<grid, threads, 0, stream>>>(stage_args<F>(d, z, s, s1, skew, z_stride));
         if (check_launch() != G2D_OK) return G2D_ERR_CUDA;
     }
     return G2D_OK;
 }
 
+template int launch_stage_commit<float>(const g2d_stage_desc &, const float *, int64_t, cudaStream_t, const int32_t *, int64_t);
+template int launch_stage_commit<double>(const g2d_stage_desc &, const double *, int64_t, cudaStream_t, const int32_t *, int64_t);
 template int launch_stage_push<float>(const g2d_stage_desc &, const float *, int64_t, int64_t, cudaStream_t, const int32_t *, int64_t);
 template int launch_stage_push<double>(const g2d_stage_desc &, const double *, int64_t, int64_t, cudaStream_t, const int32_t *, int64_t);
 

@@ -46,6 +46,10 @@ struct SuperArgs {
     F *xs, *row_scale;                 // trellis: gathered sequences and their scales
     LeadModes lead;
     F *fold;                           // lead.count planes [batch, m, n]
+    F *c, *e;
+    const F *l, *u;
+    const int64_t *l_off, *u_off;
+    int64_t s0;                        // first stage of the inner block: pushes of the stages s0 .. stage - 1 are pending
 };
 
 // Entry (k, a, b) of the stage of `batch`: false when the batch has no such entry at this global stage.
@@ -169,6 +173,161 @@ __global__ void quantize_absmax_kernel(SuperArgs<F> A) {
     }
 }
 
+constexpr int PTH = 256;       // threads of a CTA of the pull kernel
+constexpr int PULL_ROOM = 2048;  // (source stage, entry) pairs whose sums wait in shared memory
+constexpr int Q_PULL_ONLY = -1;  // KIND: only bring Y and C up to date
+
+// One CTA per super-entry of the stage: first what the earlier stages of the inner block owe it, then its quantizer, then its
+// error, completed C and rounded values.  One launch per stage where the sources used to push (error, push and quantizer
+// kernels, 3 launches), because a super-entry that fetches its own feedback when its turn comes needs no launch for it.
+// Bound by launch latency and the chain of one stage: the sums of all source stages are formed side by side, each in the
+// order and from the start that the push had, and added in the order of the stages, so the values are bit for bit the same.
+// Stage kernels follow each other with programmatic dependent launch: a CTA of the next stage is resident when this one ends.
+template <typename F, int KIND>
+__global__ void __launch_bounds__(PTH) stage_pull_kernel(SuperArgs<F> A) {
+    __shared__ F down_s[PULL_ROOM], right_s[PULL_ROOM];
+    asm volatile("griddepcontrol.launch_dependents;");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    const int p = A.p, q = A.q, pq = p * q;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int64_t m = A.m, n = A.n;
+    for (int64_t batch = blockIdx.y; batch < A.batch; batch += gridDim.y) {
+        int64_t i0, j0;
+        if (!locate(A, batch, (int64_t)blockIdx.x, 0, 0, i0, j0)) continue;
+        F *yg = A.y + batch * m * n, *cg = A.c + batch * m * n, *eg = A.e + batch * m * n;
+        const F *lg = A.l + (A.l_off ? A.l_off[batch] : 0), *ug = A.u + (A.u_off ? A.u_off[batch] : 0);
+        const int64_t ib = i0 / p, jb = j0 / q;
+        const int pulls = (int)min(A.stage - A.s0, max(ib, jb));  // source stages, dd = pulls .. 1 before this one
+        const int64_t seq = batch * A.dmax + blockIdx.x;
+        auto sums = [&](int dd, int a, int b, F &down, F &right) {
+            const int64_t i = i0 + a, j = j0 + b;
+            down = right = (F)0;
+            if (ib - dd >= 0) {
+                const F *lp = lg + i * m + (ib - dd) * p, *ep = eg + (ib - dd) * p * n + j;
+#pragma unroll 4
+                for (int x = 0; x < p; ++x) down += lp[x] * ep[x * n];
+            }
+            if (jb - dd >= 0) {
+                const F *cp = cg + i * n + (jb - dd) * q, *up = ug + (jb - dd) * q * n + j;
+#pragma unroll 8
+                for (int x = 0; x < q; ++x) right += cp[x] * up[x * n];
+            }
+        };
+        const bool staged = (int64_t)pulls * pq <= PULL_ROOM;
+        if (staged) {
+            for (int t = tid; t < pulls * pq; t += PTH) {
+                const int at = t % pq;
+                sums(pulls - t / pq, at / q, at % q, down_s[t], right_s[t]);
+            }
+            __syncthreads();
+        }
+        // a warp per row of the super-entry
+        for (int a = warp; a < p; a += PTH / 32) {
+            constexpr int KEEP = 4;  // values of a row that stay in a lane's registers
+            F yv[KEEP], cv[KEEP], top = (F)0;
+            auto update = [&](int b, F &y, F &c) {  // entry (a, b) with all pending feedback
+                const int64_t at = (i0 + a) * n + j0 + b;
+                y = yg[at];
+                c = cg[at];
+                for (int x = 0; x < pulls; ++x) {
+                    const int dd = pulls - x;
+                    F down, right;
+                    if (staged) {
+                        down = down_s[x * pq + a * q + b];
+                        right = right_s[x * pq + a * q + b];
+                    } else {
+                        sums(dd, a, b, down, right);
+                    }
+                    if (ib - dd >= 0) c += down;
+                    if (ib - dd >= 0 || jb - dd >= 0) y += down + right;
+                }
+            };
+            auto finish = [&](int b, F y, F c, F s) {
+                const int64_t i = i0 + a, j = j0 + b, at = i * n + j;
+                if (KIND == Q_PULL_ONLY) {
+                    yg[at] = y;
+                    cg[at] = c;
+                } else if (KIND == G2D_Q_TRELLIS) {
+                    yg[at] = y;
+                    cg[at] = c;
+                    A.xs[seq * pq + a * q + b] = div_rn(y, s);
+                } else {
+                    F z;
+                    if (KIND == G2D_Q_ROUND) {
+                        z = rint_even(y);
+                    } else if (KIND == G2D_Q_AFFINE) {
+                        const F sc = A.scale[(A.scale_off ? A.scale_off[batch] : 0) + i * A.srs + j * A.scs];
+                        const F zp = A.zero[(A.zero_off ? A.zero_off[batch] : 0) + i * A.zrs + j * A.zcs];
+                        z = affine_value(y, sc, zp, A.qmin, A.qmax);
+                    } else {
+                        F t = rint_even(div_rn(y, s));
+                        t = t < A.qmin ? A.qmin : t;
+                        t = t > A.qmax ? A.qmax : t;
+                        z = mul_rn(t, s);
+                    }
+                    const F ev = z - y;
+                    eg[at] = ev;
+                    cg[at] = c + ev;
+                    yg[at] = z;
+                }
+            };
+            F s = (F)1;
+            if (KIND == G2D_Q_TRELLIS) {
+                s = A.scale[A.scale_off ? A.scale_off[batch] : 0];
+                if (a == 0 && lane == 0) A.row_scale[seq] = s;
+            }
+            if (KIND == G2D_Q_ABSMAX_DYNAMIC && q <= 32 * KEEP) {
+#pragma unroll
+                for (int x = 0; x < KEEP; ++x)
+                    if (lane + 32 * x < q) {
+                        update(lane + 32 * x, yv[x], cv[x]);
+                        top = fmax(top, fabs(yv[x]));
+                    }
+                s = absmax_scale_value(warp_max(top), A.divisor, A.half);
+#pragma unroll
+                for (int x = 0; x < KEEP; ++x)
+                    if (lane + 32 * x < q) finish(lane + 32 * x, yv[x], cv[x], s);
+            } else if (KIND == G2D_Q_ABSMAX_DYNAMIC) {
+                for (int b = lane; b < q; b += 32) {
+                    const int64_t at = (i0 + a) * n + j0 + b;
+                    F y, c;
+                    update(b, y, c);
+                    yg[at] = y;
+                    cg[at] = c;
+                    top = fmax(top, fabs(y));
+                }
+                s = absmax_scale_value(warp_max(top), A.divisor, A.half);
+                for (int b = lane; b < q; b += 32) {
+                    const int64_t at = (i0 + a) * n + j0 + b;
+                    finish(b, yg[at], cg[at], s);  // this lane's own stores
+                }
+            } else {
+                for (int b = lane; b < q; b += 32) {
+                    F y, c;
+                    update(b, y, c);
+                    finish(b, y, c, s);
+                }
+            }
+        }
+        __syncthreads();  // the next batch reuses the staged sums
+    }
+}
+
+template <typename F, int KIND>
+int launch_stage_pull(const SuperArgs<F> &A, cudaStream_t st) {
+    cudaLaunchConfig_t config{};
+    config.gridDim = dim3((unsigned)A.dmax, (unsigned)(A.batch < 65535 ? A.batch : 65535));
+    config.blockDim = dim3(PTH);
+    config.stream = st;
+    cudaLaunchAttribute attribute{};
+    attribute.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attribute.val.programmaticStreamSerializationAllowed = 1;
+    config.attrs = &attribute;
+    config.numAttrs = 1;
+    if (cudaLaunchKernelEx(&config, stage_pull_kernel<F, KIND>, A) != cudaSuccess) return G2D_ERR_CUDA;
+    return check_launch();
+}
+
 // Packed trellis paths of one stage into the matrix-level array [batch, m / p, n / q, bytes].
 template <typename F>
 __global__ void scatter_codes_kernel(SuperArgs<F> A, const uint8_t *__restrict__ stage_codes, uint8_t *__restrict__ codes, int64_t bytes) {
@@ -275,6 +434,8 @@ int sweep_super(const g2d_super_desc *d, const Plan &plan, cudaStream_t st) {
     A.batch = d->batch; A.m = d->m; A.n = d->n; A.p = d->p; A.q = d->q;
     A.xs = (F *)(ws + plan.xs); A.row_scale = (F *)(ws + plan.row_scale);
     A.fold = (F *)(ws + plan.fold);
+    A.c = c; A.e = e;
+    A.l = (const F *)d->l; A.u = (const F *)d->u; A.l_off = d->l_offsets; A.u_off = d->u_offsets;
     A.lead.count = d->lead_count;
     int64_t stride = d->batch;
     for (int k = 0; k < d->lead_count; ++k) {
@@ -321,19 +482,32 @@ int sweep_super(const g2d_super_desc *d, const Plan &plan, cudaStream_t st) {
                 int64_t dmax = 0;
                 for (int64_t behind = 0; behind <= plan.lead_total; ++behind) dmax = on_stage(s - behind) > dmax ? on_stage(s - behind) : dmax;
                 if (dmax == 0) continue;
-                A.stage = s; A.dmax = dmax;
+                A.stage = s; A.dmax = dmax; A.s0 = s0;
                 const int64_t work = d->batch * dmax * pq;
-                if (d->lead_count > 0) {
+                if (d->lead_count == 0) {
+                    int status;
+                    switch (d->quant_kind) {
+                    case G2D_Q_ROUND: status = launch_stage_pull<F, G2D_Q_ROUND>(A, st); break;
+                    case G2D_Q_AFFINE: status = launch_stage_pull<F, G2D_Q_AFFINE>(A, st); break;
+                    case G2D_Q_ABSMAX_DYNAMIC: status = launch_stage_pull<F, G2D_Q_ABSMAX_DYNAMIC>(A, st); break;
+                    default: status = launch_stage_pull<F, G2D_Q_TRELLIS>(A, st); break;
+                    }
+                    if (status != G2D_OK) return status;
+                    if (d->quant_kind != G2D_Q_TRELLIS) continue;
+                } else {
+                    // the leading modes' feedback comes between the pending pushes and the quantizer
+                    const int status = launch_stage_pull<F, Q_PULL_ONLY>(A, st);
+                    if (status != G2D_OK) return status;
                     fold_kernel<F><<<blocks_for(work, 128), 128, 0, st>>>(A);
                     if (check_launch() != G2D_OK) return G2D_ERR_CUDA;
+                    switch (d->quant_kind) {
+                    case G2D_Q_ROUND: quantize_entries_kernel<F, G2D_Q_ROUND><<<blocks_for(work, 128), 128, 0, st>>>(A); break;
+                    case G2D_Q_AFFINE: quantize_entries_kernel<F, G2D_Q_AFFINE><<<blocks_for(work, 128), 128, 0, st>>>(A); break;
+                    case G2D_Q_ABSMAX_DYNAMIC: quantize_absmax_kernel<F><<<blocks_for(d->batch * dmax * d->p * 32, 128), 128, 0, st>>>(A); break;
+                    default: quantize_entries_kernel<F, G2D_Q_TRELLIS><<<blocks_for(work, 128), 128, 0, st>>>(A); break;
+                    }
+                    if (check_launch() != G2D_OK) return G2D_ERR_CUDA;
                 }
-                switch (d->quant_kind) {
-                case G2D_Q_ROUND: quantize_entries_kernel<F, G2D_Q_ROUND><<<blocks_for(work, 128), 128, 0, st>>>(A); break;
-                case G2D_Q_AFFINE: quantize_entries_kernel<F, G2D_Q_AFFINE><<<blocks_for(work, 128), 128, 0, st>>>(A); break;
-                case G2D_Q_ABSMAX_DYNAMIC: quantize_absmax_kernel<F><<<blocks_for(d->batch * dmax * d->p * 32, 128), 128, 0, st>>>(A); break;
-                default: quantize_entries_kernel<F, G2D_Q_TRELLIS><<<blocks_for(work, 128), 128, 0, st>>>(A); break;
-                }
-                if (check_launch() != G2D_OK) return G2D_ERR_CUDA;
                 if (d->quant_kind == G2D_Q_TRELLIS) {
                     uint8_t *stage_codes = d->codes ? (uint8_t *)(ws + plan.stage_codes) : nullptr;
                     const TrellisIndex index{d->table_distinct, d->table_ids, d->table_distinct_count};
@@ -350,7 +524,7 @@ int sweep_super(const g2d_super_desc *d, const Plan &plan, cudaStream_t st) {
                     fold_commit_kernel<F><<<blocks_for(work, 128), 128, 0, st>>>(A);
                     if (check_launch() != G2D_OK) return G2D_ERR_CUDA;
                 }
-                const int status = launch_stage_push<F>(sd, z, s, s1, st, skew, dmax * pq);
+                const int status = launch_stage_commit<F>(sd, z, s, st, skew, dmax * pq);
                 if (status != G2D_OK) return status;
             }
             if (s1 < outer_stop) {
