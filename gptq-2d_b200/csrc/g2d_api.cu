@@ -369,12 +369,118 @@ int sweep_pipelined(const g2d_sweep_desc *d, SweepArgs<float> &a, const TcPlanes
     return G2D_OK;
 }
 
+}  // namespace
+
+// Tile anti-diagonal s waits for the updates whose targets it holds and for nothing else:
+//   * into its next anti-diagonal, where the tiles do not push themselves: a launch of its own between the two tile launches;
+//   * from s + 2 up to where the far update of the group of s starts: on a second stream, beside the tile launch of s + 1;
+//   * into everything beyond, once per group of kGroup anti-diagonals, on a third stream and into planes of its own, which a
+//     tile adds when it loads: first the anti-diagonals that come up before the next group's update, then the rest.
+// Updates that share targets and planes follow each other on one stream, so the additions have a fixed order.  Inside a
+// stream capture that finds no lanes (the first call on a device), everything runs in order on the caller's stream.
+int g2d::sweep_overlapped(int waves, bool pushes, cudaStream_t caller, const TileLauncher &tiles, const UpdateLauncher &update) {
+    constexpr int kGroup = 8, kLag = 2;
+    std::unique_lock<std::mutex> held;
+    int status = G2D_OK;
+    PipeLane *lane = waves > 2 ? acquire_pipe_lane(caller, held, &status) : nullptr;
+    if (!lane && status != G2D_OK && status != G2D_ERR_UNSUPPORTED) return status;
+    cudaStream_t main = lane ? lane->tiles : caller, side = lane ? lane->near : caller, far = lane ? lane->far : caller;
+    bool ok = true;
+    auto record = [&](cudaEvent_t e, cudaStream_t st) { if (lane) ok = ok && cudaEventRecord(e, st) == cudaSuccess; };
+    auto wait = [&](cudaStream_t st, cudaEvent_t e) { if (lane) ok = ok && cudaStreamWaitEvent(st, e, 0) == cudaSuccess; };
+    static cudaEvent_t none = nullptr;
+    auto event = [&](cudaEvent_t *list, int k) { return lane ? list[k] : none; };
+    if (lane) {
+        record(lane->fork, caller);
+        wait(main, lane->fork);
+    }
+    int last_side = -1, last_far = -1;
+    for (int s = 0; s < waves && ok; ++s) {
+        if (s >= 2 && last_side >= s - 2) wait(main, event(lane ? lane->near_done : nullptr, (s - 2) & 7));
+        if (s >= kGroup + kLag && (s - kLag) % kGroup == 0) {
+            const int g = (s - kLag) / kGroup - 1;
+            if (last_far >= g) wait(main, event(lane ? lane->far_first : nullptr, g & 3));
+            if (g >= 1 && last_far >= g - 1) wait(main, event(lane ? lane->far_done : nullptr, (g - 1) & 3));
+        }
+        status = tiles(s, main);
+        if (status != G2D_OK) return status;
+        const int group_end = (s / kGroup + 1) * kGroup, reach = group_end + kLag;  // the far update of s's group starts at `reach`
+        const bool feeds_side = s + 2 < waves, feeds_far = s + 1 == group_end && reach < waves;
+        if (feeds_side || feeds_far) record(event(lane ? lane->swept : nullptr, s & 7), main);
+        if (!pushes && s + 1 < waves) {
+            // shares its targets with the side update of s - 1
+            if (s >= 1 && last_side >= s - 1) wait(main, event(lane ? lane->near_done : nullptr, (s - 1) & 7));
+            status = update(s, s + 1, s + 1, s + 2, false, main);
+            if (status != G2D_OK) return status;
+        }
+        if (feeds_side) {
+            wait(side, event(lane ? lane->swept : nullptr, s & 7));
+            status = update(s, s + 1, s + 2, reach < waves ? reach : waves, false, side);
+            if (status != G2D_OK) return status;
+            record(event(lane ? lane->near_done : nullptr, s & 7), side);
+            last_side = s;
+        }
+        if (feeds_far) {
+            const int g = s / kGroup, split = reach + kGroup < waves ? reach + kGroup : waves;
+            wait(far, event(lane ? lane->swept : nullptr, s & 7));
+            status = update(group_end - kGroup, group_end, reach, split, true, far);
+            if (status != G2D_OK) return status;
+            record(event(lane ? lane->far_first : nullptr, g & 3), far);
+            if (split < waves) status = update(group_end - kGroup, group_end, split, waves, true, far);
+            if (status != G2D_OK) return status;
+            record(event(lane ? lane->far_done : nullptr, g & 3), far);
+            last_far = g;
+        }
+    }
+    if (lane) {
+        if (last_side >= 0) wait(main, lane->near_done[last_side & 7]);
+        if (last_far >= 0) wait(main, lane->far_done[last_far & 3]);
+        record(lane->join, main);
+        wait(caller, lane->join);
+    }
+    return ok ? G2D_OK : G2D_ERR_CUDA;
+}
+
+namespace {
+
+// Floats beyond C and E that the overlapped schedule keeps: the far planes, and for float the planes of the neighbour push.
+template <typename F>
+constexpr int overlap_planes() { return sizeof(F) == sizeof(float) ? 4 : 2; }
+inline bool overlap_eligible(const g2d_sweep_desc *d) { return d->reserved == 0 && !tc_eligible(d); }
+
+template <typename F>
+int sweep_tiles_overlapped(const g2d_sweep_desc *d, SweepArgs<F> &a, F *planes, size_t plane, cudaStream_t stream, LaunchTimer *timer, double *flops) {
+    auto at = [&](int k) { return (F *)((char *)planes + (size_t)k * plane); };
+    F *yf = at(0), *cf = at(1);
+    if (cudaMemsetAsync(yf, 0, 2 * plane, stream) != cudaSuccess) return G2D_ERR_CUDA;
+    a.yf = yf; a.cf = cf;
+    if (sizeof(F) == sizeof(float)) { a.yn = at(2); a.cn = at(3); }  // written before they are read
+    BlockUpdateArgs<F> b;
+    b.e = a.e; b.c_from = a.c; b.l = a.l; b.u = a.u; b.l_off = a.l_off; b.u_off = a.u_off;
+    b.batch = a.batch; b.m = a.m; b.n = a.n; b.TR = TILE; b.TC = TILE;
+    auto timed = [&](int kind, cudaStream_t st, auto &&launch) {
+        if (timer) timer->begin_on(kind, st);
+        const int status = launch();
+        if (timer) timer->end();
+        return status;
+    };
+    return sweep_overlapped(
+        a.nI + a.nJ - 1, a.yn != nullptr, stream, [&](int s, cudaStream_t st) { return timed(0, st, [&] { return launch_tile_sweep<F>(a, s, st); }); },
+        [&](int s0, int s1, int t0, int t1, bool far, cudaStream_t st) {
+            b.y = far ? yf : a.y; b.c = far ? cf : a.c;
+            b.s0 = s0; b.s1 = s1; b.t0 = t0; b.t1 = t1;
+            if (flops) flops[far ? 2 : 1] += (band_flops(d->m, d->n, s0, s1, t1) - band_flops(d->m, d->n, s0, s1, t0)) * (double)d->batch;
+            return timed(far ? 2 : 1, st, [&] { return launch_block_update<F>(b, st); });
+        });
+}
+
 template <typename F>
 int sweep_fused(const g2d_sweep_desc *d, cudaStream_t stream, LaunchTimer *timer = nullptr, double *flops = nullptr) {
     const int64_t count = d->batch * d->m * d->n;
     const size_t plane = align256(sizeof(F) * (size_t)count);
     const bool tc = tc_eligible(d);
-    if (!d->workspace || d->workspace_bytes < 2 * plane + (tc ? tc_extra_bytes(d) : 0)) return G2D_ERR_WORKSPACE;
+    const size_t extra = tc ? tc_extra_bytes(d) : overlap_eligible(d) ? overlap_planes<F>() * plane : 0;
+    if (!d->workspace || d->workspace_bytes < 2 * plane + extra) return G2D_ERR_WORKSPACE;
     if (((uintptr_t)d->workspace & 255) != 0) return G2D_ERR_WORKSPACE;
     SweepArgs<F> a;
     a.y = (F *)d->y;
@@ -426,6 +532,7 @@ int sweep_fused(const g2d_sweep_desc *d, cudaStream_t stream, LaunchTimer *timer
         return launch_sweep_finish(planes.error_flag, d->status, (float *)d->y, d->m * d->n, stream);
     }
     if (d->reserved == 2) return sweep_macro<F>(d, a, b, stream, timer, flops, nullptr);
+    if (overlap_eligible(d)) return sweep_tiles_overlapped<F>(d, a, (F *)((char *)d->workspace + 2 * plane), plane, stream, timer, flops);
 
     const int waves = a.nI + a.nJ - 1;
     const int outer = d->outer_tiles > 0 ? d->outer_tiles : kDefaultOuterTiles;
@@ -495,8 +602,9 @@ extern "C" int g2d_abi_version(void) { return 2; }
 extern "C" int g2d_sweep_workspace_bytes(const g2d_sweep_desc *desc, size_t *bytes) {
     const int status = check_sweep(desc);
     if (status != G2D_OK || !bytes) return status != G2D_OK ? status : G2D_ERR_BAD_ARGUMENT;
-    const size_t elem = desc->dtype == G2D_F32 ? 4 : 8;
-    *bytes = 2 * align256(elem * (size_t)(desc->batch * desc->m * desc->n)) + (tc_eligible(desc) ? tc_extra_bytes(desc) : 0);
+    const size_t plane = align256((desc->dtype == G2D_F32 ? 4 : 8) * (size_t)(desc->batch * desc->m * desc->n));
+    const int planes = !overlap_eligible(desc) ? 0 : desc->dtype == G2D_F32 ? overlap_planes<float>() : overlap_planes<double>();
+    *bytes = (2 + planes) * plane + (tc_eligible(desc) ? tc_extra_bytes(desc) : 0);
     return G2D_OK;
 }
 

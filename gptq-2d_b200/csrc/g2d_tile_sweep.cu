@@ -173,9 +173,9 @@ __global__ void __launch_bounds__(TTH, 1) tile_sweep_kernel(SweepArgs<F> P, int 
         const F *zg = KIND == G2D_Q_AFFINE ? P.zero + (P.zero_off ? P.zero_off[batch] : 0) : nullptr;
         const F *fg = KIND == G2D_Q_FORCED ? P.forced + batch * m * n : nullptr;
         F *pre = P.y_pre ? P.y_pre + batch * m * n : nullptr;
-        const F *yfg = P.yf, *cfg = P.cf;
+        const F *yfg = P.yf ? P.yf + batch * m * ld : nullptr, *cfg = P.yf ? P.cf + batch * m * ld : nullptr;
         // neighbour push (pipelined schedule): what this tile receives and what it owes
-        F *yng = P.yn, *cng = P.cn;  // these planes exist for a single matrix only
+        F *yng = P.yn ? P.yn + batch * m * ld : nullptr, *cng = P.yn ? P.cn + batch * m * ld : nullptr;
         const bool gets_right = yng != nullptr && J > 0, gets_down = yng != nullptr && I > 0;
         const bool owes_right = yng != nullptr && J + 1 < P.nJ, owes_down = yng != nullptr && I + 1 < P.nI;
 
@@ -677,7 +677,7 @@ __global__ void __launch_bounds__(TTH, 1) tile_sweep_kernel(SweepArgs<F> P, int 
             }
         }
         // ---- store the errors and the completed C of the tile, unless only their operand planes are read from here on ----
-        if (yng != nullptr) {
+        if (P.c_hi != nullptr && yng != nullptr) {
         } else if (vec) {
             for (int idx = tid; idx < TILE * TILE / 4; idx += TTH) {
                 const int r = idx / (TILE / 4), c = (idx % (TILE / 4)) * 4;
