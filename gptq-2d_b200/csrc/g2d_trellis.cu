@@ -450,6 +450,293 @@ __global__ void __launch_bounds__(VT) viterbi_indexed_kernel(int64_t rows, int T
     }
 }
 
+// The search for 2^16 states in float, one sequence per cluster of four CTAs: every thread owns 32 states for good and
+// keeps their table values in registers.
+//
+// A step of the search is 2^16 times (table - x)^2 summed, plus the group minimum of the predecessors, compared: nine
+// operations per state with nothing to load but the minima (one per predecessor and up to 16 groups), 900 cycles on four
+// SMs, against a table read or a look-up of the local cost per state in the kernels above (11 k cycles on one SM, bound by
+// shared memory).  Four CTAs are what it takes to hold 2^16 value pairs in registers, and a coarse stage of a sweep
+// rarely has more sequences than the GPU has clusters of four.  What a step adds is the exchange: the group minimum of
+// g is needed by the CTA that owns the groups (g mod G / H) H .. + H - 1 and goes straight into its shared memory, then the cluster
+// synchronises.  HYB, T = 256, 32 sequences: 1.47 ms before, FIGURE now.
+//
+// Mapping.  G = 2^16 / H groups, Gc = G / 4 per CTA.  A thread has NG neighbouring groups and NH = 32 / NG predecessors of
+// each; with more than 32 predecessors per group, H / 32 neighbouring lanes share a group and settle its minimum by shuffle.
+// The arg-mins of a thread's groups are packed into one unit of one or two bytes per step, kept in shared memory where
+// they fit and in the global scratch otherwise.  The walk back is one warp's: its lanes fetch the units of the next
+// steps for every choice that could lead there (1 + H + H^2 lanes), so that one round of latency settles several steps.
+// Costs, sums and tie rules are those of viterbi_kernel: same values, same states.
+constexpr int CT = 512;  // threads
+constexpr int CCL = 4;   // CTAs per cluster
+constexpr int CSTATES = 32;
+
+__device__ __forceinline__ uint32_t cluster_rank() { uint32_t r; asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r)); return r; }
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ uint32_t remote(const void *p, uint32_t rank) {  // the same variable in another CTA of the cluster
+    uint32_t r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"((uint32_t)__cvta_generic_to_shared(p)), "r"(rank));
+    return r;
+}
+__device__ __forceinline__ void remote_store(uint32_t at, float v) { asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(at), "f"(v) : "memory"); }
+__device__ __forceinline__ void remote_store(uint32_t at, int v) { asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(at), "r"(v) : "memory"); }
+__device__ __forceinline__ uint32_t remote_load_unit(uint32_t at, int bytes) {
+    uint32_t v;
+    if (bytes == 1) asm volatile("ld.shared::cluster.u8 %0, [%1];" : "=r"(v) : "r"(at) : "memory");
+    else asm volatile("ld.shared::cluster.u16 %0, [%1];" : "=r"(v) : "r"(at) : "memory");
+    return v;
+}
+
+template <int V, int LOG_NG>
+__global__ void __launch_bounds__(CT, 1) viterbi_cluster_kernel(int64_t rows, int T, const float *__restrict__ x, const float *__restrict__ table, int shift,
+                                                                int tail_biting, const float *__restrict__ scale, float *__restrict__ out,
+                                                                int64_t *__restrict__ states, uint8_t *__restrict__ scratch, int64_t scratch_row,
+                                                                int choices_in_smem, uint8_t *__restrict__ codes, int64_t code_bytes) {
+    constexpr int NG = 1 << LOG_NG, NH = CSTATES / NG;
+    extern __shared__ __align__(16) unsigned char g2d_vsmem[];
+    const int H = 1 << shift, G = (1 << 16) >> shift, Gc = G / CCL, parts = H / NH;
+    const int steps = T / V, slots = steps > 1 ? steps - 1 : 1;
+    const int PW = Gc >= H ? Gc >> shift : 1;          // minima per predecessor number that this CTA's groups need
+    const int period = G >> shift;                     // G / H
+    const int minima = H * PW;
+    const int units = CT / parts, unit_bytes = NG * shift > 8 ? 2 : 1;
+    float *const prev = reinterpret_cast<float *>(g2d_vsmem);        // [2][H][PW]
+    float *const xs = prev + 2 * minima;                             // [T]
+    int *const path = reinterpret_cast<int *>(xs + T);               // [steps]
+    uint8_t *const kept = reinterpret_cast<uint8_t *>(path + steps); // [slots][units] units
+    __shared__ float red_val[CT / 32];
+    __shared__ int red_arg[CT / 32];
+    __shared__ float all_val[CCL];
+    __shared__ int all_arg[CCL];
+    __shared__ int overlap;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const uint32_t rank = cluster_rank();
+    const int unit = tid / parts, part = tid % parts, gl0 = unit * NG, h0 = part * NH, g0 = (int)rank * Gc + gl0;
+
+    float tv[CSTATES][V];
+#pragma unroll
+    for (int e = 0; e < CSTATES; ++e) {
+        const int s = (h0 + e / NG) * G + g0 + e % NG;
+        if constexpr (V == 2) load_pair(table + 2 * s, tv[e][0], tv[e][1]);
+        else tv[e][0] = table[s];
+    }
+    // where the minima of this thread's groups go: CTA and place by group
+    uint32_t to[NG];
+#pragma unroll
+    for (int q = 0; q < NG; ++q) {
+        const int g = g0 + q, within = g & (period - 1);
+        to[q] = Gc >= H ? remote(prev + (g / period) * PW + (within & (PW - 1)), (uint32_t)(within / PW)) : 0u;
+    }
+    const int64_t clusters = gridDim.x / CCL;
+    for (int64_t row = blockIdx.x / CCL; row < rows; row += clusters) {
+        for (int i = tid; i < T; i += CT) xs[i] = x[row * T + i];
+        if (tid == 0) overlap = -1;
+        uint8_t *const far = scratch + row * scratch_row + (int64_t)rank * units * unit_bytes;  // + slot * CCL * units * unit_bytes
+        __syncthreads();
+        for (int pass = tail_biting ? 0 : 1; pass < 2; ++pass) {
+            const int half = steps / 2, roll = pass == 0 ? steps - half : 0, stop = pass == 0 ? half : 0;
+            const int ov = overlap;
+            // "minima before the first step": nothing, or the tail-biting constraint on the predecessors
+            for (int i = tid; i < minima; i += CT) {
+                const int low = (i / PW) * period + (Gc >= H ? (int)rank * PW + i % PW : 0);
+                prev[minima + i] = ov >= 0 && low != ov ? INFINITY : 0.f;
+            }
+            cluster_sync();  // and every CTA is done with the last pass
+            float best[NG];
+            int arg[NG];
+            for (int t = 0; t < steps; ++t) {
+                const float *const before = prev + ((t + 1) & 1) * minima + h0 * PW + (gl0 >> shift);
+                int at = t + roll;
+                if (at >= steps) at -= steps;
+                const float x0 = xs[at * V], x1 = V == 2 ? xs[at * V + 1] : 0.f;
+#pragma unroll
+                for (int hh = 0; hh < NH; ++hh) {
+                    float pv[NG];
+                    // neighbouring groups share their predecessor's minimum where H >= NG
+#pragma unroll
+                    for (int q = 0; q < NG; ++q) pv[q] = (q == 0 || (q & (NH - 1)) == 0) ? before[hh * PW + (NG > NH ? q / NH : 0)] : pv[q - 1];
+#pragma unroll
+                    for (int q = 0; q < NG; ++q) {
+                        const float d0 = sub_rn(tv[hh * NG + q][0], x0);
+                        float c = mul_rn(d0, d0);
+                        if constexpr (V == 2) {
+                            const float d1 = sub_rn(tv[hh * NG + q][V - 1], x1);
+                            c = add_rn(c, mul_rn(d1, d1));
+                        }
+                        c = add_rn(pv[q], c);
+                        if (hh == 0 || c < best[q]) { best[q] = c; arg[q] = h0 + hh; }
+                    }
+                }
+                if constexpr (NG == 1) {
+                    for (int o = 1; o < parts; o <<= 1) {  // the lanes that share a group: smaller cost, then smaller number
+                        const float ob = __shfl_xor_sync(0xffffffffu, best[0], o);
+                        const int oa = __shfl_xor_sync(0xffffffffu, arg[0], o);
+                        if (ob < best[0] || (ob == best[0] && oa < arg[0])) { best[0] = ob; arg[0] = oa; }
+                    }
+                }
+                if (t + 1 < steps) {
+                    if (part == 0) {
+                        const uint32_t buffer = (uint32_t)((t & 1) * minima * (int)sizeof(float));
+                        uint32_t packed = 0;
+#pragma unroll
+                        for (int q = 0; q < NG; ++q) {
+                            if (Gc >= H) remote_store(to[q] + buffer, best[q]);
+                            else
+                                for (int r = 0; r < CCL; ++r) remote_store(remote(prev + g0 + q, r) + buffer, best[q]);
+                            packed |= (uint32_t)arg[q] << (q * shift);
+                        }
+                        uint8_t *const u = choices_in_smem ? kept + ((size_t)t * units + unit) * unit_bytes : far + ((int64_t)t * CCL * units + unit) * unit_bytes;
+                        if (unit_bytes == 1) *u = (uint8_t)packed;
+                        else *reinterpret_cast<uint16_t *>(u) = (uint16_t)packed;
+                    }
+                    cluster_sync();
+                }
+            }
+            // ---- first arg-min over all states of the last step, with the final mask ----
+            float b = INFINITY;
+            int a = 1 << 16;
+#pragma unroll
+            for (int q = 0; q < NG; ++q) {
+                const float c = ov >= 0 && g0 + q != ov ? INFINITY : best[q];
+                // a masked group offers its first state, as a masked search over its states would
+                const int s = (ov >= 0 && g0 + q != ov ? 0 : arg[q]) * G + g0 + q;
+                if (a == 1 << 16 || c < b || (c == b && s < a)) { b = c; a = s; }
+            }
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) {
+                const float ob = __shfl_xor_sync(0xffffffffu, b, o);
+                const int oa = __shfl_xor_sync(0xffffffffu, a, o);
+                if (ob < b || (ob == b && oa < a)) { b = ob; a = oa; }
+            }
+            if (lane == 0) { red_val[warp] = b; red_arg[warp] = a; }
+            __syncthreads();
+            if (tid == 0) {
+                for (int w = 1; w < CT / 32; ++w)
+                    if (red_val[w] < b || (red_val[w] == b && red_arg[w] < a)) { b = red_val[w]; a = red_arg[w]; }
+                remote_store(remote(all_val + rank, 0), b);
+                remote_store(remote(all_arg + rank, 0), a);
+            }
+            if (!choices_in_smem) __threadfence();  // the walk back reads other CTAs' units
+            cluster_sync();
+            // ---- walk back ----
+            if (rank == 0 && warp == 0) {
+                b = all_val[0];
+                a = all_arg[0];
+                for (int r = 1; r < CCL; ++r)
+                    if (all_val[r] < b || (all_val[r] == b && all_arg[r] < a)) { b = all_val[r]; a = all_arg[r]; }
+                const int levels = 1 + H + H * H <= 32 ? 3 : 1 + H <= 32 ? 2 : 1;
+                // this lane's place: level 0 is the next step, level l the step reached through l choices
+                int level = 0, combo = 0;
+                if (lane >= 1 + H && levels >= 3) { level = 2; combo = lane - 1 - H; }
+                else if (lane >= 1 && levels >= 2) { level = 1; combo = lane - 1; }
+                const bool used = level == 0 ? lane == 0 : level == 1 ? combo < H : combo < H * H;
+                int state = a;
+                if (lane == 0) path[steps - 1] = state;
+                for (int t = steps - 1; t > stop; t -= levels) {
+                    int low = state >> shift;
+                    if (level == 1) low = combo * period + (low >> shift);
+                    if (level == 2) low = (combo & (H - 1)) * period + (((combo >> shift) * period + (low >> shift)) >> shift);
+                    int choice = 0;
+                    const int slot = t - 1 - level;
+                    if (used && slot >= stop) {
+                        const int owner = low / Gc, gl = low & (Gc - 1), u = gl >> LOG_NG;
+                        const uint32_t packed =
+                            choices_in_smem ? remote_load_unit(remote(kept + ((size_t)slot * units + u) * unit_bytes, (uint32_t)owner), unit_bytes)
+                            : unit_bytes == 1 ? (uint32_t)__ldcg(scratch + row * scratch_row + ((int64_t)slot * CCL + owner) * units + u)
+                                              : (uint32_t)__ldcg(reinterpret_cast<const uint16_t *>(scratch + row * scratch_row) + ((int64_t)slot * CCL + owner) * units + u);
+                        choice = (int)(packed >> ((gl & (NG - 1)) * shift)) & (H - 1);
+                    }
+                    int from = 0;
+                    for (int l = 0; l < levels && t - 1 - l >= stop; ++l) {
+                        const int c = __shfl_sync(0xffffffffu, choice, l == 0 ? 0 : l == 1 ? 1 + from : 1 + H + from);
+                        state = c * G + (state >> shift);
+                        if (lane == 0) path[t - 1 - l] = state;
+                        from = from * H + c;
+                    }
+                }
+                if (lane == 0 && pass == 0)
+                    for (int r = 0; r < CCL; ++r) remote_store(remote(&overlap, r), state >> shift);
+            }
+            cluster_sync();
+        }
+        if (rank == 0) {
+            const float sc = scale ? scale[row] : 1.f;
+            for (int t = tid; t < steps; t += CT) {
+                const int state = path[t];
+#pragma unroll
+                for (int v = 0; v < V; ++v) out[row * T + (int64_t)t * V + v] = mul_rn(table[state * V + v], sc);
+                if (states) states[row * steps + t] = state;
+            }
+            if (codes) {
+                const int header = tail_biting ? 0 : 16 - shift;
+                for (int64_t byte = tid; byte < code_bytes; byte += CT) {
+                    uint32_t v = 0;
+                    for (int k = 0; k < 8; ++k) {
+                        const int64_t at = byte * 8 + k;
+                        int bit = 0;
+                        if (at < header) bit = path[0] >> (15 - (int)at) & 1;
+                        else if (at - header < (int64_t)steps * shift) bit = path[(at - header) / shift] >> (shift - 1 - (int)((at - header) % shift)) & 1;
+                        v |= (uint32_t)bit << k;
+                    }
+                    codes[row * code_bytes + byte] = (uint8_t)v;
+                }
+            }
+        }
+        __syncthreads();  // the next row reuses the buffers (other CTAs' ones are guarded by the first cluster_sync of its passes)
+    }
+}
+
+template <int V, int LOG_NG>
+static int launch_viterbi_cluster(int64_t rows, int T, const void *x, const void *table, int shift, int tail, const void *scale, void *out, int64_t *states,
+                                  void *workspace, uint8_t *codes, int64_t code_bytes, cudaStream_t st) {
+    static PerDeviceOnce configured;
+    constexpr int NG = 1 << LOG_NG, NH = CSTATES / NG, LIMIT = 200 * 1024;
+    const int H = 1 << shift, G = (1 << 16) >> shift, Gc = G / CCL, parts = H / NH, steps = T / V, slots = steps > 1 ? steps - 1 : 1;
+    const int minima = Gc >= H ? Gc : H, unit_bytes = NG * shift > 8 ? 2 : 1;
+    const size_t base = sizeof(float) * (2 * (size_t)minima + T) + sizeof(int) * (size_t)steps, kept = (size_t)slots * (CT / parts) * unit_bytes;
+    const int in_smem = base + kept <= LIMIT;
+    const size_t smem = base + (in_smem ? kept : 0);
+    if (smem > LIMIT) return G2D_ERR_UNSUPPORTED;
+    if (configured.run([&] { return cudaFuncSetAttribute(viterbi_cluster_kernel<V, LOG_NG>, cudaFuncAttributeMaxDynamicSharedMemorySize, LIMIT) == cudaSuccess; }) != G2D_OK)
+        return G2D_ERR_CUDA;
+    const int64_t clusters = rows < 148 / CCL ? rows : 148 / CCL;
+    cudaLaunchConfig_t config{};
+    config.gridDim = dim3((unsigned)(clusters * CCL));
+    config.blockDim = dim3(CT);
+    config.dynamicSmemBytes = smem;
+    config.stream = st;
+    cudaLaunchAttribute attribute{};
+    attribute.id = cudaLaunchAttributeClusterDimension;
+    attribute.val.clusterDim.x = CCL;
+    attribute.val.clusterDim.y = attribute.val.clusterDim.z = 1;
+    config.attrs = &attribute;
+    config.numAttrs = 1;
+    const int64_t scratch_row = (int64_t)slots * G;  // what the scratch holds per row; the units take no more
+    if (cudaLaunchKernelEx(&config, viterbi_cluster_kernel<V, LOG_NG>, rows, T, (const float *)x, (const float *)table, shift, tail, (const float *)scale,
+                           (float *)out, states, (uint8_t *)workspace, scratch_row, in_smem, codes, code_bytes) != cudaSuccess)
+        return G2D_ERR_CUDA;
+    return check_launch();
+}
+
+// Float searches over 2^16 states with 4 to 256 predecessors per state, the path short enough for shared memory; the others
+// go to the kernels above.
+static bool cluster_search_serves(int dtype, int T, int L, int shift, int V) {
+    return dtype == G2D_F32 && L == 16 && shift >= 2 && T >= 2 * V && T <= 8192;
+}
+template <int V>
+static int cluster_search(int64_t rows, int T, const void *x, const void *table, int shift, int tail, const void *scale, void *out, int64_t *states,
+                          void *workspace, uint8_t *codes, int64_t code_bytes, cudaStream_t st) {
+    switch (shift) {
+    case 2: return launch_viterbi_cluster<V, 3>(rows, T, x, table, shift, tail, scale, out, states, workspace, codes, code_bytes, st);
+    case 3: return launch_viterbi_cluster<V, 2>(rows, T, x, table, shift, tail, scale, out, states, workspace, codes, code_bytes, st);
+    case 4: return launch_viterbi_cluster<V, 1>(rows, T, x, table, shift, tail, scale, out, states, workspace, codes, code_bytes, st);
+    default: return launch_viterbi_cluster<V, 0>(rows, T, x, table, shift, tail, scale, out, states, workspace, codes, code_bytes, st);
+    }
+}
+
 // Values (and optionally states) of stored bit strings: one thread per (sequence, step) rebuilds the state from the L
 // bits of the string that end with the step's symbol.
 template <typename F>
@@ -555,6 +842,10 @@ static int indexed_sequences_per_cta(const TrellisIndex *index, int64_t rows, in
 int launch_trellis(int dtype, int64_t rows, int T, const void *x, const void *table, int L, int K, int V, int tail, const void *scale,
                    void *out, int64_t *states, void *workspace, uint8_t *codes, cudaStream_t st, const TrellisIndex *index) {
     const int64_t code_bytes = trellis_code_bytes(T, L, K, V, tail);
+    if (cluster_search_serves(dtype, T, L, K * V, V)) {
+        if (V == 2) return cluster_search<2>(rows, T, x, table, K * V, tail, scale, out, states, workspace, codes, code_bytes, st);
+        return cluster_search<1>(rows, T, x, table, K * V, tail, scale, out, states, workspace, codes, code_bytes, st);
+    }
     const int R = dtype == G2D_F32 ? indexed_sequences_per_cta<float>(index, rows, L, K, V) : indexed_sequences_per_cta<double>(index, rows, L, K, V);
     if (R == 1 && dtype == G2D_F32) return launch_viterbi_indexed<float, 1>(rows, T, x, table, *index, L, K, V, tail, scale, out, states, workspace, codes, code_bytes, st);
     if (R == 1) return launch_viterbi_indexed<double, 1>(rows, T, x, table, *index, L, K, V, tail, scale, out, states, workspace, codes, code_bytes, st);
