@@ -458,8 +458,9 @@ __global__ void __launch_bounds__(VT) viterbi_indexed_kernel(int64_t rows, int T
 // SMs, against a table read or a look-up of the local cost per state in the kernels above (11 k cycles on one SM, bound by
 // shared memory).  Four CTAs are what it takes to hold 2^16 value pairs in registers, and a coarse stage of a sweep
 // rarely has more sequences than the GPU has clusters of four.  What a step adds is the exchange: the group minimum of
-// g is needed by the CTA that owns the groups (g mod G / H) H .. + H - 1 and goes straight into its shared memory, then the cluster
-// synchronises.  HYB, T = 256, 32 sequences: 1.47 ms before, FIGURE now.
+// g is needed by the CTA that owns the groups (g mod G / H) H .. + H - 1 and goes straight into its shared memory, counted in
+// by an mbarrier there (650 cycles from one step to the next; a cluster barrier behind plain remote stores takes 1560).
+// HYB, T = 256, 32 sequences (one coarse stage of a sweep): 1.47 ms on one SM each, 0.40 ms with the cluster barrier, 0.29 ms now.
 //
 // Mapping.  G = 2^16 / H groups, Gc = G / 4 per CTA.  A thread has NG neighbouring groups and NH = 32 / NG predecessors of
 // each; with more than 32 predecessors per group, H / 32 neighbouring lanes share a group and settle its minimum by shuffle.
@@ -481,6 +482,35 @@ __device__ __forceinline__ uint32_t remote(const void *p, uint32_t rank) {  // t
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"((uint32_t)__cvta_generic_to_shared(p)), "r"(rank));
     return r;
 }
+// Stores that count towards the transaction count of an mbarrier of the same CTA as the destination
+__device__ __forceinline__ void async_store(uint32_t at, float v, uint32_t bar) {
+    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.f32 [%0], %1, [%2];" ::"r"(at), "f"(v), "r"(bar) : "memory");
+}
+__device__ __forceinline__ void async_store(uint32_t at, float a, float b, uint32_t bar) {
+    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v2.f32 [%0], {%1, %2}, [%3];" ::"r"(at), "f"(a), "f"(b), "r"(bar) : "memory");
+}
+__device__ __forceinline__ void async_store(uint32_t at, float a, float b, float c, float d, uint32_t bar) {
+    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.f32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(at), "f"(a), "f"(b), "f"(c), "f"(d), "r"(bar)
+                 : "memory");
+}
+// Bounded wait (about a second) for a phase of this CTA's barrier; false when it ran out.
+__device__ __forceinline__ bool cluster_wait(uint32_t bar, uint32_t parity) {
+    const long long start = clock64();
+    for (;;) {
+        uint32_t ok;
+        asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+                     : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+        if (ok) return true;
+        if (clock64() - start > 2000000000LL) return false;
+    }
+}
+// Two floats in one register pair: the packed additions and products round each half on its own, so a pair of states costs one
+// issue slot per operation and the same bits.
+typedef unsigned long long pair32;
+__device__ __forceinline__ pair32 pack2(float a, float b) { pair32 r; asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b)); return r; }
+__device__ __forceinline__ void unpack2(pair32 v, float &a, float &b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
+__device__ __forceinline__ pair32 add2(pair32 a, pair32 b) { pair32 r; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
+__device__ __forceinline__ pair32 mul2(pair32 a, pair32 b) { pair32 r; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
 __device__ __forceinline__ void remote_store(uint32_t at, float v) { asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(at), "f"(v) : "memory"); }
 __device__ __forceinline__ void remote_store(uint32_t at, int v) { asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(at), "r"(v) : "memory"); }
 __device__ __forceinline__ uint32_t remote_load_unit(uint32_t at, int bytes) {
@@ -511,25 +541,31 @@ __global__ void __launch_bounds__(CT, 1) viterbi_cluster_kernel(int64_t rows, in
     __shared__ int red_arg[CT / 32];
     __shared__ float all_val[CCL];
     __shared__ int all_arg[CCL];
-    __shared__ int overlap;
+    __shared__ int overlap, failed;
+    __shared__ __align__(8) uint64_t arrived[2];  // the minima of a step have arrived in prev[0] / prev[1]
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const uint32_t rank = cluster_rank();
+    const uint32_t bar0 = (uint32_t)__cvta_generic_to_shared(arrived);
+    uint32_t phases = 0;  // bit b: parity of the next wait on arrived[b]
+    if (tid == 0) {
+        failed = 0;
+        for (int b = 0; b < 2; ++b) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar0 + 8 * b) : "memory");
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
     const int unit = tid / parts, part = tid % parts, gl0 = unit * NG, h0 = part * NH, g0 = (int)rank * Gc + gl0;
 
-    float tv[CSTATES][V];
+    // states in pairs: of neighbouring groups, or of neighbouring predecessors where a thread has one group
+    pair32 tv[CSTATES / 2][V];
 #pragma unroll
-    for (int e = 0; e < CSTATES; ++e) {
-        const int s = (h0 + e / NG) * G + g0 + e % NG;
-        if constexpr (V == 2) load_pair(table + 2 * s, tv[e][0], tv[e][1]);
-        else tv[e][0] = table[s];
-    }
-    // where the minima of this thread's groups go: CTA and place by group
-    uint32_t to[NG];
+    for (int e = 0; e < CSTATES; e += 2) {
+        const int s0 = (h0 + e / NG) * G + g0 + e % NG, s1 = (h0 + (e + 1) / NG) * G + g0 + (e + 1) % NG;
 #pragma unroll
-    for (int q = 0; q < NG; ++q) {
-        const int g = g0 + q, within = g & (period - 1);
-        to[q] = Gc >= H ? remote(prev + (g / period) * PW + (within & (PW - 1)), (uint32_t)(within / PW)) : 0u;
+        for (int v = 0; v < V; ++v) tv[e / 2][v] = pack2(table[s0 * V + v], table[s1 * V + v]);
     }
+    // where the minima of this thread's groups go: neighbouring groups are neighbours there too (PW is a multiple of NG)
+    const int within = g0 & (period - 1);
+    const uint32_t to_rank = Gc >= H ? (uint32_t)(within / PW) : 0u;
+    const uint32_t to = remote(prev + (Gc >= H ? (g0 / period) * PW + (within & (PW - 1)) : g0), to_rank), to_bar = remote(arrived, to_rank);
     const int64_t clusters = gridDim.x / CCL;
     for (int64_t row = blockIdx.x / CCL; row < rows; row += clusters) {
         for (int i = tid; i < T; i += CT) xs[i] = x[row * T + i];
@@ -544,7 +580,7 @@ __global__ void __launch_bounds__(CT, 1) viterbi_cluster_kernel(int64_t rows, in
                 const int low = (i / PW) * period + (Gc >= H ? (int)rank * PW + i % PW : 0);
                 prev[minima + i] = ov >= 0 && low != ov ? INFINITY : 0.f;
             }
-            cluster_sync();  // and every CTA is done with the last pass
+            cluster_sync();  // every CTA is done with the last pass (and has its barriers initialised)
             float best[NG];
             int arg[NG];
             for (int t = 0; t < steps; ++t) {
@@ -552,22 +588,37 @@ __global__ void __launch_bounds__(CT, 1) viterbi_cluster_kernel(int64_t rows, in
                 int at = t + roll;
                 if (at >= steps) at -= steps;
                 const float x0 = xs[at * V], x1 = V == 2 ? xs[at * V + 1] : 0.f;
+                const pair32 nx0 = pack2(-x0, -x0), nx1 = pack2(-x1, -x1);
+                auto local = [&](int e) {  // the local costs of the pair e
+                    const pair32 d0 = add2(tv[e][0], nx0);
+                    pair32 c = mul2(d0, d0);
+                    if constexpr (V == 2) {
+                        const pair32 d1 = add2(tv[e][V - 1], nx1);
+                        c = add2(c, mul2(d1, d1));
+                    }
+                    return c;
+                };
+                if constexpr (NG == 1) {
 #pragma unroll
-                for (int hh = 0; hh < NH; ++hh) {
-                    float pv[NG];
-                    // neighbouring groups share their predecessor's minimum where H >= NG
+                    for (int hh = 0; hh < NH; hh += 2) {
+                        float c0, c1;
+                        unpack2(add2(pack2(before[hh * PW], before[(hh + 1) * PW]), local(hh / 2)), c0, c1);
+                        if (hh == 0 || c0 < best[0]) { best[0] = c0; arg[0] = h0 + hh; }
+                        if (c1 < best[0]) { best[0] = c1; arg[0] = h0 + hh + 1; }
+                    }
+                } else {
 #pragma unroll
-                    for (int q = 0; q < NG; ++q) pv[q] = (q == 0 || (q & (NH - 1)) == 0) ? before[hh * PW + (NG > NH ? q / NH : 0)] : pv[q - 1];
+                    for (int hh = 0; hh < NH; ++hh) {
+                        float pv = 0.f;
 #pragma unroll
-                    for (int q = 0; q < NG; ++q) {
-                        const float d0 = sub_rn(tv[hh * NG + q][0], x0);
-                        float c = mul_rn(d0, d0);
-                        if constexpr (V == 2) {
-                            const float d1 = sub_rn(tv[hh * NG + q][V - 1], x1);
-                            c = add_rn(c, mul_rn(d1, d1));
+                        for (int q = 0; q < NG; q += 2) {
+                            // neighbouring groups share their predecessor's minimum, as far as there are predecessors per group
+                            if (q % NH == 0) pv = before[hh * PW + q / NH];
+                            float c0, c1;
+                            unpack2(add2(pack2(pv, pv), local((hh * NG + q) / 2)), c0, c1);
+                            if (hh == 0 || c0 < best[q]) { best[q] = c0; arg[q] = h0 + hh; }
+                            if (hh == 0 || c1 < best[q + 1]) { best[q + 1] = c1; arg[q + 1] = h0 + hh; }
                         }
-                        c = add_rn(pv[q], c);
-                        if (hh == 0 || c < best[q]) { best[q] = c; arg[q] = h0 + hh; }
                     }
                 }
                 if constexpr (NG == 1) {
@@ -578,21 +629,35 @@ __global__ void __launch_bounds__(CT, 1) viterbi_cluster_kernel(int64_t rows, in
                     }
                 }
                 if (t + 1 < steps) {
+                    const int buf = t & 1;
+                    const uint32_t bar = bar0 + 8 * buf;
+                    if (tid == 0) asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(minima * (int)sizeof(float)) : "memory");
+                    // Every thread of this CTA has read the minima of step t - 1 when the first of step t leaves.  A CTA overwrites
+                    // a buffer two steps later, after it has received minima of the step between from every CTA of the
+                    // cluster (each sends to all four), so it never overwrites what is still being read.
+                    __syncthreads();
                     if (part == 0) {
-                        const uint32_t buffer = (uint32_t)((t & 1) * minima * (int)sizeof(float));
+                        const uint32_t at_buf = to + (uint32_t)(buf * minima * (int)sizeof(float)), at_bar = to_bar + 8 * buf;
+                        if constexpr (NG == 1) {
+                            if (Gc >= H) async_store(at_buf, best[0], at_bar);
+                            else
+                                for (uint32_t r = 0; r < CCL; ++r)
+                                    async_store(remote(prev + g0, r) + (uint32_t)(buf * minima * (int)sizeof(float)), best[0], remote(arrived, r) + 8 * buf);
+                        } else if constexpr (NG == 2) {
+                            async_store(at_buf, best[0], best[1], at_bar);
+                        } else {
+#pragma unroll
+                            for (int q = 0; q < NG; q += 4) async_store(at_buf + q * 4, best[q], best[q + 1], best[q + 2], best[q + 3], at_bar);
+                        }
                         uint32_t packed = 0;
 #pragma unroll
-                        for (int q = 0; q < NG; ++q) {
-                            if (Gc >= H) remote_store(to[q] + buffer, best[q]);
-                            else
-                                for (int r = 0; r < CCL; ++r) remote_store(remote(prev + g0 + q, r) + buffer, best[q]);
-                            packed |= (uint32_t)arg[q] << (q * shift);
-                        }
+                        for (int q = 0; q < NG; ++q) packed |= (uint32_t)arg[q] << (q * shift);
                         uint8_t *const u = choices_in_smem ? kept + ((size_t)t * units + unit) * unit_bytes : far + ((int64_t)t * CCL * units + unit) * unit_bytes;
                         if (unit_bytes == 1) *u = (uint8_t)packed;
                         else *reinterpret_cast<uint16_t *>(u) = (uint16_t)packed;
                     }
-                    cluster_sync();
+                    if (!failed && !cluster_wait(bar, (phases >> buf) & 1)) failed = 1;
+                    phases ^= 1u << buf;
                 }
             }
             // ---- first arg-min over all states of the last step, with the final mask ----
@@ -662,7 +727,9 @@ __global__ void __launch_bounds__(CT, 1) viterbi_cluster_kernel(int64_t rows, in
             }
             cluster_sync();
         }
-        if (rank == 0) {
+        if (failed) {  // a wait of this CTA ran out, which a healthy GPU does not do: no value of the row may pass for a result
+            for (int t = tid; t < T; t += CT) out[row * T + t] = __int_as_float(0x7fc00000);
+        } else if (rank == 0) {
             const float sc = scale ? scale[row] : 1.f;
             for (int t = tid; t < steps; t += CT) {
                 const int state = path[t];
