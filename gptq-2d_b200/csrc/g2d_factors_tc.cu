@@ -45,10 +45,6 @@ constexpr int TRINV_STAGE_BYTES = 6 * TILE_BYTES;          // A hi, mid, lo; B h
 constexpr int TRINV_SLICE = 8;                             // chunks per slice: k = 256
 constexpr uint32_t TRINV_TMEM_COLS = 4 * MT;               // two alternating pairs of (main, correction) accumulators
 
-__device__ __forceinline__ void trinv_arrive(uint64_t *bar) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
-
 __global__ void __launch_bounds__(TC_THREADS) trinv_tc_kernel(const __grid_constant__ TrinvJob job) {
     extern __shared__ unsigned char tc_smem_raw[];
     __shared__ __align__(8) TcRing ring;
@@ -170,7 +166,7 @@ __global__ void __launch_bounds__(TC_THREADS) trinv_tc_kernel(const __grid_const
             // this warp has read the accumulators: hand them back to the MMA warp
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();
-            if (lane == 0) trinv_arrive(&acc_empty[buf]);
+            if (lane == 0) mbar_arrive(&acc_empty[buf]);
         }
         if (go) {
             const int64_t gi = m0 + q * 32 + lane;

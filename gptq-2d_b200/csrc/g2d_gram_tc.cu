@@ -3,93 +3,165 @@
 // Hessian factors from the caller (demo.ipynb:103-106 forms them with a plain matrix product), so this entry has no
 // counterpart there.
 //
-// X^T is first written as K-major tf32 hi / lo planes [n][k] (one transposing pass), then every 128 x 128 tile of the
-// lower triangle of H is one CTA of the same pipeline as the other tensor-core kernels: TMA into a three-stage ring,
-// tcgen05.mma kind::tf32 with the 3xTF32 split (hi hi + lo hi + hi lo) into tensor memory, and an epilogue that adds
-// alpha times the accumulator to the lower triangle of H, slice of k by slice of k; a last pass mirrors the lower triangle
-// into the upper one (H is symmetric on entry and stays so bit for bit).  Every entry of H has one owner, so the result does not depend on scheduling.
+// X^T is first written as K-major fp16 pairs [n][k], every channel scaled by a power of two of its own (the channel is the
+// index that is not summed over, so the scale comes out of the product again), then every 128 x 256 tile that touches the
+// lower triangle of H is one CTA: TMA into a two-stage ring of 96 KB, tcgen05.mma kind::f16 with three products per k step
+// into tensor memory, eight warps that add the accumulators up in registers slice of k by slice of k, and at the end
+// write H and its mirror image.  Every entry of H has one owner, so the result does not depend on scheduling.
+//
+// Bound: tensor pipe and shared-memory port.  A 128 x 256 x 16 MMA reads 12 KB of operands in 128 cycles and a chunk's 96 KB
+// arrive in the 1536 cycles of its MMAs: 160 of the port's 128 bytes per cycle, so 80 % of the tensor rate; the 128 x 128
+// tf32 tiles before it were held at 60 % of half that rate, and added every slice to H in global memory (8.6 GB of
+// reductions at 8192 x 8192).  Measured at 8192 samples of 8192 channels: 4.61 ms before, 1.63 ms now (1.01 PFLOP/s of fp16
+// products; 8 waves of tiles of which the last is a seventh full).
 #include "g2d_tc.cuh"
 
 namespace g2d {
 
-// X [k][n] -> planes [n][kp], kp = k rounded up to a multiple of 4 (a TMA stride must be a multiple of 16 bytes); the
-// padding columns are zero
-__global__ void gram_split_transposed_kernel(const float *__restrict__ x, int64_t k, int64_t n, int64_t kp, float *__restrict__ hi,
-                                             float *__restrict__ lo) {
-    __shared__ float tile[32][33];
-    const int64_t tiles_s = ceil_div(kp, (int64_t)32), tiles_j = ceil_div(n, (int64_t)32);
-    for (int64_t b = blockIdx.x; b < tiles_s * tiles_j; b += gridDim.x) {
-        const int64_t s0 = (b / tiles_j) * 32, j0 = (b % tiles_j) * 32;  // source block: samples s, channels j
-        for (int r = threadIdx.y; r < 32; r += blockDim.y) {
-            const int64_t s = s0 + r, j = j0 + threadIdx.x;
-            tile[r][threadIdx.x] = (s < k && j < n) ? x[s * n + j] : 0.f;
-        }
+constexpr int GRAM_THREADS = 320;  // TMA, MMA and eight reading warps
+constexpr int GRAM_STAGES = 2;
+// The tensor cores add into their fp32 accumulator with truncation, which biases a long sum of same-sign terms (the
+// diagonal of a Gram matrix is a sum of squares): measured 9e-5 relative over k = 8192 in one accumulator.  So the k
+// range is cut into slices; each slice is accumulated in tensor memory and then added up in registers, round to nearest.
+// Two accumulators alternate, so the additions of a slice overlap the MMAs of the next.
+constexpr int GRAM_SLICE = 2;  // chunks per slice: 128 samples
+
+// four neighbouring channels of a sample; `vec`: 16-byte aligned (n is a multiple of 4, the array itself may start anywhere)
+__device__ __forceinline__ float4 four_channels(const float *p, bool vec) {
+    return vec ? *reinterpret_cast<const float4 *>(p) : make_float4(p[0], p[1], p[2], p[3]);
+}
+
+// largest |x| of every channel, as the bits of a non-negative float
+__global__ void gram_range_kernel(const float *__restrict__ x, int64_t k, int64_t n, int64_t rows_per_block, bool vec, unsigned *__restrict__ largest) {
+    const int64_t c = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) * 4;
+    if (c >= n) return;
+    const int64_t s0 = blockIdx.y * rows_per_block, s1 = min(k, s0 + rows_per_block);
+    unsigned m[4] = {0u, 0u, 0u, 0u};
+#pragma unroll 8
+    for (int64_t s = s0; s < s1; ++s) {
+        const float4 v = four_channels(x + s * n + c, vec);
+        m[0] = max(m[0], __float_as_uint(v.x) & 0x7fffffffu);
+        m[1] = max(m[1], __float_as_uint(v.y) & 0x7fffffffu);
+        m[2] = max(m[2], __float_as_uint(v.z) & 0x7fffffffu);
+        m[3] = max(m[3], __float_as_uint(v.w) & 0x7fffffffu);
+    }
+#pragma unroll
+    for (int e = 0; e < 4; ++e) atomicMax(largest + c + e, m[e]);
+}
+
+// X [k][n] -> scaled pairs [n][kp], kp = k rounded up to a multiple of 8 (a TMA stride must be a multiple of 16 bytes); the
+// padding columns are zero.  64 x 64 blocks through shared memory, 16-byte loads and stores.
+// OWN_RANGE: the block finds its channels' largest values itself, from all of their samples.  For small inputs only, where
+// a launch less (and the clearing of the array) is worth more than reading the samples once per block.
+template <bool OWN_RANGE>
+__global__ void __launch_bounds__(256) gram_split_transposed_kernel(const float *__restrict__ x, int64_t k, int64_t n, int64_t kp, bool vec,
+                                                                    unsigned *__restrict__ largest, __half *__restrict__ hi, __half *__restrict__ lo) {
+    __shared__ float tile[64][65];
+    __shared__ unsigned range[64];
+    const int tid = threadIdx.x;
+    const int64_t j0 = (int64_t)blockIdx.x * 64, s0 = (int64_t)blockIdx.y * 64;
+    if (OWN_RANGE) {
+        if (tid < 64) range[tid] = 0u;
         __syncthreads();
-        for (int r = threadIdx.y; r < 32; r += blockDim.y) {
-            const int64_t j = j0 + r, s = s0 + threadIdx.x;
-            if (j < n && s < kp) {
-                float h, l;
-                split_tf32(tile[threadIdx.x][r], h, l);
-                hi[j * kp + s] = h;
-                lo[j * kp + s] = l;
+        const int c = (tid & 15) * 4;
+        unsigned m[4] = {0u, 0u, 0u, 0u};
+        if (j0 + c < n) {
+#pragma unroll 8
+            for (int64_t s = tid >> 4; s < k; s += 16) {
+                const float4 v = four_channels(x + s * n + j0 + c, vec);
+                m[0] = max(m[0], __float_as_uint(v.x) & 0x7fffffffu);
+                m[1] = max(m[1], __float_as_uint(v.y) & 0x7fffffffu);
+                m[2] = max(m[2], __float_as_uint(v.z) & 0x7fffffffu);
+                m[3] = max(m[3], __float_as_uint(v.w) & 0x7fffffffu);
             }
         }
+#pragma unroll
+        for (int e = 0; e < 4; ++e) atomicMax(&range[c + e], m[e]);
         __syncthreads();
+        if (blockIdx.y == 0 && tid < 64 && j0 + tid < n) largest[j0 + tid] = range[tid];
+    } else if (tid < 64 && j0 + tid < n) {
+        range[tid] = largest[j0 + tid];
+    }
+#pragma unroll
+    for (int t = 0; t < 4; ++t) {
+        const int idx = t * 256 + tid, r = idx >> 4, c = (idx & 15) * 4;
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (s0 + r < k && j0 + c < n) v = four_channels(x + (s0 + r) * n + j0 + c, vec);
+        tile[r][c] = v.x; tile[r][c + 1] = v.y; tile[r][c + 2] = v.z; tile[r][c + 3] = v.w;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int t = 0; t < 2; ++t) {
+        const int idx = t * 256 + tid, j = idx >> 3, s = (idx & 7) * 8;
+        if (j0 + j >= n || s0 + s >= kp) continue;
+        const float scale = power_of_two(-range_exponent(__uint_as_float(range[j])));
+        __align__(16) __half h[8];
+        __align__(16) __half l[8];
+#pragma unroll
+        for (int e = 0; e < 8; ++e) split_half(tile[s + e][j] * scale, h[e], l[e]);
+        *reinterpret_cast<uint4 *>(hi + (j0 + j) * kp + s0 + s) = *reinterpret_cast<const uint4 *>(h);
+        *reinterpret_cast<uint4 *>(lo + (j0 + j) * kp + s0 + s) = *reinterpret_cast<const uint4 *>(l);
     }
 }
 
 struct GramJob {
-    CUtensorMap hi, lo;
+    CUtensorMap a_hi, a_lo, b_hi, b_lo;  // the same planes in boxes of 128 and of NT rows
     float *h;
+    const unsigned *largest;
     int64_t n;
     int chunks;
     float alpha;
     int *flag;
 };
 
-// The tensor cores add into their fp32 accumulator with truncation, which biases a long sum of same-sign terms (the
-// diagonal of a Gram matrix is a sum of squares): measured 9e-5 relative over k = 8192 in one accumulator.  So the k
-// range is cut into slices of SLICE chunks; each slice is accumulated in tensor memory and then added to H in global
-// memory with round-to-nearest reductions.  Two accumulators alternate, so the epilogue of a slice overlaps the MMAs
-// of the next.
-constexpr int SLICE = 4;  // 128 samples per slice
-constexpr uint32_t GRAM_TMEM_COLS = 256;
-
-__device__ __forceinline__ void mbar_arrive(uint64_t *bar) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
-
-__global__ void __launch_bounds__(TC_THREADS) gram_tc_kernel(const __grid_constant__ GramJob job) {
+template <int NT>
+__global__ void __launch_bounds__(GRAM_THREADS, 1) gram_tc_kernel(const __grid_constant__ GramJob job) {
+    constexpr int B_BYTES = NT * KH * 2, GSTAGE = 2 * HTILE_BYTES + 2 * B_BYTES;
+    constexpr uint32_t COLS = 2 * NT, DESC = idesc_16(NT, 0);
+    constexpr int MINE = NT / 2;  // columns per reading warp
     extern __shared__ unsigned char tc_smem_raw[];
-    __shared__ __align__(8) uint64_t full_bar[STAGES], empty_bar[STAGES], acc_full[2], acc_empty[2];
+    __shared__ __align__(8) uint64_t full_bar[GRAM_STAGES], empty_bar[GRAM_STAGES], acc_full[2], acc_empty[2];
     __shared__ uint32_t tmem_slot;
     __shared__ int failed;
-    // tile (I2, J2), J2 <= I2, from the linear index
-    const int64_t lin = blockIdx.x;
-    int I2 = (int)((sqrt(8.0 * (double)lin + 1.0) - 1.0) / 2.0);
-    while ((int64_t)(I2 + 1) * (I2 + 2) / 2 <= lin) ++I2;
-    while ((int64_t)I2 * (I2 + 1) / 2 > lin) --I2;
-    const int J2 = (int)(lin - (int64_t)I2 * (I2 + 1) / 2);
-    const int i0 = I2 * MT, j0 = J2 * MT;
+    // tiles that touch the lower triangle: a row of 128 has row * 128 / NT + 1 of them
+    int I2, J2;
+    {
+        const int64_t lin = blockIdx.x;
+        if (NT == 256) {  // rows 2 a and 2 a + 1 have a + 1 tiles each
+            int64_t a = (int64_t)((sqrt(4.0 * (double)lin + 1.0) - 1.0) / 2.0);
+            while ((a + 1) * (a + 2) <= lin) ++a;
+            while (a * (a + 1) > lin) --a;
+            const int64_t rest = lin - a * (a + 1);
+            I2 = (int)(2 * a + rest / (a + 1));
+            J2 = (int)(rest % (a + 1));
+        } else {
+            int64_t a = (int64_t)((sqrt(8.0 * (double)lin + 1.0) - 1.0) / 2.0);
+            while ((a + 1) * (a + 2) / 2 <= lin) ++a;
+            while (a * (a + 1) / 2 > lin) --a;
+            I2 = (int)a;
+            J2 = (int)(lin - a * (a + 1) / 2);
+        }
+    }
+    const int i0 = I2 * MT, j0 = J2 * NT;
     const int64_t n = job.n;
-    const int chunks = job.chunks, slices = (chunks + SLICE - 1) / SLICE;
+    const int chunks = job.chunks, slices = (chunks + GRAM_SLICE - 1) / GRAM_SLICE;
 
     const uint32_t smem_base = (smem_u32(tc_smem_raw) + 1023u) & ~1023u;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (threadIdx.x == 0) {
-        for (int s = 0; s < STAGES; ++s) {
+        for (int s = 0; s < GRAM_STAGES; ++s) {
             mbar_init(&full_bar[s], 1);
             mbar_init(&empty_bar[s], 1);
         }
         for (int s = 0; s < 2; ++s) {
             mbar_init(&acc_full[s], 1);
-            mbar_init(&acc_empty[s], 4);  // one arrival per epilogue warp
+            mbar_init(&acc_empty[s], 8);  // one arrival per reading warp
         }
         failed = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 1) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)), "r"(GRAM_TMEM_COLS) : "memory");
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)), "r"(COLS) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -100,79 +172,103 @@ __global__ void __launch_bounds__(TC_THREADS) gram_tc_kernel(const __grid_consta
     if (warp == 0) {
         if (lane == 0) {
             for (int ch = 0; ch < chunks; ++ch) {
-                const int stage = ch % STAGES, round = ch / STAGES;
+                const int stage = ch % GRAM_STAGES, round = ch / GRAM_STAGES;
                 if (round > 0 && !mbar_wait(&empty_bar[stage], (round - 1) & 1)) { failed = 1; break; }
-                const uint32_t dst = smem_base + stage * STAGE_BYTES;
-                mbar_expect_tx(&full_bar[stage], STAGE_BYTES);
-                tma_load_2d(dst, &job.hi, ch * KC, i0, &full_bar[stage]);
-                tma_load_2d(dst + TILE_BYTES, &job.lo, ch * KC, i0, &full_bar[stage]);
-                tma_load_2d(dst + 2 * TILE_BYTES, &job.hi, ch * KC, j0, &full_bar[stage]);
-                tma_load_2d(dst + 3 * TILE_BYTES, &job.lo, ch * KC, j0, &full_bar[stage]);
+                const uint32_t dst = smem_base + stage * GSTAGE;
+                mbar_expect_tx(&full_bar[stage], GSTAGE);
+                tma_load_2d(dst, &job.a_hi, ch * KH, i0, &full_bar[stage]);
+                tma_load_2d(dst + HTILE_BYTES, &job.a_lo, ch * KH, i0, &full_bar[stage]);
+                tma_load_2d(dst + 2 * HTILE_BYTES, &job.b_hi, ch * KH, j0, &full_bar[stage]);
+                tma_load_2d(dst + 2 * HTILE_BYTES + B_BYTES, &job.b_lo, ch * KH, j0, &full_bar[stage]);
             }
         }
     } else if (warp == 1) {
         if (lane == 0) {
             for (int ch = 0; ch < chunks; ++ch) {
-                const int stage = ch % STAGES, round = ch / STAGES;
-                const int slice = ch / SLICE, buf = slice & 1;
-                const bool opens = ch % SLICE == 0, closes = ch % SLICE == SLICE - 1 || ch == chunks - 1;
-                // the accumulator must have been read out by the epilogue of the slice two before
+                const int stage = ch % GRAM_STAGES, round = ch / GRAM_STAGES;
+                const int slice = ch / GRAM_SLICE, buf = slice & 1;
+                const bool opens = ch % GRAM_SLICE == 0, closes = ch % GRAM_SLICE == GRAM_SLICE - 1 || ch == chunks - 1;
+                // the accumulator must have been read out by the warps of the slice two before
                 if (opens && slice >= 2 && !mbar_wait(&acc_empty[buf], ((slice >> 1) - 1) & 1)) { failed = 1; break; }
                 if (!mbar_wait(&full_bar[stage], round & 1)) { failed = 1; break; }
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const uint32_t d = tmem + (uint32_t)(buf * MT);
-                const uint32_t a_hi = smem_base + stage * STAGE_BYTES, a_lo = a_hi + TILE_BYTES, b_hi = a_hi + 2 * TILE_BYTES, b_lo = a_hi + 3 * TILE_BYTES;
+                const uint32_t d = tmem + (uint32_t)(buf * NT);
+                const uint32_t a_hi = smem_base + stage * GSTAGE, a_lo = a_hi + HTILE_BYTES, b_hi = a_hi + 2 * HTILE_BYTES, b_lo = b_hi + B_BYTES;
 #pragma unroll
-                for (int ks = 0; ks < KC / 8; ++ks) {
-                    const uint32_t off = ks * 32;  // 8 tf32 values = 32 bytes along the swizzled row
-                    umma_tf32(d, umma_desc(a_hi + off), umma_desc(b_hi + off), IDESC, (opens && ks == 0) ? 0u : 1u);
-                    umma_tf32(d, umma_desc(a_lo + off), umma_desc(b_hi + off), IDESC, 1u);
-                    umma_tf32(d, umma_desc(a_hi + off), umma_desc(b_lo + off), IDESC, 1u);
+                for (int ks = 0; ks < KH / 16; ++ks) {
+                    const uint32_t off = ks * 32;  // 16 values = 32 bytes along the swizzled row
+                    umma_16(d, umma_desc(a_hi + off), umma_desc(b_hi + off), DESC, (opens && ks == 0) ? 0u : 1u);
+                    umma_16(d, umma_desc(a_lo + off), umma_desc(b_hi + off), DESC, 1u);
+                    umma_16(d, umma_desc(a_hi + off), umma_desc(b_lo + off), DESC, 1u);
                 }
                 umma_commit(&empty_bar[stage]);            // arrives when the MMAs above have read the stage
                 if (closes) umma_commit(&acc_full[buf]);   // arrives when the slice is complete in tensor memory
             }
         }
     } else {
-        // epilogue warps: lanes 32 q .. 32 q + 31 of tensor memory, q = warp % 4; one accumulator row per thread
-        const int q = warp & 3;
-        const int64_t gi = (int64_t)i0 + q * 32 + lane;
+        // reading warps: lanes 32 q .. 32 q + 31 of tensor memory, q = warp % 4, one accumulator row per thread, and half of
+        // the columns
+        const int q = warp & 3, c0 = ((warp - 2) >> 2) * MINE;
+        float total[MINE];
+#pragma unroll
+        for (int x = 0; x < MINE; ++x) total[x] = 0.f;
+        bool go = true;
         for (int slice = 0; slice < slices; ++slice) {
             const int buf = slice & 1;
             const bool ok = mbar_wait(&acc_full[buf], (slice >> 1) & 1, 64);
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             if (!ok) failed = 1;
-            if (!__all_sync(0xffffffffu, ok && !failed)) break;  // warp-uniform: the tensor-memory loads are warp-wide
-            for (int cb = 0; cb < MT / 32; ++cb) {
+            go = __all_sync(0xffffffffu, ok && !failed);  // warp-uniform: the tensor-memory loads are warp-wide
+            if (!go) break;
+#pragma unroll
+            for (int cb = 0; cb < MINE / 32; ++cb) {
                 uint32_t v[32];
-                tmem_load_32(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(buf * MT + cb * 32), v);
-                const int64_t gj0 = (int64_t)j0 + cb * 32;
-                if (gi < n) {
-                    // only the lower triangle is accumulated here; a pass at the end copies it to the upper one
-                    float *dst = job.h + gi * n + gj0;
-                    if (I2 != J2) {
+                tmem_load_32(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(buf * NT + c0 + cb * 32), v);
 #pragma unroll
-                        for (int x = 0; x < 32; x += 4) {
-                            if (gj0 + x < n) {  // n is a multiple of 4: a group is inside or outside as a whole
-                                asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dst + x), "f"(job.alpha * __uint_as_float(v[x])),
-                                             "f"(job.alpha * __uint_as_float(v[x + 1])), "f"(job.alpha * __uint_as_float(v[x + 2])),
-                                             "f"(job.alpha * __uint_as_float(v[x + 3]))
-                                             : "memory");
-                            }
-                        }
-                    } else {
-#pragma unroll
-                        for (int x = 0; x < 32; ++x) {
-                            if (gj0 + x <= gi)
-                                asm volatile("red.global.add.f32 [%0], %1;" ::"l"(dst + x), "f"(job.alpha * __uint_as_float(v[x])) : "memory");
-                        }
-                    }
-                }
+                for (int x = 0; x < 32; ++x) total[cb * 32 + x] += __uint_as_float(v[x]);
             }
             // this warp has read the accumulator: hand it back to the MMA warp
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();
             if (lane == 0) mbar_arrive(&acc_empty[buf]);
+        }
+        const int64_t gi = (int64_t)i0 + q * 32 + lane;
+        if (go && gi < n) {
+            constexpr int GROUP = 16;
+            const int row_exponent = range_exponent(__uint_as_float(job.largest[gi]));
+#pragma unroll
+            for (int x0 = 0; x0 < MINE; x0 += GROUP) {
+                const int64_t gj0 = (int64_t)j0 + c0 + x0;
+                if (gj0 > gi) continue;  // the upper triangle is the mirror image of the lower one
+                float *const dst = job.h + gi * n + gj0;
+                // the old values of sixteen columns travel together, before the first is used
+                const bool whole = gj0 + GROUP - 1 <= gi;
+                float old[GROUP];
+                if (whole) {
+#pragma unroll
+                    for (int x = 0; x < GROUP; x += 4) {
+                        const float4 v = *reinterpret_cast<const float4 *>(dst + x);
+                        old[x] = v.x; old[x + 1] = v.y; old[x + 2] = v.z; old[x + 3] = v.w;
+                    }
+                } else {
+#pragma unroll
+                    for (int x = 0; x < GROUP; ++x) old[x] = gj0 + x <= gi ? dst[x] : 0.f;
+                }
+#pragma unroll
+                for (int x = 0; x < GROUP; ++x) {
+                    const int64_t at = min(gj0 + x, n - 1);
+                    old[x] += job.alpha * scalbnf(total[x0 + x], row_exponent + range_exponent(__uint_as_float(job.largest[at])));
+                }
+                if (whole) {
+#pragma unroll
+                    for (int x = 0; x < GROUP; x += 4) *reinterpret_cast<float4 *>(dst + x) = make_float4(old[x], old[x + 1], old[x + 2], old[x + 3]);
+                }
+#pragma unroll
+                for (int x = 0; x < GROUP; ++x) {
+                    if (!whole && gj0 + x <= gi) dst[x] = old[x];
+                    if (gj0 + x < gi) job.h[(gj0 + x) * n + gi] = old[x];  // consecutive lanes write consecutive columns
+                }
+            }
         }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -183,42 +279,33 @@ __global__ void __launch_bounds__(TC_THREADS) gram_tc_kernel(const __grid_consta
             if (lane == 0) mbar_wait(&acc_full[((slices - 1) & 1)], ((slices - 1) >> 1) & 1);
             __syncwarp();
         }
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(GRAM_TMEM_COLS) : "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(COLS) : "memory");
     }
     if (threadIdx.x == 0 && failed && job.flag) atomicExch(job.flag, -1);
 }
 
-// H[j][i] = H[i][j] for j < i: the upper triangle from the lower one, 32 x 32 blocks through shared memory
-__global__ void gram_mirror_kernel(float *__restrict__ h, int64_t n) {
-    __shared__ float tile[32][33];
-    const int64_t tiles = ceil_div(n, (int64_t)32);
-    for (int64_t b = blockIdx.x; b < tiles * tiles; b += gridDim.x) {
-        const int64_t bi = b / tiles, bj = b % tiles;
-        if (bj > bi) continue;  // source blocks of the lower triangle, the diagonal blocks included
-        for (int r = threadIdx.y; r < 32; r += blockDim.y) {
-            const int64_t i = bi * 32 + r, j = bj * 32 + threadIdx.x;
-            tile[r][threadIdx.x] = (i < n && j < n) ? h[i * n + j] : 0.f;
-        }
-        __syncthreads();
-        for (int r = threadIdx.y; r < 32; r += blockDim.y) {
-            const int64_t j = bj * 32 + r, i = bi * 32 + threadIdx.x;  // target (j, i), strictly above the diagonal
-            if (i < n && j < n && j < i) h[j * n + i] = tile[threadIdx.x][r];
-        }
-        __syncthreads();
-    }
+template <int NT>
+static int launch_gram(GramJob &job, const __half *hi, const __half *lo, int64_t kp, int64_t tiles, cudaStream_t st) {
+    static PerDeviceOnce configured;
+    constexpr size_t smem = (size_t)GRAM_STAGES * (2 * HTILE_BYTES + 2 * NT * KH * 2) + 1024;
+    if (configured.run([&] { return cudaFuncSetAttribute(gram_tc_kernel<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) == cudaSuccess; }) != G2D_OK)
+        return G2D_ERR_CUDA;
+    if (!make_map_16(&job.a_hi, hi, job.n, kp, MT) || !make_map_16(&job.a_lo, lo, job.n, kp, MT) || !make_map_16(&job.b_hi, hi, job.n, kp, NT) ||
+        !make_map_16(&job.b_lo, lo, job.n, kp, NT))
+        return G2D_ERR_CUDA;
+    gram_tc_kernel<NT><<<(unsigned)tiles, GRAM_THREADS, smem, st>>>(job);
+    return check_launch();
 }
 
 }  // namespace g2d
 
 using namespace g2d;
 
-// samples rounded up to a multiple of 4 (16-byte strides), at least one k chunk
-static int64_t gram_padded(int64_t k) { return k < 32 ? 32 : (k + 3) / 4 * 4; }
+// samples rounded up to a multiple of 8 (16-byte strides), at least one k chunk
+static int64_t gram_padded(int64_t k) { return k < KH ? KH : (k + 7) / 8 * 8; }
 
-static size_t gram_bytes(int64_t n, int64_t k) {
-    const size_t kp = (size_t)gram_padded(k);
-    return (2 * (size_t)n * kp * sizeof(float) + 255) & ~(size_t)255;
-}
+static size_t gram_plane(int64_t n, int64_t k) { return (2 * (size_t)n * (size_t)gram_padded(k) + 255) & ~(size_t)255; }
+static size_t gram_bytes(int64_t n, int64_t k) { return 2 * gram_plane(n, k) + ((sizeof(unsigned) * (size_t)n + 255) & ~(size_t)255); }
 
 extern "C" int g2d_gram_workspace_bytes(int64_t n, int64_t k, size_t *bytes) {
     if (n < 0 || k < 0 || !bytes) return G2D_ERR_BAD_ARGUMENT;
@@ -230,27 +317,37 @@ extern "C" int g2d_gram_accumulate(int64_t n, int64_t k, const float *x, float a
                                    size_t workspace_bytes, void *stream) {
     if (n < 0 || k < 0) return G2D_ERR_BAD_ARGUMENT;
     if (n == 0 || k == 0) return G2D_OK;
-    if (!x || !h || n % 4 != 0 || ((uintptr_t)h & 15) != 0) return G2D_ERR_BAD_ARGUMENT;
+    if (!x || !h || n % 4 != 0 || ((uintptr_t)h & 15) != 0 || ((uintptr_t)x & 3) != 0) return G2D_ERR_BAD_ARGUMENT;
     if (!workspace || workspace_bytes < gram_bytes(n, k) || ((uintptr_t)workspace & 255) != 0) return G2D_ERR_WORKSPACE;
-    const int64_t kp = gram_padded(k), tiles = ceil_div(n, (int64_t)MT);
-    if (tiles * (tiles + 1) / 2 > 0x7fffffff || kp > 0x7fffffff) return G2D_ERR_TOO_LARGE;
+    const int64_t kp = gram_padded(k), rows = ceil_div(n, (int64_t)MT);
+    if (rows * (rows + 1) / 2 > 0x7fffffff || kp > 0x3fffffff || ceil_div(kp, (int64_t)64) > 65535) return G2D_ERR_TOO_LARGE;
     cudaStream_t st = (cudaStream_t)stream;
-    static PerDeviceOnce configured;
-    const size_t smem = (size_t)STAGES * STAGE_BYTES + 1024;
-    if (configured.run([&] { return cudaFuncSetAttribute(gram_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) == cudaSuccess; }) != G2D_OK)
-        return G2D_ERR_CUDA;
-    float *hi = (float *)workspace, *lo = hi + n * kp;
-    gram_split_transposed_kernel<<<148 * 8, dim3(32, 8), 0, st>>>(x, k, n, kp, hi, lo);
+    __half *hi = (__half *)workspace, *lo = (__half *)((char *)workspace + gram_plane(n, k));
+    unsigned *largest = (unsigned *)((char *)workspace + 2 * gram_plane(n, k));
+    const bool vec = ((uintptr_t)x & 15) == 0;
+    const dim3 split_grid((unsigned)ceil_div(n, (int64_t)64), (unsigned)ceil_div(kp, (int64_t)64));
+    if (k <= 512 && n <= 2048) {
+        gram_split_transposed_kernel<true><<<split_grid, 256, 0, st>>>(x, k, n, kp, vec, largest, hi, lo);
+    } else {
+        if (cudaMemsetAsync(largest, 0, sizeof(unsigned) * (size_t)n, st) != cudaSuccess) return G2D_ERR_CUDA;
+        const int64_t across = ceil_div(n / 4, (int64_t)128);
+        int64_t parts = ceil_div((int64_t)148 * 8, across);  // about eight blocks per SM, at least 32 samples each
+        if (parts > ceil_div(k, (int64_t)32)) parts = ceil_div(k, (int64_t)32);
+        const int64_t per = ceil_div(k, parts);
+        gram_range_kernel<<<dim3((unsigned)across, (unsigned)ceil_div(k, per)), 128, 0, st>>>(x, k, n, per, vec, largest);
+        if (check_launch() != G2D_OK) return G2D_ERR_CUDA;
+        gram_split_transposed_kernel<false><<<split_grid, 256, 0, st>>>(x, k, n, kp, vec, largest, hi, lo);
+    }
     if (check_launch() != G2D_OK) return G2D_ERR_CUDA;
     GramJob job;
-    if (!make_map(&job.hi, hi, n, kp) || !make_map(&job.lo, lo, n, kp)) return G2D_ERR_CUDA;
     job.h = h;
+    job.largest = largest;
     job.n = n;
-    job.chunks = (int)ceil_div(kp, (int64_t)KC);
+    job.chunks = (int)ceil_div(kp, (int64_t)KH);
     job.alpha = alpha;
     job.flag = status_flag;
-    gram_tc_kernel<<<(unsigned)(tiles * (tiles + 1) / 2), TC_THREADS, smem, st>>>(job);
-    if (check_launch() != G2D_OK) return G2D_ERR_CUDA;
-    gram_mirror_kernel<<<148 * 8, dim3(32, 8), 0, st>>>(h, n);
-    return check_launch();
+    // 128 x 256 tiles take 1.5 times as long as 128 x 128 ones; narrow factors have too few of them to fill the GPU
+    const int64_t wide = (rows / 2) * (rows / 2 + 1) + (rows % 2) * (rows / 2 + 1), square = rows * (rows + 1) / 2;
+    if (3 * ceil_div(wide, (int64_t)148) <= 2 * ceil_div(square, (int64_t)148)) return launch_gram<256>(job, hi, lo, kp, wide, st);
+    return launch_gram<128>(job, hi, lo, kp, square, st);
 }

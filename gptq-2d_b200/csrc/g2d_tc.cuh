@@ -89,6 +89,39 @@ __device__ __forceinline__ void tmem_load_32(uint32_t taddr, uint32_t (&v)[32]) 
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
 
+// ---- 16-bit operands: K-major tiles of 64 values = 128 bytes per row, the same swizzle and descriptor as above ----
+constexpr int KH = 64;                     // k per chunk
+constexpr int HTILE_BYTES = MT * KH * 2;   // 16 KB: 128 rows
+// D fp32, A and B 16 bits (format 0: fp16, 1: bf16), both K-major, M = 128, N = nt
+__host__ __device__ constexpr uint32_t idesc_16(int nt, uint32_t format) {
+    return (1u << 4) | (format << 7) | (format << 10) | ((uint32_t)(nt >> 3) << 17) | ((uint32_t)(MT >> 4) << 24);
+}
+__device__ __forceinline__ void umma_16(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+        ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+__device__ __forceinline__ void mbar_arrive(uint64_t *bar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
+
+// Float operands as fp16 pairs.  A value times a power of two, chosen so that the largest value it shares its scale with lies
+// in [2^14, 2^15), is hi + lo with 11 significant bits each: relative error 2^-23 down to 2^-17 of the largest value (the same
+// as a tf32 pair), an absolute error of 2^-40 of it below.  The three products hi hi + lo hi + hi lo then cost half of
+// their tf32 counterparts in tensor cycles and operand bytes.  `range_exponent` is the power: x 2^-e in (2^14, 2^15].
+__device__ __forceinline__ int range_exponent(float largest) {
+    const int e = (int)((__float_as_uint(largest) >> 23) & 255) - 127;  // largest in [2^e, 2^(e + 1))
+    return e == 128 ? 0 : (e < -100 ? -100 : e) - 14;                   // infinities and NaN stay what they are; zeros and tiny rows: any scale
+}
+__device__ __forceinline__ float power_of_two(int e) { return __uint_as_float((uint32_t)(e + 127) << 23); }  // -126 <= e <= 127
+__device__ __forceinline__ void split_half(float scaled, __half &hi, __half &lo) {
+    hi = __float2half_rn(scaled);
+    lo = __float2half_rn(scaled - __half2float(hi));
+}
+
 // ---- one-accumulator pipeline: C[128 x 128] = sum over k chunks of A[128 x 32] B[128 x 32]^T, 3xTF32 ----
 // Shared state of a CTA of TC_THREADS threads: warp 0 loads, warp 1 issues the MMAs, warps 2-5 read the accumulator.
 struct TcRing {
@@ -207,5 +240,16 @@ static bool make_map(CUtensorMap *map, const float *base, int64_t rows, int64_t 
               CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+// row-major 16-bit matrix [rows][cols]; boxes of box_rows rows x 64 columns
+static bool make_map_16(CUtensorMap *map, const void *base, int64_t rows, int64_t cols, int box_rows, bool bf16 = false) {
+    EncodeTiledFn fn = encode_tiled_fn();
+    if (!fn) return false;
+    const cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
+    const cuuint64_t strides[1] = {(cuuint64_t)cols * 2};
+    const cuuint32_t box[2] = {KH, (cuuint32_t)box_rows};
+    const cuuint32_t elem[2] = {1, 1};
+    return fn(map, bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void *>(base), dims, strides, box, elem,
+              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
 
 }  // namespace g2d
