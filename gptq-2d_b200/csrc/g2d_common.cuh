@@ -179,19 +179,6 @@ __device__ __forceinline__ void split_tf32(float a, float &hi, float &lo) {
     lo = a - hi;
 }
 
-// fp32 -> three tf32 values with a = hi + mid + lo exactly (11 + 11 + the last 2 significant bits).  The six products
-// hi hi' + hi mid' + mid hi' + mid mid' + hi lo' + lo hi' then carry the fp32 product to about 2^-32: used where the
-// 2^-21 of the two-plane split is not enough (the triangular inverse, whose error the condition number amplifies).
-__device__ __forceinline__ void split_tf32_3(float a, float &hi, float &mid, float &lo) {
-    uint32_t h, m;
-    asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(h) : "f"(a));
-    hi = __uint_as_float(h);
-    const float r = a - hi;
-    asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(m) : "f"(r));
-    mid = __uint_as_float(m);
-    lo = r - mid;
-}
-
 // Operand planes of the tensor-core macro updates (all float; see g2d_macro_update_tc.cu).
 struct TcPlanes {
     float *et_hi, *et_lo, *c_hi, *c_lo;  // written by the tile sweep
@@ -216,35 +203,41 @@ int macro_tc_prepare(MacroTcMaps *maps, const TcPlanes &planes, int64_t m, int64
 int launch_macro_update_tc(const MacroTcMaps *maps, const TcPlanes &planes, float *y, float *c, int64_t m, int64_t n, int s0, int s1, int s_end,
                            cudaStream_t stream, int t_first = 0, int stages = 3);
 
-// One problem of the tensor-core triangular inverse of the factor preparation (all [n][n] float; see g2d_factors_tc.cu).
+// One problem of the tensor-core triangular inverse of the factor preparation (see g2d_factors_tc.cu).
 struct FactorPlanes {
-    const float *a;            // Cholesky factor T in its lower triangle
-    float *out;                // the inverse being built
-    // every operand as three tf32 planes hi + mid + lo = the float32 value exactly (see split_tf32_3):
-    float *out_hi, *out_mid, *out_lo;      // the inverse
-    float *outt_hi, *outt_mid, *outt_lo;   // its transpose
-    float *tw_hi, *tw_mid, *tw_lo;         // lower triangle: T; upper triangle: the transposed intermediate product
-    int64_t n;
+    const float *a;            // [n][n], Cholesky factor T in its lower triangle
+    float *out;                // [n][n], the inverse being built
+    // every operand as three bf16 planes hi + mid + lo = the float32 value exactly, rows of ld values:
+    __nv_bfloat16 *out_hi, *out_mid, *out_lo;      // the inverse
+    __nv_bfloat16 *outt_hi, *outt_mid, *outt_lo;   // its transpose
+    __nv_bfloat16 *tw_hi, *tw_mid, *tw_lo;         // lower triangle: T; upper triangle: the transposed intermediate product
+    int64_t n, ld;
     int *flag;                 // receives -1 when a bounded wait inside a kernel ran out (may be null)
 };
 int launch_trinv_tc(int count, const FactorPlanes *problems, cudaStream_t stream);
 
 // Tensor-core trailing update of the blocked Cholesky factorization (see g2d_factors_tc.cu).  pt planes are
-// [n][SYRK_TC_K] float: pt[r][k] = a[o + k][r] for the group of block rows that starts at row o.
+// [n][SYRK_TC_K] fp16 pairs: pt[r][k] = a[o + k][r] / unscale[r] for the group of block rows that starts at row o.
 constexpr int SYRK_TC_K = 256;
 struct SyrkTcMaps {
-    alignas(64) unsigned char hi[128], lo[128];  // tensor maps of the hi and lo planes (opaque here)
+    alignas(64) unsigned char hi[128], lo[128], wide_hi[128], wide_lo[128], target[128];  // tensor maps of the planes and of the matrix (opaque here)
 };
 struct SyrkTcTarget {
     const SyrkTcMaps *maps;
-    const float *pt_hi, *pt_lo;  // the planes the maps describe
     float *a;
-    int64_t n;
+    const float *unscale;
+    int64_t n, o;
     int t_lo, t_hi;  // target 128-row tile rows [t_lo, t_hi), tile columns up to the diagonal
     int kw;          // rows of the group (<= SYRK_TC_K)
     int *flag;
 };
-bool syrk_tc_maps(SyrkTcMaps *maps, const float *pt_hi, const float *pt_lo, int64_t n);
+struct SyrkRange {
+    const float *a[2];
+    float *unscale[2];
+    int64_t n[2];
+};
+int launch_syrk_range(int count, const SyrkRange &r, cudaStream_t stream);
+bool syrk_tc_maps(SyrkTcMaps *maps, const __half *pt_hi, const __half *pt_lo, float *a, int64_t n);
 int launch_syrk_tc(int count, const SyrkTcTarget *targets, cudaStream_t stream);
 
 // Trellis (Viterbi) search of `rows` sequences (see g2d_trellis.cu); `codes` optional packed paths, code bytes apart.

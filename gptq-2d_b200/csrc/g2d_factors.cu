@@ -76,8 +76,9 @@ struct LdlProblem {
     F *a, *out, *tinv, *w;
     int64_t n;
     int *flag;
-    int tc;                       // trailing updates of whole groups run on the tensor cores (float, n % 4 == 0)
-    float *pt_hi[2], *pt_lo[2];   // [n][GROUP * 64] transposed split panels of the even and odd groups
+    int tc;                       // trailing updates of whole groups run on the tensor cores (float)
+    __half *pt_hi[2], *pt_lo[2];  // [n][GROUP * 64] transposed, scaled split panels of the even and odd groups
+    float *unscale;               // [n] powers of two: the panels hold value / unscale[column]
 };
 template <typename F>
 struct LdlBatch {
@@ -250,21 +251,25 @@ __global__ void __launch_bounds__(FTH) ldl_trsm_kernel(LdlBatch<F> B, int step_d
         // update (columns left of the group only); rows beyond a ragged block are zero in acc already
         const int kb_lo = kb / GROUP * GROUP;
         if (Q.tc && j < kb_lo) {
-            float *hi = Q.pt_hi[(kb / GROUP) & 1], *lo = Q.pt_lo[(kb / GROUP) & 1];
+            __half *hi = Q.pt_hi[(kb / GROUP) & 1], *lo = Q.pt_lo[(kb / GROUP) & 1];
             const int k0 = (kb - kb_lo) * FB;
 #pragma unroll
             for (int y = 0; y < 8; ++y) {
                 const int64_t c = c0 + own8(tx, y);
+                const float scale = 1.f / Q.unscale[c];  // a power of two: exact
 #pragma unroll
                 for (int half = 0; half < 2; ++half) {
-                    float4 h, l;
-                    split_tf32(acc[4 * half][y], h.x, l.x);
-                    split_tf32(acc[4 * half + 1][y], h.y, l.y);
-                    split_tf32(acc[4 * half + 2][y], h.z, l.z);
-                    split_tf32(acc[4 * half + 3][y], h.w, l.w);
+                    __align__(8) __half h[4];
+                    __align__(8) __half l[4];
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {
+                        const float v = acc[4 * half + e][y] * scale;
+                        h[e] = __float2half_rn(v);
+                        l[e] = __float2half_rn(v - __half2float(h[e]));
+                    }
                     const int64_t at = c * (GROUP * FB) + k0 + own8(ty, 4 * half);
-                    *reinterpret_cast<float4 *>(hi + at) = h;
-                    *reinterpret_cast<float4 *>(lo + at) = l;
+                    *reinterpret_cast<uint2 *>(hi + at) = *reinterpret_cast<const uint2 *>(h);
+                    *reinterpret_cast<uint2 *>(lo + at) = *reinterpret_cast<const uint2 *>(l);
                 }
             }
         }
@@ -432,6 +437,27 @@ static SideLane *acquire_side_lane() {
     return lane;
 }
 
+// Workspace of one problem: inverted diagonal blocks, normalisation blocks, scratch of the doubling steps and, for float, the
+// nine operand planes of the tensor-core triangular inverse, two pairs of transposed split panels and their scales.
+inline int64_t plane_pitch(int64_t n) { return (n + 7) / 8 * 8; }  // rows of the 16-bit planes are 16-byte multiples (a TMA requirement)
+struct LdlLayout {
+    size_t tinv, dblk, w, planes, panels, unscale, total;
+};
+static LdlLayout ldl_layout(size_t elem, int64_t n) {
+    LdlLayout lay;
+    size_t at = 0;
+    auto take = [&](size_t bytes) { const size_t where = at; at += (bytes + 255) & ~(size_t)255; return where; };
+    lay.tinv = take(elem * (size_t)ceil_div(n, (int64_t)FB) * FB * FB);  // [blocks][64][64]
+    lay.dblk = take(elem * (size_t)n * FB);                              // [n / size][size][size]
+    lay.w = take(elem * (size_t)n * n);                                  // [n][n]
+    const bool tc = elem == 4;
+    lay.planes = take(tc ? 9 * sizeof(__nv_bfloat16) * (size_t)n * plane_pitch(n) : 0);
+    lay.panels = take(tc ? 4 * sizeof(__half) * (size_t)n * GROUP * FB : 0);
+    lay.unscale = take(tc ? sizeof(float) * (size_t)n : 0);
+    lay.total = at;
+    return lay;
+}
+
 template <typename F>
 int ldl_run(int count, const int64_t *ns, F *const *as, const int *sizes, F *const *outs, int *flags, void *const *workspaces, cudaStream_t st) {
     LdlBatch<F> B;
@@ -441,23 +467,27 @@ int ldl_run(int count, const int64_t *ns, F *const *as, const int *sizes, F *con
     SyrkTcMaps pt_maps[2][2];
     int64_t n_max = 0;
     bool any_tc = false;
+    SyrkRange range{};
+    LdlLayout layout[2];
     for (int z = 0; z < count; ++z) {
         const int64_t n = ns[z];
-        const int nb = (int)ceil_div(n, FB);
-        F *tinv = (F *)workspaces[z];                             // [nb][64][64]
-        dblks[z] = tinv + (int64_t)nb * FB * FB;                  // [n / size][size][size]
+        layout[z] = ldl_layout(sizeof(F), n);
+        const LdlLayout &lay = layout[z];
+        char *ws = (char *)workspaces[z];
+        dblks[z] = (F *)(ws + lay.dblk);
         LdlProblem<F> &P = B.p[z];
-        P = LdlProblem<F>{as[z], outs[z], tinv, dblks[z] + n * (int64_t)FB /* [n][n] scratch of the doubling steps */, n,
-                          flags ? flags + z : nullptr, 0, {nullptr, nullptr}, {nullptr, nullptr}};
-        // float problems whose rows are 16-byte multiples use the tensor cores; the choice depends on the problem alone,
-        // never on its partner in the batch, so that a pair gives the results of two single calls
-        if (std::is_same<F, float>::value && n % 4 == 0) {
-            float *base = (float *)P.w + 10 * n * n;  // behind the scratch and the nine planes of the triangular inverse
+        P = LdlProblem<F>{as[z], outs[z], (F *)(ws + lay.tinv), (F *)(ws + lay.w), n, flags ? flags + z : nullptr, 0, {nullptr, nullptr}, {nullptr, nullptr}, nullptr};
+        if (std::is_same<F, float>::value) {
+            const size_t panel = sizeof(__half) * (size_t)n * GROUP * FB;
             for (int k = 0; k < 2; ++k) {
-                P.pt_hi[k] = base + (2 * k) * n * (GROUP * FB);
-                P.pt_lo[k] = base + (2 * k + 1) * n * (GROUP * FB);
-                if (!syrk_tc_maps(&pt_maps[z][k], P.pt_hi[k], P.pt_lo[k], n)) return G2D_ERR_CUDA;
+                P.pt_hi[k] = (__half *)(ws + lay.panels + (2 * k) * panel);
+                P.pt_lo[k] = (__half *)(ws + lay.panels + (2 * k + 1) * panel);
+                if (!syrk_tc_maps(&pt_maps[z][k], P.pt_hi[k], P.pt_lo[k], (float *)as[z], n)) return G2D_ERR_CUDA;
             }
+            P.unscale = (float *)(ws + lay.unscale);
+            range.a[z] = (const float *)as[z];
+            range.unscale[z] = P.unscale;
+            range.n[z] = n;
             P.tc = 1;
             any_tc = true;
         }
@@ -466,6 +496,7 @@ int ldl_run(int count, const int64_t *ns, F *const *as, const int *sizes, F *con
         n_max = n > n_max ? n : n_max;
         if (cudaMemsetAsync(outs[z], 0, sizeof(F) * (size_t)n * n, st) != cudaSuccess) return G2D_ERR_CUDA;
     }
+    if (any_tc && n_max > GROUP * FB && launch_syrk_range(count, range, st) != G2D_OK) return G2D_ERR_CUDA;
     if (count == 1) B.p[1] = B.p[0];
     if (flags && cudaMemsetAsync(flags, 0, sizeof(int) * count, st) != cudaSuccess) return G2D_ERR_CUDA;
     // Each step factors one 64-row block row (last first): diagonal block, panel to its left, trailing update.  The
@@ -518,8 +549,7 @@ int ldl_run(int count, const int64_t *ns, F *const *as, const int *sizes, F *con
             const int64_t o = (int64_t)kb_lo * FB;
             const int t_all = (int)(o / 128), t_next = t_all - GROUP * FB / 128;  // tile rows above the group; those of the next group start at t_next
             const int kw = (int)(ns[z] - o < GROUP * FB ? ns[z] - o : GROUP * FB);
-            SyrkTcTarget t{&pt_maps[z][(kb_lo / GROUP) & 1], B.p[z].pt_hi[(kb_lo / GROUP) & 1], B.p[z].pt_lo[(kb_lo / GROUP) & 1],
-                           (float *)B.p[z].a, ns[z], t_next, t_all, kw, B.p[z].flag};
+            SyrkTcTarget t{&pt_maps[z][(kb_lo / GROUP) & 1], (float *)B.p[z].a, B.p[z].unscale, ns[z], o, t_next, t_all, kw, B.p[z].flag};
             next[targets] = t;
             t.t_lo = 0;
             t.t_hi = t_next;
@@ -546,8 +576,7 @@ int ldl_run(int count, const int64_t *ns, F *const *as, const int *sizes, F *con
         if (rest_recorded[k] && cudaStreamWaitEvent(st, lane->rest[k], 0) != cudaSuccess) return G2D_ERR_CUDA;
     ldl_copy_diag_inverse_kernel<F><<<dim3(B.steps, count), FTH, 0, st>>>(B);
     if (check_launch() != G2D_OK) return G2D_ERR_CUDA;
-    // The 64-level for everyone; from the 128-level on, float problems whose rows are 16-byte multiples continue on the
-    // tensor cores and the others here.  The choice depends on the problem alone, never on its partner in the batch.
+    // The 64-level for everyone; from the 128-level on, float problems continue on the tensor cores.
     auto ffma_levels = [&](const LdlBatch<F> &batch, int problems, int64_t n_top, int64_t b_first, int64_t b_end) {
         for (int64_t b = b_first; b < n_top && b < b_end; b *= 2) {
             const int64_t pairs = ceil_div(n_top, 2 * b), tiles = b / FB;
@@ -560,32 +589,17 @@ int ldl_run(int count, const int64_t *ns, F *const *as, const int *sizes, F *con
         }
         return (int)G2D_OK;
     };
-    int status = ffma_levels(B, count, n_max, FB, 2 * FB);
+    int status = ffma_levels(B, count, n_max, FB, any_tc ? 2 * FB : INT64_MAX);
     if (status != G2D_OK) return status;
-    FactorPlanes planes[2];
-    int tensor_count = 0;
-    LdlBatch<F> rest = B;
-    int rest_count = 0;
-    int64_t rest_max = 0;
-    for (int z = 0; z < count; ++z) {
-        const int64_t n = ns[z];
-        if (std::is_same<F, float>::value && n % 4 == 0) {
-            float *base = (float *)B.p[z].w + n * n;  // nine [n][n] planes behind the scratch of the 64-level
-            planes[tensor_count++] = FactorPlanes{(const float *)as[z], (float *)outs[z], base, base + n * n, base + 2 * n * n,
-                                                  base + 3 * n * n, base + 4 * n * n, base + 5 * n * n, base + 6 * n * n, base + 7 * n * n,
-                                                  base + 8 * n * n, n, flags ? flags + z : nullptr};
-        } else {
-            rest.p[rest_count++] = B.p[z];
-            rest_max = n > rest_max ? n : rest_max;
+    if (any_tc && n_max > 2 * FB) {
+        FactorPlanes planes[2];
+        for (int z = 0; z < count; ++z) {
+            const int64_t n = ns[z], ld = plane_pitch(n);
+            auto plane = [&](int k) { return (__nv_bfloat16 *)((char *)workspaces[z] + layout[z].planes) + (size_t)k * n * ld; };
+            planes[z] = FactorPlanes{(const float *)as[z], (float *)outs[z], plane(0), plane(1), plane(2), plane(3), plane(4), plane(5), plane(6), plane(7), plane(8),
+                                     n, ld, flags ? flags + z : nullptr};
         }
-    }
-    if (rest_count == 1) rest.p[1] = rest.p[0];
-    if (rest_count > 0) {
-        status = ffma_levels(rest, rest_count, rest_max, 2 * FB, INT64_MAX);
-        if (status != G2D_OK) return status;
-    }
-    if (tensor_count > 0) {
-        status = launch_trinv_tc(tensor_count, planes, st);
+        status = launch_trinv_tc(count, planes, st);
         if (status != G2D_OK) return status;
     }
     for (int z = 0; z < count; ++z) {
@@ -606,13 +620,7 @@ int ldl_run(int count, const int64_t *ns, F *const *as, const int *sizes, F *con
 
 using namespace g2d;
 
-static size_t ldl_bytes(int dtype, int64_t n) {
-    const size_t elem = dtype == G2D_F32 ? 4 : 8;
-    const size_t nb = (size_t)ceil_div(n, FB);
-    // float: nine operand planes of the tensor-core triangular inverse and two pairs of transposed split panels
-    const size_t planes = dtype == G2D_F32 ? 9 * (size_t)n * n + 4 * (size_t)n * GROUP * FB : 0;
-    return ((nb * FB * FB + (size_t)n * FB + (size_t)n * n + planes) * elem + 255) & ~(size_t)255;
-}
+static size_t ldl_bytes(int dtype, int64_t n) { return ldl_layout(dtype == G2D_F32 ? 4 : 8, n).total; }
 
 extern "C" int g2d_ldl_workspace_bytes(int dtype, int64_t n, size_t *bytes) {
     if ((dtype != G2D_F32 && dtype != G2D_F64) || n < 0 || !bytes) return G2D_ERR_BAD_ARGUMENT;

@@ -4,7 +4,7 @@
 // The inverse Lf = T^{-1} of the lower triangular Cholesky factor is built by doubling: at level b every aligned pair
 // of finished b x b diagonal blocks [A^{-1} 0; . B^{-1}] of Lf is completed by X = -B^{-1} (C A^{-1}) with
 // C = T[second half rows, first half columns].  From b = 128 on, both products of a level run here as tcgen05.mma
-// kind::tf32 GEMMs over 128 x 128 output tiles on three tf32 planes per operand (six products per k step, see
+// kind::f16 GEMMs over 128 x 128 output tiles on three bf16 planes per operand (six products per k step, see
 // "Precision" below).  The MMA wants both operands K-major, so the first product is formed transposed,
 //     W^T[j][i] = sum_k Lf^T[j][k] T[i][k]        (k from the tile's first row j0 to the end of the first half)
 //     X[i][j]   = -sum_k Lf[i][k] W^T[j][k]       (k from the start of the second half through the tile's rows)
@@ -31,19 +31,30 @@ struct TrinvJob {
 };
 
 // Precision.  The inverse is where a badly conditioned factor shows: every level multiplies explicit inverse blocks, and
-// the error of each product is amplified by the cancellation in -B^{-1} (C A^{-1}); with the two-plane 3xTF32 split
-// (2^-21 per product) the factors of a heavy-tailed, 1 %-damped 4096 x 4096 Gram came out 4e-5 from the float64 result
-// where a float32 LAPACK factorization is 1.5e-6 away.  So this kernel uses three planes per operand and six products
-// (about 2^-32 per product), and keeps the one large product (hi hi') in an accumulator of its own, so that the five
-// small ones are not truncated against it.  What then remained (1.4e-5 at 4096, growing with n where the same algorithm
-// on FFMA stays at 2.4e-6) was the tensor cores' accumulation itself: every add into the float accumulator truncates, and
-// the sums here run over up to n / 2 terms.  So the k range is cut into slices of 256: each slice is accumulated in
+// the error of each product is amplified by the cancellation in -B^{-1} (C A^{-1}); with a two-plane split (2^-21 per
+// product) the factors of a heavy-tailed, 1 %-damped 4096 x 4096 Gram came out 4e-5 from the float64 result where a float32
+// LAPACK factorization is 1.5e-6 away.  So this kernel uses three planes per operand, a = hi + mid + lo exactly, and keeps the
+// one large product (hi hi') in an accumulator of its own, so that the small ones are not truncated against it.  The planes
+// are bf16 (8 + 8 + 8 bits, the exponent range of float): the six products leave out mid lo' and what is smaller, 2^-26 of a
+// product, a quarter of what a float32 multiplication rounds off; they cost half of six tf32 products in tensor cycles and
+// bytes, and the factors did not move (FACTORERR).
+// The second source of error is the tensor cores' accumulation: every add into the float accumulator truncates, and the sums
+// here run over up to n / 2 terms.  So the k range is cut into slices of 256: each slice is accumulated in
 // tensor memory, and the epilogue warps add the slices up in registers with round-to-nearest additions while the MMAs
 // of the next slice run into a second pair of accumulators.
 constexpr int TRINV_STAGES = 2;
-constexpr int TRINV_STAGE_BYTES = 6 * TILE_BYTES;          // A hi, mid, lo; B hi, mid, lo
-constexpr int TRINV_SLICE = 8;                             // chunks per slice: k = 256
+constexpr int TRINV_STAGE_BYTES = 6 * HTILE_BYTES;         // A hi, mid, lo; B hi, mid, lo
+constexpr int TRINV_SLICE = 4;                             // chunks per slice: k = 256
 constexpr uint32_t TRINV_TMEM_COLS = 4 * MT;               // two alternating pairs of (main, correction) accumulators
+constexpr uint32_t TRINV_DESC = idesc_16(MT, 1);           // bf16
+
+// fp32 -> three bf16 values with a = hi + mid + lo exactly (8 significant bits each)
+__device__ __forceinline__ void split_bf16_3(float a, __nv_bfloat16 &hi, __nv_bfloat16 &mid, __nv_bfloat16 &lo) {
+    hi = __float2bfloat16_rn(a);
+    const float r = a - __bfloat162float(hi);
+    mid = __float2bfloat16_rn(r);
+    lo = __float2bfloat16_rn(r - __bfloat162float(mid));
+}
 
 __global__ void __launch_bounds__(TC_THREADS) trinv_tc_kernel(const __grid_constant__ TrinvJob job) {
     extern __shared__ unsigned char tc_smem_raw[];
@@ -75,7 +86,7 @@ __global__ void __launch_bounds__(TC_THREADS) trinv_tc_kernel(const __grid_const
         k_hi = min(m0 + MT, r2);
         a_maps = maps->out;
     }
-    const int chunks = (int)ceil_div(k_hi - k_lo, (int64_t)KC);  // a ragged tail reads zeros beyond the matrix
+    const int chunks = (int)ceil_div(k_hi - k_lo, (int64_t)KH);  // a ragged tail reads zeros beyond the matrix
     const int slices = (chunks + TRINV_SLICE - 1) / TRINV_SLICE;
 
     const uint32_t smem_base = (smem_u32(tc_smem_raw) + 1023u) & ~1023u;
@@ -95,12 +106,12 @@ __global__ void __launch_bounds__(TC_THREADS) trinv_tc_kernel(const __grid_const
                     ring.failed = 1;
                     break;
                 }
-                const int k = (int)(k_lo + (int64_t)ch * KC);
+                const int k = (int)(k_lo + (int64_t)ch * KH);
                 const uint32_t dst = smem_base + stage * TRINV_STAGE_BYTES;
                 mbar_expect_tx(&ring.full[stage], TRINV_STAGE_BYTES);
                 for (int part = 0; part < 3; ++part) {
-                    tma_load_2d(dst + part * TILE_BYTES, &a_maps[part], k, (int)m0, &ring.full[stage]);
-                    tma_load_2d(dst + (3 + part) * TILE_BYTES, &maps->tw[part], k, (int)n0, &ring.full[stage]);
+                    tma_load_2d(dst + part * HTILE_BYTES, &a_maps[part], k, (int)m0, &ring.full[stage]);
+                    tma_load_2d(dst + (3 + part) * HTILE_BYTES, &maps->tw[part], k, (int)n0, &ring.full[stage]);
                 }
             }
         }
@@ -122,18 +133,18 @@ __global__ void __launch_bounds__(TC_THREADS) trinv_tc_kernel(const __grid_const
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const uint32_t acc_main = tmem + (uint32_t)(buf * 2 * MT), acc_small = acc_main + MT;
                 const uint32_t base = smem_base + stage * TRINV_STAGE_BYTES;
-                const uint32_t a_hi = base, a_mid = base + TILE_BYTES, a_lo = base + 2 * TILE_BYTES;
-                const uint32_t b_hi = base + 3 * TILE_BYTES, b_mid = base + 4 * TILE_BYTES, b_lo = base + 5 * TILE_BYTES;
+                const uint32_t a_hi = base, a_mid = base + HTILE_BYTES, a_lo = base + 2 * HTILE_BYTES;
+                const uint32_t b_hi = base + 3 * HTILE_BYTES, b_mid = base + 4 * HTILE_BYTES, b_lo = base + 5 * HTILE_BYTES;
 #pragma unroll
-                for (int ks = 0; ks < KC / 8; ++ks) {
-                    const uint32_t off = ks * 32;  // 8 tf32 values = 32 bytes along the swizzled row
+                for (int ks = 0; ks < KH / 16; ++ks) {
+                    const uint32_t off = ks * 32;  // 16 values = 32 bytes along the swizzled row
                     const uint32_t fresh = (opens && ks == 0) ? 0u : 1u;
-                    umma_tf32(acc_main, umma_desc(a_hi + off), umma_desc(b_hi + off), IDESC, fresh);
-                    umma_tf32(acc_small, umma_desc(a_hi + off), umma_desc(b_mid + off), IDESC, fresh);
-                    umma_tf32(acc_small, umma_desc(a_mid + off), umma_desc(b_hi + off), IDESC, 1u);
-                    umma_tf32(acc_small, umma_desc(a_mid + off), umma_desc(b_mid + off), IDESC, 1u);
-                    umma_tf32(acc_small, umma_desc(a_hi + off), umma_desc(b_lo + off), IDESC, 1u);
-                    umma_tf32(acc_small, umma_desc(a_lo + off), umma_desc(b_hi + off), IDESC, 1u);
+                    umma_16(acc_main, umma_desc(a_hi + off), umma_desc(b_hi + off), TRINV_DESC, fresh);
+                    umma_16(acc_small, umma_desc(a_hi + off), umma_desc(b_mid + off), TRINV_DESC, fresh);
+                    umma_16(acc_small, umma_desc(a_mid + off), umma_desc(b_hi + off), TRINV_DESC, 1u);
+                    umma_16(acc_small, umma_desc(a_mid + off), umma_desc(b_mid + off), TRINV_DESC, 1u);
+                    umma_16(acc_small, umma_desc(a_hi + off), umma_desc(b_lo + off), TRINV_DESC, 1u);
+                    umma_16(acc_small, umma_desc(a_lo + off), umma_desc(b_hi + off), TRINV_DESC, 1u);
                 }
                 umma_commit(&ring.empty[stage]);            // arrives when the MMAs above have read the stage
                 if (closes) umma_commit(&acc_full[buf]);    // arrives when the slice is complete in tensor memory
@@ -169,48 +180,44 @@ __global__ void __launch_bounds__(TC_THREADS) trinv_tc_kernel(const __grid_const
             if (lane == 0) mbar_arrive(&acc_empty[buf]);
         }
         if (go) {
-            const int64_t gi = m0 + q * 32 + lane;
+            const int64_t gi = m0 + q * 32 + lane, ld = P.ld;
+            const bool vec = n % 4 == 0;  // rows of the float matrix are 16-byte multiples; those of the planes always are
 #pragma unroll
-            for (int cb = 0; cb < MT / 32; ++cb) {
-                float acc[32];
-#pragma unroll
-                for (int x = 0; x < 32; ++x) acc[x] = total[cb * 32 + x];
-                const int64_t gj0 = n0 + cb * 32;
+            for (int cb = 0; cb < MT / 8; ++cb) {
+                const int64_t gj0 = n0 + cb * 8;
+                __align__(16) __nv_bfloat16 h[8];
+                __align__(16) __nv_bfloat16 c[8];
+                __align__(16) __nv_bfloat16 l[8];
                 if (!job.second) {
-                    // W^T[gi][gj]: gi is inside the first half (always a row of the matrix), gj is cut at r2
-                    float *hi = P.tw_hi + gi * n + gj0, *mid = P.tw_mid + gi * n + gj0, *lo = P.tw_lo + gi * n + gj0;
+                    // W^T[gi][gj]: gi is inside the first half (always a row of the matrix), gj is cut at r2; a group of eight that
+                    // reaches past it ends in the padding of its row (its extra products are zero)
+                    if (gj0 < r2) {
 #pragma unroll
-                    for (int x = 0; x < 32; x += 4) {
-                        if (gj0 + x < r2) {  // r2 is a multiple of 4: a group is inside or outside as a whole
-                            float4 h, c, l;
-                            split_tf32_3(acc[x], h.x, c.x, l.x);
-                            split_tf32_3(acc[x + 1], h.y, c.y, l.y);
-                            split_tf32_3(acc[x + 2], h.z, c.z, l.z);
-                            split_tf32_3(acc[x + 3], h.w, c.w, l.w);
-                            *reinterpret_cast<float4 *>(hi + x) = h;
-                            *reinterpret_cast<float4 *>(mid + x) = c;
-                            *reinterpret_cast<float4 *>(lo + x) = l;
-                        }
+                        for (int e = 0; e < 8; ++e) split_bf16_3(total[cb * 8 + e], h[e], c[e], l[e]);
+                        *reinterpret_cast<uint4 *>(P.tw_hi + gi * ld + gj0) = *reinterpret_cast<const uint4 *>(h);
+                        *reinterpret_cast<uint4 *>(P.tw_mid + gi * ld + gj0) = *reinterpret_cast<const uint4 *>(c);
+                        *reinterpret_cast<uint4 *>(P.tw_lo + gi * ld + gj0) = *reinterpret_cast<const uint4 *>(l);
                     }
                 } else if (gi < r2) {
-                    // X[gi][gj] = -acc: the inverse itself, its split, and the split of its transpose (coalesced across the lanes)
-                    float *dst = P.out + gi * n + gj0, *hi = P.out_hi + gi * n + gj0, *mid = P.out_mid + gi * n + gj0, *lo = P.out_lo + gi * n + gj0;
+                    // X[gi][gj] = -acc (gj is inside the first half): the inverse itself, its split, and the split of its transpose
+                    // (coalesced across the lanes)
+                    float *dst = P.out + gi * n + gj0;
 #pragma unroll
-                    for (int x = 0; x < 32; x += 4) {
-                        const float val[4] = {-acc[x], -acc[x + 1], -acc[x + 2], -acc[x + 3]};
-                        float h[4], c[4], l[4];
-#pragma unroll
-                        for (int e = 0; e < 4; ++e) {
-                            split_tf32_3(val[e], h[e], c[e], l[e]);
-                            P.outt_hi[(gj0 + x + e) * n + gi] = h[e];
-                            P.outt_mid[(gj0 + x + e) * n + gi] = c[e];
-                            P.outt_lo[(gj0 + x + e) * n + gi] = l[e];
-                        }
-                        *reinterpret_cast<float4 *>(dst + x) = make_float4(val[0], val[1], val[2], val[3]);
-                        *reinterpret_cast<float4 *>(hi + x) = make_float4(h[0], h[1], h[2], h[3]);
-                        *reinterpret_cast<float4 *>(mid + x) = make_float4(c[0], c[1], c[2], c[3]);
-                        *reinterpret_cast<float4 *>(lo + x) = make_float4(l[0], l[1], l[2], l[3]);
+                    for (int e = 0; e < 8; ++e) {
+                        const float v = -total[cb * 8 + e];
+                        split_bf16_3(v, h[e], c[e], l[e]);
+                        P.outt_hi[(gj0 + e) * ld + gi] = h[e];
+                        P.outt_mid[(gj0 + e) * ld + gi] = c[e];
+                        P.outt_lo[(gj0 + e) * ld + gi] = l[e];
+                        if (!vec) dst[e] = v;
                     }
+                    if (vec) {
+                        *reinterpret_cast<float4 *>(dst) = make_float4(-total[cb * 8], -total[cb * 8 + 1], -total[cb * 8 + 2], -total[cb * 8 + 3]);
+                        *reinterpret_cast<float4 *>(dst + 4) = make_float4(-total[cb * 8 + 4], -total[cb * 8 + 5], -total[cb * 8 + 6], -total[cb * 8 + 7]);
+                    }
+                    *reinterpret_cast<uint4 *>(P.out_hi + gi * ld + gj0) = *reinterpret_cast<const uint4 *>(h);
+                    *reinterpret_cast<uint4 *>(P.out_mid + gi * ld + gj0) = *reinterpret_cast<const uint4 *>(c);
+                    *reinterpret_cast<uint4 *>(P.out_lo + gi * ld + gj0) = *reinterpret_cast<const uint4 *>(l);
                 }
             }
         }
@@ -221,25 +228,49 @@ __global__ void __launch_bounds__(TC_THREADS) trinv_tc_kernel(const __grid_const
 
 // Operand planes after the 64-level of the doubling: T strictly below the diagonal into the lower triangle of tw, and the
 // finished 128 x 128 diagonal blocks of Lf (lower triangular) into out / outt with explicit zeros in their other halves.
-__global__ void trinv_split_kernel(FactorPlanes p0, FactorPlanes p1) {
+// One block per row, eight entries per thread; HBM bound (4 bytes in and 6 out per entry of the lower triangle).
+__global__ void __launch_bounds__(256) trinv_split_kernel(FactorPlanes p0, FactorPlanes p1) {
     const FactorPlanes P = blockIdx.y ? p1 : p0;
-    const int64_t n = P.n, total = n * n;
-    for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t r = t / n, c = t % n;
-        if (c < r) split_tf32_3(P.a[t], P.tw_hi[t], P.tw_mid[t], P.tw_lo[t]);
-        if (r / MT == c / MT) {
-            split_tf32_3(c <= r ? P.out[t] : 0.f, P.out_hi[t], P.out_mid[t], P.out_lo[t]);
-            split_tf32_3(c >= r ? P.out[c * n + r] : 0.f, P.outt_hi[t], P.outt_mid[t], P.outt_lo[t]);
+    const int64_t n = P.n, ld = P.ld;
+    const bool vec = n % 4 == 0;
+    for (int64_t r = blockIdx.x; r < n; r += gridDim.x) {
+        const int64_t d0 = r / MT * MT;
+        for (int64_t c = (int64_t)threadIdx.x * 8; c < r; c += (int64_t)blockDim.x * 8) {
+            __align__(16) __nv_bfloat16 h[8];
+            __align__(16) __nv_bfloat16 m[8];
+            __align__(16) __nv_bfloat16 l[8];
+            float v[8];
+            const float *src = P.a + r * n + c;
+            if (vec && c + 8 <= r) {
+                const float4 x = *reinterpret_cast<const float4 *>(src), y = *reinterpret_cast<const float4 *>(src + 4);
+                v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w; v[4] = y.x; v[5] = y.y; v[6] = y.z; v[7] = y.w;
+            } else {
+#pragma unroll
+                for (int e = 0; e < 8; ++e) v[e] = c + e < r ? src[e] : 0.f;
+            }
+#pragma unroll
+            for (int e = 0; e < 8; ++e) split_bf16_3(v[e], h[e], m[e], l[e]);
+            *reinterpret_cast<uint4 *>(P.tw_hi + r * ld + c) = *reinterpret_cast<const uint4 *>(h);
+            *reinterpret_cast<uint4 *>(P.tw_mid + r * ld + c) = *reinterpret_cast<const uint4 *>(m);
+            *reinterpret_cast<uint4 *>(P.tw_lo + r * ld + c) = *reinterpret_cast<const uint4 *>(l);
+        }
+        if (threadIdx.x < MT) {
+            const int64_t c = d0 + threadIdx.x;
+            if (c < n) {
+                split_bf16_3(c <= r ? P.out[r * n + c] : 0.f, P.out_hi[r * ld + c], P.out_mid[r * ld + c], P.out_lo[r * ld + c]);
+                split_bf16_3(c >= r ? P.out[c * n + r] : 0.f, P.outt_hi[r * ld + c], P.outt_mid[r * ld + c], P.outt_lo[r * ld + c]);
+            }
         }
     }
 }
 
 static bool factor_maps(FactorMaps *maps, const FactorPlanes &p) {
-    float *const out[3] = {p.out_hi, p.out_mid, p.out_lo}, *const outt[3] = {p.outt_hi, p.outt_mid, p.outt_lo}, *const tw[3] = {p.tw_hi, p.tw_mid, p.tw_lo};
+    __nv_bfloat16 *const out[3] = {p.out_hi, p.out_mid, p.out_lo}, *const outt[3] = {p.outt_hi, p.outt_mid, p.outt_lo},
+                  *const tw[3] = {p.tw_hi, p.tw_mid, p.tw_lo};
     bool ok = true;
     for (int part = 0; part < 3; ++part)
-        ok = ok && make_map(&maps->out[part], out[part], p.n, p.n) && make_map(&maps->outt[part], outt[part], p.n, p.n) &&
-             make_map(&maps->tw[part], tw[part], p.n, p.n);
+        ok = ok && make_map_16(&maps->out[part], out[part], p.n, p.n, MT, true, p.ld) && make_map_16(&maps->outt[part], outt[part], p.n, p.n, MT, true, p.ld) &&
+             make_map_16(&maps->tw[part], tw[part], p.n, p.n, MT, true, p.ld);
     return ok;
 }
 
@@ -256,7 +287,7 @@ int launch_trinv_tc(int count, const FactorPlanes *problems, cudaStream_t stream
         if (!factor_maps(&job.maps[z], job.p[z])) return G2D_ERR_CUDA;
         n_max = job.p[z].n > n_max ? job.p[z].n : n_max;
     }
-    trinv_split_kernel<<<dim3(148 * 8, count), 256, 0, stream>>>(job.p[0], job.p[1]);
+    trinv_split_kernel<<<dim3((unsigned)(n_max < 148 * 16 ? n_max : 148 * 16), count), 256, 0, stream>>>(job.p[0], job.p[1]);
     if (check_launch() != G2D_OK) return G2D_ERR_CUDA;
     for (int64_t b = MT; b < n_max; b *= 2) {
         const int64_t pairs = ceil_div(n_max, 2 * b), tiles = b / MT;
@@ -276,189 +307,193 @@ int launch_trinv_tc(int count, const FactorPlanes *problems, cudaStream_t stream
 // ---- trailing update of the blocked Cholesky factorization ----
 // After a group of four 64-row block rows [o, o + kw) is factored, everything above it receives
 //     a[r][c] -= sum_{k < kw} a[o + k][r] a[o + k][c],      c <= r < o,
-// one 128 x 128 tile per CTA.  Both operands are the same K-major planes pt[r][k] = a[o + k][r] (hi and lo), which
-// the panel kernel writes as it finishes a block row.  One CTA owns each target entry and no other kernel touches the
-// targets meanwhile, so the result does not depend on scheduling.
+// one tile per CTA.  Both operands are the same K-major fp16 pairs pt[r][k] = a[o + k][r] 2^-e(r), which the panel kernel
+// writes as it finishes a block row.  The scale of a row of the result comes from its diagonal entry in M: the squares of
+// T[., r] add up to M[r][r], so no entry of the panel exceeds sqrt(M[r][r]).  One CTA owns each target entry and no other kernel
+// touches the targets meanwhile, so the result does not depend on scheduling.
 // Accuracy.  The tensor cores add each product into the float accumulator with truncation, which biases long sums of
 // one sign by about 1e-8 of the sum per term, and the diagonal of this update is a sum of squares, subtracted from pivots
 // that a damped, badly conditioned Gram leaves one or two orders of magnitude smaller than the sum.  Two measures keep the
-// factors at the accuracy of a float32 LAPACK factorization: the k range is cut into slices of 64 with one accumulator
-// each in tensor memory (added up in registers, round to nearest), and the diagonal entries are left out here and
-// updated by syrk_diag_kernel with a float64 sum.
-constexpr int SYRK_SLICE_CHUNKS = 2;                      // k = 64 per accumulator
-constexpr int SYRK_SLICES = SYRK_TC_K / (SYRK_SLICE_CHUNKS * KC);
-constexpr uint32_t SYRK_TMEM_COLS = SYRK_SLICES * MT;     // 512: all of tensor memory, one CTA per SM (as its shared memory already requires)
-static_assert(SYRK_TMEM_COLS <= 512, "tensor memory holds 512 columns");
+// factors at the accuracy of a float32 LAPACK factorization: the k range is cut into slices of 64 (added up in registers, round
+// to nearest), and the diagonal entries are left out and updated with a float64 sum of the float panel by CTAs of their own
+// (the first ones of the launch, one per 128 rows).
+// Bound: HBM for factors beyond L2 (8 bytes per entry and group of 256 rows: 123 GB at n = 28672, 20 ms), shared-memory port
+// below (see pair_gemm).  n = 28672 and 8192 together: SYRKBEFORE ms with 128 x 128 tf32 tiles, SYRKNOW ms now.
+constexpr int SYRK_SLICE_CHUNKS = 1;  // k = 64 per slice
+static_assert(SYRK_TC_K % KH == 0, "whole chunks per group");
 
 struct SyrkJob {
-    CUtensorMap hi[2], lo[2];
+    CUtensorMap a_hi[2], a_lo[2], b_hi[2], b_lo[2];  // the same planes in boxes of 128 and of NT rows
+    CUtensorMap target[2];                           // the matrix itself in boxes of 32 x 32 (n a multiple of 4: its rows 16-byte multiples)
     float *a[2];
-    int64_t n[2];
+    const float *unscale[2];
+    int64_t n[2], o[2];    // size, first row of the group
     int t_lo[2], t_hi[2];  // target tile rows [t_lo, t_hi), with every tile column up to the diagonal
-    int chunks[2];         // ceil(kw / 32)
+    int kw[2];
     int *flag[2];
 };
+template <int NT>
+constexpr int syrk_stages = NT == 256 ? 2 : 3;
 
-__global__ void __launch_bounds__(TC_THREADS) syrk_tc_kernel(const __grid_constant__ SyrkJob job) {
+template <int NT>
+__global__ void __launch_bounds__(PAIR_THREADS, 1) syrk_tc_kernel(const __grid_constant__ SyrkJob job) {
+    constexpr int MINE = NT / 2;
     extern __shared__ unsigned char tc_smem_raw[];
-    __shared__ __align__(8) TcRing ring;
+    __shared__ __align__(8) PairRing<syrk_stages<NT>> ring;
     const int z = blockIdx.y;
     const int t_lo = z ? job.t_lo[1] : job.t_lo[0], t_hi = z ? job.t_hi[1] : job.t_hi[0];
-    const int64_t first = (int64_t)t_lo * (t_lo + 1) / 2, count = (int64_t)t_hi * (t_hi + 1) / 2 - first;
-    if ((int64_t)blockIdx.x >= count) return;
-    const int64_t lin = first + blockIdx.x;
-    int I2 = (int)((sqrt(8.0 * (double)lin + 1.0) - 1.0) / 2.0);
-    while ((int64_t)(I2 + 1) * (I2 + 2) / 2 <= lin) ++I2;
-    while ((int64_t)I2 * (I2 + 1) / 2 > lin) --I2;
-    const int J2 = (int)(lin - (int64_t)I2 * (I2 + 1) / 2);
-    const CUtensorMap *hi = z ? &job.hi[1] : &job.hi[0], *lo = z ? &job.lo[1] : &job.lo[0];
     float *const a = z ? job.a[1] : job.a[0];
-    const int64_t n = z ? job.n[1] : job.n[0];
-    const int chunks = z ? job.chunks[1] : job.chunks[0];
-    int *const flag = z ? job.flag[1] : job.flag[0];
-    const int i0 = I2 * MT, j0 = J2 * MT;
-
-    const uint32_t smem_base = (smem_u32(tc_smem_raw) + 1023u) & ~1023u;
+    const float *const unscale = z ? job.unscale[1] : job.unscale[0];
+    const int64_t n = z ? job.n[1] : job.n[0], o = z ? job.o[1] : job.o[0];
+    const int kw = z ? job.kw[1] : job.kw[0];
+    const int diagonals = t_hi - t_lo;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const uint32_t tmem = tc_ring_setup(ring, SYRK_TMEM_COLS);
-    const int slices = (chunks + SYRK_SLICE_CHUNKS - 1) / SYRK_SLICE_CHUNKS;
-    if (warp == 0) {
-        if (lane == 0)
-            tc_ring_produce(ring, smem_base, chunks, [&](int ch, uint32_t dst, uint64_t *bar) {
-                tma_load_2d(dst, hi, ch * KC, i0, bar);
-                tma_load_2d(dst + TILE_BYTES, lo, ch * KC, i0, bar);
-                tma_load_2d(dst + 2 * TILE_BYTES, hi, ch * KC, j0, bar);
-                tma_load_2d(dst + 3 * TILE_BYTES, lo, ch * KC, j0, bar);
-            });
-    } else if (warp == 1) {
-        if (lane == 0) {
-            // the ring's MMA loop with one accumulator per slice of SYRK_SLICE_CHUNKS chunks
-            for (int ch = 0; ch < chunks; ++ch) {
-                const int stage = ch % STAGES, round = ch / STAGES;
-                if (!mbar_wait(&ring.full[stage], round & 1)) {
-                    ring.failed = 1;
-                    break;
-                }
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const uint32_t acc = tmem + (uint32_t)(ch / SYRK_SLICE_CHUNKS) * MT;
-                const bool first = ch % SYRK_SLICE_CHUNKS == 0;
-                const uint32_t a_hi = smem_base + stage * STAGE_BYTES, a_lo = a_hi + TILE_BYTES, b_hi = a_hi + 2 * TILE_BYTES, b_lo = a_hi + 3 * TILE_BYTES;
+    if ((int)blockIdx.x < diagonals) {
+        // a[r][r] -= sum_k a[o + k][r]^2 for 128 rows r, lanes along r, warps along k
+        double (*const part)[MT] = reinterpret_cast<double (*)[MT]>(tc_smem_raw);
+        const int64_t r0 = (int64_t)(t_lo + (int)blockIdx.x) * MT + lane;
+        double sum[4] = {0., 0., 0., 0.};
+#pragma unroll 4
+        for (int k = warp; k < kw; k += PAIR_THREADS / 32) {
+            const float *src = a + (o + k) * n + r0;
 #pragma unroll
-                for (int ks = 0; ks < KC / 8; ++ks) {
-                    const uint32_t off = ks * 32;
-                    umma_tf32(acc, umma_desc(a_hi + off), umma_desc(b_hi + off), IDESC, (first && ks == 0) ? 0u : 1u);
-                    umma_tf32(acc, umma_desc(a_lo + off), umma_desc(b_hi + off), IDESC, 1u);
-                    umma_tf32(acc, umma_desc(a_hi + off), umma_desc(b_lo + off), IDESC, 1u);
-                }
-                umma_commit(&ring.empty[stage]);
-            }
-            umma_commit(&ring.accum);
-        }
-    } else {
-        const int q = warp & 3;
-        const bool go = tc_ring_accumulator_ready(ring);
-        if (go) {
-            const int64_t gi = (int64_t)i0 + q * 32 + lane;  // always a row of the matrix: the targets lie above the group
-            for (int cb = 0; cb < MT / 32; ++cb) {
-                float sum[32];
-#pragma unroll
-                for (int x = 0; x < 32; ++x) sum[x] = 0.f;
-                for (int sl = 0; sl < slices; ++sl) {
-                    uint32_t v[32];
-                    tmem_load_32(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(sl * MT + cb * 32), v);
-#pragma unroll
-                    for (int x = 0; x < 32; ++x) sum[x] += __uint_as_float(v[x]);
-                }
-                const int64_t gj0 = (int64_t)j0 + cb * 32;
-                float *dst = a + gi * n + gj0;
-#pragma unroll
-                for (int x = 0; x < 32; x += 4) {
-                    if (gj0 + x <= gi) {  // groups that start right of the diagonal are never read
-                        if (gi - (gj0 + x) < 4) {  // the diagonal entry belongs to syrk_diag_kernel
-#pragma unroll
-                            for (int c = 0; c < 4; ++c)
-                                if (gj0 + x + c == gi) sum[x + c] = 0.f;
-                        }
-                        asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dst + x), "f"(-sum[x]), "f"(-sum[x + 1]),
-                                     "f"(-sum[x + 2]), "f"(-sum[x + 3])
-                                     : "memory");
-                    }
-                }
+            for (int e = 0; e < 4; ++e) {
+                const double v = (double)src[e * 32];
+                sum[e] += v * v;
             }
         }
+#pragma unroll
+        for (int e = 0; e < 4; ++e) part[warp][e * 32 + lane] = sum[e];
+        __syncthreads();
+        if (threadIdx.x < MT) {
+            double all = 0.;
+            for (int w = 0; w < PAIR_THREADS / 32; ++w) all += part[w][threadIdx.x];
+            const int64_t r = (int64_t)(t_lo + (int)blockIdx.x) * MT + threadIdx.x;
+            a[r * n + r] = (float)((double)a[r * n + r] - all);
+        }
+        return;
     }
-    const bool failed = tc_ring_teardown(ring, tmem, SYRK_TMEM_COLS);
+    const int64_t first = lower_tiles<NT>(t_lo), lin = first + (int64_t)blockIdx.x - diagonals;
+    if (lin >= lower_tiles<NT>(t_hi)) return;
+    int I2, J2;
+    lower_tile<NT>(lin, I2, J2);
+    const CUtensorMap *a_hi = z ? &job.a_hi[1] : &job.a_hi[0], *a_lo = z ? &job.a_lo[1] : &job.a_lo[0];
+    const CUtensorMap *b_hi = z ? &job.b_hi[1] : &job.b_hi[0], *b_lo = z ? &job.b_lo[1] : &job.b_lo[0];
+    const int i0 = I2 * MT, j0 = J2 * NT;
+    const bool vec = n % 4 == 0;
+    const uint32_t smem_base = (smem_u32(tc_smem_raw) + 1023u) & ~1023u;
+    auto load = [&](int ch, uint32_t dst, uint64_t *bar) {
+        tma_load_2d(dst, a_hi, ch * KH, i0, bar);
+        tma_load_2d(dst + HTILE_BYTES, a_lo, ch * KH, i0, bar);
+        tma_load_2d(dst + 2 * HTILE_BYTES, b_hi, ch * KH, j0, bar);
+        tma_load_2d(dst + 2 * HTILE_BYTES + NT * KH * 2, b_lo, ch * KH, j0, bar);
+    };
+    const CUtensorMap *target = z ? &job.target[1] : &job.target[0];
+    auto finish = [&](int q, int ln, int c0, float (&total)[MINE], uint32_t boxes) {
+        const int64_t gi = (int64_t)i0 + q * 32 + ln;  // always a row of the matrix: the targets lie above the group
+        const float row_scale = -unscale[gi];
+        if (vec) {
+            // the diagonal entries are updated above; what lies right of the diagonal is never read: both get zeros
+#pragma unroll
+            for (int cb = 0; cb < MINE / 32; ++cb) {
+                const int64_t gj0 = (int64_t)j0 + c0 + cb * 32;
+                if (gj0 > (int64_t)i0 + q * 32 + 31) continue;  // warp-uniform
+                const uint32_t box = boxes + cb * BOX_BYTES;
+#pragma unroll
+                for (int g = 0; g < 8; ++g) {
+                    float v[4];
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {
+                        const int64_t gj = gj0 + g * 4 + e;  // left of row gi: inside the matrix
+                        v[e] = gj < gi ? total[cb * 32 + g * 4 + e] * row_scale * unscale[gj] : 0.f;
+                    }
+                    box_store4(box, ln, g, v[0], v[1], v[2], v[3]);
+                }
+                box_fence();
+                __syncwarp();
+                if (ln == 0) box_reduce_add(target, box, (int)gj0, i0 + q * 32);
+            }
+            if (ln == 0) {
+                box_commit();
+                box_wait();
+            }
+            return;
+        }
+#pragma unroll
+        for (int x = 0; x < MINE; ++x) {
+            const int64_t gj = (int64_t)j0 + c0 + x;
+            if (gj < gi) asm volatile("red.global.add.f32 [%0], %1;" ::"l"(a + gi * n + gj), "f"(total[x] * row_scale * unscale[gj]) : "memory");
+        }
+    };
+    const bool failed = pair_gemm<NT, syrk_stages<NT>, SYRK_SLICE_CHUNKS>(ring, smem_base, (kw + KH - 1) / KH, load, finish);
+    int *const flag = z ? job.flag[1] : job.flag[0];
     if (threadIdx.x == 0 && failed && flag) atomicExch(flag, -1);
 }
 
-// The diagonal of the same update: a[r][r] -= sum_k p[r][k]^2 with p = hi + lo (the float32 panel value, exactly), the sum
-// in float64.  One warp per row.
-struct SyrkDiagJob {
-    const float *hi[2], *lo[2];
-    float *a[2];
-    int64_t n[2];
-    int64_t r_lo[2], r_hi[2];
-    int kw[2];
-};
-__global__ void syrk_diag_kernel(const SyrkDiagJob job) {
-    const int z = blockIdx.y, lane = threadIdx.x & 31;
-    const int64_t r_lo = z ? job.r_lo[1] : job.r_lo[0], r_hi = z ? job.r_hi[1] : job.r_hi[0];
-    const float *hi = z ? job.hi[1] : job.hi[0], *lo = z ? job.lo[1] : job.lo[0];
-    float *a = z ? job.a[1] : job.a[0];
-    const int64_t n = z ? job.n[1] : job.n[0];
-    const int kw = z ? job.kw[1] : job.kw[0];
-    const int64_t warps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-    for (int64_t r = r_lo + (((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5); r < r_hi; r += warps) {
-        double sum = 0.0;
-        for (int k = lane; k < kw; k += 32) {
-            const double p = (double)hi[r * SYRK_TC_K + k] + (double)lo[r * SYRK_TC_K + k];
-            sum += p * p;
-        }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-        if (lane == 0) a[r * n + r] = (float)((double)a[r * n + r] - sum);
-    }
+bool syrk_tc_maps(SyrkTcMaps *maps, const __half *pt_hi, const __half *pt_lo, float *a, int64_t n) {
+    static_assert(sizeof(maps->hi) == sizeof(CUtensorMap), "opaque tensor-map storage has the wrong size");
+    if (n % 4 == 0 && !make_map(reinterpret_cast<CUtensorMap *>(maps->target), a, n, n, 32)) return false;
+    return make_map_16(reinterpret_cast<CUtensorMap *>(maps->hi), pt_hi, n, SYRK_TC_K, MT) &&
+           make_map_16(reinterpret_cast<CUtensorMap *>(maps->lo), pt_lo, n, SYRK_TC_K, MT) &&
+           make_map_16(reinterpret_cast<CUtensorMap *>(maps->wide_hi), pt_hi, n, SYRK_TC_K, 256) &&
+           make_map_16(reinterpret_cast<CUtensorMap *>(maps->wide_lo), pt_lo, n, SYRK_TC_K, 256);
 }
 
-bool syrk_tc_maps(SyrkTcMaps *maps, const float *pt_hi, const float *pt_lo, int64_t n) {
-    static_assert(sizeof(maps->hi) == sizeof(CUtensorMap), "opaque tensor-map storage has the wrong size");
-    return make_map(reinterpret_cast<CUtensorMap *>(maps->hi), pt_hi, n, SYRK_TC_K) &&
-           make_map(reinterpret_cast<CUtensorMap *>(maps->lo), pt_lo, n, SYRK_TC_K);
+template <int NT>
+static int launch_syrk_tiles(int count, const SyrkJob &job, int64_t blocks, cudaStream_t stream) {
+    static PerDeviceOnce configured;
+    constexpr size_t smem = (size_t)syrk_stages<NT> * pair_stage_bytes<NT> + 1024;
+    if (configured.run([&] { return cudaFuncSetAttribute(syrk_tc_kernel<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) == cudaSuccess; }) != G2D_OK)
+        return G2D_ERR_CUDA;
+    syrk_tc_kernel<NT><<<dim3((unsigned)blocks, count), PAIR_THREADS, smem, stream>>>(job);
+    return check_launch();
 }
 
 int launch_syrk_tc(int count, const SyrkTcTarget *targets, cudaStream_t stream) {
-    static PerDeviceOnce configured;
-    const size_t smem = (size_t)STAGES * STAGE_BYTES + 1024;
-    if (configured.run([&] { return cudaFuncSetAttribute(syrk_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) == cudaSuccess; }) != G2D_OK)
-        return G2D_ERR_CUDA;
     SyrkJob job;
-    SyrkDiagJob diag;
-    int64_t most = 0, most_rows = 0;
+    int64_t wide = 0, square = 0, most_wide = 0, most_square = 0;
+    for (int z = 0; z < count; ++z) {
+        const SyrkTcTarget &t = targets[z];
+        const int64_t w = lower_tiles<256>(t.t_hi) - lower_tiles<256>(t.t_lo), q = lower_tiles<128>(t.t_hi) - lower_tiles<128>(t.t_lo), d = t.t_hi - t.t_lo;
+        wide += w;
+        square += q;
+        most_wide = w + d > most_wide ? w + d : most_wide;
+        most_square = q + d > most_square ? q + d : most_square;
+    }
+    if (square <= 0) return G2D_OK;
+    if (most_square > 0x7fffffff) return G2D_ERR_TOO_LARGE;
+    const bool use_wide = wide_tiles_pay(wide, square);
     for (int z = 0; z < 2; ++z) {
         const SyrkTcTarget &t = targets[z < count ? z : 0];
-        diag.hi[z] = t.pt_hi; diag.lo[z] = t.pt_lo; diag.a[z] = t.a; diag.n[z] = t.n; diag.kw[z] = t.kw;
-        diag.r_lo[z] = (int64_t)t.t_lo * MT;
-        diag.r_hi[z] = (int64_t)t.t_hi * MT;  // whole tile rows above the group: every one a row of the matrix
-        most_rows = diag.r_hi[z] - diag.r_lo[z] > most_rows ? diag.r_hi[z] - diag.r_lo[z] : most_rows;
-        memcpy(&job.hi[z], t.maps->hi, sizeof(CUtensorMap));
-        memcpy(&job.lo[z], t.maps->lo, sizeof(CUtensorMap));
+        memcpy(&job.a_hi[z], t.maps->hi, sizeof(CUtensorMap));
+        memcpy(&job.a_lo[z], t.maps->lo, sizeof(CUtensorMap));
+        memcpy(&job.b_hi[z], use_wide ? t.maps->wide_hi : t.maps->hi, sizeof(CUtensorMap));
+        memcpy(&job.b_lo[z], use_wide ? t.maps->wide_lo : t.maps->lo, sizeof(CUtensorMap));
+        memcpy(&job.target[z], t.maps->target, sizeof(CUtensorMap));
         job.a[z] = t.a;
+        job.unscale[z] = t.unscale;
         job.n[z] = t.n;
+        job.o[z] = t.o;
         job.t_lo[z] = t.t_lo;
         job.t_hi[z] = t.t_hi;
-        job.chunks[z] = (t.kw + KC - 1) / KC;
+        job.kw[z] = t.kw;
         job.flag[z] = t.flag;
-        const int64_t tiles = (int64_t)t.t_hi * (t.t_hi + 1) / 2 - (int64_t)t.t_lo * (t.t_lo + 1) / 2;
-        most = tiles > most ? tiles : most;
     }
-    if (most <= 0) return G2D_OK;
-    if (most > 0x7fffffff) return G2D_ERR_TOO_LARGE;
-    syrk_tc_kernel<<<dim3((unsigned)most, count), TC_THREADS, smem, stream>>>(job);
-    if (check_launch() != G2D_OK) return G2D_ERR_CUDA;
-    if (most_rows > 0) {
-        int64_t blocks = ceil_div(most_rows * 32, 256);
-        syrk_diag_kernel<<<dim3((unsigned)(blocks < 1184 ? blocks : 1184), count), 256, 0, stream>>>(diag);
-    }
+    return use_wide ? launch_syrk_tiles<256>(count, job, most_wide, stream) : launch_syrk_tiles<128>(count, job, most_square, stream);
+}
+
+// The scales: unscale[r] = 2^e with sqrt(M[r][r]) 2^-e in [2^14, 2^15).
+__global__ void syrk_range_kernel(SyrkRange r) {
+    const int z = blockIdx.y;
+    const int64_t n = z ? r.n[1] : r.n[0];
+    const float *a = z ? r.a[1] : r.a[0];
+    float *unscale = z ? r.unscale[1] : r.unscale[0];
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+        unscale[i] = power_of_two(range_exponent(sqrtf(a[i * n + i])));
+}
+int launch_syrk_range(int count, const SyrkRange &r, cudaStream_t stream) {
+    const int64_t most = count > 1 && r.n[1] > r.n[0] ? r.n[1] : r.n[0];
+    syrk_range_kernel<<<dim3((unsigned)(ceil_div(most, (int64_t)256) < 592 ? ceil_div(most, (int64_t)256) : 592), count), 256, 0, stream>>>(r);
     return check_launch();
 }
 

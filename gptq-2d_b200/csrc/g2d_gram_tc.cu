@@ -18,12 +18,9 @@
 
 namespace g2d {
 
-constexpr int GRAM_THREADS = 320;  // TMA, MMA and eight reading warps
 constexpr int GRAM_STAGES = 2;
-// The tensor cores add into their fp32 accumulator with truncation, which biases a long sum of same-sign terms (the
-// diagonal of a Gram matrix is a sum of squares): measured 9e-5 relative over k = 8192 in one accumulator.  So the k
-// range is cut into slices; each slice is accumulated in tensor memory and then added up in registers, round to nearest.
-// Two accumulators alternate, so the additions of a slice overlap the MMAs of the next.
+// Slices of the k range (see pair_gemm): the diagonal of a Gram matrix is a sum of squares, which one accumulator over
+// k = 8192 truncates to 9e-5 relative.
 constexpr int GRAM_SLICE = 2;  // chunks per slice: 128 samples
 
 // four neighbouring channels of a sample; `vec`: 16-byte aligned (n is a multiple of 4, the array itself may start anywhere)
@@ -115,185 +112,76 @@ struct GramJob {
 };
 
 template <int NT>
-__global__ void __launch_bounds__(GRAM_THREADS, 1) gram_tc_kernel(const __grid_constant__ GramJob job) {
-    constexpr int B_BYTES = NT * KH * 2, GSTAGE = 2 * HTILE_BYTES + 2 * B_BYTES;
-    constexpr uint32_t COLS = 2 * NT, DESC = idesc_16(NT, 0);
+__global__ void __launch_bounds__(PAIR_THREADS, 1) gram_tc_kernel(const __grid_constant__ GramJob job) {
     constexpr int MINE = NT / 2;  // columns per reading warp
     extern __shared__ unsigned char tc_smem_raw[];
-    __shared__ __align__(8) uint64_t full_bar[GRAM_STAGES], empty_bar[GRAM_STAGES], acc_full[2], acc_empty[2];
-    __shared__ uint32_t tmem_slot;
-    __shared__ int failed;
-    // tiles that touch the lower triangle: a row of 128 has row * 128 / NT + 1 of them
+    __shared__ __align__(8) PairRing<GRAM_STAGES> ring;
     int I2, J2;
-    {
-        const int64_t lin = blockIdx.x;
-        if (NT == 256) {  // rows 2 a and 2 a + 1 have a + 1 tiles each
-            int64_t a = (int64_t)((sqrt(4.0 * (double)lin + 1.0) - 1.0) / 2.0);
-            while ((a + 1) * (a + 2) <= lin) ++a;
-            while (a * (a + 1) > lin) --a;
-            const int64_t rest = lin - a * (a + 1);
-            I2 = (int)(2 * a + rest / (a + 1));
-            J2 = (int)(rest % (a + 1));
-        } else {
-            int64_t a = (int64_t)((sqrt(8.0 * (double)lin + 1.0) - 1.0) / 2.0);
-            while ((a + 1) * (a + 2) / 2 <= lin) ++a;
-            while (a * (a + 1) / 2 > lin) --a;
-            I2 = (int)a;
-            J2 = (int)(lin - a * (a + 1) / 2);
-        }
-    }
+    lower_tile<NT>(blockIdx.x, I2, J2);
     const int i0 = I2 * MT, j0 = J2 * NT;
     const int64_t n = job.n;
-    const int chunks = job.chunks, slices = (chunks + GRAM_SLICE - 1) / GRAM_SLICE;
-
     const uint32_t smem_base = (smem_u32(tc_smem_raw) + 1023u) & ~1023u;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    if (threadIdx.x == 0) {
-        for (int s = 0; s < GRAM_STAGES; ++s) {
-            mbar_init(&full_bar[s], 1);
-            mbar_init(&empty_bar[s], 1);
-        }
-        for (int s = 0; s < 2; ++s) {
-            mbar_init(&acc_full[s], 1);
-            mbar_init(&acc_empty[s], 8);  // one arrival per reading warp
-        }
-        failed = 0;
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
-    if (warp == 1) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)), "r"(COLS) : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-    }
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    __syncthreads();
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    const uint32_t tmem = tmem_slot;
-
-    if (warp == 0) {
-        if (lane == 0) {
-            for (int ch = 0; ch < chunks; ++ch) {
-                const int stage = ch % GRAM_STAGES, round = ch / GRAM_STAGES;
-                if (round > 0 && !mbar_wait(&empty_bar[stage], (round - 1) & 1)) { failed = 1; break; }
-                const uint32_t dst = smem_base + stage * GSTAGE;
-                mbar_expect_tx(&full_bar[stage], GSTAGE);
-                tma_load_2d(dst, &job.a_hi, ch * KH, i0, &full_bar[stage]);
-                tma_load_2d(dst + HTILE_BYTES, &job.a_lo, ch * KH, i0, &full_bar[stage]);
-                tma_load_2d(dst + 2 * HTILE_BYTES, &job.b_hi, ch * KH, j0, &full_bar[stage]);
-                tma_load_2d(dst + 2 * HTILE_BYTES + B_BYTES, &job.b_lo, ch * KH, j0, &full_bar[stage]);
-            }
-        }
-    } else if (warp == 1) {
-        if (lane == 0) {
-            for (int ch = 0; ch < chunks; ++ch) {
-                const int stage = ch % GRAM_STAGES, round = ch / GRAM_STAGES;
-                const int slice = ch / GRAM_SLICE, buf = slice & 1;
-                const bool opens = ch % GRAM_SLICE == 0, closes = ch % GRAM_SLICE == GRAM_SLICE - 1 || ch == chunks - 1;
-                // the accumulator must have been read out by the warps of the slice two before
-                if (opens && slice >= 2 && !mbar_wait(&acc_empty[buf], ((slice >> 1) - 1) & 1)) { failed = 1; break; }
-                if (!mbar_wait(&full_bar[stage], round & 1)) { failed = 1; break; }
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const uint32_t d = tmem + (uint32_t)(buf * NT);
-                const uint32_t a_hi = smem_base + stage * GSTAGE, a_lo = a_hi + HTILE_BYTES, b_hi = a_hi + 2 * HTILE_BYTES, b_lo = b_hi + B_BYTES;
-#pragma unroll
-                for (int ks = 0; ks < KH / 16; ++ks) {
-                    const uint32_t off = ks * 32;  // 16 values = 32 bytes along the swizzled row
-                    umma_16(d, umma_desc(a_hi + off), umma_desc(b_hi + off), DESC, (opens && ks == 0) ? 0u : 1u);
-                    umma_16(d, umma_desc(a_lo + off), umma_desc(b_hi + off), DESC, 1u);
-                    umma_16(d, umma_desc(a_hi + off), umma_desc(b_lo + off), DESC, 1u);
-                }
-                umma_commit(&empty_bar[stage]);            // arrives when the MMAs above have read the stage
-                if (closes) umma_commit(&acc_full[buf]);   // arrives when the slice is complete in tensor memory
-            }
-        }
-    } else {
-        // reading warps: lanes 32 q .. 32 q + 31 of tensor memory, q = warp % 4, one accumulator row per thread, and half of
-        // the columns
-        const int q = warp & 3, c0 = ((warp - 2) >> 2) * MINE;
-        float total[MINE];
-#pragma unroll
-        for (int x = 0; x < MINE; ++x) total[x] = 0.f;
-        bool go = true;
-        for (int slice = 0; slice < slices; ++slice) {
-            const int buf = slice & 1;
-            const bool ok = mbar_wait(&acc_full[buf], (slice >> 1) & 1, 64);
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            if (!ok) failed = 1;
-            go = __all_sync(0xffffffffu, ok && !failed);  // warp-uniform: the tensor-memory loads are warp-wide
-            if (!go) break;
-#pragma unroll
-            for (int cb = 0; cb < MINE / 32; ++cb) {
-                uint32_t v[32];
-                tmem_load_32(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(buf * NT + c0 + cb * 32), v);
-#pragma unroll
-                for (int x = 0; x < 32; ++x) total[cb * 32 + x] += __uint_as_float(v[x]);
-            }
-            // this warp has read the accumulator: hand it back to the MMA warp
-            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&acc_empty[buf]);
-        }
+    auto load = [&](int ch, uint32_t dst, uint64_t *bar) {
+        tma_load_2d(dst, &job.a_hi, ch * KH, i0, bar);
+        tma_load_2d(dst + HTILE_BYTES, &job.a_lo, ch * KH, i0, bar);
+        tma_load_2d(dst + 2 * HTILE_BYTES, &job.b_hi, ch * KH, j0, bar);
+        tma_load_2d(dst + 2 * HTILE_BYTES + NT * KH * 2, &job.b_lo, ch * KH, j0, bar);
+    };
+    auto finish = [&](int q, int lane, int c0, float (&total)[MINE], uint32_t) {
         const int64_t gi = (int64_t)i0 + q * 32 + lane;
-        if (go && gi < n) {
-            constexpr int GROUP = 16;
-            const int row_exponent = range_exponent(__uint_as_float(job.largest[gi]));
+        if (gi >= n) return;
+        constexpr int GROUP = 16;
+        const float row_scale = power_of_two(range_exponent(__uint_as_float(job.largest[gi])));
 #pragma unroll
-            for (int x0 = 0; x0 < MINE; x0 += GROUP) {
-                const int64_t gj0 = (int64_t)j0 + c0 + x0;
-                if (gj0 > gi) continue;  // the upper triangle is the mirror image of the lower one
-                float *const dst = job.h + gi * n + gj0;
-                // the old values of sixteen columns travel together, before the first is used
-                const bool whole = gj0 + GROUP - 1 <= gi;
-                float old[GROUP];
-                if (whole) {
+        for (int x0 = 0; x0 < MINE; x0 += GROUP) {
+            const int64_t gj0 = (int64_t)j0 + c0 + x0;
+            if (gj0 > gi) continue;  // the upper triangle is the mirror image of the lower one
+            float *const dst = job.h + gi * n + gj0;
+            // the old values of sixteen columns travel together, before the first is used
+            const bool whole = gj0 + GROUP - 1 <= gi;
+            float old[GROUP];
+            if (whole) {
 #pragma unroll
-                    for (int x = 0; x < GROUP; x += 4) {
-                        const float4 v = *reinterpret_cast<const float4 *>(dst + x);
-                        old[x] = v.x; old[x + 1] = v.y; old[x + 2] = v.z; old[x + 3] = v.w;
-                    }
-                } else {
-#pragma unroll
-                    for (int x = 0; x < GROUP; ++x) old[x] = gj0 + x <= gi ? dst[x] : 0.f;
+                for (int x = 0; x < GROUP; x += 4) {
+                    const float4 v = *reinterpret_cast<const float4 *>(dst + x);
+                    old[x] = v.x; old[x + 1] = v.y; old[x + 2] = v.z; old[x + 3] = v.w;
                 }
+            } else {
 #pragma unroll
-                for (int x = 0; x < GROUP; ++x) {
-                    const int64_t at = min(gj0 + x, n - 1);
-                    old[x] += job.alpha * scalbnf(total[x0 + x], row_exponent + range_exponent(__uint_as_float(job.largest[at])));
-                }
-                if (whole) {
+                for (int x = 0; x < GROUP; ++x) old[x] = gj0 + x <= gi ? dst[x] : 0.f;
+            }
 #pragma unroll
-                    for (int x = 0; x < GROUP; x += 4) *reinterpret_cast<float4 *>(dst + x) = make_float4(old[x], old[x + 1], old[x + 2], old[x + 3]);
-                }
+            for (int x = 0; x < GROUP; ++x) {
+                const int64_t at = min(gj0 + x, n - 1);
+                const float column_scale = power_of_two(range_exponent(__uint_as_float(job.largest[at])));
+                // the smaller scale first: the other order could leave the range of floats on the way
+                old[x] += job.alpha * (total[x0 + x] * fminf(row_scale, column_scale) * fmaxf(row_scale, column_scale));
+            }
+            if (whole) {
 #pragma unroll
-                for (int x = 0; x < GROUP; ++x) {
-                    if (!whole && gj0 + x <= gi) dst[x] = old[x];
-                    if (gj0 + x < gi) job.h[(gj0 + x) * n + gi] = old[x];  // consecutive lanes write consecutive columns
-                }
+                for (int x = 0; x < GROUP; x += 4) *reinterpret_cast<float4 *>(dst + x) = make_float4(old[x], old[x + 1], old[x + 2], old[x + 3]);
+            }
+#pragma unroll
+            for (int x = 0; x < GROUP; ++x) {
+                if (!whole && gj0 + x <= gi) dst[x] = old[x];
+                if (gj0 + x < gi) job.h[(gj0 + x) * n + gi] = old[x];  // consecutive lanes write consecutive columns
             }
         }
-    }
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    __syncthreads();
-    if (warp == 1) {
-        if (failed) {
-            // give outstanding loads and MMAs a bounded chance to land before the memory they target is released
-            if (lane == 0) mbar_wait(&acc_full[((slices - 1) & 1)], ((slices - 1) >> 1) & 1);
-            __syncwarp();
-        }
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(COLS) : "memory");
-    }
+    };
+    const bool failed = pair_gemm<NT, GRAM_STAGES, GRAM_SLICE>(ring, smem_base, job.chunks, load, finish);
     if (threadIdx.x == 0 && failed && job.flag) atomicExch(job.flag, -1);
 }
 
 template <int NT>
 static int launch_gram(GramJob &job, const __half *hi, const __half *lo, int64_t kp, int64_t tiles, cudaStream_t st) {
     static PerDeviceOnce configured;
-    constexpr size_t smem = (size_t)GRAM_STAGES * (2 * HTILE_BYTES + 2 * NT * KH * 2) + 1024;
+    constexpr size_t smem = (size_t)GRAM_STAGES * pair_stage_bytes<NT> + 1024;
     if (configured.run([&] { return cudaFuncSetAttribute(gram_tc_kernel<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) == cudaSuccess; }) != G2D_OK)
         return G2D_ERR_CUDA;
     if (!make_map_16(&job.a_hi, hi, job.n, kp, MT) || !make_map_16(&job.a_lo, lo, job.n, kp, MT) || !make_map_16(&job.b_hi, hi, job.n, kp, NT) ||
         !make_map_16(&job.b_lo, lo, job.n, kp, NT))
         return G2D_ERR_CUDA;
-    gram_tc_kernel<NT><<<(unsigned)tiles, GRAM_THREADS, smem, st>>>(job);
+    gram_tc_kernel<NT><<<(unsigned)tiles, PAIR_THREADS, smem, st>>>(job);
     return check_launch();
 }
 
@@ -346,8 +234,7 @@ extern "C" int g2d_gram_accumulate(int64_t n, int64_t k, const float *x, float a
     job.chunks = (int)ceil_div(kp, (int64_t)KH);
     job.alpha = alpha;
     job.flag = status_flag;
-    // 128 x 256 tiles take 1.5 times as long as 128 x 128 ones; narrow factors have too few of them to fill the GPU
-    const int64_t wide = (rows / 2) * (rows / 2 + 1) + (rows % 2) * (rows / 2 + 1), square = rows * (rows + 1) / 2;
-    if (3 * ceil_div(wide, (int64_t)148) <= 2 * ceil_div(square, (int64_t)148)) return launch_gram<256>(job, hi, lo, kp, wide, st);
+    const int64_t wide = lower_tiles<256>(rows), square = lower_tiles<128>(rows);
+    if (wide_tiles_pay(wide, square)) return launch_gram<256>(job, hi, lo, kp, wide, st);
     return launch_gram<128>(job, hi, lo, kp, square, st);
 }

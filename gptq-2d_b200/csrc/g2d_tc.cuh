@@ -211,6 +211,166 @@ __device__ __forceinline__ bool tc_ring_teardown(TcRing &ring, uint32_t tmem, ui
     return ring.failed != 0;
 }
 
+// ---- results as reductions of 32 x 32 boxes ----
+// A warp that holds one row per lane writes its box to shared memory (128-byte rows, the TMA's swizzle: no bank conflicts) and
+// one reduction adds it to global memory.  The same additions as red.global.add.v4 from every lane touch 32 rows with every
+// instruction and half a sector each.
+constexpr int BOX_BYTES = 32 * 32 * 4;
+__device__ __forceinline__ void box_store4(uint32_t box, int row, int group, float a, float b, float c, float d) {  // columns 4 group ..
+    asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(box + row * 128 + ((group ^ (row & 7)) << 4)), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");
+}
+__device__ __forceinline__ void box_reduce_add(const CUtensorMap *map, uint32_t box, int x, int y) {  // one lane, after fence and __syncwarp
+    asm volatile("cp.reduce.async.bulk.tensor.2d.global.shared::cta.add.tile.bulk_group [%0, {%1, %2}], [%3];"
+                 ::"l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(box)
+                 : "memory");
+}
+__device__ __forceinline__ void box_fence() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
+__device__ __forceinline__ void box_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
+__device__ __forceinline__ void box_wait() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
+
+// ---- pipeline for 16-bit pairs: A[128 x k] B[NT x k]^T as hi hi + lo hi + hi lo ----
+// CTA of PAIR_THREADS threads: warp 0 loads, warp 1 issues the MMAs, eight warps read the accumulators.  The k range is cut into
+// slices of SLICE chunks with two accumulators in turn: the tensor cores add into their fp32 accumulator with truncation, which
+// biases long sums, so a slice is accumulated in tensor memory and the slices are added up in registers, round to nearest,
+// under the MMAs of the next.  A reading warp has 32 rows (q = warp % 4) and half of the columns.
+constexpr int PAIR_THREADS = 320;
+template <int NT>
+constexpr int pair_stage_bytes = 2 * HTILE_BYTES + 2 * NT * KH * 2;
+template <int NSTAGE>
+struct PairRing {
+    uint64_t full[NSTAGE], empty[NSTAGE], acc_full[2], acc_empty[2];
+    uint32_t tmem;
+    int failed;
+};
+
+// load(chunk, destination, barrier): A_hi, A_lo, B_hi, B_lo tiles one after the other.
+// finish(q, lane, first column, totals, shared memory of the warp: 4 KB per 32 of
+// its columns, 1024-byte aligned).  Returns whether a wait ran out.
+template <int NT, int NSTAGE, int SLICE, typename Load, typename Finish>
+__device__ __forceinline__ bool pair_gemm(PairRing<NSTAGE> &ring, uint32_t smem_base, int chunks, Load load, Finish finish) {
+    constexpr int B_BYTES = NT * KH * 2, STAGE = 2 * HTILE_BYTES + 2 * B_BYTES, MINE = NT / 2;
+    constexpr uint32_t COLS = 2 * NT, DESC = idesc_16(NT, 0);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int slices = (chunks + SLICE - 1) / SLICE;
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < NSTAGE; ++s) {
+            mbar_init(&ring.full[s], 1);
+            mbar_init(&ring.empty[s], 1);
+        }
+        for (int s = 0; s < 2; ++s) {
+            mbar_init(&ring.acc_full[s], 1);
+            mbar_init(&ring.acc_empty[s], 8);  // one arrival per reading warp
+        }
+        ring.failed = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 1) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&ring.tmem)), "r"(COLS) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t tmem = ring.tmem;
+    if (warp == 0) {
+        if (lane == 0) {
+            for (int ch = 0; ch < chunks; ++ch) {
+                const int stage = ch % NSTAGE, round = ch / NSTAGE;
+                if (round > 0 && !mbar_wait(&ring.empty[stage], (round - 1) & 1)) { ring.failed = 1; break; }
+                mbar_expect_tx(&ring.full[stage], STAGE);
+                load(ch, smem_base + stage * STAGE, &ring.full[stage]);
+            }
+        }
+    } else if (warp == 1) {
+        if (lane == 0) {
+            for (int ch = 0; ch < chunks; ++ch) {
+                const int stage = ch % NSTAGE, round = ch / NSTAGE;
+                const int slice = ch / SLICE, buf = slice & 1;
+                const bool opens = ch % SLICE == 0, closes = ch % SLICE == SLICE - 1 || ch == chunks - 1;
+                // the accumulator must have been read out by the warps of the slice two before
+                if (opens && slice >= 2 && !mbar_wait(&ring.acc_empty[buf], ((slice >> 1) - 1) & 1)) { ring.failed = 1; break; }
+                if (!mbar_wait(&ring.full[stage], round & 1)) { ring.failed = 1; break; }
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                const uint32_t d = tmem + (uint32_t)(buf * NT);
+                const uint32_t a_hi = smem_base + stage * STAGE, a_lo = a_hi + HTILE_BYTES, b_hi = a_hi + 2 * HTILE_BYTES, b_lo = b_hi + B_BYTES;
+#pragma unroll
+                for (int ks = 0; ks < KH / 16; ++ks) {
+                    const uint32_t off = ks * 32;  // 16 values = 32 bytes along the swizzled row
+                    umma_16(d, umma_desc(a_hi + off), umma_desc(b_hi + off), DESC, (opens && ks == 0) ? 0u : 1u);
+                    umma_16(d, umma_desc(a_lo + off), umma_desc(b_hi + off), DESC, 1u);
+                    umma_16(d, umma_desc(a_hi + off), umma_desc(b_lo + off), DESC, 1u);
+                }
+                umma_commit(&ring.empty[stage]);           // arrives when the MMAs above have read the stage
+                if (closes) umma_commit(&ring.acc_full[buf]);  // arrives when the slice is complete in tensor memory
+            }
+        }
+    } else {
+        const int q = warp & 3, c0 = ((warp - 2) >> 2) * MINE;
+        float total[MINE];
+#pragma unroll
+        for (int x = 0; x < MINE; ++x) total[x] = 0.f;
+        bool go = true;
+        for (int slice = 0; slice < slices; ++slice) {
+            const int buf = slice & 1;
+            const bool ok = mbar_wait(&ring.acc_full[buf], (slice >> 1) & 1, 64);
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            if (!ok) ring.failed = 1;
+            go = __all_sync(0xffffffffu, ok && !ring.failed);  // warp-uniform: the tensor-memory loads are warp-wide
+            if (!go) break;
+#pragma unroll
+            for (int cb = 0; cb < MINE / 32; ++cb) {
+                uint32_t v[32];
+                tmem_load_32(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(buf * NT + c0 + cb * 32), v);
+#pragma unroll
+                for (int x = 0; x < 32; ++x) total[cb * 32 + x] += __uint_as_float(v[x]);
+            }
+            // this warp has read the accumulator: hand it back to the MMA warp
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&ring.acc_empty[buf]);
+        }
+        // every chunk has been multiplied when the last slice is complete: the stages are free
+        if (go) finish(q, lane, c0, total, smem_base + (uint32_t)((warp - 2) * (MINE / 32) * BOX_BYTES));
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    if (warp == 1) {
+        if (ring.failed) {
+            // give outstanding loads and MMAs a bounded chance to land before the memory they target is released
+            if (lane == 0) mbar_wait(&ring.acc_full[((slices - 1) & 1)], ((slices - 1) >> 1) & 1);
+            __syncwarp();
+        }
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(COLS) : "memory");
+    }
+    return ring.failed != 0;
+}
+
+// Tiles of 128 x NT that touch the lower triangle, row by row: row I has I * 128 / NT + 1 of them.
+template <int NT>
+__host__ __device__ inline int64_t lower_tiles(int64_t rows) {  // of the first `rows` tile rows
+    return NT == 256 ? (rows / 2) * (rows / 2 + 1) + (rows % 2) * (rows / 2 + 1) : rows * (rows + 1) / 2;
+}
+template <int NT>
+__device__ __forceinline__ void lower_tile(int64_t lin, int &I, int &J) {
+    if (NT == 256) {  // rows 2 a and 2 a + 1 have a + 1 tiles each
+        int64_t a = (int64_t)((sqrt(4.0 * (double)lin + 1.0) - 1.0) / 2.0);
+        while ((a + 1) * (a + 2) <= lin) ++a;
+        while (a * (a + 1) > lin) --a;
+        const int64_t rest = lin - a * (a + 1);
+        I = (int)(2 * a + rest / (a + 1));
+        J = (int)(rest % (a + 1));
+    } else {
+        int64_t a = (int64_t)((sqrt(8.0 * (double)lin + 1.0) - 1.0) / 2.0);
+        while ((a + 1) * (a + 2) / 2 <= lin) ++a;
+        while (a * (a + 1) / 2 > lin) --a;
+        I = (int)a;
+        J = (int)(lin - a * (a + 1) / 2);
+    }
+}
+// A 128 x 256 tile takes 1.5 times as long as a 128 x 128 one (80 against 60 % of the tensor rate for twice the work), so the wide
+// tiles are for problems with enough of them: whole waves over the 148 SMs decide.
+inline bool wide_tiles_pay(int64_t wide, int64_t square) { return 3 * ceil_div(wide, (int64_t)148) <= 2 * ceil_div(square, (int64_t)148); }
+
 // ---- host side: tensor maps ----
 typedef CUresult (*EncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *,
                                   const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle,
@@ -240,12 +400,12 @@ static bool make_map(CUtensorMap *map, const float *base, int64_t rows, int64_t 
               CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// row-major 16-bit matrix [rows][cols]; boxes of box_rows rows x 64 columns
-static bool make_map_16(CUtensorMap *map, const void *base, int64_t rows, int64_t cols, int box_rows, bool bf16 = false) {
+// row-major 16-bit matrix [rows][cols] whose rows are `pitch` values apart (0: cols); boxes of box_rows rows x 64 columns
+static bool make_map_16(CUtensorMap *map, const void *base, int64_t rows, int64_t cols, int box_rows, bool bf16 = false, int64_t pitch = 0) {
     EncodeTiledFn fn = encode_tiled_fn();
     if (!fn) return false;
     const cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
-    const cuuint64_t strides[1] = {(cuuint64_t)cols * 2};
+    const cuuint64_t strides[1] = {(cuuint64_t)(pitch ? pitch : cols) * 2};
     const cuuint32_t box[2] = {KH, (cuuint32_t)box_rows};
     const cuuint32_t elem[2] = {1, 1};
     return fn(map, bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void *>(base), dims, strides, box, elem,
