@@ -217,26 +217,25 @@ struct FactorPlanes {
 int launch_trinv_tc(int count, const FactorPlanes *problems, cudaStream_t stream);
 
 // Tensor-core trailing update of the blocked Cholesky factorization (see g2d_factors_tc.cu).  pt planes are
-// [n][SYRK_TC_K] fp16 pairs: pt[r][k] = a[o + k][r] / unscale[r] for the group of block rows that starts at row o.
+// [n][SYRK_TC_K] fp16 pairs: pt[r][k] = SYRK_PANEL_SCALE a[o + k][r] for the group of block rows that starts at row o.
 constexpr int SYRK_TC_K = 256;
+constexpr float SYRK_PANEL_SCALE = 8192.f;
 struct SyrkTcMaps {
     alignas(64) unsigned char hi[128], lo[128], wide_hi[128], wide_lo[128], target[128];  // tensor maps of the planes and of the matrix (opaque here)
 };
 struct SyrkTcTarget {
     const SyrkTcMaps *maps;
     float *a;
-    const float *unscale;
     int64_t n, o;
     int t_lo, t_hi;  // target 128-row tile rows [t_lo, t_hi), tile columns up to the diagonal
     int kw;          // rows of the group (<= SYRK_TC_K)
     int *flag;
 };
-struct SyrkRange {
-    const float *a[2];
-    float *unscale[2];
+struct Equilibration {
+    float *a[2], *s[2];  // matrix and scales of its rows
     int64_t n[2];
 };
-int launch_syrk_range(int count, const SyrkRange &r, cudaStream_t stream);
+int launch_equilibrate(int count, const Equilibration &q, cudaStream_t stream);
 bool syrk_tc_maps(SyrkTcMaps *maps, const __half *pt_hi, const __half *pt_lo, float *a, int64_t n);
 int launch_syrk_tc(int count, const SyrkTcTarget *targets, cudaStream_t stream);
 

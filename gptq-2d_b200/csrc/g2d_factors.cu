@@ -78,7 +78,6 @@ struct LdlProblem {
     int *flag;
     int tc;                       // trailing updates of whole groups run on the tensor cores (float)
     __half *pt_hi[2], *pt_lo[2];  // [n][GROUP * 64] transposed, scaled split panels of the even and odd groups
-    float *unscale;               // [n] powers of two: the panels hold value / unscale[column]
 };
 template <typename F>
 struct LdlBatch {
@@ -256,14 +255,13 @@ __global__ void __launch_bounds__(FTH) ldl_trsm_kernel(LdlBatch<F> B, int step_d
 #pragma unroll
             for (int y = 0; y < 8; ++y) {
                 const int64_t c = c0 + own8(tx, y);
-                const float scale = 1.f / Q.unscale[c];  // a power of two: exact
 #pragma unroll
                 for (int half = 0; half < 2; ++half) {
                     __align__(8) __half h[4];
                     __align__(8) __half l[4];
 #pragma unroll
                     for (int e = 0; e < 4; ++e) {
-                        const float v = acc[4 * half + e][y] * scale;
+                        const float v = acc[4 * half + e][y] * SYRK_PANEL_SCALE;
                         h[e] = __float2half_rn(v);
                         l[e] = __float2half_rn(v - __half2float(h[e]));
                     }
@@ -386,26 +384,33 @@ __global__ void ldl_normalize_kernel(F *out, int64_t n, int size) {
 
 // The normalisation reads the diagonal blocks while other rows are rewritten, so the blocks are copied out first.
 template <typename F>
-__global__ void ldl_copy_diag_kernel(const F *out, int64_t n, int size, F *dblk) {
+__global__ void ldl_copy_diag_kernel(const F *out, int64_t n, int size, F *dblk, const F *scales) {
     const int64_t total = (n / size) * size * size;
     for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
         const int64_t b = t / ((int64_t)size * size);
         const int r = (int)(t / size % size), c = (int)(t % size);
-        dblk[t] = out[(b * size + r) * n + b * size + c];
+        dblk[t] = out[(b * size + r) * n + b * size + c] * (scales ? scales[b * size + r] : (F)1);
     }
 }
 
-// One CTA walks rows, its threads the column blocks left of the row's diagonal block (no index divisions per entry).
+// One CTA walks rows, its threads the column blocks left of the row's diagonal block (no index divisions per entry).  `scales`:
+// the rows of an equilibrated problem are scaled back on the way (may be null).
 template <typename F>
-__global__ void ldl_scale_kernel(F *out, int64_t n, int size, const F *dblk) {
+__global__ void ldl_scale_kernel(F *out, int64_t n, int size, const F *dblk, const F *scales) {
     for (int64_t row = blockIdx.x; row < n; row += gridDim.x) {
         const int64_t below = row / size;  // column blocks strictly left of the diagonal block
+        const F scale = scales ? scales[row] : (F)1;
+        if (size == 1) {
+#pragma unroll 4
+            for (int64_t b = threadIdx.x; b < below; b += blockDim.x) out[row * n + b] = out[row * n + b] * scale / dblk[b];
+            continue;
+        }
         for (int64_t b = threadIdx.x; b < below; b += blockDim.x) {
             F *p = out + row * n + b * size;
             const F *d = dblk + b * size * size;
             // x D = r with D lower triangular: back substitution from the last column of the block
             for (int x = size - 1; x >= 0; --x) {
-                F acc = p[x];
+                F acc = p[x] * scale;
                 for (int x2 = x + 1; x2 < size; ++x2) acc -= p[x2] * d[x2 * size + x];
                 p[x] = acc / d[x * size + x];
             }
@@ -413,11 +418,14 @@ __global__ void ldl_scale_kernel(F *out, int64_t n, int size, const F *dblk) {
     }
 }
 
-// Side streams for the look-ahead of the trailing updates.  Calls take lanes round robin, so two factorizations that
-// a caller runs concurrently on two streams do not share one.  Created on first use per device and kept.
+// Streams for the look-ahead of the trailing updates: the chain of diagonal blocks and panels on one of the highest priority, the
+// bulk of the updates on one of the lowest, so that a kernel of the chain takes the next SM that comes free instead of queueing
+// behind a millisecond of update CTAs (on two streams of one priority the two ran one after the other).  Calls take lanes round
+// robin, so two factorizations that a caller runs concurrently on two streams do not share one.  Created on first use per
+// device and kept.
 struct SideLane {
-    cudaStream_t stream = nullptr;
-    cudaEvent_t panel[4] = {}, rest[4] = {};
+    cudaStream_t stream = nullptr, chain = nullptr;
+    cudaEvent_t panel[4] = {}, rest[4] = {}, fork = nullptr, join = nullptr;
 };
 static SideLane *acquire_side_lane() {
     static std::mutex mutex;
@@ -428,7 +436,12 @@ static SideLane *acquire_side_lane() {
     std::lock_guard<std::mutex> lock(mutex);
     SideLane *lane = &lanes[device][next[device]++ & 3];
     if (!lane->stream) {
-        if (cudaStreamCreateWithFlags(&lane->stream, cudaStreamNonBlocking) != cudaSuccess) return nullptr;
+        int least = 0, greatest = 0;
+        if (cudaDeviceGetStreamPriorityRange(&least, &greatest) != cudaSuccess) return nullptr;
+        if (cudaStreamCreateWithPriority(&lane->stream, cudaStreamNonBlocking, least) != cudaSuccess ||
+            cudaStreamCreateWithPriority(&lane->chain, cudaStreamNonBlocking, greatest) != cudaSuccess ||
+            cudaEventCreateWithFlags(&lane->fork, cudaEventDisableTiming) != cudaSuccess || cudaEventCreateWithFlags(&lane->join, cudaEventDisableTiming) != cudaSuccess)
+            return nullptr;
         for (int k = 0; k < 4; ++k)
             if (cudaEventCreateWithFlags(&lane->panel[k], cudaEventDisableTiming) != cudaSuccess ||
                 cudaEventCreateWithFlags(&lane->rest[k], cudaEventDisableTiming) != cudaSuccess)
@@ -441,7 +454,7 @@ static SideLane *acquire_side_lane() {
 // nine operand planes of the tensor-core triangular inverse, two pairs of transposed split panels and their scales.
 inline int64_t plane_pitch(int64_t n) { return (n + 7) / 8 * 8; }  // rows of the 16-bit planes are 16-byte multiples (a TMA requirement)
 struct LdlLayout {
-    size_t tinv, dblk, w, planes, panels, unscale, total;
+    size_t tinv, dblk, w, planes, panels, scales, total;
 };
 static LdlLayout ldl_layout(size_t elem, int64_t n) {
     LdlLayout lay;
@@ -453,21 +466,24 @@ static LdlLayout ldl_layout(size_t elem, int64_t n) {
     const bool tc = elem == 4;
     lay.planes = take(tc ? 9 * sizeof(__nv_bfloat16) * (size_t)n * plane_pitch(n) : 0);
     lay.panels = take(tc ? 4 * sizeof(__half) * (size_t)n * GROUP * FB : 0);
-    lay.unscale = take(tc ? sizeof(float) * (size_t)n : 0);
+    lay.scales = take(tc ? sizeof(float) * (size_t)n : 0);
     lay.total = at;
     return lay;
 }
 
 template <typename F>
-int ldl_run(int count, const int64_t *ns, F *const *as, const int *sizes, F *const *outs, int *flags, void *const *workspaces, cudaStream_t st) {
+int ldl_run(int count, const int64_t *ns, F *const *as, const int *sizes, F *const *outs, int *flags, void *const *workspaces, cudaStream_t caller) {
     LdlBatch<F> B;
+    cudaStream_t st = caller;
     B.count = count;
     B.steps = 0;
     F *dblks[2] = {nullptr, nullptr};
     SyrkTcMaps pt_maps[2][2];
     int64_t n_max = 0;
     bool any_tc = false;
-    SyrkRange range{};
+    Equilibration equilibrated{};
+    float *scales[2] = {nullptr, nullptr};  // of the equilibrated problems
+    int problems = 0;
     LdlLayout layout[2];
     for (int z = 0; z < count; ++z) {
         const int64_t n = ns[z];
@@ -476,7 +492,7 @@ int ldl_run(int count, const int64_t *ns, F *const *as, const int *sizes, F *con
         char *ws = (char *)workspaces[z];
         dblks[z] = (F *)(ws + lay.dblk);
         LdlProblem<F> &P = B.p[z];
-        P = LdlProblem<F>{as[z], outs[z], (F *)(ws + lay.tinv), (F *)(ws + lay.w), n, flags ? flags + z : nullptr, 0, {nullptr, nullptr}, {nullptr, nullptr}, nullptr};
+        P = LdlProblem<F>{as[z], outs[z], (F *)(ws + lay.tinv), (F *)(ws + lay.w), n, flags ? flags + z : nullptr, 0, {nullptr, nullptr}, {nullptr, nullptr}};
         if (std::is_same<F, float>::value) {
             const size_t panel = sizeof(__half) * (size_t)n * GROUP * FB;
             for (int k = 0; k < 2; ++k) {
@@ -484,10 +500,12 @@ int ldl_run(int count, const int64_t *ns, F *const *as, const int *sizes, F *con
                 P.pt_lo[k] = (__half *)(ws + lay.panels + (2 * k + 1) * panel);
                 if (!syrk_tc_maps(&pt_maps[z][k], P.pt_hi[k], P.pt_lo[k], (float *)as[z], n)) return G2D_ERR_CUDA;
             }
-            P.unscale = (float *)(ws + lay.unscale);
-            range.a[z] = (const float *)as[z];
-            range.unscale[z] = P.unscale;
-            range.n[z] = n;
+            if (n > GROUP * FB) {  // more than one group: there are trailing updates on the tensor cores
+                scales[z] = (float *)(ws + lay.scales);
+                equilibrated.a[problems] = (float *)as[z];
+                equilibrated.s[problems] = scales[z];
+                equilibrated.n[problems++] = n;
+            }
             P.tc = 1;
             any_tc = true;
         }
@@ -496,7 +514,7 @@ int ldl_run(int count, const int64_t *ns, F *const *as, const int *sizes, F *con
         n_max = n > n_max ? n : n_max;
         if (cudaMemsetAsync(outs[z], 0, sizeof(F) * (size_t)n * n, st) != cudaSuccess) return G2D_ERR_CUDA;
     }
-    if (any_tc && n_max > GROUP * FB && launch_syrk_range(count, range, st) != G2D_OK) return G2D_ERR_CUDA;
+    if (problems > 0 && launch_equilibrate(problems, equilibrated, st) != G2D_OK) return G2D_ERR_CUDA;
     if (count == 1) B.p[1] = B.p[0];
     if (flags && cudaMemsetAsync(flags, 0, sizeof(int) * count, st) != cudaSuccess) return G2D_ERR_CUDA;
     // Each step factors one 64-row block row (last first): diagonal block, panel to its left, trailing update.  The
@@ -509,6 +527,8 @@ int ldl_run(int count, const int64_t *ns, F *const *as, const int *sizes, F *con
     // it shares (the order of the additions is fixed, hence the result).
     SideLane *lane = acquire_side_lane();
     if (!lane) return G2D_ERR_CUDA;
+    if (cudaEventRecord(lane->fork, caller) != cudaSuccess || cudaStreamWaitEvent(lane->chain, lane->fork, 0) != cudaSuccess) return G2D_ERR_CUDA;
+    st = lane->chain;
     bool rest_recorded[4] = {false, false, false, false};
     const int groups = B.steps / GROUP;
     auto wait_rest = [&](int g) {
@@ -549,7 +569,7 @@ int ldl_run(int count, const int64_t *ns, F *const *as, const int *sizes, F *con
             const int64_t o = (int64_t)kb_lo * FB;
             const int t_all = (int)(o / 128), t_next = t_all - GROUP * FB / 128;  // tile rows above the group; those of the next group start at t_next
             const int kw = (int)(ns[z] - o < GROUP * FB ? ns[z] - o : GROUP * FB);
-            SyrkTcTarget t{&pt_maps[z][(kb_lo / GROUP) & 1], (float *)B.p[z].a, B.p[z].unscale, ns[z], o, t_next, t_all, kw, B.p[z].flag};
+            SyrkTcTarget t{&pt_maps[z][(kb_lo / GROUP) & 1], (float *)B.p[z].a, ns[z], o, t_next, t_all, kw, B.p[z].flag};
             next[targets] = t;
             t.t_lo = 0;
             t.t_hi = t_next;
@@ -571,9 +591,11 @@ int ldl_run(int count, const int64_t *ns, F *const *as, const int *sizes, F *con
         if (status != G2D_OK) return status;
         rest_recorded[g & 3] = any_rest;
     }
-    // everything the side stream did joins the caller's stream before the inverse starts
+    // everything the side streams did joins the caller's stream before the inverse starts
     for (int k = 0; k < 4; ++k)
-        if (rest_recorded[k] && cudaStreamWaitEvent(st, lane->rest[k], 0) != cudaSuccess) return G2D_ERR_CUDA;
+        if (rest_recorded[k] && cudaStreamWaitEvent(caller, lane->rest[k], 0) != cudaSuccess) return G2D_ERR_CUDA;
+    if (cudaEventRecord(lane->join, st) != cudaSuccess || cudaStreamWaitEvent(caller, lane->join, 0) != cudaSuccess) return G2D_ERR_CUDA;
+    st = caller;
     ldl_copy_diag_inverse_kernel<F><<<dim3(B.steps, count), FTH, 0, st>>>(B);
     if (check_launch() != G2D_OK) return G2D_ERR_CUDA;
     // The 64-level for everyone; from the 128-level on, float problems continue on the tensor cores.
@@ -606,9 +628,9 @@ int ldl_run(int count, const int64_t *ns, F *const *as, const int *sizes, F *con
         const int64_t n = ns[z];
         const int size = sizes[z];
         const int64_t blocks = n < 148 * 16 ? n : 148 * 16;  // rows are dealt out to CTAs
-        ldl_copy_diag_kernel<F><<<(unsigned)(ceil_div(n * size, 256) < 148 * 64 ? ceil_div(n * size, 256) : 148 * 64), 256, 0, st>>>(outs[z], n, size, dblks[z]);
+        ldl_copy_diag_kernel<F><<<(unsigned)(ceil_div(n * size, 256) < 148 * 64 ? ceil_div(n * size, 256) : 148 * 64), 256, 0, st>>>(outs[z], n, size, dblks[z], (const F *)scales[z]);
         if (check_launch() != G2D_OK) return G2D_ERR_CUDA;
-        ldl_scale_kernel<F><<<(unsigned)blocks, 256, 0, st>>>(outs[z], n, size, dblks[z]);
+        ldl_scale_kernel<F><<<(unsigned)blocks, 256, 0, st>>>(outs[z], n, size, dblks[z], (const F *)scales[z]);
         if (check_launch() != G2D_OK) return G2D_ERR_CUDA;
         ldl_normalize_kernel<F><<<(unsigned)ceil_div(n, (int64_t)256), 256, 0, st>>>(outs[z], n, size);
         if (check_launch() != G2D_OK) return G2D_ERR_CUDA;

@@ -307,29 +307,30 @@ int launch_trinv_tc(int count, const FactorPlanes *problems, cudaStream_t stream
 // ---- trailing update of the blocked Cholesky factorization ----
 // After a group of four 64-row block rows [o, o + kw) is factored, everything above it receives
 //     a[r][c] -= sum_{k < kw} a[o + k][r] a[o + k][c],      c <= r < o,
-// one tile per CTA.  Both operands are the same K-major fp16 pairs pt[r][k] = a[o + k][r] 2^-e(r), which the panel kernel
-// writes as it finishes a block row.  The scale of a row of the result comes from its diagonal entry in M: the squares of
-// T[., r] add up to M[r][r], so no entry of the panel exceeds sqrt(M[r][r]).  One CTA owns each target entry and no other kernel
-// touches the targets meanwhile, so the result does not depend on scheduling.
+// a few tiles per CTA.  Both operands are the same K-major fp16 pairs pt[r][k] = 2^13 a[o + k][r], which the panel kernel writes
+// as it finishes a block row.  M is equilibrated first (rows and columns scaled by powers of two, exactly, to diagonal
+// entries in [1, 4)): the squares of T[., r] add up to M[r][r], so every entry of a panel is below 2 and one scale serves all
+// of them.  One CTA owns each target entry and no other kernel touches the targets meanwhile, so the result does not depend on
+// scheduling.
 // Accuracy.  The tensor cores add each product into the float accumulator with truncation, which biases long sums of
 // one sign by about 1e-8 of the sum per term, and the diagonal of this update is a sum of squares, subtracted from pivots
 // that a damped, badly conditioned Gram leaves one or two orders of magnitude smaller than the sum.  Two measures keep the
-// factors at the accuracy of a float32 LAPACK factorization: the k range is cut into slices of 64 (added up in registers, round
+// factors at the accuracy of a float32 LAPACK factorization: the k range is cut into slices of 128 (added up in registers, round
 // to nearest), and the diagonal entries are left out and updated with a float64 sum of the float panel by CTAs of their own
 // (the first ones of the launch, one per 128 rows).
 // Bound: HBM for factors beyond L2 (8 bytes per entry and group of 256 rows: 123 GB at n = 28672, 20 ms), shared-memory port
-// below (see pair_gemm).  n = 28672 and 8192 together: SYRKBEFORE ms with 128 x 128 tf32 tiles, SYRKNOW ms now.
-constexpr int SYRK_SLICE_CHUNKS = 1;  // k = 64 per slice
+// below (see pair_gemm).  n = 28672 and 8192 together: 73 ms with 128 x 128 tf32 tiles, SYRKNOW ms now.
+constexpr int SYRK_SLICE_CHUNKS = 2;  // k = 128 per slice: as many additions into one accumulator as 64 take in tf32
 static_assert(SYRK_TC_K % KH == 0, "whole chunks per group");
 
 struct SyrkJob {
     CUtensorMap a_hi[2], a_lo[2], b_hi[2], b_lo[2];  // the same planes in boxes of 128 and of NT rows
     CUtensorMap target[2];                           // the matrix itself in boxes of 32 x 32 (n a multiple of 4: its rows 16-byte multiples)
     float *a[2];
-    const float *unscale[2];
     int64_t n[2], o[2];    // size, first row of the group
     int t_lo[2], t_hi[2];  // target tile rows [t_lo, t_hi), with every tile column up to the diagonal
     int kw[2];
+    int tiles_per_cta;
     int *flag[2];
 };
 template <int NT>
@@ -343,7 +344,6 @@ __global__ void __launch_bounds__(PAIR_THREADS, 1) syrk_tc_kernel(const __grid_c
     const int z = blockIdx.y;
     const int t_lo = z ? job.t_lo[1] : job.t_lo[0], t_hi = z ? job.t_hi[1] : job.t_hi[0];
     float *const a = z ? job.a[1] : job.a[0];
-    const float *const unscale = z ? job.unscale[1] : job.unscale[0];
     const int64_t n = z ? job.n[1] : job.n[0], o = z ? job.o[1] : job.o[0];
     const int kw = z ? job.kw[1] : job.kw[0];
     const int diagonals = t_hi - t_lo;
@@ -373,59 +373,63 @@ __global__ void __launch_bounds__(PAIR_THREADS, 1) syrk_tc_kernel(const __grid_c
         }
         return;
     }
-    const int64_t first = lower_tiles<NT>(t_lo), lin = first + (int64_t)blockIdx.x - diagonals;
-    if (lin >= lower_tiles<NT>(t_hi)) return;
-    int I2, J2;
-    lower_tile<NT>(lin, I2, J2);
+    const int64_t first = lower_tiles<NT>(t_lo) + ((int64_t)blockIdx.x - diagonals) * job.tiles_per_cta, last = lower_tiles<NT>(t_hi);
+    if (first >= last) return;
     const CUtensorMap *a_hi = z ? &job.a_hi[1] : &job.a_hi[0], *a_lo = z ? &job.a_lo[1] : &job.a_lo[0];
     const CUtensorMap *b_hi = z ? &job.b_hi[1] : &job.b_hi[0], *b_lo = z ? &job.b_lo[1] : &job.b_lo[0];
-    const int i0 = I2 * MT, j0 = J2 * NT;
     const bool vec = n % 4 == 0;
     const uint32_t smem_base = (smem_u32(tc_smem_raw) + 1023u) & ~1023u;
-    auto load = [&](int ch, uint32_t dst, uint64_t *bar) {
-        tma_load_2d(dst, a_hi, ch * KH, i0, bar);
-        tma_load_2d(dst + HTILE_BYTES, a_lo, ch * KH, i0, bar);
-        tma_load_2d(dst + 2 * HTILE_BYTES, b_hi, ch * KH, j0, bar);
-        tma_load_2d(dst + 2 * HTILE_BYTES + NT * KH * 2, b_lo, ch * KH, j0, bar);
+    int I_first, J_first;
+    lower_tile<NT>(first, I_first, J_first);
+    auto next = [&](int it, PairTile &t) {
+        if (it >= job.tiles_per_cta || first + it >= last) return false;
+        int I2 = I_first, J2 = J_first + it;
+        for (int row; J2 >= (row = NT == 256 ? I2 / 2 + 1 : I2 + 1); ++I2) J2 -= row;
+        t = PairTile{I2 * MT, J2 * NT, (kw + KH - 1) / KH};
+        return true;
     };
+    auto load = [&](const PairTile &t, int ch, uint32_t dst, uint64_t *bar) {
+        tma_load_2d(dst, a_hi, ch * KH, t.i0, bar);
+        tma_load_2d(dst + HTILE_BYTES, a_lo, ch * KH, t.i0, bar);
+        tma_load_2d(dst + 2 * HTILE_BYTES, b_hi, ch * KH, t.j0, bar);
+        tma_load_2d(dst + 2 * HTILE_BYTES + NT * KH * 2, b_lo, ch * KH, t.j0, bar);
+    };
+    constexpr float UNSCALE = -1.f / (SYRK_PANEL_SCALE * SYRK_PANEL_SCALE);
     const CUtensorMap *target = z ? &job.target[1] : &job.target[0];
-    auto finish = [&](int q, int ln, int c0, float (&total)[MINE], uint32_t boxes) {
-        const int64_t gi = (int64_t)i0 + q * 32 + ln;  // always a row of the matrix: the targets lie above the group
-        const float row_scale = -unscale[gi];
+    auto finish = [&](const PairTile &t, int q, int ln, int c0, float (&total)[MINE], uint32_t box) {
+        const int i0 = t.i0 + q * 32, gi = i0 + ln;  // always a row of the matrix: the targets lie above the group
         if (vec) {
-            // the diagonal entries are updated above; what lies right of the diagonal is never read: both get zeros
 #pragma unroll
             for (int cb = 0; cb < MINE / 32; ++cb) {
-                const int64_t gj0 = (int64_t)j0 + c0 + cb * 32;
-                if (gj0 > (int64_t)i0 + q * 32 + 31) continue;  // warp-uniform
-                const uint32_t box = boxes + cb * BOX_BYTES;
+                const int gj0 = t.j0 + c0 + cb * 32;
+                if (gj0 > i0 + 31) continue;  // warp-uniform
+                if (gj0 + 31 >= i0) {
+                    // the diagonal entries are updated above; what lies right of the diagonal is never read: both get zeros
 #pragma unroll
-                for (int g = 0; g < 8; ++g) {
-                    float v[4];
-#pragma unroll
-                    for (int e = 0; e < 4; ++e) {
-                        const int64_t gj = gj0 + g * 4 + e;  // left of row gi: inside the matrix
-                        v[e] = gj < gi ? total[cb * 32 + g * 4 + e] * row_scale * unscale[gj] : 0.f;
-                    }
-                    box_store4(box, ln, g, v[0], v[1], v[2], v[3]);
+                    for (int x = 0; x < 32; ++x) total[cb * 32 + x] = gj0 + x < gi ? total[cb * 32 + x] : 0.f;
                 }
+                if (ln == 0) box_free();
+                __syncwarp();
+#pragma unroll
+                for (int g = 0; g < 8; ++g)
+                    box_store4(box, ln, g, UNSCALE * total[cb * 32 + g * 4], UNSCALE * total[cb * 32 + g * 4 + 1], UNSCALE * total[cb * 32 + g * 4 + 2],
+                               UNSCALE * total[cb * 32 + g * 4 + 3]);
                 box_fence();
                 __syncwarp();
-                if (ln == 0) box_reduce_add(target, box, (int)gj0, i0 + q * 32);
-            }
-            if (ln == 0) {
-                box_commit();
-                box_wait();
+                if (ln == 0) {
+                    box_reduce_add(target, box, gj0, i0);
+                    box_commit();
+                }
             }
             return;
         }
 #pragma unroll
         for (int x = 0; x < MINE; ++x) {
-            const int64_t gj = (int64_t)j0 + c0 + x;
-            if (gj < gi) asm volatile("red.global.add.f32 [%0], %1;" ::"l"(a + gi * n + gj), "f"(total[x] * row_scale * unscale[gj]) : "memory");
+            const int gj = t.j0 + c0 + x;
+            if (gj < gi) asm volatile("red.global.add.f32 [%0], %1;" ::"l"(a + (int64_t)gi * n + gj), "f"(UNSCALE * total[x]) : "memory");
         }
     };
-    const bool failed = pair_gemm<NT, syrk_stages<NT>, SYRK_SLICE_CHUNKS>(ring, smem_base, (kw + KH - 1) / KH, load, finish);
+    const bool failed = pair_gemm<NT, syrk_stages<NT>, SYRK_SLICE_CHUNKS>(ring, smem_base, next, load, finish);
     int *const flag = z ? job.flag[1] : job.flag[0];
     if (threadIdx.x == 0 && failed && flag) atomicExch(flag, -1);
 }
@@ -442,7 +446,7 @@ bool syrk_tc_maps(SyrkTcMaps *maps, const __half *pt_hi, const __half *pt_lo, fl
 template <int NT>
 static int launch_syrk_tiles(int count, const SyrkJob &job, int64_t blocks, cudaStream_t stream) {
     static PerDeviceOnce configured;
-    constexpr size_t smem = (size_t)syrk_stages<NT> * pair_stage_bytes<NT> + 1024;
+    constexpr size_t smem = (size_t)syrk_stages<NT> * pair_stage_bytes<NT> + PAIR_BOXES + 1024;
     if (configured.run([&] { return cudaFuncSetAttribute(syrk_tc_kernel<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) == cudaSuccess; }) != G2D_OK)
         return G2D_ERR_CUDA;
     syrk_tc_kernel<NT><<<dim3((unsigned)blocks, count), PAIR_THREADS, smem, stream>>>(job);
@@ -451,18 +455,25 @@ static int launch_syrk_tiles(int count, const SyrkJob &job, int64_t blocks, cuda
 
 int launch_syrk_tc(int count, const SyrkTcTarget *targets, cudaStream_t stream) {
     SyrkJob job;
-    int64_t wide = 0, square = 0, most_wide = 0, most_square = 0;
+    int64_t wide = 0, square = 0;
     for (int z = 0; z < count; ++z) {
-        const SyrkTcTarget &t = targets[z];
-        const int64_t w = lower_tiles<256>(t.t_hi) - lower_tiles<256>(t.t_lo), q = lower_tiles<128>(t.t_hi) - lower_tiles<128>(t.t_lo), d = t.t_hi - t.t_lo;
-        wide += w;
-        square += q;
-        most_wide = w + d > most_wide ? w + d : most_wide;
-        most_square = q + d > most_square ? q + d : most_square;
+        wide += lower_tiles<256>(targets[z].t_hi) - lower_tiles<256>(targets[z].t_lo);
+        square += lower_tiles<128>(targets[z].t_hi) - lower_tiles<128>(targets[z].t_lo);
     }
     if (square <= 0) return G2D_OK;
-    if (most_square > 0x7fffffff) return G2D_ERR_TOO_LARGE;
     const bool use_wide = wide_tiles_pay(wide, square);
+    // Several tiles per CTA once there are more than two waves of them, but few enough that an SM comes free every other
+    // moment: the diagonal blocks and panels of the next group, on a stream of higher priority, wait for one.
+    const int64_t tiles = use_wide ? wide : square;
+    job.tiles_per_cta = (int)(tiles / (2 * 148) < 1 ? 1 : tiles / (2 * 148) > 6 ? 6 : tiles / (2 * 148));
+    int64_t blocks = 0;
+    for (int z = 0; z < count; ++z) {
+        const SyrkTcTarget &t = targets[z];
+        const int64_t mine = use_wide ? lower_tiles<256>(t.t_hi) - lower_tiles<256>(t.t_lo) : lower_tiles<128>(t.t_hi) - lower_tiles<128>(t.t_lo);
+        const int64_t need = ceil_div(mine, (int64_t)job.tiles_per_cta) + t.t_hi - t.t_lo;
+        blocks = need > blocks ? need : blocks;
+    }
+    if (blocks > 0x7fffffff) return G2D_ERR_TOO_LARGE;
     for (int z = 0; z < 2; ++z) {
         const SyrkTcTarget &t = targets[z < count ? z : 0];
         memcpy(&job.a_hi[z], t.maps->hi, sizeof(CUtensorMap));
@@ -471,7 +482,6 @@ int launch_syrk_tc(int count, const SyrkTcTarget *targets, cudaStream_t stream) 
         memcpy(&job.b_lo[z], use_wide ? t.maps->wide_lo : t.maps->lo, sizeof(CUtensorMap));
         memcpy(&job.target[z], t.maps->target, sizeof(CUtensorMap));
         job.a[z] = t.a;
-        job.unscale[z] = t.unscale;
         job.n[z] = t.n;
         job.o[z] = t.o;
         job.t_lo[z] = t.t_lo;
@@ -479,21 +489,44 @@ int launch_syrk_tc(int count, const SyrkTcTarget *targets, cudaStream_t stream) 
         job.kw[z] = t.kw;
         job.flag[z] = t.flag;
     }
-    return use_wide ? launch_syrk_tiles<256>(count, job, most_wide, stream) : launch_syrk_tiles<128>(count, job, most_square, stream);
+    return use_wide ? launch_syrk_tiles<256>(count, job, blocks, stream) : launch_syrk_tiles<128>(count, job, blocks, stream);
 }
 
-// The scales: unscale[r] = 2^e with sqrt(M[r][r]) 2^-e in [2^14, 2^15).
-__global__ void syrk_range_kernel(SyrkRange r) {
+// Equilibration: s[r] = 2^-e with sqrt(M[r][r]) in [2^e, 2^(e + 1)), M[r][c] *= s[r] s[c].  Exact short of the ends of the
+// range of floats; the factor of the scaled matrix is T diag(s), and the rows of its inverse are scaled back at the end.
+__global__ void equilibrate_scale_kernel(Equilibration q) {
     const int z = blockIdx.y;
-    const int64_t n = z ? r.n[1] : r.n[0];
-    const float *a = z ? r.a[1] : r.a[0];
-    float *unscale = z ? r.unscale[1] : r.unscale[0];
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-        unscale[i] = power_of_two(range_exponent(sqrtf(a[i * n + i])));
+    const int64_t n = q.n[z];
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+        const float root = sqrtf(q.a[z][i * n + i]);
+        const int e = (int)((__float_as_uint(root) >> 23) & 255) - 127;
+        q.s[z][i] = root > 0.f && e < 128 ? power_of_two(-e) : 1.f;  // not a positive definite matrix: the pivots will tell
+    }
 }
-int launch_syrk_range(int count, const SyrkRange &r, cudaStream_t stream) {
-    const int64_t most = count > 1 && r.n[1] > r.n[0] ? r.n[1] : r.n[0];
-    syrk_range_kernel<<<dim3((unsigned)(ceil_div(most, (int64_t)256) < 592 ? ceil_div(most, (int64_t)256) : 592), count), 256, 0, stream>>>(r);
+__global__ void __launch_bounds__(256) equilibrate_kernel(Equilibration q) {
+    const int z = blockIdx.y;
+    const int64_t n = q.n[z];
+    const float *s = q.s[z];
+    for (int64_t r = blockIdx.x; r < n; r += gridDim.x) {
+        float *row = q.a[z] + r * n;
+        const float sr = s[r];
+        if (n % 4 == 0) {
+            for (int64_t c = (int64_t)threadIdx.x * 4; c <= r; c += (int64_t)blockDim.x * 4) {  // a group may reach past the diagonal: never read there
+                float4 v = *reinterpret_cast<const float4 *>(row + c);
+                const float4 sc = *reinterpret_cast<const float4 *>(s + c);
+                v.x = v.x * sr * sc.x; v.y = v.y * sr * sc.y; v.z = v.z * sr * sc.z; v.w = v.w * sr * sc.w;
+                *reinterpret_cast<float4 *>(row + c) = v;
+            }
+        } else {
+            for (int64_t c = threadIdx.x; c <= r; c += blockDim.x) row[c] = row[c] * sr * s[c];
+        }
+    }
+}
+int launch_equilibrate(int count, const Equilibration &q, cudaStream_t stream) {
+    const int64_t most = count > 1 && q.n[1] > q.n[0] ? q.n[1] : q.n[0];
+    equilibrate_scale_kernel<<<dim3((unsigned)(ceil_div(most, (int64_t)128) < 592 ? ceil_div(most, (int64_t)128) : 592), count), 128, 0, stream>>>(q);
+    if (check_launch() != G2D_OK) return G2D_ERR_CUDA;
+    equilibrate_kernel<<<dim3((unsigned)(most < 148 * 16 ? most : 148 * 16), count), 256, 0, stream>>>(q);
     return check_launch();
 }
 

@@ -5,7 +5,7 @@
 //
 // X^T is first written as K-major fp16 pairs [n][k], every channel scaled by a power of two of its own (the channel is the
 // index that is not summed over, so the scale comes out of the product again), then every 128 x 256 tile that touches the
-// lower triangle of H is one CTA: TMA into a two-stage ring of 96 KB, tcgen05.mma kind::f16 with three products per k step
+// lower triangle of H is one CTA's (of one CTA per SM): TMA into a two-stage ring of 96 KB, tcgen05.mma kind::f16 with three products per k step
 // into tensor memory, eight warps that add the accumulators up in registers slice of k by slice of k, and at the end
 // write H and its mirror image.  Every entry of H has one owner, so the result does not depend on scheduling.
 //
@@ -105,7 +105,7 @@ struct GramJob {
     CUtensorMap a_hi, a_lo, b_hi, b_lo;  // the same planes in boxes of 128 and of NT rows
     float *h;
     const unsigned *largest;
-    int64_t n;
+    int64_t n, tiles;
     int chunks;
     float alpha;
     int *flag;
@@ -116,25 +116,30 @@ __global__ void __launch_bounds__(PAIR_THREADS, 1) gram_tc_kernel(const __grid_c
     constexpr int MINE = NT / 2;  // columns per reading warp
     extern __shared__ unsigned char tc_smem_raw[];
     __shared__ __align__(8) PairRing<GRAM_STAGES> ring;
-    int I2, J2;
-    lower_tile<NT>(blockIdx.x, I2, J2);
-    const int i0 = I2 * MT, j0 = J2 * NT;
     const int64_t n = job.n;
     const uint32_t smem_base = (smem_u32(tc_smem_raw) + 1023u) & ~1023u;
-    auto load = [&](int ch, uint32_t dst, uint64_t *bar) {
-        tma_load_2d(dst, &job.a_hi, ch * KH, i0, bar);
-        tma_load_2d(dst + HTILE_BYTES, &job.a_lo, ch * KH, i0, bar);
-        tma_load_2d(dst + 2 * HTILE_BYTES, &job.b_hi, ch * KH, j0, bar);
-        tma_load_2d(dst + 2 * HTILE_BYTES + NT * KH * 2, &job.b_lo, ch * KH, j0, bar);
+    auto next = [&](int it, PairTile &t) {
+        const int64_t lin = blockIdx.x + (int64_t)it * gridDim.x;
+        if (lin >= job.tiles) return false;
+        int I2, J2;
+        lower_tile<NT>(lin, I2, J2);
+        t = PairTile{I2 * MT, J2 * NT, job.chunks};
+        return true;
     };
-    auto finish = [&](int q, int lane, int c0, float (&total)[MINE], uint32_t) {
-        const int64_t gi = (int64_t)i0 + q * 32 + lane;
+    auto load = [&](const PairTile &t, int ch, uint32_t dst, uint64_t *bar) {
+        tma_load_2d(dst, &job.a_hi, ch * KH, t.i0, bar);
+        tma_load_2d(dst + HTILE_BYTES, &job.a_lo, ch * KH, t.i0, bar);
+        tma_load_2d(dst + 2 * HTILE_BYTES, &job.b_hi, ch * KH, t.j0, bar);
+        tma_load_2d(dst + 2 * HTILE_BYTES + NT * KH * 2, &job.b_lo, ch * KH, t.j0, bar);
+    };
+    auto finish = [&](const PairTile &t, int q, int lane, int c0, float (&total)[MINE], uint32_t) {
+        const int64_t gi = (int64_t)t.i0 + q * 32 + lane;
         if (gi >= n) return;
         constexpr int GROUP = 16;
         const float row_scale = power_of_two(range_exponent(__uint_as_float(job.largest[gi])));
 #pragma unroll
         for (int x0 = 0; x0 < MINE; x0 += GROUP) {
-            const int64_t gj0 = (int64_t)j0 + c0 + x0;
+            const int64_t gj0 = (int64_t)t.j0 + c0 + x0;
             if (gj0 > gi) continue;  // the upper triangle is the mirror image of the lower one
             float *const dst = job.h + gi * n + gj0;
             // the old values of sixteen columns travel together, before the first is used
@@ -168,7 +173,7 @@ __global__ void __launch_bounds__(PAIR_THREADS, 1) gram_tc_kernel(const __grid_c
             }
         }
     };
-    const bool failed = pair_gemm<NT, GRAM_STAGES, GRAM_SLICE>(ring, smem_base, job.chunks, load, finish);
+    const bool failed = pair_gemm<NT, GRAM_STAGES, GRAM_SLICE>(ring, smem_base, next, load, finish);
     if (threadIdx.x == 0 && failed && job.flag) atomicExch(job.flag, -1);
 }
 
@@ -181,7 +186,8 @@ static int launch_gram(GramJob &job, const __half *hi, const __half *lo, int64_t
     if (!make_map_16(&job.a_hi, hi, job.n, kp, MT) || !make_map_16(&job.a_lo, lo, job.n, kp, MT) || !make_map_16(&job.b_hi, hi, job.n, kp, NT) ||
         !make_map_16(&job.b_lo, lo, job.n, kp, NT))
         return G2D_ERR_CUDA;
-    gram_tc_kernel<NT><<<(unsigned)tiles, PAIR_THREADS, smem, st>>>(job);
+    job.tiles = tiles;
+    gram_tc_kernel<NT><<<(unsigned)(tiles < 148 ? tiles : 148), PAIR_THREADS, smem, st>>>(job);
     return check_launch();
 }
 

@@ -224,8 +224,14 @@ __device__ __forceinline__ void box_reduce_add(const CUtensorMap *map, uint32_t 
                  ::"l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(box)
                  : "memory");
 }
+__device__ __forceinline__ void box_store(const CUtensorMap *map, uint32_t box, int x, int y) {
+    asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.tile.bulk_group [%0, {%1, %2}], [%3];"
+                 ::"l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(box)
+                 : "memory");
+}
 __device__ __forceinline__ void box_fence() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 __device__ __forceinline__ void box_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
+__device__ __forceinline__ void box_free() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }  // the lane's boxes may be overwritten
 __device__ __forceinline__ void box_wait() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 
 // ---- pipeline for 16-bit pairs: A[128 x k] B[NT x k]^T as hi hi + lo hi + hi lo ----
@@ -236,6 +242,7 @@ __device__ __forceinline__ void box_wait() { asm volatile("cp.async.bulk.wait_gr
 constexpr int PAIR_THREADS = 320;
 template <int NT>
 constexpr int pair_stage_bytes = 2 * HTILE_BYTES + 2 * NT * KH * 2;
+constexpr int PAIR_BOXES = 8 * BOX_BYTES;  // one per reading warp, where the results leave as boxes
 template <int NSTAGE>
 struct PairRing {
     uint64_t full[NSTAGE], empty[NSTAGE], acc_full[2], acc_empty[2];
@@ -243,15 +250,18 @@ struct PairRing {
     int failed;
 };
 
-// load(chunk, destination, barrier): A_hi, A_lo, B_hi, B_lo tiles one after the other.
-// finish(q, lane, first column, totals, shared memory of the warp: 4 KB per 32 of
-// its columns, 1024-byte aligned).  Returns whether a wait ran out.
-template <int NT, int NSTAGE, int SLICE, typename Load, typename Finish>
-__device__ __forceinline__ bool pair_gemm(PairRing<NSTAGE> &ring, uint32_t smem_base, int chunks, Load load, Finish finish) {
+// A CTA takes several tiles, one after the other, so that a tile's loads and MMAs run while the results of the one before leave.
+// next(number, tile): the CTA's tile of that number, false past the last.  load(tile, chunk, destination, barrier): A_hi, A_lo,
+// B_hi, B_lo tiles one after the other.  finish(tile, q, lane, first column, totals, 4 KB of shared memory of the warp's own
+// behind the stages).  Returns whether a wait ran out.
+struct PairTile {
+    int i0, j0, chunks;
+};
+template <int NT, int NSTAGE, int SLICE, typename Next, typename Load, typename Finish>
+__device__ __forceinline__ bool pair_gemm(PairRing<NSTAGE> &ring, uint32_t smem_base, Next next, Load load, Finish finish) {
     constexpr int B_BYTES = NT * KH * 2, STAGE = 2 * HTILE_BYTES + 2 * B_BYTES, MINE = NT / 2;
     constexpr uint32_t COLS = 2 * NT, DESC = idesc_16(NT, 0);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int slices = (chunks + SLICE - 1) / SLICE;
     if (threadIdx.x == 0) {
         for (int s = 0; s < NSTAGE; ++s) {
             mbar_init(&ring.full[s], 1);
@@ -272,76 +282,88 @@ __device__ __forceinline__ bool pair_gemm(PairRing<NSTAGE> &ring, uint32_t smem_
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = ring.tmem;
+    // the roles count chunks and slices over all tiles of the CTA: stages and accumulators are used in turn throughout
     if (warp == 0) {
         if (lane == 0) {
-            for (int ch = 0; ch < chunks; ++ch) {
-                const int stage = ch % NSTAGE, round = ch / NSTAGE;
-                if (round > 0 && !mbar_wait(&ring.empty[stage], (round - 1) & 1)) { ring.failed = 1; break; }
-                mbar_expect_tx(&ring.full[stage], STAGE);
-                load(ch, smem_base + stage * STAGE, &ring.full[stage]);
+            PairTile tile;
+            int c = 0;
+            for (int it = 0; !ring.failed && next(it, tile); ++it) {
+                for (int ch = 0; ch < tile.chunks; ++ch, ++c) {
+                    const int stage = c % NSTAGE, round = c / NSTAGE;
+                    if (round > 0 && !mbar_wait(&ring.empty[stage], (round - 1) & 1)) { ring.failed = 1; break; }
+                    mbar_expect_tx(&ring.full[stage], STAGE);
+                    load(tile, ch, smem_base + stage * STAGE, &ring.full[stage]);
+                }
             }
         }
     } else if (warp == 1) {
         if (lane == 0) {
-            for (int ch = 0; ch < chunks; ++ch) {
-                const int stage = ch % NSTAGE, round = ch / NSTAGE;
-                const int slice = ch / SLICE, buf = slice & 1;
-                const bool opens = ch % SLICE == 0, closes = ch % SLICE == SLICE - 1 || ch == chunks - 1;
-                // the accumulator must have been read out by the warps of the slice two before
-                if (opens && slice >= 2 && !mbar_wait(&ring.acc_empty[buf], ((slice >> 1) - 1) & 1)) { ring.failed = 1; break; }
-                if (!mbar_wait(&ring.full[stage], round & 1)) { ring.failed = 1; break; }
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const uint32_t d = tmem + (uint32_t)(buf * NT);
-                const uint32_t a_hi = smem_base + stage * STAGE, a_lo = a_hi + HTILE_BYTES, b_hi = a_hi + 2 * HTILE_BYTES, b_lo = b_hi + B_BYTES;
+            PairTile tile;
+            int c = 0, slice = 0;
+            for (int it = 0; !ring.failed && next(it, tile); ++it) {
+                for (int ch = 0; ch < tile.chunks; ++ch, ++c) {
+                    const int stage = c % NSTAGE, round = c / NSTAGE, buf = slice & 1;
+                    const bool opens = ch % SLICE == 0, closes = ch % SLICE == SLICE - 1 || ch == tile.chunks - 1;
+                    // the accumulator must have been read out by the warps of the slice two before
+                    if (opens && slice >= 2 && !mbar_wait(&ring.acc_empty[buf], ((slice >> 1) - 1) & 1)) { ring.failed = 1; break; }
+                    if (!mbar_wait(&ring.full[stage], round & 1)) { ring.failed = 1; break; }
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    const uint32_t d = tmem + (uint32_t)(buf * NT);
+                    const uint32_t a_hi = smem_base + stage * STAGE, a_lo = a_hi + HTILE_BYTES, b_hi = a_hi + 2 * HTILE_BYTES, b_lo = b_hi + B_BYTES;
 #pragma unroll
-                for (int ks = 0; ks < KH / 16; ++ks) {
-                    const uint32_t off = ks * 32;  // 16 values = 32 bytes along the swizzled row
-                    umma_16(d, umma_desc(a_hi + off), umma_desc(b_hi + off), DESC, (opens && ks == 0) ? 0u : 1u);
-                    umma_16(d, umma_desc(a_lo + off), umma_desc(b_hi + off), DESC, 1u);
-                    umma_16(d, umma_desc(a_hi + off), umma_desc(b_lo + off), DESC, 1u);
+                    for (int ks = 0; ks < KH / 16; ++ks) {
+                        const uint32_t off = ks * 32;  // 16 values = 32 bytes along the swizzled row
+                        umma_16(d, umma_desc(a_hi + off), umma_desc(b_hi + off), DESC, (opens && ks == 0) ? 0u : 1u);
+                        umma_16(d, umma_desc(a_lo + off), umma_desc(b_hi + off), DESC, 1u);
+                        umma_16(d, umma_desc(a_hi + off), umma_desc(b_lo + off), DESC, 1u);
+                    }
+                    umma_commit(&ring.empty[stage]);  // arrives when the MMAs above have read the stage
+                    if (closes) {
+                        umma_commit(&ring.acc_full[buf]);  // arrives when the slice is complete in tensor memory
+                        ++slice;
+                    }
                 }
-                umma_commit(&ring.empty[stage]);           // arrives when the MMAs above have read the stage
-                if (closes) umma_commit(&ring.acc_full[buf]);  // arrives when the slice is complete in tensor memory
             }
+            // on time-out, give what is in flight a bounded chance to land before its memory is released
+            if (ring.failed && slice > 0) mbar_wait(&ring.acc_full[(slice - 1) & 1], ((slice - 1) >> 1) & 1);
         }
     } else {
         const int q = warp & 3, c0 = ((warp - 2) >> 2) * MINE;
-        float total[MINE];
-#pragma unroll
-        for (int x = 0; x < MINE; ++x) total[x] = 0.f;
+        PairTile tile;
+        int slice = 0;
         bool go = true;
-        for (int slice = 0; slice < slices; ++slice) {
-            const int buf = slice & 1;
-            const bool ok = mbar_wait(&ring.acc_full[buf], (slice >> 1) & 1, 64);
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            if (!ok) ring.failed = 1;
-            go = __all_sync(0xffffffffu, ok && !ring.failed);  // warp-uniform: the tensor-memory loads are warp-wide
-            if (!go) break;
+        for (int it = 0; go && next(it, tile); ++it) {
+            const int slices = (tile.chunks + SLICE - 1) / SLICE;
+            float total[MINE];
 #pragma unroll
-            for (int cb = 0; cb < MINE / 32; ++cb) {
-                uint32_t v[32];
-                tmem_load_32(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(buf * NT + c0 + cb * 32), v);
+            for (int x = 0; x < MINE; ++x) total[x] = 0.f;
+            for (int s = 0; s < slices; ++s, ++slice) {
+                const int buf = slice & 1;
+                const bool ok = mbar_wait(&ring.acc_full[buf], (slice >> 1) & 1, 64);
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                if (!ok) ring.failed = 1;
+                go = __all_sync(0xffffffffu, ok && !ring.failed);  // warp-uniform: the tensor-memory loads are warp-wide
+                if (!go) break;
 #pragma unroll
-                for (int x = 0; x < 32; ++x) total[cb * 32 + x] += __uint_as_float(v[x]);
+                for (int cb = 0; cb < MINE / 32; ++cb) {
+                    uint32_t v[32];
+                    tmem_load_32(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(buf * NT + c0 + cb * 32), v);
+#pragma unroll
+                    for (int x = 0; x < 32; ++x) total[cb * 32 + x] += __uint_as_float(v[x]);
+                }
+                // this warp has read the accumulator: hand it back to the MMA warp
+                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&ring.acc_empty[buf]);
             }
-            // this warp has read the accumulator: hand it back to the MMA warp
-            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&ring.acc_empty[buf]);
+            if (go) finish(tile, q, lane, c0, total, smem_base + (uint32_t)(NSTAGE * STAGE + (warp - 2) * BOX_BYTES));
         }
-        // every chunk has been multiplied when the last slice is complete: the stages are free
-        if (go) finish(q, lane, c0, total, smem_base + (uint32_t)((warp - 2) * (MINE / 32) * BOX_BYTES));
+        box_wait();  // results that are still on their way out of shared memory
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
-    if (warp == 1) {
-        if (ring.failed) {
-            // give outstanding loads and MMAs a bounded chance to land before the memory they target is released
-            if (lane == 0) mbar_wait(&ring.acc_full[((slices - 1) & 1)], ((slices - 1) >> 1) & 1);
-            __syncwarp();
-        }
+    if (warp == 1)
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(COLS) : "memory");
-    }
     return ring.failed != 0;
 }
 
