@@ -102,149 +102,284 @@ __device__ __forceinline__ void zero_acc(F (&acc)[8][8]) {
 }
 
 // ---- step 1a: factor the diagonal block kb (bs x bs), M_kk = T_kk^T T_kk, and invert T_kk ----
-// One CTA of 16 x 16 threads; thread (ty, tx) keeps the entries (ty + 16 a, tx + 16 b) of the (symmetric) working
-// block in registers.  Step j (last row first): the owners of row j publish it, then everyone subtracts row j's outer
-// product, scaled by 1 / pivot, from its part of the leading j x j block.  Row j is never touched again, the rows
-// alternate between two buffers, so one barrier per step is enough.  Rows scaled by 1 / sqrt(pivot) are the factor.
+// One CTA of 256 threads; sixteen rows are factored at a time, the last ones first.  Warp 0 holds their columns 0 .. r0 + 15 in
+// registers, two per lane, and eliminates row after row: the pivot's column goes through shared memory to all lanes, the
+// pivot row is scaled and stored as a row of T.  Then all threads subtract the rows' Gram from what is left.  At the end four
+// warps invert the four 16 x 16 diagonal blocks of T by columns, and two doubling levels join them.  Bound by the chain of 64
+// pivots, about 190 cycles each.  At n = 1024 a step of 64 rows took 25 us with one barrier per pivot over the whole block
+// and exact divisions, 17 us now.
+constexpr int DTH = 256;
+constexpr int DS = 16;          // rows factored at a time
+constexpr int DLDS = FB + 4;    // shared row stride: rows are 16-byte multiples
 template <typename F>
-__global__ void __launch_bounds__(256) ldl_diag_kernel(LdlBatch<F> B, int step_down) {
+constexpr int diag_smem = (int)sizeof(F) * (2 * FB * DLDS + FB * FB / 4);
+
+// sqrt(d), its reciprocal and 1 / d of a pivot.  float: from the reciprocal square root approximation with one Newton step and
+// a residual correction each (within an ulp), without the branches of the exact divisions: three of those were 500 of a
+// step's 750 cycles.
+__device__ __forceinline__ void pivot_roots(float d, float &root, float &inv_root, float &inv) {
+    float r;
+    asm("rsqrt.approx.f32 %0, %1;" : "=f"(r) : "f"(d));
+    r = fmaf(0.5f * r, fmaf(-(d * r), r, 1.f), r);
+    const float s = d * r;
+    root = fmaf(fmaf(-s, s, d), 0.5f * r, s);
+    inv_root = r;
+    const float q = r * r;
+    inv = fmaf(fmaf(-d, q, 1.f), q, q);
+}
+__device__ __forceinline__ void pivot_roots(double d, double &root, double &inv_root, double &inv) {
+    root = sqrt(d);
+    inv_root = 1.0 / root;
+    inv = 1.0 / d;
+}
+
+template <typename F>
+__global__ void __launch_bounds__(DTH) ldl_diag_kernel(LdlBatch<F> B, int step_down) {
     LDL_PROBLEM(blockIdx.y)
     F *const tinv = Q.tinv;
     int *const flag = Q.flag;
-    __shared__ F S[FB][FB + 1];   // the block as loaded (lower triangle), later T in the lower and V^T in the upper triangle
-    __shared__ F rowbuf[2][FB];   // published rows of the even and odd steps
-    __shared__ F piv[FB];         // pivots
-    __shared__ F Vd[FB];          // diagonal of the inverse
-    __shared__ F Wt[FB * FB / 4]; // intermediate product of a doubling level
+    extern __shared__ __align__(16) unsigned char ldl_smem[];
+    F *const S = reinterpret_cast<F *>(ldl_smem);  // the block (lower triangle), later T
+    F *const V = S + FB * DLDS;                    // inverse of T, lower triangle
+    F *const Wt = V + FB * DLDS;                   // intermediate product of a doubling level
+    __shared__ __align__(16) F column[2][DS];  // the pivot's column of the even and odd steps
+    __shared__ F pivots[FB];                   // 1 / T[r][r]
     __shared__ int bad;
-    const int tid = threadIdx.x, ty = tid >> 4, tx = tid & 15;
+    constexpr int VLD = DLDS;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int64_t o = (int64_t)kb * FB;
     const int bs = (int)min((int64_t)FB, n - o);
-    if (tid == 0) bad = 0;
-    for (int idx = tid; idx < FB * FB; idx += 256) {
-        const int r = idx / FB, c = idx % FB;
-        F v = (F)0;
-        if (r < bs && c <= r) v = a[(o + r) * n + o + c];
-        if (r >= bs && r == c) v = (F)1;  // identity beyond a ragged block: its steps change nothing and the inverse stays finite
-        S[r][c] = v;
+    if (tid == 0) bad = FB + 1;  // none
+    F loaded[FB * FB / DTH];
+#pragma unroll
+    for (int t = 0; t < FB * FB / DTH; ++t) {
+        const int idx = t * DTH + tid, r = idx / FB, c = idx % FB;
+        // identity beyond a ragged block: its steps change nothing and the inverse stays finite
+        loaded[t] = r < bs && c <= r ? a[(o + r) * n + o + c] : (r >= bs && r == c ? (F)1 : (F)0);
+    }
+#pragma unroll
+    for (int t = 0; t < FB * FB / DTH; ++t) {
+        const int idx = t * DTH + tid, r = idx / FB, c = idx % FB;
+        S[r * DLDS + c] = loaded[t];
+        V[r * VLD + c] = (F)0;
     }
     __syncthreads();
-    F reg[FB / 16][FB / 16];
+#pragma unroll 1
+    for (int r0 = FB - DS; r0 >= 0; r0 -= DS) {
+        if (warp == 0) {
+            const int owner = r0 & 16;       // first of the lanes that hold the rows' own columns, in the second set from 32 on
+            const bool second = r0 >= 32;    // columns 32 .. r0 + 15 are there
+            F v0[DS], v1[DS];                // register r: row r0 + r of columns lane and lane + 32 (by symmetry where it lies above the diagonal)
 #pragma unroll
-    for (int aa = 0; aa < FB / 16; ++aa)
-#pragma unroll
-        for (int bb = 0; bb < FB / 16; ++bb) {
-            const int i1 = ty + 16 * aa, i2 = tx + 16 * bb;
-            reg[aa][bb] = i1 >= i2 ? S[i1][i2] : S[i2][i1];
-        }
-#pragma unroll
-    for (int j = FB - 1; j >= 0; --j) {
-        if (ty == (j & 15)) {
-#pragma unroll
-            for (int bb = 0; bb < FB / 16; ++bb) rowbuf[j & 1][tx + 16 * bb] = reg[j / 16][bb];
-        }
-        __syncthreads();
-        const F d2 = rowbuf[j & 1][j];
-        if (tid == 0) {
-            piv[j] = d2;
-            if (j < bs && !(d2 > (F)0)) bad = j + 1;
-        }
-        const F inv_d2 = (F)1 / d2;
-        F rb[FB / 16];
-#pragma unroll
-        for (int bb = 0; bb < FB / 16; ++bb) rb[bb] = rowbuf[j & 1][tx + 16 * bb];
-#pragma unroll
-        for (int aa = 0; aa < FB / 16; ++aa) {
-            if (16 * aa < j) {  // known at compile time: later blocks of rows are final already
-                const int i1 = ty + 16 * aa;
-                const F f = rowbuf[j & 1][i1] * inv_d2;
-#pragma unroll
-                for (int bb = 0; bb < FB / 16; ++bb)
-                    if (16 * bb < j && i1 < j && tx + 16 * bb < j) reg[aa][bb] -= f * rb[bb];
+            for (int r = 0; r < DS; ++r) {
+                const int row = r0 + r, c1 = lane + 32;
+                v0[r] = row >= lane ? S[row * DLDS + lane] : S[lane * DLDS + row];
+                v1[r] = row >= c1 ? S[row * DLDS + c1] : S[c1 * DLDS + row];
             }
-        }
-    }
-    __syncthreads();
-    if (tid < FB) Vd[tid] = (F)1 / sqrt(piv[tid]);  // 1 / T[r][r]
-    __syncthreads();
+            int worst = FB + 1;
+            // The row that is eliminated sits in the last register: a step moves the others up by one, so that all steps are the
+            // same instructions and fit the instruction cache.
+#pragma unroll 2
+            for (int j = DS - 1; j >= 0; --j) {
+                F *const col = column[j & 1];
+                if (lane == owner + j) {
 #pragma unroll
-    for (int aa = 0; aa < FB / 16; ++aa)
+                    for (int r = 0; r < DS; ++r) col[r] = second ? v1[r] : v0[r];
+                }
+                __syncwarp();
+                F w[DS];
 #pragma unroll
-        for (int bb = 0; bb < FB / 16; ++bb) {
-            const int i1 = ty + 16 * aa, i2 = tx + 16 * bb;
-            if (i1 > i2) S[i1][i2] = reg[aa][bb] * Vd[i1];
-            if (i1 == i2) S[i1][i1] = sqrt(piv[i1]);
-        }
-    __syncthreads();
-    // Inverse V of the lower triangular T_kk.  The strict upper triangle of S is free, so V is kept transposed there
-    // (V[r][c] = S[c][r] for r > c) with its diagonal in Vd.  First the four 16 x 16 diagonal blocks by forward
-    // substitution (one thread per column), then two doubling levels, each completing pairs of finished blocks
-    // [A^{-1} 0; X B^{-1}] with X = -B^{-1} (C A^{-1}) as two small products over all threads.
-    if (tid < FB) {
-        const int c = tid, end = (tid & ~15) + 16;
-        for (int r = c + 1; r < end; ++r) {
-            F acc = -S[r][c] * Vd[c];
-#pragma unroll 4
-            for (int k = c + 1; k < r; ++k) acc -= S[r][k] * S[c][k];
-            S[c][r] = acc * Vd[r];
-        }
-    }
-    __syncthreads();
-    for (int b = 16; b < FB; b *= 2) {
-        const int outputs = (FB / (2 * b)) * b * b;
-        for (int idx = tid; idx < outputs; idx += 256) {  // W = C A^{-1}, C = T[second half rows][first half columns]
-            const int p = idx / (b * b), i = (idx / b) % b, j = idx % b, r0 = p * 2 * b, r1 = r0 + b;
-            F acc = S[r1 + i][r0 + j] * Vd[r0 + j];
-#pragma unroll 4
-            for (int k = j + 1; k < b; ++k) acc += S[r1 + i][r0 + k] * S[r0 + j][r0 + k];
-            Wt[idx] = acc;
+                for (int r = 0; r < DS; ++r) w[r] = col[r];
+                F root, inv_root, inv;
+                pivot_roots(w[DS - 1], root, inv_root, inv);
+                worst = r0 + j < bs && !(w[DS - 1] > (F)0) ? r0 + j + 1 : worst;
+                const F f0 = v0[DS - 1] * inv, f1 = v1[DS - 1] * inv;
+                // what lies right of the diagonal is stored along and never read
+                F *const row = S + (r0 + j) * DLDS;
+                row[lane] = lane == r0 + j ? root : v0[DS - 1] * inv_root;
+                if (second) row[lane + 32] = lane + 32 == r0 + j ? root : v1[DS - 1] * inv_root;
+                pivots[r0 + j] = inv_root;
+#pragma unroll
+                for (int r = DS - 1; r > 0; --r) {
+                    v0[r] = v0[r - 1] - f0 * w[r - 1];
+                    v1[r] = v1[r - 1] - f1 * w[r - 1];
+                }
+            }
+            if (lane == 0 && worst < bad) bad = worst;
         }
         __syncthreads();
-        for (int idx = tid; idx < outputs; idx += 256) {  // X = -B^{-1} W, stored transposed
-            const int p = idx / (b * b), i = (idx / b) % b, j = idx % b, r0 = p * 2 * b, r1 = r0 + b;
-            F acc = Vd[r1 + i] * Wt[idx];
+        if (r0 == 0) break;
+        // what is left: M[i][j] -= sum_k T[r0 + k][i] T[r0 + k][j], 4 x 4 entries per thread (the strict upper ones are not read)
+        const int ti = (tid / 12) * 4, tj = (tid % 12) * 4;
+        if (ti < r0 && tj <= ti) {
+            F d[4][4];
+#pragma unroll
+            for (int x = 0; x < 4; ++x)
+#pragma unroll
+                for (int y = 0; y < 4; ++y) d[x][y] = S[(ti + x) * DLDS + tj + y];
 #pragma unroll 4
-            for (int k = 0; k < i; ++k) acc += S[r1 + k][r1 + i] * Wt[(p * b + k) * b + j];
-            S[r0 + j][r1 + i] = -acc;
+            for (int k = 0; k < DS; ++k) {
+                F p[4], q[4];
+#pragma unroll
+                for (int x = 0; x < 4; ++x) {
+                    p[x] = S[(r0 + k) * DLDS + ti + x];
+                    q[x] = S[(r0 + k) * DLDS + tj + x];
+                }
+#pragma unroll
+                for (int x = 0; x < 4; ++x)
+#pragma unroll
+                    for (int y = 0; y < 4; ++y) d[x][y] -= p[x] * q[y];
+            }
+#pragma unroll
+            for (int x = 0; x < 4; ++x)
+#pragma unroll
+                for (int y = 0; y < 4; ++y) S[(ti + x) * DLDS + tj + y] = d[x][y];
         }
         __syncthreads();
     }
-    for (int idx = tid; idx < FB * FB; idx += 256) {
-        const int r = idx / FB, c = idx % FB;
-        tinv[(int64_t)kb * FB * FB + idx] = (r < bs && c < bs && r >= c) ? (r == c ? Vd[r] : S[c][r]) : (F)0;
+    // inverses of the four diagonal blocks, one per warp, column c per lane: once an entry is known it is subtracted from those
+    // below, which move up by one register
+    if (warp < FB / DS) {
+        const int r0 = warp * DS, c = lane & (DS - 1);
+        F x[DS];
+#pragma unroll
+        for (int r = 0; r < DS; ++r) x[r] = r == c ? (F)1 : (F)0;
+#pragma unroll 4
+        for (int k = 0; k < DS; ++k) {
+            F t[DS - 1];  // T below (r0 + k, r0 + k); past the block's end: read, never used
+#pragma unroll
+            for (int r = 0; r < DS - 1; ++r) t[r] = S[(r0 + k + 1 + r) * DLDS + r0 + k];
+            const F xk = x[0] * pivots[r0 + k];
+#pragma unroll
+            for (int r = 0; r < DS - 1; ++r) x[r] = x[r + 1] - t[r] * xk;
+            V[(r0 + k) * VLD + r0 + c] = xk;  // zero above the diagonal; both halves of the warp store the same
+        }
     }
-    for (int idx = tid; idx < FB * FB; idx += 256) {
-        const int r = idx / FB, c = idx % FB;
-        if (r < bs && c < bs && r >= c) a[(o + r) * n + o + c] = S[r][c];
+    __syncthreads();
+    // doubling: X = -B^{-1} (C A^{-1}) completes pairs of finished blocks; 2 x 2 outputs per thread and round
+#pragma unroll 1
+    for (int b = DS; b < FB; b *= 2) {
+        const int half = b / 2, pairs = FB / (2 * b), cells = pairs * half * half;
+        for (int idx = tid; idx < cells; idx += DTH) {  // W = C A^{-1}, C = T[second half rows][first half columns]
+            const int p = idx / (half * half), i = (idx / half) % half * 2, j = idx % half * 2, s0 = p * 2 * b, s1 = s0 + b;
+            F w[2][2] = {{(F)0, (F)0}, {(F)0, (F)0}};
+#pragma unroll 4
+            for (int k = 0; k < b; k += 4) {  // the inverse has zeros above its diagonal
+                F c0[4], c1[4];
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    c0[e] = S[(s1 + i) * DLDS + s0 + k + e];
+                    c1[e] = S[(s1 + i + 1) * DLDS + s0 + k + e];
+                }
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    const F v0 = V[(s0 + k + e) * VLD + s0 + j], v1 = V[(s0 + k + e) * VLD + s0 + j + 1];
+                    w[0][0] += c0[e] * v0; w[0][1] += c0[e] * v1;
+                    w[1][0] += c1[e] * v0; w[1][1] += c1[e] * v1;
+                }
+            }
+#pragma unroll
+            for (int x = 0; x < 2; ++x)
+#pragma unroll
+                for (int y = 0; y < 2; ++y) Wt[(p * b + i + x) * b + j + y] = w[x][y];
+        }
+        __syncthreads();
+        for (int idx = tid; idx < cells; idx += DTH) {  // X = -B^{-1} W
+            const int p = idx / (half * half), i = (idx / half) % half * 2, j = idx % half * 2, s0 = p * 2 * b, s1 = s0 + b;
+            F x[2][2] = {{(F)0, (F)0}, {(F)0, (F)0}};
+#pragma unroll 4
+            for (int k = 0; k < b; k += 4) {
+                F v0[4], v1[4];
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    v0[e] = V[(s1 + i) * VLD + s1 + k + e];
+                    v1[e] = V[(s1 + i + 1) * VLD + s1 + k + e];
+                }
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    const F w0 = Wt[(p * b + k + e) * b + j], w1 = Wt[(p * b + k + e) * b + j + 1];
+                    x[0][0] -= v0[e] * w0; x[0][1] -= v0[e] * w1;
+                    x[1][0] -= v1[e] * w0; x[1][1] -= v1[e] * w1;
+                }
+            }
+#pragma unroll
+            for (int e = 0; e < 2; ++e)
+#pragma unroll
+                for (int y = 0; y < 2; ++y) V[(s1 + i + e) * VLD + s0 + j + y] = x[e][y];
+        }
+        __syncthreads();
     }
-    if (tid == 0 && bad && flag) atomicCAS(flag, 0, (int)(o + bad));
+    for (int idx = tid; idx < FB * FB; idx += DTH) {
+        const int r = idx / FB, c = idx % FB;
+        tinv[(int64_t)kb * FB * FB + idx] = (r < bs && c < bs && r >= c) ? V[r * VLD + c] : (F)0;
+        if (r < bs && c < bs && r >= c) a[(o + r) * n + o + c] = S[r * DLDS + c];
+    }
+    if (tid == 0 && bad <= FB && flag) atomicCAS(flag, 0, (int)(o + bad));
+}
+
+// ---- products with one block row (at most 64 rows): 64 x 64 outputs, 4 x 4 per thread ----
+// acc[4][4] += sum_{k < K} A(k, 4 ty ..) B(k, 4 tx ..); both operands are staged whole (float; double in two halves) with
+// coalesced rows, so a CTA waits for memory once: these launches are short and the next step waits for them.
+constexpr int CTH = 256;
+constexpr int CLD = FB + 4;
+template <typename F>
+constexpr int chain_k = sizeof(F) == 4 ? 64 : 32;
+template <typename F, typename LA, typename LB>
+__device__ __forceinline__ void chain_product(F (&acc)[4][4], int K, LA la, LB lb, F *As, F *Bs) {
+    constexpr int CK = chain_k<F>, PER = CK * FB / CTH;
+    const int tid = threadIdx.x, ty = tid >> 4, tx = tid & 15;
+    for (int k0 = 0; k0 < K; k0 += CK) {
+        F ra[PER], rb[PER];
+#pragma unroll
+        for (int t = 0; t < PER; ++t) {
+            const int idx = t * CTH + tid, k = k0 + idx / FB, c = idx % FB;
+            ra[t] = k < K ? la(k, c) : (F)0;
+            rb[t] = k < K ? lb(k, c) : (F)0;
+        }
+        __syncthreads();  // the previous half has been consumed
+#pragma unroll
+        for (int t = 0; t < PER; ++t) {
+            const int idx = t * CTH + tid;
+            As[(idx / FB) * CLD + idx % FB] = ra[t];
+            Bs[(idx / FB) * CLD + idx % FB] = rb[t];
+        }
+        __syncthreads();
+#pragma unroll 16
+        for (int k = 0; k < CK; ++k) {
+            F p[4], q[4];
+#pragma unroll
+            for (int x = 0; x < 4; ++x) p[x] = As[k * CLD + ty * 4 + x];
+#pragma unroll
+            for (int y = 0; y < 4; ++y) q[y] = Bs[k * CLD + tx * 4 + y];
+#pragma unroll
+            for (int x = 0; x < 4; ++x)
+#pragma unroll
+                for (int y = 0; y < 4; ++y) acc[x][y] += p[x] * q[y];
+        }
+    }
 }
 
 // ---- step 1b: block row to the left of the diagonal block: T[kb, j] = T_kk^{-T} M'[kb, j] ----
 template <typename F>
-__global__ void __launch_bounds__(FTH) ldl_trsm_kernel(LdlBatch<F> B, int step_down) {
+__global__ void __launch_bounds__(CTH) ldl_trsm_kernel(LdlBatch<F> B, int step_down) {
     LDL_PROBLEM(blockIdx.y)
     const F *const tinv = Q.tinv;
     if ((int)blockIdx.x >= kb) return;
-    __shared__ __align__(16) F As[FK * FLD];
-    __shared__ __align__(16) F Bs[FK * FLD];
+    __shared__ __align__(16) F As[chain_k<F> * CLD];
+    __shared__ __align__(16) F Bs[chain_k<F> * CLD];
     const int j = blockIdx.x;  // column tile, j < kb
     const int64_t o = (int64_t)kb * FB, c0 = (int64_t)j * FB;
     const int bs = (int)min((int64_t)FB, n - o);
     const F *ti = tinv + (int64_t)kb * FB * FB;
-    F acc[8][8];
-    zero_acc(acc);
-    // A(r, k) = Tinv[k][r] (transposed), B(k, col) = M'[o + k][c0 + col]
-    tile_product<F>(acc, bs, [&](int r, int64_t k) { return ti[k * FB + r]; },
-                    [&](int64_t k, int col) { return a[(o + k) * n + c0 + col]; }, As, Bs, false);
-    const int tid = threadIdx.x, ty = tid >> 3, tx = tid & 7;
+    F acc[4][4] = {};
+    // A(k, r) = Tinv[k][r], B(k, col) = M'[o + k][c0 + col]
+    chain_product<F>(acc, bs, [&](int k, int r) { return ti[k * FB + r]; }, [&](int k, int col) { return a[(o + k) * n + c0 + col]; }, As, Bs);
+    const int tid = threadIdx.x, ty = tid >> 4, tx = tid & 15;
 #pragma unroll
-    for (int x = 0; x < 8; ++x) {
-        const int r = own8(ty, x);
+    for (int x = 0; x < 4; ++x)
 #pragma unroll
-        for (int y = 0; y < 8; ++y)
-            if (r < bs) a[(o + r) * n + c0 + own8(tx, y)] = acc[x][y];
-    }
+        for (int y = 0; y < 4; ++y)
+            if (ty * 4 + x < bs) a[(o + ty * 4 + x) * n + c0 + tx * 4 + y] = acc[x][y];
     if constexpr (std::is_same<F, float>::value) {
         // tensor-core problems: the finished block row, transposed and split, is an operand of the group's trailing
         // update (columns left of the group only); rows beyond a ragged block are zero in acc already
@@ -252,23 +387,27 @@ __global__ void __launch_bounds__(FTH) ldl_trsm_kernel(LdlBatch<F> B, int step_d
         if (Q.tc && j < kb_lo) {
             __half *hi = Q.pt_hi[(kb / GROUP) & 1], *lo = Q.pt_lo[(kb / GROUP) & 1];
             const int k0 = (kb - kb_lo) * FB;
+            __syncthreads();
+            F *const Ts = As;  // [column][k], row stride 65
 #pragma unroll
-            for (int y = 0; y < 8; ++y) {
-                const int64_t c = c0 + own8(tx, y);
+            for (int x = 0; x < 4; ++x)
 #pragma unroll
-                for (int half = 0; half < 2; ++half) {
-                    __align__(8) __half h[4];
-                    __align__(8) __half l[4];
+                for (int y = 0; y < 4; ++y) Ts[(tx * 4 + y) * (FB + 1) + ty * 4 + x] = acc[x][y] * SYRK_PANEL_SCALE;
+            __syncthreads();
 #pragma unroll
-                    for (int e = 0; e < 4; ++e) {
-                        const float v = acc[4 * half + e][y] * SYRK_PANEL_SCALE;
-                        h[e] = __float2half_rn(v);
-                        l[e] = __float2half_rn(v - __half2float(h[e]));
-                    }
-                    const int64_t at = c * (GROUP * FB) + k0 + own8(ty, 4 * half);
-                    *reinterpret_cast<uint2 *>(hi + at) = *reinterpret_cast<const uint2 *>(h);
-                    *reinterpret_cast<uint2 *>(lo + at) = *reinterpret_cast<const uint2 *>(l);
+            for (int t = 0; t < FB * FB / 8 / CTH; ++t) {
+                const int idx = t * CTH + tid, c = idx >> 3, k = (idx & 7) * 8;
+                __align__(16) __half h[8];
+                __align__(16) __half l[8];
+#pragma unroll
+                for (int e = 0; e < 8; ++e) {
+                    const float v = Ts[c * (FB + 1) + k + e];
+                    h[e] = __float2half_rn(v);
+                    l[e] = __float2half_rn(v - __half2float(h[e]));
                 }
+                const int64_t at = (c0 + c) * (GROUP * FB) + k0 + k;
+                *reinterpret_cast<uint4 *>(hi + at) = *reinterpret_cast<const uint4 *>(h);
+                *reinterpret_cast<uint4 *>(lo + at) = *reinterpret_cast<const uint4 *>(l);
             }
         }
     }
@@ -276,34 +415,38 @@ __global__ void __launch_bounds__(FTH) ldl_trsm_kernel(LdlBatch<F> B, int step_d
 
 // ---- step 1c: M'[TI, TJ] -= T[kb, TI]^T T[kb, TJ] for TJ <= TI < kb (lower triangle of tiles) ----
 template <typename F>
-__global__ void __launch_bounds__(FTH) ldl_syrk_kernel(LdlBatch<F> B, int step_down) {
+__global__ void __launch_bounds__(CTH) ldl_syrk_kernel(LdlBatch<F> B, int step_down) {
     LDL_PROBLEM(blockIdx.y)
     // tile pairs (TI, TJ), TJ <= TI < kb, in row order.  A tensor-core problem updates only the block rows of its own
     // group here (TI >= first block row of the group); the rows above wait for the group's update.
     const int kb_lo = Q.tc ? kb / GROUP * GROUP : 0;
     const int64_t first = (int64_t)kb_lo * (kb_lo + 1) / 2;
     if ((int64_t)blockIdx.x >= (int64_t)kb * (kb + 1) / 2 - first) return;
-    __shared__ __align__(16) F As[FK * FLD];
-    __shared__ __align__(16) F Bs[FK * FLD];
-    // linear index -> (TI, TJ) with TJ <= TI
-    const int64_t lin = first + blockIdx.x;
-    int TI = (int)((sqrt(8.0 * (double)lin + 1.0) - 1.0) / 2.0);
-    while ((int64_t)(TI + 1) * (TI + 2) / 2 <= lin) ++TI;
-    while ((int64_t)TI * (TI + 1) / 2 > lin) --TI;
+    __shared__ __align__(16) F As[chain_k<F> * CLD];
+    __shared__ __align__(16) F Bs[chain_k<F> * CLD];
+    // linear index -> (TI, TJ) with TJ <= TI: few rows in a group, so walk there; else from the square root
+    int64_t lin = first + blockIdx.x;
+    int TI;
+    if (Q.tc) {
+        TI = kb_lo;
+        while ((int64_t)(TI + 1) * (TI + 2) / 2 <= lin) ++TI;
+    } else {
+        TI = (int)((sqrt(8.0 * (double)lin + 1.0) - 1.0) / 2.0);
+        while ((int64_t)(TI + 1) * (TI + 2) / 2 <= lin) ++TI;
+        while ((int64_t)TI * (TI + 1) / 2 > lin) --TI;
+    }
     const int TJ = (int)(lin - (int64_t)TI * (TI + 1) / 2);
     const int64_t o = (int64_t)kb * FB, r0 = (int64_t)TI * FB, c0 = (int64_t)TJ * FB;
     const int bs = (int)min((int64_t)FB, n - o);
-    F acc[8][8];
-    zero_acc(acc);
-    tile_product<F>(acc, bs, [&](int i, int64_t k) { return a[(o + k) * n + r0 + i]; },
-                    [&](int64_t k, int j) { return a[(o + k) * n + c0 + j]; }, As, Bs, false);
-    const int tid = threadIdx.x, ty = tid >> 3, tx = tid & 7;
+    F acc[4][4] = {};
+    chain_product<F>(acc, bs, [&](int k, int i) { return a[(o + k) * n + r0 + i]; }, [&](int k, int j) { return a[(o + k) * n + c0 + j]; }, As, Bs);
+    const int tid = threadIdx.x, ty = tid >> 4, tx = tid & 15;
 #pragma unroll
-    for (int x = 0; x < 8; ++x) {
-        const int64_t r = r0 + own8(ty, x);
+    for (int x = 0; x < 4; ++x) {
+        const int64_t r = r0 + ty * 4 + x;
 #pragma unroll
-        for (int y = 0; y < 8; ++y) {
-            const int64_t c = c0 + own8(tx, y);
+        for (int y = 0; y < 4; ++y) {
+            const int64_t c = c0 + tx * 4 + y;
             if (c <= r) a[r * n + c] -= acc[x][y];
         }
     }
@@ -525,6 +668,9 @@ int ldl_run(int count, const int64_t *ns, F *const *as, const int *sizes, F *con
     // bulk of the update.  rest(g) touches the groups <= g - 2: group g needs rest(g + 2) and older before its first
     // kernel (which also frees the panel planes that it reuses), and next(g) must follow rest(g + 1), whose targets
     // it shares (the order of the additions is fixed, hence the result).
+    static PerDeviceOnce configured;
+    if (configured.run([&] { return cudaFuncSetAttribute(ldl_diag_kernel<F>, cudaFuncAttributeMaxDynamicSharedMemorySize, diag_smem<F>) == cudaSuccess; }) != G2D_OK)
+        return G2D_ERR_CUDA;
     SideLane *lane = acquire_side_lane();
     if (!lane) return G2D_ERR_CUDA;
     if (cudaEventRecord(lane->fork, caller) != cudaSuccess || cudaStreamWaitEvent(lane->chain, lane->fork, 0) != cudaSuccess) return G2D_ERR_CUDA;
@@ -538,7 +684,7 @@ int ldl_run(int count, const int64_t *ns, F *const *as, const int *sizes, F *con
     for (int s = B.steps - 1; s >= 0; --s) {  // block row of the largest problem; smaller problems are lined up by groups
         const int g = s / GROUP;
         if (s % GROUP == GROUP - 1 && !wait_rest(g + 2)) return G2D_ERR_CUDA;
-        ldl_diag_kernel<F><<<dim3(1, count), 256, 0, st>>>(B, s);
+        ldl_diag_kernel<F><<<dim3(1, count), DTH, diag_smem<F>, st>>>(B, s);
         if (check_launch() != G2D_OK) return G2D_ERR_CUDA;
         if (s == 0) break;
         int64_t panel_tiles = 0, update_tiles = 0;
@@ -551,11 +697,11 @@ int ldl_run(int count, const int64_t *ns, F *const *as, const int *sizes, F *con
             update_tiles = tiles > update_tiles ? tiles : update_tiles;
         }
         if (panel_tiles > 0) {
-            ldl_trsm_kernel<F><<<dim3((unsigned)panel_tiles, count), FTH, 0, st>>>(B, s);
+            ldl_trsm_kernel<F><<<dim3((unsigned)panel_tiles, count), CTH, 0, st>>>(B, s);
             if (check_launch() != G2D_OK) return G2D_ERR_CUDA;
         }
         if (update_tiles > 0) {
-            ldl_syrk_kernel<F><<<dim3((unsigned)update_tiles, count), FTH, 0, st>>>(B, s);
+            ldl_syrk_kernel<F><<<dim3((unsigned)update_tiles, count), CTH, 0, st>>>(B, s);
             if (check_launch() != G2D_OK) return G2D_ERR_CUDA;
         }
         if (s % GROUP != 0 || !any_tc) continue;
