@@ -74,14 +74,51 @@ constexpr int kDefaultOuterTiles = 8;  // tile anti-diagonals gathered into one 
 
 inline size_t align256(size_t v) { return (v + 255) & ~(size_t)255; }
 
-// The tensor-core macro updates serve one float matrix whose rows are 16-byte multiples (a TMA requirement).
+// The tensor-core schedules serve one float matrix.  TMA wants rows of 16-byte multiples: the operand planes have them in any
+// case; rows of Y, L and U that are not are copied to padded rows first (Y also back), one pass over each.  The macro schedule,
+// which only runs on request, takes sizes that need no copy.
 inline bool tc_eligible(const g2d_sweep_desc *d) {
-    return d->dtype == G2D_F32 && d->batch == 1 && d->m % 4 == 0 && d->n % 4 == 0 && d->reserved != 1;
+    return d->dtype == G2D_F32 && d->batch == 1 && d->reserved != 1 && (d->reserved != 2 || (d->m % 4 == 0 && d->n % 4 == 0));
 }
-inline size_t tc_extra_bytes(const g2d_sweep_desc *d) {
-    const size_t mn = align256(4 * (size_t)d->m * d->n), mm = align256(4 * (size_t)d->m * d->m), nn = align256(4 * (size_t)d->n * d->n);
-    return 256 + 4 * mn + 2 * mm + 2 * nn + 4 * mn;  // flag, E^T and C splits, L and U^T splits, far and neighbour planes of the pipelined schedule
+inline int64_t round_up(int64_t v, int64_t to) { return (v + to - 1) / to * to; }
+inline int64_t sweep_pitch(const g2d_sweep_desc *d) { return tc_eligible(d) ? round_up(d->n, 4) : d->n; }  // of Y, C, E and their kin
+inline size_t base_plane(const g2d_sweep_desc *d) { return align256((d->dtype == G2D_F32 ? 4 : 8) * (size_t)d->batch * d->m * sweep_pitch(d)); }
+
+// What the tensor-core schedules keep behind C and E
+struct TcWorkspace {
+    TcPlanes planes;
+    float *yf, *cf, *yn, *cn;  // far and neighbour planes of the pipelined schedule
+    float *y, *l, *u;          // padded copies, where the rows need them (else null)
+    size_t bytes;
+};
+inline TcWorkspace tc_carve(const g2d_sweep_desc *d, char *base) {
+    TcWorkspace w;
+    size_t at = 0;
+    auto take = [&](size_t bytes) {
+        char *p = base + at;
+        at += align256(bytes);
+        return p;
+    };
+    TcPlanes &pl = w.planes;
+    const int64_t m = d->m, n = d->n, ld = sweep_pitch(d), nI = ceil_div(m, (int64_t)TILE), nJ = ceil_div(n, (int64_t)TILE);
+    pl.ldm = round_up(m, 8);
+    pl.ldn = round_up(n, 8);
+    pl.error_flag = (int *)take(sizeof(int));
+    for (__half **p : {&pl.et_hi, &pl.et_lo}) *p = (__half *)take(2 * n * pl.ldm);
+    for (__half **p : {&pl.c_hi, &pl.c_lo}) *p = (__half *)take(2 * m * pl.ldn);
+    for (__half **p : {&pl.l_hi, &pl.l_lo}) *p = (__half *)take(2 * m * pl.ldm);
+    for (__half **p : {&pl.ut_hi, &pl.ut_lo}) *p = (__half *)take(2 * n * pl.ldn);
+    for (float **p : {&pl.e_scale, &pl.c_scale}) *p = (float *)take(4 * nI * nJ);
+    pl.l_scale = (float *)take(4 * nI * nI);
+    pl.u_scale = (float *)take(4 * nJ * nJ);
+    for (float **p : {&w.yf, &w.cf, &w.yn, &w.cn}) *p = (float *)take(4 * m * ld);
+    w.y = n % 4 ? (float *)take(4 * m * ld) : nullptr;
+    w.l = m % 4 ? (float *)take(4 * m * round_up(m, 4)) : nullptr;
+    w.u = n % 4 ? (float *)take(4 * n * ld) : nullptr;
+    w.bytes = at;
+    return w;
 }
+inline size_t tc_extra_bytes(const g2d_sweep_desc *d) { return tc_carve(d, nullptr).bytes; }
 
 int check_sweep(const g2d_sweep_desc *d) {
     if (!d) return G2D_ERR_BAD_ARGUMENT;
@@ -97,7 +134,7 @@ template <typename F>
 int launch_macro_update(const BandArgs<F> &bm, const TcPlanes *planes, const MacroTcMaps *maps, cudaStream_t stream) {
     if (planes != nullptr) {
         if constexpr (sizeof(F) == sizeof(float))
-            return launch_macro_update_tc(maps, *planes, (float *)bm.y, (float *)bm.c, bm.m, bm.n, (int)bm.s0, (int)bm.s1, (int)bm.s_end, stream);
+            return launch_macro_update_tc(maps, *planes, bm.m, bm.n, (int)bm.s0, (int)bm.s1, (int)bm.s_end, stream);
     }
     return launch_band_update<F>(bm, stream);
 }
@@ -115,7 +152,7 @@ int sweep_macro(const g2d_sweep_desc *d, SweepArgs<F> &a, BandArgs<F> &b64, cuda
                 const TcPlanes *planes) {
     MacroTcMaps maps;
     if (planes != nullptr) {
-        const int status = macro_tc_prepare(&maps, *planes, d->m, d->n);
+        const int status = macro_tc_prepare(&maps, *planes, (float *)a.y, (float *)a.c, d->m, d->n, a.ld);
         if (status != G2D_OK) return status;
     }
     const int nI2 = (int)ceil_div(d->m, MACRO), nJ2 = (int)ceil_div(d->n, MACRO);
@@ -289,8 +326,7 @@ constexpr int kFarLagMacro = 1;  // a far update reaches the macro anti-diagonal
 // with it: the updates run on the SMs that the tile launch of the moment leaves free, and the far update may as well use
 // its full three-stage ring there.  Updates that share target planes are
 // ordered on one stream, so the additions have a fixed order.
-int sweep_pipelined(const g2d_sweep_desc *d, SweepArgs<float> &a, const TcPlanes &planes, float *yf, float *cf, cudaStream_t caller,
-                    LaunchTimer *timer, double *flops) {
+int sweep_pipelined(const g2d_sweep_desc *d, SweepArgs<float> &a, const TcPlanes &planes, cudaStream_t caller, LaunchTimer *timer, double *flops) {
     std::unique_lock<std::mutex> held;
     int lane_status = G2D_OK;
     PipeLane *lane = acquire_pipe_lane(caller, held, &lane_status);
@@ -300,10 +336,9 @@ int sweep_pipelined(const g2d_sweep_desc *d, SweepArgs<float> &a, const TcPlanes
     if (cudaEventRecord(lane->fork, caller) != cudaSuccess || cudaStreamWaitEvent(stream, lane->fork, 0) != cudaSuccess) return G2D_ERR_CUDA;
     BandTcMaps maps;
     MacroTcMaps far_maps;
-    int status = band_tc_prepare(&maps, planes, d->m, d->n);
-    if (status == G2D_OK) status = macro_tc_prepare(&far_maps, planes, d->m, d->n);
+    int status = band_tc_prepare(&maps, planes, a.y, a.c, d->m, d->n, a.ld);
+    if (status == G2D_OK) status = macro_tc_prepare(&far_maps, planes, (float *)a.yf, (float *)a.cf, d->m, d->n, a.ld);
     if (status != G2D_OK) return status;
-    a.yf = yf; a.cf = cf; a.neighbours = 1;
     const int waves = a.nI + a.nJ - 1;
     const int waves_macro = (int)(ceil_div(d->m, MACRO) + ceil_div(d->n, MACRO)) - 1;
     const int outer = d->outer_tiles > 0 ? (d->outer_tiles + 1) / 2 : kDefaultOuterMacro;  // macro anti-diagonals per far update
@@ -332,7 +367,7 @@ int sweep_pipelined(const g2d_sweep_desc *d, SweepArgs<float> &a, const TcPlanes
             const int t0 = s + 2, t1 = 2 * reach < waves - 1 ? 2 * reach : waves - 1;
             if (cudaStreamWaitEvent(lane->near, lane->swept[s & 7], 0) != cudaSuccess) return G2D_ERR_CUDA;
             if (timer) timer->begin_on(1, lane->near);
-            status = launch_band_tc(&maps, a.y, a.c, d->m, d->n, s, s + 1, t0, t1, outer, kFarLagMacro, planes.error_flag, lane->near);
+            status = launch_band_tc(&maps, planes, d->m, d->n, s, t0, t1, outer, kFarLagMacro, lane->near);
             if (timer) timer->end();
             if (status != G2D_OK) return status;
             if (flops) flops[1] += near_flops(d->m, d->n, s, t0, t1, outer, kFarLagMacro);
@@ -344,13 +379,13 @@ int sweep_pipelined(const g2d_sweep_desc *d, SweepArgs<float> &a, const TcPlanes
             if (cudaStreamWaitEvent(lane->far, lane->swept[s & 7], 0) != cudaSuccess) return G2D_ERR_CUDA;
             const int t_first = W1 + kFarLagMacro, t_split = t_first + outer < waves_macro ? t_first + outer : waves_macro;
             if (timer) timer->begin_on(2, lane->far);
-            status = launch_macro_update_tc(&far_maps, planes, yf, cf, d->m, d->n, W1 - outer, W1, t_split, lane->far, t_first, 3);
+            status = launch_macro_update_tc(&far_maps, planes, d->m, d->n, W1 - outer, W1, t_split, lane->far, t_first);
             if (timer) timer->end();
             if (status != G2D_OK) return status;
             if (cudaEventRecord(lane->far_first[g & 3], lane->far) != cudaSuccess) return G2D_ERR_CUDA;
             if (t_split < waves_macro) {
                 if (timer) timer->begin_on(2, lane->far);
-                status = launch_macro_update_tc(&far_maps, planes, yf, cf, d->m, d->n, W1 - outer, W1, waves_macro, lane->far, t_split, 3);
+                status = launch_macro_update_tc(&far_maps, planes, d->m, d->n, W1 - outer, W1, waves_macro, lane->far, t_split);
                 if (timer) timer->end();
                 if (status != G2D_OK) return status;
             }
@@ -363,7 +398,8 @@ int sweep_pipelined(const g2d_sweep_desc *d, SweepArgs<float> &a, const TcPlanes
     // join: what follows the call on the caller's stream follows everything the call did
     if (last_near >= 0 && cudaStreamWaitEvent(stream, lane->near_done[last_near & 7], 0) != cudaSuccess) return G2D_ERR_CUDA;
     if (last_far >= 0 && cudaStreamWaitEvent(stream, lane->far_done[last_far & 3], 0) != cudaSuccess) return G2D_ERR_CUDA;
-    status = launch_sweep_finish(planes.error_flag, d->status, a.y, d->m * d->n, stream);
+    if (a.y != d->y && cudaMemcpy2DAsync(d->y, d->n * 4, a.y, a.ld * 4, d->n * 4, d->m, cudaMemcpyDeviceToDevice, stream) != cudaSuccess) return G2D_ERR_CUDA;
+    status = launch_sweep_finish(planes.error_flag, d->status, (float *)d->y, d->m * d->n, stream);
     if (status != G2D_OK) return status;
     if (cudaEventRecord(lane->join, stream) != cudaSuccess || cudaStreamWaitEvent(caller, lane->join, 0) != cudaSuccess) return G2D_ERR_CUDA;
     return G2D_OK;
@@ -476,8 +512,7 @@ int sweep_tiles_overlapped(const g2d_sweep_desc *d, SweepArgs<F> &a, F *planes, 
 
 template <typename F>
 int sweep_fused(const g2d_sweep_desc *d, cudaStream_t stream, LaunchTimer *timer = nullptr, double *flops = nullptr) {
-    const int64_t count = d->batch * d->m * d->n;
-    const size_t plane = align256(sizeof(F) * (size_t)count);
+    const size_t plane = base_plane(d);
     const bool tc = tc_eligible(d);
     const size_t extra = tc ? tc_extra_bytes(d) : overlap_eligible(d) ? overlap_planes<F>() * plane : 0;
     if (!d->workspace || d->workspace_bytes < 2 * plane + extra) return G2D_ERR_WORKSPACE;
@@ -498,38 +533,44 @@ int sweep_fused(const g2d_sweep_desc *d, cudaStream_t stream, LaunchTimer *timer
     a.kind = d->quant_kind;
     a.batch = d->batch; a.m = d->m; a.n = d->n;
     a.nI = (int)ceil_div(d->m, TILE); a.nJ = (int)ceil_div(d->n, TILE);
-    a.ld = d->n; a.ldl = d->m; a.ldu = d->n; a.ldm = d->m;
-    if (cudaMemsetAsync(a.c, 0, sizeof(F) * (size_t)count, stream) != cudaSuccess) return G2D_ERR_CUDA;
+    a.ld = sweep_pitch(d); a.ldl = d->m; a.ldu = d->n;
+    if (cudaMemsetAsync(a.c, 0, sizeof(F) * (size_t)d->batch * d->m * a.ld, stream) != cudaSuccess) return G2D_ERR_CUDA;
 
     BandArgs<F> b;
     b.y = a.y; b.c = a.c; b.e = a.e; b.l = a.l; b.u = a.u; b.l_off = a.l_off; b.u_off = a.u_off;
     b.batch = a.batch; b.m = a.m; b.n = a.n; b.P = TILE; b.Q = TILE; b.down_into_y = 0; b.mode = BAND_TILE; b.filter = 0;
     if (tc) {
-        // carve the operand planes behind C and E, prepare the static operands, run the macro schedule
-        char *p = (char *)d->workspace + 2 * plane;
-        const size_t mn = align256(4 * (size_t)d->m * d->n), mm = align256(4 * (size_t)d->m * d->m), nn = align256(4 * (size_t)d->n * d->n);
-        TcPlanes planes;
-        planes.error_flag = (int *)p; p += 256;
-        planes.et_hi = (float *)p; p += mn; planes.et_lo = (float *)p; p += mn;
-        planes.c_hi = (float *)p; p += mn; planes.c_lo = (float *)p; p += mn;
-        planes.l_hi = (float *)p; p += mm; planes.l_lo = (float *)p; p += mm;
-        planes.ut_hi = (float *)p; p += nn; planes.ut_lo = (float *)p; p += nn;
-        if (((uintptr_t)d->y & 15) != 0) return G2D_ERR_BAD_ARGUMENT;
-        if (cudaMemsetAsync(planes.error_flag, 0, sizeof(int), stream) != cudaSuccess) return G2D_ERR_CUDA;
-        const int status = tc_prepare_operands((const float *)d->l, (const float *)d->u, d->m, d->n, planes, stream);
-        if (status != G2D_OK) return status;
-        a.et_hi = planes.et_hi; a.et_lo = planes.et_lo; a.c_hi = planes.c_hi; a.c_lo = planes.c_lo;
         if constexpr (sizeof(F) == sizeof(float)) {
-            if (d->reserved == 3 || d->reserved == 0) {
-                float *yf = (float *)p, *cf = (float *)(p + mn);
-                a.yn = (float *)(p + 2 * mn); a.cn = (float *)(p + 3 * mn);  // written before they are read: no clearing
-                if (cudaMemsetAsync(yf, 0, 2 * mn, stream) != cudaSuccess) return G2D_ERR_CUDA;
-                return sweep_pipelined(d, a, planes, yf, cf, stream, timer, flops);
+            const TcWorkspace w = tc_carve(d, (char *)d->workspace + 2 * plane);
+            const TcPlanes &planes = w.planes;
+            if (w.y == nullptr && ((uintptr_t)d->y & 15) != 0) return G2D_ERR_BAD_ARGUMENT;
+            if (cudaMemsetAsync(planes.error_flag, 0, sizeof(int), stream) != cudaSuccess) return G2D_ERR_CUDA;
+            auto padded = [&](float *to, int64_t pitch, const void *from, int64_t rows, int64_t cols) {
+                return cudaMemcpy2DAsync(to, 4 * pitch, from, 4 * cols, 4 * cols, rows, cudaMemcpyDeviceToDevice, stream) == cudaSuccess;
+            };
+            if (w.y) {
+                if (!padded(w.y, a.ld, d->y, d->m, d->n) || !padded(w.u, a.ld, d->u, d->n, d->n)) return G2D_ERR_CUDA;
+                a.y = w.y; a.u = w.u; a.ldu = a.ld;
             }
+            if (w.l) {
+                a.ldl = round_up(d->m, 4);
+                if (!padded(w.l, a.ldl, d->l, d->m, d->m)) return G2D_ERR_CUDA;
+                a.l = w.l;
+            }
+            const int status = tc_prepare_operands(a.l, a.ldl, a.u, a.ldu, d->m, d->n, planes, stream);
+            if (status != G2D_OK) return status;
+            a.et_hi = planes.et_hi; a.et_lo = planes.et_lo; a.c_hi = planes.c_hi; a.c_lo = planes.c_lo;
+            a.e_scale = planes.e_scale; a.c_scale = planes.c_scale; a.ldm = planes.ldm; a.ldn = planes.ldn;
+            if (d->reserved != 2) {
+                a.yf = w.yf; a.cf = w.cf;
+                a.yn = w.yn; a.cn = w.cn;  // written before they are read: no clearing
+                if (cudaMemsetAsync(w.yf, 0, (char *)w.yn - (char *)w.yf, stream) != cudaSuccess) return G2D_ERR_CUDA;
+                return sweep_pipelined(d, a, planes, stream, timer, flops);
+            }
+            const int swept = sweep_macro<F>(d, a, b, stream, timer, flops, &planes);
+            if (swept != G2D_OK) return swept;
+            return launch_sweep_finish(planes.error_flag, d->status, (float *)d->y, d->m * d->n, stream);
         }
-        const int swept = sweep_macro<F>(d, a, b, stream, timer, flops, &planes);
-        if (swept != G2D_OK) return swept;
-        return launch_sweep_finish(planes.error_flag, d->status, (float *)d->y, d->m * d->n, stream);
     }
     if (d->reserved == 2) return sweep_macro<F>(d, a, b, stream, timer, flops, nullptr);
     if (overlap_eligible(d)) return sweep_tiles_overlapped<F>(d, a, (F *)((char *)d->workspace + 2 * plane), plane, stream, timer, flops);
@@ -602,7 +643,7 @@ extern "C" int g2d_abi_version(void) { return 2; }
 extern "C" int g2d_sweep_workspace_bytes(const g2d_sweep_desc *desc, size_t *bytes) {
     const int status = check_sweep(desc);
     if (status != G2D_OK || !bytes) return status != G2D_OK ? status : G2D_ERR_BAD_ARGUMENT;
-    const size_t plane = align256((desc->dtype == G2D_F32 ? 4 : 8) * (size_t)(desc->batch * desc->m * desc->n));
+    const size_t plane = base_plane(desc);
     const int planes = !overlap_eligible(desc) ? 0 : desc->dtype == G2D_F32 ? overlap_planes<float>() : overlap_planes<double>();
     *bytes = (2 + planes) * plane + (tc_eligible(desc) ? tc_extra_bytes(desc) : 0);
     return G2D_OK;
@@ -637,7 +678,7 @@ extern "C" int g2d_sweep_fused_profile(const g2d_sweep_desc *desc, void *stream,
     if (cudaStreamSynchronize(st) != cudaSuccess) status = status == G2D_OK ? G2D_ERR_CUDA : status;
     if (status == G2D_OK && tc_eligible(desc)) {
         // the tensor-core kernels report a bounded wait that ran out through a flag behind the C and E planes
-        const size_t elem = 4, plane = align256(elem * (size_t)(desc->batch * desc->m * desc->n));
+        const size_t plane = base_plane(desc);
         int flag = 0;
         if (cudaMemcpy(&flag, (const char *)desc->workspace + 2 * plane, sizeof(int), cudaMemcpyDeviceToHost) != cudaSuccess || flag != 0)
             status = G2D_ERR_CUDA;

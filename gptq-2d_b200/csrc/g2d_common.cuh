@@ -157,51 +157,62 @@ struct SweepArgs {
     int kind;
     int64_t batch, m, n;
     int nI, nJ;  // tiles per column / per row
-    int64_t ld, ldl, ldu, ldm;  // row strides of Y, C, E and the planes; of L; of U; of the transposed planes
-    // float, single matrix, tensor-core updates only (else null): tf32 hi / lo copies of the finished tiles,
-    // E transposed ([n, m]) and the completed C ([m, n]), operands of the macro updates
-    float *et_hi = nullptr, *et_lo = nullptr, *c_hi = nullptr, *c_lo = nullptr;
+    int64_t ld, ldl, ldu;      // row strides of Y, C, E and the float planes; of L; of U
+    int64_t ldm = 0, ldn = 0;  // of E^T and of C among the operand planes
+    // float, single matrix, tensor-core updates only (else null): scaled fp16 pairs of the finished tiles, E transposed (rows of
+    // ldm values) and the completed C (rows of ldn), with the tiles' scales: operands of the updates (see TcPlanes)
+    __half *et_hi = nullptr, *et_lo = nullptr, *c_hi = nullptr, *c_lo = nullptr;
+    float *e_scale = nullptr, *c_scale = nullptr;
     // pipelined schedule only (else null / 0): planes that collect the far feedback apart from Y and C, added when a
-    // tile is loaded, and the switch that makes a tile apply the feedback of its two nearest finished neighbours itself
+    // tile is loaded
     const F *yf = nullptr, *cf = nullptr;
-    int neighbours = 0;
     // pipelined schedule only: the planes through which a tile hands the feedback for its lower and its right neighbour
     // on (the neighbour adds them when it loads); every entry that is read has been written one launch before
     F *yn = nullptr, *cn = nullptr;
 };
 
-// fp32 -> tf32 hi (round to nearest) and the fp32 remainder: a = hi + lo exactly, and hi*hi' + lo*hi' + hi*lo' recovers
-// the fp32 product to about 2^-21 relative
-__device__ __forceinline__ void split_tf32(float a, float &hi, float &lo) {
-    uint32_t h;
-    asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(h) : "f"(a));
-    hi = __uint_as_float(h);
-    lo = a - hi;
+// Float operands as fp16 pairs.  A value times a power of two, chosen so that the largest value it shares its scale with lies
+// in [2^14, 2^15), is hi + lo with 11 significant bits each: relative error 2^-23 down to 2^-17 of the largest value (the same
+// as a tf32 pair), an absolute error of 2^-40 of it below.  The three products hi hi + lo hi + hi lo then cost half of
+// their tf32 counterparts in tensor cycles and operand bytes.  `range_exponent` is the power: x 2^-e in (2^14, 2^15].
+__device__ __forceinline__ int range_exponent(float largest) {
+    const int e = (int)((__float_as_uint(largest) >> 23) & 255) - 127;  // largest in [2^e, 2^(e + 1))
+    return e == 128 ? 0 : (e < -100 ? -100 : e) - 14;                   // infinities and NaN stay what they are; zeros and tiny rows: any scale
+}
+__device__ __forceinline__ float power_of_two(int e) { return __uint_as_float((uint32_t)(e + 127) << 23); }  // -126 <= e <= 127
+__device__ __forceinline__ void split_half(float scaled, __half &hi, __half &lo) {
+    hi = __float2half_rn(scaled);
+    lo = __float2half_rn(scaled - __half2float(hi));
 }
 
-// Operand planes of the tensor-core macro updates (all float; see g2d_macro_update_tc.cu).
+// Operand planes of the tensor-core updates of the sweep (see g2d_macro_update_tc.cu): fp16 pairs, K-major, each 64 x 64 tile under
+// a power of two of its own.  A slice of k is one tile wide, so the scales come out of a product slice by slice:
+// `*_scale` holds what a product with the tile has to be multiplied by.
 struct TcPlanes {
-    float *et_hi, *et_lo, *c_hi, *c_lo;  // written by the tile sweep
-    float *l_hi, *l_lo, *ut_hi, *ut_lo;  // written once per sweep from L and U
-    int *error_flag;                     // set when a bounded wait inside a kernel ran out
+    __half *et_hi, *et_lo, *c_hi, *c_lo;  // E^T [n][ldm] and the completed C [m][ldn], written by the tile sweep
+    __half *l_hi, *l_lo, *ut_hi, *ut_lo;  // L [m][ldm] and U^T [n][ldn], below the diagonal tiles, written once per sweep
+    float *e_scale, *c_scale;             // [nI][nJ]
+    float *l_scale, *u_scale;             // [nI][nI], [nJ][nJ] (tile row of U^T, tile of k)
+    int64_t ldm, ldn;                     // m and n rounded up to multiples of 8 (rows of 16-byte multiples, a TMA requirement)
+    int *error_flag;                      // set when a bounded wait inside a kernel ran out
 };
-// Band updates between tiles on the tensor cores (pipelined schedule; see g2d_band_tc.cu): sources are the tile
-// anti-diagonals s0..s1-1, targets t0..t1 (t0 >= s1 + 1), feedback is added into the planes y (right) and c (down).
+// Band updates between tiles on the tensor cores (pipelined schedule; see g2d_band_tc.cu): sources are the tiles of the
+// anti-diagonal s, targets those of t0..t1 (t0 >= s + 2), feedback is added into the planes y (right) and c (down) of the maps.
 // With outer_macro > 0 a target is left out when a far update on 128 x 128 macro tiles carries its source instead:
 // when its macro anti-diagonal is lag_macro or more past the end of the source's group of outer_macro macro anti-diagonals.
 struct BandTcMaps {
-    alignas(64) unsigned char bytes[8 * 128];  // tensor maps of the eight operand planes (opaque here)
+    alignas(64) unsigned char bytes[10 * 128];  // tensor maps of the eight operand planes and the two targets (opaque here)
 };
-int band_tc_prepare(BandTcMaps *maps, const TcPlanes &planes, int64_t m, int64_t n);
-int launch_band_tc(const BandTcMaps *maps, float *y, float *c, int64_t m, int64_t n, int s0, int s1, int t0, int t1, int outer_macro,
-                   int lag_macro, int *error_flag, cudaStream_t stream);
-int tc_prepare_operands(const float *l, const float *u, int64_t m, int64_t n, const TcPlanes &planes, cudaStream_t stream);
+int band_tc_prepare(BandTcMaps *maps, const TcPlanes &planes, float *y, float *c, int64_t m, int64_t n, int64_t ld);
+int launch_band_tc(const BandTcMaps *maps, const TcPlanes &planes, int64_t m, int64_t n, int s, int t0, int t1, int outer_macro, int lag_macro, cudaStream_t stream);
+// l and u: rows of ldl and ldu values
+int tc_prepare_operands(const float *l, int64_t ldl, const float *u, int64_t ldu, int64_t m, int64_t n, const TcPlanes &planes, cudaStream_t stream);
 struct MacroTcMaps {
-    alignas(64) unsigned char bytes[8 * 128];  // tensor maps of the eight operand planes with 128-row boxes (opaque here)
+    alignas(64) unsigned char bytes[10 * 128];  // tensor maps of the eight operand planes with 128-row boxes and of the two targets
 };
-int macro_tc_prepare(MacroTcMaps *maps, const TcPlanes &planes, int64_t m, int64_t n);
-int launch_macro_update_tc(const MacroTcMaps *maps, const TcPlanes &planes, float *y, float *c, int64_t m, int64_t n, int s0, int s1, int s_end,
-                           cudaStream_t stream, int t_first = 0, int stages = 3);
+// y and c: the planes that receive the right and the down feedback, rows of ld values (a multiple of 4)
+int macro_tc_prepare(MacroTcMaps *maps, const TcPlanes &planes, float *y, float *c, int64_t m, int64_t n, int64_t ld);
+int launch_macro_update_tc(const MacroTcMaps *maps, const TcPlanes &planes, int64_t m, int64_t n, int s0, int s1, int s_end, cudaStream_t stream, int t_first = 0);
 
 // One problem of the tensor-core triangular inverse of the factor preparation (see g2d_factors_tc.cu).
 struct FactorPlanes {

@@ -37,7 +37,7 @@ struct TrinvJob {
 // one large product (hi hi') in an accumulator of its own, so that the small ones are not truncated against it.  The planes
 // are bf16 (8 + 8 + 8 bits, the exponent range of float): the six products leave out mid lo' and what is smaller, 2^-26 of a
 // product, a quarter of what a float32 multiplication rounds off; they cost half of six tf32 products in tensor cycles and
-// bytes, and the factors did not move (n = 4096: 1.3e-6 from float64, 2.8e-6 before).
+// bytes, and the factors came closer (n = 4096: 1.3e-6 from float64, 2.8e-6 before).
 // The second source of error is the tensor cores' accumulation: every add into the float accumulator truncates, and the sums
 // here run over up to n / 2 terms.  So the k range is cut into slices of 256: each slice is accumulated in
 // tensor memory, and the epilogue warps add the slices up in registers with round-to-nearest additions while the MMAs

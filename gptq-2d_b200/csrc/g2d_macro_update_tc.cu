@@ -1,38 +1,44 @@
-// Feedback between macro tiles on the tensor cores (float only): tcgen05.mma kind::tf32 with accumulators in
+// Feedback between macro tiles on the tensor cores (float only): tcgen05.mma kind::f16 on fp16 pairs with accumulators in
 // tensor memory, operands brought into shared memory by TMA (cp.async.bulk.tensor, 128-byte swizzle).
 //
 // One CTA owns one 128 x 128 target macro tile and forms both products of the band update
 //     down :  C[I, J] += sum_k L[I, k] E[k, J]      right:  Y[I, J] += sum_k C[I, k] U[k, J]
 // over the k ranges that hold the sources of the macro anti-diagonals s0..s1-1 (whole 128-blocks, no masks).
-// fp32 fidelity comes from the 3xTF32 split: every operand exists as hi = tf32(a) and lo = a - hi, and each
-// k step issues hi*hi + lo*hi + hi*lo into the same fp32 accumulator.  All four operand kinds are stored K-major
-// for the MMA: L and C as they are (rows x k), E and U transposed (columns x k); the split copies of L and U^T are
-// made once per sweep by the kernels at the end of this file, those of E^T and C by the tile sweep as it finishes
-// a tile.
+// float32 fidelity comes from the split of every operand into hi + lo with 11 significant bits each under a power of two per
+// 64 x 64 tile (see split_half) and three products per k step, hi hi + lo hi + hi lo.  A slice of k is one tile wide, so the
+// product of the two tiles' scales is a constant of a slice and of 64 rows and columns: it rides on the additions that
+// add the slices up in registers.  All four operand kinds are stored K-major for the MMA: L and C as they are (rows x k), E and U
+// transposed (columns x k); the split copies of L and U^T are made once per sweep by the kernels at the end of this file,
+// those of E^T and C by the tile sweep as it finishes a tile.
 //
-// Warp roles (6 warps): warp 0 issues the TMA loads, warp 1 allocates tensor memory and issues the MMAs,
-// warps 2-5 read the accumulators (each its own 32 lanes) and add them into C / Y.  A three-stage ring of
-// 64 KB (A_hi, A_lo, B_hi, B_lo tiles of 128 x 32) is handed over with mbarriers; tcgen05.commit releases a stage
-// when its MMAs have read it.  Every wait is bounded: on time-out a flag is set and the CTA winds down.
+// Bound: the shared-memory port (a 128 x 128 x 16 MMA reads its 8 KB in exactly the 64 cycles it takes, and the operands' arrival
+// shares the port: 60 % of the tensor rate); with tf32 pairs that was 60 % of half the rate and twice the bytes.  128 x 256
+// tiles would reach 80 %, but the k ranges of two neighbouring macro columns differ.  Each product's results leave as TMA
+// reductions while the next product is multiplied.  With the near updates converted alike,
+// the sweep of 8192 x 28672 went from 96 to 70 ms.
 #include "g2d_tc.cuh"
 
 namespace g2d {
 
 constexpr int RB_I = 8, RB_J = 16;  // rasterisation block of the far updates: 128 macro tiles, about one wave of CTAs
+constexpr int MACRO_STAGES = 3;
 
 struct TcMaps {
     CUtensorMap l_hi, l_lo, c_hi, c_lo;      // A operands: [rows][k]
     CUtensorMap et_hi, et_lo, ut_hi, ut_lo;  // B operands: [columns][k]
+    CUtensorMap y, c;                        // targets, boxes of 32 x 32
+};
+struct MacroScales {
+    const float *l, *c, *e, *u;
+    int nI, nJ;  // 64 x 64 tiles
+    int m, n;
 };
 
-template <int NSTAGES>
-__global__ void __launch_bounds__(TC_THREADS) macro_update_tc_kernel(const __grid_constant__ TcMaps maps, float *y, float *c, int64_t m,
-                                                                     int64_t n, int nI2, int nJ2, int s0, int s1, int t_first, int s_end,
-                                                                     int raster, int *error_flag) {
+__global__ void __launch_bounds__(PAIR_THREADS, 1) macro_update_tc_kernel(const __grid_constant__ TcMaps maps, const MacroScales S, int nI2, int nJ2, int s0,
+                                                                          int s1, int t_first, int s_end, int raster, int *error_flag) {
+    constexpr int NT = 128, MINE = NT / 2;
     extern __shared__ unsigned char tc_smem_raw[];
-    __shared__ __align__(8) uint64_t full_bar[NSTAGES], empty_bar[NSTAGES], accum_bar[2];  // one accumulator barrier per product
-    __shared__ uint32_t tmem_slot;
-    __shared__ int failed;
+    __shared__ __align__(8) PairRing<MACRO_STAGES> ring;
     // Target macro tile.  With gridDim.y > 1, blockIdx.y selects the macro anti-diagonal and blockIdx.x the tile on it
     // (few anti-diagonals: near updates).  Otherwise the whole macro grid is walked in RB_I x RB_J blocks, so that the
     // CTAs resident at one time cover a compact patch and share their L / C row strips and E^T / U^T column strips in L2.
@@ -53,202 +59,152 @@ __global__ void __launch_bounds__(TC_THREADS) macro_update_tc_kernel(const __gri
     // source macro rows (down) and macro columns (right) of the band
     const int kd_lo = max(s0 - J2, 0), kd_hi = min(s1 - J2, I2);
     const int kr_lo = max(s0 - I2, 0), kr_hi = min(s1 - I2, J2);
-    const int chunks_d = kd_hi > kd_lo ? (kd_hi - kd_lo) * (MT / KC) : 0;
-    const int chunks_r = kr_hi > kr_lo ? (kr_hi - kr_lo) * (MT / KC) : 0;
-    const int chunks = chunks_d + chunks_r;
-    if (chunks == 0) return;
-
+    const int chunks_d = kd_hi > kd_lo ? (kd_hi - kd_lo) * (MT / KH) : 0;
+    const int chunks_r = kr_hi > kr_lo ? (kr_hi - kr_lo) * (MT / KH) : 0;
+    if (chunks_d + chunks_r == 0) return;
     const uint32_t smem_base = (smem_u32(tc_smem_raw) + 1023u) & ~1023u;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    if (threadIdx.x == 0) {
-        for (int s = 0; s < NSTAGES; ++s) {
-            mbar_init(&full_bar[s], 1);
-            mbar_init(&empty_bar[s], 1);
-        }
-        mbar_init(&accum_bar[0], 1);
-        mbar_init(&accum_bar[1], 1);
-        failed = 0;
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
-    if (warp == 1) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)), "r"(TMEM_COLS) : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-    }
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    __syncthreads();
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    const uint32_t tmem = tmem_slot;
-    const int i0 = I2 * MT, j0 = J2 * MT;
-
-    if (warp == 0) {
-        if (lane == 0) {
-            for (int ch = 0; ch < chunks; ++ch) {
-                const int stage = ch % NSTAGES, round = ch / NSTAGES;
-                if (round > 0 && !mbar_wait(&empty_bar[stage], (round - 1) & 1)) { failed = 1; break; }
-                const bool down = ch < chunks_d;
-                const int k = down ? kd_lo * MT + ch * KC : kr_lo * MT + (ch - chunks_d) * KC;
-                const uint32_t dst = smem_base + stage * STAGE_BYTES;
-                mbar_expect_tx(&full_bar[stage], STAGE_BYTES);
-                tma_load_2d(dst, down ? &maps.l_hi : &maps.c_hi, k, i0, &full_bar[stage]);
-                tma_load_2d(dst + TILE_BYTES, down ? &maps.l_lo : &maps.c_lo, k, i0, &full_bar[stage]);
-                tma_load_2d(dst + 2 * TILE_BYTES, down ? &maps.et_hi : &maps.ut_hi, k, j0, &full_bar[stage]);
-                tma_load_2d(dst + 3 * TILE_BYTES, down ? &maps.et_lo : &maps.ut_lo, k, j0, &full_bar[stage]);
-            }
-        }
-    } else if (warp == 1) {
-        if (lane == 0) {
-            bool ok = true;
-            for (int ch = 0; ch < chunks && ok; ++ch) {
-                const int stage = ch % NSTAGES, round = ch / NSTAGES;
-                if (!mbar_wait(&full_bar[stage], round & 1)) { failed = 1; ok = false; break; }
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const bool down = ch < chunks_d;
-                const uint32_t d_addr = tmem + (down ? 0u : (uint32_t)MT);
-                const bool first = down ? ch == 0 : ch == chunks_d;
-                const uint32_t a_hi = smem_base + stage * STAGE_BYTES, a_lo = a_hi + TILE_BYTES, b_hi = a_hi + 2 * TILE_BYTES,
-                               b_lo = a_hi + 3 * TILE_BYTES;
+    auto next = [&](int it, PairTile &t) {  // the down product, then the right one (`which`), each where it has sources
+        const int which = it + (chunks_d == 0 ? 1 : 0);
+        if (which > 1 || (which == 1 && chunks_r == 0)) return false;
+        t = PairTile{I2 * MT, J2 * MT, which ? chunks_r : chunks_d, (which ? kr_lo : kd_lo) * MT, which};
+        return true;
+    };
+    auto load = [&](const PairTile &t, int ch, uint32_t dst, uint64_t *bar) {
+        const int k = t.k0 + ch * KH;
+        tma_load_2d(dst, t.which ? &maps.c_hi : &maps.l_hi, k, t.i0, bar);
+        tma_load_2d(dst + HTILE_BYTES, t.which ? &maps.c_lo : &maps.l_lo, k, t.i0, bar);
+        tma_load_2d(dst + 2 * HTILE_BYTES, t.which ? &maps.ut_hi : &maps.et_hi, k, t.j0, bar);
+        tma_load_2d(dst + 3 * HTILE_BYTES, t.which ? &maps.ut_lo : &maps.et_lo, k, t.j0, bar);
+    };
+    auto scale = [&](const PairTile &t, int slice, int q, int column) {
+        const int k = t.k0 / TILE + slice, i = min(t.i0 / TILE + (q >> 1), S.nI - 1), j = min((t.j0 + column) / TILE, S.nJ - 1);
+        return t.which ? S.c[(int64_t)i * S.nJ + k] * S.u[(int64_t)j * S.nJ + k] : S.l[(int64_t)i * S.nI + k] * S.e[(int64_t)k * S.nJ + j];
+    };
+    auto finish = [&](const PairTile &t, int q, int lane, int c0, float (&total)[MINE], uint32_t box) {
 #pragma unroll
-                for (int ks = 0; ks < KC / 8; ++ks) {
-                    const uint32_t off = ks * 32;  // 8 tf32 values = 32 bytes along the swizzled row
-                    umma_tf32(d_addr, umma_desc(a_hi + off), umma_desc(b_hi + off), IDESC, (first && ks == 0) ? 0u : 1u);
-                    umma_tf32(d_addr, umma_desc(a_lo + off), umma_desc(b_hi + off), IDESC, 1u);
-                    umma_tf32(d_addr, umma_desc(a_hi + off), umma_desc(b_lo + off), IDESC, 1u);
-                }
-                umma_commit(&empty_bar[stage]);  // arrives when the MMAs above have read the stage
-                // the down product is complete with its last chunk: its accumulator is read out and added to C by the
-                // epilogue warps while the MMAs of the right product run into the other accumulator
-                if (ch == chunks_d - 1) umma_commit(&accum_bar[0]);
-            }
-            if (ok && chunks_r > 0) umma_commit(&accum_bar[1]);  // arrives when every MMA issued so far has completed
-        }
-    } else {
-        // epilogue warps: lanes 32 q .. 32 q + 31 of tensor memory, q = warp % 4
-        const int q = warp & 3;
-        const int64_t row = (int64_t)i0 + q * 32 + lane;
-        bool go = true;
-        {
-            for (int prod = 0; prod < 2 && go; ++prod) {
-                if ((prod == 0 ? chunks_d : chunks_r) == 0) continue;
-                const bool ok = mbar_wait(&accum_bar[prod], 0, 256);
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                if (!ok) failed = 1;
-                go = __all_sync(0xffffffffu, ok && !failed);  // warp-uniform: the tensor-memory loads are warp-wide
-                if (!go) break;
-                float *plane = prod == 0 ? c : y;
-                for (int cb = 0; cb < MT / 32; ++cb) {
-                    uint32_t v[32];
-                    const uint32_t taddr = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(prod * MT + cb * 32);
-                    asm volatile(
-                        "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-                        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-                        "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
-                        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
-                          "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]), "=r"(v[16]),
-                          "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]), "=r"(v[24]),
-                          "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
-                        : "r"(taddr)
-                        : "memory");
-                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                    if (row < m) {
-                        float *p = plane + row * n + j0 + cb * 32;
-#pragma unroll
-                        for (int x = 0; x < 32; x += 4) {
-                            if ((int64_t)j0 + cb * 32 + x < n) {  // n is a multiple of 4: a group is inside or outside as a whole
-                                // one CTA owns each target entry, so the reduction needs no read-back and stays deterministic
-                                asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p + x), "f"(__uint_as_float(v[x])),
-                                             "f"(__uint_as_float(v[x + 1])), "f"(__uint_as_float(v[x + 2])), "f"(__uint_as_float(v[x + 3]))
-                                             : "memory");
-                            }
-                        }
-                    }
-                }
-            }
-        }
-    }
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    __syncthreads();
-    if (warp == 1) {
-        if (failed) {
-            // give outstanding loads and MMAs a bounded chance to land before the memory they target is released
-            if (lane == 0) mbar_wait(&accum_bar[chunks_r > 0 ? 1 : 0], 0);
+        for (int cb = 0; cb < MINE / 32; ++cb) {
+            if (lane == 0) box_free();
             __syncwarp();
+#pragma unroll
+            for (int g = 0; g < 8; ++g) box_store4(box, lane, g, total[cb * 32 + g * 4], total[cb * 32 + g * 4 + 1], total[cb * 32 + g * 4 + 2], total[cb * 32 + g * 4 + 3]);
+            box_fence();
+            __syncwarp();
+            if (lane == 0 && t.i0 + q * 32 < S.m && t.j0 + c0 + cb * 32 < S.n) {
+                // one CTA owns each target entry, so the reduction needs no read-back and stays deterministic; what lies outside the
+                // matrix is not written
+                box_reduce_add(t.which ? &maps.y : &maps.c, box, t.j0 + c0 + cb * 32, t.i0 + q * 32);
+                box_commit();
+            }
         }
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TMEM_COLS) : "memory");
-    }
+    };
+    const bool failed = pair_gemm<NT, MACRO_STAGES, 1>(ring, smem_base, next, load, finish, scale);
     if (threadIdx.x == 0 && failed && error_flag) atomicExch(error_flag, 1);
 }
 
-// ---- one-time operand preparation ---------------------------------------------------------------------
+// ---- one-time operand preparation: a 64 x 64 tile per CTA, strictly below the diagonal tiles (no update reads the others) ----
 
-// L (row-major, read strictly below the diagonal) -> hi / lo copies with zeros elsewhere
-__global__ void split_lower_kernel(const float *__restrict__ l, int64_t m, float *__restrict__ hi, float *__restrict__ lo) {
-    const int64_t total = m * m;
-    for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t r = t / m, cidx = t % m;
-        float h = 0.f, o = 0.f;
-        if (cidx < r) split_tf32(l[t], h, o);
-        hi[t] = h;
-        lo[t] = o;
-    }
+// Tile (I, K), K < I, of a lower triangle of nT tile rows from a linear index
+__device__ __forceinline__ void below_diagonal(int64_t lin, int &I, int &K) {
+    int64_t a = (int64_t)((sqrt(8.0 * (double)lin + 1.0) - 1.0) / 2.0);
+    while ((a + 1) * (a + 2) / 2 <= lin) ++a;
+    while (a * (a + 1) / 2 > lin) --a;
+    I = (int)a + 1;
+    K = (int)(lin - a * (a + 1) / 2);
 }
 
-// U (row-major, read strictly above the diagonal) -> transposed hi / lo copies: out[j][k] = U[k][j] for k < j
-__global__ void split_upper_transposed_kernel(const float *__restrict__ u, int64_t n, float *__restrict__ hi, float *__restrict__ lo) {
-    __shared__ float tile[32][33];
-    const int64_t tiles = ceil_div(n, 32);
-    for (int64_t b = blockIdx.x; b < tiles * tiles; b += gridDim.x) {
-        const int64_t k0 = (b / tiles) * 32, j0 = (b % tiles) * 32;  // source block: rows k, columns j
-        for (int r = threadIdx.y; r < 32; r += blockDim.y) {
-            const int64_t k = k0 + r, j = j0 + threadIdx.x;
-            tile[r][threadIdx.x] = (k < n && j < n && k < j) ? u[k * n + j] : 0.f;
-        }
-        __syncthreads();
-        for (int r = threadIdx.y; r < 32; r += blockDim.y) {
-            const int64_t j = j0 + r, k = k0 + threadIdx.x;
-            if (j < n && k < n) {
-                float h, o;
-                split_tf32(tile[threadIdx.x][r], h, o);
-                hi[j * n + k] = h;
-                lo[j * n + k] = o;
+// UPPER: U (row-major), transposed: out[j][k] = U[k][j]; else L: out[i][k] = L[i][k].  HBM bound: 4 bytes in, 4 out per entry.
+template <bool UPPER>
+__global__ void __launch_bounds__(256) split_tile_kernel(const float *__restrict__ src, int64_t pitch, int64_t size, int nT, __half *__restrict__ hi,
+                                                         __half *__restrict__ lo, int64_t ld, float *__restrict__ scales) {
+    __shared__ float tile[TILE][TILE + 1];
+    __shared__ unsigned part[8];
+    int I, K;
+    below_diagonal(blockIdx.x, I, K);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    // source block: rows a0 .., columns b0 ..
+    const int64_t a0 = (int64_t)(UPPER ? K : I) * TILE, b0 = (int64_t)(UPPER ? I : K) * TILE;
+    const bool vec = pitch % 4 == 0 && (reinterpret_cast<uintptr_t>(src) & 15) == 0 && b0 + TILE <= size;
+    unsigned most = 0u;
+#pragma unroll
+    for (int t = 0; t < TILE * TILE / 4 / 256; ++t) {
+        const int idx = t * 256 + tid, r = idx / (TILE / 4), c = (idx % (TILE / 4)) * 4;
+        float v[4] = {0.f, 0.f, 0.f, 0.f};
+        if (a0 + r < size) {
+            const float *p = src + (a0 + r) * pitch + b0 + c;
+            if (vec) {
+                const float4 f = *reinterpret_cast<const float4 *>(p);
+                v[0] = f.x; v[1] = f.y; v[2] = f.z; v[3] = f.w;
+            } else {
+#pragma unroll
+                for (int x = 0; x < 4; ++x) v[x] = b0 + c + x < size ? p[x] : 0.f;
             }
         }
-        __syncthreads();
+#pragma unroll
+        for (int x = 0; x < 4; ++x) {
+            most = max(most, __float_as_uint(v[x]) & 0x7fffffffu);
+            if (UPPER) tile[c + x][r] = v[x];
+            else tile[r][c + x] = v[x];
+        }
+    }
+    most = __reduce_max_sync(0xffffffffu, most);
+    if (lane == 0) part[warp] = most;
+    __syncthreads();
+#pragma unroll
+    for (int w = 0; w < 8; ++w) most = max(most, part[w]);
+    const int e = range_exponent(__uint_as_float(most));
+    if (tid == 0) scales[(int64_t)I * nT + K] = power_of_two(e);
+    const float by = power_of_two(-e);
+#pragma unroll
+    for (int t = 0; t < TILE * TILE / 8 / 256; ++t) {
+        const int idx = t * 256 + tid, r = idx / (TILE / 8), c = (idx % (TILE / 8)) * 8;
+        if ((int64_t)I * TILE + r >= size) continue;
+        __align__(16) __half h[8];
+        __align__(16) __half l[8];
+#pragma unroll
+        for (int x = 0; x < 8; ++x) split_half(tile[r][c + x] * by, h[x], l[x]);
+        const int64_t at = ((int64_t)I * TILE + r) * ld + (int64_t)K * TILE + c;  // K < I: whole tiles of columns
+        *reinterpret_cast<uint4 *>(hi + at) = *reinterpret_cast<const uint4 *>(h);
+        *reinterpret_cast<uint4 *>(lo + at) = *reinterpret_cast<const uint4 *>(l);
     }
 }
 
 // ---- host side ---------------------------------------------------------------------------------------
 
-int tc_prepare_operands(const float *l, const float *u, int64_t m, int64_t n, const TcPlanes &pl, cudaStream_t stream) {
-    split_lower_kernel<<<148 * 8, 256, 0, stream>>>(l, m, pl.l_hi, pl.l_lo);
-    if (check_launch() != G2D_OK) return G2D_ERR_CUDA;
-    split_upper_transposed_kernel<<<148 * 8, dim3(32, 8), 0, stream>>>(u, n, pl.ut_hi, pl.ut_lo);
-    return check_launch();
+int tc_prepare_operands(const float *l, int64_t ldl, const float *u, int64_t ldu, int64_t m, int64_t n, const TcPlanes &pl, cudaStream_t stream) {
+    const int nI = (int)ceil_div(m, (int64_t)TILE), nJ = (int)ceil_div(n, (int64_t)TILE);
+    const int64_t below_l = (int64_t)nI * (nI - 1) / 2, below_u = (int64_t)nJ * (nJ - 1) / 2;
+    if (below_l > 0x7fffffff || below_u > 0x7fffffff) return G2D_ERR_TOO_LARGE;
+    if (below_l > 0) {
+        split_tile_kernel<false><<<(unsigned)below_l, 256, 0, stream>>>(l, ldl, m, nI, pl.l_hi, pl.l_lo, pl.ldm, pl.l_scale);
+        if (check_launch() != G2D_OK) return G2D_ERR_CUDA;
+    }
+    if (below_u > 0) {
+        split_tile_kernel<true><<<(unsigned)below_u, 256, 0, stream>>>(u, ldu, n, nJ, pl.ut_hi, pl.ut_lo, pl.ldn, pl.u_scale);
+        if (check_launch() != G2D_OK) return G2D_ERR_CUDA;
+    }
+    return G2D_OK;
 }
 
-// Sources: the macro anti-diagonals s0..s1-1; targets: t_first..s_end-1 (t_first >= s1).  `stages` 3 is the full pipeline
-// (one CTA per SM); 2 leaves shared memory for CTAs of other kernels beside it.
 static_assert(sizeof(TcMaps) <= sizeof(MacroTcMaps), "opaque tensor-map storage is too small");
+constexpr size_t MACRO_SMEM = (size_t)MACRO_STAGES * pair_stage_bytes<128> + PAIR_BOXES + 1024;
 
 // Tensor maps of one sweep (encoded once, reused by every macro update of the sweep) and the kernels' one-time set-up.
-int macro_tc_prepare(MacroTcMaps *opaque, const TcPlanes &pl, int64_t m, int64_t n) {
+int macro_tc_prepare(MacroTcMaps *opaque, const TcPlanes &pl, float *y, float *c, int64_t m, int64_t n, int64_t ld) {
     TcMaps &maps = *reinterpret_cast<TcMaps *>(opaque);
-    if (!make_map(&maps.l_hi, pl.l_hi, m, m) || !make_map(&maps.l_lo, pl.l_lo, m, m) || !make_map(&maps.c_hi, pl.c_hi, m, n) ||
-        !make_map(&maps.c_lo, pl.c_lo, m, n) || !make_map(&maps.et_hi, pl.et_hi, n, m) || !make_map(&maps.et_lo, pl.et_lo, n, m) ||
-        !make_map(&maps.ut_hi, pl.ut_hi, n, n) || !make_map(&maps.ut_lo, pl.ut_lo, n, n))
+    if (!make_map_16(&maps.l_hi, pl.l_hi, m, m, MT, false, pl.ldm) || !make_map_16(&maps.l_lo, pl.l_lo, m, m, MT, false, pl.ldm) ||
+        !make_map_16(&maps.c_hi, pl.c_hi, m, n, MT, false, pl.ldn) || !make_map_16(&maps.c_lo, pl.c_lo, m, n, MT, false, pl.ldn) ||
+        !make_map_16(&maps.et_hi, pl.et_hi, n, m, MT, false, pl.ldm) || !make_map_16(&maps.et_lo, pl.et_lo, n, m, MT, false, pl.ldm) ||
+        !make_map_16(&maps.ut_hi, pl.ut_hi, n, n, MT, false, pl.ldn) || !make_map_16(&maps.ut_lo, pl.ut_lo, n, n, MT, false, pl.ldn) ||
+        !make_map(&maps.y, y, m, n, 32, ld) || !make_map(&maps.c, c, m, n, 32, ld))
         return G2D_ERR_CUDA;
     static PerDeviceOnce configured;
-    return configured.run([&] {
-        return cudaFuncSetAttribute(macro_update_tc_kernel<STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, STAGES * STAGE_BYTES + 1024) == cudaSuccess &&
-               cudaFuncSetAttribute(macro_update_tc_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * STAGE_BYTES + 1024) == cudaSuccess;
-    });
+    return configured.run([&] { return cudaFuncSetAttribute(macro_update_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MACRO_SMEM) == cudaSuccess; });
 }
 
-int launch_macro_update_tc(const MacroTcMaps *opaque, const TcPlanes &pl, float *y, float *c, int64_t m, int64_t n, int s0, int s1, int s_end,
-                           cudaStream_t stream, int t_first, int stages) {
+// Sources: the macro anti-diagonals s0..s1-1; targets: t_first..s_end-1 (t_first >= s1).
+int launch_macro_update_tc(const MacroTcMaps *opaque, const TcPlanes &pl, int64_t m, int64_t n, int s0, int s1, int s_end, cudaStream_t stream, int t_first) {
     const TcMaps &maps = *reinterpret_cast<const TcMaps *>(opaque);
     if (t_first < s1) t_first = s1;
-    const int depth = stages == 2 ? 2 : STAGES;
-    const size_t smem = (size_t)depth * STAGE_BYTES + 1024;
     const int nI2 = (int)ceil_div(m, MT), nJ2 = (int)ceil_div(n, MT);
     if (s_end <= t_first) return G2D_OK;
     const int raster = s_end - t_first > 8 ? 1 : 0;
@@ -257,10 +213,8 @@ int launch_macro_update_tc(const MacroTcMaps *opaque, const TcPlanes &pl, float 
         const int64_t blocks = ceil_div(nI2, RB_I) * ceil_div(nJ2, RB_J);
         grid = dim3((unsigned)(blocks * RB_I * RB_J), 1);
     }
-    if (depth == 2)
-        macro_update_tc_kernel<2><<<grid, TC_THREADS, smem, stream>>>(maps, y, c, m, n, nI2, nJ2, s0, s1, t_first, s_end, raster, pl.error_flag);
-    else
-        macro_update_tc_kernel<STAGES><<<grid, TC_THREADS, smem, stream>>>(maps, y, c, m, n, nI2, nJ2, s0, s1, t_first, s_end, raster, pl.error_flag);
+    const MacroScales scales{pl.l_scale, pl.c_scale, pl.e_scale, pl.u_scale, (int)ceil_div(m, (int64_t)TILE), (int)ceil_div(n, (int64_t)TILE), (int)m, (int)n};
+    macro_update_tc_kernel<<<grid, PAIR_THREADS, MACRO_SMEM, stream>>>(maps, scales, nI2, nJ2, s0, s1, t_first, s_end, raster, pl.error_flag);
     return check_launch();
 }
 

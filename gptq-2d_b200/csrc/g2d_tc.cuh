@@ -3,14 +3,14 @@
 #pragma once
 #include <cuda.h>
 
+#include <type_traits>
+
 #include "g2d_common.cuh"
 
 namespace g2d {
 
 constexpr int MT = 128;                    // macro tile edge
-constexpr int KC = 32;                     // k per chunk: 32 floats = one 128-byte swizzle row
-constexpr int TILE_BYTES = MT * KC * 4;    // 16 KB
-constexpr int STAGE_BYTES = 4 * TILE_BYTES;
+constexpr int KC = 32;                     // floats per 128-byte swizzle row
 constexpr int STAGES = 3;
 constexpr int TC_THREADS = 192;
 constexpr uint32_t TMEM_COLS = 256;
@@ -50,14 +50,6 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap *map
                  ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(smem_u32(bar))
                  : "memory");
 }
-__device__ __forceinline__ void umma_tf32(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n\t}"
-        ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-        : "memory");
-}
 __device__ __forceinline__ void umma_commit(uint64_t *bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
@@ -71,9 +63,6 @@ __device__ __forceinline__ uint64_t umma_desc(uint32_t smem_addr) {
     d |= (uint64_t)2 << 61;                       // SWIZZLE_128B
     return d;
 }
-// D fp32, A and B tf32, both K-major, M = 128, N = 128
-constexpr uint32_t IDESC = (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(MT >> 3) << 17) | ((uint32_t)(MT >> 4) << 24);
-
 // 32 consecutive accumulator columns of this warp's 32 tensor-memory lanes (one row per thread)
 __device__ __forceinline__ void tmem_load_32(uint32_t taddr, uint32_t (&v)[32]) {
     asm volatile(
@@ -108,22 +97,7 @@ __device__ __forceinline__ void mbar_arrive(uint64_t *bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
 
-// Float operands as fp16 pairs.  A value times a power of two, chosen so that the largest value it shares its scale with lies
-// in [2^14, 2^15), is hi + lo with 11 significant bits each: relative error 2^-23 down to 2^-17 of the largest value (the same
-// as a tf32 pair), an absolute error of 2^-40 of it below.  The three products hi hi + lo hi + hi lo then cost half of
-// their tf32 counterparts in tensor cycles and operand bytes.  `range_exponent` is the power: x 2^-e in (2^14, 2^15].
-__device__ __forceinline__ int range_exponent(float largest) {
-    const int e = (int)((__float_as_uint(largest) >> 23) & 255) - 127;  // largest in [2^e, 2^(e + 1))
-    return e == 128 ? 0 : (e < -100 ? -100 : e) - 14;                   // infinities and NaN stay what they are; zeros and tiny rows: any scale
-}
-__device__ __forceinline__ float power_of_two(int e) { return __uint_as_float((uint32_t)(e + 127) << 23); }  // -126 <= e <= 127
-__device__ __forceinline__ void split_half(float scaled, __half &hi, __half &lo) {
-    hi = __float2half_rn(scaled);
-    lo = __float2half_rn(scaled - __half2float(hi));
-}
-
-// ---- one-accumulator pipeline: C[128 x 128] = sum over k chunks of A[128 x 32] B[128 x 32]^T, 3xTF32 ----
-// Shared state of a CTA of TC_THREADS threads: warp 0 loads, warp 1 issues the MMAs, warps 2-5 read the accumulator.
+// ---- shared state of a CTA of TC_THREADS threads: warp 0 loads, warp 1 issues the MMAs, warps 2-5 read the accumulators ----
 struct TcRing {
     uint64_t full[STAGES], empty[STAGES], accum;
     uint32_t tmem_slot;
@@ -151,51 +125,6 @@ __device__ __forceinline__ uint32_t tc_ring_setup(TcRing &ring, uint32_t cols) {
     return ring.tmem_slot;
 }
 
-// One thread: for every chunk, wait for its stage to be free and call load(chunk, destination, barrier), which must
-// issue TMA loads of STAGE_BYTES in total (A_hi, A_lo, B_hi, B_lo tiles, TILE_BYTES apart).
-template <typename Load>
-__device__ __forceinline__ void tc_ring_produce(TcRing &ring, uint32_t smem_base, int chunks, Load load) {
-    for (int ch = 0; ch < chunks; ++ch) {
-        const int stage = ch % STAGES, round = ch / STAGES;
-        if (round > 0 && !mbar_wait(&ring.empty[stage], (round - 1) & 1)) {
-            ring.failed = 1;
-            break;
-        }
-        mbar_expect_tx(&ring.full[stage], STAGE_BYTES);
-        load(ch, smem_base + stage * STAGE_BYTES, &ring.full[stage]);
-    }
-}
-
-// One thread: the MMAs of every chunk into the accumulator at `tmem`, then the commit that the epilogue waits for.
-__device__ __forceinline__ void tc_ring_mma(TcRing &ring, uint32_t smem_base, uint32_t tmem, int chunks) {
-    for (int ch = 0; ch < chunks; ++ch) {
-        const int stage = ch % STAGES, round = ch / STAGES;
-        if (!mbar_wait(&ring.full[stage], round & 1)) {
-            ring.failed = 1;
-            break;
-        }
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const uint32_t a_hi = smem_base + stage * STAGE_BYTES, a_lo = a_hi + TILE_BYTES, b_hi = a_hi + 2 * TILE_BYTES, b_lo = a_hi + 3 * TILE_BYTES;
-#pragma unroll
-        for (int ks = 0; ks < KC / 8; ++ks) {
-            const uint32_t off = ks * 32;  // 8 tf32 values = 32 bytes along the swizzled row
-            umma_tf32(tmem, umma_desc(a_hi + off), umma_desc(b_hi + off), IDESC, (ch == 0 && ks == 0) ? 0u : 1u);
-            umma_tf32(tmem, umma_desc(a_lo + off), umma_desc(b_hi + off), IDESC, 1u);
-            umma_tf32(tmem, umma_desc(a_hi + off), umma_desc(b_lo + off), IDESC, 1u);
-        }
-        umma_commit(&ring.empty[stage]);  // arrives when the MMAs above have read the stage
-    }
-    umma_commit(&ring.accum);             // arrives when every MMA issued so far has completed
-}
-
-// Epilogue warps: wait for the accumulator; false (for the whole warp) if any wait of the CTA ran out.
-__device__ __forceinline__ bool tc_ring_accumulator_ready(TcRing &ring) {
-    const bool ok = mbar_wait(&ring.accum, 0, 256);
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    if (!ok) ring.failed = 1;
-    return __all_sync(0xffffffffu, ok && !ring.failed);  // warp-uniform: the tensor-memory loads are warp-wide
-}
-
 // All threads: release tensor memory; returns whether a wait ran out (meaningful in every thread).
 __device__ __forceinline__ bool tc_ring_teardown(TcRing &ring, uint32_t tmem, uint32_t cols) {
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -219,13 +148,11 @@ constexpr int BOX_BYTES = 32 * 32 * 4;
 __device__ __forceinline__ void box_store4(uint32_t box, int row, int group, float a, float b, float c, float d) {  // columns 4 group ..
     asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(box + row * 128 + ((group ^ (row & 7)) << 4)), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");
 }
+__device__ __forceinline__ void box_store1(uint32_t box, int row, int column, float v) {
+    asm volatile("st.shared.f32 [%0], %1;" ::"r"(box + row * 128 + (((column >> 2) ^ (row & 7)) << 4) + (column & 3) * 4), "f"(v) : "memory");
+}
 __device__ __forceinline__ void box_reduce_add(const CUtensorMap *map, uint32_t box, int x, int y) {  // one lane, after fence and __syncwarp
     asm volatile("cp.reduce.async.bulk.tensor.2d.global.shared::cta.add.tile.bulk_group [%0, {%1, %2}], [%3];"
-                 ::"l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(box)
-                 : "memory");
-}
-__device__ __forceinline__ void box_store(const CUtensorMap *map, uint32_t box, int x, int y) {
-    asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.tile.bulk_group [%0, {%1, %2}], [%3];"
                  ::"l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(box)
                  : "memory");
 }
@@ -253,12 +180,16 @@ struct PairRing {
 // A CTA takes several tiles, one after the other, so that a tile's loads and MMAs run while the results of the one before leave.
 // next(number, tile): the CTA's tile of that number, false past the last.  load(tile, chunk, destination, barrier): A_hi, A_lo,
 // B_hi, B_lo tiles one after the other.  finish(tile, q, lane, first column, totals, 4 KB of shared memory of the warp's own
-// behind the stages).  Returns whether a wait ran out.
+// behind the stages).  scale(tile, slice, q, column), optional: what a slice's sums are multiplied by, the same for 64 columns.
+// Returns whether a wait ran out.
 struct PairTile {
     int i0, j0, chunks;
+    int k0 = 0, which = 0;  // first k and a number of the caller's
 };
-template <int NT, int NSTAGE, int SLICE, typename Next, typename Load, typename Finish>
-__device__ __forceinline__ bool pair_gemm(PairRing<NSTAGE> &ring, uint32_t smem_base, Next next, Load load, Finish finish) {
+struct PairNoScale {};
+template <int NT, int NSTAGE, int SLICE, typename Next, typename Load, typename Finish, typename Scale = PairNoScale>
+__device__ __forceinline__ bool pair_gemm(PairRing<NSTAGE> &ring, uint32_t smem_base, Next next, Load load, Finish finish, Scale scale = Scale()) {
+    constexpr bool SCALED = !std::is_same<Scale, PairNoScale>::value;
     constexpr int B_BYTES = NT * KH * 2, STAGE = 2 * HTILE_BYTES + 2 * B_BYTES, MINE = NT / 2;
     constexpr uint32_t COLS = 2 * NT, DESC = idesc_16(NT, 0);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -339,6 +270,11 @@ __device__ __forceinline__ bool pair_gemm(PairRing<NSTAGE> &ring, uint32_t smem_
             for (int x = 0; x < MINE; ++x) total[x] = 0.f;
             for (int s = 0; s < slices; ++s, ++slice) {
                 const int buf = slice & 1;
+                float factor[MINE / 64];  // of this slice's columns, on their way while the slice is awaited
+                if constexpr (SCALED) {
+#pragma unroll
+                    for (int g = 0; g < MINE / 64; ++g) factor[g] = scale(tile, s, q, c0 + g * 64);
+                }
                 const bool ok = mbar_wait(&ring.acc_full[buf], (slice >> 1) & 1, 64);
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 if (!ok) ring.failed = 1;
@@ -349,7 +285,10 @@ __device__ __forceinline__ bool pair_gemm(PairRing<NSTAGE> &ring, uint32_t smem_
                     uint32_t v[32];
                     tmem_load_32(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(buf * NT + c0 + cb * 32), v);
 #pragma unroll
-                    for (int x = 0; x < 32; ++x) total[cb * 32 + x] += __uint_as_float(v[x]);
+                    for (int x = 0; x < 32; ++x) {
+                        if constexpr (SCALED) total[cb * 32 + x] = fmaf(__uint_as_float(v[x]), factor[cb / 2], total[cb * 32 + x]);
+                        else total[cb * 32 + x] += __uint_as_float(v[x]);
+                    }
                 }
                 // this warp has read the accumulator: hand it back to the MMA warp
                 asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -411,11 +350,11 @@ static EncodeTiledFn encode_tiled_fn() {
 }
 
 // row-major fp32 matrix [rows][cols]; boxes of box_rows rows x 32 columns, 128-byte swizzle, zero fill outside
-static bool make_map(CUtensorMap *map, const float *base, int64_t rows, int64_t cols, int box_rows = MT) {
+static bool make_map(CUtensorMap *map, const float *base, int64_t rows, int64_t cols, int box_rows = MT, int64_t pitch = 0) {
     EncodeTiledFn fn = encode_tiled_fn();
     if (!fn) return false;
     const cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
-    const cuuint64_t strides[1] = {(cuuint64_t)cols * sizeof(float)};
+    const cuuint64_t strides[1] = {(cuuint64_t)(pitch ? pitch : cols) * sizeof(float)};
     const cuuint32_t box[2] = {KC, (cuuint32_t)box_rows};
     const cuuint32_t elem[2] = {1, 1};
     return fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<float *>(base), dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE,

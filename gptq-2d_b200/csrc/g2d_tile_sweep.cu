@@ -147,6 +147,7 @@ __global__ void __launch_bounds__(TTH, 1) tile_sweep_kernel(SweepArgs<F> P, int 
     F *Lbs = Ubs + TILE * LD;                 // the same: L[I + 1, I], the lower neighbour's
     F *Yns = Lbs + TILE * LD;                 // the same: the feedback for the right neighbour, C[I, J] U[J, J + 1], growing sub-tile by sub-tile
     F *Cns = Yns + TILE * LD;                 // and for the lower one, L[I + 1, I] E[I, J]
+    __shared__ unsigned tile_max[2][TTH / 32];
     __shared__ unsigned fast_div[NSUB];       // every scale of the sub-tile allows the division by reciprocal
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -613,64 +614,61 @@ __global__ void __launch_bounds__(TTH, 1) tile_sweep_kernel(SweepArgs<F> P, int 
                 }
             }
         }
-        // ---- operands of the tensor-core macro updates: tf32 hi / lo of E (transposed) and of the completed C ----
-        if (P.c_hi != nullptr) {
-            if constexpr (sizeof(F) == sizeof(float)) {
-                auto split4 = [](const float (&v)[4], float (&hi)[4], float (&lo)[4]) {
+        // ---- operands of the tensor-core updates: fp16 pairs of E (transposed) and of the completed C under the tile's scales ----
+        if constexpr (sizeof(F) == sizeof(float)) {
+            if (P.c_hi != nullptr) {
+                // largest value of the tile (entries outside the matrix are zero)
+                unsigned me = 0u, mc = 0u;
+                for (int idx = tid; idx < TILE * TILE / 4; idx += TTH) {
+                    const int r = idx / (TILE / 4), c = (idx % (TILE / 4)) * 4;
+                    F ve[4], vc[4];
+                    load4(Ys + r * LD + c, ve);
+                    load4(Cs + r * LD + c, vc);
 #pragma unroll
                     for (int x = 0; x < 4; ++x) {
-                        uint32_t h;
-                        asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(h) : "f"(v[x]));
-                        hi[x] = __uint_as_float(h);
-                        lo[x] = v[x] - hi[x];
+                        me = max(me, __float_as_uint((float)ve[x]) & 0x7fffffffu);
+                        mc = max(mc, __float_as_uint((float)vc[x]) & 0x7fffffffu);
                     }
-                };
-                if (vec) {
-                    // whole tile, rows of 16-byte multiples: four entries per thread and store.  C along its rows; E
-                    // transposed: a thread gathers four rows of one column (consecutive threads take consecutive
-                    // columns, so the shared-memory reads do not collide) and writes them as one vector of a row of E^T
-                    for (int idx = tid; idx < TILE * TILE / 4; idx += TTH) {
-                        {
-                            const int r = idx / (TILE / 4), c = (idx % (TILE / 4)) * 4;
-                            float v[4], hi[4], lo[4];
-                            load4(reinterpret_cast<const float *>(Cs) + r * LD + c, v);
-                            split4(v, hi, lo);
-                            store4(P.c_hi + (i0 + r) * ld + j0 + c, hi);
-                            store4(P.c_lo + (i0 + r) * ld + j0 + c, lo);
-                        }
-                        {
-                            const int c = idx % TILE, r = (idx / TILE) * 4;
-                            float v[4], hi[4], lo[4];
+                }
+                me = __reduce_max_sync(0xffffffffu, me);
+                mc = __reduce_max_sync(0xffffffffu, mc);
+                if (lane == 0) { tile_max[0][warp] = me; tile_max[1][warp] = mc; }
+                __syncthreads();
 #pragma unroll
-                            for (int x = 0; x < 4; ++x) v[x] = (float)Ys[(r + x) * LD + c];
-                            split4(v, hi, lo);
-                            store4(P.et_hi + (j0 + c) * P.ldm + i0 + r, hi);
-                            store4(P.et_lo + (j0 + c) * P.ldm + i0 + r, lo);
+                for (int w2 = 0; w2 < TTH / 32; ++w2) {
+                    me = max(me, tile_max[0][w2]);
+                    mc = max(mc, tile_max[1][w2]);
+                }
+                const int ee = range_exponent(__uint_as_float(me)), ec = range_exponent(__uint_as_float(mc));
+                if (tid == 0) {
+                    P.e_scale[(int64_t)I * P.nJ + J] = power_of_two(ee);
+                    P.c_scale[(int64_t)I * P.nJ + J] = power_of_two(ec);
+                }
+                const float e_by = power_of_two(-ee), c_by = power_of_two(-ec);
+                // eight entries per thread and store.  C along its rows; E transposed: a thread gathers eight rows of one column
+                // (consecutive threads take consecutive columns, so the shared-memory reads do not collide) and writes them as
+                // one vector of a row of E^T.  A row's last vector may reach into its padding.
+                for (int idx = tid; idx < TILE * TILE / 8; idx += TTH) {
+                    __align__(16) __half h[8];
+                    __align__(16) __half l[8];
+                    {
+                        const int r = idx / (TILE / 8), c = (idx % (TILE / 8)) * 8;
+                        if (r < rows_in && c < cols_in) {
+#pragma unroll
+                            for (int x = 0; x < 8; ++x) split_half((float)Cs[r * LD + c + x] * c_by, h[x], l[x]);
+                            const int64_t at = (i0 + r) * P.ldn + j0 + c;
+                            *reinterpret_cast<uint4 *>(P.c_hi + at) = *reinterpret_cast<const uint4 *>(h);
+                            *reinterpret_cast<uint4 *>(P.c_lo + at) = *reinterpret_cast<const uint4 *>(l);
                         }
                     }
-                } else {
-                    for (int idx = tid; idx < TILE * TILE; idx += TTH) {
-                        {   // C[i][j], consecutive threads along j
-                            const int r = idx / TILE, c = idx % TILE;
-                            const int64_t gi = i0 + r, gj = j0 + c;
-                            if (gi < m && gj < n) {
-                                const float v = (float)Cs[r * LD + c];
-                                uint32_t h;
-                                asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(h) : "f"(v));
-                                P.c_hi[gi * ld + gj] = __uint_as_float(h);
-                                P.c_lo[gi * ld + gj] = v - __uint_as_float(h);
-                            }
-                        }
-                        {   // E^T[j][i], consecutive threads along i
-                            const int c = idx / TILE, r = idx % TILE;
-                            const int64_t gi = i0 + r, gj = j0 + c;
-                            if (gi < m && gj < n) {
-                                const float v = (float)Ys[r * LD + c];
-                                uint32_t h;
-                                asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(h) : "f"(v));
-                                P.et_hi[gj * P.ldm + gi] = __uint_as_float(h);
-                                P.et_lo[gj * P.ldm + gi] = v - __uint_as_float(h);
-                            }
+                    {
+                        const int c = idx % TILE, r = (idx / TILE) * 8;
+                        if (r < rows_in && c < cols_in) {
+#pragma unroll
+                            for (int x = 0; x < 8; ++x) split_half((float)Ys[(r + x) * LD + c] * e_by, h[x], l[x]);
+                            const int64_t at = (j0 + c) * P.ldm + i0 + r;
+                            *reinterpret_cast<uint4 *>(P.et_hi + at) = *reinterpret_cast<const uint4 *>(h);
+                            *reinterpret_cast<uint4 *>(P.et_lo + at) = *reinterpret_cast<const uint4 *>(l);
                         }
                     }
                 }
