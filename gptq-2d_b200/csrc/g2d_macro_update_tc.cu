@@ -1,7 +1,7 @@
 // Feedback between macro tiles on the tensor cores (float only): tcgen05.mma kind::f16 on fp16 pairs with accumulators in
 // tensor memory, operands brought into shared memory by TMA (cp.async.bulk.tensor, 128-byte swizzle).
 //
-// One CTA owns one 128 x 128 target macro tile and forms both products of the band update
+// A CTA owns one 128 x 128 target macro tile, or 2 x 2 of them, and forms both products of the band update
 //     down :  C[I, J] += sum_k L[I, k] E[k, J]      right:  Y[I, J] += sum_k C[I, k] U[k, J]
 // over the k ranges that hold the sources of the macro anti-diagonals s0..s1-1 (whole 128-blocks, no masks).
 // float32 fidelity comes from the split of every operand into hi + lo with 11 significant bits each under a power of two per
@@ -11,21 +11,19 @@
 // transposed (columns x k); the split copies of L and U^T are made once per sweep by the kernels at the end of this file,
 // those of E^T and C by the tile sweep as it finishes a tile.
 //
-// Bound: the shared-memory port (a 128 x 128 x 16 MMA reads its 8 KB in exactly the 64 cycles it takes, and the operands' arrival
-// shares the port: 60 % of the tensor rate); with tf32 pairs that was 60 % of half the rate and twice the bytes.  128 x 256
-// tiles would reach 80 %, but the k ranges of two neighbouring macro columns differ.  Each product's results leave as TMA
-// reductions while the next product is multiplied.  With the near updates converted alike,
-// the sweep of 8192 x 28672 went from 96 to 70 ms.
+// Bound: the L2 and the shared-memory port that operands come through (with tf32 pairs twice the bytes at half the tensor rate),
+// and for a short source range what a CTA spends on its first loads and its last results.  Results leave as TMA reductions while the
+// next product is multiplied.
 #include "g2d_tc.cuh"
 
 namespace g2d {
 
-constexpr int RB_I = 8, RB_J = 16;  // rasterisation block of the far updates: 128 macro tiles, about one wave of CTAs
-constexpr int MACRO_STAGES = 3;
+constexpr int RB_I = 8, RB_J = 16;  // rasterisation block: 128 macro tiles
+constexpr int MACRO_STAGES = 3, MACRO_WIDE_STAGES = 2;
 
 struct TcMaps {
-    CUtensorMap l_hi, l_lo, c_hi, c_lo;      // A operands: [rows][k]
-    CUtensorMap et_hi, et_lo, ut_hi, ut_lo;  // B operands: [columns][k]
+    CUtensorMap l_hi, l_lo, c_hi, c_lo;      // [rows][k]
+    CUtensorMap et_hi, et_lo, ut_hi, ut_lo;  // [columns][k]
     CUtensorMap y, c;                        // targets, boxes of 32 x 32
 };
 struct MacroScales {
@@ -34,40 +32,49 @@ struct MacroScales {
     int m, n;
 };
 
-__global__ void __launch_bounds__(PAIR_THREADS, 1) macro_update_tc_kernel(const __grid_constant__ TcMaps maps, const MacroScales S, int nI2, int nJ2, int s0,
-                                                                          int s1, int t_first, int s_end, int raster, int *error_flag) {
+// What a launch covers: sources and targets, in macro tiles.
+struct MacroRange {
+    int nI2, nJ2, s0, s1, t_first, s_end;  // t_first >= s1
+    __host__ __device__ bool target(int I2, int J2) const { return I2 < nI2 && J2 >= 0 && J2 < nJ2 && I2 + J2 >= t_first && I2 + J2 < s_end; }
+    // the source macro rows of a target's column `across` (down) or macro columns of its row (right); every one lies before the
+    // target, so they do not depend on its other index
+    __device__ bool sources(int across, int &k, int &count) const {
+        k = max(s0 - across, 0);
+        count = s1 - across - k;
+        return count > 0;
+    }
+    // Rasterisation blocks of block row b that can hold a target with a source (I2 or J2 below s1): the first and past the last
+    __host__ __device__ void row(int b, int &first, int &last) const {
+        const int i_lo = b * RB_I, i_hi = i_lo + RB_I < nI2 ? i_lo + RB_I : nI2;
+        int j_lo = t_first - (i_hi - 1), j_hi = s_end - i_lo;
+        if (j_lo < 0) j_lo = 0;
+        if (j_hi > nJ2) j_hi = nJ2;
+        if (i_lo >= s1 && j_hi > s1) j_hi = s1;
+        first = j_lo / RB_J;
+        last = j_hi > j_lo ? (j_hi + RB_J - 1) / RB_J : first;
+    }
+};
+
+// Few anti-diagonals of targets: one macro tile per CTA, the down product and then the right one.  It is the part of a far update
+// that the tile launches wait for, so what counts is that it ends soon.
+__global__ void __launch_bounds__(PAIR_THREADS, 1) macro_update_tc_kernel(const __grid_constant__ TcMaps maps, const MacroScales S, const MacroRange R,
+                                                                          int *error_flag) {
     constexpr int NT = 128, MINE = NT / 2;
     extern __shared__ unsigned char tc_smem_raw[];
     __shared__ __align__(8) PairRing<MACRO_STAGES> ring;
-    // Target macro tile.  With gridDim.y > 1, blockIdx.y selects the macro anti-diagonal and blockIdx.x the tile on it
-    // (few anti-diagonals: near updates).  Otherwise the whole macro grid is walked in RB_I x RB_J blocks, so that the
-    // CTAs resident at one time cover a compact patch and share their L / C row strips and E^T / U^T column strips in L2.
-    int I2, J2;
-    if (raster == 0) {
-        const int W = t_first + (int)blockIdx.y;
-        const int ti_lo = max(0, W - nJ2 + 1), ti_hi = min(W + 1, nI2);
-        I2 = ti_lo + (int)blockIdx.x;
-        if (W >= s_end || I2 >= ti_hi) return;
-        J2 = W - I2;
-    } else {
-        const int blocks_j = (nJ2 + RB_J - 1) / RB_J;
-        const int blk = (int)blockIdx.x / (RB_I * RB_J), within = (int)blockIdx.x % (RB_I * RB_J);
-        I2 = (blk / blocks_j) * RB_I + within / RB_J;
-        J2 = (blk % blocks_j) * RB_J + within % RB_J;
-        if (I2 >= nI2 || J2 >= nJ2 || I2 + J2 < t_first || I2 + J2 >= s_end) return;
-    }
-    // source macro rows (down) and macro columns (right) of the band
-    const int kd_lo = max(s0 - J2, 0), kd_hi = min(s1 - J2, I2);
-    const int kr_lo = max(s0 - I2, 0), kr_hi = min(s1 - I2, J2);
-    const int chunks_d = kd_hi > kd_lo ? (kd_hi - kd_lo) * (MT / KH) : 0;
-    const int chunks_r = kr_hi > kr_lo ? (kr_hi - kr_lo) * (MT / KH) : 0;
-    if (chunks_d + chunks_r == 0) return;
+    const int I2 = blockIdx.y, J2 = R.t_first - I2 + (int)blockIdx.x;
+    int k, macros;
+    if (!R.target(I2, J2) || (!R.sources(J2, k, macros) && !R.sources(I2, k, macros))) return;
     const uint32_t smem_base = (smem_u32(tc_smem_raw) + 1023u) & ~1023u;
-    auto next = [&](int it, PairTile &t) {  // the down product, then the right one (`which`), each where it has sources
-        const int which = it + (chunks_d == 0 ? 1 : 0);
-        if (which > 1 || (which == 1 && chunks_r == 0)) return false;
-        t = PairTile{I2 * MT, J2 * MT, which ? chunks_r : chunks_d, (which ? kr_lo : kd_lo) * MT, which};
-        return true;
+    auto next = [&, which = 0](int, PairTile &t) mutable {
+        for (; which < 2; ++which) {
+            int k, macros;
+            if (R.sources(which ? I2 : J2, k, macros)) {
+                t = PairTile{I2 * MT, J2 * MT, macros * (MT / KH), k * MT, which++};
+                return true;
+            }
+        }
+        return false;
     };
     auto load = [&](const PairTile &t, int ch, uint32_t dst, uint64_t *bar) {
         const int k = t.k0 + ch * KH;
@@ -98,6 +105,81 @@ __global__ void __launch_bounds__(PAIR_THREADS, 1) macro_update_tc_kernel(const 
         }
     };
     const bool failed = pair_gemm<NT, MACRO_STAGES, 1>(ring, smem_base, next, load, finish, scale);
+    if (threadIdx.x == 0 && failed && error_flag) atomicExch(error_flag, 1);
+}
+
+// Many anti-diagonals: 2 x 2 macro tiles per CTA as four products of M = 128, N = 256.  The source range of a down product depends
+// on the column only, so two macro rows share it (the product is formed transposed, C^T = E^T L^T, which puts them on the N side),
+// and that of a right product on the row only.  Wide products leave the shared-memory port at 80 % of the tensor rate instead of
+// 60 %, and four of them per CTA hide what a CTA spends on its first loads and its last results: alone on the GPU at 8192 x 28672
+// 233 TFLOP/s with a macro tile per CTA, 294 now (rank 512; 370 at rank 1024).  A target outside the launch's anti-diagonals is multiplied but not written.
+// The targets are walked in RB_I x RB_J blocks, block row after block row, so that the CTAs resident at one time share
+// their row and column strips in L2.
+__global__ void __launch_bounds__(PAIR_THREADS, 1) macro_update_wide_kernel(const __grid_constant__ TcMaps maps, const MacroScales S, const MacroRange R,
+                                                                            int *error_flag) {
+    constexpr int NT = 256, MINE = NT / 2, SHARES = RB_I * RB_J / 4;
+    extern __shared__ unsigned char tc_smem_raw[];
+    __shared__ __align__(8) PairRing<MACRO_WIDE_STAGES> ring;
+    int block = (int)blockIdx.x / SHARES, row = 0, first, last;
+    for (R.row(0, first, last); block >= last - first; R.row(++row, first, last)) block -= last - first;
+    const int within = (int)blockIdx.x % SHARES;
+    const int I2 = row * RB_I + within / (RB_J / 2) * 2, J2 = (first + block) * RB_J + within % (RB_J / 2) * 2;
+    // product x: down into column J2 + x, right into row I2 + x - 2
+    auto product = [&](int x, PairTile &t) {
+        const int which = x >> 1, half = x & 1;
+        const bool wanted = which ? R.target(I2 + half, J2) || R.target(I2 + half, J2 + 1) : R.target(I2, J2 + half) || R.target(I2 + 1, J2 + half);
+        int k, macros;
+        if (!wanted || !R.sources((which ? I2 : J2) + half, k, macros)) return false;
+        t = PairTile{((which ? I2 : J2) + half) * MT, (which ? J2 : I2) * MT, macros * (MT / KH), k * MT, which};
+        return true;
+    };
+    PairTile any;
+    if (!product(0, any) && !product(1, any) && !product(2, any) && !product(3, any)) return;
+    const uint32_t smem_base = (smem_u32(tc_smem_raw) + 1023u) & ~1023u;
+    auto next = [&, x = 0](int, PairTile &t) mutable {
+        while (x < 4)
+            if (product(x++, t)) return true;
+        return false;
+    };
+    auto load = [&](const PairTile &t, int ch, uint32_t dst, uint64_t *bar) {
+        const int k = t.k0 + ch * KH;
+        tma_load_2d(dst, t.which ? &maps.c_hi : &maps.et_hi, k, t.i0, bar);
+        tma_load_2d(dst + HTILE_BYTES, t.which ? &maps.c_lo : &maps.et_lo, k, t.i0, bar);
+        for (int h = 0; h < 2; ++h) {
+            tma_load_2d(dst + (2 + h) * HTILE_BYTES, t.which ? &maps.ut_hi : &maps.l_hi, k, t.j0 + h * MT, bar);
+            tma_load_2d(dst + (4 + h) * HTILE_BYTES, t.which ? &maps.ut_lo : &maps.l_lo, k, t.j0 + h * MT, bar);
+        }
+    };
+    auto scale = [&](const PairTile &t, int slice, int q, int column) {
+        const int k = t.k0 / TILE + slice, a = t.i0 / TILE + (q >> 1), b = (t.j0 + column) / TILE;
+        if (t.which) return S.c[(int64_t)min(a, S.nI - 1) * S.nJ + k] * S.u[(int64_t)min(b, S.nJ - 1) * S.nJ + k];
+        return S.l[(int64_t)min(b, S.nI - 1) * S.nI + k] * S.e[(int64_t)k * S.nJ + min(a, S.nJ - 1)];
+    };
+    auto finish = [&](const PairTile &t, int q, int lane, int c0, float (&total)[MINE], uint32_t box) {
+        // the warp's columns lie in one macro tile
+        const int fixed = t.i0 / MT, moving = (t.j0 + c0) / MT;
+        if (!(t.which ? R.target(fixed, moving) : R.target(moving, fixed))) return;
+#pragma unroll
+        for (int cb = 0; cb < MINE / 32; ++cb) {
+            if (lane == 0) box_free();
+            __syncwarp();
+            if (t.which) {
+#pragma unroll
+                for (int g = 0; g < 8; ++g) box_store4(box, lane, g, total[cb * 32 + g * 4], total[cb * 32 + g * 4 + 1], total[cb * 32 + g * 4 + 2], total[cb * 32 + g * 4 + 3]);
+            } else {  // transposed: consecutive lanes hold consecutive columns of one row of C
+#pragma unroll
+                for (int x = 0; x < 32; ++x) box_store1(box, x, lane, total[cb * 32 + x]);
+            }
+            box_fence();
+            __syncwarp();
+            const int x = t.which ? t.j0 + c0 + cb * 32 : t.i0 + q * 32, y = t.which ? t.i0 + q * 32 : t.j0 + c0 + cb * 32;
+            if (lane == 0 && x < S.n && y < S.m) {
+                box_reduce_add(t.which ? &maps.y : &maps.c, box, x, y);
+                box_commit();
+            }
+        }
+    };
+    const bool failed = pair_gemm<NT, MACRO_WIDE_STAGES, 1>(ring, smem_base, next, load, finish, scale);
     if (threadIdx.x == 0 && failed && error_flag) atomicExch(error_flag, 1);
 }
 
@@ -187,6 +269,7 @@ int tc_prepare_operands(const float *l, int64_t ldl, const float *u, int64_t ldu
 
 static_assert(sizeof(TcMaps) <= sizeof(MacroTcMaps), "opaque tensor-map storage is too small");
 constexpr size_t MACRO_SMEM = (size_t)MACRO_STAGES * pair_stage_bytes<128> + PAIR_BOXES + 1024;
+constexpr size_t MACRO_WIDE_SMEM = (size_t)MACRO_WIDE_STAGES * pair_stage_bytes<256> + PAIR_BOXES + 1024;
 
 // Tensor maps of one sweep (encoded once, reused by every macro update of the sweep) and the kernels' one-time set-up.
 int macro_tc_prepare(MacroTcMaps *opaque, const TcPlanes &pl, float *y, float *c, int64_t m, int64_t n, int64_t ld) {
@@ -198,23 +281,33 @@ int macro_tc_prepare(MacroTcMaps *opaque, const TcPlanes &pl, float *y, float *c
         !make_map(&maps.y, y, m, n, 32, ld) || !make_map(&maps.c, c, m, n, 32, ld))
         return G2D_ERR_CUDA;
     static PerDeviceOnce configured;
-    return configured.run([&] { return cudaFuncSetAttribute(macro_update_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MACRO_SMEM) == cudaSuccess; });
+    return configured.run([&] {
+        return cudaFuncSetAttribute(macro_update_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MACRO_SMEM) == cudaSuccess &&
+               cudaFuncSetAttribute(macro_update_wide_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MACRO_WIDE_SMEM) == cudaSuccess;
+    });
 }
 
 // Sources: the macro anti-diagonals s0..s1-1; targets: t_first..s_end-1 (t_first >= s1).
 int launch_macro_update_tc(const MacroTcMaps *opaque, const TcPlanes &pl, int64_t m, int64_t n, int s0, int s1, int s_end, cudaStream_t stream, int t_first) {
     const TcMaps &maps = *reinterpret_cast<const TcMaps *>(opaque);
     if (t_first < s1) t_first = s1;
-    const int nI2 = (int)ceil_div(m, MT), nJ2 = (int)ceil_div(n, MT);
     if (s_end <= t_first) return G2D_OK;
-    const int raster = s_end - t_first > 8 ? 1 : 0;
-    dim3 grid((unsigned)(nI2 < nJ2 ? nI2 : nJ2), (unsigned)(s_end - t_first));
-    if (raster) {
-        const int64_t blocks = ceil_div(nI2, RB_I) * ceil_div(nJ2, RB_J);
-        grid = dim3((unsigned)(blocks * RB_I * RB_J), 1);
-    }
+    const MacroRange range{(int)ceil_div(m, MT), (int)ceil_div(n, MT), s0, s1, t_first, s_end};
     const MacroScales scales{pl.l_scale, pl.c_scale, pl.e_scale, pl.u_scale, (int)ceil_div(m, (int64_t)TILE), (int)ceil_div(n, (int64_t)TILE), (int)m, (int)n};
-    macro_update_tc_kernel<<<grid, PAIR_THREADS, MACRO_SMEM, stream>>>(maps, scales, nI2, nJ2, s0, s1, t_first, s_end, raster, pl.error_flag);
+    // The wide kernel's CTAs take about 60 us each: they need to be several per SM, or the launch ends in a long last wave and the
+    // tile launches wait for SMs (2048 x 2048: 1.94 ms against 1.88).  Up to RB_I anti-diagonals its blocks would be nearly empty.
+    int64_t blocks = 0;
+    if (s_end - t_first > RB_I)
+        for (int b = 0, first, last; b * RB_I < range.nI2; ++b) {
+            range.row(b, first, last);
+            blocks += last - first;
+        }
+    if (blocks * (RB_I * RB_J / 4) < 4 * 148) {
+        if (range.nI2 > 65535) return G2D_ERR_TOO_LARGE;
+        macro_update_tc_kernel<<<dim3((unsigned)(s_end - t_first), (unsigned)range.nI2), PAIR_THREADS, MACRO_SMEM, stream>>>(maps, scales, range, pl.error_flag);
+        return check_launch();
+    }
+    macro_update_wide_kernel<<<(unsigned)(blocks * (RB_I * RB_J / 4)), PAIR_THREADS, MACRO_WIDE_SMEM, stream>>>(maps, scales, range, pl.error_flag);
     return check_launch();
 }
 
