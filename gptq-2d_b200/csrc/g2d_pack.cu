@@ -5,7 +5,9 @@
 // A deployment stores the codes: here `bits`-bit unsigned fields code - qmin, packed little-endian (entry j of a row
 // occupies the bits j * bits .. j * bits + bits - 1 of the row's byte string), every row padded to whole bytes.
 // One thread handles eight consecutive entries of a row, i.e. `bits` whole bytes: 32 bytes in, `bits` bytes out.
-// Pure streaming work, bound by HBM bandwidth: 4 (or 8) bytes read and bits / 8 bytes written per entry.
+// Pure streaming work, bound by HBM bandwidth: 4 (or 8) bytes read and bits / 8 bytes written per entry, as long as the instructions
+// per entry stay few: 8192 x 28672, 4 bits, a scale per row, packing and unpacking together 585 us with a division, a conversion and
+// a clamp of integers per entry and a 64-bit division per thread, 444 now.
 #include "g2d_common.cuh"
 
 namespace g2d {
@@ -50,6 +52,61 @@ __device__ __forceinline__ float quotient(float z, float s, float rc) {
 __device__ __forceinline__ double quotient(double z, double s, double) { return div_rn(z, s); }
 __device__ __forceinline__ int to_int_rn(float a) { return __float2int_rn(a); }
 __device__ __forceinline__ int to_int_rn(double a) { return __double2int_rn(a); }
+// Row and rest of a linear index; 64-bit division only where the index needs it (it is 20 times the instructions, per thread)
+__device__ __forceinline__ void split_index(int64_t t, int64_t per_row, int64_t total, int64_t &row, int64_t &rest) {
+    if (total <= 0xffffffffLL) {
+        const unsigned q = (unsigned)t / (unsigned)per_row;
+        row = q;
+        rest = (unsigned)t - q * (unsigned)per_row;
+    } else {
+        row = t / per_row;
+        rest = t % per_row;
+    }
+}
+
+constexpr float INTEGER_UNIT = 12582912.f;  // 1.5 * 2^23: a float of at most 2^22 plus this is rounded to an integer, half to even
+constexpr unsigned INTEGER_UNIT_BITS = 0x4B400000u;
+
+// The codes of eight floats, four to a word.  False, with nothing done, where a scale or a quotient is out of the range in which
+// the reciprocal form of the division holds (NaN included): the caller's general path takes those.  Nine instructions per
+// entry: clamping before rounding is the same between integer bounds, the addition of INTEGER_UNIT is the rounding and the conversion, and
+// the codes are added up as they stand in the low bits, what the unit and qmin contribute taken off once per word.
+template <int BITS>
+__device__ __forceinline__ bool fast_codes(const float (&z)[8], const float (&s)[8], const float (&o)[8], bool one_scale, int qmin, unsigned (&word)[2]) {
+    bool ok = true, same = true;
+    if (!one_scale) {
+#pragma unroll
+        for (int x = 1; x < 8; ++x) same = same && s[x] == s[0];
+    }
+    float rc[8];
+    rc[0] = reciprocal(s[0]);
+    if (same) {
+        ok = fabsf(s[0]) > 1e-30f && fabsf(s[0]) < 1e30f;
+#pragma unroll
+        for (int x = 1; x < 8; ++x) rc[x] = rc[0];
+    } else {
+#pragma unroll
+        for (int x = 0; x < 8; ++x) {
+            ok = ok && fabsf(s[x]) > 1e-30f && fabsf(s[x]) < 1e30f;
+            rc[x] = reciprocal(s[x]);
+        }
+    }
+    const float low = (float)qmin, high = (float)(qmin + (1 << BITS) - 1);
+    unsigned sum[2] = {0u, 0u}, offset = 0u;
+#pragma unroll
+    for (int x = 0; x < 8; ++x) {
+        const float q0 = z[x] * rc[x];
+        ok = ok && fabsf(q0) < 1e30f;
+        const float q1 = fmaf(fmaf(-q0, s[x], z[x]), rc[x], q0);
+        const float v = fminf(fmaxf(add_rn(q1, o[x]), low), high);
+        sum[x >> 2] += __float_as_uint(add_rn(v, INTEGER_UNIT)) << ((x & 3) * BITS);
+    }
+#pragma unroll
+    for (int x = 0; x < 4; ++x) offset += (INTEGER_UNIT_BITS + (unsigned)qmin) << (x * BITS);
+    word[0] = sum[0] - offset;
+    word[1] = sum[1] - offset;
+    return ok;
+}
 
 template <typename F, int BITS>
 __global__ void __launch_bounds__(256, 3) pack_codes_kernel(int64_t m, int64_t n, const F *__restrict__ z, const F *__restrict__ scale, int64_t srs,
@@ -64,8 +121,11 @@ __global__ void __launch_bounds__(256, 3) pack_codes_kernel(int64_t m, int64_t n
     const bool vec_s = scs == 1 && srs % 8 == 0 && reinterpret_cast<uintptr_t>(scale) % 32 == 0;
     const bool vec_o = zcs == 1 && zrs % 8 == 0 && reinterpret_cast<uintptr_t>(zero) % 32 == 0;
     const bool wide = (bits == 2 || bits == 4 || bits == 8) && row_bytes % bits == 0 && reinterpret_cast<uintptr_t>(out) % bits == 0;
+    const bool fast = sizeof(F) == sizeof(float) && qmin_int >= -(1 << 21) && qmin_int <= 1 << 21;
     for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t r = t / pairs, g0 = (t % pairs) * 2;
+        int64_t r, g0;
+        split_index(t, pairs, total, r, g0);
+        g0 *= 2;
         F zv[2][8], sv[2][8], ov[2][8];
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
@@ -78,17 +138,20 @@ __global__ void __launch_bounds__(256, 3) pack_codes_kernel(int64_t m, int64_t n
         for (int h = 0; h < 2; ++h) {
             const int64_t c0 = (g0 + h) * 8;
             if (c0 >= n) continue;
-            const F row_rc = reciprocal(sv[h][0]);  // shared by the group when the scale is per row
-            unsigned half_field[2] = {0u, 0u};      // four codes of at most 8 bits each
+            unsigned half_field[2] = {0u, 0u};  // four codes of at most 8 bits each
+            bool done = false;
+            if constexpr (sizeof(F) == sizeof(float)) done = fast && c0 + 8 <= n && fast_codes<BITS>(zv[h], sv[h], ov[h], scs == 0, qmin_int, half_field);
+            if (!done) {
+                half_field[0] = half_field[1] = 0u;
 #pragma unroll
-            for (int x = 0; x < 8; ++x) {
-                if (c0 + x < n) {
-                    const F rc = scs == 0 ? row_rc : reciprocal(sv[h][x]);
-                    // round half to even and convert in one step (the conversion saturates); the clamp is done on
-                    // integers: the field's bounds moved by qmin, both well inside the int range
-                    int q = to_int_rn(add_rn(quotient(zv[h][x], sv[h][x], rc), ov[h][x]));
-                    q = q < qmin_int ? qmin_int : (q > qmin_int + (int)top ? qmin_int + (int)top : q);
-                    half_field[x >> 2] |= (unsigned)(q - qmin_int) << ((x & 3) * bits);
+                for (int x = 0; x < 8; ++x) {
+                    if (c0 + x < n) {
+                        // round half to even and convert in one step (the conversion saturates); the clamp is done on
+                        // integers: the field's bounds moved by qmin, both well inside the int range
+                        int q = to_int_rn(add_rn(quotient(zv[h][x], sv[h][x], reciprocal(sv[h][x])), ov[h][x]));
+                        q = q < qmin_int ? qmin_int : (q > qmin_int + (int)top ? qmin_int + (int)top : q);
+                        half_field[x >> 2] |= (unsigned)(q - qmin_int) << ((x & 3) * bits);
+                    }
                 }
             }
             const unsigned long long field = (unsigned long long)half_field[0] | ((unsigned long long)half_field[1] << (4 * bits));
@@ -105,20 +168,23 @@ __global__ void __launch_bounds__(256, 3) pack_codes_kernel(int64_t m, int64_t n
     }
 }
 
-template <typename F>
-__global__ void unpack_codes_kernel(int64_t m, int64_t n, const unsigned char *__restrict__ codes, int64_t row_bytes,
-                                    const F *__restrict__ scale, int64_t srs, int64_t scs, const F *__restrict__ zero, int64_t zrs,
-                                    int64_t zcs, F qmin, int bits, F *__restrict__ z) {
+template <typename F, int BITS>
+__global__ void __launch_bounds__(256) unpack_codes_kernel(int64_t m, int64_t n, const unsigned char *__restrict__ codes, int64_t row_bytes,
+                                                           const F *__restrict__ scale, int64_t srs, int64_t scs, const F *__restrict__ zero,
+                                                           int64_t zrs, int64_t zcs, F qmin, F *__restrict__ z) {
+    constexpr int bits = BITS;
     const int64_t groups = ceil_div(n, (int64_t)8), total = m * groups;
-    const unsigned top = (1u << bits) - 1u;
+    constexpr unsigned top = (1u << bits) - 1u;
     const bool vec_z = n % 8 == 0 && reinterpret_cast<uintptr_t>(z) % 32 == 0;
     const bool vec_s = scs == 1 && srs % 8 == 0 && reinterpret_cast<uintptr_t>(scale) % 32 == 0;
     const bool vec_o = zcs == 1 && zrs % 8 == 0 && reinterpret_cast<uintptr_t>(zero) % 32 == 0;
     const bool wide = (bits == 2 || bits == 4 || bits == 8) && row_bytes % bits == 0 && reinterpret_cast<uintptr_t>(codes) % bits == 0;
     for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t r = t / groups, c0 = (t % groups) * 8;
-        const unsigned char *src = codes + r * row_bytes + (c0 / 8) * bits;
-        const int64_t left = row_bytes - (c0 / 8) * bits;
+        int64_t r, c0;
+        split_index(t, groups, total, r, c0);
+        const unsigned char *src = codes + r * row_bytes + c0 * bits;
+        const int64_t left = row_bytes - c0 * bits;
+        c0 *= 8;
         unsigned long long field = 0;
         if (wide && left >= bits) {
             if (bits == 4) field = *reinterpret_cast<const unsigned *>(src);
@@ -127,13 +193,17 @@ __global__ void unpack_codes_kernel(int64_t m, int64_t n, const unsigned char *_
         } else {
             for (int b = 0; b < bits && b < left; ++b) field |= (unsigned long long)src[b] << (8 * b);
         }
+        const unsigned half_field[2] = {(unsigned)field, (unsigned)(field >> (4 * bits))};  // four codes each
         F sv[8], ov[8], zv[8];
         load8(scale + r * srs, c0, scs, n, vec_s, (F)1, sv);
         load8(zero + r * zrs, c0, zcs, n, vec_o, (F)0, ov);
 #pragma unroll
         for (int x = 0; x < 8; ++x) {
-            const F q = (F)((unsigned)(field >> (x * bits)) & top) + qmin;
-            zv[x] = mul_rn(sub_rn(q, ov[x]), sv[x]);  // as the affine quantizer forms its value
+            const unsigned code = (half_field[x >> 2] >> ((x & 3) * bits)) & top;
+            F q;  // the code as a floating-point number: exact, and without the slow conversion for float
+            if constexpr (sizeof(F) == sizeof(float)) q = __uint_as_float(0x4B000000u | code) - 8388608.f;
+            else q = (F)code;
+            zv[x] = mul_rn(sub_rn(add_rn(q, qmin), ov[x]), sv[x]);  // as the affine quantizer forms its value
         }
         if (vec_z && c0 + 8 <= n && sizeof(F) == 4) {
             asm volatile("st.global.v8.f32 [%8], {%0, %1, %2, %3, %4, %5, %6, %7};" ::"f"((float)zv[0]), "f"((float)zv[1]), "f"((float)zv[2]),
@@ -234,11 +304,20 @@ extern "C" int g2d_unpack_codes(int dtype, int64_t m, int64_t n, const uint8_t *
     const int status = pack_check(dtype, m, n, z, scale, zero, bits, codes, row_bytes);
     if (status != G2D_OK || m == 0 || n == 0) return status;
     cudaStream_t st = (cudaStream_t)stream;
-    if (dtype == G2D_F32)
-        unpack_codes_kernel<float><<<pack_grid(m, n), 256, 0, st>>>(m, n, codes, row_bytes, (const float *)scale, scale_row_stride, scale_col_stride,
-                                                                   (const float *)zero, zero_row_stride, zero_col_stride, (float)qmin, bits, (float *)z);
-    else
-        unpack_codes_kernel<double><<<pack_grid(m, n), 256, 0, st>>>(m, n, codes, row_bytes, (const double *)scale, scale_row_stride, scale_col_stride,
-                                                                    (const double *)zero, zero_row_stride, zero_col_stride, qmin, bits, (double *)z);
+    const unsigned grid = pack_grid(m, n);
+#define G2D_UNPACK_CASE(B)                                                                                                                   \
+    case B:                                                                                                                                  \
+        if (dtype == G2D_F32)                                                                                                                \
+            unpack_codes_kernel<float, B><<<grid, 256, 0, st>>>(m, n, codes, row_bytes, (const float *)scale, scale_row_stride, scale_col_stride, \
+                                                                (const float *)zero, zero_row_stride, zero_col_stride, (float)qmin, (float *)z); \
+        else                                                                                                                                 \
+            unpack_codes_kernel<double, B><<<grid, 256, 0, st>>>(m, n, codes, row_bytes, (const double *)scale, scale_row_stride, scale_col_stride, \
+                                                                 (const double *)zero, zero_row_stride, zero_col_stride, qmin, (double *)z); \
+        break;
+    switch (bits) {
+        G2D_UNPACK_CASE(1) G2D_UNPACK_CASE(2) G2D_UNPACK_CASE(3) G2D_UNPACK_CASE(4) G2D_UNPACK_CASE(5) G2D_UNPACK_CASE(6) G2D_UNPACK_CASE(7) G2D_UNPACK_CASE(8)
+    default: return G2D_ERR_BAD_ARGUMENT;
+    }
+#undef G2D_UNPACK_CASE
     return check_launch();
 }
