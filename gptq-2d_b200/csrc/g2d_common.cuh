@@ -228,8 +228,8 @@ struct FactorPlanes {
 int launch_trinv_tc(int count, const FactorPlanes *problems, cudaStream_t stream);
 
 // Tensor-core trailing update of the blocked Cholesky factorization (see g2d_factors_tc.cu).  pt planes are
-// [n][SYRK_TC_K] fp16 pairs: pt[r][k] = SYRK_PANEL_SCALE a[o + k][r] for the group of block rows that starts at row o.
-constexpr int SYRK_TC_K = 256;
+// [n][SYRK_TC_K] fp16 pairs: pt[r][k] = SYRK_PANEL_SCALE a[o + k][r] for the two groups of block rows that start at row o.
+constexpr int SYRK_TC_K = 512;
 constexpr float SYRK_PANEL_SCALE = 8192.f;
 struct SyrkTcMaps {
     alignas(64) unsigned char hi[128], lo[128], wide_hi[128], wide_lo[128], target[128];  // tensor maps of the planes and of the matrix (opaque here)
@@ -239,7 +239,7 @@ struct SyrkTcTarget {
     float *a;
     int64_t n, o;
     int t_lo, t_hi;  // target 128-row tile rows [t_lo, t_hi), tile columns up to the diagonal
-    int kw;          // rows of the group (<= SYRK_TC_K)
+    int k0, kw;      // first column of the planes, and how many of them; row o of the matrix belongs to k0
     int *flag;
 };
 struct Equilibration {

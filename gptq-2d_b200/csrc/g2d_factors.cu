@@ -77,7 +77,7 @@ struct LdlProblem {
     int64_t n;
     int *flag;
     int tc;                       // trailing updates of whole groups run on the tensor cores (float)
-    __half *pt_hi[2], *pt_lo[2];  // [n][GROUP * 64] transposed, scaled split panels of the even and odd groups
+    __half *pt_hi[2], *pt_lo[2];  // [n][2 GROUP * 64] transposed, scaled split panels of the even and odd pairs of groups
 };
 template <typename F>
 struct LdlBatch {
@@ -385,8 +385,9 @@ __global__ void __launch_bounds__(CTH) ldl_trsm_kernel(LdlBatch<F> B, int step_d
         // update (columns left of the group only); rows beyond a ragged block are zero in acc already
         const int kb_lo = kb / GROUP * GROUP;
         if (Q.tc && j < kb_lo) {
-            __half *hi = Q.pt_hi[(kb / GROUP) & 1], *lo = Q.pt_lo[(kb / GROUP) & 1];
-            const int k0 = (kb - kb_lo) * FB;
+            const int pair = step_down / (2 * GROUP);  // groups pair up by the steps of the largest problem
+            __half *hi = Q.pt_hi[pair & 1], *lo = Q.pt_lo[pair & 1];
+            const int k0 = step_down % (2 * GROUP) * FB;
             __syncthreads();
             F *const Ts = As;  // [column][k], row stride 65
 #pragma unroll
@@ -405,7 +406,7 @@ __global__ void __launch_bounds__(CTH) ldl_trsm_kernel(LdlBatch<F> B, int step_d
                     h[e] = __float2half_rn(v);
                     l[e] = __float2half_rn(v - __half2float(h[e]));
                 }
-                const int64_t at = (c0 + c) * (GROUP * FB) + k0 + k;
+                const int64_t at = (c0 + c) * SYRK_TC_K + k0 + k;
                 *reinterpret_cast<uint4 *>(hi + at) = *reinterpret_cast<const uint4 *>(h);
                 *reinterpret_cast<uint4 *>(lo + at) = *reinterpret_cast<const uint4 *>(l);
             }
@@ -568,7 +569,7 @@ __global__ void ldl_scale_kernel(F *out, int64_t n, int size, const F *dblk, con
 // device and kept.
 struct SideLane {
     cudaStream_t stream = nullptr, chain = nullptr;
-    cudaEvent_t panel[4] = {}, rest[4] = {}, fork = nullptr, join = nullptr;
+    cudaEvent_t panel[4] = {}, near[4] = {}, rest[4] = {}, fork = nullptr, join = nullptr;
 };
 static SideLane *acquire_side_lane() {
     static std::mutex mutex;
@@ -587,6 +588,7 @@ static SideLane *acquire_side_lane() {
             return nullptr;
         for (int k = 0; k < 4; ++k)
             if (cudaEventCreateWithFlags(&lane->panel[k], cudaEventDisableTiming) != cudaSuccess ||
+                cudaEventCreateWithFlags(&lane->near[k], cudaEventDisableTiming) != cudaSuccess ||
                 cudaEventCreateWithFlags(&lane->rest[k], cudaEventDisableTiming) != cudaSuccess)
                 return nullptr;
     }
@@ -608,7 +610,7 @@ static LdlLayout ldl_layout(size_t elem, int64_t n) {
     lay.w = take(elem * (size_t)n * n);                                  // [n][n]
     const bool tc = elem == 4;
     lay.planes = take(tc ? 9 * sizeof(__nv_bfloat16) * (size_t)n * plane_pitch(n) : 0);
-    lay.panels = take(tc ? 4 * sizeof(__half) * (size_t)n * GROUP * FB : 0);
+    lay.panels = take(tc ? 4 * sizeof(__half) * (size_t)n * SYRK_TC_K : 0);
     lay.scales = take(tc ? sizeof(float) * (size_t)n : 0);
     lay.total = at;
     return lay;
@@ -637,7 +639,7 @@ int ldl_run(int count, const int64_t *ns, F *const *as, const int *sizes, F *con
         LdlProblem<F> &P = B.p[z];
         P = LdlProblem<F>{as[z], outs[z], (F *)(ws + lay.tinv), (F *)(ws + lay.w), n, flags ? flags + z : nullptr, 0, {nullptr, nullptr}, {nullptr, nullptr}};
         if (std::is_same<F, float>::value) {
-            const size_t panel = sizeof(__half) * (size_t)n * GROUP * FB;
+            const size_t panel = sizeof(__half) * (size_t)n * SYRK_TC_K;
             for (int k = 0; k < 2; ++k) {
                 P.pt_hi[k] = (__half *)(ws + lay.panels + (2 * k) * panel);
                 P.pt_lo[k] = (__half *)(ws + lay.panels + (2 * k + 1) * panel);
@@ -662,12 +664,16 @@ int ldl_run(int count, const int64_t *ns, F *const *as, const int *sizes, F *con
     if (flags && cudaMemsetAsync(flags, 0, sizeof(int) * count, st) != cudaSuccess) return G2D_ERR_CUDA;
     // Each step factors one 64-row block row (last first): diagonal block, panel to its left, trailing update.  The
     // update of a step reaches every row above for an ordinary problem, but only the rows of the step's own group of
-    // GROUP block rows for a tensor-core problem; the rows above the group get the whole group's update at once
-    // (K = 256) from the tensor cores.  Look-ahead: that update is split into the rows of the next group (kept on the
-    // caller's stream) and the rest (a side stream), so that the latency-bound kernels of the next group overlap the
-    // bulk of the update.  rest(g) touches the groups <= g - 2: group g needs rest(g + 2) and older before its first
-    // kernel (which also frees the panel planes that it reuses), and next(g) must follow rest(g + 1), whose targets
-    // it shares (the order of the additions is fixed, hence the result).
+    // GROUP block rows for a tensor-core problem; the rows above the group are updated from the tensor cores, by two groups at
+    // a time (K = 512: an entry of the matrix is read and written half as often as with one, 106 -> 99 ms for the factors of
+    // n = 28672 and 8192).  Groups pair up as (g + 1, g), g even.  Look-ahead, so that the latency-bound kernels of the
+    // next groups overlap the bulk of the updates:
+    //   * group g + 1 updates only the rows of group g (K = 256), on the chain's stream;
+    //   * group g then updates with both groups, in three launches: the rows of group g - 1 on the chain's stream, the rows of the
+    //     groups g - 2 and g - 3 (near) and everything above (rest) on a side stream.
+    // Group g - 1's own update shares its targets with near(g), which it follows; no other update on the chain meets one on the
+    // side stream, so the order of the additions is fixed, hence the result.  A pair writes the panel planes that rest of the pair
+    // two before it read, and waits for that.
     static PerDeviceOnce configured;
     if (configured.run([&] { return cudaFuncSetAttribute(ldl_diag_kernel<F>, cudaFuncAttributeMaxDynamicSharedMemorySize, diag_smem<F>) == cudaSuccess; }) != G2D_OK)
         return G2D_ERR_CUDA;
@@ -675,15 +681,12 @@ int ldl_run(int count, const int64_t *ns, F *const *as, const int *sizes, F *con
     if (!lane) return G2D_ERR_CUDA;
     if (cudaEventRecord(lane->fork, caller) != cudaSuccess || cudaStreamWaitEvent(lane->chain, lane->fork, 0) != cudaSuccess) return G2D_ERR_CUDA;
     st = lane->chain;
-    bool rest_recorded[4] = {false, false, false, false};
-    const int groups = B.steps / GROUP;
-    auto wait_rest = [&](int g) {
-        if (g < groups && rest_recorded[g & 3]) return cudaStreamWaitEvent(st, lane->rest[g & 3], 0) == cudaSuccess;
-        return true;
-    };
+    bool recorded[4] = {false, false, false, false};  // near and rest of the last four pairs
+    int newest = -1;                                  // the last pair with an update on the side stream
     for (int s = B.steps - 1; s >= 0; --s) {  // block row of the largest problem; smaller problems are lined up by groups
         const int g = s / GROUP;
-        if (s % GROUP == GROUP - 1 && !wait_rest(g + 2)) return G2D_ERR_CUDA;
+        const int pair = g / 2;
+        if (s % (2 * GROUP) == 2 * GROUP - 1 && recorded[(pair + 2) & 3] && cudaStreamWaitEvent(st, lane->rest[(pair + 2) & 3], 0) != cudaSuccess) return G2D_ERR_CUDA;
         ldl_diag_kernel<F><<<dim3(1, count), DTH, diag_smem<F>, st>>>(B, s);
         if (check_launch() != G2D_OK) return G2D_ERR_CUDA;
         if (s == 0) break;
@@ -705,41 +708,47 @@ int ldl_run(int count, const int64_t *ns, F *const *as, const int *sizes, F *con
             if (check_launch() != G2D_OK) return G2D_ERR_CUDA;
         }
         if (s % GROUP != 0 || !any_tc) continue;
-        // the group g is complete: its update of everything above, for the tensor-core problems
-        SyrkTcTarget next[2], rest[2];
-        int targets = 0;
-        bool any_rest = false;
+        // the group g is complete: the updates above it, for the tensor-core problems
+        const bool closes = g % 2 == 0;
+        SyrkTcTarget next[2], near[2], rest[2];
+        int targets = 0, near_rows = 0, rest_rows = 0;
         for (int z = 0; z < count; ++z) {
             const int kb_lo = s - (B.steps - padded_block_rows(ns[z]));
             if (!B.p[z].tc || kb_lo <= 0) continue;
+            constexpr int PER = GROUP * FB / 128;  // tile rows per group
             const int64_t o = (int64_t)kb_lo * FB;
-            const int t_all = (int)(o / 128), t_next = t_all - GROUP * FB / 128;  // tile rows above the group; those of the next group start at t_next
-            const int kw = (int)(ns[z] - o < GROUP * FB ? ns[z] - o : GROUP * FB);
-            SyrkTcTarget t{&pt_maps[z][(kb_lo / GROUP) & 1], (float *)B.p[z].a, ns[z], o, t_next, t_all, kw, B.p[z].flag};
+            const int t_all = (int)(o / 128), t_next = t_all - PER, t_near = t_next > 2 * PER ? t_next - 2 * PER : 0;  // t_next >= 0: o is at least a group
+            const int64_t most = closes ? 2 * GROUP * FB : GROUP * FB;
+            SyrkTcTarget t{&pt_maps[z][pair & 1], (float *)B.p[z].a, ns[z], o, t_next, t_all, closes ? 0 : GROUP * FB, (int)(ns[z] - o < most ? ns[z] - o : most), B.p[z].flag};
             next[targets] = t;
-            t.t_lo = 0;
+            t.t_lo = t_near;
             t.t_hi = t_next;
-            rest[targets] = t;
-            any_rest = any_rest || t_next > 0;
-            ++targets;
+            near[targets] = t;
+            t.t_lo = 0;
+            t.t_hi = t_near;
+            rest[targets++] = t;
+            near_rows += t_next - t_near;
+            rest_rows += t_near;
         }
         if (targets == 0) continue;
-        rest_recorded[g & 3] = false;
-        if (any_rest) {  // the panels are final: the side stream may start on the rows above the next group
-            if (cudaEventRecord(lane->panel[g & 3], st) != cudaSuccess || cudaStreamWaitEvent(lane->stream, lane->panel[g & 3], 0) != cudaSuccess)
+        recorded[pair & 3] = closes && near_rows > 0;
+        if (recorded[pair & 3]) {  // the panels are final
+            if (cudaEventRecord(lane->panel[pair & 3], st) != cudaSuccess || cudaStreamWaitEvent(lane->stream, lane->panel[pair & 3], 0) != cudaSuccess)
                 return G2D_ERR_CUDA;
-            const int status = launch_syrk_tc(targets, rest, lane->stream);
+            int status = launch_syrk_tc(targets, near, lane->stream);
             if (status != G2D_OK) return status;
-            if (cudaEventRecord(lane->rest[g & 3], lane->stream) != cudaSuccess) return G2D_ERR_CUDA;
+            if (cudaEventRecord(lane->near[pair & 3], lane->stream) != cudaSuccess) return G2D_ERR_CUDA;
+            if (rest_rows > 0) status = launch_syrk_tc(targets, rest, lane->stream);
+            if (status != G2D_OK) return status;
+            if (cudaEventRecord(lane->rest[pair & 3], lane->stream) != cudaSuccess) return G2D_ERR_CUDA;
+            newest = pair;
         }
-        if (!wait_rest(g + 1)) return G2D_ERR_CUDA;
+        if (!closes && recorded[(pair + 1) & 3] && cudaStreamWaitEvent(st, lane->near[(pair + 1) & 3], 0) != cudaSuccess) return G2D_ERR_CUDA;
         const int status = launch_syrk_tc(targets, next, st);
         if (status != G2D_OK) return status;
-        rest_recorded[g & 3] = any_rest;
     }
-    // everything the side streams did joins the caller's stream before the inverse starts
-    for (int k = 0; k < 4; ++k)
-        if (rest_recorded[k] && cudaStreamWaitEvent(caller, lane->rest[k], 0) != cudaSuccess) return G2D_ERR_CUDA;
+    // everything the side stream did joins the caller's stream before the inverse starts
+    if (newest >= 0 && cudaStreamWaitEvent(caller, lane->rest[newest & 3], 0) != cudaSuccess) return G2D_ERR_CUDA;
     if (cudaEventRecord(lane->join, st) != cudaSuccess || cudaStreamWaitEvent(caller, lane->join, 0) != cudaSuccess) return G2D_ERR_CUDA;
     st = caller;
     ldl_copy_diag_inverse_kernel<F><<<dim3(B.steps, count), FTH, 0, st>>>(B);

@@ -321,7 +321,7 @@ int launch_trinv_tc(int count, const FactorPlanes *problems, cudaStream_t stream
 // Bound: HBM for factors beyond L2 (8 bytes per entry and group of 256 rows: 123 GB at n = 28672, 20 ms), shared-memory port
 // below (see pair_gemm).  n = 28672 and 8192 together: 73 ms with 128 x 128 tf32 tiles, 36 ms now.
 constexpr int SYRK_SLICE_CHUNKS = 2;  // k = 128 per slice: as many additions into one accumulator as 64 take in tf32
-static_assert(SYRK_TC_K % KH == 0, "whole chunks per group");
+static_assert(SYRK_TC_K % (2 * KH) == 0, "whole chunks per group");
 
 struct SyrkJob {
     CUtensorMap a_hi[2], a_lo[2], b_hi[2], b_lo[2];  // the same planes in boxes of 128 and of NT rows
@@ -329,7 +329,7 @@ struct SyrkJob {
     float *a[2];
     int64_t n[2], o[2];    // size, first row of the group
     int t_lo[2], t_hi[2];  // target tile rows [t_lo, t_hi), with every tile column up to the diagonal
-    int kw[2];
+    int k0[2], kw[2];
     int tiles_per_cta;
     int *flag[2];
 };
@@ -345,7 +345,7 @@ __global__ void __launch_bounds__(PAIR_THREADS, 1) syrk_tc_kernel(const __grid_c
     const int t_lo = z ? job.t_lo[1] : job.t_lo[0], t_hi = z ? job.t_hi[1] : job.t_hi[0];
     float *const a = z ? job.a[1] : job.a[0];
     const int64_t n = z ? job.n[1] : job.n[0], o = z ? job.o[1] : job.o[0];
-    const int kw = z ? job.kw[1] : job.kw[0];
+    const int k0 = z ? job.k0[1] : job.k0[0], kw = z ? job.kw[1] : job.kw[0];
     const int diagonals = t_hi - t_lo;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if ((int)blockIdx.x < diagonals) {
@@ -385,14 +385,15 @@ __global__ void __launch_bounds__(PAIR_THREADS, 1) syrk_tc_kernel(const __grid_c
         if (it >= job.tiles_per_cta || first + it >= last) return false;
         int I2 = I_first, J2 = J_first + it;
         for (int row; J2 >= (row = NT == 256 ? I2 / 2 + 1 : I2 + 1); ++I2) J2 -= row;
-        t = PairTile{I2 * MT, J2 * NT, (kw + KH - 1) / KH};
+        t = PairTile{I2 * MT, J2 * NT, (kw + KH - 1) / KH, k0};
         return true;
     };
     auto load = [&](const PairTile &t, int ch, uint32_t dst, uint64_t *bar) {
-        tma_load_2d(dst, a_hi, ch * KH, t.i0, bar);
-        tma_load_2d(dst + HTILE_BYTES, a_lo, ch * KH, t.i0, bar);
-        tma_load_2d(dst + 2 * HTILE_BYTES, b_hi, ch * KH, t.j0, bar);
-        tma_load_2d(dst + 2 * HTILE_BYTES + NT * KH * 2, b_lo, ch * KH, t.j0, bar);
+        const int k = t.k0 + ch * KH;
+        tma_load_2d(dst, a_hi, k, t.i0, bar);
+        tma_load_2d(dst + HTILE_BYTES, a_lo, k, t.i0, bar);
+        tma_load_2d(dst + 2 * HTILE_BYTES, b_hi, k, t.j0, bar);
+        tma_load_2d(dst + 2 * HTILE_BYTES + NT * KH * 2, b_lo, k, t.j0, bar);
     };
     constexpr float UNSCALE = -1.f / (SYRK_PANEL_SCALE * SYRK_PANEL_SCALE);
     const CUtensorMap *target = z ? &job.target[1] : &job.target[0];
@@ -486,6 +487,7 @@ int launch_syrk_tc(int count, const SyrkTcTarget *targets, cudaStream_t stream) 
         job.o[z] = t.o;
         job.t_lo[z] = t.t_lo;
         job.t_hi[z] = t.t_hi;
+        job.k0[z] = t.k0;
         job.kw[z] = t.kw;
         job.flag[z] = t.flag;
     }
