@@ -325,7 +325,7 @@ static_assert(SYRK_TC_K % (2 * KH) == 0, "whole chunks per group");
 
 struct SyrkJob {
     CUtensorMap a_hi[2], a_lo[2], b_hi[2], b_lo[2];  // the same planes in boxes of 128 and of NT rows
-    CUtensorMap target[2];                           // the matrix itself in boxes of 32 x 32 (n a multiple of 4: its rows 16-byte multiples)
+    CUtensorMap target[2];                           // the matrix itself in boxes of 16 x 32 (n a multiple of 4: its rows 16-byte multiples)
     float *a[2];
     int64_t n[2], o[2];    // size, first row of the group
     int t_lo[2], t_hi[2];  // target tile rows [t_lo, t_hi), with every tile column up to the diagonal
@@ -409,18 +409,7 @@ __global__ void __launch_bounds__(PAIR_THREADS, 1) syrk_tc_kernel(const __grid_c
 #pragma unroll
                     for (int x = 0; x < 32; ++x) total[cb * 32 + x] = gj0 + x < gi ? total[cb * 32 + x] : 0.f;
                 }
-                if (ln == 0) box_free();
-                __syncwarp();
-#pragma unroll
-                for (int g = 0; g < 8; ++g)
-                    box_store4(box, ln, g, UNSCALE * total[cb * 32 + g * 4], UNSCALE * total[cb * 32 + g * 4 + 1], UNSCALE * total[cb * 32 + g * 4 + 2],
-                               UNSCALE * total[cb * 32 + g * 4 + 3]);
-                box_fence();
-                __syncwarp();
-                if (ln == 0) {
-                    box_reduce_add(target, box, gj0, i0);
-                    box_commit();
-                }
+                add_block<false>(target, box, ln, total + cb * 32, UNSCALE, gj0, i0, true, (int)n);
             }
             return;
         }
@@ -437,7 +426,7 @@ __global__ void __launch_bounds__(PAIR_THREADS, 1) syrk_tc_kernel(const __grid_c
 
 bool syrk_tc_maps(SyrkTcMaps *maps, const __half *pt_hi, const __half *pt_lo, float *a, int64_t n) {
     static_assert(sizeof(maps->hi) == sizeof(CUtensorMap), "opaque tensor-map storage has the wrong size");
-    if (n % 4 == 0 && !make_map(reinterpret_cast<CUtensorMap *>(maps->target), a, n, n, 32)) return false;
+    if (n % 4 == 0 && !make_map(reinterpret_cast<CUtensorMap *>(maps->target), a, n, n, HALF_BOX_ROWS)) return false;
     return make_map_16(reinterpret_cast<CUtensorMap *>(maps->hi), pt_hi, n, SYRK_TC_K, MT) &&
            make_map_16(reinterpret_cast<CUtensorMap *>(maps->lo), pt_lo, n, SYRK_TC_K, MT) &&
            make_map_16(reinterpret_cast<CUtensorMap *>(maps->wide_hi), pt_hi, n, SYRK_TC_K, 256) &&

@@ -24,7 +24,7 @@ constexpr int MACRO_STAGES = 3, MACRO_WIDE_STAGES = 2;
 struct TcMaps {
     CUtensorMap l_hi, l_lo, c_hi, c_lo;      // [rows][k]
     CUtensorMap et_hi, et_lo, ut_hi, ut_lo;  // [columns][k]
-    CUtensorMap y, c;                        // targets, boxes of 32 x 32
+    CUtensorMap y, c;                        // targets, boxes of 16 x 32
 };
 struct MacroScales {
     const float *l, *c, *e, *u;
@@ -90,18 +90,10 @@ __global__ void __launch_bounds__(PAIR_THREADS, 1) macro_update_tc_kernel(const 
     auto finish = [&](const PairTile &t, int q, int lane, int c0, float (&total)[MINE], uint32_t box) {
 #pragma unroll
         for (int cb = 0; cb < MINE / 32; ++cb) {
-            if (lane == 0) box_free();
-            __syncwarp();
-#pragma unroll
-            for (int g = 0; g < 8; ++g) box_store4(box, lane, g, total[cb * 32 + g * 4], total[cb * 32 + g * 4 + 1], total[cb * 32 + g * 4 + 2], total[cb * 32 + g * 4 + 3]);
-            box_fence();
-            __syncwarp();
-            if (lane == 0 && t.i0 + q * 32 < S.m && t.j0 + c0 + cb * 32 < S.n) {
-                // one CTA owns each target entry, so the reduction needs no read-back and stays deterministic; what lies outside the
-                // matrix is not written
-                box_reduce_add(t.which ? &maps.y : &maps.c, box, t.j0 + c0 + cb * 32, t.i0 + q * 32);
-                box_commit();
-            }
+            // one CTA owns each target entry, so the reduction needs no read-back and stays deterministic; what lies outside the
+            // matrix is not written
+            const int x = t.j0 + c0 + cb * 32;
+            add_block<false>(t.which ? &maps.y : &maps.c, box, lane, total + cb * 32, 1.f, x, t.i0 + q * 32, x < S.n, S.m);
         }
     };
     const bool failed = pair_gemm<NT, MACRO_STAGES, 1>(ring, smem_base, next, load, finish, scale);
@@ -161,22 +153,9 @@ __global__ void __launch_bounds__(PAIR_THREADS, 1) macro_update_wide_kernel(cons
         if (!(t.which ? R.target(fixed, moving) : R.target(moving, fixed))) return;
 #pragma unroll
         for (int cb = 0; cb < MINE / 32; ++cb) {
-            if (lane == 0) box_free();
-            __syncwarp();
-            if (t.which) {
-#pragma unroll
-                for (int g = 0; g < 8; ++g) box_store4(box, lane, g, total[cb * 32 + g * 4], total[cb * 32 + g * 4 + 1], total[cb * 32 + g * 4 + 2], total[cb * 32 + g * 4 + 3]);
-            } else {  // transposed: consecutive lanes hold consecutive columns of one row of C
-#pragma unroll
-                for (int x = 0; x < 32; ++x) box_store1(box, x, lane, total[cb * 32 + x]);
-            }
-            box_fence();
-            __syncwarp();
-            const int x = t.which ? t.j0 + c0 + cb * 32 : t.i0 + q * 32, y = t.which ? t.i0 + q * 32 : t.j0 + c0 + cb * 32;
-            if (lane == 0 && x < S.n && y < S.m) {
-                box_reduce_add(t.which ? &maps.y : &maps.c, box, x, y);
-                box_commit();
-            }
+            const int a = t.i0 + q * 32, b = t.j0 + c0 + cb * 32;
+            if (t.which) add_block<false>(&maps.y, box, lane, total + cb * 32, 1.f, b, a, b < S.n, S.m);
+            else add_block<true>(&maps.c, box, lane, total + cb * 32, 1.f, a, b, a < S.n, S.m);
         }
     };
     const bool failed = pair_gemm<NT, MACRO_WIDE_STAGES, 1>(ring, smem_base, next, load, finish, scale);
@@ -278,7 +257,7 @@ int macro_tc_prepare(MacroTcMaps *opaque, const TcPlanes &pl, float *y, float *c
         !make_map_16(&maps.c_hi, pl.c_hi, m, n, MT, false, pl.ldn) || !make_map_16(&maps.c_lo, pl.c_lo, m, n, MT, false, pl.ldn) ||
         !make_map_16(&maps.et_hi, pl.et_hi, n, m, MT, false, pl.ldm) || !make_map_16(&maps.et_lo, pl.et_lo, n, m, MT, false, pl.ldm) ||
         !make_map_16(&maps.ut_hi, pl.ut_hi, n, n, MT, false, pl.ldn) || !make_map_16(&maps.ut_lo, pl.ut_lo, n, n, MT, false, pl.ldn) ||
-        !make_map(&maps.y, y, m, n, 32, ld) || !make_map(&maps.c, c, m, n, 32, ld))
+        !make_map(&maps.y, y, m, n, HALF_BOX_ROWS, ld) || !make_map(&maps.c, c, m, n, HALF_BOX_ROWS, ld))
         return G2D_ERR_CUDA;
     static PerDeviceOnce configured;
     return configured.run([&] {

@@ -77,6 +77,15 @@ __device__ __forceinline__ void tmem_load_32(uint32_t taddr, uint32_t (&v)[32]) 
         : "memory");
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
+__device__ __forceinline__ void tmem_load_16(uint32_t taddr, uint32_t (&v)[16]) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
+          "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
+        : "r"(taddr)
+        : "memory");
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+}
 
 // ---- 16-bit operands: K-major tiles of 64 values = 128 bytes per row, the same swizzle and descriptor as above ----
 constexpr int KH = 64;                     // k per chunk
@@ -159,6 +168,35 @@ __device__ __forceinline__ void box_reduce_add(const CUtensorMap *map, uint32_t 
 __device__ __forceinline__ void box_fence() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 __device__ __forceinline__ void box_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
 __device__ __forceinline__ void box_free() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }  // the lane's boxes may be overwritten
+// A 32 x 32 block of results through two boxes of 16 rows (4 KB of shared memory in turn): one is filled while the TMA still reads
+// the other.  With one box of 32 rows the warp waited for it every time, and the eight warps took 6000 cycles for the results of a
+// 128 x 256 tile, twice what the two accumulators of the pipeline hide (factors of 28672 and 8192: 97.1 -> 94.3 ms, the far updates of
+// 8192 x 28672 alone: 28.9 -> 27.7 ms).
+// v: the 32 values of the lane's row or, TRANSPOSED, of its column.
+constexpr int HALF_BOX_ROWS = 16, HALF_BOX_BYTES = HALF_BOX_ROWS * 128;
+__device__ __forceinline__ void half_box_free() { asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory"); }  // all but the latest
+template <bool TRANSPOSED>
+__device__ __forceinline__ void add_block(const CUtensorMap *map, uint32_t box, int lane, const float *v, float factor, int x, int y, bool inside, int rows) {
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        const uint32_t half = box + h * HALF_BOX_BYTES;
+        if (lane == 0) half_box_free();
+        __syncwarp();
+        if (TRANSPOSED) {
+#pragma unroll
+            for (int r = 0; r < HALF_BOX_ROWS; ++r) box_store1(half, r, lane, factor * v[h * HALF_BOX_ROWS + r]);
+        } else if ((lane >> 4) == h) {
+#pragma unroll
+            for (int g = 0; g < 8; ++g) box_store4(half, lane & 15, g, factor * v[4 * g], factor * v[4 * g + 1], factor * v[4 * g + 2], factor * v[4 * g + 3]);
+        }
+        box_fence();
+        __syncwarp();
+        if (lane == 0) {
+            if (inside && y + h * HALF_BOX_ROWS < rows) box_reduce_add(map, half, x, y + h * HALF_BOX_ROWS);
+            box_commit();  // a group per half, reduced or not: half_box_free counts them
+        }
+    }
+}
 __device__ __forceinline__ void box_wait() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 
 // ---- pipeline for 16-bit pairs: A[128 x k] B[NT x k]^T as hi hi + lo hi + hi lo ----
@@ -281,13 +319,13 @@ __device__ __forceinline__ bool pair_gemm(PairRing<NSTAGE> &ring, uint32_t smem_
                 go = __all_sync(0xffffffffu, ok && !ring.failed);  // warp-uniform: the tensor-memory loads are warp-wide
                 if (!go) break;
 #pragma unroll
-                for (int cb = 0; cb < MINE / 32; ++cb) {
-                    uint32_t v[32];
-                    tmem_load_32(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(buf * NT + c0 + cb * 32), v);
+                for (int cb = 0; cb < MINE / 16; ++cb) {  // 16 at a time: 128 totals and 32 more do not fit the 168 registers
+                    uint32_t v[16];
+                    tmem_load_16(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(buf * NT + c0 + cb * 16), v);
 #pragma unroll
-                    for (int x = 0; x < 32; ++x) {
-                        if constexpr (SCALED) total[cb * 32 + x] = fmaf(__uint_as_float(v[x]), factor[cb / 2], total[cb * 32 + x]);
-                        else total[cb * 32 + x] += __uint_as_float(v[x]);
+                    for (int x = 0; x < 16; ++x) {
+                        if constexpr (SCALED) total[cb * 16 + x] = fmaf(__uint_as_float(v[x]), factor[cb / 4], total[cb * 16 + x]);
+                        else total[cb * 16 + x] += __uint_as_float(v[x]);
                     }
                 }
                 // this warp has read the accumulator: hand it back to the MMA warp
