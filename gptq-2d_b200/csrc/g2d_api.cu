@@ -341,7 +341,10 @@ int sweep_pipelined(const g2d_sweep_desc *d, SweepArgs<float> &a, const TcPlanes
     if (status != G2D_OK) return status;
     const int waves = a.nI + a.nJ - 1;
     const int waves_macro = (int)(ceil_div(d->m, MACRO) + ceil_div(d->n, MACRO)) - 1;
-    const int outer = d->outer_tiles > 0 ? (d->outer_tiles + 1) / 2 : kDefaultOuterMacro;  // macro anti-diagonals per far update
+    // Macro anti-diagonals per far update.  The far updates' share of the SMs grows with m n, the tile launches' time does not: from
+    // about 12288 x 12288 on the far updates bound the sweep, and twice the rank costs them less (results leave half as often)
+    // than the near updates that it adds (16384 x 16384: 56.3 -> 53.8 ms, 8192 x 28672: 56.7 -> 55.0; 8192 x 8192: 10.9 -> 11.3).
+    const int outer = d->outer_tiles > 0 ? (d->outer_tiles + 1) / 2 : (double)d->m * (double)d->n >= 1.5e8 ? 2 * kDefaultOuterMacro : kDefaultOuterMacro;
     int last_near = -1, last_far = -1;
     for (int s = 0; s < waves; ++s) {
         // what the tiles of s need: every near update up to s - 2, and the far update whose first targets they are
