@@ -89,7 +89,7 @@ struct TcWorkspace {
     TcPlanes planes;
     float *yf, *cf, *yn, *cn;  // far and neighbour planes of the pipelined schedule
     float *y, *l, *u;          // padded copies, where the rows need them (else null)
-    size_t bytes;
+    size_t cleared, bytes;     // bytes that start as zeros (the error flag and the far planes, first), all bytes
 };
 inline TcWorkspace tc_carve(const g2d_sweep_desc *d, char *base) {
     TcWorkspace w;
@@ -103,7 +103,9 @@ inline TcWorkspace tc_carve(const g2d_sweep_desc *d, char *base) {
     const int64_t m = d->m, n = d->n, ld = sweep_pitch(d), nI = ceil_div(m, (int64_t)TILE), nJ = ceil_div(n, (int64_t)TILE);
     pl.ldm = round_up(m, 8);
     pl.ldn = round_up(n, 8);
-    pl.error_flag = (int *)take(sizeof(int));
+    pl.error_flag = (int *)take(sizeof(int));  // first: read there when a sweep is profiled
+    for (float **p : {&w.yf, &w.cf}) *p = (float *)take(4 * m * ld);
+    w.cleared = at;
     for (__half **p : {&pl.et_hi, &pl.et_lo}) *p = (__half *)take(2 * n * pl.ldm);
     for (__half **p : {&pl.c_hi, &pl.c_lo}) *p = (__half *)take(2 * m * pl.ldn);
     for (__half **p : {&pl.l_hi, &pl.l_lo}) *p = (__half *)take(2 * m * pl.ldm);
@@ -111,7 +113,7 @@ inline TcWorkspace tc_carve(const g2d_sweep_desc *d, char *base) {
     for (float **p : {&pl.e_scale, &pl.c_scale}) *p = (float *)take(4 * nI * nJ);
     pl.l_scale = (float *)take(4 * nI * nI);
     pl.u_scale = (float *)take(4 * nJ * nJ);
-    for (float **p : {&w.yf, &w.cf, &w.yn, &w.cn}) *p = (float *)take(4 * m * ld);
+    for (float **p : {&w.yn, &w.cn}) *p = (float *)take(4 * m * ld);
     w.y = n % 4 ? (float *)take(4 * m * ld) : nullptr;
     w.l = m % 4 ? (float *)take(4 * m * round_up(m, 4)) : nullptr;
     w.u = n % 4 ? (float *)take(4 * n * ld) : nullptr;
@@ -205,7 +207,7 @@ int sweep_macro(const g2d_sweep_desc *d, SweepArgs<F> &a, BandArgs<F> &b64, cuda
 // capturable): during capture, a device whose lanes do not exist yet gets G2D_ERR_UNSUPPORTED.
 struct PipeLane {
     cudaStream_t tiles = nullptr, near = nullptr, far = nullptr;  // in falling priority
-    cudaEvent_t swept[8] = {}, near_done[8] = {}, far_first[4] = {}, far_done[4] = {}, fork = nullptr, join = nullptr;
+    cudaEvent_t swept[8] = {}, near_done[8] = {}, far_first[4] = {}, far_done[4] = {}, fork = nullptr, prepared = nullptr, join = nullptr;
     std::mutex busy;
 };
 struct DeviceLanes {
@@ -224,6 +226,7 @@ void destroy_lane(PipeLane &l) {
     for (auto &e : l.far_first) drop(e);
     for (auto &e : l.far_done) drop(e);
     drop(l.fork);
+    drop(l.prepared);
     drop(l.join);
 }
 
@@ -236,6 +239,7 @@ bool build_lane(PipeLane &l) {
               cudaStreamCreateWithPriority(&l.near, cudaStreamNonBlocking, middle) == cudaSuccess &&
               cudaStreamCreateWithPriority(&l.far, cudaStreamNonBlocking, least) == cudaSuccess &&
               cudaEventCreateWithFlags(&l.fork, cudaEventDisableTiming) == cudaSuccess &&
+              cudaEventCreateWithFlags(&l.prepared, cudaEventDisableTiming) == cudaSuccess &&
               cudaEventCreateWithFlags(&l.join, cudaEventDisableTiming) == cudaSuccess;
     for (int k = 0; k < 8 && ok; ++k)
         ok = cudaEventCreateWithFlags(&l.swept[k], cudaEventDisableTiming) == cudaSuccess &&
@@ -338,7 +342,11 @@ int sweep_pipelined(const g2d_sweep_desc *d, SweepArgs<float> &a, const TcPlanes
     MacroTcMaps far_maps;
     int status = band_tc_prepare(&maps, planes, a.y, a.c, d->m, d->n, a.ld);
     if (status == G2D_OK) status = macro_tc_prepare(&far_maps, planes, (float *)a.yf, (float *)a.cf, d->m, d->n, a.ld);
+    // the operands of the updates are prepared beside the first tile launches, which do not need them
+    if (cudaStreamWaitEvent(lane->near, lane->fork, 0) != cudaSuccess) return G2D_ERR_CUDA;
+    if (status == G2D_OK) status = tc_prepare_operands(a.l, a.ldl, a.u, a.ldu, d->m, d->n, planes, lane->near);
     if (status != G2D_OK) return status;
+    if (cudaEventRecord(lane->prepared, lane->near) != cudaSuccess) return G2D_ERR_CUDA;
     const int waves = a.nI + a.nJ - 1;
     const int waves_macro = (int)(ceil_div(d->m, MACRO) + ceil_div(d->n, MACRO)) - 1;
     // Macro anti-diagonals per far update.  The far updates' share of the SMs grows with m n, the tile launches' time does not: from
@@ -380,6 +388,7 @@ int sweep_pipelined(const g2d_sweep_desc *d, SweepArgs<float> &a, const TcPlanes
         if (feeds_far) {
             const int g = W1 / outer - 1;
             if (cudaStreamWaitEvent(lane->far, lane->swept[s & 7], 0) != cudaSuccess) return G2D_ERR_CUDA;
+            if (last_far < 0 && cudaStreamWaitEvent(lane->far, lane->prepared, 0) != cudaSuccess) return G2D_ERR_CUDA;
             const int t_first = W1 + kFarLagMacro, t_split = t_first + outer < waves_macro ? t_first + outer : waves_macro;
             if (timer) timer->begin_on(2, lane->far);
             status = launch_macro_update_tc(&far_maps, planes, d->m, d->n, W1 - outer, W1, t_split, lane->far, t_first);
@@ -399,7 +408,7 @@ int sweep_pipelined(const g2d_sweep_desc *d, SweepArgs<float> &a, const TcPlanes
         }
     }
     // join: what follows the call on the caller's stream follows everything the call did
-    if (last_near >= 0 && cudaStreamWaitEvent(stream, lane->near_done[last_near & 7], 0) != cudaSuccess) return G2D_ERR_CUDA;
+    if (cudaStreamWaitEvent(stream, last_near >= 0 ? lane->near_done[last_near & 7] : lane->prepared, 0) != cudaSuccess) return G2D_ERR_CUDA;
     if (last_far >= 0 && cudaStreamWaitEvent(stream, lane->far_done[last_far & 3], 0) != cudaSuccess) return G2D_ERR_CUDA;
     if (a.y != d->y && cudaMemcpy2DAsync(d->y, d->n * 4, a.y, a.ld * 4, d->n * 4, d->m, cudaMemcpyDeviceToDevice, stream) != cudaSuccess) return G2D_ERR_CUDA;
     status = launch_sweep_finish(planes.error_flag, d->status, (float *)d->y, d->m * d->n, stream);
@@ -522,8 +531,8 @@ int sweep_fused(const g2d_sweep_desc *d, cudaStream_t stream, LaunchTimer *timer
     if (((uintptr_t)d->workspace & 255) != 0) return G2D_ERR_WORKSPACE;
     SweepArgs<F> a;
     a.y = (F *)d->y;
-    a.c = (F *)d->workspace;
-    a.e = (F *)((char *)d->workspace + plane);
+    a.e = (F *)d->workspace;
+    a.c = (F *)((char *)d->workspace + plane);
     a.l = (const F *)d->l; a.u = (const F *)d->u;
     a.l_off = d->l_offsets; a.u_off = d->u_offsets;
     a.scale = (const F *)d->scale; a.zero = (const F *)d->zero;
@@ -537,7 +546,9 @@ int sweep_fused(const g2d_sweep_desc *d, cudaStream_t stream, LaunchTimer *timer
     a.batch = d->batch; a.m = d->m; a.n = d->n;
     a.nI = (int)ceil_div(d->m, TILE); a.nJ = (int)ceil_div(d->n, TILE);
     a.ld = sweep_pitch(d); a.ldl = d->m; a.ldu = d->n;
-    if (cudaMemsetAsync(a.c, 0, sizeof(F) * (size_t)d->batch * d->m * a.ld, stream) != cudaSuccess) return G2D_ERR_CUDA;
+    // C starts as zeros, and with it what follows it in the workspace of the tensor-core schedules
+    const size_t cleared = tc ? plane + tc_carve(d, nullptr).cleared : sizeof(F) * (size_t)d->batch * d->m * a.ld;
+    if (cudaMemsetAsync(a.c, 0, cleared, stream) != cudaSuccess) return G2D_ERR_CUDA;
 
     BandArgs<F> b;
     b.y = a.y; b.c = a.c; b.e = a.e; b.l = a.l; b.u = a.u; b.l_off = a.l_off; b.u_off = a.u_off;
@@ -547,7 +558,6 @@ int sweep_fused(const g2d_sweep_desc *d, cudaStream_t stream, LaunchTimer *timer
             const TcWorkspace w = tc_carve(d, (char *)d->workspace + 2 * plane);
             const TcPlanes &planes = w.planes;
             if (w.y == nullptr && ((uintptr_t)d->y & 15) != 0) return G2D_ERR_BAD_ARGUMENT;
-            if (cudaMemsetAsync(planes.error_flag, 0, sizeof(int), stream) != cudaSuccess) return G2D_ERR_CUDA;
             auto padded = [&](float *to, int64_t pitch, const void *from, int64_t rows, int64_t cols) {
                 return cudaMemcpy2DAsync(to, 4 * pitch, from, 4 * cols, 4 * cols, rows, cudaMemcpyDeviceToDevice, stream) == cudaSuccess;
             };
@@ -560,18 +570,16 @@ int sweep_fused(const g2d_sweep_desc *d, cudaStream_t stream, LaunchTimer *timer
                 if (!padded(w.l, a.ldl, d->l, d->m, d->m)) return G2D_ERR_CUDA;
                 a.l = w.l;
             }
-            const int status = tc_prepare_operands(a.l, a.ldl, a.u, a.ldu, d->m, d->n, planes, stream);
-            if (status != G2D_OK) return status;
             a.et_hi = planes.et_hi; a.et_lo = planes.et_lo; a.c_hi = planes.c_hi; a.c_lo = planes.c_lo;
             a.e_scale = planes.e_scale; a.c_scale = planes.c_scale; a.ldm = planes.ldm; a.ldn = planes.ldn;
             if (d->reserved != 2) {
                 a.yf = w.yf; a.cf = w.cf;
                 a.yn = w.yn; a.cn = w.cn;  // written before they are read: no clearing
-                if (cudaMemsetAsync(w.yf, 0, (char *)w.yn - (char *)w.yf, stream) != cudaSuccess) return G2D_ERR_CUDA;
                 return sweep_pipelined(d, a, planes, stream, timer, flops);
             }
-            const int swept = sweep_macro<F>(d, a, b, stream, timer, flops, &planes);
-            if (swept != G2D_OK) return swept;
+            int status = tc_prepare_operands(a.l, a.ldl, a.u, a.ldu, d->m, d->n, planes, stream);
+            if (status == G2D_OK) status = sweep_macro<F>(d, a, b, stream, timer, flops, &planes);
+            if (status != G2D_OK) return status;
             return launch_sweep_finish(planes.error_flag, d->status, (float *)d->y, d->m * d->n, stream);
         }
     }
