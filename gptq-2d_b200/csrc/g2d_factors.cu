@@ -385,9 +385,9 @@ __global__ void __launch_bounds__(CTH) ldl_trsm_kernel(LdlBatch<F> B, int step_d
         // update (columns left of the group only); rows beyond a ragged block are zero in acc already
         const int kb_lo = kb / GROUP * GROUP;
         if (Q.tc && j < kb_lo) {
-            const int pair = step_down / (2 * GROUP);  // groups pair up by the steps of the largest problem
+            const int pair = kb / (2 * GROUP);
             __half *hi = Q.pt_hi[pair & 1], *lo = Q.pt_lo[pair & 1];
-            const int k0 = step_down % (2 * GROUP) * FB;
+            const int k0 = kb % (2 * GROUP) * FB;
             __syncthreads();
             F *const Ts = As;  // [column][k], row stride 65
 #pragma unroll
@@ -666,12 +666,12 @@ int ldl_run(int count, const int64_t *ns, F *const *as, const int *sizes, F *con
     // update of a step reaches every row above for an ordinary problem, but only the rows of the step's own group of
     // GROUP block rows for a tensor-core problem; the rows above the group are updated from the tensor cores, by two groups at
     // a time (K = 512: an entry of the matrix is read and written half as often as with one, 106 -> 99 ms for the factors of
-    // n = 28672 and 8192).  Groups pair up as (g + 1, g), g even.  Look-ahead, so that the latency-bound kernels of the
-    // next groups overlap the bulk of the updates:
-    //   * group g + 1 updates only the rows of group g (K = 256), on the chain's stream;
-    //   * group g then updates with both groups, in three launches: the rows of group g - 1 on the chain's stream, the rows of the
-    //     groups g - 2 and g - 3 (near) and everything above (rest) on a side stream.
-    // Group g - 1's own update shares its targets with near(g), which it follows; no other update on the chain meets one on the
+    // n = 28672 and 8192).  A problem's groups pair up as (p + 1, p), p even, whatever it is factored beside.  Look-ahead, so that the
+    // latency-bound kernels of the next groups overlap the bulk of the updates:
+    //   * group p + 1 updates only the rows of group p (K = 256), on the chain's stream;
+    //   * group p then updates with both groups, in three launches: the rows of group p - 1 on the chain's stream, the rows of the
+    //     groups p - 2 and p - 3 (near) and everything above (rest) on a side stream.
+    // Group p - 1's own update shares its targets with near(p), which it follows; no other update on the chain meets one on the
     // side stream, so the order of the additions is fixed, hence the result.  A pair writes the panel planes that rest of the pair
     // two before it read, and waits for that.
     static PerDeviceOnce configured;
@@ -681,12 +681,12 @@ int ldl_run(int count, const int64_t *ns, F *const *as, const int *sizes, F *con
     if (!lane) return G2D_ERR_CUDA;
     if (cudaEventRecord(lane->fork, caller) != cudaSuccess || cudaStreamWaitEvent(lane->chain, lane->fork, 0) != cudaSuccess) return G2D_ERR_CUDA;
     st = lane->chain;
-    bool recorded[4] = {false, false, false, false};  // near and rest of the last four pairs
-    int newest = -1;                                  // the last pair with an update on the side stream
+    bool recorded[4] = {false, false, false, false};  // near and rest of the last four groups, where a problem closed a pair
+    int newest = -1;                                  // the last group with an update on the side stream
     for (int s = B.steps - 1; s >= 0; --s) {  // block row of the largest problem; smaller problems are lined up by groups
         const int g = s / GROUP;
-        const int pair = g / 2;
-        if (s % (2 * GROUP) == 2 * GROUP - 1 && recorded[(pair + 2) & 3] && cudaStreamWaitEvent(st, lane->rest[(pair + 2) & 3], 0) != cudaSuccess) return G2D_ERR_CUDA;
+        // a pair that opens here writes the planes of the pair that closed three groups ago
+        if (s % GROUP == GROUP - 1 && recorded[(g + 3) & 3] && cudaStreamWaitEvent(st, lane->rest[(g + 3) & 3], 0) != cudaSuccess) return G2D_ERR_CUDA;
         ldl_diag_kernel<F><<<dim3(1, count), DTH, diag_smem<F>, st>>>(B, s);
         if (check_launch() != G2D_OK) return G2D_ERR_CUDA;
         if (s == 0) break;
@@ -709,41 +709,43 @@ int ldl_run(int count, const int64_t *ns, F *const *as, const int *sizes, F *con
         }
         if (s % GROUP != 0 || !any_tc) continue;
         // the group g is complete: the updates above it, for the tensor-core problems
-        const bool closes = g % 2 == 0;
         SyrkTcTarget next[2], near[2], rest[2];
-        int targets = 0, near_rows = 0, rest_rows = 0;
+        int targets = 0, closing = 0, rest_rows = 0;
+        bool opens = false;
         for (int z = 0; z < count; ++z) {
             const int kb_lo = s - (B.steps - padded_block_rows(ns[z]));
             if (!B.p[z].tc || kb_lo <= 0) continue;
             constexpr int PER = GROUP * FB / 128;  // tile rows per group
             const int64_t o = (int64_t)kb_lo * FB;
             const int t_all = (int)(o / 128), t_next = t_all - PER, t_near = t_next > 2 * PER ? t_next - 2 * PER : 0;  // t_next >= 0: o is at least a group
+            const bool closes = kb_lo / GROUP % 2 == 0;
             const int64_t most = closes ? 2 * GROUP * FB : GROUP * FB;
-            SyrkTcTarget t{&pt_maps[z][pair & 1], (float *)B.p[z].a, ns[z], o, t_next, t_all, closes ? 0 : GROUP * FB, (int)(ns[z] - o < most ? ns[z] - o : most), B.p[z].flag};
-            next[targets] = t;
+            SyrkTcTarget t{&pt_maps[z][kb_lo / (2 * GROUP) & 1], (float *)B.p[z].a, ns[z], o, t_next, t_all, closes ? 0 : GROUP * FB, (int)(ns[z] - o < most ? ns[z] - o : most), B.p[z].flag};
+            next[targets++] = t;
+            opens = opens || !closes;
+            if (!closes || t_next == 0) continue;
             t.t_lo = t_near;
             t.t_hi = t_next;
-            near[targets] = t;
+            near[closing] = t;
             t.t_lo = 0;
             t.t_hi = t_near;
-            rest[targets++] = t;
-            near_rows += t_next - t_near;
+            rest[closing++] = t;
             rest_rows += t_near;
         }
+        recorded[g & 3] = closing > 0;
         if (targets == 0) continue;
-        recorded[pair & 3] = closes && near_rows > 0;
-        if (recorded[pair & 3]) {  // the panels are final
-            if (cudaEventRecord(lane->panel[pair & 3], st) != cudaSuccess || cudaStreamWaitEvent(lane->stream, lane->panel[pair & 3], 0) != cudaSuccess)
+        if (closing > 0) {  // the panels are final
+            if (cudaEventRecord(lane->panel[g & 3], st) != cudaSuccess || cudaStreamWaitEvent(lane->stream, lane->panel[g & 3], 0) != cudaSuccess)
                 return G2D_ERR_CUDA;
-            int status = launch_syrk_tc(targets, near, lane->stream);
+            int status = launch_syrk_tc(closing, near, lane->stream);
             if (status != G2D_OK) return status;
-            if (cudaEventRecord(lane->near[pair & 3], lane->stream) != cudaSuccess) return G2D_ERR_CUDA;
-            if (rest_rows > 0) status = launch_syrk_tc(targets, rest, lane->stream);
+            if (cudaEventRecord(lane->near[g & 3], lane->stream) != cudaSuccess) return G2D_ERR_CUDA;
+            if (rest_rows > 0) status = launch_syrk_tc(closing, rest, lane->stream);
             if (status != G2D_OK) return status;
-            if (cudaEventRecord(lane->rest[pair & 3], lane->stream) != cudaSuccess) return G2D_ERR_CUDA;
-            newest = pair;
+            if (cudaEventRecord(lane->rest[g & 3], lane->stream) != cudaSuccess) return G2D_ERR_CUDA;
+            newest = g;
         }
-        if (!closes && recorded[(pair + 1) & 3] && cudaStreamWaitEvent(st, lane->near[(pair + 1) & 3], 0) != cudaSuccess) return G2D_ERR_CUDA;
+        if (opens && recorded[(g + 1) & 3] && cudaStreamWaitEvent(st, lane->near[(g + 1) & 3], 0) != cudaSuccess) return G2D_ERR_CUDA;
         const int status = launch_syrk_tc(targets, next, st);
         if (status != G2D_OK) return status;
     }

@@ -89,13 +89,14 @@ def test_cluster_search_matches_the_oracle(oracle, rows, T, K, V, tail):
 
 
 # k and n around the 64-wide chunks and the 128- and 256-wide tiles; k = 512 and n = 2048 end the range in which the split kernel
-# finds the channels' ranges itself; rows of x that are not 16-byte multiples
-@pytest.mark.parametrize("k, n", [(1, 4), (63, 129), (65, 255), (512, 2048), (513, 2048), (512, 2052), (300, 1001), (2000, 4100)])
-def test_gram_at_edges(k, n):
+# finds the channels' ranges itself; x that starts off a 16-byte boundary
+@pytest.mark.parametrize("k, n, offset", [(1, 4, 0), (63, 132, 0), (65, 252, 1), (512, 2048, 0), (513, 2048, 0), (512, 2052, 0), (300, 1004, 1), (2000, 4100, 0)])
+def test_gram_at_edges(k, n, offset):
     import kron_factors as K
 
     gen = torch.Generator(device="cuda").manual_seed(k + n)
-    x = torch.randn(k, n, generator=gen, device="cuda") * torch.exp(2 * torch.randn(n, generator=gen, device="cuda"))
+    x = torch.randn(offset + k * n, generator=gen, device="cuda")[offset:].view(k, n)
+    x *= torch.exp(2 * torch.randn(n, generator=gen, device="cuda"))
     x[:, n // 2] = 0
     h0 = torch.randn(n, n, generator=gen, device="cuda")
     h0 = h0 + h0.T
