@@ -261,37 +261,32 @@ def run_reference(args) -> None:
     print(json.dumps(line))
 
 
-def measure_tf32_peak(device) -> dict:
-    """Dense TF32 matrix-product throughput of this GPU through torch.matmul (cuBLAS), measured the way the bf16 figure of
+def measure_fp16_peak(device) -> dict:
+    """Dense fp16 matrix-product throughput of this GPU through torch.matmul (cuBLAS), measured the way the bf16 figure of
     MEASURED_PEAKS.json was: 8192^3, best of 10 (burst) and back to back for about a second (sustained)."""
     import torch
 
     n = 8192
-    a, b = torch.randn(n, n, device=device), torch.randn(n, n, device=device)
-    before = torch.backends.cuda.matmul.allow_tf32
-    torch.backends.cuda.matmul.allow_tf32 = True
-    try:
-        begin, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
-        for _ in range(3):
-            a @ b
-        best = float("inf")
-        for _ in range(10):
-            begin.record()
-            a @ b
-            end.record()
-            torch.cuda.synchronize()
-            best = min(best, begin.elapsed_time(end))
-        count = max(10, int(1000.0 / best))
+    a, b = (torch.randn(n, n, device=device, dtype=torch.float16) for _ in range(2))
+    begin, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+    for _ in range(3):
+        a @ b
+    best = float("inf")
+    for _ in range(10):
         begin.record()
-        for _ in range(count):
-            a @ b
+        a @ b
         end.record()
         torch.cuda.synchronize()
-        sustained = begin.elapsed_time(end) / count
-    finally:
-        torch.backends.cuda.matmul.allow_tf32 = before
+        best = min(best, begin.elapsed_time(end))
+    count = max(10, int(1000.0 / best))
+    begin.record()
+    for _ in range(count):
+        a @ b
+    end.record()
+    torch.cuda.synchronize()
+    sustained = begin.elapsed_time(end) / count
     flops = 2.0 * n ** 3
-    return {"burst_tflops": flops / best / 1e9, "sustained_tflops": flops / sustained / 1e9, "how": f"torch.matmul fp32 with TF32 allowed, {n}^3, best of 10 and {count} back to back"}
+    return {"burst_tflops": flops / best / 1e9, "sustained_tflops": flops / sustained / 1e9, "how": f"torch.matmul fp16, {n}^3, best of 10 and {count} back to back"}
 
 
 def main() -> None:
@@ -303,7 +298,7 @@ def main() -> None:
     parser.add_argument("--size", type=int, default=8192)
     parser.add_argument("--cpu-sample", type=int, default=0, help="side of the CPU arm's sweep sample; 0 chooses by the time budget")
     parser.add_argument("--no-cpu-baseline", action="store_true")
-    parser.add_argument("--no-peak-probe", action="store_true", help="skip the TF32 matrix-product measurement (for runs under a profiler)")
+    parser.add_argument("--no-peak-probe", action="store_true", help="skip the fp16 matrix-product measurement (for runs under a profiler)")
     parser.add_argument("--layer-set-blocks", type=int, default=8, help="blocks of the 70B-shaped layer set run after the timed steps (0: none)")
     args = parser.parse_args()
     if args.steps is None:
@@ -502,24 +497,24 @@ def main() -> None:
     alone_tflops = alone_flops / (alone_ms * 1e-3) / 1e12 if alone_ms > 0 else 0.0
     del y_alone
     pk = peaks()
-    tensor_peak = pk["bf16_tflops_sustained"] / 6.0  # fp32-faithful tensor roofline: TF32 = bf16 / 2, three TF32 products per fp32 product
+    tensor_peak = pk["bf16_tflops_sustained"] / 3.0  # fp32-faithful tensor roofline: three products of 16-bit halves per fp32 product
     far_tflops = far_flops / (far_ms * 1e-3) / 1e12 if far_ms > 0 else 0.0
     near_tflops = near_flops / (near_ms * 1e-3) / 1e12 if near_ms > 0 else 0.0
     panel_tflops = (near_flops + far_flops) / ((near_ms + far_ms) * 1e-3) / 1e12 if near_ms + far_ms > 0 else 0.0
-    tf32 = {"burst_tflops": None, "sustained_tflops": None, "how": "skipped"} if args.no_peak_probe else measure_tf32_peak(device)
-    measured_peak = tf32["sustained_tflops"] / 3.0 if tf32["sustained_tflops"] else None
+    fp16 = {"burst_tflops": None, "sustained_tflops": None, "how": "skipped"} if args.no_peak_probe else measure_fp16_peak(device)
+    measured_peak = fp16["sustained_tflops"] / 3.0 if fp16["sustained_tflops"] else None
     rtn = torch.clamp(torch.round(w / scale), -8, 7) * scale
     objective_vs_rtn = synthetic.objective(z, w, g, h) / synthetic.objective(rtn, w, g, h)
     roofline = {
-        "bound": "tensor", "kernel": "macro_update_tc_kernel (tcgen05 kind::tf32, 3xTF32 split; far updates: the lowest-priority stream of three, on the SMs that the tile launch of the moment leaves free)",
+        "bound": "tensor", "kernel": "macro_update_wide_kernel, macro_update_tc_kernel (tcgen05 kind::f16, fp16 pairs under a scale per tile, three products; far updates: the lowest-priority stream of three, on the SMs that the tile launch of the moment leaves free)",
         "achieved": far_tflops, "peak": tensor_peak, "unit": "TFLOP/s", "frac": far_tflops / tensor_peak if tensor_peak else None,
-        # DRAM bytes of one launch are not measured live: an ncu capture of this kernel at 4096 x 4096 read and wrote
-        # 149.7 MB for 946 target macro tiles; that figure scaled by the target tiles of an average launch here
-        "traffic": 149.7e6 / 946 * (far_flops / far_n / (2 * 2 * 128 * 128 * 512)) if far_n else None,
-        "traffic_basis": "ncu capture at 4096 x 4096 (dram__bytes_read.sum + dram__bytes_write.sum of one launch), scaled by target macro tiles; not measured in this run",
-        "peak_basis": f"{pk['source']} bf16 sustained {pk['bf16_tflops_sustained']} TFLOP/s / 2 (TF32) / 3 (three tf32 products per fp32 product)",
-        "peak_measured_tf32": {**tf32, "fp32_faithful_peak": measured_peak, "frac_of_it": far_tflops / measured_peak if measured_peak else None},
-        "near": {"kernel": "band_tc_kernel (tcgen05 kind::tf32, M 128 x N 64, rank-64 updates on a side stream)", "achieved": near_tflops,
+        # DRAM bytes of one launch are not measured live: an ncu capture of a far update at 8192 x 8192 read and wrote 741.1 MB
+        # for 46.0 GFLOP (rank 512); that ratio applied to the flops of an average launch here
+        "traffic": 741.1e6 / 46.0e9 * far_flops / far_n if far_n else None,
+        "traffic_basis": "ncu capture at 8192 x 8192 (dram__bytes_read.sum + dram__bytes_write.sum of one launch), scaled by algorithmic flops; not measured in this run",
+        "peak_basis": f"{pk['source']} bf16 sustained {pk['bf16_tflops_sustained']} TFLOP/s / 3 (three products of 16-bit halves per fp32 product)",
+        "peak_measured_fp16": {**fp16, "fp32_faithful_peak": measured_peak, "frac_of_it": far_tflops / measured_peak if measured_peak else None},
+        "near": {"kernel": "band_tc_kernel (tcgen05 kind::f16, M 128 x N 64, rank-64 updates on a side stream)", "achieved": near_tflops,
                  "frac": near_tflops / tensor_peak if tensor_peak else None, "launches": int(near_n), "algorithmic_flops": near_flops},
         "panel_gemms": {"what": "near + far updates: their algorithmic flops over their summed stream time", "achieved": panel_tflops,
                         "frac": panel_tflops / tensor_peak if tensor_peak else None, "algorithmic_flops": near_flops + far_flops,

@@ -317,7 +317,7 @@ constexpr int kFarLagMacro = 1;  // a far update reaches the macro anti-diagonal
 //     load one launch later;
 //   * near update of the tile anti-diagonal s (its tiles as sources, targets from s + 2 on), on a side stream,
 //     concurrent with the tile launch of s + 1;
-//   * far update of a group of macro anti-diagonals (128 x 128 macro tiles = 2 x 2 tiles; rank 512 by default), on a
+//   * far update of a group of macro anti-diagonals (128 x 128 macro tiles = 2 x 2 tiles; rank 512 or 1024), on a
 //     second side stream, into planes of its own that a tile adds when it loads.  It reaches the macro anti-diagonals
 //     from kFarLagMacro past the group's end, which the tile launches get to two launches after the group's last
 //     tile; the near updates stop where the far update of their source's group starts.  A far update runs as two
@@ -326,9 +326,8 @@ constexpr int kFarLagMacro = 1;  // a far update reaches the macro anti-diagonal
 //     them, which the tile launches only need a whole group later.
 // The tile launches run on a stream of the library's own with the highest priority, the near updates below it, the far
 // updates lowest: a CTA slot that frees up goes to the critical path first.  A CTA of the tile sweep fills the registers
-// of two of its SM's four schedulers (six warps of up to 240 registers), so no CTA of an update kernel ever shares an SM
-// with it: the updates run on the SMs that the tile launch of the moment leaves free, and the far update may as well use
-// its full three-stage ring there.  Updates that share target planes are
+// of its SM (eight warps of up to 233), so no CTA of an update kernel ever shares one with it: the updates run on the SMs
+// that the tile launch of the moment leaves free.  Updates that share target planes are
 // ordered on one stream, so the additions have a fixed order.
 int sweep_pipelined(const g2d_sweep_desc *d, SweepArgs<float> &a, const TcPlanes &planes, cudaStream_t caller, LaunchTimer *timer, double *flops) {
     std::unique_lock<std::mutex> held;

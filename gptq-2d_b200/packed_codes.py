@@ -20,12 +20,19 @@ import _abi
 
 
 def _operands(m: int, n: int, scale: torch.Tensor, zero_point: torch.Tensor, dtype, device):
+    """The two parameters with their strides over the matrix.  Small calls are bound by this host code, so the strides of a
+    broadcast are formed here instead of through an expanded view (pack and unpack of 64 x 256 together: 40 -> 33 us)."""
     out = []
     for name, t in (("scale", scale), ("zero_point", zero_point)):
-        t = torch.as_tensor(t, dtype=dtype, device=device)
-        assert t.dim() <= 2, f"{name} must broadcast to the matrix"
-        t = torch.broadcast_to(t, (m, n))
-        out.append((t, t.stride(0), t.stride(1)))
+        if not isinstance(t, torch.Tensor) or t.dtype != dtype or t.device != device:
+            t = torch.as_tensor(t, dtype=dtype, device=device)
+        shape = t.shape
+        assert len(shape) <= 2, f"{name} must broadcast to the matrix"
+        rows, cols = (1, 1, *shape)[-2:]
+        if rows not in (1, m) or cols not in (1, n):
+            t = torch.broadcast_to(t, (m, n))  # raises
+        strides = (0, 0, *t.stride())[-2:]
+        out.append((t, strides[0] if rows == m else 0, strides[1] if cols == n else 0))
     return out
 
 

@@ -102,9 +102,8 @@ int g2d_sweep_fused(const g2d_sweep_desc *desc, void *stream);
  *  - All calls on a device share the array, which keeps the previous call's contents (the sweep clears what it
  *    needs cleared).  Two calls that overlap on the GPU, e.g. on different streams, race: serialise them.
  *  - Calls no cudaMalloc / cudaFree and no allocating library routine.  It always takes the tile schedule, so its
- *    results are those of g2d_sweep_fused with desc->reserved = 1, bit for bit (for one fp32 matrix whose sides are
- *    multiples of 4, g2d_sweep_fused by default takes the pipelined schedule, which sums the feedback in another
- *    order and may differ at rounding ties). */
+ *    results are those of g2d_sweep_fused with desc->reserved = 1, bit for bit (by default g2d_sweep_fused takes a
+ *    schedule with concurrent updates, which sums the feedback in another order and may differ at rounding ties). */
 #define G2D_STATIC_SCRATCH_BYTES (32u * 1024u * 1024u)
 int g2d_sweep_fused_static(const g2d_sweep_desc *desc, void *stream);
 
