@@ -13,7 +13,6 @@ constexpr int MT = 128;                    // macro tile edge
 constexpr int KC = 32;                     // floats per 128-byte swizzle row
 constexpr int STAGES = 3;
 constexpr int TC_THREADS = 192;
-constexpr uint32_t TMEM_COLS = 256;
 constexpr long long WAIT_CYCLES = 2000000000LL;  // about a second
 
 __device__ __forceinline__ uint32_t smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -167,7 +166,6 @@ __device__ __forceinline__ void box_reduce_add(const CUtensorMap *map, uint32_t 
 }
 __device__ __forceinline__ void box_fence() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 __device__ __forceinline__ void box_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
-__device__ __forceinline__ void box_free() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }  // the lane's boxes may be overwritten
 // A 32 x 32 block of results through two boxes of 16 rows (4 KB of shared memory in turn): one is filled while the TMA still reads
 // the other.  With one box of 32 rows the warp waited for it every time, and the eight warps took 6000 cycles for the results of a
 // 128 x 256 tile, twice what the two accumulators of the pipeline hide (factors of 28672 and 8192: 97.1 -> 94.3 ms, the far updates of
