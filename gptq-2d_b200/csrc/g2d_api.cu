@@ -200,8 +200,8 @@ int sweep_macro(const g2d_sweep_desc *d, SweepArgs<F> &a, BandArgs<F> &b64, cuda
     return G2D_OK;
 }
 
-// Side streams and events of the pipelined schedule.  A device has four lanes; calls take them round robin and hold a
-// lane's lock while they enqueue, so sweeps that a caller runs concurrently on several streams (or from several host
+// Side streams and events of the pipelined schedule.  A device has four lanes; a call takes one (see LaneChoice) and holds its
+// lock while it enqueues, so sweeps that a caller runs concurrently on several streams (or from several host
 // threads) never interleave their event records on one lane.  All four lanes of a device are built by the first
 // pipelined call on it, which therefore must not run inside a stream capture (stream and event creation is not
 // capturable): during capture, a device whose lanes do not exist yet gets G2D_ERR_UNSUPPORTED.
@@ -213,7 +213,7 @@ struct PipeLane {
 struct DeviceLanes {
     std::mutex build;
     bool ready = false;
-    unsigned next = 0;
+    LaneChoice choice;
     PipeLane lane[4];
 };
 
@@ -257,7 +257,7 @@ PipeLane *acquire_pipe_lane(cudaStream_t caller, std::unique_lock<std::mutex> &h
     *status = G2D_ERR_CUDA;
     if (cudaGetDevice(&device) != cudaSuccess || device < 0 || device >= 64) return nullptr;
     DeviceLanes &dl = devices[device];
-    unsigned slot;
+    int slot;
     {
         std::lock_guard<std::mutex> lock(dl.build);
         if (!dl.ready) {
@@ -275,7 +275,7 @@ PipeLane *acquire_pipe_lane(cudaStream_t caller, std::unique_lock<std::mutex> &h
             }
             dl.ready = true;
         }
-        slot = dl.next++ & 3;
+        slot = dl.choice.pick(caller);
     }
     held = std::unique_lock<std::mutex>(dl.lane[slot].busy);
     *status = G2D_OK;

@@ -299,6 +299,23 @@ struct BlockUpdateArgs {
 template <typename F>
 int launch_block_update(const BlockUpdateArgs<F> &args, cudaStream_t stream);
 
+// Which of four lanes of side streams a call takes: the one that the last call on the same stream took (the two run in order
+// anyway), else the next in turn.  The GPU has few hardware queues (eight connections by default): a program that issues
+// its calls on one or two streams then keeps to as many lanes, and its streams do not share a queue with one another.
+struct LaneChoice {
+    cudaStream_t last[4] = {};
+    bool used[4] = {};
+    unsigned next = 0;
+    int pick(cudaStream_t caller) {  // under the owner's lock
+        for (int k = 0; k < 4; ++k)
+            if (used[k] && last[k] == caller) return k;
+        const int k = (int)(next++ & 3);
+        last[k] = caller;
+        used[k] = true;
+        return k;
+    }
+};
+
 // Overlapped schedule: tile launches on the critical path, everything else beside them (see g2d_api.cu).
 // tiles(s, stream) sweeps tile anti-diagonal s; update(s0, s1, t0, t1, far, stream) carries the sources s0..s1-1 into the
 // targets t0..t1-1, into the far planes or into Y and C.  `pushes`: a tile hands the feedback for its two neighbours on itself.

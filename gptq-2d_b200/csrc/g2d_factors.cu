@@ -564,21 +564,21 @@ __global__ void ldl_scale_kernel(F *out, int64_t n, int size, const F *dblk, con
 
 // Streams for the look-ahead of the trailing updates: the chain of diagonal blocks and panels on one of the highest priority, the
 // bulk of the updates on one of the lowest, so that a kernel of the chain takes the next SM that comes free instead of queueing
-// behind a millisecond of update CTAs (on two streams of one priority the two ran one after the other).  Calls take lanes round
-// robin, so two factorizations that a caller runs concurrently on two streams do not share one.  Created on first use per
+// behind a millisecond of update CTAs (on two streams of one priority the two ran one after the other).  Two
+// factorizations that a caller runs concurrently on two streams take two lanes (see LaneChoice).  Created on first use per
 // device and kept.
 struct SideLane {
     cudaStream_t stream = nullptr, chain = nullptr;
     cudaEvent_t panel[4] = {}, near[4] = {}, rest[4] = {}, fork = nullptr, join = nullptr;
 };
-static SideLane *acquire_side_lane() {
+static SideLane *acquire_side_lane(cudaStream_t caller) {
     static std::mutex mutex;
     static SideLane lanes[64][4];
-    static unsigned next[64] = {};
+    static LaneChoice choice[64];
     int device = 0;
     if (cudaGetDevice(&device) != cudaSuccess || device < 0 || device >= 64) return nullptr;
     std::lock_guard<std::mutex> lock(mutex);
-    SideLane *lane = &lanes[device][next[device]++ & 3];
+    SideLane *lane = &lanes[device][choice[device].pick(caller)];
     if (!lane->stream) {
         int least = 0, greatest = 0;
         if (cudaDeviceGetStreamPriorityRange(&least, &greatest) != cudaSuccess) return nullptr;
@@ -677,7 +677,7 @@ int ldl_run(int count, const int64_t *ns, F *const *as, const int *sizes, F *con
     static PerDeviceOnce configured;
     if (configured.run([&] { return cudaFuncSetAttribute(ldl_diag_kernel<F>, cudaFuncAttributeMaxDynamicSharedMemorySize, diag_smem<F>) == cudaSuccess; }) != G2D_OK)
         return G2D_ERR_CUDA;
-    SideLane *lane = acquire_side_lane();
+    SideLane *lane = acquire_side_lane(caller);
     if (!lane) return G2D_ERR_CUDA;
     if (cudaEventRecord(lane->fork, caller) != cudaSuccess || cudaStreamWaitEvent(lane->chain, lane->fork, 0) != cudaSuccess) return G2D_ERR_CUDA;
     st = lane->chain;

@@ -44,7 +44,7 @@ def ldl_of_inverse(M: torch.Tensor, size: int = 1, check: bool = True) -> torch.
         if pivot:
             raise torch.linalg.LinAlgError(f"ldl_of_inverse: the matrix is not positive definite (pivot {pivot} is not positive)")
     else:
-        _PENDING.append((flag, ("the matrix",)))  # settled by check_pending(), like the pair call's flags
+        _remember(flag, ("the matrix",))  # settled by check_pending(), like the pair call's flags
     return out
 
 
@@ -186,15 +186,53 @@ def feedback_factors_from_grams(g: torch.Tensor, h: torch.Tensor, super_entry_sh
     if check:
         _raise_for_flags(flags.tolist(), ("G", "H"))
     else:
-        _PENDING.append((flags, ("G", "H")))
-        if len(_PENDING) > _PENDING_LIMIT:  # a long unchecked run: settle the oldest call (it finished long ago)
-            oldest, names = _PENDING.pop(0)
-            _raise_for_flags(oldest.tolist(), names)
+        _remember(flags, ("G", "H"))
+        if len(_PENDING) > _PENDING_LIMIT and not torch.cuda.is_current_stream_capturing():
+            _settle_oldest()
     return outs[0], outs[1].t()
 
 
-_PENDING: list[tuple[torch.Tensor, tuple[str, ...]]] = []  # status flags of the calls made with check=False, oldest first
+_PENDING: list[tuple[torch.Tensor, tuple[str, ...], torch.cuda.Event | None]] = []  # status flags of the calls made with check=False, oldest first
 _PENDING_LIMIT = 256
+_SETTLING: dict[torch.device, torch.cuda.Stream] = {}
+
+
+def _remember(flags: torch.Tensor, names: tuple[str, ...]) -> None:
+    """Keeps the flags of an unchecked call with the event of its end (a call inside a stream capture has none)."""
+    event = None
+    if not torch.cuda.is_current_stream_capturing():
+        event = torch.cuda.Event()
+        event.record(torch.cuda.current_stream(flags.device))
+    _PENDING.append((flags, names, event))
+
+
+def _settle_oldest() -> None:
+    """A long unchecked run: settle the older half of the calls, all of which finished long ago.  Their flags are read on a stream of
+    this module's own: a read on the caller's stream would wait for everything issued so far, and the host would stay
+    one call ahead of the GPU (a block of seven matrices of width 1024: 15.4 -> 12.9 ms)."""
+    batch = []
+    while len(batch) < _PENDING_LIMIT // 2 and _PENDING:
+        batch.append(_PENDING.pop(0))
+    values: list[list[int]] = [[] for _ in batch]
+    for device in {flags.device for flags, _, _ in batch}:
+        mine = [k for k, (flags, _, event) in enumerate(batch) if flags.device == device and event is not None]
+        if not mine:
+            continue
+        for k in mine:
+            batch[k][2].synchronize()
+        if device not in _SETTLING:
+            _SETTLING[device] = torch.cuda.Stream(device=device)
+        with torch.cuda.stream(_SETTLING[device]):
+            read = torch.cat([batch[k][0] for k in mine]).tolist()
+        for k in mine:
+            count = batch[k][0].numel()
+            values[k], read = read[:count], read[count:]
+    for k, (flags, names, event) in enumerate(batch):
+        try:
+            _raise_for_flags(flags.tolist() if event is None else values[k], names)
+        except Exception:
+            _PENDING[:0] = batch[k + 1:]  # as if only the calls up to the failing one had been settled
+            raise
 
 
 def _raise_for_flags(pivots, names) -> None:
@@ -216,5 +254,5 @@ def check_pending() -> None:
     ``check=True`` would have raised (``torch.linalg.LinAlgError`` for a Gram that is not positive definite, as the
     reference's ``torch.linalg.cholesky`` does; ``RuntimeError`` for a bounded wait that ran out)."""
     while _PENDING:
-        flags, names = _PENDING.pop(0)
+        flags, names, _ = _PENDING.pop(0)
         _raise_for_flags(flags.tolist(), names)

@@ -133,6 +133,24 @@ def test_float_factors_at_group_edges(n, other):
         assert torch.equal(got, K.ldl_of_inverse(m.float()))  # two problems in one pass equal two passes
 
 
+@pytest.mark.parametrize("before", [0, 127, 128, 200])
+def test_flags_of_a_long_unchecked_run(before):
+    """A matrix that is not positive definite is reported by one of the next 256 calls; the calls around it stay settled or pending."""
+    import kron_factors as K
+
+    K.check_pending()
+    good = 2 * torch.eye(64, device="cuda")
+    bad = good.clone()
+    bad[5, 5] = -1
+    for _ in range(before):
+        K.feedback_factors_from_grams(good, good)
+    K.feedback_factors_from_grams(good, bad)
+    with pytest.raises(torch.linalg.LinAlgError, match="H is not positive definite"):
+        for _ in range(256):
+            K.feedback_factors_from_grams(good, good)
+    K.check_pending()
+
+
 @pytest.mark.parametrize("bits", range(1, 9))
 def test_pack_out_of_the_fast_range(oracle, bits):
     """Scales and quotients beyond the reciprocal form's range, a field far from zero, a ragged last group, ties to even."""
