@@ -192,7 +192,7 @@ __global__ void __launch_bounds__(DTH) ldl_diag_kernel(LdlBatch<F> B, int step_d
                 for (int r = 0; r < DS; ++r) w[r] = col[r];
                 F root, inv_root, inv;
                 pivot_roots(w[DS - 1], root, inv_root, inv);
-                worst = r0 + j < bs && !(w[DS - 1] > (F)0) ? r0 + j + 1 : worst;
+                worst = worst > FB && r0 + j < bs && !(w[DS - 1] > (F)0) ? r0 + j + 1 : worst;  // the first: its root makes the later ones NaN
                 const F f0 = v0[DS - 1] * inv, f1 = v1[DS - 1] * inv;
                 // what lies right of the diagonal is stored along and never read
                 F *const row = S + (r0 + j) * DLDS;
@@ -205,7 +205,7 @@ __global__ void __launch_bounds__(DTH) ldl_diag_kernel(LdlBatch<F> B, int step_d
                     v1[r] = v1[r - 1] - f1 * w[r - 1];
                 }
             }
-            if (lane == 0 && worst < bad) bad = worst;
+            if (lane == 0 && bad > FB) bad = worst;
         }
         __syncthreads();
         if (r0 == 0) break;

@@ -133,6 +133,19 @@ def test_float_factors_at_group_edges(n, other):
         assert torch.equal(got, K.ldl_of_inverse(m.float()))  # two problems in one pass equal two passes
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
+@pytest.mark.parametrize("n, k", [(1, 0), (64, 5), (64, 16), (64, 60), (130, 122), (400, 85), (1000, 3)])
+def test_the_failing_pivot_is_named(n, k, dtype):
+    """Pivots are eliminated from the last to the first, 16 rows of a block of 64 at a time."""
+    import kron_factors as K
+
+    x = torch.randn(2 * n, n, generator=torch.Generator(device="cuda").manual_seed(n), device="cuda", dtype=dtype)
+    h = x.T @ x / (2 * n) + torch.eye(n, device="cuda", dtype=dtype)
+    h[k, k] = -1
+    with pytest.raises(torch.linalg.LinAlgError, match=rf"pivot {k + 1} "):
+        K.ldl_of_inverse(h)
+
+
 @pytest.mark.parametrize("before", [0, 127, 128, 200])
 def test_flags_of_a_long_unchecked_run(before):
     """A matrix that is not positive definite is reported by one of the next 256 calls; the calls around it stay settled or pending."""
