@@ -337,21 +337,25 @@ int sweep_pipelined(const g2d_sweep_desc *d, SweepArgs<float> &a, const TcPlanes
     // fork: everything the caller's stream holds so far comes first
     cudaStream_t stream = lane->tiles;
     if (cudaEventRecord(lane->fork, caller) != cudaSuccess || cudaStreamWaitEvent(stream, lane->fork, 0) != cudaSuccess) return G2D_ERR_CUDA;
-    BandTcMaps maps;
-    MacroTcMaps far_maps;
-    int status = band_tc_prepare(&maps, planes, a.y, a.c, d->m, d->n, a.ld);
-    if (status == G2D_OK) status = macro_tc_prepare(&far_maps, planes, (float *)a.yf, (float *)a.cf, d->m, d->n, a.ld);
-    // the operands of the updates are prepared beside the first tile launches, which do not need them
-    if (cudaStreamWaitEvent(lane->near, lane->fork, 0) != cudaSuccess) return G2D_ERR_CUDA;
-    if (status == G2D_OK) status = tc_prepare_operands(a.l, a.ldl, a.u, a.ldu, d->m, d->n, planes, lane->near);
-    if (status != G2D_OK) return status;
-    if (cudaEventRecord(lane->prepared, lane->near) != cudaSuccess) return G2D_ERR_CUDA;
     const int waves = a.nI + a.nJ - 1;
     const int waves_macro = (int)(ceil_div(d->m, MACRO) + ceil_div(d->n, MACRO)) - 1;
     // Macro anti-diagonals per far update.  The far updates' share of the SMs grows with m n, the tile launches' time does not: from
     // about 12288 x 12288 on the far updates bound the sweep, and twice the rank costs them less (results leave half as often)
     // than the near updates that it adds (16384 x 16384: 56.3 -> 53.8 ms, 8192 x 28672: 56.7 -> 55.0; 8192 x 8192: 10.9 -> 11.3).
     const int outer = d->outer_tiles > 0 ? (d->outer_tiles + 1) / 2 : (double)d->m * (double)d->n >= 1.5e8 ? 2 * kDefaultOuterMacro : kDefaultOuterMacro;
+    // what the updates need, where there are any: the smallest sweeps are bound by this host code
+    BandTcMaps maps;
+    MacroTcMaps far_maps;
+    int status = G2D_OK;
+    if (waves > 2) {
+        status = band_tc_prepare(&maps, planes, a.y, a.c, d->m, d->n, a.ld);
+        if (status == G2D_OK && outer + kFarLagMacro < waves_macro) status = macro_tc_prepare(&far_maps, planes, (float *)a.yf, (float *)a.cf, d->m, d->n, a.ld);
+        // the operands of the updates are prepared beside the first tile launches, which do not need them
+        if (status == G2D_OK && cudaStreamWaitEvent(lane->near, lane->fork, 0) != cudaSuccess) status = G2D_ERR_CUDA;
+        if (status == G2D_OK) status = tc_prepare_operands(a.l, a.ldl, a.u, a.ldu, d->m, d->n, planes, lane->near);
+        if (status == G2D_OK && cudaEventRecord(lane->prepared, lane->near) != cudaSuccess) status = G2D_ERR_CUDA;
+        if (status != G2D_OK) return status;
+    }
     int last_near = -1, last_far = -1;
     for (int s = 0; s < waves; ++s) {
         // what the tiles of s need: every near update up to s - 2, and the far update whose first targets they are
@@ -407,7 +411,7 @@ int sweep_pipelined(const g2d_sweep_desc *d, SweepArgs<float> &a, const TcPlanes
         }
     }
     // join: what follows the call on the caller's stream follows everything the call did
-    if (cudaStreamWaitEvent(stream, last_near >= 0 ? lane->near_done[last_near & 7] : lane->prepared, 0) != cudaSuccess) return G2D_ERR_CUDA;
+    if (last_near >= 0 && cudaStreamWaitEvent(stream, lane->near_done[last_near & 7], 0) != cudaSuccess) return G2D_ERR_CUDA;
     if (last_far >= 0 && cudaStreamWaitEvent(stream, lane->far_done[last_far & 3], 0) != cudaSuccess) return G2D_ERR_CUDA;
     if (a.y != d->y && cudaMemcpy2DAsync(d->y, d->n * 4, a.y, a.ld * 4, d->n * 4, d->m, cudaMemcpyDeviceToDevice, stream) != cudaSuccess) return G2D_ERR_CUDA;
     status = launch_sweep_finish(planes.error_flag, d->status, (float *)d->y, d->m * d->n, stream);
