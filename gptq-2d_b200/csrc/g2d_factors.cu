@@ -566,33 +566,38 @@ __global__ void ldl_scale_kernel(F *out, int64_t n, int size, const F *dblk, con
 // bulk of the updates on one of the lowest, so that a kernel of the chain takes the next SM that comes free instead of queueing
 // behind a millisecond of update CTAs (on two streams of one priority the two ran one after the other).  Two
 // factorizations that a caller runs concurrently on two streams take two lanes (see LaneChoice).  Created on first use per
-// device and kept.
+// device and kept.  A call holds its lane's lock while it enqueues: two host threads whose streams share a lane (more than four
+// streams, or one handle such as the per-thread default stream's) would otherwise record and wait for each other's events,
+// and a chain could start before its own matrix is there.
 struct SideLane {
     cudaStream_t stream = nullptr, chain = nullptr;
     cudaEvent_t panel[4] = {}, near[4] = {}, rest[4] = {}, fork = nullptr, join = nullptr;
+    bool ready = false;
+    std::mutex busy;
 };
-static SideLane *acquire_side_lane(cudaStream_t caller) {
-    static std::mutex mutex;
+static bool build_side_lane(SideLane &l) {
+    int least = 0, greatest = 0;
+    if (cudaDeviceGetStreamPriorityRange(&least, &greatest) != cudaSuccess) return false;
+    auto stream = [](cudaStream_t &s, int priority) { return s || cudaStreamCreateWithPriority(&s, cudaStreamNonBlocking, priority) == cudaSuccess; };
+    auto event = [](cudaEvent_t &e) { return e || cudaEventCreateWithFlags(&e, cudaEventDisableTiming) == cudaSuccess; };
+    bool ok = stream(l.stream, least) && stream(l.chain, greatest) && event(l.fork) && event(l.join);
+    for (int k = 0; k < 4 && ok; ++k) ok = event(l.panel[k]) && event(l.near[k]) && event(l.rest[k]);
+    return l.ready = ok;
+}
+// A lane of the current device with its lock held (through `held`), or null.
+static SideLane *acquire_side_lane(cudaStream_t caller, std::unique_lock<std::mutex> &held) {
+    static std::mutex choosing;
     static SideLane lanes[64][4];
     static LaneChoice choice[64];
     int device = 0;
     if (cudaGetDevice(&device) != cudaSuccess || device < 0 || device >= 64) return nullptr;
-    std::lock_guard<std::mutex> lock(mutex);
-    SideLane *lane = &lanes[device][choice[device].pick(caller)];
-    if (!lane->stream) {
-        int least = 0, greatest = 0;
-        if (cudaDeviceGetStreamPriorityRange(&least, &greatest) != cudaSuccess) return nullptr;
-        if (cudaStreamCreateWithPriority(&lane->stream, cudaStreamNonBlocking, least) != cudaSuccess ||
-            cudaStreamCreateWithPriority(&lane->chain, cudaStreamNonBlocking, greatest) != cudaSuccess ||
-            cudaEventCreateWithFlags(&lane->fork, cudaEventDisableTiming) != cudaSuccess || cudaEventCreateWithFlags(&lane->join, cudaEventDisableTiming) != cudaSuccess)
-            return nullptr;
-        for (int k = 0; k < 4; ++k)
-            if (cudaEventCreateWithFlags(&lane->panel[k], cudaEventDisableTiming) != cudaSuccess ||
-                cudaEventCreateWithFlags(&lane->near[k], cudaEventDisableTiming) != cudaSuccess ||
-                cudaEventCreateWithFlags(&lane->rest[k], cudaEventDisableTiming) != cudaSuccess)
-                return nullptr;
+    SideLane *lane;
+    {
+        std::lock_guard<std::mutex> lock(choosing);
+        lane = &lanes[device][choice[device].pick(caller)];
     }
-    return lane;
+    held = std::unique_lock<std::mutex>(lane->busy);
+    return lane->ready || build_side_lane(*lane) ? lane : nullptr;
 }
 
 // Workspace of one problem: inverted diagonal blocks, normalisation blocks, scratch of the doubling steps and, for float, the
@@ -677,7 +682,8 @@ int ldl_run(int count, const int64_t *ns, F *const *as, const int *sizes, F *con
     static PerDeviceOnce configured;
     if (configured.run([&] { return cudaFuncSetAttribute(ldl_diag_kernel<F>, cudaFuncAttributeMaxDynamicSharedMemorySize, diag_smem<F>) == cudaSuccess; }) != G2D_OK)
         return G2D_ERR_CUDA;
-    SideLane *lane = acquire_side_lane(caller);
+    std::unique_lock<std::mutex> held;  // until everything is enqueued
+    SideLane *lane = acquire_side_lane(caller, held);
     if (!lane) return G2D_ERR_CUDA;
     if (cudaEventRecord(lane->fork, caller) != cudaSuccess || cudaStreamWaitEvent(lane->chain, lane->fork, 0) != cudaSuccess) return G2D_ERR_CUDA;
     st = lane->chain;
