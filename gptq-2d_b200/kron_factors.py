@@ -7,6 +7,7 @@ blocked triangular inverse, normalisation by the diagonal blocks.
 from __future__ import annotations
 
 import ctypes
+import threading
 
 import torch
 
@@ -187,32 +188,36 @@ def feedback_factors_from_grams(g: torch.Tensor, h: torch.Tensor, super_entry_sh
         _raise_for_flags(flags.tolist(), ("G", "H"))
     else:
         _remember(flags, ("G", "H"))
-        if len(_PENDING) > _PENDING_LIMIT and not torch.cuda.is_current_stream_capturing():
-            _settle_oldest()
     return outs[0], outs[1].t()
 
 
 _PENDING: list[tuple[torch.Tensor, tuple[str, ...], torch.cuda.Event | None]] = []  # status flags of the calls made with check=False, oldest first
 _PENDING_LIMIT = 256
+_PENDING_LOCK = threading.Lock()  # held while entries are added or taken, never while the GPU is waited for
 _SETTLING: dict[torch.device, torch.cuda.Stream] = {}
 
 
 def _remember(flags: torch.Tensor, names: tuple[str, ...]) -> None:
-    """Keeps the flags of an unchecked call with the event of its end (a call inside a stream capture has none)."""
-    event = None
-    if not torch.cuda.is_current_stream_capturing():
-        event = torch.cuda.Event()
-        event.record(torch.cuda.current_stream(flags.device))
-    _PENDING.append((flags, names, event))
+    """Keeps the flags of an unchecked call with the event of its end (a call inside a stream capture has none).  A long
+    unchecked run settles the older half of its calls, all of which finished long ago."""
+    with torch.cuda.device(flags.device):
+        event = None
+        if not torch.cuda.is_current_stream_capturing():
+            event = torch.cuda.Event()
+            event.record()
+        oldest = []
+        with _PENDING_LOCK:
+            _PENDING.append((flags, names, event))
+            if event is not None and len(_PENDING) > _PENDING_LIMIT:
+                oldest, _PENDING[:_PENDING_LIMIT // 2] = _PENDING[:_PENDING_LIMIT // 2], []
+    _settle(oldest)
 
 
-def _settle_oldest() -> None:
-    """A long unchecked run: settle the older half of the calls, all of which finished long ago.  Their flags are read on a stream of
-    this module's own: a read on the caller's stream would wait for everything issued so far, and the host would stay
-    one call ahead of the GPU (a block of seven matrices of width 1024: 15.4 -> 12.9 ms)."""
-    batch = []
-    while len(batch) < _PENDING_LIMIT // 2 and _PENDING:
-        batch.append(_PENDING.pop(0))
+def _settle(batch: list) -> None:
+    """Waits for the given calls and raises for the first that failed; those behind it stay pending, as if only the calls up to
+    it had been settled.  Their flags are read on a stream of this module's own, behind the events of the calls: a read on
+    the current stream would not wait for calls on other streams, and would wait for everything issued so far on its own, so
+    that the host stayed one call ahead of the GPU (a block of seven matrices of width 1024: 15.4 -> 12.9 ms)."""
     values: list[list[int]] = [[] for _ in batch]
     for device in {flags.device for flags, _, _ in batch}:
         mine = [k for k, (flags, _, event) in enumerate(batch) if flags.device == device and event is not None]
@@ -231,7 +236,8 @@ def _settle_oldest() -> None:
         try:
             _raise_for_flags(flags.tolist() if event is None else values[k], names)
         except Exception:
-            _PENDING[:0] = batch[k + 1:]  # as if only the calls up to the failing one had been settled
+            with _PENDING_LOCK:
+                _PENDING[:0] = batch[k + 1:]
             raise
 
 
@@ -250,9 +256,9 @@ def last_flags() -> torch.Tensor | None:
 
 
 def check_pending() -> None:
-    """Settle every ``feedback_factors_from_grams(..., check=False)`` call made so far: wait for them and raise what
-    ``check=True`` would have raised (``torch.linalg.LinAlgError`` for a Gram that is not positive definite, as the
-    reference's ``torch.linalg.cholesky`` does; ``RuntimeError`` for a bounded wait that ran out)."""
-    while _PENDING:
-        flags, names, _ = _PENDING.pop(0)
-        _raise_for_flags(flags.tolist(), names)
+    """Settle every ``check=False`` call made so far, on whatever stream: wait for them and raise what ``check=True`` would
+    have raised (``torch.linalg.LinAlgError`` for a Gram that is not positive definite, as the reference's
+    ``torch.linalg.cholesky`` does; ``RuntimeError`` for a bounded wait that ran out)."""
+    with _PENDING_LOCK:
+        batch, _PENDING[:] = _PENDING[:], []
+    _settle(batch)

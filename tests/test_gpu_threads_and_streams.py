@@ -57,3 +57,41 @@ def test_factors_from_more_threads_than_lanes(dtype):
     for k in range(count):
         for got in results[k]:
             assert torch.equal(got, want[k])
+
+
+@pytest.mark.parametrize("single", [True, False])
+def test_pending_flags_of_another_stream(single):
+    """A matrix that is not positive definite, prepared on a stream that the current one does not wait for."""
+    import kron_factors as K
+
+    K.check_pending()
+    good = 2 * torch.eye(64, device="cuda")
+    bad = good.clone()
+    bad[7, 7] = -1
+    K.ldl_of_inverse(good)  # the library is loaded and its lanes exist
+    torch.cuda.synchronize()
+    stream = torch.cuda.Stream()
+    with torch.cuda.stream(stream):
+        heavy = torch.randn(8192, 8192, device="cuda")
+        for _ in range(10):
+            heavy = heavy @ heavy / 8192  # some ten milliseconds ahead of the factors
+        if single:
+            K.ldl_of_inverse(bad, check=False)
+        else:
+            K.feedback_factors_from_grams(good, bad)
+    with pytest.raises(torch.linalg.LinAlgError, match="pivot 8 "):
+        K.check_pending()
+    K.check_pending()
+    torch.cuda.synchronize()
+
+
+def test_unchecked_calls_do_not_pile_up():
+    import kron_factors as K
+
+    K.check_pending()
+    good = 2 * torch.eye(8, device="cuda")
+    for _ in range(3 * K._PENDING_LIMIT):
+        K.ldl_of_inverse(good, check=False)
+    assert len(K._PENDING) <= K._PENDING_LIMIT
+    K.check_pending()
+    assert not K._PENDING
