@@ -88,6 +88,8 @@ _SIGNATURES = {
     "g2d_trellis_quantize_indexed": (ctypes.c_int, [ctypes.c_int, _i64, _i32, _vp, _vp, _i32, _i32, _i32, _i32, _vp, _vp, _vp, _vp, _vp, _i32, _vp, _vp,
                                                     ctypes.c_size_t, _vp]),
     "g2d_trellis_decode": (ctypes.c_int, [ctypes.c_int, _i64, _i32, _vp, _vp, _i32, _i32, _i32, _i32, _vp, _vp, _vp, _vp]),
+    "g2d_search_status": (ctypes.c_int, [ctypes.POINTER(_i32)]),
+    "g2d_trellis_quantize_limited": (ctypes.c_int, [_i64, _i32, _vp, _vp, _i32, _i32, _i32, _vp, _vp, _vp, _vp, ctypes.c_size_t, _i64, _vp]),
     "g2d_sweep_fused_profile": (ctypes.c_int, [ctypes.POINTER(SweepDesc), _vp, ctypes.POINTER(ctypes.c_double)]),
     "g2d_launch_count": (ctypes.c_ulonglong, []),
     "g2d_stage_push": (ctypes.c_int, [ctypes.POINTER(StageDesc), _vp, _i64, _i64, _vp]),
@@ -180,7 +182,12 @@ def check_status(device: torch.device, what: str = "gptq2d_b200") -> None:
     value = int(word.item())
     if value != 0:
         word.zero_()
-        raise RuntimeError(f"{what}: a bounded wait inside a tensor-core kernel ran out (status {value}); results since the last check are not valid")
+    search = _i32()
+    with torch.cuda.device(device):
+        check(library().g2d_search_status(ctypes.byref(search)), "g2d_search_status")
+    value = value or search.value
+    if value != 0:
+        raise RuntimeError(f"{what}: a bounded wait inside a kernel ran out (status {value}); results since the last check are not valid")
 
 
 def batch_offsets(x: torch.Tensor, batch_shape: torch.Size) -> torch.Tensor | None:

@@ -493,15 +493,18 @@ __device__ __forceinline__ void async_store(uint32_t at, float a, float b, float
     asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.f32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(at), "f"(a), "f"(b), "f"(c), "f"(d), "r"(bar)
                  : "memory");
 }
-// Bounded wait (about a second) for a phase of this CTA's barrier; false when it ran out.
-__device__ __forceinline__ bool cluster_wait(uint32_t bar, uint32_t parity) {
-    const long long start = clock64();
+// Bounded wait for a phase of this CTA's barrier; false when it ran out.
+constexpr unsigned SEARCH_WAIT_CYCLES = 2000000000u;  // about a second
+constexpr unsigned SEARCH_DRAIN_CYCLES = 1 << 20;      // half a millisecond: a store to another CTA is on its way for a few hundred cycles
+__device__ __forceinline__ bool cluster_wait(uint32_t bar, uint32_t parity, unsigned limit) {
+    if (limit == 0) return false;  // a test's wait: it runs out whether the phase is complete or not
+    const unsigned start = (unsigned)clock();
     for (;;) {
         uint32_t ok;
         asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
                      : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
         if (ok) return true;
-        if (clock64() - start > 2000000000LL) return false;
+        if ((unsigned)clock() - start > limit) return false;
     }
 }
 // Two floats in one register pair: the packed additions and products round each half on its own, so a pair of states costs one
@@ -520,11 +523,19 @@ __device__ __forceinline__ uint32_t remote_load_unit(uint32_t at, int bytes) {
     return v;
 }
 
+// Set to -1 by a search whose bounded wait ran out; never cleared by a kernel (see g2d_search_status).
+__device__ int search_status;
+
+// Waits.  The four CTAs of a cluster are resident together, so a step's minima arrive unless the GPU is broken.  A wait that runs
+// out all the same ends the CTA's steps one step later, so the others run out of minima as well; every wait between two
+// cluster barriers being bounded, so are the barriers.  At the barrier that ends the pass the CTAs learn of one
+// another's failure, the first of them overwrites the rows of the cluster from this one on with what no search returns (NaN,
+// states of -1, codes of zeros) and sets the status word, and all of them stay until the stores on their way have landed.
 template <int V, int LOG_NG>
 __global__ void __launch_bounds__(CT, 1) viterbi_cluster_kernel(int64_t rows, int T, const float *__restrict__ x, const float *__restrict__ table, int shift,
                                                                 int tail_biting, const float *__restrict__ scale, float *__restrict__ out,
                                                                 int64_t *__restrict__ states, uint8_t *__restrict__ scratch, int64_t scratch_row,
-                                                                int choices_in_smem, uint8_t *__restrict__ codes, int64_t code_bytes) {
+                                                                int choices_in_smem, uint8_t *__restrict__ codes, int64_t code_bytes, unsigned wait_limit) {
     constexpr int NG = 1 << LOG_NG, NH = CSTATES / NG;
     extern __shared__ __align__(16) unsigned char g2d_vsmem[];
     const int H = 1 << shift, G = (1 << 16) >> shift, Gc = G / CCL, parts = H / NH;
@@ -541,14 +552,16 @@ __global__ void __launch_bounds__(CT, 1) viterbi_cluster_kernel(int64_t rows, in
     __shared__ int red_arg[CT / 32];
     __shared__ float all_val[CCL];
     __shared__ int all_arg[CCL];
-    __shared__ int overlap, failed;
+    __shared__ int overlap;
+    __shared__ int late;    // a wait of this CTA ran out
+    __shared__ int failed;  // a wait of one of the four CTAs did; read behind a cluster barrier
     __shared__ __align__(8) uint64_t arrived[2];  // the minima of a step have arrived in prev[0] / prev[1]
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const uint32_t rank = cluster_rank();
     const uint32_t bar0 = (uint32_t)__cvta_generic_to_shared(arrived);
     uint32_t phases = 0;  // bit b: parity of the next wait on arrived[b]
     if (tid == 0) {
-        failed = 0;
+        late = failed = 0;
         for (int b = 0; b < 2; ++b) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar0 + 8 * b) : "memory");
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -636,6 +649,9 @@ __global__ void __launch_bounds__(CT, 1) viterbi_cluster_kernel(int64_t rows, in
                     // a buffer two steps later, after it has received minima of the step between from every CTA of the
                     // cluster (each sends to all four), so it never overwrites what is still being read.
                     __syncthreads();
+                    // Whether a wait of step t - 1 ran out.  The answer is used behind this step's own wait, so that the load is on its
+                    // way meanwhile: the barrier that the next step would arm is the one whose phase is not complete.
+                    const bool stop_here = late;
                     if (part == 0) {
                         const uint32_t at_buf = to + (uint32_t)(buf * minima * (int)sizeof(float)), at_bar = to_bar + 8 * buf;
                         if constexpr (NG == 1) {
@@ -656,8 +672,9 @@ __global__ void __launch_bounds__(CT, 1) viterbi_cluster_kernel(int64_t rows, in
                         if (unit_bytes == 1) *u = (uint8_t)packed;
                         else *reinterpret_cast<uint16_t *>(u) = (uint16_t)packed;
                     }
-                    if (!failed && !cluster_wait(bar, (phases >> buf) & 1)) failed = 1;
+                    if (!cluster_wait(bar, (phases >> buf) & 1, wait_limit)) late = 1;
                     phases ^= 1u << buf;
+                    if (stop_here) break;
                 }
             }
             // ---- first arg-min over all states of the last step, with the final mask ----
@@ -678,6 +695,7 @@ __global__ void __launch_bounds__(CT, 1) viterbi_cluster_kernel(int64_t rows, in
             }
             if (lane == 0) { red_val[warp] = b; red_arg[warp] = a; }
             __syncthreads();
+            if (late && tid < CCL) remote_store(remote(&failed, tid), 1);
             if (tid == 0) {
                 for (int w = 1; w < CT / 32; ++w)
                     if (red_val[w] < b || (red_val[w] == b && red_arg[w] < a)) { b = red_val[w]; a = red_arg[w]; }
@@ -686,6 +704,7 @@ __global__ void __launch_bounds__(CT, 1) viterbi_cluster_kernel(int64_t rows, in
             }
             if (!choices_in_smem) __threadfence();  // the walk back reads other CTAs' units
             cluster_sync();
+            if (failed) break;
             // ---- walk back ----
             if (rank == 0 && warp == 0) {
                 b = all_val[0];
@@ -727,9 +746,21 @@ __global__ void __launch_bounds__(CT, 1) viterbi_cluster_kernel(int64_t rows, in
             }
             cluster_sync();
         }
-        if (failed) {  // a wait of this CTA ran out, which a healthy GPU does not do: no value of the row may pass for a result
-            for (int t = tid; t < T; t += CT) out[row * T + t] = __int_as_float(0x7fc00000);
-        } else if (rank == 0) {
+        if (failed) {
+            if (rank == 0) {
+                for (; row < rows; row += clusters) {
+                    for (int t = tid; t < T; t += CT) out[row * T + t] = __int_as_float(0x7fc00000);
+                    for (int t = tid; states && t < steps; t += CT) states[row * steps + t] = -1;
+                    for (int64_t byte = tid; codes && byte < code_bytes; byte += CT) codes[row * code_bytes + byte] = 0;
+                }
+                if (tid == 0) atomicExch(&search_status, -1);
+            }
+            for (const unsigned start = (unsigned)clock(); (unsigned)clock() - start < SEARCH_DRAIN_CYCLES;) __nanosleep(1000);
+            __syncthreads();
+            cluster_sync();
+            return;
+        }
+        if (rank == 0) {
             const float sc = scale ? scale[row] : 1.f;
             for (int t = tid; t < steps; t += CT) {
                 const int state = path[t];
@@ -758,7 +789,7 @@ __global__ void __launch_bounds__(CT, 1) viterbi_cluster_kernel(int64_t rows, in
 
 template <int V, int LOG_NG>
 static int launch_viterbi_cluster(int64_t rows, int T, const void *x, const void *table, int shift, int tail, const void *scale, void *out, int64_t *states,
-                                  void *workspace, uint8_t *codes, int64_t code_bytes, cudaStream_t st) {
+                                  void *workspace, uint8_t *codes, int64_t code_bytes, unsigned wait_limit, cudaStream_t st) {
     static PerDeviceOnce configured;
     constexpr int NG = 1 << LOG_NG, NH = CSTATES / NG, LIMIT = 200 * 1024;
     const int H = 1 << shift, G = (1 << 16) >> shift, Gc = G / CCL, parts = H / NH, steps = T / V, slots = steps > 1 ? steps - 1 : 1;
@@ -783,7 +814,7 @@ static int launch_viterbi_cluster(int64_t rows, int T, const void *x, const void
     config.numAttrs = 1;
     const int64_t scratch_row = (int64_t)slots * G;  // what the scratch holds per row; the units take no more
     if (cudaLaunchKernelEx(&config, viterbi_cluster_kernel<V, LOG_NG>, rows, T, (const float *)x, (const float *)table, shift, tail, (const float *)scale,
-                           (float *)out, states, (uint8_t *)workspace, scratch_row, in_smem, codes, code_bytes) != cudaSuccess)
+                           (float *)out, states, (uint8_t *)workspace, scratch_row, in_smem, codes, code_bytes, wait_limit) != cudaSuccess)
         return G2D_ERR_CUDA;
     return check_launch();
 }
@@ -795,12 +826,12 @@ static bool cluster_search_serves(int dtype, int T, int L, int shift, int V) {
 }
 template <int V>
 static int cluster_search(int64_t rows, int T, const void *x, const void *table, int shift, int tail, const void *scale, void *out, int64_t *states,
-                          void *workspace, uint8_t *codes, int64_t code_bytes, cudaStream_t st) {
+                          void *workspace, uint8_t *codes, int64_t code_bytes, unsigned wait_limit, cudaStream_t st) {
     switch (shift) {
-    case 2: return launch_viterbi_cluster<V, 3>(rows, T, x, table, shift, tail, scale, out, states, workspace, codes, code_bytes, st);
-    case 3: return launch_viterbi_cluster<V, 2>(rows, T, x, table, shift, tail, scale, out, states, workspace, codes, code_bytes, st);
-    case 4: return launch_viterbi_cluster<V, 1>(rows, T, x, table, shift, tail, scale, out, states, workspace, codes, code_bytes, st);
-    default: return launch_viterbi_cluster<V, 0>(rows, T, x, table, shift, tail, scale, out, states, workspace, codes, code_bytes, st);
+    case 2: return launch_viterbi_cluster<V, 3>(rows, T, x, table, shift, tail, scale, out, states, workspace, codes, code_bytes, wait_limit, st);
+    case 3: return launch_viterbi_cluster<V, 2>(rows, T, x, table, shift, tail, scale, out, states, workspace, codes, code_bytes, wait_limit, st);
+    case 4: return launch_viterbi_cluster<V, 1>(rows, T, x, table, shift, tail, scale, out, states, workspace, codes, code_bytes, wait_limit, st);
+    default: return launch_viterbi_cluster<V, 0>(rows, T, x, table, shift, tail, scale, out, states, workspace, codes, code_bytes, wait_limit, st);
     }
 }
 
@@ -910,8 +941,8 @@ int launch_trellis(int dtype, int64_t rows, int T, const void *x, const void *ta
                    void *out, int64_t *states, void *workspace, uint8_t *codes, cudaStream_t st, const TrellisIndex *index) {
     const int64_t code_bytes = trellis_code_bytes(T, L, K, V, tail);
     if (cluster_search_serves(dtype, T, L, K * V, V)) {
-        if (V == 2) return cluster_search<2>(rows, T, x, table, K * V, tail, scale, out, states, workspace, codes, code_bytes, st);
-        return cluster_search<1>(rows, T, x, table, K * V, tail, scale, out, states, workspace, codes, code_bytes, st);
+        if (V == 2) return cluster_search<2>(rows, T, x, table, K * V, tail, scale, out, states, workspace, codes, code_bytes, SEARCH_WAIT_CYCLES, st);
+        return cluster_search<1>(rows, T, x, table, K * V, tail, scale, out, states, workspace, codes, code_bytes, SEARCH_WAIT_CYCLES, st);
     }
     const int R = dtype == G2D_F32 ? indexed_sequences_per_cta<float>(index, rows, L, K, V) : indexed_sequences_per_cta<double>(index, rows, L, K, V);
     if (R == 1 && dtype == G2D_F32) return launch_viterbi_indexed<float, 1>(rows, T, x, table, *index, L, K, V, tail, scale, out, states, workspace, codes, code_bytes, st);
@@ -981,6 +1012,29 @@ extern "C" int g2d_trellis_quantize_indexed(int dtype, int64_t rows, int32_t T, 
     if (!workspace || workspace_bytes < trellis_scratch_bytes(dtype, rows, T, L, K, V)) return G2D_ERR_WORKSPACE;
     const TrellisIndex index{distinct, ids, distinct_count};
     return launch_trellis(dtype, rows, T, x, table, L, K, V, tail_biting, scale, out, states, workspace, codes, (cudaStream_t)stream, &index);
+}
+
+extern "C" int g2d_trellis_quantize_limited(int64_t rows, int32_t T, const void *x, const void *table, int32_t K, int32_t V, int32_t tail_biting,
+                                            void *out, int64_t *states, uint8_t *codes, void *workspace, size_t workspace_bytes, int64_t wait_cycles,
+                                            void *stream) {
+    const int status = trellis_check(G2D_F32, rows, T, 16, K, V);
+    if (status != G2D_OK) return status;
+    if (rows == 0) return G2D_OK;
+    if (!x || !table || !out || wait_cycles < 0 || wait_cycles > SEARCH_WAIT_CYCLES) return G2D_ERR_BAD_ARGUMENT;
+    if (!workspace || workspace_bytes < trellis_scratch_bytes(G2D_F32, rows, T, 16, K, V)) return G2D_ERR_WORKSPACE;
+    if (!cluster_search_serves(G2D_F32, T, 16, K * V, V)) return G2D_ERR_UNSUPPORTED;
+    const int64_t code_bytes = trellis_code_bytes(T, 16, K, V, tail_biting);
+    const auto search = V == 2 ? cluster_search<2> : cluster_search<1>;
+    return search(rows, T, x, table, K * V, tail_biting, nullptr, out, states, workspace, codes, code_bytes, (unsigned)wait_cycles, (cudaStream_t)stream);
+}
+
+extern "C" int g2d_search_status(int32_t *status) {
+    if (!status) return G2D_ERR_BAD_ARGUMENT;
+    *status = 0;
+    if (cudaDeviceSynchronize() != cudaSuccess || cudaMemcpyFromSymbol(status, search_status, sizeof(int)) != cudaSuccess) return G2D_ERR_CUDA;
+    const int none = 0;
+    if (*status != 0 && cudaMemcpyToSymbol(search_status, &none, sizeof(int)) != cudaSuccess) return G2D_ERR_CUDA;
+    return G2D_OK;
 }
 
 extern "C" int g2d_trellis_decode(int dtype, int64_t rows, int32_t T, const uint8_t *codes, const void *table, int32_t L, int32_t K,

@@ -250,6 +250,18 @@ int g2d_trellis_quantize_indexed(int dtype, int64_t rows, int32_t T, const void 
                                  const void *distinct, int32_t distinct_count, const uint16_t *ids, void *workspace,
                                  size_t workspace_bytes, void *stream);
 
+/* The trellis searches make bounded waits of about a second between CTAs that share a sequence.  One that runs out, which a
+ * healthy GPU does not do, leaves NaN in the values, -1 in the states and zeros in the stored paths of the sequences
+ * concerned and sets a word of the device's.  This call waits for the current device, returns that word (0, or -1: some
+ * search since the last call of this function has no result) and clears it. */
+int g2d_search_status(int32_t *status);
+
+/* The search of g2d_trellis_quantize for 2^16 states in float32 (K V from 2 to 8, T from 2 V to 8192; others are
+ * G2D_ERR_UNSUPPORTED), without a scale, under a wait limit of the caller's: a limit of 0 lets a test see a wait that ran out. */
+int g2d_trellis_quantize_limited(int64_t rows, int32_t T, const void *x, const void *table, int32_t K, int32_t V,
+                                 int32_t tail_biting, void *out, int64_t *states, uint8_t *codes, void *workspace,
+                                 size_t workspace_bytes, int64_t wait_cycles, void *stream);
+
 /* Unit (block) lower triangular factor of the inverse of a symmetric positive definite matrix:
  * a^{-1} = out Lambda out^T with size x size identity diagonal blocks.  a is [n, n] and is overwritten
  * (scratch); workspace: g2d_ldl_workspace_bytes().  status_flag (device int32, may be NULL) receives the
