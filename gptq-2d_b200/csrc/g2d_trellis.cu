@@ -798,20 +798,29 @@ static int launch_viterbi_cluster(int64_t rows, int T, const void *x, const void
     const int in_smem = base + kept <= LIMIT;
     const size_t smem = base + (in_smem ? kept : 0);
     if (smem > LIMIT) return G2D_ERR_UNSUPPORTED;
-    if (configured.run([&] { return cudaFuncSetAttribute(viterbi_cluster_kernel<V, LOG_NG>, cudaFuncAttributeMaxDynamicSharedMemorySize, LIMIT) == cudaSuccess; }) != G2D_OK)
-        return G2D_ERR_CUDA;
-    const int64_t clusters = rows < 148 / CCL ? rows : 148 / CCL;
     cudaLaunchConfig_t config{};
-    config.gridDim = dim3((unsigned)(clusters * CCL));
+    config.gridDim = dim3(CCL);
     config.blockDim = dim3(CT);
-    config.dynamicSmemBytes = smem;
-    config.stream = st;
+    config.dynamicSmemBytes = LIMIT;
     cudaLaunchAttribute attribute{};
     attribute.id = cudaLaunchAttributeClusterDimension;
     attribute.val.clusterDim.x = CCL;
     attribute.val.clusterDim.y = attribute.val.clusterDim.z = 1;
     config.attrs = &attribute;
     config.numAttrs = 1;
+    // Clusters that are resident together: fewer than SMs / 4, since a cluster lies within one of the GPU's partitions.  A grid of
+    // more would deal sequences out to clusters that start when the others are done (148 sequences: 2.26 ms against 1.5).
+    static int resident[64];
+    int device = 0;
+    if (cudaGetDevice(&device) != cudaSuccess || configured.run([&] {
+            return cudaFuncSetAttribute(viterbi_cluster_kernel<V, LOG_NG>, cudaFuncAttributeMaxDynamicSharedMemorySize, LIMIT) == cudaSuccess &&
+                   cudaOccupancyMaxActiveClusters(&resident[device], viterbi_cluster_kernel<V, LOG_NG>, &config) == cudaSuccess && resident[device] > 0;
+        }) != G2D_OK)
+        return G2D_ERR_CUDA;
+    const int64_t clusters = rows < resident[device] ? rows : resident[device];
+    config.gridDim = dim3((unsigned)(clusters * CCL));
+    config.dynamicSmemBytes = smem;
+    config.stream = st;
     const int64_t scratch_row = (int64_t)slots * G;  // what the scratch holds per row; the units take no more
     if (cudaLaunchKernelEx(&config, viterbi_cluster_kernel<V, LOG_NG>, rows, T, (const float *)x, (const float *)table, shift, tail, (const float *)scale,
                            (float *)out, states, (uint8_t *)workspace, scratch_row, in_smem, codes, code_bytes, wait_limit) != cudaSuccess)
@@ -819,10 +828,21 @@ static int launch_viterbi_cluster(int64_t rows, int T, const void *x, const void
     return check_launch();
 }
 
-// Float searches over 2^16 states with 4 to 256 predecessors per state, the path short enough for shared memory; the others
-// go to the kernels above.
-static bool cluster_search_serves(int dtype, int T, int L, int shift, int V) {
-    return dtype == G2D_F32 && L == 16 && shift >= 2 && T >= 2 * V && T <= 8192;
+// Float searches over 2^16 states with 4 to 256 predecessors per state, the path short enough for shared memory, choices that may
+// be stored two bytes at a time; the others go to the kernels above.
+static bool cluster_search_serves(int dtype, int T, int L, int shift, int V, const void *workspace) {
+    return dtype == G2D_F32 && L == 16 && shift >= 2 && T >= 2 * V && T <= 8192 && ((uintptr_t)workspace & 1) == 0;
+}
+// Whether the cluster search is the faster one.  It takes 33 to 36 sequences at a time, each in a quarter of the time of the kernels
+// above or less; those take 148, 296 (two per SM) or 592 (four) at a time.  Up to 148 sequences the cluster search wins throughout;
+// beyond, `pair` and `four` are the rounds of it that take as long as one round of 296 and of 592 sequences.  Measured, in
+// us at T = 64, cluster search and the other: V = 2, 4 bits per step: 296 sequences 695 / 695, 592: 1355 / 1166, 593: 1356 / 2269,
+// 1184: 2663 / 2292; V = 1, 2 bits: 592: 4253 / 7895; V = 1, 8 bits: 148: 1831 / 2156, 224: 2545 / 2531, 592: 6474 / 3310.
+static bool cluster_search_pays(int64_t rows, int shift, int V) {
+    static const int pair[2][9] = {{0, 0, 16, 13, 14, 12, 11, 7, 7}, {0, 0, 15, 0, 9, 0, 11, 0, 7}};
+    static const int four[2][9] = {{0, 0, 33, 27, 19, 16, 14, 10, 9}, {0, 0, 30, 0, 15, 0, 15, 0, 9}};
+    const int64_t rounds = ceil_div(rows, (int64_t)33);
+    return rows <= 148 || rounds <= (rows <= 296 ? pair[V - 1][shift] : four[V - 1][shift] * ceil_div(rows, (int64_t)592));
 }
 template <int V>
 static int cluster_search(int64_t rows, int T, const void *x, const void *table, int shift, int tail, const void *scale, void *out, int64_t *states,
@@ -940,7 +960,7 @@ static int indexed_sequences_per_cta(const TrellisIndex *index, int64_t rows, in
 int launch_trellis(int dtype, int64_t rows, int T, const void *x, const void *table, int L, int K, int V, int tail, const void *scale,
                    void *out, int64_t *states, void *workspace, uint8_t *codes, cudaStream_t st, const TrellisIndex *index) {
     const int64_t code_bytes = trellis_code_bytes(T, L, K, V, tail);
-    if (cluster_search_serves(dtype, T, L, K * V, V)) {
+    if (cluster_search_serves(dtype, T, L, K * V, V, workspace) && cluster_search_pays(rows, K * V, V)) {
         if (V == 2) return cluster_search<2>(rows, T, x, table, K * V, tail, scale, out, states, workspace, codes, code_bytes, SEARCH_WAIT_CYCLES, st);
         return cluster_search<1>(rows, T, x, table, K * V, tail, scale, out, states, workspace, codes, code_bytes, SEARCH_WAIT_CYCLES, st);
     }
@@ -1022,7 +1042,7 @@ extern "C" int g2d_trellis_quantize_limited(int64_t rows, int32_t T, const void 
     if (rows == 0) return G2D_OK;
     if (!x || !table || !out || wait_cycles < 0 || wait_cycles > SEARCH_WAIT_CYCLES) return G2D_ERR_BAD_ARGUMENT;
     if (!workspace || workspace_bytes < trellis_scratch_bytes(G2D_F32, rows, T, 16, K, V)) return G2D_ERR_WORKSPACE;
-    if (!cluster_search_serves(G2D_F32, T, 16, K * V, V)) return G2D_ERR_UNSUPPORTED;
+    if (!cluster_search_serves(G2D_F32, T, 16, K * V, V, workspace)) return G2D_ERR_UNSUPPORTED;
     const int64_t code_bytes = trellis_code_bytes(T, 16, K, V, tail_biting);
     const auto search = V == 2 ? cluster_search<2> : cluster_search<1>;
     return search(rows, T, x, table, K * V, tail_biting, nullptr, out, states, workspace, codes, code_bytes, (unsigned)wait_cycles, (cudaStream_t)stream);

@@ -216,7 +216,7 @@ def _sweep_super(y, l, u, batch_shape, options: dict, quantizer_inputs, super_en
             offsets = torch.arange(per_batch.numel(), dtype=torch.int64, device=y.device)
         import quantizer_trellis
 
-        table, index = quantizer_trellis.prepared_table(options["table"], y, options["K"])
+        table, index = quantizer_trellis.prepared_table(options["table"], y)
         keep += [per_batch, table, offsets, index]
         if index is not None:
             desc.table_distinct, desc.table_ids, desc.table_distinct_count = index[0].data_ptr(), index[1].data_ptr(), index[0].size(0)

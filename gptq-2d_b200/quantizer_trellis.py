@@ -77,21 +77,18 @@ _TABLE_INDEX: dict = {}
 _INDEX_LIMIT = 2048  # distinct rows whose local costs fit shared memory beside the search's own buffers
 
 
-def prepared_table(table: torch.Tensor, like: torch.Tensor, K: int) -> tuple[torch.Tensor, tuple[torch.Tensor, torch.Tensor] | None]:
+def prepared_table(table: torch.Tensor, like: torch.Tensor) -> tuple[torch.Tensor, tuple[torch.Tensor, torch.Tensor] | None]:
     """The table in ``like``'s dtype and device, contiguous, and its index ``(distinct [D, V], ids int16 [2^L])`` when it has at
     most 2048 distinct rows and at most 2^16 states (else None).  The shipped codes have about a thousand distinct rows
-    (``hyb``: 2^9 lookup rows times a sign), and the search is much faster when it knows them, except for float32 over 2^16
-    states at two or more bits per step, where it keeps the table's values in registers and gets no index.  Both are
-    remembered per table (keyed by its storage and version), so a sweep that calls the quantizer a thousand times
-    prepares them once."""
-    in_registers = like.dtype == torch.float32 and table.size(0) == 1 << 16 and K * table.size(1) >= 2
-    key = (table.data_ptr(), table._version, tuple(table.shape), table.dtype, table.device, like.dtype, like.device, in_registers)
+    (``hyb``: 2^9 lookup rows times a sign), and most searches are much faster when they know them.  Both are remembered per
+    table (keyed by its storage and version), so a sweep that calls the quantizer a thousand times prepares them once."""
+    key = (table.data_ptr(), table._version, tuple(table.shape), table.dtype, table.device, like.dtype, like.device)
     if key not in _TABLE_INDEX:
         if len(_TABLE_INDEX) > 16:
             _TABLE_INDEX.clear()
         converted = table.to(like).contiguous()
         index = None
-        if converted.is_cuda and 64 <= converted.size(0) <= 1 << 16 and not in_registers:
+        if converted.is_cuda and 64 <= converted.size(0) <= 1 << 16:
             distinct, inverse = torch.unique(converted, dim=0, return_inverse=True)
             if distinct.size(0) <= _INDEX_LIMIT:
                 index = (distinct.contiguous(), inverse.to(torch.int16).contiguous())
@@ -121,7 +118,7 @@ def _trellis_quantize_cuda(
     L = num_states.bit_length() - 1
     assert out.is_contiguous() and out.numel() == rows * T and out.dtype == x.dtype, "out must be contiguous [..., T] in x's dtype"
     scale = scale.to(x.dtype).broadcast_to(out.shape[:-1]).reshape(rows).contiguous()
-    table, index = prepared_table(table, x, K)
+    table, index = prepared_table(table, x)
     if states is not None:
         assert states.is_contiguous() and states.dtype == torch.int64 and states.numel() == rows * (T // V)
     lib = _abi.library()

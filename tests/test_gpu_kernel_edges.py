@@ -3,6 +3,7 @@
 Bounds are worst-case rounding bounds: a sum of k products is off by at most (k + 2) u of the sum of their magnitudes
 (u = 2^-24 for float32, 2^-53 for float64), whatever the order of its additions.
 """
+import ctypes
 import functools
 
 import numpy as np
@@ -184,3 +185,24 @@ def test_pack_out_of_the_fast_range(oracle, bits):
         assert np.array_equal(packed.cpu().numpy(), oracle.pack_codes(z, scale, zero, qmin, bits))
         back = P.unpack_codes(packed, cuda(scale), cuda(zero), qmin=qmin, bits=bits, n=n)
         assert np.array_equal(back.cpu().numpy(), oracle.unpack_codes(packed.cpu().numpy(), scale, zero, qmin, bits, n))
+
+
+# both sides of each line at which a search over 2^16 states changes kernels: 148 sequences, 296, 592, and those between where the
+# cluster search stops being the faster one; and choices that may only be stored byte by byte
+@pytest.mark.parametrize("rows, K, V, offset", [(148, 8, 1, 0), (149, 8, 1, 0), (231, 8, 1, 0), (232, 8, 1, 0), (297, 4, 2, 0), (298, 4, 2, 0), (495, 2, 2, 0),
+                                                (496, 2, 2, 0), (593, 2, 2, 0), (5, 2, 2, 1)])
+def test_searches_on_both_sides_of_the_dispatch(oracle, rows, K, V, offset):
+    import _abi
+
+    T = 8 * V
+    rng = np.random.default_rng(rows + K)
+    table = rng.standard_normal((1 << 16, V)).astype(np.float32)
+    x = rng.standard_normal((rows, T)).astype(np.float32)
+    values, path = oracle.trellis_quantize(x, table, K, True)
+    out, states = torch.empty(rows, T, device="cuda"), torch.empty(rows, T // V, dtype=torch.int64, device="cuda")
+    size = ctypes.c_size_t()
+    _abi.check(_abi.library().g2d_trellis_workspace_bytes(_abi.F32, rows, T, 16, K, V, ctypes.byref(size)), "g2d_trellis_workspace_bytes")
+    workspace, xs, ts = torch.empty(size.value + 16, dtype=torch.uint8, device="cuda"), cuda(x), cuda(table)
+    _abi.check(_abi.library().g2d_trellis_quantize(_abi.F32, rows, T, xs.data_ptr(), ts.data_ptr(), 16, K, V, 1, None, out.data_ptr(), states.data_ptr(),
+                                                   workspace.data_ptr() + offset, size.value, _abi.stream_of(xs)), "g2d_trellis_quantize")
+    assert torch.equal(states.cpu(), torch.from_numpy(path)) and torch.equal(out.cpu(), torch.from_numpy(values))
