@@ -177,8 +177,44 @@ constexpr int PTH = 256;       // threads of a CTA of the pull kernel
 constexpr int PULL_ROOM = 2048;  // (source stage, entry) pairs whose sums wait in shared memory
 constexpr int Q_PULL_ONLY = -1;  // KIND: only bring Y and C up to date
 
-// One CTA per super-entry of the stage: first what the earlier stages of the inner block owe it, then its quantizer, then its
-// error, completed C and rounded values.  One launch per stage where the sources used to push (error, push and quantizer
+// Loads that stay where they are written: the compiler moved plain ones down to their uses in some of the kernels below (512 x 512
+// as 16 x 16 under the round quantizer: 1349 us against 940).
+__device__ __forceinline__ float load_here(const float *p) {
+    float v;
+    asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ double load_here(const double *p) {
+    double v;
+    asm volatile("ld.global.f64 %0, [%1];" : "=d"(v) : "l"(p) : "memory");
+    return v;
+}
+template <int BATCH, typename F>
+__device__ __forceinline__ void dot_batches(F &sum, int &x, const F *a, const F *b, int64_t ld, int count) {
+    for (; x + BATCH <= count; x += BATCH) {
+        F av[BATCH], bv[BATCH];
+#pragma unroll
+        for (int e = 0; e < BATCH; ++e) {
+            av[e] = load_here(a + x + e);
+            bv[e] = load_here(b + (x + e) * ld);
+        }
+#pragma unroll
+        for (int e = 0; e < BATCH; ++e) sum += av[e] * bv[e];
+    }
+}
+// sum over x of a[x] b[x ld], ascending; the loads of eight terms travel together (double: of sixteen, whose sums take longer)
+template <typename F>
+__device__ __forceinline__ F dot(const F *a, const F *b, int64_t ld, int count) {
+    F sum = (F)0;
+    int x = 0;
+    if (sizeof(F) == sizeof(double)) dot_batches<16>(sum, x, a, b, ld, count);
+    dot_batches<8>(sum, x, a, b, ld, count);
+    for (; x < count; ++x) sum += a[x] * b[x * ld];
+    return sum;
+}
+
+// Sweeps whose blocks are short enough (see pull_pays).  One CTA per super-entry of the stage: first what the earlier stages of the
+// inner block owe it, then its quantizer, then its error, completed C and rounded values.  One launch per stage where the sources used to push (error, push and quantizer
 // kernels, 3 launches), because a super-entry that fetches its own feedback when its turn comes needs no launch for it.
 // Bound by launch latency and the chain of one stage: the sums of all source stages are formed side by side, each in the
 // order and from the start that the push had, and added in the order of the stages, so the values are bit for bit the same.
@@ -203,24 +239,17 @@ __global__ void __launch_bounds__(PTH) stage_pull_kernel(SuperArgs<F> A) {
             const int64_t i = i0 + a, j = j0 + b;
             down = right = (F)0;
             if (ib - dd >= 0) {
-                const F *lp = lg + i * m + (ib - dd) * p, *ep = eg + (ib - dd) * p * n + j;
-#pragma unroll 4
-                for (int x = 0; x < p; ++x) down += lp[x] * ep[x * n];
+                down = dot(lg + i * m + (ib - dd) * p, eg + (ib - dd) * p * n + j, n, p);
             }
             if (jb - dd >= 0) {
-                const F *cp = cg + i * n + (jb - dd) * q, *up = ug + (jb - dd) * q * n + j;
-#pragma unroll 8
-                for (int x = 0; x < q; ++x) right += cp[x] * up[x * n];
+                right = dot(cg + i * n + (jb - dd) * q, ug + (jb - dd) * q * n + j, n, q);
             }
         };
-        const bool staged = (int64_t)pulls * pq <= PULL_ROOM;
-        if (staged) {
-            for (int t = tid; t < pulls * pq; t += PTH) {
-                const int at = t % pq;
-                sums(pulls - t / pq, at / q, at % q, down_s[t], right_s[t]);
-            }
-            __syncthreads();
+        for (int t = tid; t < pulls * pq; t += PTH) {  // at most PULL_ROOM (see pull_pays)
+            const int at = t % pq;
+            sums(pulls - t / pq, at / q, at % q, down_s[t], right_s[t]);
         }
+        __syncthreads();
         // a warp per row of the super-entry
         for (int a = warp; a < p; a += PTH / 32) {
             constexpr int KEEP = 4;  // values of a row that stay in a lane's registers
@@ -231,13 +260,7 @@ __global__ void __launch_bounds__(PTH) stage_pull_kernel(SuperArgs<F> A) {
                 c = cg[at];
                 for (int x = 0; x < pulls; ++x) {
                     const int dd = pulls - x;
-                    F down, right;
-                    if (staged) {
-                        down = down_s[x * pq + a * q + b];
-                        right = right_s[x * pq + a * q + b];
-                    } else {
-                        sums(dd, a, b, down, right);
-                    }
+                    const F down = down_s[x * pq + a * q + b], right = right_s[x * pq + a * q + b];
                     if (ib - dd >= 0) c += down;
                     if (ib - dd >= 0 || jb - dd >= 0) y += down + right;
                 }
@@ -276,14 +299,14 @@ __global__ void __launch_bounds__(PTH) stage_pull_kernel(SuperArgs<F> A) {
                 s = A.scale[A.scale_off ? A.scale_off[batch] : 0];
                 if (a == 0 && lane == 0) A.row_scale[seq] = s;
             }
-            if (KIND == G2D_Q_ABSMAX_DYNAMIC && q <= 32 * KEEP) {
+            if (q <= 32 * KEEP) {
 #pragma unroll
                 for (int x = 0; x < KEEP; ++x)
                     if (lane + 32 * x < q) {
                         update(lane + 32 * x, yv[x], cv[x]);
                         top = fmax(top, fabs(yv[x]));
                     }
-                s = absmax_scale_value(warp_max(top), A.divisor, A.half);
+                if (KIND == G2D_Q_ABSMAX_DYNAMIC) s = absmax_scale_value(warp_max(top), A.divisor, A.half);
 #pragma unroll
                 for (int x = 0; x < KEEP; ++x)
                     if (lane + 32 * x < q) finish(lane + 32 * x, yv[x], cv[x], s);
@@ -311,6 +334,17 @@ __global__ void __launch_bounds__(PTH) stage_pull_kernel(SuperArgs<F> A) {
         }
         __syncthreads();  // the next batch reuses the staged sums
     }
+}
+
+// Whether a sweep pulls.  A CTA forms stages p q sums of p + q products with 256 threads, where a push spreads them over the whole
+// GPU: from about 600 products per thread on, the push is the faster one, and beyond PULL_ROOM sums there is no room for
+// them.  Measured, push and pull in us: 256 x 1024 as 1 x 32, blocks of 64 stages (264 products per thread) 4437 / 3151;
+// 64 x 2048 as 1 x 128, 8 stages (516) 2265 / 2053, 16 stages (1032) 2028 / 2716; 512 x 512 as 32 x 32, 2 stages (512) 866 / 764;
+// 512 x 1024 as 4 x 128, 4 stages (1056) 3835 / 4005; 2048 x 64 as 512 x 1, 1 stage (1026) 5925 / 8467.  With leading modes a pull
+// is a launch of its own, which blocks of one or two stages do not repay (8 x 64 x 128 as 1 x 2, one stage: 4149 / 4429).
+bool pull_pays(int64_t stages, int p, int q, bool leading) {
+    const double sums = (double)stages * p * q;
+    return sums <= PULL_ROOM && sums * (p + q) <= 600.0 * PTH && (!leading || stages > 2);
 }
 
 template <typename F, int KIND>
@@ -474,6 +508,7 @@ int sweep_super(const g2d_super_desc *d, const Plan &plan, cudaStream_t st) {
     const int64_t inner = d->inner_block > 0 && d->inner_block <= stages ? d->inner_block : stages;
     const int64_t outer = d->outer_block > inner && d->outer_block < stages ? d->outer_block : inner;
     const int T = d->p * d->q;
+    const bool pull = pull_pays(inner, d->p, d->q, d->lead_count > 0);
     for (int64_t outer_start = 0; outer_start < stages; outer_start += outer) {
         const int64_t outer_stop = outer_start + outer < stages ? outer_start + outer : stages;
         for (int64_t s0 = outer_start; s0 < outer_stop; s0 += inner) {
@@ -484,7 +519,7 @@ int sweep_super(const g2d_super_desc *d, const Plan &plan, cudaStream_t st) {
                 if (dmax == 0) continue;
                 A.stage = s; A.dmax = dmax; A.s0 = s0;
                 const int64_t work = d->batch * dmax * pq;
-                if (d->lead_count == 0) {
+                if (pull && d->lead_count == 0) {
                     int status;
                     switch (d->quant_kind) {
                     case G2D_Q_ROUND: status = launch_stage_pull<F, G2D_Q_ROUND>(A, st); break;
@@ -496,10 +531,14 @@ int sweep_super(const g2d_super_desc *d, const Plan &plan, cudaStream_t st) {
                     if (d->quant_kind != G2D_Q_TRELLIS) continue;
                 } else {
                     // the leading modes' feedback comes between the pending pushes and the quantizer
-                    const int status = launch_stage_pull<F, Q_PULL_ONLY>(A, st);
-                    if (status != G2D_OK) return status;
-                    fold_kernel<F><<<blocks_for(work, 128), 128, 0, st>>>(A);
-                    if (check_launch() != G2D_OK) return G2D_ERR_CUDA;
+                    if (pull) {
+                        const int status = launch_stage_pull<F, Q_PULL_ONLY>(A, st);
+                        if (status != G2D_OK) return status;
+                    }
+                    if (d->lead_count > 0) {
+                        fold_kernel<F><<<blocks_for(work, 128), 128, 0, st>>>(A);
+                        if (check_launch() != G2D_OK) return G2D_ERR_CUDA;
+                    }
                     switch (d->quant_kind) {
                     case G2D_Q_ROUND: quantize_entries_kernel<F, G2D_Q_ROUND><<<blocks_for(work, 128), 128, 0, st>>>(A); break;
                     case G2D_Q_AFFINE: quantize_entries_kernel<F, G2D_Q_AFFINE><<<blocks_for(work, 128), 128, 0, st>>>(A); break;
@@ -524,7 +563,7 @@ int sweep_super(const g2d_super_desc *d, const Plan &plan, cudaStream_t st) {
                     fold_commit_kernel<F><<<blocks_for(work, 128), 128, 0, st>>>(A);
                     if (check_launch() != G2D_OK) return G2D_ERR_CUDA;
                 }
-                const int status = launch_stage_commit<F>(sd, z, s, st, skew, dmax * pq);
+                const int status = pull ? launch_stage_commit<F>(sd, z, s, st, skew, dmax * pq) : launch_stage_push<F>(sd, z, s, s1, st, skew, dmax * pq);
                 if (status != G2D_OK) return status;
             }
             if (s1 < outer_stop) {

@@ -206,3 +206,39 @@ def test_searches_on_both_sides_of_the_dispatch(oracle, rows, K, V, offset):
     _abi.check(_abi.library().g2d_trellis_quantize(_abi.F32, rows, T, xs.data_ptr(), ts.data_ptr(), 16, K, V, 1, None, out.data_ptr(), states.data_ptr(),
                                                    workspace.data_ptr() + offset, size.value, _abi.stream_of(xs)), "g2d_trellis_quantize")
     assert torch.equal(states.cpu(), torch.from_numpy(path)) and torch.equal(out.cpu(), torch.from_numpy(values))
+
+
+# sums per stage on both sides of the shared-memory room (2048) and of the work (600 products per thread) up to which a super-entry
+# fetches its feedback itself; a single block (0); leading modes with short blocks
+@pytest.mark.parametrize("m, n, p, q, inner, outer", [(40, 96, 1, 16, 128, 0), (40, 96, 1, 16, 129, 0), (96, 96, 16, 16, 8, 64), (96, 96, 16, 16, 9, 64), (96, 96, 32, 32, 2, 0),
+                                                      (128, 128, 64, 64, 8, 64), (12, 1024, 1, 128, 9, 64), (12, 1024, 1, 128, 10, 64), (60, 120, 2, 4, 0, 0)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
+def test_blocks_on_both_sides_of_the_pull(m, n, p, q, inner, outer, dtype):
+    """The two ways to bring feedback to a stage add the same sums in the same order: the fused sweep equals the engine that calls the
+    quantizer once per stage, bit for bit."""
+    import gptq_2d as G
+    import quantizer_int as Q
+
+    gen = torch.Generator(device="cuda").manual_seed(m + n + inner)
+    rand = lambda *shape: torch.randn(*shape, generator=gen, device="cuda", dtype=dtype)
+    w, l, u = 0.02 * rand(m, n), torch.tril(rand(m, m) * (0.3 / m ** .5), -1), torch.triu(rand(n, n) * (0.3 / n ** .5), 1)
+    quantizer = functools.partial(Q.int_abs_max_quantizer_cuda, qmin=-8, qmax=7, dtype=torch.float16)
+    options = dict(super_entry_shape=(p, q), inner_block_size=inner, outer_block_size=outer)
+    fused = G.gptq_2d_super_entry(w, l, u, quantizer=quantizer, **options)
+    generic = G.gptq_2d_super_entry(w, l, u, quantizer=lambda *a, **k: quantizer(*a, **k), **options)
+    assert torch.equal(fused, generic)
+
+
+@pytest.mark.parametrize("inner", [1, 2, 3, 0])
+def test_leading_modes_on_both_sides_of_the_pull(inner):
+    import kron_factors as K
+
+    gen = torch.Generator(device="cuda").manual_seed(inner)
+    x = 3 * torch.randn(3, 12, 16, generator=gen, device="cuda", dtype=torch.float64)
+    factors = []
+    for k, block in zip(x.shape, (1, 2, 2)):  # identity diagonal blocks, which the two routes share
+        index = torch.arange(k, device="cuda") // block
+        f = 0.2 * torch.randn(k, k, generator=gen, device="cuda", dtype=torch.float64)
+        factors.append(f.masked_fill(index[:, None] <= index[None, :], 0) + torch.eye(k, device="cuda", dtype=torch.float64))
+    want = K.gptq_d_sided(x, factors, super_entry_shape=(2, 2), dense_row_factor=True)
+    assert torch.equal(K.gptq_d_sided(x, factors, super_entry_shape=(2, 2), inner_block_size=inner, outer_block_size=0), want)
