@@ -250,13 +250,18 @@ bool build_lane(PipeLane &l) {
     return ok;
 }
 
-// Returns a lane of the current device with its lock held (through `held`), or null with *status set.
-PipeLane *acquire_pipe_lane(cudaStream_t caller, std::unique_lock<std::mutex> &held, int *status) {
+DeviceLanes *device_lanes() {  // of the current device
     static DeviceLanes devices[64];
     int device = 0;
+    return cudaGetDevice(&device) == cudaSuccess && device >= 0 && device < 64 ? &devices[device] : nullptr;
+}
+
+// Returns a lane of the current device with its lock held (through `held`), or null with *status set.
+PipeLane *acquire_pipe_lane(cudaStream_t caller, std::unique_lock<std::mutex> &held, int *status) {
     *status = G2D_ERR_CUDA;
-    if (cudaGetDevice(&device) != cudaSuccess || device < 0 || device >= 64) return nullptr;
-    DeviceLanes &dl = devices[device];
+    DeviceLanes *lanes = device_lanes();
+    if (!lanes) return nullptr;
+    DeviceLanes &dl = *lanes;
     int slot;
     {
         std::lock_guard<std::mutex> lock(dl.build);
@@ -280,6 +285,20 @@ PipeLane *acquire_pipe_lane(cudaStream_t caller, std::unique_lock<std::mutex> &h
     held = std::unique_lock<std::mutex>(dl.lane[slot].busy);
     *status = G2D_OK;
     return &dl.lane[slot];
+}
+
+// Whether a sweep that tc_eligible admits runs on the tensor-core schedules.  Two kinds of calls with a side that is no multiple of 4
+// keep to the tile schedule, which takes them as they are: those inside a stream capture on a device without lanes (see
+// acquire_pipe_lane; they need no warm-up call), and those whose Y, used where it lies, starts off a 16-byte boundary.
+bool takes_tensor_cores(const g2d_sweep_desc *d, cudaStream_t stream) {
+    if (!tc_eligible(d)) return false;
+    if (d->m % 4 == 0 && d->n % 4 == 0) return true;
+    if (d->n % 4 == 0 && ((uintptr_t)d->y & 15) != 0) return false;
+    DeviceLanes *lanes = device_lanes();
+    if (!lanes) return true;  // the launch reports it
+    std::lock_guard<std::mutex> lock(lanes->build);
+    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+    return lanes->ready || cudaStreamIsCapturing(stream, &capturing) != cudaSuccess || capturing == cudaStreamCaptureStatusNone;
 }
 
 // Algorithmic flops of one near update of the pipelined schedule: the tiles of the tile anti-diagonal s as sources, the
@@ -528,8 +547,8 @@ int sweep_tiles_overlapped(const g2d_sweep_desc *d, SweepArgs<F> &a, F *planes, 
 template <typename F>
 int sweep_fused(const g2d_sweep_desc *d, cudaStream_t stream, LaunchTimer *timer = nullptr, double *flops = nullptr) {
     const size_t plane = base_plane(d);
-    const bool tc = tc_eligible(d);
-    const size_t extra = tc ? tc_extra_bytes(d) : overlap_eligible(d) ? overlap_planes<F>() * plane : 0;
+    const bool tc = takes_tensor_cores(d, stream);
+    const size_t extra = tc_eligible(d) ? tc_extra_bytes(d) : overlap_eligible(d) ? overlap_planes<F>() * plane : 0;
     if (!d->workspace || d->workspace_bytes < 2 * plane + extra) return G2D_ERR_WORKSPACE;
     if (((uintptr_t)d->workspace & 255) != 0) return G2D_ERR_WORKSPACE;
     SweepArgs<F> a;
@@ -548,7 +567,7 @@ int sweep_fused(const g2d_sweep_desc *d, cudaStream_t stream, LaunchTimer *timer
     a.kind = d->quant_kind;
     a.batch = d->batch; a.m = d->m; a.n = d->n;
     a.nI = (int)ceil_div(d->m, TILE); a.nJ = (int)ceil_div(d->n, TILE);
-    a.ld = sweep_pitch(d); a.ldl = d->m; a.ldu = d->n;
+    a.ld = tc ? sweep_pitch(d) : d->n; a.ldl = d->m; a.ldu = d->n;
     // C starts as zeros, and with it what follows it in the workspace of the tensor-core schedules
     const size_t cleared = tc ? plane + tc_carve(d, nullptr).cleared : sizeof(F) * (size_t)d->batch * d->m * a.ld;
     if (cudaMemsetAsync(a.c, 0, cleared, stream) != cudaSuccess) return G2D_ERR_CUDA;
@@ -690,7 +709,7 @@ extern "C" int g2d_sweep_fused_profile(const g2d_sweep_desc *desc, void *stream,
     double flops[3] = {0, 0, 0};
     status = desc->dtype == G2D_F32 ? sweep_fused<float>(desc, st, &timer, flops) : sweep_fused<double>(desc, st, &timer, flops);
     if (cudaStreamSynchronize(st) != cudaSuccess) status = status == G2D_OK ? G2D_ERR_CUDA : status;
-    if (status == G2D_OK && tc_eligible(desc)) {
+    if (status == G2D_OK && takes_tensor_cores(desc, st)) {
         // the tensor-core kernels report a bounded wait that ran out through a flag behind the C and E planes
         const size_t plane = base_plane(desc);
         int flag = 0;
