@@ -89,10 +89,10 @@ struct TcWorkspace {
     TcPlanes planes;
     float *yf, *cf, *yn, *cn;  // far and neighbour planes of the pipelined schedule
     float *y, *l, *u;          // padded copies, where the rows need them (else null)
-    size_t cleared, bytes;     // bytes that start as zeros (the error flag and the far planes, first), all bytes
+    size_t cleared, bytes;     // bytes that start as zeros (the error flag, the count of wide tiles and the far planes, first), all bytes
 };
 inline TcWorkspace tc_carve(const g2d_sweep_desc *d, char *base) {
-    TcWorkspace w;
+    TcWorkspace w{};
     size_t at = 0;
     auto take = [&](size_t bytes) {
         char *p = base + at;
@@ -103,7 +103,8 @@ inline TcWorkspace tc_carve(const g2d_sweep_desc *d, char *base) {
     const int64_t m = d->m, n = d->n, ld = sweep_pitch(d), nI = ceil_div(m, (int64_t)TILE), nJ = ceil_div(n, (int64_t)TILE);
     pl.ldm = round_up(m, 8);
     pl.ldn = round_up(n, 8);
-    pl.error_flag = (int *)take(sizeof(int));  // first: read there when a sweep is profiled
+    pl.error_flag = (int *)take(2 * sizeof(int));  // first: read there when a sweep is profiled
+    pl.wide_count = pl.error_flag + 1;
     for (float **p : {&w.yf, &w.cf}) *p = (float *)take(4 * m * ld);
     w.cleared = at;
     for (__half **p : {&pl.et_hi, &pl.et_lo}) *p = (__half *)take(2 * n * pl.ldm);
@@ -577,8 +578,8 @@ int sweep_fused(const g2d_sweep_desc *d, cudaStream_t stream, LaunchTimer *timer
     b.batch = a.batch; b.m = a.m; b.n = a.n; b.P = TILE; b.Q = TILE; b.down_into_y = 0; b.mode = BAND_TILE; b.filter = 0;
     if (tc) {
         if constexpr (sizeof(F) == sizeof(float)) {
-            const TcWorkspace w = tc_carve(d, (char *)d->workspace + 2 * plane);
-            const TcPlanes &planes = w.planes;
+            TcWorkspace w = tc_carve(d, (char *)d->workspace + 2 * plane);
+            TcPlanes &planes = w.planes;
             if (w.y == nullptr && ((uintptr_t)d->y & 15) != 0) return G2D_ERR_BAD_ARGUMENT;
             auto padded = [&](float *to, int64_t pitch, const void *from, int64_t rows, int64_t cols) {
                 return cudaMemcpy2DAsync(to, 4 * pitch, from, 4 * cols, 4 * cols, rows, cudaMemcpyDeviceToDevice, stream) == cudaSuccess;
@@ -594,6 +595,9 @@ int sweep_fused(const g2d_sweep_desc *d, cudaStream_t stream, LaunchTimer *timer
             }
             a.et_hi = planes.et_hi; a.et_lo = planes.et_lo; a.c_hi = planes.c_hi; a.c_lo = planes.c_lo;
             a.e_scale = planes.e_scale; a.c_scale = planes.c_scale; a.ldm = planes.ldm; a.ldn = planes.ldn;
+            a.wide_count = planes.wide_count;
+            planes.l = a.l; planes.u = a.u; planes.e = a.e; planes.c = a.c;
+            planes.ldl = a.ldl; planes.ldu = a.ldu; planes.ld = a.ld;
             if (d->reserved != 2) {
                 a.yf = w.yf; a.cf = w.cf;
                 a.yn = w.yn; a.cn = w.cn;  // written before they are read: no clearing

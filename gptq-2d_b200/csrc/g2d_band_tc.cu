@@ -30,7 +30,55 @@ struct BandJob {
     int s, t0, t1;
     int outer_macro, lag_macro;            // > 0: targets that the far update of the source's macro group reaches are left out
     int *error_flag;
+    const float *l, *u, *e, *c_from;       // for the products with wide tiles: the float values
+    float *y_to, *c_to;                    // and the targets
+    int64_t ldl, ldu, ld;
 };
+
+// The product with a wide source tile (see TcPlanes), in float32 from the float values, by the whole CTA: 128 (r) x 64 (x) results,
+// both operands staged whole where the tensor cores' operands would lie, 4 x 4 results per thread at a time.  Few registers: the
+// kernel's other path shares SMs.  The rare path.
+constexpr int WIDE_R = 128, WIDE_X = 64;
+static_assert((WIDE_R + WIDE_X) * TILE * 4 <= BAND_BYTES, "the float operands fit where the 16-bit ones lie");
+__device__ __forceinline__ void wide_product(const BandJob &job, bool right, int a_row, int b_row, int k0, bool valid_a, bool valid_b, float *As) {
+    float *const Bs = As + TILE * WIDE_R;  // As[k][r], Bs[k][x]
+    const int r_end = right ? job.n : job.m, x_end = right ? job.m : job.n;
+    for (int idx = threadIdx.x; idx < TILE * WIDE_R; idx += TC_THREADS) {  // neighbouring threads along the rows of the source
+        const int r = right ? idx % WIDE_R : idx / TILE, k = right ? idx / WIDE_R : idx % TILE;
+        const int64_t at = a_row + r;
+        As[k * WIDE_R + r] = at < r_end ? (right ? job.u[(int64_t)(k0 + k) * job.ldu + at] : job.l[at * job.ldl + k0 + k]) : 0.f;
+    }
+    for (int idx = threadIdx.x; idx < TILE * WIDE_X; idx += TC_THREADS) {
+        const int x = right ? idx / TILE : idx % WIDE_X, k = right ? idx % TILE : idx / WIDE_X;
+        const int64_t at = b_row + x;
+        Bs[k * WIDE_X + x] = at < x_end ? (right ? job.c_from[at * job.ld + k0 + k] : job.e[(int64_t)(k0 + k) * job.ld + at]) : 0.f;
+    }
+    __syncthreads();
+#pragma unroll 1
+    for (int block = threadIdx.x; block < (WIDE_R / 4) * (WIDE_X / 4); block += TC_THREADS) {
+        const int r0 = (right ? block % (WIDE_R / 4) : block / (WIDE_X / 4)) * 4, x0 = (right ? block / (WIDE_R / 4) : block % (WIDE_X / 4)) * 4;
+        if (!(r0 < TILE ? valid_a : valid_b)) continue;
+        float acc[4][4] = {};
+#pragma unroll 2
+        for (int k = 0; k < TILE; ++k) {
+            const float4 p = *reinterpret_cast<const float4 *>(As + k * WIDE_R + r0), q = *reinterpret_cast<const float4 *>(Bs + k * WIDE_X + x0);
+            const float pv[4] = {p.x, p.y, p.z, p.w}, qv[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+            for (int r = 0; r < 4; ++r)
+#pragma unroll
+                for (int x = 0; x < 4; ++x) acc[r][x] = fmaf(pv[r], qv[x], acc[r][x]);
+        }
+#pragma unroll
+        for (int r = 0; r < 4; ++r)
+#pragma unroll
+            for (int x = 0; x < 4; ++x) {
+                const int64_t at_r = a_row + r0 + r, at_x = b_row + x0 + x;
+                if (at_r >= r_end || at_x >= x_end) continue;
+                if (right) job.y_to[at_x * job.ld + at_r] += acc[r][x];
+                else job.c_to[at_r * job.ld + at_x] += acc[r][x];
+            }
+    }
+}
 
 // grid: x = tile column (down jobs) or tile row (right jobs), y = pair slot along the target range, z = 0 down, 1 right
 __global__ void __launch_bounds__(TC_THREADS) band_tc_kernel(const __grid_constant__ BandJob job) {
@@ -61,6 +109,9 @@ __global__ void __launch_bounds__(TC_THREADS) band_tc_kernel(const __grid_consta
     const CUtensorMap *a_hi = right ? &job.ut_hi : &job.l_hi, *a_lo = right ? &job.ut_lo : &job.l_lo;
     const CUtensorMap *b_hi = right ? &job.c_hi : &job.et_hi, *b_lo = right ? &job.c_lo : &job.et_lo;
 
+    // asked for here, used behind the set-up: negative where the source tile is wide
+    const float source_scale = right ? job.c_scale[(int64_t)fixed * job.nJ + k_tile] : job.e_scale[(int64_t)k_tile * job.nJ + fixed];
+
     const uint32_t smem_base = (smem_u32(tc_smem_raw) + 1023u) & ~1023u;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (threadIdx.x == 0) {
@@ -78,7 +129,9 @@ __global__ void __launch_bounds__(TC_THREADS) band_tc_kernel(const __grid_consta
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = tmem_slot;
 
-    if (warp == 0) {
+    if (source_scale < 0.f) {
+        wide_product(job, right, a_row, b_row, k_tile * TILE, valid_a, valid_b, reinterpret_cast<float *>(tc_smem_raw + (smem_base - smem_u32(tc_smem_raw))));
+    } else if (warp == 0) {
         if (lane == 0) {
             const int k = k_tile * TILE;
             mbar_expect_tx(&full_bar, BAND_BYTES);
@@ -112,8 +165,7 @@ __global__ void __launch_bounds__(TC_THREADS) band_tc_kernel(const __grid_consta
         const int target = q < 2 ? t_a : t_b;                    // tile row (down) or column (right) of this warp's results
         float factor = 0.f;
         if (mine)
-            factor = right ? job.u_scale[(int64_t)target * job.nJ + k_tile] * job.c_scale[(int64_t)fixed * job.nJ + k_tile]
-                           : job.l_scale[(int64_t)target * job.nI + k_tile] * job.e_scale[(int64_t)k_tile * job.nJ + fixed];
+            factor = source_scale * (right ? job.u_scale[(int64_t)target * job.nJ + k_tile] : job.l_scale[(int64_t)target * job.nI + k_tile]);
         const bool ok = mbar_wait(&accum_bar, 0, 256);
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         if (!ok) failed = 1;
@@ -170,10 +222,12 @@ __global__ void __launch_bounds__(TC_THREADS) band_tc_kernel(const __grid_consta
 struct BandMaps {
     CUtensorMap l_hi, l_lo, ut_hi, ut_lo, et_hi, et_lo, c_hi, c_lo, y, c;
 };
-static_assert(sizeof(BandMaps) <= sizeof(BandTcMaps), "opaque tensor-map storage is too small");
+static_assert(sizeof(BandMaps) <= sizeof(BandTcMaps::bytes), "opaque tensor-map storage is too small");
 
 int band_tc_prepare(BandTcMaps *opaque, const TcPlanes &pl, float *y, float *c, int64_t m, int64_t n, int64_t ld) {
     BandMaps *maps = reinterpret_cast<BandMaps *>(opaque);
+    opaque->y = y;
+    opaque->c = c;
     if (!make_map_16(&maps->l_hi, pl.l_hi, m, m, MT, false, pl.ldm) || !make_map_16(&maps->l_lo, pl.l_lo, m, m, MT, false, pl.ldm) ||
         !make_map_16(&maps->ut_hi, pl.ut_hi, n, n, MT, false, pl.ldn) || !make_map_16(&maps->ut_lo, pl.ut_lo, n, n, MT, false, pl.ldn) ||
         !make_map_16(&maps->et_hi, pl.et_hi, n, m, BN, false, pl.ldm) || !make_map_16(&maps->et_lo, pl.et_lo, n, m, BN, false, pl.ldm) ||
@@ -206,6 +260,9 @@ int launch_band_tc(const BandTcMaps *opaque, const TcPlanes &pl, int64_t m, int6
     job.s = s; job.t0 = t0; job.t1 = t1;
     job.outer_macro = outer_macro; job.lag_macro = lag_macro;
     job.error_flag = pl.error_flag;
+    job.l = pl.l; job.u = pl.u; job.e = pl.e; job.c_from = pl.c;
+    job.y_to = opaque->y; job.c_to = opaque->c;
+    job.ldl = pl.ldl; job.ldu = pl.ldu; job.ld = pl.ld;
     // pairs along the moving index that can hold a target: at most (t1 - t0) / 2 + 2, never more than the matrix has
     const int longest = job.nI > job.nJ ? job.nI : job.nJ;
     int slots = (t1 - t0) / 2 + 2;

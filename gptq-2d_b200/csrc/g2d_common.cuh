@@ -163,6 +163,7 @@ struct SweepArgs {
     // ldm values) and the completed C (rows of ldn), with the tiles' scales: operands of the updates (see TcPlanes)
     __half *et_hi = nullptr, *et_lo = nullptr, *c_hi = nullptr, *c_lo = nullptr;
     float *e_scale = nullptr, *c_scale = nullptr;
+    int *wide_count = nullptr;
     // pipelined schedule only (else null / 0): planes that collect the far feedback apart from Y and C, added when a
     // tile is loaded
     const F *yf = nullptr, *cf = nullptr;
@@ -188,6 +189,14 @@ __device__ __forceinline__ void split_half(float scaled, __half &hi, __half &lo)
 // Operand planes of the tensor-core updates of the sweep (see g2d_macro_update_tc.cu): fp16 pairs, K-major, each 64 x 64 tile under
 // a power of two of its own.  A slice of k is one tile wide, so the scales come out of a product slice by slice:
 // `*_scale` holds what a product with the tile has to be multiplied by.
+// Wide tiles.  What lies far below the tile's largest value loses bits (see split_half), which matters where whole rows or columns
+// do: with rows in units of their own, L[i, k] grows as E[k, j] falls, and the rows of the small units consist of products of
+// what is lost (rows apart by a factor of 2^12 alternately: 9 times the error of float32, by 2^20: three per cent of the
+// values).  The tile sweep therefore compares the largest values of the rows and columns of E and of C; where one is
+// 2^8 or more below the tile's (zeros apart), or not finite, the planes of that tile get zeros, its scale is stored with its sign
+// set and its float values are stored too, and the products with it are formed from them in float32: by the near update itself, and by
+// wide_update_kernel behind every far one.  Up to that ratio the error is that of an even tile.
+constexpr unsigned WIDE_RATIO_BITS = 8u << 7;  // 2^8 in the upper halves of floats
 struct TcPlanes {
     __half *et_hi, *et_lo, *c_hi, *c_lo;  // E^T [n][ldm] and the completed C [m][ldn], written by the tile sweep
     __half *l_hi, *l_lo, *ut_hi, *ut_lo;  // L [m][ldm] and U^T [n][ldn], below the diagonal tiles, written once per sweep
@@ -195,6 +204,9 @@ struct TcPlanes {
     float *l_scale, *u_scale;             // [nI][nI], [nJ][nJ] (tile row of U^T, tile of k)
     int64_t ldm, ldn;                     // m and n rounded up to multiples of 8 (rows of 16-byte multiples, a TMA requirement)
     int *error_flag;                      // set when a bounded wait inside a kernel ran out
+    const float *l, *u, *e, *c;           // the float values: rows of ldl, ldu and (E and C, of wide tiles only) ld
+    int64_t ldl, ldu, ld;
+    int *wide_count;                      // wide tiles of the sweep so far, E and C each
 };
 // Band updates between tiles on the tensor cores (pipelined schedule; see g2d_band_tc.cu): sources are the tiles of the
 // anti-diagonal s, targets those of t0..t1 (t0 >= s + 2), feedback is added into the planes y (right) and c (down) of the maps.
@@ -202,6 +214,7 @@ struct TcPlanes {
 // when its macro anti-diagonal is lag_macro or more past the end of the source's group of outer_macro macro anti-diagonals.
 struct BandTcMaps {
     alignas(64) unsigned char bytes[10 * 128];  // tensor maps of the eight operand planes and the two targets (opaque here)
+    float *y, *c;                               // the targets
 };
 int band_tc_prepare(BandTcMaps *maps, const TcPlanes &planes, float *y, float *c, int64_t m, int64_t n, int64_t ld);
 int launch_band_tc(const BandTcMaps *maps, const TcPlanes &planes, int64_t m, int64_t n, int s, int t0, int t1, int outer_macro, int lag_macro, cudaStream_t stream);
@@ -209,6 +222,7 @@ int launch_band_tc(const BandTcMaps *maps, const TcPlanes &planes, int64_t m, in
 int tc_prepare_operands(const float *l, int64_t ldl, const float *u, int64_t ldu, int64_t m, int64_t n, const TcPlanes &planes, cudaStream_t stream);
 struct MacroTcMaps {
     alignas(64) unsigned char bytes[10 * 128];  // tensor maps of the eight operand planes with 128-row boxes and of the two targets
+    float *y, *c;                               // the targets
 };
 // y and c: the planes that receive the right and the down feedback, rows of ld values (a multiple of 4)
 int macro_tc_prepare(MacroTcMaps *maps, const TcPlanes &planes, float *y, float *c, int64_t m, int64_t n, int64_t ld);

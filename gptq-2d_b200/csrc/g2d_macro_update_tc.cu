@@ -162,6 +162,65 @@ __global__ void __launch_bounds__(PAIR_THREADS, 1) macro_update_wide_kernel(cons
     if (threadIdx.x == 0 && failed && error_flag) atomicExch(error_flag, 1);
 }
 
+// ---- far products with wide tiles (see TcPlanes), in float32 from the float values ----
+// A few CTAs behind every far update, which leave again where the sweep has no wide tile (a load: about 2 us beside the tile launch
+// of the moment; behind the near updates, which the tile launches wait for sooner, the same launch took 1.5 % of a sweep).
+// Else each walks over the targets, looks for sources among the wide tiles and adds their products, 64 x 64 targets at a time, 4 x 4 per
+// thread, both operands of a source tile staged whole.  One CTA owns each target and the launch follows its update on one stream: a
+// fixed order of additions.  The rare path: FFMA, about a tenth of the tensor cores' rate.
+constexpr int WTH = 256, WLD = TILE + 4;
+__global__ void __launch_bounds__(WTH) wide_update_kernel(TcPlanes P, MacroRange R, float *y, float *c, int m, int n) {
+    __shared__ __align__(16) float As[TILE * WLD], Bs[TILE * WLD];
+    __shared__ int wide;  // one answer for the CTA: the tile launch of the moment may be counting
+    if (threadIdx.x == 0) wide = *P.wide_count;
+    __syncthreads();
+    if (wide == 0) return;
+    const int nI = (m + TILE - 1) / TILE, nJ = (n + TILE - 1) / TILE, longest = min(nI, nJ);
+    const int d0 = 2 * R.t_first, d1 = min(2 * R.s_end, nI + nJ - 2);  // tile anti-diagonals that can hold targets
+    const int tid = threadIdx.x, ty = tid >> 4, tx = tid & 15;
+    for (int64_t at = blockIdx.x; at < (int64_t)(d1 - d0 + 1) * longest; at += gridDim.x) {
+        const int d = d0 + (int)(at / longest), TI = max(0, d - nJ + 1) + (int)(at % longest), TJ = d - TI;
+        if (TI >= nI || TJ < 0 || !R.target(TI >> 1, TJ >> 1)) continue;
+        const int64_t i0 = (int64_t)TI * TILE, j0 = (int64_t)TJ * TILE;
+        for (int right = 0; right < 2; ++right) {
+            int k0, macros;
+            if (!R.sources((right ? TI : TJ) >> 1, k0, macros)) continue;
+            float acc[4][4] = {};
+            bool any = false;
+            for (int k = 2 * k0; k < 2 * (k0 + macros); ++k) {
+                if ((right ? P.c_scale[(int64_t)TI * nJ + k] : P.e_scale[(int64_t)k * nJ + TJ]) >= 0.f) continue;  // the same for the whole CTA
+                any = true;
+                const int64_t kk = (int64_t)k * TILE;
+                const float *const a = right ? P.c + i0 * P.ld + kk : P.l + i0 * P.ldl + kk, *const b = right ? P.u + kk * P.ldu + j0 : P.e + kk * P.ld + j0;
+                const int64_t lda = right ? P.ld : P.ldl, ldb = right ? P.ldu : P.ld;
+                __syncthreads();  // the products before have been formed
+                for (int idx = tid; idx < TILE * TILE; idx += WTH) {
+                    const int r = idx / TILE, x = idx % TILE;
+                    As[x * WLD + r] = i0 + r < m ? a[r * lda + x] : 0.f;
+                    Bs[r * WLD + x] = j0 + x < n ? b[r * ldb + x] : 0.f;
+                }
+                __syncthreads();
+#pragma unroll 8
+                for (int x = 0; x < TILE; ++x) {
+                    const float4 p = *reinterpret_cast<const float4 *>(As + x * WLD + ty * 4), q = *reinterpret_cast<const float4 *>(Bs + x * WLD + tx * 4);
+                    const float pv[4] = {p.x, p.y, p.z, p.w}, qv[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+                    for (int r = 0; r < 4; ++r)
+#pragma unroll
+                        for (int s = 0; s < 4; ++s) acc[r][s] = fmaf(pv[r], qv[s], acc[r][s]);
+                }
+            }
+            if (!any) continue;
+            float *const out = right ? y : c;
+#pragma unroll
+            for (int r = 0; r < 4; ++r)
+#pragma unroll
+                for (int s = 0; s < 4; ++s)
+                    if (i0 + ty * 4 + r < m && j0 + tx * 4 + s < n) out[(i0 + ty * 4 + r) * P.ld + j0 + tx * 4 + s] += acc[r][s];
+        }
+    }
+}
+
 // ---- one-time operand preparation: a 64 x 64 tile per CTA, strictly below the diagonal tiles (no update reads the others) ----
 
 // Tile (I, K), K < I, of a lower triangle of nT tile rows from a linear index
@@ -202,7 +261,8 @@ __global__ void __launch_bounds__(256) split_tile_kernel(const float *__restrict
         }
 #pragma unroll
         for (int x = 0; x < 4; ++x) {
-            most = max(most, __float_as_uint(v[x]) & 0x7fffffffu);
+            const unsigned size = __float_as_uint(v[x]) & 0x7fffffffu;
+            most = max(most, size < 0x7f800000u ? size : 0u);  // infinities and NaN stay what they are under any scale
             if (UPPER) tile[c + x][r] = v[x];
             else tile[r][c + x] = v[x];
         }
@@ -246,13 +306,15 @@ int tc_prepare_operands(const float *l, int64_t ldl, const float *u, int64_t ldu
     return G2D_OK;
 }
 
-static_assert(sizeof(TcMaps) <= sizeof(MacroTcMaps), "opaque tensor-map storage is too small");
+static_assert(sizeof(TcMaps) <= sizeof(MacroTcMaps::bytes), "opaque tensor-map storage is too small");
 constexpr size_t MACRO_SMEM = (size_t)MACRO_STAGES * pair_stage_bytes<128> + PAIR_BOXES + 1024;
 constexpr size_t MACRO_WIDE_SMEM = (size_t)MACRO_WIDE_STAGES * pair_stage_bytes<256> + PAIR_BOXES + 1024;
 
 // Tensor maps of one sweep (encoded once, reused by every macro update of the sweep) and the kernels' one-time set-up.
 int macro_tc_prepare(MacroTcMaps *opaque, const TcPlanes &pl, float *y, float *c, int64_t m, int64_t n, int64_t ld) {
     TcMaps &maps = *reinterpret_cast<TcMaps *>(opaque);
+    opaque->y = y;
+    opaque->c = c;
     if (!make_map_16(&maps.l_hi, pl.l_hi, m, m, MT, false, pl.ldm) || !make_map_16(&maps.l_lo, pl.l_lo, m, m, MT, false, pl.ldm) ||
         !make_map_16(&maps.c_hi, pl.c_hi, m, n, MT, false, pl.ldn) || !make_map_16(&maps.c_lo, pl.c_lo, m, n, MT, false, pl.ldn) ||
         !make_map_16(&maps.et_hi, pl.et_hi, n, m, MT, false, pl.ldm) || !make_map_16(&maps.et_lo, pl.et_lo, n, m, MT, false, pl.ldm) ||
@@ -284,9 +346,11 @@ int launch_macro_update_tc(const MacroTcMaps *opaque, const TcPlanes &pl, int64_
     if (blocks * (RB_I * RB_J / 4) < 4 * 148) {
         if (range.nI2 > 65535) return G2D_ERR_TOO_LARGE;
         macro_update_tc_kernel<<<dim3((unsigned)(s_end - t_first), (unsigned)range.nI2), PAIR_THREADS, MACRO_SMEM, stream>>>(maps, scales, range, pl.error_flag);
-        return check_launch();
+    } else {
+        macro_update_wide_kernel<<<(unsigned)(blocks * (RB_I * RB_J / 4)), PAIR_THREADS, MACRO_WIDE_SMEM, stream>>>(maps, scales, range, pl.error_flag);
     }
-    macro_update_wide_kernel<<<(unsigned)(blocks * (RB_I * RB_J / 4)), PAIR_THREADS, MACRO_WIDE_SMEM, stream>>>(maps, scales, range, pl.error_flag);
+    if (check_launch() != G2D_OK) return G2D_ERR_CUDA;
+    wide_update_kernel<<<2 * 148, WTH, 0, stream>>>(pl, range, opaque->y, opaque->c, (int)m, (int)n);
     return check_launch();
 }
 

@@ -160,7 +160,8 @@ __global__ void __launch_bounds__(TTH, 1) tile_sweep_kernel(SweepArgs<F> P, int 
     F *Lbs = Ubs + TILE * LD;                 // the same: L[I + 1, I], the lower neighbour's
     F *Yns = Lbs + TILE * LD;                 // the same: the feedback for the right neighbour, C[I, J] U[J, J + 1], growing sub-tile by sub-tile
     F *Cns = Yns + TILE * LD;                 // and for the lower one, L[I + 1, I] E[I, J]
-    __shared__ unsigned tile_max[2][TTH / 32];
+    __shared__ unsigned row_max[TILE];
+    __shared__ __align__(16) unsigned column_max[TTH / 32][TILE];
     __shared__ unsigned fast_div[NSUB];       // every scale of the sub-tile allows the division by reciprocal
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -627,34 +628,52 @@ __global__ void __launch_bounds__(TTH, 1) tile_sweep_kernel(SweepArgs<F> P, int 
             }
         }
         // ---- operands of the tensor-core updates: fp16 pairs of E (transposed) and of the completed C under the tile's scales ----
+        bool wide_e = false, wide_c = false;
         if constexpr (sizeof(F) == sizeof(float)) {
             if (P.c_hi != nullptr) {
-                // largest value of the tile (entries outside the matrix are zero)
-                unsigned me = 0u, mc = 0u;
-                for (int idx = tid; idx < TILE * TILE / 4; idx += TTH) {
-                    const int r = idx / (TILE / 4), c = (idx % (TILE / 4)) * 4;
+                // Largest values of the rows, the columns and the tile (entries outside the matrix are zero), of E in the lower and of C in
+                // the upper half of a word: the upper halves of floats are all that the scale and the comparison need.
+                unsigned column[4] = {0u, 0u, 0u, 0u};
+#pragma unroll
+                for (int t = 0; t < TILE * TILE / 4 / TTH; ++t) {  // a thread's vectors lie in the same four columns
+                    const int idx = t * TTH + tid, r = idx / (TILE / 4), c = (idx % (TILE / 4)) * 4;
                     F ve[4], vc[4];
                     load4(Ys + r * LD + c, ve);
                     load4(Cs + r * LD + c, vc);
+                    unsigned row = 0u;
 #pragma unroll
                     for (int x = 0; x < 4; ++x) {
-                        me = max(me, __float_as_uint((float)ve[x]) & 0x7fffffffu);
-                        mc = max(mc, __float_as_uint((float)vc[x]) & 0x7fffffffu);
+                        const unsigned both = __byte_perm(__float_as_uint((float)ve[x]), __float_as_uint((float)vc[x]), 0x7632) & 0x7fff7fffu;
+                        row = __vmaxu2(row, both);
+                        column[x] = __vmaxu2(column[x], both);
                     }
-                }
-                me = __reduce_max_sync(0xffffffffu, me);
-                mc = __reduce_max_sync(0xffffffffu, mc);
-                if (lane == 0) { tile_max[0][warp] = me; tile_max[1][warp] = mc; }
-                __syncthreads();
 #pragma unroll
-                for (int w2 = 0; w2 < TTH / 32; ++w2) {
-                    me = max(me, tile_max[0][w2]);
-                    mc = max(mc, tile_max[1][w2]);
+                    for (int o = 1; o < TILE / 4; o <<= 1) row = __vmaxu2(row, __shfl_xor_sync(0xffffffffu, row, o));
+                    if ((lane & 15) == 0) row_max[r] = row;
                 }
-                const int ee = range_exponent(__uint_as_float(me)), ec = range_exponent(__uint_as_float(mc));
+#pragma unroll
+                for (int x = 0; x < 4; ++x) column[x] = __vmaxu2(column[x], __shfl_xor_sync(0xffffffffu, column[x], 16));
+                if (lane < 16) *reinterpret_cast<uint4 *>(&column_max[warp][lane * 4]) = make_uint4(column[0], column[1], column[2], column[3]);
+                __syncthreads();
+                unsigned most = 0u, least = 0xffffffffu;  // every warp for itself: two rows and two columns per lane
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    unsigned col = column_max[0][h * 32 + lane];
+#pragma unroll
+                    for (int w2 = 1; w2 < TTH / 32; ++w2) col = __vmaxu2(col, column_max[w2][h * 32 + lane]);
+                    const unsigned row = row_max[h * 32 + lane];
+                    most = __vmaxu2(most, row);
+                    least = __vminu2(least, __vminu2(row | __vcmpeq2(row, 0u), col | __vcmpeq2(col, 0u)));  // zeros apart
+                }
+                const unsigned most_e = __reduce_max_sync(0xffffffffu, most & 0xffffu), most_c = __reduce_max_sync(0xffffffffu, most >> 16);
+                const unsigned least_e = __reduce_min_sync(0xffffffffu, least & 0xffffu), least_c = __reduce_min_sync(0xffffffffu, least >> 16);
+                wide_e = most_e >= 0x7f80u || least_e + WIDE_RATIO_BITS <= most_e;
+                wide_c = most_c >= 0x7f80u || least_c + WIDE_RATIO_BITS <= most_c;
+                const int ee = range_exponent(__uint_as_float(most_e << 16)), ec = range_exponent(__uint_as_float(most_c << 16));
                 if (tid == 0) {
-                    P.e_scale[(int64_t)I * P.nJ + J] = power_of_two(ee);
-                    P.c_scale[(int64_t)I * P.nJ + J] = power_of_two(ec);
+                    P.e_scale[(int64_t)I * P.nJ + J] = wide_e ? -1.f : power_of_two(ee);
+                    P.c_scale[(int64_t)I * P.nJ + J] = wide_c ? -1.f : power_of_two(ec);
+                    if (wide_e || wide_c) atomicAdd(P.wide_count, wide_e + wide_c);
                 }
                 const float e_by = power_of_two(-ee), c_by = power_of_two(-ec);
                 // eight entries per thread and store.  C along its rows; E transposed: a thread gathers eight rows of one column
@@ -667,7 +686,7 @@ __global__ void __launch_bounds__(TTH, 1) tile_sweep_kernel(SweepArgs<F> P, int 
                         const int r = idx / (TILE / 8), c = (idx % (TILE / 8)) * 8;
                         if (r < rows_in && c < cols_in) {
 #pragma unroll
-                            for (int x = 0; x < 8; ++x) split_half((float)Cs[r * LD + c + x] * c_by, h[x], l[x]);
+                            for (int x = 0; x < 8; ++x) split_half(wide_c ? 0.f : (float)Cs[r * LD + c + x] * c_by, h[x], l[x]);
                             const int64_t at = (i0 + r) * P.ldn + j0 + c;
                             *reinterpret_cast<uint4 *>(P.c_hi + at) = *reinterpret_cast<const uint4 *>(h);
                             *reinterpret_cast<uint4 *>(P.c_lo + at) = *reinterpret_cast<const uint4 *>(l);
@@ -677,7 +696,7 @@ __global__ void __launch_bounds__(TTH, 1) tile_sweep_kernel(SweepArgs<F> P, int 
                         const int c = idx % TILE, r = (idx / TILE) * 8;
                         if (r < rows_in && c < cols_in) {
 #pragma unroll
-                            for (int x = 0; x < 8; ++x) split_half((float)Ys[(r + x) * LD + c] * e_by, h[x], l[x]);
+                            for (int x = 0; x < 8; ++x) split_half(wide_e ? 0.f : (float)Ys[(r + x) * LD + c] * e_by, h[x], l[x]);
                             const int64_t at = (j0 + c) * P.ldm + i0 + r;
                             *reinterpret_cast<uint4 *>(P.et_hi + at) = *reinterpret_cast<const uint4 *>(h);
                             *reinterpret_cast<uint4 *>(P.et_lo + at) = *reinterpret_cast<const uint4 *>(l);
@@ -687,25 +706,24 @@ __global__ void __launch_bounds__(TTH, 1) tile_sweep_kernel(SweepArgs<F> P, int 
             }
         }
         // ---- store the errors and the completed C of the tile, unless only their operand planes are read from here on ----
-        if (P.c_hi != nullptr && yng != nullptr) {
+        const bool planes_only = P.c_hi != nullptr && yng != nullptr;
+        const bool keep_e = !planes_only || wide_e, keep_c = !planes_only || wide_c;
+        if (!keep_e && !keep_c) {
         } else if (vec) {
             for (int idx = tid; idx < TILE * TILE / 4; idx += TTH) {
                 const int r = idx / (TILE / 4), c = (idx % (TILE / 4)) * 4;
                 F ve[4], vc[4];
                 load4(Ys + r * LD + c, ve);
                 load4(Cs + r * LD + c, vc);
-                store4(eg + (i0 + r) * ld + j0 + c, ve);
-                store4(cg + (i0 + r) * ld + j0 + c, vc);
+                if (keep_e) store4(eg + (i0 + r) * ld + j0 + c, ve);
+                if (keep_c) store4(cg + (i0 + r) * ld + j0 + c, vc);
             }
         } else {
-            for (int idx = tid; idx < TILE * TILE; idx += TTH) {
-                const int r = idx / TILE, c = idx % TILE;
-                const int64_t gi = i0 + r, gj = j0 + c;
-                if (gi < m && gj < n) {
-                    eg[gi * ld + gj] = Ys[r * LD + c];
-                    cg[gi * ld + gj] = Cs[r * LD + c];
+            for (int r = warp; r < rows_in; r += TTH / 32)
+                for (int c = lane; c < cols_in; c += 32) {
+                    if (keep_e) eg[(i0 + r) * ld + j0 + c] = Ys[r * LD + c];
+                    if (keep_c) cg[(i0 + r) * ld + j0 + c] = Cs[r * LD + c];
                 }
-            }
         }
         __syncthreads();
     }
