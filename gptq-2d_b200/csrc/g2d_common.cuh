@@ -72,11 +72,13 @@ __device__ __forceinline__ float affine_value_fast(float y, float scale, float z
 __device__ __forceinline__ double affine_value_fast(double y, double, double, double, double, double) { return y; }  // not used: see the dispatch
 // double: `rc` is the correctly rounded reciprocal; two residual corrections make the quotient correctly rounded (the
 // first brings it within an ulp, and Markstein's theorem then gives RN(q + r rc) = RN(y / s)).  Same bits as
-// affine_value, without the division's hundred-odd cycles on the critical path of every stage.
+// affine_value, without the division's hundred-odd cycles on the critical path of every stage.  An infinite quotient (y infinite, or
+// beyond the range of doubles in units of the scale) has no residual and stays, to be clamped.
 __device__ __forceinline__ double affine_value_rcp(double y, double scale, double zp, double rc, double qmin, double qmax) {
-    double q = y * rc;
+    const double q0 = y * rc;
+    double q = fma(fma(-q0, scale, y), rc, q0);
     q = fma(fma(-q, scale, y), rc, q);
-    q = fma(fma(-q, scale, y), rc, q);
+    q = fabs(q0) <= 1.7976931348623157e308 ? q : q0;
     double t = rint(__dadd_rn(q, zp));
     t = t < qmin ? qmin : t;
     t = t > qmax ? qmax : t;

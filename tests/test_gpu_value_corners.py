@@ -1,0 +1,31 @@
+"""Values at the edges of what the kernels' short forms of the quantizer serve: signs of zero, infinities, NaN."""
+import functools
+
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("value, scale", [(float("inf"), 0.1), (-float("inf"), 0.1), (1e300, 1e-100), (-1e300, 1e-100), (1.7e308, 0.5), (float("nan"), 0.1), (1e300, 0.1)])
+def test_double_quotients_beyond_the_range(value, scale):
+    """The fused float64 sweep against the engine whose quantizer divides: an infinite quotient is clamped, NaN stays NaN."""
+    import gptq_2d as G
+    import quantizer_int as Q
+
+    gen = torch.Generator(device="cuda").manual_seed(3)
+    rand = lambda *shape: torch.randn(*shape, generator=gen, device="cuda", dtype=torch.float64)
+    m, n = 20, 70
+    w, l, u = rand(m, n), torch.tril(rand(m, m) * 0.1, -1), torch.triu(rand(n, n) * 0.1, 1)
+    w[4, 9] = value
+    inputs = (torch.full((m, n), scale, device="cuda", dtype=torch.float64), torch.zeros(m, n, device="cuda", dtype=torch.float64))
+    quantizer = functools.partial(Q.affine_quantizer_cuda, qmin=-8, qmax=7)
+    fused = G.gptq_2d(w, l, u, quantizer=quantizer, quantizer_inputs=inputs)
+    generic = G.gptq_2d(w, l, u, quantizer=lambda *a, **k: quantizer(*a, **k), quantizer_inputs=inputs)
+    assert torch.equal(fused[4, 9].isnan(), generic[4, 9].isnan())
+    if not generic[4, 9].isnan():
+        assert fused[4, 9] == generic[4, 9]
+    fed = torch.zeros(m, n, dtype=torch.bool, device="cuda")
+    fed[4:, 9:] = True
+    assert torch.equal(fused[~fed], generic[~fed])
