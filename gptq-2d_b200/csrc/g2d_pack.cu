@@ -68,7 +68,7 @@ constexpr float INTEGER_UNIT = 12582912.f;  // 1.5 * 2^23: a float of at most 2^
 constexpr unsigned INTEGER_UNIT_BITS = 0x4B400000u;
 
 // The codes of eight floats, four to a word.  False, with nothing done, where a scale or a quotient is out of the range in which
-// the reciprocal form of the division holds (NaN included): the caller's general path takes those.  Nine instructions per
+// the reciprocal form of the division holds (NaN included, of the zero point too): the caller's general path takes those.  Nine instructions per
 // entry: clamping before rounding is the same between integer bounds, the addition of INTEGER_UNIT is the rounding and the conversion, and
 // the codes are added up as they stand in the low bits, what the unit and qmin contribute taken off once per word.
 template <int BITS>
@@ -96,9 +96,10 @@ __device__ __forceinline__ bool fast_codes(const float (&z)[8], const float (&s)
 #pragma unroll
     for (int x = 0; x < 8; ++x) {
         const float q0 = z[x] * rc[x];
-        ok = ok && fabsf(q0) < 1e30f;
         const float q1 = fmaf(fmaf(-q0, s[x], z[x]), rc[x], q0);
-        const float v = fminf(fmaxf(add_rn(q1, o[x]), low), high);
+        const float sum1 = add_rn(q1, o[x]);
+        ok = ok && fabsf(sum1) < 1e30f;  // with a zero point that is NaN: it converts to 0, a clamp would make it qmin
+        const float v = fminf(fmaxf(sum1, low), high);
         sum[x >> 2] += __float_as_uint(add_rn(v, INTEGER_UNIT)) << ((x & 3) * BITS);
     }
 #pragma unroll

@@ -29,3 +29,15 @@ def test_double_quotients_beyond_the_range(value, scale):
     fed = torch.zeros(m, n, dtype=torch.bool, device="cuda")
     fed[4:, 9:] = True
     assert torch.equal(fused[~fed], generic[~fed])
+
+
+@pytest.mark.parametrize("n", [8, 9, 32])
+def test_packing_under_a_zero_point_that_is_nan(n):
+    """Converts to 0 before it is clamped, in whole groups of eight as in ragged ones."""
+    import packed_codes as P
+
+    z, scale, zero = torch.zeros(2, n, device="cuda"), torch.ones(2, n, device="cuda"), torch.zeros(2, n, device="cuda")
+    zero[1, n - 1] = float("nan")
+    for zeros, at in ((zero, (1, n - 1)), (torch.full((2, 1), float("nan"), device="cuda"), None)):
+        codes = P.pack_codes(z, scale, zeros, qmin=-8, bits=8).cpu().numpy()
+        assert np.array_equal(codes, np.full_like(codes, 8))
