@@ -127,9 +127,11 @@ __device__ __forceinline__ void pivot_roots(float d, float &root, float &inv_roo
     const float q = r * r;
     inv = fmaf(fmaf(-d, q, 1.f), q, q);
 }
+// double: the chain takes the reciprocal only.  Rows are stored as they are and scaled sixteen at a time, a pivot's roots per lane (all
+// three roots of a pivot in the chain: 640 x 640 in 64 x 64 blocks 1098 us, 1008 with one barrier per pivot over the whole block).
 __device__ __forceinline__ void pivot_roots(double d, double &root, double &inv_root, double &inv) {
-    root = sqrt(d);
-    inv_root = 1.0 / root;
+    root = d;
+    inv_root = 1.0;
     inv = 1.0 / d;
 }
 
@@ -203,6 +205,23 @@ __global__ void __launch_bounds__(DTH) ldl_diag_kernel(LdlBatch<F> B, int step_d
                 for (int r = DS - 1; r > 0; --r) {
                     v0[r] = v0[r - 1] - f0 * w[r - 1];
                     v1[r] = v1[r - 1] - f1 * w[r - 1];
+                }
+            }
+            if constexpr (sizeof(F) == sizeof(double)) {
+                __syncwarp();
+                if (lane < DS) {
+                    F &diagonal = S[(r0 + lane) * DLDS + r0 + lane];
+                    const F root = sqrt(diagonal);
+                    diagonal = root;
+                    pivots[r0 + lane] = (F)1 / root;
+                }
+                __syncwarp();
+#pragma unroll 4
+                for (int r = 0; r < DS; ++r) {
+                    F *const row = S + (r0 + r) * DLDS;
+                    const F by = pivots[r0 + r];
+                    if (lane != r0 + r) row[lane] *= by;
+                    if (second && lane + 32 != r0 + r) row[lane + 32] *= by;
                 }
             }
             if (lane == 0 && bad > FB) bad = worst;
@@ -682,11 +701,15 @@ int ldl_run(int count, const int64_t *ns, F *const *as, const int *sizes, F *con
     static PerDeviceOnce configured;
     if (configured.run([&] { return cudaFuncSetAttribute(ldl_diag_kernel<F>, cudaFuncAttributeMaxDynamicSharedMemorySize, diag_smem<F>) == cudaSuccess; }) != G2D_OK)
         return G2D_ERR_CUDA;
+    // Updates on the side stream begin with the third group; without them (and for double) the chain stays on the caller's stream, which
+    // saves the two hand-overs (64 x 64 and 64 x 64 in double: 166 us against 146).
+    const bool beside = any_tc && B.steps > 2 * GROUP;
     std::unique_lock<std::mutex> held;  // until everything is enqueued
-    SideLane *lane = acquire_side_lane(caller, held);
-    if (!lane) return G2D_ERR_CUDA;
-    if (cudaEventRecord(lane->fork, caller) != cudaSuccess || cudaStreamWaitEvent(lane->chain, lane->fork, 0) != cudaSuccess) return G2D_ERR_CUDA;
-    st = lane->chain;
+    SideLane *lane = beside ? acquire_side_lane(caller, held) : nullptr;
+    if (beside) {
+        if (!lane || cudaEventRecord(lane->fork, caller) != cudaSuccess || cudaStreamWaitEvent(lane->chain, lane->fork, 0) != cudaSuccess) return G2D_ERR_CUDA;
+        st = lane->chain;
+    }
     bool recorded[4] = {false, false, false, false};  // near and rest of the last four groups, where a problem closed a pair
     int newest = -1;                                  // the last group with an update on the side stream
     for (int s = B.steps - 1; s >= 0; --s) {  // block row of the largest problem; smaller problems are lined up by groups
@@ -757,7 +780,7 @@ int ldl_run(int count, const int64_t *ns, F *const *as, const int *sizes, F *con
     }
     // everything the side stream did joins the caller's stream before the inverse starts
     if (newest >= 0 && cudaStreamWaitEvent(caller, lane->rest[newest & 3], 0) != cudaSuccess) return G2D_ERR_CUDA;
-    if (cudaEventRecord(lane->join, st) != cudaSuccess || cudaStreamWaitEvent(caller, lane->join, 0) != cudaSuccess) return G2D_ERR_CUDA;
+    if (beside && (cudaEventRecord(lane->join, st) != cudaSuccess || cudaStreamWaitEvent(caller, lane->join, 0) != cudaSuccess)) return G2D_ERR_CUDA;
     st = caller;
     ldl_copy_diag_inverse_kernel<F><<<dim3(B.steps, count), FTH, 0, st>>>(B);
     if (check_launch() != G2D_OK) return G2D_ERR_CUDA;
