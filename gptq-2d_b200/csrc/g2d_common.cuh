@@ -60,16 +60,18 @@ __device__ __forceinline__ float affine_value_rcp(float y, float scale, float zp
 }
 // The same for bounds that are integers below 2^22 in size: then clamping and rounding commute, and a clamped value is
 // rounded half to even by adding and subtracting 1.5 * 2^23, eight cycles instead of the conversion unit's twenty-odd.
-// NaN stays NaN as with the comparisons above.
-__device__ __forceinline__ float affine_value_fast(float y, float scale, float zp, float rc, float qmin, float qmax) {
+// NaN stays NaN as with the comparisons above.  The sum of the two has lost the sign of a zero (a quotient of -0.3 rounds to -0), so
+// `signed_value` is formed once more from a code that has it, beside the chain that goes on with the value.
+__device__ __forceinline__ float affine_value_fast(float y, float scale, float zp, float rc, float qmin, float qmax, float &signed_value) {
     const float q0 = y * rc;
     float t = __fadd_rn(fmaf(fmaf(-q0, scale, y), rc, q0), zp);
     asm("min.NaN.f32 %0, %0, %1;" : "+f"(t) : "f"(qmax));
     asm("max.NaN.f32 %0, %0, %1;" : "+f"(t) : "f"(qmin));
-    t = __fsub_rn(__fadd_rn(t, 12582912.f), 12582912.f);
-    return __fmul_rn(__fsub_rn(t, zp), scale);
+    const float code = __fsub_rn(__fadd_rn(t, 12582912.f), 12582912.f);
+    signed_value = __fmul_rn(__fsub_rn(copysignf(code, t), zp), scale);
+    return __fmul_rn(__fsub_rn(code, zp), scale);
 }
-__device__ __forceinline__ double affine_value_fast(double y, double, double, double, double, double) { return y; }  // not used: see the dispatch
+__device__ __forceinline__ double affine_value_fast(double y, double, double, double, double, double, double &) { return y; }  // not used: see the dispatch
 // double: `rc` is the correctly rounded reciprocal; two residual corrections make the quotient correctly rounded (the
 // first brings it within an ulp, and Markstein's theorem then gives RN(q + r rc) = RN(y / s)).  Same bits as
 // affine_value, without the division's hundred-odd cycles on the critical path of every stage.  An infinite quotient (y infinite, or

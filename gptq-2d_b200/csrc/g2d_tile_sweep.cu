@@ -478,16 +478,17 @@ __global__ void __launch_bounds__(TTH, 1) tile_sweep_kernel(SweepArgs<F> P, int 
                                 fetch(dg + (uint32_t)((j + 1) * DLD * (int)sizeof(F)), par + par_bytes, kc_next, pa_next);
                                 const F carry = role ? other : (F)0;
                                 const F yv = acc[0] + other;
-                                F z;
-                                if (KIND == G2D_Q_AFFINE) {
-                                    z = DIVIDE == 2   ? affine_value(yv, pa[0], pa[1], P.qmin, P.qmax)
-                                        : DIVIDE == 1 ? affine_value_rcp(yv, pa[0], pa[1], pa[2], P.qmin, P.qmax)
-                                                      : affine_value_fast(yv, pa[0], pa[1], pa[2], P.qmin, P.qmax);
+                                F z, z_out;  // what is stored: z, with the sign of a zero
+                                if (KIND == G2D_Q_AFFINE && DIVIDE == 0) {
+                                    z = affine_value_fast(yv, pa[0], pa[1], pa[2], P.qmin, P.qmax, z_out);
+                                } else if (KIND == G2D_Q_AFFINE) {
+                                    z = DIVIDE == 2 ? affine_value(yv, pa[0], pa[1], P.qmin, P.qmax) : affine_value_rcp(yv, pa[0], pa[1], pa[2], P.qmin, P.qmax);
                                 } else if (KIND == G2D_Q_FORCED) {
                                     z = pa[0];
                                 } else {
                                     z = rint_even(yv);
                                 }
+                                if (KIND != G2D_Q_AFFINE || DIVIDE != 0) z_out = z;
                                 const F carried = (z - yv) + carry;  // completed C (row lanes) or error (column lanes)
                                 const F v = ok ? carried : (F)0;     // lanes without an entry push zero
 #pragma unroll
@@ -497,7 +498,7 @@ __global__ void __launch_bounds__(TTH, 1) tile_sweep_kernel(SweepArgs<F> P, int 
                                 for (int dd = 1; dd < SUB; ++dd) acc[dd - 1] = acc[dd] + kc[dd] * v;
                                 acc[SUB - 1] = last;
                                 store_shared_if(own, carried, ok);
-                                store_shared_if(par + 3 * (uint32_t)sizeof(F), z, ok);  // both lanes of an entry store the same value
+                                store_shared_if(par + 3 * (uint32_t)sizeof(F), z_out, ok);  // both lanes of an entry store the same value
                                 if (RECORD && ok && !role) pre_ptr[(int64_t)p * n] = yv;
                                 own += (uint32_t)(step * (int)sizeof(F));
                                 par += par_bytes;

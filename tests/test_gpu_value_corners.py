@@ -31,6 +31,26 @@ def test_double_quotients_beyond_the_range(value, scale):
     assert torch.equal(fused[~fed], generic[~fed])
 
 
+@pytest.mark.parametrize("qmin, qmax, zero", [(-8, 7, 0.0), (0, 15, 0.0), (-15, 0, 0.0), (0, 15, 8.0), (-8, 7, -0.0), (-8, 7, 3.0)])
+@pytest.mark.parametrize("m, n", [(64, 64), (100, 71), (200, 333)])
+@pytest.mark.parametrize("scale_sign", [1, -1])
+def test_signs_of_zeros(qmin, qmax, zero, m, n, scale_sign):
+    """Rounded values bit for bit as (clamp(round(y / scale + zero)) - zero) * scale gives them, zeros included.  No factor, so y is the
+    input; the quotients are sixteenths of powers of two, exact in any form of the division."""
+    import gptq_2d as G
+    import quantizer_int as Q
+
+    gen = torch.Generator(device="cuda").manual_seed(m + n)
+    scale = torch.full((m, n), 0.125 * scale_sign, device="cuda")
+    y = torch.randint(-200, 201, (m, n), generator=gen, device="cuda") / 16 * scale
+    zeros = torch.full((m, n), zero, device="cuda")
+    z = G.gptq_2d(y, torch.eye(m, device="cuda"), torch.eye(n, device="cuda"), quantizer=functools.partial(Q.affine_quantizer_cuda, qmin=qmin, qmax=qmax),
+                  quantizer_inputs=(scale, zeros))
+    want = (torch.clamp(torch.round(y / scale + zeros), qmin, qmax) - zeros) * scale
+    assert torch.equal(z, want)
+    assert torch.equal(torch.signbit(z), torch.signbit(want))
+
+
 @pytest.mark.parametrize("n", [8, 9, 32])
 def test_packing_under_a_zero_point_that_is_nan(n):
     """Converts to 0 before it is clamped, in whole groups of eight as in ragged ones."""
