@@ -292,7 +292,9 @@ __global__ void __launch_bounds__(TTH, 1) tile_sweep_kernel(SweepArgs<F> P, int 
                 if (owes_right)
                     for (int c = tid; c < TILE * TILE / 4; c += TTH) {
                         const int row = c / (TILE / 4), col = c % (TILE / 4) * 4;
-                        const bool in = j0 + TILE + col < n;  // n is not always a multiple of 4, the row stride is: the tail is zero there
+                        // n is not always a multiple of 4, the row stride is.  The tail of a padded copy is not defined: what is formed
+                        // with it goes to columns from n on, which are not stored, or stored to padding that nothing reads.
+                        const bool in = j0 + TILE + col < n;
                         async16(Ubs + row * LD + col, ug + (j0 + row) * ldu + (in ? j0 + TILE + col : 0), in);
                     }
                 if (owes_down)
@@ -334,10 +336,10 @@ __global__ void __launch_bounds__(TTH, 1) tile_sweep_kernel(SweepArgs<F> P, int 
                     const int idx = t * TTH + tid, r = idx / (TILE / 4), c = (idx % (TILE / 4)) * 4;
 #pragma unroll
                     for (int x = 0; x < 4; ++x) {
-                        vy[t][x] += fy[t][x];
-                        vc[t][x] += fc[t][x];
-                        vy[t][x] += ny[t][x];
-                        vc[t][x] += nc[t][x];
+                        // the two feedbacks first, which are smaller: one rounding at the size of Y (error of 777 x 1333 from float64
+                        // 1.568e-7 with two, 1.556e-7 with one, 1.548e-7 for float32 products throughout)
+                        vy[t][x] += fy[t][x] + ny[t][x];
+                        vc[t][x] += fc[t][x] + nc[t][x];
                     }
                     store4(Ys + r * LD + c, vy[t]);
                     store4(Cs + r * LD + c, vc[t]);
@@ -366,10 +368,8 @@ __global__ void __launch_bounds__(TTH, 1) tile_sweep_kernel(SweepArgs<F> P, int 
                     vy[t] = in ? yg[gi * ld + gj] : (F)0;
                     vc[t] = in ? cg[gi * ld + gj] : (F)0;
                     if (in && yfg != nullptr) {
-                        vy[t] += yfg[gi * ld + gj];
-                        vc[t] += cfg[gi * ld + gj];
-                        if (gets_right) vy[t] += yng[gi * ld + gj];
-                        if (gets_down) vc[t] += cng[gi * ld + gj];
+                        vy[t] += yfg[gi * ld + gj] + (gets_right ? yng[gi * ld + gj] : (F)0);
+                        vc[t] += cfg[gi * ld + gj] + (gets_down ? cng[gi * ld + gj] : (F)0);
                     }
                     vl[t] = (F)0;
                     if (r > c) {
