@@ -73,8 +73,8 @@ def test_absmax_super_entries_match_the_generic_engine(m, n, p, q):
     assert (fused - generic).abs().max().item() <= 1e-12 * w.abs().max().item()
 
 
-# 2^16 states: the cluster search from 2 to 8 bits per step; one step per sequence, the longest whose choices stay in
-# shared memory and one past it, more sequences than clusters run at a time, with and without the wrap-around
+# 2^16 states: the cluster search from 2 to 8 bits per step; few steps and many, with the choices in shared memory and beyond it,
+# more sequences than clusters run at a time, with and without the wrap-around
 @pytest.mark.parametrize("rows, T, K, V, tail", [(1, 2, 2, 1, False), (3, 32, 2, 1, True), (2, 24, 3, 1, True), (3, 16, 4, 2, True), (2, 40, 1, 2, False),
                                                  (1, 16, 8, 1, True), (90, 8, 2, 2, False), (1, 256, 2, 1, True), (1, 1500, 2, 2, False)])
 def test_cluster_search_matches_the_oracle(oracle, rows, T, K, V, tail):
@@ -242,3 +242,23 @@ def test_leading_modes_on_both_sides_of_the_pull(inner):
         factors.append(f.masked_fill(index[:, None] <= index[None, :], 0) + torch.eye(k, device="cuda", dtype=torch.float64))
     want = K.gptq_d_sided(x, factors, super_entry_shape=(2, 2), dense_row_factor=True)
     assert torch.equal(K.gptq_d_sided(x, factors, super_entry_shape=(2, 2), inner_block_size=inner, outer_block_size=0), want)
+
+
+# the longest sequences whose choices stay in the 200 KB of shared memory, and the next: 2 bits per step as 1024 bytes of choices per
+# step beside 32 KB of minima, 4 bits as 512 beside 8 KB
+@pytest.mark.parametrize("T, K, V", [(167, 2, 1), (168, 2, 1), (752, 2, 2), (754, 2, 2)])
+@pytest.mark.parametrize("tail", [False, True])
+def test_cluster_search_where_the_choices_leave_shared_memory(oracle, T, K, V, tail):
+    import quantizer_trellis as Q
+
+    shift, steps = K * V, T // V
+    minima, unit = (1 << 16 >> shift) // 4, 2 if K * V == 2 else 1
+    need = lambda n: 4 * (2 * minima + n * V + n) + (n - 1) * 512 * unit
+    assert (need(steps) <= 200 * 1024) == (T in (167, 752))
+    rng = np.random.default_rng(T)
+    table = rng.standard_normal((1 << 16, V)).astype(np.float32)
+    x = rng.standard_normal((1, T)).astype(np.float32)
+    values, path = oracle.trellis_quantize(x, table, K, tail)
+    out, states = torch.empty(1, T, device="cuda"), torch.empty(1, steps, dtype=torch.int64, device="cuda")
+    Q._trellis_quantize_triton(cuda(x), cuda(table), K, tail, out=out, scale=torch.ones(1, device="cuda"), states=states)
+    assert torch.equal(states.cpu(), torch.from_numpy(path)) and torch.equal(out.cpu(), torch.from_numpy(values))
