@@ -450,6 +450,8 @@ int sweep_pipelined(const g2d_sweep_desc *d, SweepArgs<float> &a, const TcPlanes
 // Updates that share targets and planes follow each other on one stream, so the additions have a fixed order.  Inside a
 // stream capture that finds no lanes (the first call on a device), everything runs in order on the caller's stream.
 int g2d::sweep_overlapped(int waves, bool pushes, cudaStream_t caller, const TileLauncher &tiles, const UpdateLauncher &update) {
+    // Groups of 4, 8 and 16 anti-diagonals, in us: float64 1024 x 1024 2515, 2566, 2607, 2048 x 2048 5775, 5934, 6163; eight float
+    // matrices of 1024 x 1024 1520, 1573, 1657; 200 x 300, 4 x 256 x 256 and 512 x 512 do not care.
     constexpr int kGroup = 8, kLag = 2;
     std::unique_lock<std::mutex> held;
     int status = G2D_OK;

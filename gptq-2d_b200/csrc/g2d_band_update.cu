@@ -330,7 +330,8 @@ int launch_band_update(const BandArgs<F> &args, cudaStream_t stream) {
         band_update_kernel<F><<<grid, BTH, 0, stream>>>(args, nTI, nTJ, (int)args.s1);
         return check_launch();
     }
-    // 64-row tiles when the band's windows are at least as wide as what a tile of that many rows adds to them
+    // 64-row tiles when the band's windows are at least as wide as what a tile of that many rows adds to them (512 x 2048 as 1 x 32 with
+    // the line at 16, 64 and 256 rows: 5880, 5881 and 5695 us)
     BandArgs<F> a = args;
     if (a.mode == BAND_PLAIN) a.P = a.Q = 1;
     const int BM = (a.s1 - a.s0) * a.P >= 64 || a.m > 16 * 65535 ? 64 : 16;

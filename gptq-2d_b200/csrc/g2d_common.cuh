@@ -90,7 +90,9 @@ __device__ __forceinline__ double affine_value_rcp(double y, double scale, doubl
 __device__ __forceinline__ float rounding_reciprocal(float s) {
     float v;
     asm("rcp.approx.f32 %0, %1;" : "=f"(v) : "f"(s));
-    return fmaf(fmaf(-s, v, 1.f), v, v);  // one Newton step: the reciprocal to within half an ulp
+    // one Newton-Raphson step: the correctly rounded reciprocal for every mantissa at the exponents from -100 to 125 that were tried,
+    // those of reciprocal_is_safe (-60 to 59) among them; the intrinsic that rounds correctly by contract takes 4 % of a sweep more
+    return fmaf(fmaf(-s, v, 1.f), v, v);
 }
 __device__ __forceinline__ double rounding_reciprocal(double s) { return __drcp_rn(s); }
 __device__ __forceinline__ bool reciprocal_is_safe(float s) { return fabsf(s) > 1e-18f && fabsf(s) < 1e18f; }

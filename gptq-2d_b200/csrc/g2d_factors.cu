@@ -114,9 +114,10 @@ constexpr int DLDS = FB + 4;    // shared row stride: rows are 16-byte multiples
 template <typename F>
 constexpr int diag_smem = (int)sizeof(F) * (2 * FB * DLDS + FB * FB / 4);
 
-// sqrt(d), its reciprocal and 1 / d of a pivot.  float: from the reciprocal square root approximation with one Newton step and
-// a residual correction each (within an ulp), without the branches of the exact divisions: three of those were 500 of a
-// step's 750 cycles.
+// sqrt(d), its reciprocal and 1 / d of a pivot.  float: from the reciprocal square root approximation with one Newton-Raphson step
+// and a residual correction each, without the branches of the exact divisions: three of those were 500 of a step's 750
+// cycles.  Largest error over all mantissas, at exponents from -126 to 127: root 0.5 ulp (0.75 below 2^-124), inverse root
+// 1.0, inverse 0.5 (of the subnormal where it is one, as for the division).
 __device__ __forceinline__ void pivot_roots(float d, float &root, float &inv_root, float &inv) {
     float r;
     asm("rsqrt.approx.f32 %0, %1;" : "=f"(r) : "f"(d));

@@ -318,8 +318,8 @@ int launch_trinv_tc(int count, const FactorPlanes *problems, cudaStream_t stream
 // factors at the accuracy of a float32 LAPACK factorization: the k range is cut into slices of 128 (added up in registers, round
 // to nearest), and the diagonal entries are left out and updated with a float64 sum of the float panel by CTAs of their own
 // (the first ones of the launch, one per 128 rows).
-// Bound: HBM for factors beyond L2 (8 bytes per entry and group of 256 rows: 123 GB at n = 28672, 20 ms), shared-memory port
-// below (see pair_gemm).  n = 28672 and 8192 together: 73 ms with 128 x 128 tf32 tiles, 36 ms now.
+// Bound: HBM for factors beyond L2 (8 bytes per entry and pair of groups, 512 rows: 61 GB at n = 28672, 10 ms), shared-memory port
+// below (see pair_gemm).  n = 28672 and 8192 together: 73 ms with 128 x 128 tf32 tiles, 36 ms with a group at a time, 28 ms now.
 constexpr int SYRK_SLICE_CHUNKS = 2;  // k = 128 per slice: as many additions into one accumulator as 64 take in tf32
 static_assert(SYRK_TC_K % (2 * KH) == 0, "whole chunks per group");
 

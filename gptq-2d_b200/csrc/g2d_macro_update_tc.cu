@@ -104,7 +104,7 @@ __global__ void __launch_bounds__(PAIR_THREADS, 1) macro_update_tc_kernel(const 
 // on the column only, so two macro rows share it (the product is formed transposed, C^T = E^T L^T, which puts them on the N side),
 // and that of a right product on the row only.  Wide products leave the shared-memory port at 80 % of the tensor rate instead of
 // 60 %, and four of them per CTA hide what a CTA spends on its first loads and its last results: alone on the GPU at 8192 x 28672
-// 233 TFLOP/s with a macro tile per CTA, 294 now (rank 512; 370 at rank 1024).  A target outside the launch's anti-diagonals is multiplied but not written.
+// 233 TFLOP/s with a macro tile per CTA, 304 now (rank 512; 386 at rank 1024).  A target outside the launch's anti-diagonals is multiplied but not written.
 // The targets are walked in RB_I x RB_J blocks, block row after block row, so that the CTAs resident at one time share
 // their row and column strips in L2.
 __global__ void __launch_bounds__(PAIR_THREADS, 1) macro_update_wide_kernel(const __grid_constant__ TcMaps maps, const MacroScales S, const MacroRange R,

@@ -1,5 +1,5 @@
 // Building blocks shared by the tensor-core kernels: mbarrier, TMA and tcgen05 wrappers, the shared-memory operand
-// descriptor of a K-major 128 x 32 fp32 tile with 128-byte swizzle, and the host-side tensor-map encoder.
+// descriptor of a K-major tile of 128-byte rows (64 values of 16 bits) with 128-byte swizzle, and the host-side tensor-map encoder.
 #pragma once
 #include <cuda.h>
 
@@ -34,8 +34,8 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t *bar, uint32_t parity) {
         : "memory");
     return ok != 0;
 }
-// false on time-out.  Between polls the warp sleeps for `nap` nanoseconds: these kernels share SMs with the tile sweep,
-// whose two working warps should not lose issue slots to a spinning neighbour.
+// false on time-out.  Between polls the warp sleeps for `nap` nanoseconds: several CTAs of an update kernel share an SM, and the
+// warps that work should not lose issue slots to those that wait.
 __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, unsigned nap = 32) {
     const long long start = clock64();
     while (!mbar_try_wait(bar, parity)) {

@@ -452,13 +452,14 @@ def run(items: list[dict], process: Callable[[dict], dict], *, rank: int, world:
     assert len(results) == len(items) and done == {(i["block"], i["name"]) for i in items}, "every matrix exactly once"
     by_shape: dict[str, dict] = {}
     for r in results:
-        entry = by_shape.setdefault(f"{r['m']}x{r['n']}", {"count": 0, "prep_ms": 0.0, "sweep_ms": 0.0})
+        entry = by_shape.setdefault(f"{r['m']}x{r['n']}", {"count": 0, "prep_ms": [], "sweep_ms": []})
         entry["count"] += 1
-        entry["prep_ms"] += r.get("prep_ms") or 0.0
-        entry["sweep_ms"] += r.get("sweep_ms") or 0.0
+        for key in ("prep_ms", "sweep_ms"):
+            if r.get(key) is not None:
+                entry[key].append(r[key])
     for entry in by_shape.values():
-        entry["prep_ms"] /= entry["count"]
-        entry["sweep_ms"] /= entry["count"]
+        for key in ("prep_ms", "sweep_ms"):  # None where it was not measured
+            entry[key] = sum(entry[key]) / len(entry[key]) if entry[key] else None
     return {
         "matrices": len(results), "n_gpus": world, "wall_s": max(p["wall_s"] for p in everyone),
         "busy_s": [p["busy_s"] for p in sorted(everyone, key=lambda p: p["rank"])],
