@@ -16,8 +16,8 @@ blocks of 7 matrices at full size, dealt out longest first, no collective on the
 metric, reported under ``layer_set`` with the wall time over ranks.
 Rank 0 prints one JSON line.  ``--impl reference`` times the reference's PyTorch path on the host cores instead, on a
 bounded sample scaled by the algorithmic work: the reference's own ``gptq_2d_torch`` and ``ldl_of_inverse`` when a copy
-of the reference is importable from ``baseline/_ref``, else the CPU restatement under ``oracle/`` (OpenMP sweep, LAPACK
-factorisation); the line says which.
+of the reference is importable from ``baseline/_ref``, else it prints an ``unavailable`` line.  ``cpu_baseline`` of the
+other arm then times the CPU restatement under ``oracle/`` (OpenMP sweep, LAPACK factorisation) and says so.
 """
 from __future__ import annotations
 
@@ -227,16 +227,20 @@ def cpu_layer_estimate(args, sample: int, reference, threads: int) -> dict:
 
 
 def run_reference(args) -> None:
-    """The reference arm: the reference's CPU path (or its oracle port), all host threads, a bounded sample per step."""
+    """The reference arm: the reference's own CPU path, all host threads, a bounded sample per step."""
     rank = int(os.environ.get("RANK", "0"))
     if rank != 0:
         return
     threads = host_threads()
     reference = reference_modules()
-    # the sample is sized so that warm-up + steps end within a few minutes: the port takes about 10 s at 4096 and 1.2 s
-    # at 2048 on 16 cores, the reference's PyTorch path about twice that
+    if reference is None:
+        # a stand-in of this repository's own would not be the reference: the port times `cpu_baseline` of the other arm only
+        print(json.dumps({"impl": "reference", "unavailable": "no installed copy of the reference in baseline/_ref, and none to install it from"}), flush=True)
+        return
+    # the sample is sized so that warm-up + steps end within a few minutes: the reference's PyTorch path takes about 20 s at
+    # 4096 and 2.5 s at 2048 on 16 cores
     budget = 200.0 / max(1, args.steps)
-    sample = args.cpu_sample or (4096 if budget >= (24 if reference is not None else 12) else 2048)
+    sample = args.cpu_sample or (4096 if budget >= 24 else 2048)
     sample = min(sample, args.size)
     times, raw, last = [], [], None
     for step in range(args.warmup + args.steps):
