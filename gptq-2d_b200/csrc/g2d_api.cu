@@ -330,6 +330,18 @@ double near_flops(int64_t m, int64_t n, int s, int t0, int t1, int outer_macro, 
 
 constexpr int kFarLagMacro = 1;  // a far update reaches the macro anti-diagonals from this many past its group's end (its first, short launch has two tile launches of time; measured against 2 and 3: less work for the near updates, the sweep 2 % shorter at 8192 x 8192 and unchanged at 2048 and 4096)
 
+constexpr double kFarBound = 1.5e8;  // entries from which on the far updates bound the sweep
+
+// Whether the tiles of an anti-diagonal and the near update of the one before are one launch (g2d_tile_sweep_step.cu).  The updating CTAs hold an SM
+// each: they keep far updates waiting where those bound the sweep, and too few SMs are left for them beside many tiles.  Apart -> together, by
+// the tiles of the longest anti-diagonal: 32, 2048 x 65536: 84.4 -> 61.7 ms; 64, 4096 x 28672: 31.5 -> 27.4; 96, 6144 x 24000: 34.0 -> 31.7; 128,
+// 8192 x 8192: 12.08 -> 11.64 and 8192 x 16384: 26.0 -> 26.9; 140, 8960 x 8960: 14.3 -> 15.1; far updates as the bound, 8192 x 28672: 55 -> 71.
+bool together(const SweepArgs<float> &a) {
+    const int tiles = a.nI < a.nJ ? a.nI : a.nJ;
+    const double entries = (double)a.m * (double)a.n;
+    return a.nI + a.nJ > 3 && (tiles <= 96 ? entries < kFarBound : tiles <= 128 && entries < 1e8);
+}
+
 // Pipelined schedule (float, tensor cores): one tile launch per tile anti-diagonal, and the feedback between tiles
 // carried by three mechanisms with growing lag, so that only the tile launches remain on the critical path:
 //   * a tile hands the feedback for its lower and its right neighbour on itself: its helper warps form the two products
@@ -362,7 +374,8 @@ int sweep_pipelined(const g2d_sweep_desc *d, SweepArgs<float> &a, const TcPlanes
     // Macro anti-diagonals per far update.  The far updates' share of the SMs grows with m n, the tile launches' time does not: from
     // about 12288 x 12288 on the far updates bound the sweep, and twice the rank costs them less (results leave half as often)
     // than the near updates that it adds (16384 x 16384: 56.3 -> 53.8 ms, 8192 x 28672: 56.7 -> 55.0; 8192 x 8192: 10.9 -> 11.3).
-    const int outer = d->outer_tiles > 0 ? (d->outer_tiles + 1) / 2 : (double)d->m * (double)d->n >= 1.5e8 ? 2 * kDefaultOuterMacro : kDefaultOuterMacro;
+    const bool far_bound = (double)d->m * (double)d->n >= kFarBound;
+    const int outer = d->outer_tiles > 0 ? (d->outer_tiles + 1) / 2 : far_bound ? 2 * kDefaultOuterMacro : kDefaultOuterMacro;
     // what the updates need, where there are any: the smallest sweeps are bound by this host code
     BandTcMaps maps;
     MacroTcMaps far_maps;
@@ -376,29 +389,36 @@ int sweep_pipelined(const g2d_sweep_desc *d, SweepArgs<float> &a, const TcPlanes
         if (status == G2D_OK && cudaEventRecord(lane->prepared, lane->near) != cudaSuccess) status = G2D_ERR_CUDA;
         if (status != G2D_OK) return status;
     }
+    const bool joint = together(a);
     int last_near = -1, last_far = -1;
     for (int s = 0; s < waves; ++s) {
         // what the tiles of s need: every near update up to s - 2, and the far update whose first targets they are
-        if (s >= 2 && last_near >= s - 2 && cudaStreamWaitEvent(stream, lane->near_done[(s - 2) & 7], 0) != cudaSuccess) return G2D_ERR_CUDA;
+        if (!joint && s >= 2 && last_near >= s - 2 && cudaStreamWaitEvent(stream, lane->near_done[(s - 2) & 7], 0) != cudaSuccess) return G2D_ERR_CUDA;
         if (s % 2 == 0 && s / 2 - kFarLagMacro > 0 && (s / 2 - kFarLagMacro) % outer == 0) {
             // the group that ended kFarLagMacro macro anti-diagonals ago: the first part of its update; the group before it: the rest
             const int gf = (s / 2 - kFarLagMacro) / outer - 1;
             if (last_far >= gf && cudaStreamWaitEvent(stream, lane->far_first[gf & 3], 0) != cudaSuccess) return G2D_ERR_CUDA;
             if (gf >= 1 && last_far >= gf - 1 && cudaStreamWaitEvent(stream, lane->far_done[(gf - 1) & 3], 0) != cudaSuccess) return G2D_ERR_CUDA;
         }
+        const auto near_end = [&](int source) {  // of the latest group that has a source tile on the anti-diagonal
+            const int reach = 2 * (((source / 2) / outer + 1) * outer + kFarLagMacro);
+            return reach < waves - 1 ? reach : waves - 1;
+        };
+        const bool step = joint && s >= 1 && s + 1 <= waves - 1;  // with the near update of s - 1
+        if (step && s == 1 && cudaStreamWaitEvent(stream, lane->prepared, 0) != cudaSuccess) return G2D_ERR_CUDA;
         if (timer) timer->begin_on(0, stream);
-        status = launch_tile_sweep<float>(a, s, stream);
+        status = step ? launch_sweep_step(a, s, &maps, planes, s - 1, s + 1, near_end(s - 1), outer, kFarLagMacro, stream) : launch_tile_sweep<float>(a, s, stream);
         if (timer) timer->end();
         if (status != G2D_OK) return status;
-        const bool feeds_near = s + 2 <= waves - 1;
+        if (step && flops) flops[1] += near_flops(d->m, d->n, s - 1, s + 1, near_end(s - 1), outer, kFarLagMacro);
+        const bool feeds_near = !joint && s + 2 <= waves - 1;
         // the last tiles of the macro anti-diagonal W1 - 1 lie on the tile anti-diagonal 2 W1
         const int W1 = s / 2;
         const bool feeds_far = s % 2 == 0 && W1 > 0 && W1 % outer == 0 && W1 + kFarLagMacro <= waves_macro - 1;
         if (!feeds_near && !feeds_far) continue;
         if (cudaEventRecord(lane->swept[s & 7], stream) != cudaSuccess) return G2D_ERR_CUDA;
         if (feeds_near) {
-            const int reach = ((s / 2) / outer + 1) * outer + kFarLagMacro;  // of the latest group that has a source tile here
-            const int t0 = s + 2, t1 = 2 * reach < waves - 1 ? 2 * reach : waves - 1;
+            const int t0 = s + 2, t1 = near_end(s);
             if (cudaStreamWaitEvent(lane->near, lane->swept[s & 7], 0) != cudaSuccess) return G2D_ERR_CUDA;
             if (timer) timer->begin_on(1, lane->near);
             status = launch_band_tc(&maps, planes, d->m, d->n, s, t0, t1, outer, kFarLagMacro, lane->near);

@@ -11,106 +11,28 @@
 // applied as the accumulator is read; the results leave as TMA reductions of 32 x 32 boxes.
 // Every target entry is owned by one CTA of one launch and launches that share targets are ordered by the caller: the result does
 // not depend on scheduling.  Latency bound (one TMA round trip, 12 MMAs, one reduction): several CTAs share an SM.
-#include "g2d_tc.cuh"
+#include "g2d_band_tc.cuh"
 
 namespace g2d {
 
-constexpr int BN = 64;                               // N of the MMA: one tile
-constexpr int BB_BYTES = BN * KH * 2;                // 8 KB
-constexpr int BAND_BYTES = 2 * HTILE_BYTES + 2 * BB_BYTES;  // A_hi, A_lo, B_hi, B_lo: 48 KB, so several CTAs per SM
-constexpr uint32_t BAND_TMEM_COLS = 64;
-
-struct BandJob {
-    CUtensorMap l_hi, l_lo, ut_hi, ut_lo;  // A operands: boxes of 128 rows
-    CUtensorMap et_hi, et_lo, c_hi, c_lo;  // B operands: boxes of 64 rows
-    CUtensorMap y, c;                      // planes that receive the right and the down feedback, boxes of 32 x 32
-    const float *l_scale, *c_scale, *e_scale, *u_scale;
-    int nI, nJ;                            // tiles per column / per row
-    int m, n;
-    int s, t0, t1;
-    int outer_macro, lag_macro;            // > 0: targets that the far update of the source's macro group reaches are left out
-    int *error_flag;
-    const float *l, *u, *e, *c_from;       // for the products with wide tiles: the float values
-    float *y_to, *c_to;                    // and the targets
-    int64_t ldl, ldu, ld;
-};
-
-// The product with a wide source tile (see TcPlanes), in float32 from the float values, by the whole CTA: 128 (r) x 64 (x) results,
-// both operands staged whole where the tensor cores' operands would lie, 4 x 4 results per thread at a time.  Few registers: the
-// kernel's other path shares SMs.  The rare path.
-constexpr int WIDE_R = 128, WIDE_X = 64;
-static_assert((WIDE_R + WIDE_X) * TILE * 4 <= BAND_BYTES, "the float operands fit where the 16-bit ones lie");
-__device__ __forceinline__ void wide_product(const BandJob &job, bool right, int a_row, int b_row, int k0, bool valid_a, bool valid_b, float *As) {
-    float *const Bs = As + TILE * WIDE_R;  // As[k][r], Bs[k][x]
-    const int r_end = right ? job.n : job.m, x_end = right ? job.m : job.n;
-    for (int idx = threadIdx.x; idx < TILE * WIDE_R; idx += TC_THREADS) {  // neighbouring threads along the rows of the source
-        const int r = right ? idx % WIDE_R : idx / TILE, k = right ? idx / WIDE_R : idx % TILE;
-        const int64_t at = a_row + r;
-        As[k * WIDE_R + r] = at < r_end ? (right ? job.u[(int64_t)(k0 + k) * job.ldu + at] : job.l[at * job.ldl + k0 + k]) : 0.f;
-    }
-    for (int idx = threadIdx.x; idx < TILE * WIDE_X; idx += TC_THREADS) {
-        const int x = right ? idx / TILE : idx % WIDE_X, k = right ? idx % TILE : idx / WIDE_X;
-        const int64_t at = b_row + x;
-        Bs[k * WIDE_X + x] = at < x_end ? (right ? job.c_from[at * job.ld + k0 + k] : job.e[(int64_t)(k0 + k) * job.ld + at]) : 0.f;
-    }
-    __syncthreads();
-#pragma unroll 1
-    for (int block = threadIdx.x; block < (WIDE_R / 4) * (WIDE_X / 4); block += TC_THREADS) {
-        const int r0 = (right ? block % (WIDE_R / 4) : block / (WIDE_X / 4)) * 4, x0 = (right ? block / (WIDE_R / 4) : block % (WIDE_X / 4)) * 4;
-        if (!(r0 < TILE ? valid_a : valid_b)) continue;
-        float acc[4][4] = {};
-#pragma unroll 2
-        for (int k = 0; k < TILE; ++k) {
-            const float4 p = *reinterpret_cast<const float4 *>(As + k * WIDE_R + r0), q = *reinterpret_cast<const float4 *>(Bs + k * WIDE_X + x0);
-            const float pv[4] = {p.x, p.y, p.z, p.w}, qv[4] = {q.x, q.y, q.z, q.w};
-#pragma unroll
-            for (int r = 0; r < 4; ++r)
-#pragma unroll
-                for (int x = 0; x < 4; ++x) acc[r][x] = fmaf(pv[r], qv[x], acc[r][x]);
-        }
-#pragma unroll
-        for (int r = 0; r < 4; ++r)
-#pragma unroll
-            for (int x = 0; x < 4; ++x) {
-                const int64_t at_r = a_row + r0 + r, at_x = b_row + x0 + x;
-                if (at_r >= r_end || at_x >= x_end) continue;
-                if (right) job.y_to[at_x * job.ld + at_r] += acc[r][x];
-                else job.c_to[at_r * job.ld + at_x] += acc[r][x];
-            }
-    }
-}
-
 // grid: x = tile column (down jobs) or tile row (right jobs), y = pair slot along the target range, z = 0 down, 1 right
+constexpr uint32_t BAND_TMEM_COLS = 64;
 __global__ void __launch_bounds__(TC_THREADS) band_tc_kernel(const __grid_constant__ BandJob job) {
     extern __shared__ unsigned char tc_smem_raw[];
     __shared__ __align__(8) uint64_t full_bar, accum_bar;
     __shared__ uint32_t tmem_slot;
     __shared__ int failed;
-    const bool right = blockIdx.z != 0;
-    const int fixed = blockIdx.x;                        // J (down) or I (right)
-    const int fixed_count = right ? job.nI : job.nJ, moving_count = right ? job.nJ : job.nI;
-    if (fixed >= fixed_count) return;
-    const int first = max(job.t0 - fixed, 0);
-    const int pair = (first >> 1) + (int)blockIdx.y;     // tiles 2 pair, 2 pair + 1 along the moving index
-    const int t_a = 2 * pair, t_b = 2 * pair + 1;
-    bool valid_a = t_a < moving_count && t_a + fixed >= job.t0 && t_a + fixed <= job.t1;
-    bool valid_b = t_b < moving_count && t_b + fixed >= job.t0 && t_b + fixed <= job.t1;
-    if (!valid_a && !valid_b) return;
-    const int k_tile = job.s - fixed;                    // the source tile along k; it lies before both targets
-    if (k_tile < 0 || k_tile >= moving_count) return;
-    if (job.outer_macro > 0) {
-        // both targets lie in one macro tile
-        const int w_source = (k_tile >> 1) + (fixed >> 1), w_target = pair + (fixed >> 1);
-        const int reach = (w_source / job.outer_macro + 1) * job.outer_macro + job.lag_macro;  // the far update starts here
-        if (w_target >= reach) return;
-    }
+    BandTarget t;
+    if (!band_target(job, blockIdx.x, blockIdx.y, blockIdx.z != 0, t)) return;
+    const bool right = t.right, valid_a = t.valid_a, valid_b = t.valid_b;
+    const int fixed = t.fixed, k_tile = t.k_tile, t_a = t.t_a, t_b = t.t_a + 1;
     const int a_row = t_a * TILE;                        // first of the 128 rows of the A operand
     const int b_row = fixed * TILE;                      // first of the 64 rows of the B operand
     const CUtensorMap *a_hi = right ? &job.ut_hi : &job.l_hi, *a_lo = right ? &job.ut_lo : &job.l_lo;
     const CUtensorMap *b_hi = right ? &job.c_hi : &job.et_hi, *b_lo = right ? &job.c_lo : &job.et_lo;
 
     // asked for here, used behind the set-up: negative where the source tile is wide
-    const float source_scale = right ? job.c_scale[(int64_t)fixed * job.nJ + k_tile] : job.e_scale[(int64_t)k_tile * job.nJ + fixed];
+    const float source_scale = band_source_scale(job, t);
 
     const uint32_t smem_base = (smem_u32(tc_smem_raw) + 1023u) & ~1023u;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -130,7 +52,7 @@ __global__ void __launch_bounds__(TC_THREADS) band_tc_kernel(const __grid_consta
     const uint32_t tmem = tmem_slot;
 
     if (source_scale < 0.f) {
-        wide_product(job, right, a_row, b_row, k_tile * TILE, valid_a, valid_b, reinterpret_cast<float *>(tc_smem_raw + (smem_base - smem_u32(tc_smem_raw))));
+        wide_product<TC_THREADS>(job, right, a_row, b_row, k_tile * TILE, valid_a, valid_b, reinterpret_cast<float *>(tc_smem_raw + (smem_base - smem_u32(tc_smem_raw))));
     } else if (warp == 0) {
         if (lane == 0) {
             const int k = k_tile * TILE;
@@ -244,9 +166,8 @@ int band_tc_prepare(BandTcMaps *opaque, const TcPlanes &pl, float *y, float *c, 
     });
 }
 
-int launch_band_tc(const BandTcMaps *opaque, const TcPlanes &pl, int64_t m, int64_t n, int s, int t0, int t1, int outer_macro, int lag_macro, cudaStream_t stream) {
+bool make_band_job(BandJob &job, const BandTcMaps *opaque, const TcPlanes &pl, int64_t m, int64_t n, int s, int t0, int t1, int outer_macro, int lag_macro) {
     const BandMaps *maps = reinterpret_cast<const BandMaps *>(opaque);
-    BandJob job;
     job.l_hi = maps->l_hi; job.l_lo = maps->l_lo; job.ut_hi = maps->ut_hi; job.ut_lo = maps->ut_lo;
     job.et_hi = maps->et_hi; job.et_lo = maps->et_lo; job.c_hi = maps->c_hi; job.c_lo = maps->c_lo;
     job.y = maps->y; job.c = maps->c;
@@ -255,20 +176,25 @@ int launch_band_tc(const BandTcMaps *opaque, const TcPlanes &pl, int64_t m, int6
     job.m = (int)m; job.n = (int)n;
     const int waves = job.nI + job.nJ - 1;
     if (t1 > waves - 1) t1 = waves - 1;
-    if (t1 < t0) return G2D_OK;
-    if (t0 < s + 2) return G2D_ERR_BAD_ARGUMENT;
+    if (t1 < t0) return false;
     job.s = s; job.t0 = t0; job.t1 = t1;
     job.outer_macro = outer_macro; job.lag_macro = lag_macro;
-    job.error_flag = pl.error_flag;
+    job.error_flag = pl.error_flag; job.wide_count = pl.wide_count;
     job.l = pl.l; job.u = pl.u; job.e = pl.e; job.c_from = pl.c;
     job.y_to = opaque->y; job.c_to = opaque->c;
     job.ldl = pl.ldl; job.ldu = pl.ldu; job.ld = pl.ld;
     // pairs along the moving index that can hold a target: at most (t1 - t0) / 2 + 2, never more than the matrix has
-    const int longest = job.nI > job.nJ ? job.nI : job.nJ;
-    int slots = (t1 - t0) / 2 + 2;
-    if (slots > (longest + 1) / 2) slots = (longest + 1) / 2;
-    dim3 grid((unsigned)longest, (unsigned)slots, 2);
-    band_tc_kernel<<<grid, TC_THREADS, BAND_BYTES + 1024, stream>>>(job);
+    job.longest = job.nI > job.nJ ? job.nI : job.nJ;
+    job.slots = (t1 - t0) / 2 + 2;
+    if (job.slots > (job.longest + 1) / 2) job.slots = (job.longest + 1) / 2;
+    return true;
+}
+
+int launch_band_tc(const BandTcMaps *maps, const TcPlanes &pl, int64_t m, int64_t n, int s, int t0, int t1, int outer_macro, int lag_macro, cudaStream_t stream) {
+    if (t1 >= t0 && t0 < s + 2) return G2D_ERR_BAD_ARGUMENT;
+    BandJob job;
+    if (!make_band_job(job, maps, pl, m, n, s, t0, t1, outer_macro, lag_macro)) return G2D_OK;
+    band_tc_kernel<<<dim3((unsigned)job.longest, (unsigned)job.slots, 2), TC_THREADS, BAND_BYTES + 1024, stream>>>(job);
     return check_launch();
 }
 

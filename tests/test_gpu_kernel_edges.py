@@ -55,6 +55,13 @@ def test_sweep_identity(batch, m, n, dtype, outer):
     assert torch.equal(again, y)
 
 
+# tiles and near updates in one launch: two tiles and three along a side, one tile across the other, ragged last tiles, more jobs than stages per
+# updating CTA, with far updates beside; and both sides of the limit of 128 tiles
+@pytest.mark.parametrize("m, n", [(65, 130), (129, 192), (64, 640), (641, 63), (1000, 1028), (640, 8190), (8192, 8180), (8193, 8256)])
+def test_sweep_identity_where_a_launch_updates_and_sweeps(m, n):
+    test_sweep_identity(1, m, n, "float32", 0)
+
+
 # p * q entries per super-entry: rows and column groups that end inside a flush, one and several column groups per CTA, more columns
 # than a CTA has threads for (q > 128), a single row, more stages than one flush collects
 @pytest.mark.parametrize("m, n, p, q", [(1, 64, 1, 16), (13, 96, 1, 32), (70, 640, 1, 64), (20, 768, 4, 32), (9, 768, 1, 192), (150, 2048, 1, 16), (64, 4096, 4, 128)])
