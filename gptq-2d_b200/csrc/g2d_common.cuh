@@ -355,4 +355,10 @@ int launch_stage_push(const g2d_stage_desc &d, const F *z, int64_t s, int64_t s1
 template <typename F>
 int launch_stage_commit(const g2d_stage_desc &d, const F *z, int64_t s, cudaStream_t stream, const int32_t *skew = nullptr, int64_t z_stride = 0);
 
+// Launches that follow each other on one stream without a wait between them can be programmatic dependent launches: the CTAs of a launch
+// start when those of the one before have all asked for it or ended, and SMs are free.  What a launch before writes is read, and
+// anything is written, only behind the wait, which holds until that launch has ended.
+__device__ __forceinline__ void after_the_launch_before() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void let_the_next_launch_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 }  // namespace g2d

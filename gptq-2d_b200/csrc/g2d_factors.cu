@@ -101,6 +101,48 @@ __device__ __forceinline__ void zero_acc(F (&acc)[8][8]) {
         for (int y = 0; y < 8; ++y) acc[x][y] = (F)0;
 }
 
+// ---- products with one block row (at most 64 rows): 64 x 64 outputs, 4 x 4 per thread ----
+// acc[4][4] += sum_{k < K} A(k, 4 ty ..) B(k, 4 tx ..); both operands are staged whole (float; double in two halves) with
+// coalesced rows, so a CTA waits for memory once: these launches are short and the next step waits for them.
+constexpr int CTH = 256;
+constexpr int CLD = FB + 4;
+template <typename F>
+constexpr int chain_k = sizeof(F) == 4 ? 64 : 32;
+template <typename F, typename LA, typename LB>
+__device__ __forceinline__ void chain_product(F (&acc)[4][4], int K, LA la, LB lb, F *As, F *Bs) {
+    constexpr int CK = chain_k<F>, PER = CK * FB / CTH;
+    const int tid = threadIdx.x, ty = tid >> 4, tx = tid & 15;
+    for (int k0 = 0; k0 < K; k0 += CK) {
+        F ra[PER], rb[PER];
+#pragma unroll
+        for (int t = 0; t < PER; ++t) {
+            const int idx = t * CTH + tid, k = k0 + idx / FB, c = idx % FB;
+            ra[t] = k < K ? la(k, c) : (F)0;
+            rb[t] = k < K ? lb(k, c) : (F)0;
+        }
+        __syncthreads();  // the previous half has been consumed
+#pragma unroll
+        for (int t = 0; t < PER; ++t) {
+            const int idx = t * CTH + tid;
+            As[(idx / FB) * CLD + idx % FB] = ra[t];
+            Bs[(idx / FB) * CLD + idx % FB] = rb[t];
+        }
+        __syncthreads();
+#pragma unroll 16
+        for (int k = 0; k < CK; ++k) {
+            F p[4], q[4];
+#pragma unroll
+            for (int x = 0; x < 4; ++x) p[x] = As[k * CLD + ty * 4 + x];
+#pragma unroll
+            for (int y = 0; y < 4; ++y) q[y] = Bs[k * CLD + tx * 4 + y];
+#pragma unroll
+            for (int x = 0; x < 4; ++x)
+#pragma unroll
+                for (int y = 0; y < 4; ++y) acc[x][y] += p[x] * q[y];
+        }
+    }
+}
+
 // ---- step 1a: factor the diagonal block kb (bs x bs), M_kk = T_kk^T T_kk, and invert T_kk ----
 // One CTA of 256 threads; sixteen rows are factored at a time, the last ones first.  Warp 0 holds their columns 0 .. r0 + 15 in
 // registers, two per lane, and eliminates row after row: the pivot's column goes through shared memory to all lanes, the
@@ -136,13 +178,51 @@ __device__ __forceinline__ void pivot_roots(double d, double &root, double &inv_
     inv = 1.0 / d;
 }
 
+// Float: the CTAs behind the first bring the block row's tiles left of the diagonal up to date with the block rows of its group that are
+// finished, tile j = blockIdx.x - 1.  They only need the diagonal block after it is factored, so they run beside the factorization
+// and a step has two launches.  (With a launch of its own that carried every finished block row into the rest of the group, and launches that wait for
+// the last CTA of the one before: 1024 and 1024 797 us against 693, 8192 and 8192 8.77 ms against 7.64, 8192 and 28672 96.0 - 99.5
+// against 88.3 - 97.5.  An entry gets the same products in the same order, so the results are the same bits.)
+template <typename F>
+__device__ __forceinline__ void update_row_tile(const LdlProblem<F> &Q, int kb, int j, F *As, F *Bs) {
+    F *const a = Q.a;
+    const int64_t n = Q.n, r0 = (int64_t)kb * FB, c0 = (int64_t)j * FB;
+    const int last = min(kb / GROUP * GROUP + GROUP, (int)((n + FB - 1) / FB)) - 1;
+    if (last <= kb) return;
+    const int tid = threadIdx.x, ty = tid >> 4, tx = tid & 15;
+    F left[4][4];  // block rows follow, so all 64 rows of this one are there
+#pragma unroll
+    for (int x = 0; x < 4; ++x)
+#pragma unroll
+        for (int y = 0; y < 4; ++y) left[x][y] = a[(r0 + ty * 4 + x) * n + c0 + tx * 4 + y];
+    for (int k = last; k > kb; --k) {
+        const int64_t o = (int64_t)k * FB;
+        F acc[4][4] = {};
+        chain_product<F>(acc, (int)min((int64_t)FB, n - o), [&](int kk, int i) { return a[(o + kk) * n + r0 + i]; }, [&](int kk, int c) { return a[(o + kk) * n + c0 + c]; }, As, Bs);
+#pragma unroll
+        for (int x = 0; x < 4; ++x)
+#pragma unroll
+            for (int y = 0; y < 4; ++y) left[x][y] -= acc[x][y];
+    }
+#pragma unroll
+    for (int x = 0; x < 4; ++x)
+#pragma unroll
+        for (int y = 0; y < 4; ++y) a[(r0 + ty * 4 + x) * n + c0 + tx * 4 + y] = left[x][y];
+}
+
 template <typename F>
 __global__ void __launch_bounds__(DTH) ldl_diag_kernel(LdlBatch<F> B, int step_down) {
+    after_the_launch_before();
     LDL_PROBLEM(blockIdx.y)
     F *const tinv = Q.tinv;
     int *const flag = Q.flag;
     extern __shared__ __align__(16) unsigned char ldl_smem[];
     F *const S = reinterpret_cast<F *>(ldl_smem);  // the block (lower triangle), later T
+    if constexpr (std::is_same<F, float>::value)
+        if (blockIdx.x > 0) {
+            if ((int)blockIdx.x <= kb) update_row_tile<F>(Q, kb, (int)blockIdx.x - 1, S, S + chain_k<F> * CLD);
+            return;
+        }
     F *const V = S + FB * DLDS;                    // inverse of T, lower triangle
     F *const Wt = V + FB * DLDS;                   // intermediate product of a doubling level
     __shared__ __align__(16) F column[2][DS];  // the pivot's column of the even and odd steps
@@ -257,6 +337,8 @@ __global__ void __launch_bounds__(DTH) ldl_diag_kernel(LdlBatch<F> B, int step_d
         }
         __syncthreads();
     }
+    // the panel's CTAs, which need the inverse, take their places while it is formed
+    let_the_next_launch_start();
     // inverses of the four diagonal blocks, one per warp, column c per lane: once an entry is known it is subtracted from those
     // below, which move up by one register
     if (warp < FB / DS) {
@@ -337,51 +419,10 @@ __global__ void __launch_bounds__(DTH) ldl_diag_kernel(LdlBatch<F> B, int step_d
     if (tid == 0 && bad <= FB && flag) atomicCAS(flag, 0, (int)(o + bad));
 }
 
-// ---- products with one block row (at most 64 rows): 64 x 64 outputs, 4 x 4 per thread ----
-// acc[4][4] += sum_{k < K} A(k, 4 ty ..) B(k, 4 tx ..); both operands are staged whole (float; double in two halves) with
-// coalesced rows, so a CTA waits for memory once: these launches are short and the next step waits for them.
-constexpr int CTH = 256;
-constexpr int CLD = FB + 4;
-template <typename F>
-constexpr int chain_k = sizeof(F) == 4 ? 64 : 32;
-template <typename F, typename LA, typename LB>
-__device__ __forceinline__ void chain_product(F (&acc)[4][4], int K, LA la, LB lb, F *As, F *Bs) {
-    constexpr int CK = chain_k<F>, PER = CK * FB / CTH;
-    const int tid = threadIdx.x, ty = tid >> 4, tx = tid & 15;
-    for (int k0 = 0; k0 < K; k0 += CK) {
-        F ra[PER], rb[PER];
-#pragma unroll
-        for (int t = 0; t < PER; ++t) {
-            const int idx = t * CTH + tid, k = k0 + idx / FB, c = idx % FB;
-            ra[t] = k < K ? la(k, c) : (F)0;
-            rb[t] = k < K ? lb(k, c) : (F)0;
-        }
-        __syncthreads();  // the previous half has been consumed
-#pragma unroll
-        for (int t = 0; t < PER; ++t) {
-            const int idx = t * CTH + tid;
-            As[(idx / FB) * CLD + idx % FB] = ra[t];
-            Bs[(idx / FB) * CLD + idx % FB] = rb[t];
-        }
-        __syncthreads();
-#pragma unroll 16
-        for (int k = 0; k < CK; ++k) {
-            F p[4], q[4];
-#pragma unroll
-            for (int x = 0; x < 4; ++x) p[x] = As[k * CLD + ty * 4 + x];
-#pragma unroll
-            for (int y = 0; y < 4; ++y) q[y] = Bs[k * CLD + tx * 4 + y];
-#pragma unroll
-            for (int x = 0; x < 4; ++x)
-#pragma unroll
-                for (int y = 0; y < 4; ++y) acc[x][y] += p[x] * q[y];
-        }
-    }
-}
-
 // ---- step 1b: block row to the left of the diagonal block: T[kb, j] = T_kk^{-T} M'[kb, j] ----
 template <typename F>
 __global__ void __launch_bounds__(CTH) ldl_trsm_kernel(LdlBatch<F> B, int step_down) {
+    after_the_launch_before();
     LDL_PROBLEM(blockIdx.y)
     const F *const tinv = Q.tinv;
     if ((int)blockIdx.x >= kb) return;
@@ -400,13 +441,41 @@ __global__ void __launch_bounds__(CTH) ldl_trsm_kernel(LdlBatch<F> B, int step_d
 #pragma unroll
         for (int y = 0; y < 4; ++y)
             if (ty * 4 + x < bs) a[(o + ty * 4 + x) * n + c0 + tx * 4 + y] = acc[x][y];
+    let_the_next_launch_start();
     if constexpr (std::is_same<F, float>::value) {
+        const int kb_lo = kb / GROUP * GROUP;
+        if (j >= kb_lo) {
+            // the diagonal block of a block row of the group, which is factored one to three steps on: its own tile is all it takes
+            F gram[4][4] = {};
+            __syncthreads();
+#pragma unroll
+            for (int x = 0; x < 4; ++x)
+#pragma unroll
+                for (int y = 0; y < 4; ++y) As[(ty * 4 + x) * CLD + tx * 4 + y] = acc[x][y];
+            __syncthreads();
+#pragma unroll 16
+            for (int k = 0; k < FB; ++k) {
+                F p[4], q[4];
+#pragma unroll
+                for (int x = 0; x < 4; ++x) p[x] = As[k * CLD + ty * 4 + x];
+#pragma unroll
+                for (int y = 0; y < 4; ++y) q[y] = As[k * CLD + tx * 4 + y];
+#pragma unroll
+                for (int x = 0; x < 4; ++x)
+#pragma unroll
+                    for (int y = 0; y < 4; ++y) gram[x][y] += p[x] * q[y];
+            }
+#pragma unroll
+            for (int x = 0; x < 4; ++x)
+#pragma unroll
+                for (int y = 0; y < 4; ++y)
+                    if (tx * 4 + y <= ty * 4 + x) a[(c0 + ty * 4 + x) * n + c0 + tx * 4 + y] -= gram[x][y];
+        }
         // tensor-core problems: the finished block row, transposed and split, is an operand of the group's trailing
         // update (columns left of the group only); rows beyond a ragged block are zero in acc already
-        const int kb_lo = kb / GROUP * GROUP;
         if (Q.tc && j < kb_lo) {
             const int pair = kb / (2 * GROUP);
-            __half *hi = Q.pt_hi[pair & 1], *lo = Q.pt_lo[pair & 1];
+            __half *hi = pair & 1 ? Q.pt_hi[1] : Q.pt_hi[0], *lo = pair & 1 ? Q.pt_lo[1] : Q.pt_lo[0];
             const int k0 = kb % (2 * GROUP) * FB;
             __syncthreads();
             F *const Ts = As;  // [column][k], row stride 65
@@ -434,28 +503,19 @@ __global__ void __launch_bounds__(CTH) ldl_trsm_kernel(LdlBatch<F> B, int step_d
     }
 }
 
-// ---- step 1c: M'[TI, TJ] -= T[kb, TI]^T T[kb, TJ] for TJ <= TI < kb (lower triangle of tiles) ----
+// ---- step 1c (double): M'[TI, TJ] -= T[kb, TI]^T T[kb, TJ] for TJ <= TI < kb (lower triangle of tiles) ----
 template <typename F>
 __global__ void __launch_bounds__(CTH) ldl_syrk_kernel(LdlBatch<F> B, int step_down) {
+    after_the_launch_before();
     LDL_PROBLEM(blockIdx.y)
-    // tile pairs (TI, TJ), TJ <= TI < kb, in row order.  A tensor-core problem updates only the block rows of its own
-    // group here (TI >= first block row of the group); the rows above wait for the group's update.
-    const int kb_lo = Q.tc ? kb / GROUP * GROUP : 0;
-    const int64_t first = (int64_t)kb_lo * (kb_lo + 1) / 2;
-    if ((int64_t)blockIdx.x >= (int64_t)kb * (kb + 1) / 2 - first) return;
+    // tile pairs (TI, TJ), TJ <= TI < kb, in row order
+    if ((int64_t)blockIdx.x >= (int64_t)kb * (kb + 1) / 2) return;
     __shared__ __align__(16) F As[chain_k<F> * CLD];
     __shared__ __align__(16) F Bs[chain_k<F> * CLD];
-    // linear index -> (TI, TJ) with TJ <= TI: few rows in a group, so walk there; else from the square root
-    int64_t lin = first + blockIdx.x;
-    int TI;
-    if (Q.tc) {
-        TI = kb_lo;
-        while ((int64_t)(TI + 1) * (TI + 2) / 2 <= lin) ++TI;
-    } else {
-        TI = (int)((sqrt(8.0 * (double)lin + 1.0) - 1.0) / 2.0);
-        while ((int64_t)(TI + 1) * (TI + 2) / 2 <= lin) ++TI;
-        while ((int64_t)TI * (TI + 1) / 2 > lin) --TI;
-    }
+    const int64_t lin = blockIdx.x;
+    int TI = (int)((sqrt(8.0 * (double)lin + 1.0) - 1.0) / 2.0);
+    while ((int64_t)(TI + 1) * (TI + 2) / 2 <= lin) ++TI;
+    while ((int64_t)TI * (TI + 1) / 2 > lin) --TI;
     const int TJ = (int)(lin - (int64_t)TI * (TI + 1) / 2);
     const int64_t o = (int64_t)kb * FB, r0 = (int64_t)TI * FB, c0 = (int64_t)TJ * FB;
     const int bs = (int)min((int64_t)FB, n - o);
@@ -641,6 +701,23 @@ static LdlLayout ldl_layout(size_t elem, int64_t n) {
     return lay;
 }
 
+// A kernel of the chain: on its stream behind the one before, as a programmatic dependent launch.
+template <typename F>
+static int launch_chain(void (*kernel)(LdlBatch<F>, int), dim3 grid, int threads, size_t smem, cudaStream_t stream, const LdlBatch<F> &B, int step) {
+    cudaLaunchConfig_t config{};
+    config.gridDim = grid;
+    config.blockDim = dim3((unsigned)threads);
+    config.dynamicSmemBytes = smem;
+    config.stream = stream;
+    cudaLaunchAttribute attribute{};
+    attribute.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attribute.val.programmaticStreamSerializationAllowed = 1;
+    config.attrs = &attribute;
+    config.numAttrs = 1;
+    if (cudaLaunchKernelEx(&config, kernel, B, step) != cudaSuccess) return G2D_ERR_CUDA;
+    return check_launch();
+}
+
 template <typename F>
 int ldl_run(int count, const int64_t *ns, F *const *as, const int *sizes, F *const *outs, int *flags, void *const *workspaces, cudaStream_t caller) {
     LdlBatch<F> B;
@@ -717,25 +794,21 @@ int ldl_run(int count, const int64_t *ns, F *const *as, const int *sizes, F *con
         const int g = s / GROUP;
         // a pair that opens here writes the planes of the pair that closed three groups ago
         if (s % GROUP == GROUP - 1 && recorded[(g + 3) & 3] && cudaStreamWaitEvent(st, lane->rest[(g + 3) & 3], 0) != cudaSuccess) return G2D_ERR_CUDA;
-        ldl_diag_kernel<F><<<dim3(1, count), DTH, diag_smem<F>, st>>>(B, s);
-        if (check_launch() != G2D_OK) return G2D_ERR_CUDA;
-        if (s == 0) break;
-        int64_t panel_tiles = 0, update_tiles = 0;
+        int64_t panel_tiles = 0, row_tiles = 0;  // row_tiles: of block rows with finished ones in their groups
         for (int z = 0; z < count; ++z) {
             const int kb = s - (B.steps - padded_block_rows(ns[z]));
             if (kb <= 0 || (int64_t)kb * FB >= ns[z]) continue;
-            const int kb_lo = B.p[z].tc ? kb / GROUP * GROUP : 0;
-            const int64_t tiles = (int64_t)kb * (kb + 1) / 2 - (int64_t)kb_lo * (kb_lo + 1) / 2;
             panel_tiles = kb > panel_tiles ? kb : panel_tiles;
-            update_tiles = tiles > update_tiles ? tiles : update_tiles;
+            if (B.p[z].tc && kb % GROUP != GROUP - 1 && (int64_t)(kb + 1) * FB < ns[z] && kb > row_tiles) row_tiles = kb;
         }
+        int status = launch_chain<F>(ldl_diag_kernel<F>, dim3((unsigned)(1 + row_tiles), count), DTH, diag_smem<F>, st, B, s);
+        if (status != G2D_OK) return status;
+        if (s == 0) break;
         if (panel_tiles > 0) {
-            ldl_trsm_kernel<F><<<dim3((unsigned)panel_tiles, count), CTH, 0, st>>>(B, s);
-            if (check_launch() != G2D_OK) return G2D_ERR_CUDA;
-        }
-        if (update_tiles > 0) {
-            ldl_syrk_kernel<F><<<dim3((unsigned)update_tiles, count), CTH, 0, st>>>(B, s);
-            if (check_launch() != G2D_OK) return G2D_ERR_CUDA;
+            status = launch_chain<F>(ldl_trsm_kernel<F>, dim3((unsigned)panel_tiles, count), CTH, 0, st, B, s);
+            if (status != G2D_OK) return status;
+            if constexpr (!std::is_same<F, float>::value) status = launch_chain<F>(ldl_syrk_kernel<F>, dim3((unsigned)(panel_tiles * (panel_tiles + 1) / 2), count), CTH, 0, st, B, s);
+            if (status != G2D_OK) return status;
         }
         if (s % GROUP != 0 || !any_tc) continue;
         // the group g is complete: the updates above it, for the tensor-core problems
@@ -767,7 +840,7 @@ int ldl_run(int count, const int64_t *ns, F *const *as, const int *sizes, F *con
         if (closing > 0) {  // the panels are final
             if (cudaEventRecord(lane->panel[g & 3], st) != cudaSuccess || cudaStreamWaitEvent(lane->stream, lane->panel[g & 3], 0) != cudaSuccess)
                 return G2D_ERR_CUDA;
-            int status = launch_syrk_tc(closing, near, lane->stream);
+            status = launch_syrk_tc(closing, near, lane->stream);
             if (status != G2D_OK) return status;
             if (cudaEventRecord(lane->near[g & 3], lane->stream) != cudaSuccess) return G2D_ERR_CUDA;
             if (rest_rows > 0) status = launch_syrk_tc(closing, rest, lane->stream);
@@ -776,7 +849,7 @@ int ldl_run(int count, const int64_t *ns, F *const *as, const int *sizes, F *con
             newest = g;
         }
         if (opens && recorded[(g + 1) & 3] && cudaStreamWaitEvent(st, lane->near[(g + 1) & 3], 0) != cudaSuccess) return G2D_ERR_CUDA;
-        const int status = launch_syrk_tc(targets, next, st);
+        status = launch_syrk_tc(targets, next, st);
         if (status != G2D_OK) return status;
     }
     // everything the side stream did joins the caller's stream before the inverse starts

@@ -8,12 +8,6 @@
 
 namespace g2d {
 
-// Launches that follow each other on one stream without a wait between them are programmatic dependent launches: the CTAs of a launch
-// start when those of the one before have swept their last sub-tiles and SMs are free, and load what no launch writes (factors, scales)
-// while those push, convert and store.  What a launch before writes is read, and anything is written, only behind this wait.
-__device__ __forceinline__ void after_the_launch_before() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void let_the_next_launch_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-
 template <typename F, int KIND>
 __global__ void __launch_bounds__(TTH, 1) sweep_step_kernel(const __grid_constant__ SweepArgs<F> P, int S, int i_first, int tiles, const __grid_constant__ BandJob job) {
     extern __shared__ __align__(16) unsigned char g2d_smem[];

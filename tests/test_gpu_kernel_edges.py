@@ -141,6 +141,13 @@ def test_float_factors_at_group_edges(n, other):
         assert torch.equal(got, K.ldl_of_inverse(m.float()))  # two problems in one pass equal two passes
 
 
+# block rows brought up to date beside the factorization of their diagonal block: groups with one to four block rows, ragged last ones, two
+# problems whose groups end at different block rows
+@pytest.mark.parametrize("n, other", [(64, 65), (127, 256), (255, 449), (448, 2047), (511, 512)])
+def test_float_factors_of_short_groups(n, other):
+    test_float_factors_at_group_edges(n, other)
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
 @pytest.mark.parametrize("n, k", [(1, 0), (64, 5), (64, 16), (64, 60), (130, 122), (400, 85), (1000, 3)])
 def test_the_failing_pivot_is_named(n, k, dtype):
