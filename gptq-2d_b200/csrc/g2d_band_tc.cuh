@@ -1,6 +1,8 @@
 // The near update of the sweep (see g2d_band_tc.cu): what its two kernels share.
 #pragma once
 
+#include <type_traits>
+
 #include "g2d_tc.cuh"
 
 namespace g2d {
@@ -105,9 +107,87 @@ __device__ __forceinline__ void wide_product(const BandJob &job, bool right, int
     }
 }
 
+// ---- the parts of a job, down and right ones apart: which tensor maps a TMA instruction takes is fixed where the code is compiled.
+// (Chosen in the ring's loop, under one lane, compiled code lost boxes of right jobs: their targets stayed without them.  The cause
+// is not known.) ----
+template <bool RIGHT>
+__device__ __forceinline__ void band_load(const BandJob &job, const BandTarget &t, uint32_t dst, uint64_t *full) {
+    const int k = t.k_tile * TILE, a_row = t.t_a * TILE, b_row = t.fixed * TILE;
+    mbar_expect_tx(full, BAND_BYTES);
+    tma_load_2d(dst, RIGHT ? &job.ut_hi : &job.l_hi, k, a_row, full);
+    tma_load_2d(dst + HTILE_BYTES, RIGHT ? &job.ut_lo : &job.l_lo, k, a_row, full);
+    tma_load_2d(dst + 2 * HTILE_BYTES, RIGHT ? &job.c_hi : &job.et_hi, k, b_row, full);
+    tma_load_2d(dst + 2 * HTILE_BYTES + BB_BYTES, RIGHT ? &job.c_lo : &job.et_lo, k, b_row, full);
+}
+__device__ __forceinline__ void band_mma(uint32_t d, uint32_t operands, uint64_t *accum) {
+    constexpr uint32_t DESC = idesc_16(BN, 0);
+    const uint32_t s_a_hi = operands, s_a_lo = s_a_hi + HTILE_BYTES, s_b_hi = s_a_hi + 2 * HTILE_BYTES, s_b_lo = s_b_hi + BB_BYTES;
+#pragma unroll
+    for (int ks = 0; ks < KH / 16; ++ks) {
+        const uint32_t off = ks * 32;  // 16 values = 32 bytes along the swizzled row
+        umma_16(d, umma_desc(s_a_hi + off), umma_desc(s_b_hi + off), DESC, ks == 0 ? 0u : 1u);
+        umma_16(d, umma_desc(s_a_lo + off), umma_desc(s_b_hi + off), DESC, 1u);
+        umma_16(d, umma_desc(s_a_hi + off), umma_desc(s_b_lo + off), DESC, 1u);
+    }
+    umma_commit(accum);  // arrives when every MMA so far has completed
+}
+// What the results of reading warp q (lanes 32 q .. of tensor memory; lanes 0-63 belong to the first tile, 64-127 to the second) are
+// multiplied by
+template <bool RIGHT>
+__device__ __forceinline__ float band_factor(const BandJob &job, const BandTarget &t, int q, float source_scale) {
+    const int target = t.t_a + (q >> 1);  // tile row (down) or column (right) of this warp's results
+    return source_scale * (RIGHT ? job.u_scale[(int64_t)target * job.nJ + t.k_tile] : job.l_scale[(int64_t)target * job.nI + t.k_tile]);
+}
+// The accumulator's rows of this warp, through two boxes per warp where the operands lay, and off as reductions (one group of lane 0)
+template <bool RIGHT>
+__device__ __forceinline__ void band_results(const BandJob &job, const BandTarget &t, int q, int lane, float factor, uint32_t accumulator, uint32_t operands) {
+    const uint32_t boxes = operands + (uint32_t)(q * 2 * BOX_BYTES);
+    const int along = t.t_a * TILE + q * 32;  // row (down) or column (right) of lane 0
+#pragma unroll
+    for (int cb = 0; cb < BN / 32; ++cb) {
+        uint32_t v[32];
+        tmem_load_32(accumulator + ((uint32_t)(q * 32) << 16) + (uint32_t)(cb * 32), v);
+        const uint32_t box = boxes + cb * BOX_BYTES;
+        if (!RIGHT) {
+#pragma unroll
+            for (int g = 0; g < 8; ++g)
+                box_store4(box, lane, g, factor * __uint_as_float(v[4 * g]), factor * __uint_as_float(v[4 * g + 1]), factor * __uint_as_float(v[4 * g + 2]),
+                           factor * __uint_as_float(v[4 * g + 3]));
+        } else {
+            // transposed product: consecutive lanes hold consecutive columns of one row of Y
+#pragma unroll
+            for (int x = 0; x < 32; ++x) box_store1(box, x, lane, factor * __uint_as_float(v[x]));
+        }
+    }
+    box_fence();
+    __syncwarp();
+    if (lane == 0) {
+#pragma unroll
+        for (int cb = 0; cb < BN / 32; ++cb) {
+            const int across = t.fixed * TILE + cb * 32;  // first column (down) or row (right) of the box
+            if (along < (RIGHT ? job.n : job.m) && across < (RIGHT ? job.m : job.n))
+                box_reduce_add(RIGHT ? &job.y : &job.c, boxes + cb * BOX_BYTES, RIGHT ? along : across, RIGHT ? across : along);
+        }
+        box_commit();
+    }
+}
+// The jobs of one of `ctas` CTAs, down jobs first, until body(std::bool_constant<right>, target) is false.
+template <typename Body>
+__device__ __forceinline__ void band_jobs(const BandJob &job, int cta, int ctas, Body body) {
+    const int half = job.longest * job.slots;
+    BandTarget t;
+    int index = cta;
+    for (; index < half; index += ctas)
+        if (band_target(job, index % job.longest, index / job.longest, false, t) && !body(std::false_type{}, t)) return;
+    for (index -= half; index < half; index += ctas)
+        if (band_target(job, index % job.longest, index / job.longest, true, t) && !body(std::true_type{}, t)) return;
+}
+
 // All jobs of a near update, dealt out to `ctas` CTAs of 256 threads that have shared memory to themselves: warp 0 loads, warp 1 issues the
 // MMAs, warps 2 to 5 read the accumulators and send the results off, through BAND_STAGES stages of 48 KB and as many accumulators.  Jobs with
 // wide source tiles come last, by the whole CTA.  Every target entry belongs to one job.
+// A stage and its accumulator go round together: the four reading warps arrive at `empty` once they have read the accumulator and the TMA
+// has read their boxes; the loading lane waits for that and arrives at `full`; the MMAs that overwrite the accumulator wait for `full`.
 constexpr int BAND_STAGES = 3;
 constexpr uint32_t BAND_RING_COLS = 256;
 constexpr int BAND_RING_SMEM = BAND_STAGES * BAND_BYTES + 1024;
@@ -118,12 +198,6 @@ struct BandRing {
 };
 __device__ __forceinline__ void band_ring_cta(const BandJob &job, BandRing &ring, uint32_t smem_base, float *smem_floats, int cta, int ctas) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int total = 2 * job.longest * job.slots;
-    auto next = [&](int &index, BandTarget &t) {  // the next job of this CTA from `index` on
-        for (; index < total; index += ctas)
-            if (band_target(job, index % job.longest, index / job.longest % job.slots, index / job.longest >= job.slots, t)) return true;
-        return false;
-    };
     if (threadIdx.x == 0) {
         for (int s = 0; s < BAND_STAGES; ++s) {
             mbar_init(&ring.full[s], 1);
@@ -142,116 +216,70 @@ __device__ __forceinline__ void band_ring_cta(const BandJob &job, BandRing &ring
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = ring.tmem;
-    BandTarget t;
+    int c = 0;  // jobs so far: stages and accumulators are used in turn
     if (warp == 0) {
         if (lane == 0) {
-            int c = 0;
-            for (int index = cta; next(index, t); index += ctas) {
-                if (band_source_scale(job, t) < 0.f) continue;
+            band_jobs(job, cta, ctas, [&](auto right, const BandTarget &t) {
+                if (band_source_scale(job, t) < 0.f) return true;
                 const int stage = c % BAND_STAGES, round = c / BAND_STAGES;
                 if (round > 0 && !mbar_wait(&ring.empty[stage], (round - 1) & 1)) ring.failed = 1;
-                if (*(volatile int *)&ring.failed) break;
-                const uint32_t dst = smem_base + stage * BAND_BYTES;
-                const int k = t.k_tile * TILE, a_row = t.t_a * TILE, b_row = t.fixed * TILE;
-                mbar_expect_tx(&ring.full[stage], BAND_BYTES);
-                tma_load_2d(dst, t.right ? &job.ut_hi : &job.l_hi, k, a_row, &ring.full[stage]);
-                tma_load_2d(dst + HTILE_BYTES, t.right ? &job.ut_lo : &job.l_lo, k, a_row, &ring.full[stage]);
-                tma_load_2d(dst + 2 * HTILE_BYTES, t.right ? &job.c_hi : &job.et_hi, k, b_row, &ring.full[stage]);
-                tma_load_2d(dst + 2 * HTILE_BYTES + BB_BYTES, t.right ? &job.c_lo : &job.et_lo, k, b_row, &ring.full[stage]);
+                if (*(volatile int *)&ring.failed) return false;
+                band_load<decltype(right)::value>(job, t, smem_base + stage * BAND_BYTES, &ring.full[stage]);
                 ++c;
-            }
+                return true;
+            });
         }
     } else if (warp == 1) {
         if (lane == 0) {
-            int c = 0;
-            for (int index = cta; next(index, t); index += ctas) {
-                if (band_source_scale(job, t) < 0.f) continue;
+            band_jobs(job, cta, ctas, [&](auto, const BandTarget &t) {
+                if (band_source_scale(job, t) < 0.f) return true;
                 const int stage = c % BAND_STAGES, round = c / BAND_STAGES;
                 if (!mbar_wait(&ring.full[stage], round & 1)) ring.failed = 1;
-                if (*(volatile int *)&ring.failed) break;
+                if (*(volatile int *)&ring.failed) return false;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                constexpr uint32_t DESC = idesc_16(BN, 0);
-                const uint32_t d = tmem + stage * BN;
-                const uint32_t s_a_hi = smem_base + stage * BAND_BYTES, s_a_lo = s_a_hi + HTILE_BYTES, s_b_hi = s_a_hi + 2 * HTILE_BYTES, s_b_lo = s_b_hi + BB_BYTES;
-#pragma unroll
-                for (int ks = 0; ks < KH / 16; ++ks) {
-                    const uint32_t off = ks * 32;  // 16 values = 32 bytes along the swizzled row
-                    umma_16(d, umma_desc(s_a_hi + off), umma_desc(s_b_hi + off), DESC, ks == 0 ? 0u : 1u);
-                    umma_16(d, umma_desc(s_a_lo + off), umma_desc(s_b_hi + off), DESC, 1u);
-                    umma_16(d, umma_desc(s_a_hi + off), umma_desc(s_b_lo + off), DESC, 1u);
-                }
-                umma_commit(&ring.accum[stage]);  // arrives when every MMA so far has completed
+                band_mma(tmem + stage * BN, smem_base + stage * BAND_BYTES, &ring.accum[stage]);
                 ++c;
-            }
+                return true;
+            });
             // on time-out, give what is in flight a bounded chance to land before its memory is released
             if (ring.failed && c > 0) mbar_wait(&ring.accum[(c - 1) % BAND_STAGES], ((c - 1) / BAND_STAGES) & 1);
         }
     } else if (warp < 6) {
-        const int q = warp & 3;  // lanes 32 q .. of tensor memory; lanes 0-63 belong to the first tile, 64-127 to the second
-        int c = 0;
-        for (int index = cta; next(index, t); index += ctas) {
+        const int q = warp & 3;
+        band_jobs(job, cta, ctas, [&](auto right, const BandTarget &t) {
+            constexpr bool RIGHT = decltype(right)::value;
             const float source_scale = band_source_scale(job, t);
-            if (source_scale < 0.f) continue;
+            if (source_scale < 0.f) return true;
             const int stage = c % BAND_STAGES, round = c / BAND_STAGES;
             ++c;
             const bool mine = q < 2 ? t.valid_a : t.valid_b;  // warp-uniform
-            const int target = t.t_a + (q >> 1);
-            float factor = 0.f;
-            if (mine) factor = source_scale * (t.right ? job.u_scale[(int64_t)target * job.nJ + t.k_tile] : job.l_scale[(int64_t)target * job.nI + t.k_tile]);
+            const float factor = mine ? band_factor<RIGHT>(job, t, q, source_scale) : 0.f;
             const bool ok = mbar_wait(&ring.accum[stage], round & 1, 64);
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             if (!ok) ring.failed = 1;
-            if (!__all_sync(0xffffffffu, ok && !*(volatile int *)&ring.failed)) break;  // warp-uniform: the tensor-memory loads are warp-wide
+            if (!__all_sync(0xffffffffu, ok && !*(volatile int *)&ring.failed)) return false;  // warp-uniform: the tensor-memory loads are warp-wide
             if (mine) {
-                // the operands have been multiplied: their shared memory takes the results, two boxes per warp
-                const uint32_t boxes = smem_base + stage * BAND_BYTES + (uint32_t)(q * 2 * BOX_BYTES);
-                const int along = t.t_a * TILE + q * 32;  // row (down) or column (right) of lane 0
-#pragma unroll
-                for (int cb = 0; cb < BN / 32; ++cb) {
-                    uint32_t v[32];
-                    tmem_load_32(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(stage * BN + cb * 32), v);
-                    const uint32_t box = boxes + cb * BOX_BYTES;
-                    if (!t.right) {
-#pragma unroll
-                        for (int g = 0; g < 8; ++g)
-                            box_store4(box, lane, g, factor * __uint_as_float(v[4 * g]), factor * __uint_as_float(v[4 * g + 1]), factor * __uint_as_float(v[4 * g + 2]),
-                                       factor * __uint_as_float(v[4 * g + 3]));
-                    } else {
-#pragma unroll
-                        for (int x = 0; x < 32; ++x) box_store1(box, x, lane, factor * __uint_as_float(v[x]));
-                    }
-                }
-                // Chosen before one lane goes on alone: with the choice in the loop below, compiled code lost boxes of right jobs.
-                const CUtensorMap *to = t.right ? &job.y : &job.c;
-                const int along_end = t.right ? job.n : job.m, across_end = t.right ? job.m : job.n;
-                box_fence();
-                __syncwarp();
-                if (lane == 0) {
-#pragma unroll
-                    for (int cb = 0; cb < BN / 32; ++cb) {
-                        const int across = t.fixed * TILE + cb * 32;  // first column (down) or row (right) of the box
-                        if (along < along_end && across < across_end) box_reduce_add(to, boxes + cb * BOX_BYTES, t.right ? along : across, t.right ? across : along);
-                    }
-                    box_commit();
-                    asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
-                }
+                band_results<RIGHT>(job, t, q, lane, factor, tmem + (uint32_t)(stage * BN), smem_base + stage * BAND_BYTES);
+                if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
             }
             // this warp is done with the stage and its accumulator
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();
             if (lane == 0) mbar_arrive(&ring.empty[stage]);
-        }
+            return true;
+        });
         box_wait();
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(BAND_RING_COLS) : "memory");
     if (ring.wide != 0 && !ring.failed)
-        for (int index = cta; next(index, t); index += ctas) {
-            if (band_source_scale(job, t) >= 0.f) continue;
+        band_jobs(job, cta, ctas, [&](auto, const BandTarget &t) {
+            if (band_source_scale(job, t) >= 0.f) return true;
             wide_product<256>(job, t.right, t.t_a * TILE, t.fixed * TILE, t.k_tile * TILE, t.valid_a, t.valid_b, smem_floats);
             __syncthreads();
-        }
+            return true;
+        });
     if (threadIdx.x == 0 && ring.failed && job.error_flag) atomicExch(job.error_flag, 1);
 }
 
