@@ -228,6 +228,8 @@ __device__ __forceinline__ void band_ring_cta(const BandJob &job, BandRing &ring
                 ++c;
                 return true;
             });
+            // the last loads have landed (or had their time to) before their shared memory is released, whatever became of the MMAs
+            for (int back = 1; back <= BAND_STAGES && back <= c; ++back) mbar_wait(&ring.full[(c - back) % BAND_STAGES], ((c - back) / BAND_STAGES) & 1);
         }
     } else if (warp == 1) {
         if (lane == 0) {
