@@ -288,6 +288,7 @@ int launch_trellis(int dtype, int64_t rows, int T, const void *x, const void *ta
 
 template <typename F>
 int launch_tile_sweep(const SweepArgs<F> &args, int S, cudaStream_t stream, int parity = 0);
+bool load_tile_sweep();  // brings the kernel's code to the current device
 
 enum BandMode { BAND_TILE = 0, BAND_PLAIN = 1, BAND_GENERAL = 2 };
 

@@ -74,6 +74,11 @@ int launch_tile_sweep(const SweepArgs<F> &args, int S, cudaStream_t stream, int 
     }
 }
 
+bool load_tile_sweep() {
+    cudaFuncAttributes attributes;
+    return cudaFuncGetAttributes(&attributes, tile_sweep_kernel<float, G2D_Q_AFFINE>) == cudaSuccess;
+}
+
 template int launch_tile_sweep<float>(const SweepArgs<float> &, int, cudaStream_t, int);
 template int launch_tile_sweep<double>(const SweepArgs<double> &, int, cudaStream_t, int);
 
