@@ -15,18 +15,41 @@
 
 namespace g2d {
 
-// grid: x = tile column (down jobs) or tile row (right jobs), y = pair slot along the target range, z = 0 down, 1 right
 constexpr uint32_t BAND_TMEM_COLS = 64;
+// grid: x = tile column (down jobs) or tile row (right jobs), y = pair slot along the target range, z = 0 down, 1 right
+// Which tensor maps an instruction takes is chosen by whole warps, before one lane goes on alone (see g2d_band_tc.cuh).  The text is the
+// kernel's own: short, and with its exits one after the other, since many CTAs have nothing to do (8192 x 28672: 56.9 ms; on
+// the ring's functions, compiled for down and right jobs apart, 57.2).
 __global__ void __launch_bounds__(TC_THREADS) band_tc_kernel(const __grid_constant__ BandJob job) {
     extern __shared__ unsigned char tc_smem_raw[];
     __shared__ __align__(8) uint64_t full_bar, accum_bar;
     __shared__ uint32_t tmem_slot;
     __shared__ int failed;
-    BandTarget t;
-    if (!band_target(job, blockIdx.x, blockIdx.y, blockIdx.z != 0, t)) return;
+    const bool right = blockIdx.z != 0;
+    const int fixed = blockIdx.x;                        // J (down) or I (right)
+    const int fixed_count = right ? job.nI : job.nJ, moving_count = right ? job.nJ : job.nI;
+    if (fixed >= fixed_count) return;
+    const int first = max(job.t0 - fixed, 0);
+    const int pair = (first >> 1) + (int)blockIdx.y;     // tiles 2 pair, 2 pair + 1 along the moving index
+    const int t_a = 2 * pair, t_b = 2 * pair + 1;
+    bool valid_a = t_a < moving_count && t_a + fixed >= job.t0 && t_a + fixed <= job.t1;
+    bool valid_b = t_b < moving_count && t_b + fixed >= job.t0 && t_b + fixed <= job.t1;
+    if (!valid_a && !valid_b) return;
+    const int k_tile = job.s - fixed;                    // the source tile along k; it lies before both targets
+    if (k_tile < 0 || k_tile >= moving_count) return;
+    if (job.outer_macro > 0) {
+        // both targets lie in one macro tile
+        const int w_source = (k_tile >> 1) + (fixed >> 1), w_target = pair + (fixed >> 1);
+        const int reach = (w_source / job.outer_macro + 1) * job.outer_macro + job.lag_macro;  // the far update starts here
+        if (w_target >= reach) return;
+    }
+    const int a_row = t_a * TILE;                        // first of the 128 rows of the A operand
+    const int b_row = fixed * TILE;                      // first of the 64 rows of the B operand
+    const CUtensorMap *a_hi = right ? &job.ut_hi : &job.l_hi, *a_lo = right ? &job.ut_lo : &job.l_lo;
+    const CUtensorMap *b_hi = right ? &job.c_hi : &job.et_hi, *b_lo = right ? &job.c_lo : &job.et_lo;
 
     // asked for here, used behind the set-up: negative where the source tile is wide
-    const float source_scale = band_source_scale(job, t);
+    const float source_scale = right ? job.c_scale[(int64_t)fixed * job.nJ + k_tile] : job.e_scale[(int64_t)k_tile * job.nJ + fixed];
 
     const uint32_t smem_base = (smem_u32(tc_smem_raw) + 1023u) & ~1023u;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -45,38 +68,82 @@ __global__ void __launch_bounds__(TC_THREADS) band_tc_kernel(const __grid_consta
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = tmem_slot;
 
-    auto body = [&](auto right) {
-        constexpr bool RIGHT = decltype(right)::value;
-        if (source_scale < 0.f) {
-            wide_product<TC_THREADS>(job, RIGHT, t.t_a * TILE, t.fixed * TILE, t.k_tile * TILE, t.valid_a, t.valid_b,
-                                     reinterpret_cast<float *>(tc_smem_raw + (smem_base - smem_u32(tc_smem_raw))));
-        } else if (warp == 0) {
-            if (lane == 0) band_load<RIGHT>(job, t, smem_base, &full_bar);
-        } else if (warp == 1) {
-            if (lane == 0) {
-                if (mbar_wait(&full_bar, 0)) {
-                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    band_mma(tmem, smem_base, &accum_bar);
-                } else {
-                    failed = 1;
+    if (source_scale < 0.f) {
+        wide_product<TC_THREADS>(job, right, a_row, b_row, k_tile * TILE, valid_a, valid_b, reinterpret_cast<float *>(tc_smem_raw + (smem_base - smem_u32(tc_smem_raw))));
+    } else if (warp == 0) {
+        if (lane == 0) {
+            const int k = k_tile * TILE;
+            mbar_expect_tx(&full_bar, BAND_BYTES);
+            tma_load_2d(smem_base, a_hi, k, a_row, &full_bar);
+            tma_load_2d(smem_base + HTILE_BYTES, a_lo, k, a_row, &full_bar);
+            tma_load_2d(smem_base + 2 * HTILE_BYTES, b_hi, k, b_row, &full_bar);
+            tma_load_2d(smem_base + 2 * HTILE_BYTES + BB_BYTES, b_lo, k, b_row, &full_bar);
+        }
+    } else if (warp == 1) {
+        if (lane == 0) {
+            if (mbar_wait(&full_bar, 0)) {
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                constexpr uint32_t DESC = idesc_16(BN, 0);
+                const uint32_t s_a_hi = smem_base, s_a_lo = s_a_hi + HTILE_BYTES, s_b_hi = s_a_hi + 2 * HTILE_BYTES, s_b_lo = s_b_hi + BB_BYTES;
+#pragma unroll
+                for (int ks = 0; ks < KH / 16; ++ks) {
+                    const uint32_t off = ks * 32;  // 16 values = 32 bytes along the swizzled row
+                    umma_16(tmem, umma_desc(s_a_hi + off), umma_desc(s_b_hi + off), DESC, ks == 0 ? 0u : 1u);
+                    umma_16(tmem, umma_desc(s_a_lo + off), umma_desc(s_b_hi + off), DESC, 1u);
+                    umma_16(tmem, umma_desc(s_a_hi + off), umma_desc(s_b_lo + off), DESC, 1u);
                 }
-            }
-        } else {
-            const int q = warp & 3;
-            const bool mine = q < 2 ? t.valid_a : t.valid_b;         // warp-uniform
-            const float factor = mine ? band_factor<RIGHT>(job, t, q, source_scale) : 0.f;
-            const bool ok = mbar_wait(&accum_bar, 0, 256);
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            if (!ok) failed = 1;
-            const bool go = __all_sync(0xffffffffu, ok && !failed);  // warp-uniform: the tensor-memory loads are warp-wide
-            if (go && mine) {
-                band_results<RIGHT>(job, t, q, lane, factor, tmem, smem_base);
-                if (lane == 0) box_wait();
+                umma_commit(&accum_bar);  // arrives when every MMA has completed
+            } else {
+                failed = 1;
             }
         }
-    };
-    if (blockIdx.z != 0) body(std::true_type{});
-    else body(std::false_type{});
+    } else {
+        // epilogue warps: lanes 32 q .. 32 q + 31 of tensor memory, q = warp % 4; lanes 0-63 belong to tile a, 64-127 to tile b
+        const int q = warp & 3;
+        const bool mine = q < 2 ? valid_a : valid_b;             // warp-uniform
+        const int target = q < 2 ? t_a : t_b;                    // tile row (down) or column (right) of this warp's results
+        float factor = 0.f;
+        if (mine)
+            factor = source_scale * (right ? job.u_scale[(int64_t)target * job.nJ + k_tile] : job.l_scale[(int64_t)target * job.nI + k_tile]);
+        const bool ok = mbar_wait(&accum_bar, 0, 256);
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        if (!ok) failed = 1;
+        const bool go = __all_sync(0xffffffffu, ok && !failed);  // warp-uniform: the tensor-memory loads are warp-wide
+        if (go && mine) {
+            // the operands have been multiplied: their shared memory takes the results, two boxes per warp
+            const uint32_t boxes = smem_base + (uint32_t)(q * 2 * BOX_BYTES);
+            const int along = a_row + q * 32;                    // row (down) or column (right) of lane 0
+#pragma unroll
+            for (int cb = 0; cb < BN / 32; ++cb) {
+                uint32_t v[32];
+                tmem_load_32(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(cb * 32), v);
+                const uint32_t box = boxes + cb * BOX_BYTES;
+                if (!right) {
+#pragma unroll
+                    for (int g = 0; g < 8; ++g)
+                        box_store4(box, lane, g, factor * __uint_as_float(v[4 * g]), factor * __uint_as_float(v[4 * g + 1]), factor * __uint_as_float(v[4 * g + 2]),
+                                   factor * __uint_as_float(v[4 * g + 3]));
+                } else {
+                    // transposed product: consecutive lanes hold consecutive columns of one row of Y
+#pragma unroll
+                    for (int x = 0; x < 32; ++x) box_store1(box, x, lane, factor * __uint_as_float(v[x]));
+                }
+            }
+            const CUtensorMap *const to = right ? &job.y : &job.c;
+            const int along_end = right ? job.n : job.m, across_end = right ? job.m : job.n;
+            box_fence();
+            __syncwarp();
+            if (lane == 0) {
+#pragma unroll
+                for (int cb = 0; cb < BN / 32; ++cb) {
+                    const int across = b_row + cb * 32;          // first column (down) or row (right) of the box
+                    if (along < along_end && across < across_end) box_reduce_add(to, boxes + cb * BOX_BYTES, right ? along : across, right ? across : along);
+                }
+                box_commit();
+                box_wait();
+            }
+        }
+    }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     if (warp == 1) {

@@ -19,13 +19,14 @@ struct BandJob {
     int nI, nJ;                            // tiles per column / per row
     int m, n;
     int s, t0, t1;
-    int longest, slots;                    // tiles along the longer side; pairs along the moving index that can hold a target
-    const int *wide_count;
     int outer_macro, lag_macro;            // > 0: targets that the far update of the source's macro group reaches are left out
     int *error_flag;
     const float *l, *u, *e, *c_from;       // for the products with wide tiles: the float values
     float *y_to, *c_to;                    // and the targets
     int64_t ldl, ldu, ld;
+    // for the ring
+    int longest, slots;                    // tiles along the longer side; pairs along the moving index that can hold a target
+    const int *wide_count;
 };
 
 // A job: two neighbouring tiles as targets, and their source tile.
@@ -196,7 +197,9 @@ struct BandRing {
     uint32_t tmem;
     int failed, wide;
 };
-__device__ __forceinline__ void band_ring_cta(const BandJob &job, BandRing &ring, uint32_t smem_base, float *smem_floats, int cta, int ctas) {
+// A function of its own: in line with the tiles' code in one kernel it made the tiles slower, the more the longer it was (777 x 1333: 1123 us in
+// line, 1147 with the longer products of wide tiles, 1118 apart).
+static __device__ __noinline__ void band_ring_cta(const BandJob &job, BandRing &ring, uint32_t smem_base, float *smem_floats, int cta, int ctas) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (threadIdx.x == 0) {
         for (int s = 0; s < BAND_STAGES; ++s) {
