@@ -69,7 +69,7 @@ __global__ void __launch_bounds__(TC_THREADS) band_tc_kernel(const __grid_consta
     const uint32_t tmem = tmem_slot;
 
     if (source_scale < 0.f) {
-        wide_product<TC_THREADS>(job, right, a_row, b_row, k_tile * TILE, valid_a, valid_b, reinterpret_cast<float *>(tc_smem_raw + (smem_base - smem_u32(tc_smem_raw))));
+        wide_product(job, right, a_row, b_row, k_tile * TILE, valid_a, valid_b, reinterpret_cast<float *>(tc_smem_raw + (smem_base - smem_u32(tc_smem_raw))));
     } else if (warp == 0) {
         if (lane == 0) {
             const int k = k_tile * TILE;
