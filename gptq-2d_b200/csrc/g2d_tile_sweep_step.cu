@@ -31,7 +31,8 @@ static int launch_step_kind(const SweepArgs<float> &args, int S, const BandJob &
     if (configured.run([&] { return cudaFuncSetAttribute(sweep_step_kernel<float, KIND>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) == cudaSuccess; }) != G2D_OK)
         return G2D_ERR_CUDA;
     const int i_lo = S - args.nJ + 1 > 0 ? S - args.nJ + 1 : 0, i_hi = S + 1 < args.nI ? S + 1 : args.nI, tiles = i_hi - i_lo;
-    const int jobs = 2 * job.longest * job.slots, free_sms = tiles < 147 ? 148 - tiles : 1;
+    const int jobs = 2 * job.longest * job.slots, free_sms = 148 - tiles;  // at most 128 tiles take this schedule
+    if (free_sms < 1) return G2D_ERR_BAD_ARGUMENT;
     cudaLaunchConfig_t config{};
     config.gridDim = dim3((unsigned)(tiles + (jobs < free_sms ? jobs : free_sms)));
     config.blockDim = dim3(TTH);
