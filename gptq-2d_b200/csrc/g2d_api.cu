@@ -393,7 +393,7 @@ int sweep_pipelined(const g2d_sweep_desc *d, SweepArgs<float> &a, const TcPlanes
         if (status == G2D_OK && cudaEventRecord(lane->prepared, lane->near) != cudaSuccess) status = G2D_ERR_CUDA;
         if (status != G2D_OK) return status;
     }
-    const bool joint = together(a);
+    const bool joint = d->reserved != 4 && together(a);
     int last_near = -1, last_far = -1;
     for (int s = 0; s < waves; ++s) {
         // what the tiles of s need: every near update up to s - 2, and the far update whose first targets they are

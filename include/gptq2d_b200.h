@@ -70,7 +70,8 @@ typedef struct g2d_sweep_desc {
     void *workspace;             /* g2d_sweep_workspace_bytes() bytes, 256-byte aligned */
     size_t workspace_bytes;
     int32_t outer_tiles;         /* tile anti-diagonals per far update; 0 selects the default */
-    int32_t reserved;            /* launch schedule: 0 library default, 1 tile, 2 macro, 3 pipelined schedule */
+    int32_t reserved;            /* launch schedule: 0 library default, 1 tile, 2 macro, 3 pipelined schedule, 4 the same with its
+                                    near updates in launches of their own at any size (results are the same bits) */
     int32_t *status;             /* optional device int32: set to -1 when a bounded wait inside a tensor-core update kernel
                                     ran out (the kernels never spin without limit).  Y is then overwritten with NaN as well,
                                     so such a sweep cannot be mistaken for a result.  Never cleared by the library. */

@@ -62,6 +62,11 @@ def test_sweep_identity_where_a_launch_updates_and_sweeps(m, n):
     test_sweep_identity(1, m, n, "float32", 0)
 
 
+# from 1.5e8 entries on: far updates of rank 1024 by default, near updates in launches of their own
+def test_sweep_identity_of_a_matrix_bound_by_far_updates():
+    test_sweep_identity(1, 12250, 12301, "float32", 0)
+
+
 # p * q entries per super-entry: rows and column groups that end inside a flush, one and several column groups per CTA, more columns
 # than a CTA has threads for (q > 128), a single row, more stages than one flush collects
 @pytest.mark.parametrize("m, n, p, q", [(1, 64, 1, 16), (13, 96, 1, 32), (70, 640, 1, 64), (20, 768, 4, 32), (9, 768, 1, 192), (150, 2048, 1, 16), (64, 4096, 4, 128)])

@@ -95,3 +95,64 @@ def test_error_beside_the_float32_schedule(m, n):
         finally:
             G.SWEEP_SCHEDULE = 0
     assert errors[0] <= 1.01 * errors[1], errors[0] / errors[1]
+
+
+# near updates inside the tile launches and in launches of their own: a target gets the same additions in the same order.  One tile across,
+# ragged last tiles, far updates of rank 512 and 1024 beside; every product wide, some of them, none; every quantizer
+@pytest.mark.parametrize("m, n, outer", [(64, 650, 0), (300, 450, 0), (777, 1333, 0), (1030, 901, 16), (2050, 1153, 0)])
+@pytest.mark.parametrize("what", ["rows", "columns", "one row", "not finite", "affine", "round", "forced"])
+def test_both_places_of_the_near_updates(m, n, outer, what):
+    import _abi
+    import gptq_2d as G
+
+    w, l, u = _problem(m, n, m + outer)
+    rows, columns = torch.ones(m, 1, device="cuda"), torch.ones(1, n, device="cuda")
+    if what in ("rows", "columns"):
+        (rows if what == "rows" else columns.T)[1::2] = 2.0 ** -20
+    elif what == "one row":
+        rows[7::60] = 2.0 ** -20
+    step = (w.abs().amax(1, keepdim=True) / 7.5) * rows * columns
+    w, l, u = w * rows * columns, l * rows / rows.T, u / columns.T * columns
+    if what == "not finite":
+        w[m // 3, n // 4] = float("inf")
+    kind, inputs, forced = _abi.Q_AFFINE, (step.expand(w.shape), torch.zeros(1, 1, device="cuda").expand(w.shape)), None
+    if what == "round":
+        kind, inputs, w = _abi.Q_ROUND, (), 150 * w
+    elif what == "forced":
+        kind, inputs, forced = _abi.Q_FORCED, (), torch.round(w / step) * step
+    results = []
+    for schedule in (0, 4):
+        y, _, _, batch_shape = G._prepare_output(w, l, u, False)
+        y_pre = torch.empty_like(y)
+        G.SWEEP_SCHEDULE = schedule
+        try:
+            G._sweep_fused(y, l, u, batch_shape, dict(kind=kind, qmin=-8, qmax=7), inputs, forced_z=forced, y_pre=y_pre, outer_tiles=outer)
+        finally:
+            G.SWEEP_SCHEDULE = 0
+        results.append((y, y_pre))
+    for inside, apart in zip(*results):
+        assert ((inside == apart) | (inside.isnan() & apart.isnan())).all()
+    if what != "not finite":
+        _check_identity(w, l, u, *results[1])
+
+
+def test_near_updates_of_their_own_in_a_graph():
+    import functools
+
+    import gptq_2d as G
+    import quantizer_int as Q
+
+    w, l, u = _problem(456, 328, 5)
+    w[1::2] *= 2.0 ** -20
+    l[1::2] *= 2.0 ** -20
+    l[:, 1::2] *= 2.0 ** 20
+    scale = (w.abs().amax(1, keepdim=True) / 7.5).expand(w.shape).contiguous()
+    options = dict(quantizer=functools.partial(Q.affine_quantizer_cuda, qmin=-8, qmax=7), quantizer_inputs=(scale, torch.zeros_like(scale)))
+    want = [G.gptq_2d(x, l, u, **options) for x in (w, 1.01 * w)]
+    G.SWEEP_SCHEDULE = 4
+    try:
+        replay = G.capture_gptq_2d(w, l, u, **options)
+        for x, z in ((w, want[0]), (1.01 * w, want[1]), (w, want[0])):
+            assert torch.equal(replay(x, l, u, *options["quantizer_inputs"]), z)
+    finally:
+        G.SWEEP_SCHEDULE = 0
