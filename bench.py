@@ -293,6 +293,23 @@ def measure_fp16_peak(device) -> dict:
     return {"burst_tflops": flops / best / 1e9, "sustained_tflops": flops / sustained / 1e9, "how": f"torch.matmul fp16, {n}^3, best of 10 and {count} back to back"}
 
 
+def update_rates(near_ms, near_n, near_flops, far_ms, far_flops, total_flops, peak):
+    """Rates of the near updates and of all updates with launches of their own.  Near updates without launches run inside the tile
+    launches and have no time, hence no rate, of their own."""
+    rate = lambda flops, ms: flops / (ms * 1e-3) / 1e12 if ms > 0 else None
+    of_peak = lambda tflops: tflops / peak if tflops is not None and peak else None
+    near, own_flops = rate(near_flops, near_ms), far_flops + (near_flops if near_n else 0.0)
+    panels = rate(own_flops, near_ms + far_ms)
+    return {
+        "near": {"kernel": "band_tc_kernel (tcgen05 kind::f16, M 128 x N 64, rank-64 updates on a side stream)" if near_n or not near_flops
+                 else "sweep_step_kernel (the same products inside the tile launches)", "achieved": near, "frac": of_peak(near),
+                 "launches": near_n, "algorithmic_flops": near_flops},
+        "panel_gemms": {"what": ("near + far updates" if near_n else "far updates (the near ones have no launches of their own)") + ": their algorithmic flops over their summed stream time",
+                        "achieved": panels, "frac": of_peak(panels), "algorithmic_flops": own_flops,
+                        "share_of_sweep_flops": own_flops / total_flops if total_flops else None},
+    }
+
+
 def main() -> None:
     parser = argparse.ArgumentParser()
     parser.add_argument("--gpus", type=int, default=1)
@@ -503,9 +520,6 @@ def main() -> None:
     pk = peaks()
     tensor_peak = pk["bf16_tflops_sustained"] / 3.0  # fp32-faithful tensor roofline: three products of 16-bit halves per fp32 product
     far_tflops = far_flops / (far_ms * 1e-3) / 1e12 if far_ms > 0 else 0.0
-    near_tflops = near_flops / (near_ms * 1e-3) / 1e12 if near_ms > 0 else 0.0
-    # near updates that run inside the tile launches have no time of their own
-    panel_tflops = ((near_flops if near_ms > 0 else 0.0) + far_flops) / ((near_ms + far_ms) * 1e-3) / 1e12 if near_ms + far_ms > 0 else 0.0
     fp16 = {"burst_tflops": None, "sustained_tflops": None, "how": "skipped"} if args.no_peak_probe else measure_fp16_peak(device)
     measured_peak = fp16["sustained_tflops"] / 3.0 if fp16["sustained_tflops"] else None
     rtn = torch.clamp(torch.round(w / scale), -8, 7) * scale
@@ -519,11 +533,7 @@ def main() -> None:
         "traffic_basis": "ncu capture at 8192 x 8192 (dram__bytes_read.sum + dram__bytes_write.sum of one launch), scaled by algorithmic flops; not measured in this run",
         "peak_basis": f"{pk['source']} bf16 sustained {pk['bf16_tflops_sustained']} TFLOP/s / 3 (three products of 16-bit halves per fp32 product)",
         "peak_measured_fp16": {**fp16, "fp32_faithful_peak": measured_peak, "frac_of_it": far_tflops / measured_peak if measured_peak else None},
-        "near": {"kernel": "band_tc_kernel (tcgen05 kind::f16, M 128 x N 64, rank-64 updates on a side stream; 0 launches: inside the tile launches)", "achieved": near_tflops,
-                 "frac": near_tflops / tensor_peak if tensor_peak else None, "launches": int(near_n), "algorithmic_flops": near_flops},
-        "panel_gemms": {"what": "near + far updates: their algorithmic flops over their summed stream time", "achieved": panel_tflops,
-                        "frac": panel_tflops / tensor_peak if tensor_peak else None, "algorithmic_flops": near_flops + far_flops,
-                        "share_of_sweep_flops": (near_flops + far_flops) / total_flops if total_flops else None},
+        **update_rates(near_ms, int(near_n), near_flops, far_ms, far_flops, total_flops, tensor_peak),
         "far_kernel_alone": {"what": "the same kernel in the macro schedule of the same matrix: one stream, nothing beside it", "achieved": alone_tflops,
                              "frac": alone_tflops / tensor_peak if tensor_peak else None, "launches": int(alone_n),
                              "avg_launch_ms": alone_ms / alone_n if alone_n else None, "algorithmic_flops": alone_flops},
@@ -536,7 +546,7 @@ def main() -> None:
         "timed_in": "separate profiled pass of the same step inside bench.py, one CUDA event pair per launch on the launching stream",
         # the critical path: one tile launch per tile anti-diagonal, each a chain of 7 x 32 dependent rounding stages;
         # bound by that latency, not by memory or arithmetic throughput
-        "critical_path": {"kernel": "tile_sweep_kernel", "launches": int(tile_n), "avg_launch_us": 1e3 * tile_ms / tile_n if tile_n else None,
+        "critical_path": {"kernel": "tile_sweep_kernel" if near_n or not near_flops else "sweep_step_kernel (tiles, and near updates on the SMs they leave free)", "launches": int(tile_n), "avg_launch_us": 1e3 * tile_ms / tile_n if tile_n else None,
                           "bound": "latency"},
     }
 

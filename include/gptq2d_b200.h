@@ -157,7 +157,8 @@ int g2d_sweep_super_entry(const g2d_super_desc *desc, void *stream);
  * bracketed by a CUDA event pair on `stream`; synchronizes the stream before returning, so it cannot be
  * captured.  out[0..2] = total milliseconds of the tile-sweep / near-update / far-update launches,
  * out[3..5] = their launch counts, out[6] = algorithmic flops of the whole sweep m n (m + n - 2) per
- * batch, out[7], out[8] = algorithmic flops executed by the near / far updates. */
+ * batch, out[7], out[8] = algorithmic flops executed by the near / far updates.  Where near updates run inside
+ * the tile launches, their time is part of out[0], and out[1] and out[4] are 0 while out[7] is not. */
 int g2d_sweep_fused_profile(const g2d_sweep_desc *desc, void *stream, double *out);
 
 /* Kernel launches made by this library in this process so far (host-side counter). */

@@ -117,3 +117,14 @@ def test_batch_offsets_follow_broadcasting():
     assert _abi.batch_offsets(torch.zeros(4, 4), torch.Size([])) is None
     assert _abi.batch_offsets(torch.zeros(4, 4), torch.Size([5])) is None  # fully broadcast
     assert _abi.batch_offsets(torch.zeros(2, 1, 4, 4), torch.Size([2, 3])).tolist() == [0, 0, 0, 16, 16, 16]
+
+
+def test_bench_gives_no_rate_to_updates_without_launches():
+    import bench
+
+    inside = bench.update_rates(0.0, 0, 7.5e10, 2.0, 9.0e11, 1.1e12, 400.0)
+    assert inside["near"]["achieved"] is None and inside["near"]["frac"] is None and inside["near"]["algorithmic_flops"] == 7.5e10
+    assert inside["panel_gemms"]["achieved"] == 450.0 and inside["panel_gemms"]["algorithmic_flops"] == 9.0e11
+    apart = bench.update_rates(1.0, 250, 1.0e11, 2.0, 9.0e11, 1.1e12, 400.0)
+    assert apart["near"]["achieved"] == 100.0 and apart["near"]["frac"] == 0.25
+    assert abs(apart["panel_gemms"]["achieved"] - 1.0e12 / 3.0e-3 / 1e12) < 1e-9 and apart["panel_gemms"]["algorithmic_flops"] == 1.0e12
