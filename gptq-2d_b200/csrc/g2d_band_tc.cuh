@@ -11,10 +11,12 @@ constexpr int BN = 64;                               // N of the MMA: one tile
 constexpr int BB_BYTES = BN * KH * 2;                // 8 KB
 constexpr int BAND_BYTES = 2 * HTILE_BYTES + 2 * BB_BYTES;  // A_hi, A_lo, B_hi, B_lo: 48 KB, so several CTAs per SM
 
-struct BandJob {
+struct BandTargetMaps {
     CUtensorMap l_hi, l_lo, ut_hi, ut_lo;  // A operands: boxes of 128 rows
     CUtensorMap et_hi, et_lo, c_hi, c_lo;  // B operands: boxes of 64 rows
     CUtensorMap y, c;                      // planes that receive the right and the down feedback, boxes of 32 x 32
+};
+struct BandFields {
     const float *l_scale, *c_scale, *e_scale, *u_scale;
     int nI, nJ;                            // tiles per column / per row
     int m, n;
@@ -28,6 +30,7 @@ struct BandJob {
     int longest, slots;                    // tiles along the longer side; pairs along the moving index that can hold a target
     const int *wide_count;
 };
+struct BandJob : BandTargetMaps, BandFields {};
 
 // A job: two neighbouring tiles as targets, and their source tile.
 struct BandTarget {
@@ -35,7 +38,7 @@ struct BandTarget {
     int fixed, k_tile, t_a;  // tile column (down) or row (right); tile of the source along k; first target along the moving index
 };
 // x: tile column (down jobs) or tile row (right jobs), y: pair slot along the target range.  False where nothing is to be done.
-__device__ __forceinline__ bool band_target(const BandJob &job, int x, int y, bool right, BandTarget &t) {
+__device__ __forceinline__ bool band_target(const BandFields &job, int x, int y, bool right, BandTarget &t) {
     const int fixed_count = right ? job.nI : job.nJ, moving_count = right ? job.nJ : job.nI;
     if (x >= fixed_count) return false;
     const int first = max(job.t0 - x, 0);
@@ -58,7 +61,7 @@ __device__ __forceinline__ bool band_target(const BandJob &job, int x, int y, bo
     return true;
 }
 // negative where the source tile is wide
-__device__ __forceinline__ float band_source_scale(const BandJob &job, const BandTarget &t) {
+__device__ __forceinline__ float band_source_scale(const BandFields &job, const BandTarget &t) {
     return t.right ? job.c_scale[(int64_t)t.fixed * job.nJ + t.k_tile] : job.e_scale[(int64_t)t.k_tile * job.nJ + t.fixed];
 }
 
@@ -67,7 +70,7 @@ __device__ __forceinline__ float band_source_scale(const BandJob &job, const Ban
 // kernel's other path shares SMs.  The rare path.
 constexpr int WIDE_R = 128, WIDE_X = 64;
 static_assert((WIDE_R + WIDE_X) * TILE * 4 <= BAND_BYTES, "the float operands fit where the 16-bit ones lie");
-__device__ __forceinline__ void wide_product(const BandJob &job, bool right, int a_row, int b_row, int k0, bool valid_a, bool valid_b, float *As) {
+__device__ __forceinline__ void wide_product(const BandFields &job, bool right, int a_row, int b_row, int k0, bool valid_a, bool valid_b, float *As) {
     float *const Bs = As + TILE * WIDE_R;  // As[k][r], Bs[k][x]
     const int r_end = right ? job.n : job.m, x_end = right ? job.m : job.n;
     for (int idx = threadIdx.x; idx < TILE * WIDE_R; idx += TC_THREADS) {  // neighbouring threads along the rows of the source
@@ -133,7 +136,7 @@ __device__ __forceinline__ void wide_stage(float *to, const float *from, int64_t
     }
 }
 template <int THREADS, bool RIGHT>
-__device__ __forceinline__ void wide_product_alone(const BandJob &job, const BandTarget &t, float *As) {
+__device__ __forceinline__ void wide_product_alone(const BandFields &job, const BandTarget &t, float *As) {
     constexpr int PARTS = WIDE_R / 8;                   // eight rows r, four columns x per thread
     static_assert(THREADS == PARTS * (WIDE_X / 4), "a thread has one block of results");
     float *const Bs = As + TILE * WIDE_R;               // As[k][r], Bs[k][x]
@@ -184,13 +187,13 @@ __device__ __forceinline__ void wide_product_alone(const BandJob &job, const Ban
 // (Chosen in the ring's loop, under one lane, compiled code lost boxes of right jobs: their targets stayed without them.  The cause
 // is not known.) ----
 template <bool RIGHT>
-__device__ __forceinline__ void band_load(const BandJob &job, const BandTarget &t, uint32_t dst, uint64_t *full) {
+__device__ __forceinline__ void band_load(const BandTargetMaps &maps, const BandTarget &t, uint32_t dst, uint64_t *full) {
     const int k = t.k_tile * TILE, a_row = t.t_a * TILE, b_row = t.fixed * TILE;
     mbar_expect_tx(full, BAND_BYTES);
-    tma_load_2d(dst, RIGHT ? &job.ut_hi : &job.l_hi, k, a_row, full);
-    tma_load_2d(dst + HTILE_BYTES, RIGHT ? &job.ut_lo : &job.l_lo, k, a_row, full);
-    tma_load_2d(dst + 2 * HTILE_BYTES, RIGHT ? &job.c_hi : &job.et_hi, k, b_row, full);
-    tma_load_2d(dst + 2 * HTILE_BYTES + BB_BYTES, RIGHT ? &job.c_lo : &job.et_lo, k, b_row, full);
+    tma_load_2d(dst, RIGHT ? &maps.ut_hi : &maps.l_hi, k, a_row, full);
+    tma_load_2d(dst + HTILE_BYTES, RIGHT ? &maps.ut_lo : &maps.l_lo, k, a_row, full);
+    tma_load_2d(dst + 2 * HTILE_BYTES, RIGHT ? &maps.c_hi : &maps.et_hi, k, b_row, full);
+    tma_load_2d(dst + 2 * HTILE_BYTES + BB_BYTES, RIGHT ? &maps.c_lo : &maps.et_lo, k, b_row, full);
 }
 __device__ __forceinline__ void band_mma(uint32_t d, uint32_t operands, uint64_t *accum) {
     constexpr uint32_t DESC = idesc_16(BN, 0);
@@ -207,13 +210,13 @@ __device__ __forceinline__ void band_mma(uint32_t d, uint32_t operands, uint64_t
 // What the results of reading warp q (lanes 32 q .. of tensor memory; lanes 0-63 belong to the first tile, 64-127 to the second) are
 // multiplied by
 template <bool RIGHT>
-__device__ __forceinline__ float band_factor(const BandJob &job, const BandTarget &t, int q, float source_scale) {
+__device__ __forceinline__ float band_factor(const BandFields &job, const BandTarget &t, int q, float source_scale) {
     const int target = t.t_a + (q >> 1);  // tile row (down) or column (right) of this warp's results
     return source_scale * (RIGHT ? job.u_scale[(int64_t)target * job.nJ + t.k_tile] : job.l_scale[(int64_t)target * job.nI + t.k_tile]);
 }
 // The accumulator's rows of this warp, through two boxes per warp where the operands lay, and off as reductions (one group of lane 0)
 template <bool RIGHT>
-__device__ __forceinline__ void band_results(const BandJob &job, const BandTarget &t, int q, int lane, float factor, uint32_t accumulator, uint32_t operands) {
+__device__ __forceinline__ void band_results(const BandTargetMaps &maps, const BandFields &job, const BandTarget &t, int q, int lane, float factor, uint32_t accumulator, uint32_t operands) {
     const uint32_t boxes = operands + (uint32_t)(q * 2 * BOX_BYTES);
     const int along = t.t_a * TILE + q * 32;  // row (down) or column (right) of lane 0
 #pragma unroll
@@ -239,14 +242,14 @@ __device__ __forceinline__ void band_results(const BandJob &job, const BandTarge
         for (int cb = 0; cb < BN / 32; ++cb) {
             const int across = t.fixed * TILE + cb * 32;  // first column (down) or row (right) of the box
             if (along < (RIGHT ? job.n : job.m) && across < (RIGHT ? job.m : job.n))
-                box_reduce_add(RIGHT ? &job.y : &job.c, boxes + cb * BOX_BYTES, RIGHT ? along : across, RIGHT ? across : along);
+                box_reduce_add(RIGHT ? &maps.y : &maps.c, boxes + cb * BOX_BYTES, RIGHT ? along : across, RIGHT ? across : along);
         }
         box_commit();
     }
 }
 // The jobs of one of `ctas` CTAs, down jobs first, until body(std::bool_constant<right>, target) is false.
 template <typename Body>
-__device__ __forceinline__ void band_jobs(const BandJob &job, int cta, int ctas, Body body) {
+__device__ __forceinline__ void band_jobs(const BandFields &job, int cta, int ctas, Body body) {
     const int half = job.longest * job.slots;
     BandTarget t;
     int index = cta;
@@ -271,7 +274,11 @@ struct BandRing {
 };
 // A function of its own: in line with the tiles' code in one kernel it made the tiles slower, the more the longer it was (777 x 1333: 1123 us in
 // line, 1147 with the longer products of wide tiles, 1118 apart).
-static __device__ __noinline__ void band_ring_cta(const BandJob &job, BandRing &ring, uint32_t smem_base, float *smem_floats, int cta, int ctas) {
+static __device__ __noinline__ void band_ring_cta(const BandJob &parameters, BandRing &ring, uint32_t smem_base, float *smem_floats, int cta, int ctas) {
+    // in registers: through the reference, every field is loaded again behind every barrier (8192 x 8192: 11.76 -> 11.51 ms; two sweeps of
+    // 4096 x 4096 on two streams: 2607 -> 2560 us each)
+    const BandFields job = parameters;
+    const BandTargetMaps &maps = parameters;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (threadIdx.x == 0) {
         for (int s = 0; s < BAND_STAGES; ++s) {
@@ -299,7 +306,7 @@ static __device__ __noinline__ void band_ring_cta(const BandJob &job, BandRing &
                 const int stage = c % BAND_STAGES, round = c / BAND_STAGES;
                 if (round > 0 && !mbar_wait(&ring.empty[stage], (round - 1) & 1)) ring.failed = 1;
                 if (*(volatile int *)&ring.failed) return false;
-                band_load<decltype(right)::value>(job, t, smem_base + stage * BAND_BYTES, &ring.full[stage]);
+                band_load<decltype(right)::value>(maps, t, smem_base + stage * BAND_BYTES, &ring.full[stage]);
                 ++c;
                 return true;
             });
@@ -336,7 +343,7 @@ static __device__ __noinline__ void band_ring_cta(const BandJob &job, BandRing &
             if (!ok) ring.failed = 1;
             if (!__all_sync(0xffffffffu, ok && !*(volatile int *)&ring.failed)) return false;  // warp-uniform: the tensor-memory loads are warp-wide
             if (mine) {
-                band_results<RIGHT>(job, t, q, lane, factor, tmem + (uint32_t)(stage * BN), smem_base + stage * BAND_BYTES);
+                band_results<RIGHT>(maps, job, t, q, lane, factor, tmem + (uint32_t)(stage * BN), smem_base + stage * BAND_BYTES);
                 if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
             }
             // this warp is done with the stage and its accumulator
