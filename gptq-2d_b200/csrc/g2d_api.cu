@@ -351,8 +351,10 @@ bool together(const SweepArgs<float> &a) {
 //   * a tile hands the feedback for its lower and its right neighbour on itself: its helper warps form the two products
 //     from shared memory while the tile is swept and store them into planes of their own, which the neighbours add as they
 //     load one launch later;
-//   * near update of the tile anti-diagonal s (its tiles as sources, targets from s + 2 on), on a side stream,
-//     concurrent with the tile launch of s + 1;
+//   * near update of the tile anti-diagonal s (its tiles as sources, targets from s + 2 on), beside the tiles of s + 1: on a side stream
+//     or, where together() says so, in the tile launch of s + 1 itself, on the SMs that its tiles leave free.  Those launches follow
+//     each other on one stream as programmatic dependent launches: each waits for the end of the one before it, and what it reads ahead
+//     of that wait (factors, quantizer parameters) no launch of the sweep writes;
 //   * far update of a group of macro anti-diagonals (128 x 128 macro tiles = 2 x 2 tiles; rank 512 or 1024), on a
 //     second side stream, into planes of its own that a tile adds when it loads.  It reaches the macro anti-diagonals
 //     from kFarLagMacro past the group's end, which the tile launches get to two launches after the group's last
@@ -360,8 +362,8 @@ bool together(const SweepArgs<float> &a) {
 //     launches: first the macro anti-diagonals that the tile launches reach before the next group's update (a few
 //     hundred macro tiles: short, and the only part the tile launches have to wait for soon), then everything beyond
 //     them, which the tile launches only need a whole group later.
-// The tile launches run on a stream of the library's own with the highest priority, the near updates below it, the far
-// updates lowest: a CTA slot that frees up goes to the critical path first.  A CTA of the tile sweep fills the registers
+// The tile launches run on a stream of the library's own with the highest priority, near updates with launches of their own below it,
+// the far updates lowest: a CTA slot that frees up goes to the critical path first.  A CTA of the tile sweep fills the registers
 // of its SM (eight warps of up to 233), so no CTA of an update kernel ever shares one with it: the updates run on the SMs
 // that the tile launch of the moment leaves free.  Updates that share target planes are
 // ordered on one stream, so the additions have a fixed order.

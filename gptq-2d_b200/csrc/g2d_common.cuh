@@ -226,7 +226,7 @@ int band_tc_prepare(BandTcMaps *maps, const TcPlanes &planes, float *y, float *c
 int launch_band_tc(const BandTcMaps *maps, const TcPlanes &planes, int64_t m, int64_t n, int s, int t0, int t1, int outer_macro, int lag_macro, cudaStream_t stream);
 // l and u: rows of ldl and ldu values
 int tc_prepare_operands(const float *l, int64_t ldl, const float *u, int64_t ldu, int64_t m, int64_t n, const TcPlanes &planes, cudaStream_t stream);
-// The tiles of anti-diagonal S and the near update of s = S - 1 in one launch (see g2d_tile_sweep.cu)
+// The tiles of anti-diagonal S and the near update of s = S - 1 in one launch (see g2d_tile_sweep_step.cu)
 int launch_sweep_step(const SweepArgs<float> &args, int S, const BandTcMaps *maps, const TcPlanes &planes, int s, int t0, int t1, int outer_macro, int lag_macro,
                       cudaStream_t stream);
 struct MacroTcMaps {

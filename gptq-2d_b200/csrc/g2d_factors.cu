@@ -764,10 +764,11 @@ int ldl_run(int count, const int64_t *ns, F *const *as, const int *sizes, F *con
     if (problems > 0 && launch_equilibrate(problems, equilibrated, st) != G2D_OK) return G2D_ERR_CUDA;
     if (count == 1) B.p[1] = B.p[0];
     if (flags && cudaMemsetAsync(flags, 0, sizeof(int) * count, st) != cudaSuccess) return G2D_ERR_CUDA;
-    // Each step factors one 64-row block row (last first): diagonal block, panel to its left, trailing update.  The
-    // update of a step reaches every row above for an ordinary problem, but only the rows of the step's own group of
-    // GROUP block rows for a tensor-core problem; the rows above the group are updated from the tensor cores, by two groups at
-    // a time (K = 512: an entry of the matrix is read and written half as often as with one, 106 -> 99 ms for the factors of
+    // Each step factors one 64-row block row (last first): diagonal block, panel to its left, trailing update.  For double the
+    // update of a step is a launch that reaches every row above.  For float (tensor-core problems) it is no launch of its own inside
+    // the step's group of GROUP block rows: the panel's CTAs update the group's diagonal blocks, and a block row's other tiles are
+    // brought up to date beside the factorization of its diagonal block; the rows above the group are updated from the tensor cores,
+    // by two groups at a time (K = 512: an entry of the matrix is read and written half as often as with one, 106 -> 99 ms for the factors of
     // n = 28672 and 8192).  A problem's groups pair up as (p + 1, p), p even, whatever it is factored beside.  Look-ahead, so that the
     // latency-bound kernels of the next groups overlap the bulk of the updates:
     //   * group p + 1 updates only the rows of group p (K = 256), on the chain's stream;

@@ -222,8 +222,8 @@ __device__ __forceinline__ F dot(const F *a, const F *b, int64_t ld, int count) 
 template <typename F, int KIND>
 __global__ void __launch_bounds__(PTH) stage_pull_kernel(SuperArgs<F> A) {
     __shared__ F down_s[PULL_ROOM], right_s[PULL_ROOM];
-    asm volatile("griddepcontrol.launch_dependents;");
-    asm volatile("griddepcontrol.wait;" ::: "memory");
+    let_the_next_launch_start();
+    after_the_launch_before();
     const int p = A.p, q = A.q, pq = p * q;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int64_t m = A.m, n = A.n;
