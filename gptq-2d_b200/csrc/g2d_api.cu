@@ -336,14 +336,14 @@ constexpr int kFarLagMacro = 1;  // a far update reaches the macro anti-diagonal
 constexpr double kFarBound = 1.5e8;  // entries from which on the far updates bound the sweep
 
 // Whether the tiles of an anti-diagonal and the near update of the one before are one launch (g2d_tile_sweep_step.cu).  The updating CTAs hold an SM
-// each: they keep far updates waiting where those bound the sweep, and too few SMs are left for them beside many tiles.  Apart -> together, by
-// the tiles of the longest anti-diagonal: 32, 2048 x 65536: 84.4 -> 61.7 ms; 64, 4096 x 28672: 31.5 -> 27.4; 96, 6144 x 24000: 34.0 -> 31.7; 112,
-// 7168 x 13824: 18.7 -> 17.7; 124, 7936 x 12544: 18.4 -> 18.1; 128, 8192 x 8192: 12.18 -> 11.77, 8192 x 9728: 14.40 -> 14.32, 8192 x 10240: 15.14 ->
-// 15.31, 8192 x 12160: 18.1 -> 18.7; 140, 8960 x 8960: 14.3 -> 15.1; far updates as the bound, 8192 x 28672: 55 -> 71.
+// each: they keep far updates waiting where those bound the sweep, and too few SMs are left for them beside many tiles.  Apart -> together, in
+// ms, by the tiles of the longest anti-diagonal: 32, 2048 x 65536: 84.2 -> 62.3; 64, 4096 x 28672: 31.7 -> 27.8; 96, 6144 x 22000: 31.5 -> 29.9;
+// 112, 7168 x 20900: 34.7 -> 32.3; 128, 8192 x 8192: 12.23 -> 11.55, 8192 x 12160: 18.15 -> 17.89, 8192 x 18200: 32.3 -> 31.5; 132, 8448 x 8448: 13.0 ->
+// 12.4, 8448 x 12000: 19.4 -> 19.9; 136, 8704 x 12000: 19.9 -> 21.8; 140, 8960 x 8960: 14.5 -> 14.7; far updates as the bound, 8192 x 28672: 55 -> 71.
+// Four sweeps on two streams: 8192 x 8192 40.3 -> 39.2, 8192 x 14336 81.5 -> 78.7.
 bool together(const SweepArgs<float> &a) {
     const int tiles = a.nI < a.nJ ? a.nI : a.nJ;
-    const double entries = (double)a.m * (double)a.n;
-    return a.nI + a.nJ > 3 && entries < (tiles <= 96 ? kFarBound : tiles <= 124 ? 1e8 : tiles <= 128 ? 8e7 : 0.);
+    return a.nI + a.nJ > 3 && tiles <= 128 && (double)a.m * (double)a.n < kFarBound;
 }
 
 // Pipelined schedule (float, tensor cores): one tile launch per tile anti-diagonal, and the feedback between tiles
