@@ -58,20 +58,26 @@ __device__ __forceinline__ float affine_value_rcp(float y, float scale, float zp
     t = t > qmax ? qmax : t;
     return __fmul_rn(__fsub_rn(t, zp), scale);
 }
-// The same for bounds that are integers below 2^22 in size: then clamping and rounding commute, and a clamped value is
+// The stage loop's form, for bounds that are integers below 2^22 in size: then clamping and rounding commute, and a clamped value is
 // rounded half to even by adding and subtracting 1.5 * 2^23, eight cycles instead of the conversion unit's twenty-odd.
-// NaN stays NaN as with the comparisons above.  The sum of the two has lost the sign of a zero (a quotient of -0.3 rounds to -0), so
-// `signed_value` is formed once more from a code that has it, beside the chain that goes on with the value.
-__device__ __forceinline__ float affine_value_fast(float y, float scale, float zp, float rc, float qmin, float qmax, float &signed_value) {
+// NaN stays NaN as with the comparisons above.  Returns code - zp, from which the chain goes on with one multiply-add, and in `clamped` what
+// affine_value_after needs to form the value away from the chain: the difference code + 1.5 * 2^23 - 1.5 * 2^23 has lost the sign of a zero
+// (a quotient of -0.3 rounds to -0).  ZERO: the zero point is +0, which leaves two additions out of the chain.
+template <bool ZERO>
+__device__ __forceinline__ float affine_steps_fast(float y, float scale, float zp, float rc, float qmin, float qmax, float &clamped) {
     const float q0 = y * rc;
-    float t = __fadd_rn(fmaf(fmaf(-q0, scale, y), rc, q0), zp);
+    float t = fmaf(fmaf(-q0, scale, y), rc, q0);
+    if (!ZERO) t = __fadd_rn(t, zp);
     asm("min.NaN.f32 %0, %0, %1;" : "+f"(t) : "f"(qmax));
     asm("max.NaN.f32 %0, %0, %1;" : "+f"(t) : "f"(qmin));
+    clamped = t;
     const float code = __fsub_rn(__fadd_rn(t, 12582912.f), 12582912.f);
-    signed_value = __fmul_rn(__fsub_rn(copysignf(code, t), zp), scale);
-    return __fmul_rn(__fsub_rn(code, zp), scale);
+    return ZERO ? code : __fsub_rn(code, zp);
 }
-__device__ __forceinline__ double affine_value_fast(double y, double, double, double, double, double, double &) { return y; }  // not used: see the dispatch
+__device__ __forceinline__ float affine_value_after(float clamped, float scale, float zp, bool zero) {
+    const float t = zero ? __fadd_rn(clamped, 0.f) : clamped;  // the addition that ZERO has left out: -0 + 0 = 0
+    return __fmul_rn(__fsub_rn(copysignf(__fsub_rn(__fadd_rn(t, 12582912.f), 12582912.f), t), zp), scale);
+}
 // double: `rc` is the correctly rounded reciprocal; two residual corrections make the quotient correctly rounded (the
 // first brings it within an ulp, and Markstein's theorem then gives RN(q + r rc) = RN(y / s)).  Same bits as
 // affine_value, without the division's hundred-odd cycles on the critical path of every stage.  An infinite quotient (y infinite, or
@@ -95,8 +101,8 @@ __device__ __forceinline__ float rounding_reciprocal(float s) {
     return fmaf(fmaf(-s, v, 1.f), v, v);
 }
 __device__ __forceinline__ double rounding_reciprocal(double s) { return __drcp_rn(s); }
-__device__ __forceinline__ bool reciprocal_is_safe(float s) { return fabsf(s) > 1e-18f && fabsf(s) < 1e18f; }
-__device__ __forceinline__ bool reciprocal_is_safe(double s) { return fabs(s) > 1e-150 && fabs(s) < 1e150; }
+__device__ __forceinline__ bool reciprocal_is_safe(float s) { return (fabsf(s) > 1e-18f) & (fabsf(s) < 1e18f); }
+__device__ __forceinline__ bool reciprocal_is_safe(double s) { return (fabs(s) > 1e-150) & (fabs(s) < 1e150); }
 
 // Largest value over a warp, in every lane.  Non-negative floats order like their bit patterns, so float takes one reduction
 // instruction; NaN counts as the smallest, as fmax has it.

@@ -4,14 +4,14 @@
     F *Cs = Ys + TILE * LD;                   // down feedback; the completed C once a sub-tile is swept
     F *LUs = Cs + TILE * LD;                  // strict lower part: L[I, I]; strict upper part: U[J, J]
     F *Dg = LUs + TILE * LD;                  // zero-padded diagonal blocks L[a, a] and U[b, b]^T, strictly lower, between rows of zeros
-    F *Par = Dg + DROWS * DLD;                // [NSUB][SUB][PLD][4]: scale, zero point, reciprocal, rounded value of the entries of the sub-tiles being swept
-    F *Ubs = Par + NSUB * SUB * PLD * 4;      // float only, pipelined schedule: U[J, J + 1], the right neighbour's coupling block
+    F *Par = Dg + DROWS * DLD;                // twice (by turns) two planes [NSUB][SUB][PLD][2]: scale and reciprocal, zero point and result of the entries of the sub-tiles being swept
+    F *Ubs = Par + 4 * PPLANE;                // float only, pipelined schedule: U[J, J + 1], the right neighbour's coupling block
     F *Lbs = Ubs + TILE * LD;                 // the same: L[I + 1, I], the lower neighbour's
     F *Yns = Lbs + TILE * LD;                 // the same: the feedback for the right neighbour, C[I, J] U[J, J + 1], growing sub-tile by sub-tile
     F *Cns = Yns + TILE * LD;                 // and for the lower one, L[I + 1, I] E[I, J]
-    __shared__ unsigned row_max[TILE];
-    __shared__ __align__(16) unsigned column_max[TTH / 32][TILE];
-    __shared__ unsigned fast_div[NSUB];       // every scale of the sub-tile allows the division by reciprocal
+    __shared__ unsigned row_max[TILE], column_max[TILE];  // see last_extremes
+    __shared__ int early_exponent[2];         // of E and C without the sub-tile that is swept last
+    __shared__ unsigned fast_div[2][NSUB];       // bit 0: every scale of the sub-tile allows the division by reciprocal; bit 1: its zero points are +0
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int k = lane & 15, role = lane >> 4;
@@ -41,81 +41,21 @@
         // neighbour push (pipelined schedule): what this tile receives and what it owes
         F *yng = P.yn ? P.yn + batch * m * ld : nullptr, *cng = P.yn ? P.cn + batch * m * ld : nullptr;
         const bool gets_right = yng != nullptr && J > 0, gets_down = yng != nullptr && I > 0;
+        // where the feedback for the neighbours belongs, and how much of it is inside the matrix
+        F *const yn_out = yng + i0 * ld + j0 + TILE, *const cn_out = cng + (i0 + TILE) * ld + j0;
+        const bool push_vec = ld % 4 == 0 && reinterpret_cast<uintptr_t>(yng) % (4 * sizeof(F)) == 0;
+        const int cols_right = (int)min((int64_t)TILE, n - j0 - TILE), rows_below = (int)min((int64_t)TILE, m - i0 - TILE);
         const bool owes_right = yng != nullptr && J + 1 < P.nJ, owes_down = yng != nullptr && I + 1 < P.nI;
 
-        // ---- quantizer parameters, prepared by the helper warps ----
-        // Helper warp h prepares the parameters of the sub-tile that sweeping warp h takes next: a lane has the entries
-        // (2 x + lane / 16, lane % 16).  Scale, zero point and, for the affine quantizer, the reciprocal of the scale wait
-        // in shared memory by entry, with the warp-wide decision whether every scale is in the range where the reciprocal
-        // form of the division is safe.  The loads are issued one sub-tile anti-diagonal ahead and travel while the helper
-        // does its other work.
-        constexpr int PR = SUB * SUB / 32;  // entries per helper lane
-        F sc[PR], zp[PR], rc[PR];
-        bool pfast = true;
-        unsigned pvalid = 0;  // entries inside the matrix
-        auto fetch_params = [&](int w_next) {
-            const int b = w_next - helper;
-            if (b < 0 || b >= NSUB || KIND == G2D_Q_ROUND) return;
-            const int r = helper * SUB + role, c = b * SUB + k;  // first entry; the others follow two rows apart
-            // entries outside the matrix load a value from inside it (no select waits on the load here) and get their
-            // neutral parameters in finish_params
-            const int rc_ = min(r, rows_in - 1), cc = min(c, cols_in - 1);
-            pvalid = 0;
-#pragma unroll
-            for (int x = 0; x < PR; ++x) pvalid |= (r + 2 * x < rows_in && c < cols_in) ? (1u << x) : 0u;
-            if (KIND == G2D_Q_AFFINE) {
-                const F *ps = sg + (i0 + rc_) * P.srs + (j0 + cc) * P.scs, *pz = zg + (i0 + rc_) * P.zrs + (j0 + cc) * P.zcs;
-                const int64_t ss = 2 * P.srs, zs = 2 * P.zrs;
-#pragma unroll
-                for (int x = 0; x < PR; ++x) {
-                    sc[x] = load_now(ps);
-                    zp[x] = load_now(pz);
-                    if (r + 2 * x + 2 < rows_in) {
-                        ps += ss;
-                        pz += zs;
-                    }
-                }
-            } else {
-                const F *pf = fg + (i0 + rc_) * n + j0 + cc;
-#pragma unroll
-                for (int x = 0; x < PR; ++x) {
-                    sc[x] = load_now(pf);
-                    if (r + 2 * x + 2 < rows_in) pf += 2 * n;
-                }
-            }
-        };
-        auto finish_params = [&](int w_next) {
-            if (w_next - helper < 0 || w_next - helper >= NSUB) return;
-            bool normal = true;
-#pragma unroll
-            for (int x = 0; x < PR; ++x) {
-                const bool in = (pvalid >> x) & 1u;
-                if (KIND == G2D_Q_AFFINE) {
-                    sc[x] = in ? sc[x] : (F)1;
-                    zp[x] = in ? zp[x] : (F)0;
-                    normal = normal && reciprocal_is_safe(sc[x]);
-                    rc[x] = rounding_reciprocal(sc[x]);
-                } else if (KIND == G2D_Q_FORCED) {
-                    sc[x] = in ? sc[x] : (F)0;
-                }
-            }
-            pfast = __all_sync(0xffffffffu, normal);
-        };
-        auto store_params = [&](int w_next) {
-            if (w_next - helper < 0 || w_next - helper >= NSUB) return;
-            F *dst = Par + ((helper * SUB + role) * PLD + k) * 4;
-#pragma unroll
-            for (int x = 0; x < PR; ++x) {
-                if (KIND == G2D_Q_AFFINE) {
-                    const F v[4] = {sc[x], zp[x], rc[x], (F)0};
-                    store4(dst + 2 * x * PLD * 4, v);
-                } else if (KIND == G2D_Q_FORCED) {
-                    dst[2 * x * PLD * 4] = sc[x];
-                }
-            }
-            if (lane == 0) fast_div[helper] = pfast ? 1u : 0u;
-        };
-        if (!sweeper) fetch_params(0);
+        Tile<F> tile;
+        tile.i0 = i0; tile.j0 = j0; tile.n = n; tile.ld = ld; tile.rows = rows_in; tile.cols = cols_in;
+        tile.y = yg; tile.scale = sg; tile.zero = zg; tile.forced = fg;
+        tile.srs = P.srs; tile.scs = P.scs; tile.zrs = P.zrs; tile.zcs = P.zcs;
+        tile.unfinished = pre == nullptr && P.small_integer_bounds;
+        tile.zvec = ld % 4 == 0 && reinterpret_cast<uintptr_t>(yg) % (4 * sizeof(F)) == 0;
+        const auto params_of = [&](int w) { return Par + (w & 1) * 2 * PPLANE; };
+        Params<F> params;
+        if (!sweeper) fetch_params<F, KIND>(tile, 0, helper, lane, params);
         constexpr bool PUSH = sizeof(F) == sizeof(float);  // the neighbour push exists for float (pipelined schedule) only
 
         // ---- load the tile ----
@@ -276,8 +216,7 @@
             }
         }
         if (!sweeper) {
-            finish_params(0);
-            store_params(0);
+            finish_params<F, KIND>(tile, params_of(0), &fast_div[0][helper], 0, helper, lane, params);
         }
         __syncthreads();
         // Sweep of the sub-tiles: sweeping warp a takes the sub-tiles of row a, one per sub-tile anti-diagonal.  Lane k of the
@@ -295,97 +234,77 @@
         // four unrolled stages (one branch per stage costs 40 cycles): about 120 cycles per stage for one warp on its
         // scheduler, 150 for two, against 168 with wrapped addresses and selects.
         // The two roles run the same sequence of barriers from loops of their own, so that neither holds the other's registers.
+        // Operands of the tensor-core updates: fp16 pairs of E (transposed) and of the completed C under the tile's scales, eight entries
+        // per thread and store.  C along its rows; E transposed: a thread gathers eight rows of one column (consecutive threads take
+        // consecutive columns, so the shared-memory reads do not collide) and writes them as one vector of a row of E^T.  A
+        // row's last vector may reach into its padding.  Zeros where the factor is.
+        auto split_c = [&](int r, int c, float by) {
+            if constexpr (PUSH) {
+                const int64_t at = (i0 + r) * P.ldn + j0 + c;
+                split8<false>(Cs + r * LD + c, by, P.c_hi + at, P.c_lo + at, r < rows_in && c < cols_in);
+            }
+        };
+        auto split_e = [&](int r, int c, float by) {
+            if constexpr (PUSH) {
+                const int64_t at = (j0 + c) * P.ldm + i0 + r;
+                split8<true>(Ys + r * LD + c, by, P.et_hi + at, P.et_lo + at, r < rows_in && c < cols_in);
+            }
+        };
         if (sweeper) {
             const int sub_a = number, r0 = sub_a * SUB;
-            const int par0 = (sub_a * SUB * PLD + (role ? k * PLD - k : k - k * PLD)) * 4, par_step = (role ? 1 : PLD) * 4;
+#pragma unroll 1
             for (int w = 0; w < 2 * NSUB - 1; ++w) {
                 const int b = w - sub_a;
                 if (b >= 0 && b < NSUB) {
-                    const int c0 = b * SUB;
-                    // entries of this lane inside the matrix: the first `count` of its column or row
-                    const int rows_left = rows_in - r0, cols_left = cols_in - c0;
-                    const int along = role ? cols_left : rows_left, count = k < (role ? rows_left : cols_left) ? max(0, min(along, SUB)) : 0;
-                    const int step = role ? 1 : LD;
-                    F acc[SUB];
-                    {
-                        const F *const src = role ? Ys + (r0 + k) * LD + c0 : Cs + r0 * LD + c0 + k;
-#pragma unroll
-                        for (int r = 0; r < SUB; ++r) acc[r] = src[((r - k) & (SUB - 1)) * step];
-                    }
-                    F *const pre_ptr = pre + (i0 + r0) * n + j0 + c0 + k;  // the caller's array: rows of n
-                    const int partner0 = ((role ^ 1) << 4) - k;
-                    auto stages = [&](auto divide_tag, auto record_tag) {
-                        constexpr int DIVIDE = decltype(divide_tag)::value;
-                        constexpr bool RECORD = decltype(record_tag)::value;
-                        uint32_t dg = shared_address(Dg) + (uint32_t)((SUB + ((role ? NSUB + b : sub_a)) * SUB - k) * DLD * (int)sizeof(F));
-                        uint32_t par = shared_address(Par) + (uint32_t)(par0 * (int)sizeof(F));
-                        const uint32_t par_bytes = (uint32_t)(par_step * (int)sizeof(F));
-                        uint32_t own = shared_address(role ? Cs + (r0 + k) * LD + c0 : Ys + r0 * LD + c0 + k) - (uint32_t)(k * step * (int)sizeof(F));
-                        F kc[SUB], pa[4];
-                        auto fetch = [&](uint32_t d, uint32_t q, F (&co)[SUB], F (&pq)[4]) {
-                            if (KIND != G2D_Q_ROUND) load4_here(q, pq);
-#pragma unroll
-                            for (int v4 = 0; v4 < SUB; v4 += 4) {
-                                F t[4];
-                                load4_here(d + (uint32_t)(v4 * (int)sizeof(F)), t);
-#pragma unroll
-                                for (int x = 0; x < 4; ++x) co[v4 + x] = t[x];
-                            }
-                        };
-                        fetch(dg, par, kc, pa);
-                        int p = -k;  // place of this lane's entry in its column or row
-#pragma unroll 1
-                        for (int s_first = 0; s_first < 2 * SUB; s_first += ROLL) {
-#pragma unroll
-                            for (int j = 0; j < ROLL; ++j) {
-                                const bool ok = (unsigned)p < (unsigned)count;
-                                const F other = __shfl_sync(0xffffffffu, acc[0], partner0 + s_first + j);
-                                F kc_next[SUB], pa_next[4];
-                                fetch(dg + (uint32_t)((j + 1) * DLD * (int)sizeof(F)), par + par_bytes, kc_next, pa_next);
-                                const F carry = role ? other : (F)0;
-                                const F yv = acc[0] + other;
-                                F z, z_out;  // what is stored: z, with the sign of a zero
-                                if (KIND == G2D_Q_AFFINE && DIVIDE == 0) {
-                                    z = affine_value_fast(yv, pa[0], pa[1], pa[2], P.qmin, P.qmax, z_out);
-                                } else if (KIND == G2D_Q_AFFINE) {
-                                    z = DIVIDE == 2 ? affine_value(yv, pa[0], pa[1], P.qmin, P.qmax) : affine_value_rcp(yv, pa[0], pa[1], pa[2], P.qmin, P.qmax);
-                                } else if (KIND == G2D_Q_FORCED) {
-                                    z = pa[0];
-                                } else {
-                                    z = rint_even(yv);
-                                }
-                                if (KIND != G2D_Q_AFFINE || DIVIDE != 0) z_out = z;
-                                const F carried = (z - yv) + carry;  // completed C (row lanes) or error (column lanes)
-                                const F v = ok ? carried : (F)0;     // lanes without an entry push zero
-#pragma unroll
-                                // the push moves every accumulator down by one register on the way
-                                const F last = acc[0];
-#pragma unroll
-                                for (int dd = 1; dd < SUB; ++dd) acc[dd - 1] = acc[dd] + kc[dd] * v;
-                                acc[SUB - 1] = last;
-                                store_shared_if(own, carried, ok);
-                                store_shared_if(par + 3 * (uint32_t)sizeof(F), z_out, ok);  // both lanes of an entry store the same value
-                                if (RECORD && ok && !role) pre_ptr[(int64_t)p * n] = yv;
-                                own += (uint32_t)(step * (int)sizeof(F));
-                                par += par_bytes;
-                                ++p;
-#pragma unroll
-                                for (int x = 0; x < SUB; ++x) kc[x] = kc_next[x];
-#pragma unroll
-                                for (int x = 0; x < 4; ++x) pa[x] = pa_next[x];
-                            }
-                            dg += (uint32_t)(ROLL * DLD * (int)sizeof(F));
-                        }
-                    };
-                    using std::integral_constant;
-                    // 0 and 1 for the common case, without a branch in the stages; recording the pre-rounding values is a matter of tests
-                    const bool exact = !fast_div[sub_a];
+                    SubTile<F> t;
+                    t.ys = Ys + r0 * LD + b * SUB;
+                    t.cs = Cs + r0 * LD + b * SUB;
+                    t.dg_c = Dg + (SUB + sub_a * SUB) * DLD;
+                    t.dg_y = Dg + (SUB + (NSUB + b) * SUB) * DLD;
+                    t.par = Par + (w & 1) * 2 * PPLANE + sub_a * SUB * PLD * 2;
+                    t.rows = rows_in - r0;
+                    t.cols = cols_in - b * SUB;
+                    t.qmin = P.qmin;
+                    t.qmax = P.qmax;
+                    t.pre = pre != nullptr ? pre + (i0 + r0) * n + j0 + b * SUB : nullptr;  // the caller's array: rows of n
+                    t.pre_ld = n;
+                    // 3 and 4 (float) and 1 (double) for the common case, without a branch in the stages; recording the pre-rounding
+                    // values is a matter of tests.  The zero points of symmetric codes are zeros: stages of 95 cycles with 4, 104 with 3 and 120
+                    // before there was either (one sweeping warp alone; four of them 136, 141 and 152).
+                    const unsigned how = fast_div[w & 1][sub_a];
+                    const bool exact = !(how & 1);
                     if (pre != nullptr) {
-                        if (exact) stages(integral_constant<int, 2>{}, std::true_type{});
-                        else stages(integral_constant<int, 1>{}, std::true_type{});
-                    } else if (exact) stages(integral_constant<int, 2>{}, std::false_type{});
-                    else if (sizeof(F) != sizeof(float) || !P.small_integer_bounds) stages(integral_constant<int, 1>{}, std::false_type{});
-                    else stages(integral_constant<int, 0>{}, std::false_type{});
+                        if (exact) sweep_sub_tile<F, KIND, 2, true>(t, lane);
+                        else sweep_sub_tile<F, KIND, 1, true>(t, lane);
+                    } else if (exact) sweep_sub_tile<F, KIND, 2, false>(t, lane);
+                    else if constexpr (sizeof(F) == sizeof(float)) {
+                        if (!P.small_integer_bounds) sweep_sub_tile<F, KIND, 1, false>(t, lane);
+                        else if (how & 2) sweep_sub_tile<F, KIND, 4, false>(t, lane);
+                        else sweep_sub_tile<F, KIND, 3, false>(t, lane);
+                    } else sweep_sub_tile<F, KIND, 1, false>(t, lane);
+                }
+                if constexpr (PUSH) {
+                    // While the last sub-tile is swept, the warps of rows 0 and 2 make the operand planes of everything else, under the scales that
+                    // follow from everything else: the last sub-tile seldom changes them.  (They share a scheduler; row 1 shares one with
+                    // the sweep, which took 180 cycles a stage beside it in place of 120.)
+                    if (w == 2 * NSUB - 2 && (number & 1) == 0 && P.c_hi != nullptr) {
+                        const int at = (number >> 1) * 32 + lane;  // row, then column
+                        row_max[at] = row_extreme(Ys + at * LD, Cs + at * LD, at < LAST * SUB ? TILE : LAST * SUB);
+                        early_planes_barrier();
+                        const unsigned all = __vmaxu2(row_max[lane], row_max[32 + lane]);
+                        const int ee = range_exponent(__uint_as_float(__reduce_max_sync(0xffffffffu, all & 0xffffu) << 16));
+                        const int ec = range_exponent(__uint_as_float(__reduce_max_sync(0xffffffffu, all >> 16) << 16));
+                        if (at == 0) {
+                            early_exponent[0] = ee;
+                            early_exponent[1] = ec;
+                        }
+                        const float e_by = power_of_two(-ee), c_by = power_of_two(-ec);
+#pragma unroll 2
+                        for (int r = 0; r < TILE; r += 8) {  // (the last sub-tile as it is at the moment; it is done again)
+                            split_e(r, at, e_by);
+                            split_c(r + at / 8, at % 8 * 8, c_by);
+                        }
+                    }
                 }
                 __syncthreads();
                 if (w + 1 < 2 * NSUB - 1) {
@@ -397,10 +316,12 @@
                 }
             }
         } else {
+#pragma unroll 1
             for (int w = 0; w < 2 * NSUB - 1; ++w) {
                 const bool more = w + 1 < 2 * NSUB - 1;
                 const int ap = helper;
-                if (more) fetch_params(w + 1);
+                write_rounded<F, KIND>(tile, params_of(w - 1), &fast_div[(w - 1) & 1][helper], w - 1, helper, lane);
+                if (more) fetch_params<F, KIND>(tile, w + 1, helper, lane, params);
                 // While sub-tile anti-diagonal w is swept: the products of the sub-tiles (a, b) swept one anti-diagonal ago, i.e.
                 // the row strip of each in the push to the right neighbour, the column strip in the push to the lower one
                 // (dealt out to the helpers in turn), and the feedback to the sub-tiles two or more places down (helpers 0
@@ -418,168 +339,92 @@
                     for (int job = helper; job < 2 * (a_hi - a_lo); job += HELPERS) {
                         const int a = a_lo + (job >> 1), b = w - 1 - a;
                         if (job & 1) {
-                            if (owes_down) mm16<TALL>(Cns + b * SUB, Lbs + a * SUB, Ys + a * SUB * LD + b * SUB, lane);
+                            if (!owes_down) continue;
+                            mm16<TALL>(Cns + b * SUB, Lbs + a * SUB, Ys + a * SUB * LD + b * SUB, lane);
+                            if (a == LAST) push_out<TILE, SUB>(Cns + b * SUB, cn_out + b * SUB, ld, push_vec, rows_below, cols_in - b * SUB, lane);
                         } else {
-                            if (owes_right) mm16<WIDE>(Yns + a * SUB * LD, Cs + a * SUB * LD + b * SUB, Ubs + b * SUB * LD, lane);
+                            if (!owes_right) continue;
+                            mm16<WIDE>(Yns + a * SUB * LD, Cs + a * SUB * LD + b * SUB, Ubs + b * SUB * LD, lane);
+                            if (b == LAST) push_out<SUB, TILE>(Yns + a * SUB * LD, yn_out + a * SUB * ld, ld, push_vec, rows_in - a * SUB, cols_right, lane);
                         }
                     }
                 }
-                if (more) finish_params(w + 1);
-                __syncthreads();
-                {   // the rounded values of the sub-tiles just swept: helper warp ap writes out the block of its row
-                    const int bz = w - ap;
-                    if (bz >= 0 && bz < NSUB) {
-                        const bool zvec = ld % 4 == 0 && reinterpret_cast<uintptr_t>(yg) % (4 * sizeof(F)) == 0;
-#pragma unroll
-                        for (int q = 0; q < 2; ++q) {
-                            const int e = lane * 2 + q, row = e >> 2, c4 = (e & 3) * 4;
-                            const int64_t gi = i0 + ap * SUB + row, gj = j0 + bz * SUB + c4;
-                            F v[4];
-#pragma unroll
-                            for (int x = 0; x < 4; ++x) v[x] = Par[((ap * SUB + row) * PLD + c4 + x) * 4 + 3];
-                            if (gi < m) {
-                                if (zvec) {
-                                    if (gj < n) store4(yg + gi * ld + gj, v);
-                                } else {
-#pragma unroll
-                                    for (int x = 0; x < 4; ++x)
-                                        if (gj + x < n) yg[gi * ld + gj + x] = v[x];
-                                }
-                            }
-                        }
-                        __syncwarp();  // the next parameters overwrite them
+                if constexpr (PUSH) {
+                    if (!more && helper < 2 && P.c_hi != nullptr) {
+                        const int column = helper * 32 + lane;
+                        column_max[column] = column_extreme(Ys + column, Cs + column, column < LAST * SUB ? TILE : LAST * SUB);
                     }
                 }
-                // ---- between two sweeps: the anti-diagonal just swept, carried into the next one; the next parameters ----
                 if (more) {
-                    store_params(w + 1);
+                    finish_params<F, KIND>(tile, params_of(w + 1), &fast_div[(w + 1) & 1][helper], w + 1, helper, lane, params);
+                }
+                __syncthreads();
+                // ---- between two sweeps: the anti-diagonal just swept, carried into the next one ----
+                if (more) {
                     const int bn = w + 1 - ap;
                     if (ap >= 1 && bn >= 0 && bn < NSUB)  // the right product is the sweeping warp's
                         mm16<SMALL>(Cs + ap * SUB * LD + bn * SUB, LUs + ap * SUB * LD + (ap - 1) * SUB, Ys + (ap - 1) * SUB * LD + bn * SUB, lane);
                     __syncthreads();
                 }
             }
+            write_rounded<F, KIND>(tile, params_of(2 * NSUB - 2), &fast_div[(2 * NSUB - 2) & 1][helper], 2 * NSUB - 2, helper, lane);
         }
 #if G2D_JOINT
         let_the_next_launch_start();
 #endif
-        // ---- neighbour push: the last sub-tile's terms, one product per warp, then out to the planes of the neighbours ----
+        // ---- neighbour push: the last sub-tile's terms, one product per warp ----
         if constexpr (PUSH) {
-            if (owes_right || owes_down) {
-                constexpr int last = NSUB - 1;
-                const int x = warp & 3;
-                F *const D = warp < 4 ? Yns + last * SUB * LD + x * SUB : Cns + x * SUB * LD + last * SUB;
-                const F *const A = warp < 4 ? Cs + last * SUB * LD + last * SUB : Lbs + x * SUB * LD + last * SUB;
-                const F *const B = warp < 4 ? Ubs + last * SUB * LD + x * SUB : Ys + last * SUB * LD + last * SUB;
-                if (warp < 4 ? owes_right : owes_down) mm16<SMALL>(D, A, B, lane);
-                __syncthreads();
-                // rows and columns past the matrix are not stored; a row's last group of four may reach into its padding
-                const bool pvec = ld % 4 == 0 && reinterpret_cast<uintptr_t>(yng) % (4 * sizeof(F)) == 0;
-                for (int idx = tid; idx < TILE * TILE / 4; idx += TTH) {
-                    const int r = idx / (TILE / 4), c = (idx % (TILE / 4)) * 4;
-                    F v[4];
-                    if (owes_right && i0 + r < m && j0 + TILE + c < n) {
-                        load4(Yns + r * LD + c, v);
-                        F *dst = yng + (i0 + r) * ld + j0 + TILE + c;
-                        if (pvec) store4(dst, v);
-                        else
-                            for (int x4 = 0; x4 < 4; ++x4)
-                                if (j0 + TILE + c + x4 < n) dst[x4] = v[x4];
-                    }
-                    if (owes_down && i0 + TILE + r < m && j0 + c < n) {
-                        load4(Cns + r * LD + c, v);
-                        F *dst = cng + (i0 + TILE + r) * ld + j0 + c;
-                        if (pvec) store4(dst, v);
-                        else
-                            for (int x4 = 0; x4 < 4; ++x4)
-                                if (j0 + c + x4 < n) dst[x4] = v[x4];
-                    }
+            const int x = warp & 3;
+            if (warp < 4) {
+                if (owes_right) {
+                    F *const D = Yns + LAST * SUB * LD + x * SUB;
+                    mm16<SMALL>(D, Cs + LAST * SUB * LD + LAST * SUB, Ubs + LAST * SUB * LD + x * SUB, lane);
+                    push_out<SUB, SUB>(D, yn_out + LAST * SUB * ld + x * SUB, ld, push_vec, rows_in - LAST * SUB, cols_right - x * SUB, lane);
                 }
+            } else if (owes_down) {
+                F *const D = Cns + x * SUB * LD + LAST * SUB;
+                mm16<SMALL>(D, Lbs + x * SUB * LD + LAST * SUB, Ys + LAST * SUB * LD + LAST * SUB, lane);
+                push_out<SUB, SUB>(D, cn_out + x * SUB * ld + LAST * SUB, ld, push_vec, rows_below - x * SUB, cols_in - LAST * SUB, lane);
             }
         }
-        // ---- operands of the tensor-core updates: fp16 pairs of E (transposed) and of the completed C under the tile's scales ----
-        bool wide_e = false, wide_c = false;
-        if constexpr (sizeof(F) == sizeof(float)) {
+        // ---- operands of the tensor-core updates: what the last sub-tile changes, and what it adds ----
+        const bool planes_only = P.c_hi != nullptr && yng != nullptr;  // the errors and the completed C are read from their operand planes alone
+        bool keep_e = !planes_only, keep_c = !planes_only;
+        if constexpr (PUSH) {
             if (P.c_hi != nullptr) {
-                // Largest values of the rows, the columns and the tile (entries outside the matrix are zero), of E in the lower and of C in
-                // the upper half of a word: the upper halves of floats are all that the scale and the comparison need.
-                unsigned column[4] = {0u, 0u, 0u, 0u};
-#pragma unroll
-                for (int t = 0; t < TILE * TILE / 4 / TTH; ++t) {  // a thread's vectors lie in the same four columns
-                    const int idx = t * TTH + tid, r = idx / (TILE / 4), c = (idx % (TILE / 4)) * 4;
-                    F ve[4], vc[4];
-                    load4(Ys + r * LD + c, ve);
-                    load4(Cs + r * LD + c, vc);
-                    unsigned row = 0u;
-#pragma unroll
-                    for (int x = 0; x < 4; ++x) {
-                        const unsigned both = __byte_perm(__float_as_uint((float)ve[x]), __float_as_uint((float)vc[x]), 0x7632) & 0x7fff7fffu;
-                        row = __vmaxu2(row, both);
-                        column[x] = __vmaxu2(column[x], both);
-                    }
-#pragma unroll
-                    for (int o = 1; o < TILE / 4; o <<= 1) row = __vmaxu2(row, __shfl_xor_sync(0xffffffffu, row, o));
-                    if ((lane & 15) == 0) row_max[r] = row;
-                }
-#pragma unroll
-                for (int x = 0; x < 4; ++x) column[x] = __vmaxu2(column[x], __shfl_xor_sync(0xffffffffu, column[x], 16));
-                if (lane < 16) *reinterpret_cast<uint4 *>(&column_max[warp][lane * 4]) = make_uint4(column[0], column[1], column[2], column[3]);
-                __syncthreads();
-                unsigned most = 0u, least = 0xffffffffu;  // every warp for itself: two rows and two columns per lane
-#pragma unroll
-                for (int h = 0; h < 2; ++h) {
-                    unsigned col = column_max[0][h * 32 + lane];
-#pragma unroll
-                    for (int w2 = 1; w2 < TTH / 32; ++w2) col = __vmaxu2(col, column_max[w2][h * 32 + lane]);
-                    const unsigned row = row_max[h * 32 + lane];
-                    most = __vmaxu2(most, row);
-                    least = __vminu2(least, __vminu2(row | __vcmpeq2(row, 0u), col | __vcmpeq2(col, 0u)));  // zeros apart
-                }
+                // Every warp for itself: the largest values of the rows and columns of the last sub-tile, on top of the others'
+                unsigned most, least;
+                last_extremes(Ys + LAST * SUB * LD + LAST * SUB, Cs + LAST * SUB * LD + LAST * SUB, row_max, column_max, lane, most, least);
                 const unsigned most_e = __reduce_max_sync(0xffffffffu, most & 0xffffu), most_c = __reduce_max_sync(0xffffffffu, most >> 16);
                 const unsigned least_e = __reduce_min_sync(0xffffffffu, least & 0xffffu), least_c = __reduce_min_sync(0xffffffffu, least >> 16);
-                wide_e = most_e >= 0x7f80u || least_e + WIDE_RATIO_BITS <= most_e;
-                wide_c = most_c >= 0x7f80u || least_c + WIDE_RATIO_BITS <= most_c;
+                const bool wide_e = most_e >= 0x7f80u || least_e + WIDE_RATIO_BITS <= most_e;
+                const bool wide_c = most_c >= 0x7f80u || least_c + WIDE_RATIO_BITS <= most_c;
                 const int ee = range_exponent(__uint_as_float(most_e << 16)), ec = range_exponent(__uint_as_float(most_c << 16));
                 if (tid == 0) {
                     P.e_scale[(int64_t)I * P.nJ + J] = wide_e ? -1.f : power_of_two(ee);
                     P.c_scale[(int64_t)I * P.nJ + J] = wide_c ? -1.f : power_of_two(ec);
                     if (wide_e || wide_c) atomicAdd(P.wide_count, wide_e + wide_c);
                 }
-                const float e_by = power_of_two(-ee), c_by = power_of_two(-ec);
-                // eight entries per thread and store.  C along its rows; E transposed: a thread gathers eight rows of one column
-                // (consecutive threads take consecutive columns, so the shared-memory reads do not collide) and writes them as
-                // one vector of a row of E^T.  A row's last vector may reach into its padding.
-                for (int idx = tid; idx < TILE * TILE / 8; idx += TTH) {
-                    __align__(16) __half h[8];
-                    __align__(16) __half l[8];
-                    {
-                        const int r = idx / (TILE / 8), c = (idx % (TILE / 8)) * 8;
-                        if (r < rows_in && c < cols_in) {
-#pragma unroll
-                            for (int x = 0; x < 8; ++x) split_half(wide_c ? 0.f : (float)Cs[r * LD + c + x] * c_by, h[x], l[x]);
-                            const int64_t at = (i0 + r) * P.ldn + j0 + c;
-                            *reinterpret_cast<uint4 *>(P.c_hi + at) = *reinterpret_cast<const uint4 *>(h);
-                            *reinterpret_cast<uint4 *>(P.c_lo + at) = *reinterpret_cast<const uint4 *>(l);
-                        }
-                    }
-                    {
-                        const int c = idx % TILE, r = (idx / TILE) * 8;
-                        if (r < rows_in && c < cols_in) {
-#pragma unroll
-                            for (int x = 0; x < 8; ++x) split_half(wide_e ? 0.f : (float)Ys[(r + x) * LD + c] * e_by, h[x], l[x]);
-                            const int64_t at = (j0 + c) * P.ldm + i0 + r;
-                            *reinterpret_cast<uint4 *>(P.et_hi + at) = *reinterpret_cast<const uint4 *>(h);
-                            *reinterpret_cast<uint4 *>(P.et_lo + at) = *reinterpret_cast<const uint4 *>(l);
-                        }
+                const float e_by = wide_e ? 0.f : power_of_two(-ee), c_by = wide_c ? 0.f : power_of_two(-ec);
+                const bool as_foreseen = !wide_e && !wide_c && ee == early_exponent[0] && ec == early_exponent[1];
+                if (as_foreseen) {
+                    if (warp == 0) split_c(LAST * SUB + lane / 2, LAST * SUB + lane % 2 * 8, c_by);
+                    if (warp == 1) split_e(LAST * SUB + lane / SUB * 8, LAST * SUB + lane % SUB, e_by);
+                } else {
+#pragma unroll 1
+                    for (int idx = tid; idx < TILE * TILE / 8; idx += TTH) {
+                        split_c(idx / (TILE / 8), idx % (TILE / 8) * 8, c_by);
+                        split_e(idx / TILE * 8, idx % TILE, e_by);
                     }
                 }
+                keep_e = keep_e || wide_e;
+                keep_c = keep_c || wide_c;
             }
         }
         // ---- store the errors and the completed C of the tile, unless only their operand planes are read from here on ----
-        const bool planes_only = P.c_hi != nullptr && yng != nullptr;
-        const bool keep_e = !planes_only || wide_e, keep_c = !planes_only || wide_c;
         if (!keep_e && !keep_c) {
         } else if (vec) {
+#pragma unroll 1
             for (int idx = tid; idx < TILE * TILE / 4; idx += TTH) {
                 const int r = idx / (TILE / 4), c = (idx % (TILE / 4)) * 4;
                 F ve[4], vc[4];
