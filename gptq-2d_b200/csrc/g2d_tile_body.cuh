@@ -59,9 +59,12 @@
         constexpr bool PUSH = sizeof(F) == sizeof(float);  // the neighbour push exists for float (pipelined schedule) only
 
         // ---- load the tile ----
-        const bool vec = full && ((ld | ldl | ldu) % 4 == 0) &&
-                         ((reinterpret_cast<uintptr_t>(yg) | reinterpret_cast<uintptr_t>(cg) | reinterpret_cast<uintptr_t>(eg) |
-                           reinterpret_cast<uintptr_t>(lg) | reinterpret_cast<uintptr_t>(ug)) % (4 * sizeof(F)) == 0);
+        // rows as vectors: of a tile at the matrix's edge too, which then loads from inside the matrix and puts zeros outside (a value at a time
+        // took 5 us more, on nearly every launch of a matrix that is no multiple of 64)
+        const bool row_vectors = ((ld | ldl | ldu) % 4 == 0) &&
+                                 ((reinterpret_cast<uintptr_t>(yg) | reinterpret_cast<uintptr_t>(cg) | reinterpret_cast<uintptr_t>(eg) |
+                                   reinterpret_cast<uintptr_t>(lg) | reinterpret_cast<uintptr_t>(ug)) % (4 * sizeof(F)) == 0);
+        const bool vec = full && row_vectors;
         bool have_diagonal = false;
         if constexpr (PUSH) {
             if (owes_right || owes_down)
@@ -69,14 +72,16 @@
                     const F zero[4] = {(F)0, (F)0, (F)0, (F)0};
                     store4(Yns + idx * 4, zero);
                 }
-            if (vec) {
+            if (row_vectors) {
                 // One wait on global memory: the off-diagonal blocks of L[I, I] and U[J, J] and the two coupling blocks
                 // travel to shared memory on their own (cp.async), the diagonal blocks and the six planes that make up Y and
                 // C through registers, and all of them are issued before the first is used.
                 have_diagonal = true;
                 for (int c = tid; c < 12 * SUB * 4; c += TTH) {
                     const int blk = c / (SUB * 4), ba = blk / 3, bb = blk % 3 + (blk % 3 >= ba ? 1 : 0), row = ba * SUB + c / 4 % SUB, col = bb * SUB + c % 4 * 4;
-                    async16(LUs + row * LD + col, ba > bb ? lg + (i0 + row) * ldl + i0 + col : ug + (j0 + row) * ldu + j0 + col, true);
+                    const int inside = ba > bb ? rows_in : cols_in, there = row < inside ? min(4, max(0, inside - col)) : 0;  // values of the vector
+                    const F *src = ba > bb ? lg + (i0 + row) * ldl + i0 + col : ug + (j0 + row) * ldu + j0 + col;
+                    async16(LUs + row * LD + col, there ? src : lg, there * (int)sizeof(F));
                 }
                 if (owes_right)
                     for (int c = tid; c < TILE * TILE / 4; c += TTH) {
@@ -84,13 +89,13 @@
                         // n is not always a multiple of 4, the row stride is.  The tail of a padded copy is not defined: what is formed
                         // with it goes to columns from n on, which are not stored, or stored to padding that nothing reads.
                         const bool in = j0 + TILE + col < n;
-                        async16(Ubs + row * LD + col, ug + (j0 + row) * ldu + (in ? j0 + TILE + col : 0), in);
+                        async16(Ubs + row * LD + col, ug + (j0 + row) * ldu + (in ? j0 + TILE + col : 0), in ? 16 : 0);
                     }
                 if (owes_down)
                     for (int c = tid; c < TILE * TILE / 4; c += TTH) {
                         const int row = c / (TILE / 4), col = c % (TILE / 4) * 4;
                         const bool in = i0 + TILE + row < m;
-                        async16(Lbs + row * LD + col, lg + (in ? i0 + TILE + row : 0) * ldl + i0 + col, in);
+                        async16(Lbs + row * LD + col, lg + (in ? i0 + TILE + row : 0) * ldl + i0 + col, in ? 16 : 0);
                     }
                 asm volatile("cp.async.commit_group;" ::: "memory");
                 constexpr int PER = TILE * TILE / 4 / TTH;  // vectors per thread and array
@@ -98,8 +103,9 @@
 #if G2D_JOINT  // the factors ahead of the wait
 #pragma unroll
                 for (int t = 0; t < 2; ++t) {  // the eight diagonal blocks, 64 vectors each
-                    const int idx = t * TTH + tid, blk = idx / 64, r = idx / 4 % SUB, c = idx % 4 * 4, o = (blk % NSUB) * SUB;
-                    load4(blk < NSUB ? lg + (i0 + o + r) * ldl + i0 + o + c : ug + (j0 + o + r) * ldu + j0 + o + c, dv[t]);
+                    const int idx = t * TTH + tid, blk = idx / 64, o = (blk % NSUB) * SUB, inside = blk < NSUB ? rows_in : cols_in;
+                    const int r = min(o + idx / 4 % SUB, inside - 1), c = o + idx % 4 * 4 < inside ? o + idx % 4 * 4 : 0;
+                    load4(blk < NSUB ? lg + (i0 + r) * ldl + i0 + c : ug + (j0 + r) * ldu + j0 + c, dv[t]);
                 }
                 for (int idx = tid; idx < DROWS * DLD / 4; idx += TTH) {
                     const F zero[4] = {(F)0, (F)0, (F)0, (F)0};
@@ -110,7 +116,7 @@
 #pragma unroll
                 for (int t = 0; t < PER; ++t) {
                     const int idx = t * TTH + tid, r = idx / (TILE / 4), c = (idx % (TILE / 4)) * 4;
-                    const int64_t at = (i0 + r) * ld + j0 + c;
+                    const int64_t at = (i0 + min(r, rows_in - 1)) * ld + j0 + (c < cols_in ? c : 0);
                     load4(yg + at, vy[t]);
                     load4(cg + at, vc[t]);
 #pragma unroll
@@ -125,8 +131,9 @@
 #if !G2D_JOINT
 #pragma unroll
                 for (int t = 0; t < 2; ++t) {  // the eight diagonal blocks, 64 vectors each
-                    const int idx = t * TTH + tid, blk = idx / 64, r = idx / 4 % SUB, c = idx % 4 * 4, o = (blk % NSUB) * SUB;
-                    load4(blk < NSUB ? lg + (i0 + o + r) * ldl + i0 + o + c : ug + (j0 + o + r) * ldu + j0 + o + c, dv[t]);
+                    const int idx = t * TTH + tid, blk = idx / 64, o = (blk % NSUB) * SUB, inside = blk < NSUB ? rows_in : cols_in;
+                    const int r = min(o + idx / 4 % SUB, inside - 1), c = o + idx % 4 * 4 < inside ? o + idx % 4 * 4 : 0;
+                    load4(blk < NSUB ? lg + (i0 + r) * ldl + i0 + c : ug + (j0 + r) * ldu + j0 + c, dv[t]);
                 }
                 for (int idx = tid; idx < DROWS * DLD / 4; idx += TTH) {
                     const F zero[4] = {(F)0, (F)0, (F)0, (F)0};
@@ -144,6 +151,10 @@
                         vy[t][x] += fy[t][x] + ny[t][x];
                         vc[t][x] += fc[t][x] + nc[t][x];
                     }
+                    if (!full)
+#pragma unroll
+                        for (int x = 0; x < 4; ++x)
+                            if (r >= rows_in || c + x >= cols_in) vy[t][x] = vc[t][x] = (F)0;
                     store4(Ys + r * LD + c, vy[t]);
                     store4(Cs + r * LD + c, vc[t]);
                 }
@@ -153,7 +164,8 @@
 #pragma unroll
                     for (int x = 0; x < 4; ++x) {
                         const int p = blk < NSUB ? c + x : r, q = blk < NSUB ? r : c + x;  // source and receiver
-                        if (q > p) Dg[(SUB + blk * SUB + p) * DLD + q - p] = dv[t][x];
+                        const int inside = (blk < NSUB ? rows_in : cols_in) - (blk % NSUB) * SUB;
+                        if (q > p) Dg[(SUB + blk * SUB + p) * DLD + q - p] = q < inside ? dv[t][x] : (F)0;
                     }
                 }
                 asm volatile("cp.async.wait_all;" ::: "memory");

@@ -46,9 +46,9 @@ __device__ __forceinline__ void store4<double>(double *p, const double (&v)[4]) 
     *reinterpret_cast<double2 *>(p + 2) = make_double2(v[2], v[3]);
 }
 
-// Sixteen bytes from global to shared memory without passing through registers; zeros when `in` is false.
-__device__ __forceinline__ void async16(void *dst, const void *src, bool in) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src), "r"(in ? 16 : 0) : "memory");
+// Sixteen bytes to shared memory without passing through registers: the first `bytes` from global memory, then zeros.
+__device__ __forceinline__ void async16(void *dst, const void *src, int bytes) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src), "r"(bytes) : "memory");
 }
 __device__ __forceinline__ uint32_t shared_address(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
 // Loads of the stage loop: volatile, so that they stay where they are written (one stage ahead of their use, behind the shuffle).
