@@ -33,10 +33,14 @@ static int launch_step_kind(const SweepArgs<float> &args, int S, const BandJob &
     if (configured.run([&] { return cudaFuncSetAttribute(sweep_step_kernel<float, KIND>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) == cudaSuccess; }) != G2D_OK)
         return G2D_ERR_CUDA;
     const int i_lo = S - args.nJ + 1 > 0 ? S - args.nJ + 1 : 0, i_hi = S + 1 < args.nI ? S + 1 : args.nI, tiles = i_hi - i_lo;
-    const int jobs = 2 * job.longest * job.slots, free_sms = 148 - tiles;  // at most 128 tiles take this schedule
+    // Updating CTAs: as many as there are SMs left, but sixteen jobs each, which the ring takes in 5 to 12 us of the tiles' 25.  More of them keep SMs
+    // from the far updates (4 us of set-up and first loads each): 1, 8, 16 and 24 jobs at least, in us: 2048 x 2048 1694, 1678, 1684, 1732;
+    // 4096 x 4096 3672, 3635, 3615, 3719; 8192 x 8192 11047, 11010, 10971, 10935.
+    constexpr int JOBS_EACH = 16;
+    const int jobs = 2 * job.longest * job.slots, free_sms = 148 - tiles, updating = (jobs + JOBS_EACH - 1) / JOBS_EACH;  // at most 128 tiles take this schedule
     if (free_sms < 1) return G2D_ERR_BAD_ARGUMENT;
     cudaLaunchConfig_t config{};
-    config.gridDim = dim3((unsigned)(tiles + (jobs < free_sms ? jobs : free_sms)));
+    config.gridDim = dim3((unsigned)(tiles + (updating < free_sms ? updating : free_sms)));
     config.blockDim = dim3(TTH);
     config.dynamicSmemBytes = smem;
     config.stream = stream;
