@@ -210,9 +210,15 @@ __global__ void __launch_bounds__(BTH) band_update_kernel(BandArgs<F> P, int nTI
 // shared memory with the next chunk on its way, masks from bounds that a thread computes once for the rows and columns
 // it stages (in place of divisions per element: 1 ms per flush before, 10 to 100 us now at 512 x 2048 under 1 x 32
 // super-entries).  The terms of a sum keep their order, ascending in k, and the down sum is added before the right one.
+// What bounds a flush of few stages is the row of chunks that a CTA takes one after the other: 23 at 512 x 2048 as 1 x 32 (rows of 8 x 32 k
+// shifted against each other).  A flush of eight stages there took 45 us with 64-bit bounds, single reads of B and products of zeros, 36 now
+// (512 x 2048 as 1 x 32 whole: 4970 us with two CTAs per SM, 4680 with three, 5890 with four).  Fewer threads with 4 x 4 targets read half as
+// much from shared memory and are slower (64 x 16 targets 76 us, 128 x 16 63 us).
+// SKIP: a warp passes over the chunks outside the windows of its rows.  Worth its branch where the rows of a tile lie in many super-entries:
+// 512 x 2048 as 1 x 32 4680 us with and 4890 without it, 256 x 1024 as 4 x 128 1870 and 1830.
 constexpr int MTH = 256;
-template <typename F, int BM>
-__global__ void __launch_bounds__(MTH) band_masked_kernel(BandArgs<F> P) {
+template <typename F, int BM, bool SKIP>
+__global__ void __launch_bounds__(MTH, BM == 16 && SKIP ? 3 : 1) band_masked_kernel(BandArgs<F> P) {
     constexpr int CK = sizeof(F) == sizeof(float) ? 32 : 16;  // k per chunk
     constexpr int NR = BM / 16;                               // rows per thread; 4 columns
     constexpr int LA = BM * CK / MTH, LB = 64 * CK / MTH;     // elements of A and B staged per thread
@@ -246,33 +252,39 @@ __global__ void __launch_bounds__(MTH) band_masked_kernel(BandArgs<F> P) {
             const int64_t near_hi = right ? (s1 - i0 / P.P) * P.Q : (s1 - j0 / P.Q) * P.P, far_lo = right ? (s0 - i1 / P.P) * P.Q : (s0 - j1 / P.Q) * P.P;
             const int64_t k_lo = max(far_lo, (int64_t)0), k_hi = right ? min(min(near_hi, n), j1 / P.Q * P.Q) : min(min(near_hi, m), i1 / P.P * P.P);
             if (k_lo >= k_hi) continue;
-            // bounds of k for the rows of A and the columns of B that this thread stages
-            int64_t a_lo[LA], a_hi[LA], b_lo, b_hi;
+            // bounds of k, from k_lo on, for the rows of A and the columns of B that this thread stages
+            const int count = (int)(k_hi - k_lo);
+            const auto place = [&](int64_t k) { return (int)min(max(k - k_lo, (int64_t)0), (int64_t)count); };
+            int a_lo[LA], a_hi[LA];
             const F *pa[LA];
 #pragma unroll
             for (int t = 0; t < LA; ++t) {
                 const int64_t i = i0 + (t * MTH + tid) / CK;
-                pa[t] = right ? cg + i * n : lg + i * m;
-                a_lo[t] = right ? (s0 - i / P.P) * P.Q : 0;
-                a_hi[t] = i >= m ? 0 : right ? (s1 - i / P.P) * P.Q : i / P.P * P.P;
+                pa[t] = (right ? cg + i * n : lg + i * m) + k_lo;
+                a_lo[t] = right ? place((s0 - i / P.P) * P.Q) : 0;
+                a_hi[t] = i >= m ? 0 : place(right ? (s1 - i / P.P) * P.Q : i / P.P * P.P);
             }
             const int64_t jb = j0 + (tid & 63);
-            b_lo = right ? 0 : (s0 - jb / P.Q) * P.P;
-            b_hi = jb >= n ? 0 : right ? jb / P.Q * P.Q : (s1 - jb / P.Q) * P.P;
-            const F *pb = (right ? ug : eg) + jb;
+            const int b_lo = right ? 0 : place((s0 - jb / P.Q) * P.P);
+            const int b_hi = jb >= n ? 0 : place(right ? jb / P.Q * P.Q : (s1 - jb / P.Q) * P.P);
+            const F *pb = (right ? ug : eg) + k_lo * n + jb;
             F ra[LA], rb[LB];
-            auto fetch = [&](int64_t k0) {
+            auto fetch = [&](int k0) {
 #pragma unroll
                 for (int t = 0; t < LA; ++t) {
-                    const int64_t k = k0 + (tid & (CK - 1));
-                    ra[t] = k < k_hi && k >= a_lo[t] && k < a_hi[t] ? pa[t][k] : (F)0;
+                    const int k = k0 + (tid & (CK - 1));
+                    ra[t] = k >= a_lo[t] && k < a_hi[t] ? pa[t][k] : (F)0;
                 }
 #pragma unroll
                 for (int t = 0; t < LB; ++t) {
-                    const int64_t k = k0 + t * (MTH / 64) + (tid >> 6);
-                    rb[t] = k < k_hi && k >= b_lo && k < b_hi ? pb[k * n] : (F)0;
+                    const int k = k0 + t * (MTH / 64) + (tid >> 6);
+                    rb[t] = k >= b_lo && k < b_hi ? pb[k * n] : (F)0;
                 }
             };
+            // the k of the rows that this warp holds: outside them every product is a zero (the windows of a down product go by columns)
+            constexpr int WARP_ROWS = 2 * NR;
+            const int64_t row = i0 + (tid >> 5) * WARP_ROWS;
+            const int mine_lo = right ? place((s0 - (row + WARP_ROWS - 1) / P.P) * P.Q) : 0, mine_hi = right ? place((s1 - row / P.P) * P.Q) : count;
             auto stash = [&](int buf) {
 #pragma unroll
                 for (int t = 0; t < LA; ++t) As[buf][(tid & (CK - 1)) * ALD + (t * MTH + tid) / CK] = ra[t];
@@ -284,24 +296,25 @@ __global__ void __launch_bounds__(MTH) band_masked_kernel(BandArgs<F> P) {
             for (int r = 0; r < NR; ++r)
 #pragma unroll
                 for (int c = 0; c < 4; ++c) acc[r][c] = (F)0;
-            fetch(k_lo);
+            fetch(0);
             stash(0);
             __syncthreads();
             int buf = 0;
-            for (int64_t k0 = k_lo; k0 < k_hi; k0 += CK) {
-                const bool more = k0 + CK < k_hi;
+            for (int k0 = 0; k0 < count; k0 += CK) {
+                const bool more = k0 + CK < count;
                 if (more) fetch(k0 + CK);
+                if (!SKIP || (k0 < mine_hi && k0 + CK > mine_lo)) {
 #pragma unroll
-                for (int kk = 0; kk < CK; ++kk) {
-                    F av[NR], bv[4];
+                    for (int kk = 0; kk < CK; ++kk) {
+                        F av[NR], bv[4];
 #pragma unroll
-                    for (int r = 0; r < NR; ++r) av[r] = As[buf][kk * ALD + ty * NR + r];
+                        for (int r = 0; r < NR; ++r) av[r] = As[buf][kk * ALD + ty * NR + r];
+                        ld4(&Bs[buf][kk * BLD2 + tx * 4], bv);
 #pragma unroll
-                    for (int c = 0; c < 4; ++c) bv[c] = Bs[buf][kk * BLD2 + tx * 4 + c];
+                        for (int r = 0; r < NR; ++r)
 #pragma unroll
-                    for (int r = 0; r < NR; ++r)
-#pragma unroll
-                        for (int c = 0; c < 4; ++c) acc[r][c] += av[r] * bv[c];
+                            for (int c = 0; c < 4; ++c) acc[r][c] += av[r] * bv[c];
+                    }
                 }
                 if (more) stash(buf ^ 1);
                 __syncthreads();
@@ -340,8 +353,14 @@ int launch_band_update(const BandArgs<F> &args, cudaStream_t stream) {
     if (across > all) across = all;
     if (down > 65535) return G2D_ERR_TOO_LARGE;
     dim3 grid((unsigned)across, (unsigned)down, batches);
-    if (BM == 64) band_masked_kernel<F, 64><<<grid, MTH, 0, stream>>>(a);
-    else band_masked_kernel<F, 16><<<grid, MTH, 0, stream>>>(a);
+    const bool skip = BM >= 16 * a.P;
+    if (BM == 64) {
+        if (skip) band_masked_kernel<F, 64, true><<<grid, MTH, 0, stream>>>(a);
+        else band_masked_kernel<F, 64, false><<<grid, MTH, 0, stream>>>(a);
+    } else {
+        if (skip) band_masked_kernel<F, 16, true><<<grid, MTH, 0, stream>>>(a);
+        else band_masked_kernel<F, 16, false><<<grid, MTH, 0, stream>>>(a);
+    }
     return check_launch();
 }
 

@@ -26,6 +26,7 @@ struct StageArgs {
 
 template <typename F>
 __global__ void stage_error_kernel(StageArgs<F> A) {
+    let_the_next_launch_start();  // a pull of the next stage fetches blocks of the factors ahead of its wait for this one
     const int64_t mbar = A.m / A.p, nbar = A.n / A.q;
     const int64_t pq = (int64_t)A.p * A.q;
     if (A.skew != nullptr) {

@@ -50,6 +50,7 @@ struct SuperArgs {
     const F *l, *u;
     const int64_t *l_off, *u_off;
     int64_t s0;                        // first stage of the inner block: pushes of the stages s0 .. stage - 1 are pending
+    int pull_room, pull_stages;        // stage_pull_staged_kernel: (source stage, entry) pairs and source stages that its shared memory has room for
 };
 
 // Entry (k, a, b) of the stage of `batch`: false when the batch has no such entry at this global stage.
@@ -213,6 +214,39 @@ __device__ __forceinline__ F dot(const F *a, const F *b, int64_t ld, int count) 
     return sum;
 }
 
+// A rounded entry's values, or what the quantizer of a later launch takes: Y and C with all feedback are y and c, s the row's scale.
+template <typename F, int KIND>
+__device__ __forceinline__ void finish_entry(const SuperArgs<F> &A, int64_t batch, int64_t seq, int64_t i, int64_t j, int entry, F y, F c, F s) {
+    const int64_t at = i * A.n + j, plane = batch * A.m * A.n;
+    F *const yg = A.y + plane, *const cg = A.c + plane, *const eg = A.e + plane;
+    if (KIND == Q_PULL_ONLY) {
+        yg[at] = y;
+        cg[at] = c;
+    } else if (KIND == G2D_Q_TRELLIS) {
+        yg[at] = y;
+        cg[at] = c;
+        A.xs[seq * A.p * A.q + entry] = div_rn(y, s);
+    } else {
+        F z;
+        if (KIND == G2D_Q_ROUND) {
+            z = rint_even(y);
+        } else if (KIND == G2D_Q_AFFINE) {
+            const F sc = A.scale[(A.scale_off ? A.scale_off[batch] : 0) + i * A.srs + j * A.scs];
+            const F zp = A.zero[(A.zero_off ? A.zero_off[batch] : 0) + i * A.zrs + j * A.zcs];
+            z = affine_value(y, sc, zp, A.qmin, A.qmax);
+        } else {
+            F t = rint_even(div_rn(y, s));
+            t = t < A.qmin ? A.qmin : t;
+            t = t > A.qmax ? A.qmax : t;
+            z = mul_rn(t, s);
+        }
+        const F ev = z - y;
+        eg[at] = ev;
+        cg[at] = c + ev;
+        yg[at] = z;
+    }
+}
+
 // Sweeps whose blocks are short enough (see pull_pays).  One CTA per super-entry of the stage: first what the earlier stages of the
 // inner block owe it, then its quantizer, then its error, completed C and rounded values.  One launch per stage where the sources used to push (error, push and quantizer
 // kernels, 3 launches), because a super-entry that fetches its own feedback when its turn comes needs no launch for it.
@@ -265,35 +299,7 @@ __global__ void __launch_bounds__(PTH) stage_pull_kernel(SuperArgs<F> A) {
                     if (ib - dd >= 0 || jb - dd >= 0) y += down + right;
                 }
             };
-            auto finish = [&](int b, F y, F c, F s) {
-                const int64_t i = i0 + a, j = j0 + b, at = i * n + j;
-                if (KIND == Q_PULL_ONLY) {
-                    yg[at] = y;
-                    cg[at] = c;
-                } else if (KIND == G2D_Q_TRELLIS) {
-                    yg[at] = y;
-                    cg[at] = c;
-                    A.xs[seq * pq + a * q + b] = div_rn(y, s);
-                } else {
-                    F z;
-                    if (KIND == G2D_Q_ROUND) {
-                        z = rint_even(y);
-                    } else if (KIND == G2D_Q_AFFINE) {
-                        const F sc = A.scale[(A.scale_off ? A.scale_off[batch] : 0) + i * A.srs + j * A.scs];
-                        const F zp = A.zero[(A.zero_off ? A.zero_off[batch] : 0) + i * A.zrs + j * A.zcs];
-                        z = affine_value(y, sc, zp, A.qmin, A.qmax);
-                    } else {
-                        F t = rint_even(div_rn(y, s));
-                        t = t < A.qmin ? A.qmin : t;
-                        t = t > A.qmax ? A.qmax : t;
-                        z = mul_rn(t, s);
-                    }
-                    const F ev = z - y;
-                    eg[at] = ev;
-                    cg[at] = c + ev;
-                    yg[at] = z;
-                }
-            };
+            auto finish = [&](int b, F y, F c, F s) { finish_entry<F, KIND>(A, batch, seq, i0 + a, j0 + b, a * q + b, y, c, s); };
             F s = (F)1;
             if (KIND == G2D_Q_TRELLIS) {
                 s = A.scale[A.scale_off ? A.scale_off[batch] : 0];
@@ -336,6 +342,102 @@ __global__ void __launch_bounds__(PTH) stage_pull_kernel(SuperArgs<F> A) {
     }
 }
 
+// The same where the blocks of the factors that a super-entry needs are small (see PULL_FACTORS).  The CTAs are resident long before the stage
+// before them ends and bring those blocks to shared memory ahead of the wait; behind it they fetch the errors and C of all source
+// stages and their own Y and C in one round trip.  The same sums in the same order.  A stage of 512 x 2048 as 1 x 32 takes 2.5 us, 3.6 with the
+// kernel above.  (A stage that lets the next one start behind its wait, so that the next could form the sums of all but the last stage ahead
+// of its own: 4.5 us, the start of a launch is longer than what it hides.)
+template <typename F, int KIND>
+__global__ void __launch_bounds__(PTH) stage_pull_staged_kernel(SuperArgs<F> A) {
+    extern __shared__ __align__(16) unsigned char pull_smem[];
+    let_the_next_launch_start();
+    const int p = A.p, q = A.q, pq = p * q;
+    F *const down_s = reinterpret_cast<F *>(pull_smem), *const right_s = down_s + A.pull_room;    // sums by source stage and entry
+    F *const e_src = right_s + A.pull_room, *const c_src = e_src + A.pull_room;                   // the stages' E above and C to the left
+    F *const y_s = c_src + A.pull_room, *const c_s = y_s + pq;                                    // Y and C of the super-entry
+    F *const l_s = c_s + pq, *const u_s = l_s + (A.pull_stages) * p * p;                          // blocks of L and U
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int64_t m = A.m, n = A.n;
+    bool waited = false;
+    for (int64_t batch = blockIdx.y; batch < A.batch; batch += gridDim.y) {
+        int64_t i0, j0;
+        if (!locate(A, batch, (int64_t)blockIdx.x, 0, 0, i0, j0)) continue;
+        F *yg = A.y + batch * m * n, *cg = A.c + batch * m * n, *eg = A.e + batch * m * n;
+        const F *lg = A.l + (A.l_off ? A.l_off[batch] : 0), *ug = A.u + (A.u_off ? A.u_off[batch] : 0);
+        const int64_t ib = i0 / p, jb = j0 / q;
+        const int pulls = (int)min(A.stage - A.s0, max(ib, jb));  // source stages, dd = pulls .. 1 before this one, in this order below
+        const int64_t seq = batch * A.dmax + blockIdx.x;
+        for (int t = tid; t < pulls * p * p; t += PTH) {
+            const int x = t / (p * p), r = t % (p * p);
+            if (ib - (pulls - x) >= 0) l_s[t] = lg[(i0 + r / p) * m + (ib - (pulls - x)) * p + r % p];
+        }
+        for (int t = tid; t < pulls * q * q; t += PTH) {
+            const int x = t / (q * q), r = t % (q * q);
+            if (jb - (pulls - x) >= 0) u_s[t] = ug[((jb - (pulls - x)) * q + r / q) * n + j0 + r % q];
+        }
+        if (!waited) after_the_launch_before();
+        waited = true;
+        for (int t = tid; t < (pulls + 1) * pq; t += PTH) {
+            const int x = t / pq, at = t % pq, a = at / q, b = at % q, dd = pulls - x;
+            if (x < pulls) {
+                e_src[t] = ib - dd >= 0 ? load_here(eg + (i0 - dd * p + a) * n + j0 + b) : (F)0;
+                c_src[t] = jb - dd >= 0 ? load_here(cg + (i0 + a) * n + j0 - dd * q + b) : (F)0;
+            } else {
+                y_s[at] = load_here(yg + (i0 + a) * n + j0 + b);
+                c_s[at] = load_here(cg + (i0 + a) * n + j0 + b);
+            }
+        }
+        __syncthreads();
+        for (int t = tid; t < pulls * pq; t += PTH) {
+            const int x = t / pq, at = t % pq, a = at / q, b = at % q, dd = pulls - x;
+            const F *const e = e_src + x * pq + b, *const c = c_src + x * pq + a * q;
+            F down = (F)0, right = (F)0;
+            if (ib - dd >= 0) {
+                const F *const l = l_s + x * p * p + a * p;
+                for (int k = 0; k < p; ++k) down += l[k] * e[k * q];
+            }
+            if (jb - dd >= 0) {
+                const F *const u = u_s + x * q * q + b;
+#pragma unroll 8
+                for (int k = 0; k < q; ++k) right += c[k] * u[k * q];
+            }
+            down_s[t] = down;
+            right_s[t] = right;
+        }
+        __syncthreads();
+        for (int t = tid; t < pq; t += PTH) {
+            F y = y_s[t], c = c_s[t];
+            for (int x = 0; x < pulls; ++x) {
+                const int dd = pulls - x;
+                const F down = down_s[x * pq + t], right = right_s[x * pq + t];
+                if (ib - dd >= 0) c += down;
+                if (ib - dd >= 0 || jb - dd >= 0) y += down + right;
+            }
+            y_s[t] = y;
+            c_s[t] = c;
+        }
+        __syncthreads();
+        // a warp per row of the super-entry
+        for (int a = warp; a < p; a += PTH / 32) {
+            F s = (F)1;
+            if (KIND == G2D_Q_TRELLIS) {
+                s = A.scale[A.scale_off ? A.scale_off[batch] : 0];
+                if (a == 0 && lane == 0) A.row_scale[seq] = s;
+            }
+            if (KIND == G2D_Q_ABSMAX_DYNAMIC) {
+                F top = (F)0;
+                for (int b = lane; b < q; b += 32) top = fmax(top, fabs(y_s[a * q + b]));
+                s = absmax_scale_value(warp_max(top), A.divisor, A.half);
+            }
+            for (int b = lane; b < q; b += 32) {
+                finish_entry<F, KIND>(A, batch, seq, i0 + a, j0 + b, a * q + b, y_s[a * q + b], c_s[a * q + b], s);
+            }
+        }
+        __syncthreads();  // the next batch reuses the shared memory
+    }
+    after_the_launch_before();  // a launch's end implies the ends of all before it, also through CTAs without a super-entry
+}
+
 // Whether a sweep pulls.  A CTA forms stages p q sums of p + q products with 256 threads, where a push spreads them over the whole
 // GPU: from about 600 products per thread on, the push is the faster one, and beyond PULL_ROOM sums there is no room for
 // them.  Measured, push and pull in us: 256 x 1024 as 1 x 32, blocks of 64 stages (264 products per thread) 4437 / 3151;
@@ -346,6 +448,11 @@ bool pull_pays(int64_t stages, int p, int q, bool leading) {
     const double sums = (double)stages * p * q;
     return sums <= PULL_ROOM && sums * (p + q) <= 600.0 * PTH && (!leading || stages > 2);
 }
+
+// Where a stage's blocks of the factors wait in shared memory: up to 32 KB of floats (7 blocks of 32 x 32).  In us, with loads where they are used
+// and staged, blocks of 8 stages: 512 x 2048 as 1 x 16 5250 and 4710, as 1 x 32 5870 and 4970, as 1 x 64 (115 KB) 7870 and 8670; 256 x 1024 as
+// 4 x 32 880 and 770.
+constexpr int PULL_FACTORS = 8192;
 
 template <typename F, int KIND>
 int launch_stage_pull(const SuperArgs<F> &A, cudaStream_t st) {
@@ -358,7 +465,16 @@ int launch_stage_pull(const SuperArgs<F> &A, cudaStream_t st) {
     attribute.val.programmaticStreamSerializationAllowed = 1;
     config.attrs = &attribute;
     config.numAttrs = 1;
-    if (cudaLaunchKernelEx(&config, stage_pull_kernel<F, KIND>, A) != cudaSuccess) return G2D_ERR_CUDA;
+    if (A.pull_stages > 0) {
+        constexpr size_t most = sizeof(F) * (size_t)(6 * PULL_ROOM + PULL_FACTORS);
+        static PerDeviceOnce configured;
+        if (configured.run([&] { return cudaFuncSetAttribute(stage_pull_staged_kernel<F, KIND>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most) == cudaSuccess; }) != G2D_OK)
+            return G2D_ERR_CUDA;
+        config.dynamicSmemBytes = sizeof(F) * (size_t)(4 * A.pull_room + 2 * A.p * A.q + A.pull_stages * (A.p * A.p + A.q * A.q));
+        if (cudaLaunchKernelEx(&config, stage_pull_staged_kernel<F, KIND>, A) != cudaSuccess) return G2D_ERR_CUDA;
+    } else if (cudaLaunchKernelEx(&config, stage_pull_kernel<F, KIND>, A) != cudaSuccess) {
+        return G2D_ERR_CUDA;
+    }
     return check_launch();
 }
 
@@ -509,6 +625,10 @@ int sweep_super(const g2d_super_desc *d, const Plan &plan, cudaStream_t st) {
     const int64_t outer = d->outer_block > inner && d->outer_block < stages ? d->outer_block : inner;
     const int T = d->p * d->q;
     const bool pull = pull_pays(inner, d->p, d->q, d->lead_count > 0);
+    if (pull) {
+        A.pull_room = (int)((inner - 1) * pq);
+        A.pull_stages = (inner - 1) * ((int64_t)d->p * d->p + (int64_t)d->q * d->q) <= PULL_FACTORS ? (int)(inner - 1) : 0;
+    }
     for (int64_t outer_start = 0; outer_start < stages; outer_start += outer) {
         const int64_t outer_stop = outer_start + outer < stages ? outer_start + outer : stages;
         for (int64_t s0 = outer_start; s0 < outer_stop; s0 += inner) {
