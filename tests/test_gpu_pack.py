@@ -60,3 +60,25 @@ def test_sweep_output_round_trips():
     assert packed3.shape == (m, n * 3 // 8)
     assert torch.equal(P.unpack_codes(packed3, scale3, zero3, qmin=0, bits=3, n=n), z3)
     assert P.pack_codes(z[:0], scale[:0], zero, qmin=-8, bits=4).shape == (0, n // 2)
+
+
+# n from 2048 on: rows of one part and of several, a last part and a last group of threads that are not full; scales and zero points out of the
+# range of the short forms in some rows; the same through whole matrices of scales, which the general kernels take
+@pytest.mark.parametrize("m, n", [(3, 2048), (70, 2056), (5, 8192), (2, 8200), (9, 28672)])
+@pytest.mark.parametrize("bits", [2, 4, 8])
+def test_rows_of_one_scale_against_whole_matrices(m, n, bits):
+    import packed_codes as P
+
+    gen = torch.Generator(device="cuda").manual_seed(m + n + bits)
+    qmin = -2 ** (bits - 1)
+    scale = 0.01 + torch.rand(m, 1, generator=gen, device="cuda")
+    zero = torch.randint(0, 3, (m, 1), generator=gen, device="cuda").float()
+    z = (torch.randint(qmin - 2, -qmin + 2, (m, n), generator=gen, device="cuda") - zero) * scale  # some codes out of the field's range
+    scale[0], zero[min(1, m - 1)] = 1e-35, float("nan")
+    z[m - 1, ::97], z[m - 1, 1::97], z[m - 1, 2::97] = float("inf"), float("nan"), -1e38
+    whole = lambda t: t.expand(m, n).contiguous()
+    codes = P.pack_codes(z, scale.expand(m, n), zero.expand(m, n), qmin=qmin, bits=bits)
+    assert torch.equal(codes, P.pack_codes(z, whole(scale), whole(zero), qmin=qmin, bits=bits))
+    back = P.unpack_codes(codes, scale.expand(m, n), zero.expand(m, n), qmin=qmin, bits=bits, n=n)
+    again = P.unpack_codes(codes, whole(scale), whole(zero), qmin=qmin, bits=bits, n=n)
+    assert torch.equal(back.view(torch.int32), again.view(torch.int32))
