@@ -90,8 +90,8 @@ __device__ __forceinline__ void tmem_load_16(uint32_t taddr, uint32_t (&v)[16]) 
 constexpr int KH = 64;                     // k per chunk
 constexpr int HTILE_BYTES = MT * KH * 2;   // 16 KB: 128 rows
 // D fp32, A and B 16 bits (format 0: fp16, 1: bf16), both K-major, M = 128, N = nt
-__host__ __device__ constexpr uint32_t idesc_16(int nt, uint32_t format) {
-    return (1u << 4) | (format << 7) | (format << 10) | ((uint32_t)(nt >> 3) << 17) | ((uint32_t)(MT >> 4) << 24);
+__host__ __device__ constexpr uint32_t idesc_16(int nt, uint32_t format, int mt = MT) {
+    return (1u << 4) | (format << 7) | (format << 10) | ((uint32_t)(nt >> 3) << 17) | ((uint32_t)(mt >> 4) << 24);
 }
 __device__ __forceinline__ void umma_16(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
     asm volatile(
@@ -112,7 +112,57 @@ struct TcRing {
     int failed;
 };
 
-// All threads: barriers, tensor-memory allocation of `cols` columns (by warp 1); returns the accumulator's address.
+// ---- two CTAs of a cluster on one product (cta_group::2): M = 256, 128 rows in each CTA, and half of B in each, so that a CTA fills and reads
+// shared memory for 192 rows where one on its own does for 256 of a 128 x 128 tile.  CTA 0 leads: it issues the MMAs for both. ----
+__device__ __forceinline__ uint32_t cluster_rank() {
+    uint32_t r;
+    asm volatile("mov.u32 %0, %cluster_ctarank;" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ void cluster_sync() { asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+__device__ __forceinline__ uint32_t leaders(uint64_t *bar) {  // the same barrier of CTA 0
+    uint32_t r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(r) : "r"(smem_u32(bar)));
+    return r;
+}
+__device__ __forceinline__ void mbar_arrive_at(uint32_t bar) { asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory"); }
+// as mbar_wait, for what a thread of the other CTA may have arrived at
+__device__ __forceinline__ bool mbar_wait_cluster(uint64_t *bar, uint32_t parity, unsigned nap = 32) {
+    const long long start = clock64();
+    for (;;) {
+        uint32_t ok;
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t}"
+            : "=r"(ok)
+            : "r"(smem_u32(bar)), "r"(parity)
+            : "memory");
+        if (ok) return true;
+        if (clock64() - start > WAIT_CYCLES) return false;
+        __nanosleep(nap);
+    }
+}
+// into this CTA's shared memory, counted at a barrier of either CTA
+__device__ __forceinline__ void tma_load_2d_duo(uint32_t dst, const CUtensorMap *map, int x, int y, uint32_t bar) {
+    asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes.cta_group::2 [%0], [%1, {%2, %3}], [%4];"
+                 ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(bar)
+                 : "memory");
+}
+__device__ __forceinline__ void umma_16_duo(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+        ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+__device__ __forceinline__ void umma_commit_duo(uint64_t *bar) {  // arrives at the barrier of both CTAs
+    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(smem_u32(bar)), "h"((uint16_t)3) : "memory");
+}
+
+// All threads: barriers, tensor-memory allocation of `cols` columns (by warp 1); returns the accumulator's address.  DUO: of both CTAs.
+template <bool DUO = false>
 __device__ __forceinline__ uint32_t tc_ring_setup(TcRing &ring, uint32_t cols) {
     if (threadIdx.x == 0) {
         for (int s = 0; s < STAGES; ++s) {
@@ -124,16 +174,26 @@ __device__ __forceinline__ uint32_t tc_ring_setup(TcRing &ring, uint32_t cols) {
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if ((threadIdx.x >> 5) == 1) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&ring.tmem_slot)), "r"(cols) : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        if (DUO) {
+            asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&ring.tmem_slot)), "r"(cols) : "memory");
+            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+        } else {
+            asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&ring.tmem_slot)), "r"(cols) : "memory");
+            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
+    if (DUO) {
+        __syncwarp();
+        cluster_sync();
+    }
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     return ring.tmem_slot;
 }
 
 // All threads: release tensor memory; returns whether a wait ran out (meaningful in every thread).
+template <bool DUO = false>
 __device__ __forceinline__ bool tc_ring_teardown(TcRing &ring, uint32_t tmem, uint32_t cols) {
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
@@ -143,7 +203,13 @@ __device__ __forceinline__ bool tc_ring_teardown(TcRing &ring, uint32_t tmem, ui
             if ((threadIdx.x & 31) == 0) mbar_wait(&ring.accum, 0);
             __syncwarp();
         }
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(cols) : "memory");
+        if (!DUO) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(cols) : "memory");
+    }
+    if (DUO) {
+        // neither CTA leaves while the other's MMAs may read its shared memory or arrive at its barriers
+        __syncwarp();
+        cluster_sync();
+        if ((threadIdx.x >> 5) == 1) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(cols) : "memory");
     }
     return ring.failed != 0;
 }

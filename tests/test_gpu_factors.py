@@ -65,6 +65,23 @@ def test_against_oracle_and_properties(K, oracle, n, size):
     check_structure(l32, size)
 
 
+@pytest.mark.parametrize("n", [4097, 4300, 8071, 8500])
+def test_large_blocks_against_float64(K, n):
+    """The products of two CTAs per tile (blocks of 4096 rows): second halves of one row, of a tile and a bit, ragged, and a last pair of blocks
+    without one.  Against float64; the tolerance is the one of the smaller factors above, for the largest entry and, by the root of their
+    number below it, for the norm."""
+    gen = torch.Generator(device="cuda").manual_seed(n)
+    x = torch.randn(n + n // 2, n, generator=gen, device="cuda") * torch.exp(0.5 * torch.randn(n, generator=gen, device="cuda"))
+    gram = (x.T @ x).double() / x.size(0)
+    gram += 0.01 * gram.diagonal().mean() * torch.eye(n, device="cuda", dtype=torch.float64)
+    gram = gram.float()
+    l, l32 = K.ldl_of_inverse(gram.double(), 1), K.ldl_of_inverse(gram, 1)
+    check_structure(l32, 1)
+    error = (l32.double() - l).abs()
+    assert error.max().item() < 2e-5 * max(1.0, l.abs().max().item())
+    assert error.norm().item() < 2e-6 * l.norm().item()
+
+
 def test_feedback_factors_and_errors(K):
     gen = torch.Generator(device="cuda").manual_seed(0)
     a = torch.randn(24, 24, generator=gen, device="cuda", dtype=torch.float64)
