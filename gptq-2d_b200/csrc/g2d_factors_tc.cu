@@ -170,34 +170,23 @@ __global__ void __launch_bounds__(TC_THREADS) trinv_tc_kernel(const __grid_const
                 const uint32_t base = smem_base + stage * STAGE;
                 const uint32_t a_hi = base, a_mid = base + HTILE_BYTES, a_lo = base + 2 * HTILE_BYTES;
                 const uint32_t b_hi = base + 3 * HTILE_BYTES, b_mid = b_hi + B_BYTES, b_lo = b_mid + B_BYTES;
-                const auto mma = [](uint32_t d, uint32_t a, uint32_t b, uint32_t accumulate) {
-                    if (DUO) umma_16_duo(d, umma_desc(a), umma_desc(b), DESC, accumulate);
-                    else umma_16(d, umma_desc(a), umma_desc(b), DESC, accumulate);
-                };
 #pragma unroll
                 for (int ks = 0; ks < KH / 16; ++ks) {
                     const uint32_t off = ks * 32;  // 16 values = 32 bytes along the swizzled row
                     const uint32_t fresh = (opens && ks == 0) ? 0u : 1u;
-                    mma(acc_main, a_hi + off, b_hi + off, fresh);
-                    mma(acc_small, a_hi + off, b_mid + off, fresh);
-                    mma(acc_small, a_mid + off, b_hi + off, 1u);
-                    mma(acc_small, a_mid + off, b_mid + off, 1u);
-                    mma(acc_small, a_hi + off, b_lo + off, 1u);
-                    mma(acc_small, a_lo + off, b_hi + off, 1u);
+                    mma<DUO>(acc_main, a_hi + off, b_hi + off, DESC, fresh);
+                    mma<DUO>(acc_small, a_hi + off, b_mid + off, DESC, fresh);
+                    mma<DUO>(acc_small, a_mid + off, b_hi + off, DESC, 1u);
+                    mma<DUO>(acc_small, a_mid + off, b_mid + off, DESC, 1u);
+                    mma<DUO>(acc_small, a_hi + off, b_lo + off, DESC, 1u);
+                    mma<DUO>(acc_small, a_lo + off, b_hi + off, DESC, 1u);
                 }
-                const auto commit = [](uint64_t *bar) {
-                    if (DUO) umma_commit_duo(bar);
-                    else umma_commit(bar);
-                };
-                commit(&ring.empty[stage]);            // arrives when the MMAs above have read the stage
-                if (closes) commit(&acc_full[buf]);    // arrives when the slice is complete in tensor memory
-                if (ch == chunks - 1) commit(&ring.accum);  // and when all of them have completed
+                commit<DUO>(&ring.empty[stage]);       // arrives when the MMAs above have read the stage
+                if (closes) commit<DUO>(&acc_full[buf]);    // arrives when the slice is complete in tensor memory
+                if (ch == chunks - 1) commit<DUO>(&ring.accum);  // and when all of them have completed
             }
             // on a time-out: what has been issued so far
-            if (ch < chunks) {
-                if (DUO) umma_commit_duo(&ring.accum);
-                else umma_commit(&ring.accum);
-            }
+            if (ch < chunks) commit<DUO>(&ring.accum);
         }
     } else {
         // epilogue warps: lanes 32 q .. 32 q + 31 of tensor memory, q = warp % 4; one accumulator row per thread, whose
@@ -354,18 +343,8 @@ int launch_trinv_tc(int count, const FactorPlanes *problems, cudaStream_t stream
             if (b < DUO_BLOCK) {
                 trinv_tc_kernel<false><<<dim3((unsigned)(pairs * count), (unsigned)tiles, (unsigned)tiles), TC_THREADS, smem, stream>>>(job);
             } else {
-                cudaLaunchConfig_t config{};
-                config.gridDim = dim3((unsigned)(2 * pairs * count), (unsigned)(second ? tiles / 2 : tiles), (unsigned)(second ? tiles : tiles / 2));
-                config.blockDim = dim3(TC_THREADS);
-                config.dynamicSmemBytes = duo_smem;
-                config.stream = stream;
-                cudaLaunchAttribute attribute{};
-                attribute.id = cudaLaunchAttributeClusterDimension;
-                attribute.val.clusterDim.x = 2;
-                attribute.val.clusterDim.y = attribute.val.clusterDim.z = 1;
-                config.attrs = &attribute;
-                config.numAttrs = 1;
-                if (cudaLaunchKernelEx(&config, trinv_tc_kernel<true>, job) != cudaSuccess) return G2D_ERR_CUDA;
+                const dim3 grid((unsigned)(2 * pairs * count), (unsigned)(second ? tiles / 2 : tiles), (unsigned)(second ? tiles : tiles / 2));
+                if (launch_duo(trinv_tc_kernel<true>, grid, TC_THREADS, duo_smem, stream, job) != G2D_OK) return G2D_ERR_CUDA;
             }
             if (check_launch() != G2D_OK) return G2D_ERR_CUDA;
         }
@@ -520,7 +499,7 @@ int launch_syrk_tc(int count, const SyrkTcTarget *targets, cudaStream_t stream) 
         square += lower_tiles<128>(targets[z].t_hi) - lower_tiles<128>(targets[z].t_lo);
     }
     if (square <= 0) return G2D_OK;
-    const bool use_wide = wide_tiles_pay(wide, square);
+    const bool use_wide = tiles_that_pay(square, wide) == WIDE_TILES;
     // Several tiles per CTA once there are more than two waves of them, but few enough that an SM comes free every other
     // moment: the diagonal blocks and panels of the next group, on a stream of higher priority, wait for one.
     const int64_t tiles = use_wide ? wide : square;

@@ -4,21 +4,21 @@
 // counterpart there.
 //
 // X^T is first written as K-major fp16 pairs [n][k], every channel scaled by a power of two of its own (the channel is the
-// index that is not summed over, so the scale comes out of the product again), then every 128 x 256 tile that touches the
-// lower triangle of H is one CTA's (of one CTA per SM): TMA into a two-stage ring of 96 KB, tcgen05.mma kind::f16 with three products per k step
-// into tensor memory, eight warps that add the accumulators up in registers slice of k by slice of k, and at the end
+// index that is not summed over, so the scale comes out of the product again), then every 256 x 256 tile that touches the
+// lower triangle of H is that of a cluster of two CTAs (one CTA per SM; smaller tiles where those fill their waves better, see
+// tiles_that_pay): TMA into a three-stage ring of 64 KB in each, tcgen05.mma kind::f16 with three products per k step into tensor memory, eight warps that add the accumulators up in registers slice of k by slice of k, and at the end
 // write H and its mirror image.  Every entry of H has one owner, so the result does not depend on scheduling.
 //
-// Bound: tensor pipe and shared-memory port.  A 128 x 256 x 16 MMA reads 12 KB of operands in 128 cycles and a chunk's 96 KB
-// arrive in the 1536 cycles of its MMAs: 160 of the port's 128 bytes per cycle, so 80 % of the tensor rate; the 128 x 128
-// tf32 tiles before it were held at 60 % of half that rate, and added every slice to H in global memory (8.6 GB of
-// reductions at 8192 x 8192).  Measured at 8192 samples of 8192 channels: 4.61 ms before, 1.63 ms now (1.01 PFLOP/s of fp16
-// products; 8 waves of tiles of which the last is a seventh full).
+// Bound: tensor pipe.  A 128 x 256 x 16 MMA of one CTA reads 12 KB of operands in 128 cycles and a chunk's 96 KB arrive in the 1536 cycles
+// of its MMAs: 160 of the port's 128 bytes per cycle, so 80 % of the tensor rate.  Two CTAs with half of B each read 8 KB and
+// fill 64 KB: 107 bytes per cycle.  8192 samples of 8192 channels: 4.61 ms with 128 x 128 tf32 tiles (60 % of half the rate, every slice added to
+// H in global memory), 1.69 ms with 128 x 256, 1.54 ms now; 2048 samples of 4096 channels 153 and 152 us.
 #include "g2d_tc.cuh"
 
 namespace g2d {
 
-constexpr int GRAM_STAGES = 2;
+constexpr int GRAM_STAGES = 2, GRAM_DUO_STAGES = 3;
+constexpr size_t GRAM_DUO_BYTES = 4 * HTILE_BYTES;  // 128 rows of A and of B, two planes each
 // Slices of the k range (see pair_gemm): the diagonal of a Gram matrix is a sum of squares, which one accumulator over
 // k = 8192 truncates to 9e-5 relative.
 constexpr int GRAM_SLICE = 2;  // chunks per slice: 128 samples
@@ -111,26 +111,37 @@ struct GramJob {
     int *flag;
 };
 
-template <int NT>
+template <int NT, bool DUO>
 __global__ void __launch_bounds__(PAIR_THREADS, 1) gram_tc_kernel(const __grid_constant__ GramJob job) {
     constexpr int MINE = NT / 2;  // columns per reading warp
     extern __shared__ unsigned char tc_smem_raw[];
-    __shared__ __align__(8) PairRing<GRAM_STAGES> ring;
+    constexpr int NSTAGE = DUO ? GRAM_DUO_STAGES : GRAM_STAGES, B_ROWS = DUO ? NT / 2 : NT;
+    __shared__ __align__(8) PairRing<NSTAGE> ring;
+    const int rank = DUO ? (int)cluster_rank() : 0;
     const int64_t n = job.n;
     const uint32_t smem_base = (smem_u32(tc_smem_raw) + 1023u) & ~1023u;
     auto next = [&](int it, PairTile &t) {
-        const int64_t lin = blockIdx.x + (int64_t)it * gridDim.x;
+        const int64_t lin = (blockIdx.x + (int64_t)it * gridDim.x) / (DUO ? 2 : 1);
         if (lin >= job.tiles) return false;
         int I2, J2;
-        lower_tile<NT>(lin, I2, J2);
+        if (DUO) {
+            lower_tile<128>(lin, I2, J2);
+            I2 = 2 * I2 + rank;
+        } else {
+            lower_tile<NT>(lin, I2, J2);
+        }
         t = PairTile{I2 * MT, J2 * NT, job.chunks};
         return true;
     };
     auto load = [&](const PairTile &t, int ch, uint32_t dst, uint64_t *bar) {
-        tma_load_2d(dst, &job.a_hi, ch * KH, t.i0, bar);
-        tma_load_2d(dst + HTILE_BYTES, &job.a_lo, ch * KH, t.i0, bar);
-        tma_load_2d(dst + 2 * HTILE_BYTES, &job.b_hi, ch * KH, t.j0, bar);
-        tma_load_2d(dst + 2 * HTILE_BYTES + NT * KH * 2, &job.b_lo, ch * KH, t.j0, bar);
+        const auto bring = [&](uint32_t to, const CUtensorMap *map, int row) {
+            if (DUO) tma_load_2d_duo(to, map, ch * KH, row, leaders(bar));
+            else tma_load_2d(to, map, ch * KH, row, bar);
+        };
+        bring(dst, &job.a_hi, t.i0);
+        bring(dst + HTILE_BYTES, &job.a_lo, t.i0);
+        bring(dst + 2 * HTILE_BYTES, &job.b_hi, t.j0 + rank * B_ROWS);
+        bring(dst + 2 * HTILE_BYTES + B_ROWS * KH * 2, &job.b_lo, t.j0 + rank * B_ROWS);
     };
     auto finish = [&](const PairTile &t, int q, int lane, int c0, float (&total)[MINE], uint32_t) {
         const int64_t gi = (int64_t)t.i0 + q * 32 + lane;
@@ -173,21 +184,23 @@ __global__ void __launch_bounds__(PAIR_THREADS, 1) gram_tc_kernel(const __grid_c
             }
         }
     };
-    const bool failed = pair_gemm<NT, GRAM_STAGES, GRAM_SLICE>(ring, smem_base, next, load, finish);
+    const bool failed = pair_gemm<NT, NSTAGE, GRAM_SLICE, DUO>(ring, smem_base, next, load, finish);
     if (threadIdx.x == 0 && failed && job.flag) atomicExch(job.flag, -1);
 }
 
-template <int NT>
+template <int NT, bool DUO>
 static int launch_gram(GramJob &job, const __half *hi, const __half *lo, int64_t kp, int64_t tiles, cudaStream_t st) {
     static PerDeviceOnce configured;
-    constexpr size_t smem = (size_t)GRAM_STAGES * pair_stage_bytes<NT> + 1024;
-    if (configured.run([&] { return cudaFuncSetAttribute(gram_tc_kernel<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) == cudaSuccess; }) != G2D_OK)
+    constexpr size_t smem = (DUO ? GRAM_DUO_STAGES * GRAM_DUO_BYTES : (size_t)GRAM_STAGES * pair_stage_bytes<NT>) + 1024;
+    constexpr int B_ROWS = DUO ? NT / 2 : NT;
+    if (configured.run([&] { return cudaFuncSetAttribute(gram_tc_kernel<NT, DUO>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) == cudaSuccess; }) != G2D_OK)
         return G2D_ERR_CUDA;
-    if (!make_map_16(&job.a_hi, hi, job.n, kp, MT) || !make_map_16(&job.a_lo, lo, job.n, kp, MT) || !make_map_16(&job.b_hi, hi, job.n, kp, NT) ||
-        !make_map_16(&job.b_lo, lo, job.n, kp, NT))
+    if (!make_map_16(&job.a_hi, hi, job.n, kp, MT) || !make_map_16(&job.a_lo, lo, job.n, kp, MT) || !make_map_16(&job.b_hi, hi, job.n, kp, B_ROWS) ||
+        !make_map_16(&job.b_lo, lo, job.n, kp, B_ROWS))
         return G2D_ERR_CUDA;
     job.tiles = tiles;
-    gram_tc_kernel<NT><<<(unsigned)(tiles < 148 ? tiles : 148), PAIR_THREADS, smem, st>>>(job);
+    if (DUO) return launch_duo(gram_tc_kernel<NT, DUO>, dim3(2 * (unsigned)(tiles < 74 ? tiles : 74)), PAIR_THREADS, smem, st, job);
+    gram_tc_kernel<NT, DUO><<<(unsigned)(tiles < 148 ? tiles : 148), PAIR_THREADS, smem, st>>>(job);
     return check_launch();
 }
 
@@ -242,7 +255,9 @@ extern "C" int g2d_gram_accumulate(int64_t n, int64_t k, const float *x, float a
     job.chunks = (int)ceil_div(kp, (int64_t)KH);
     job.alpha = alpha;
     job.flag = status_flag;
-    const int64_t wide = lower_tiles<256>(rows), square = lower_tiles<128>(rows);
-    if (wide_tiles_pay(wide, square)) return launch_gram<256>(job, hi, lo, kp, wide, st);
-    return launch_gram<128>(job, hi, lo, kp, square, st);
+    const int64_t square = lower_tiles<128>(rows), wide = lower_tiles<256>(rows), duo = duo_tiles(ceil_div(rows, (int64_t)2));
+    const TileChoice choice = tiles_that_pay(square, wide, duo);
+    if (choice == DUO_TILES) return launch_gram<256, true>(job, hi, lo, kp, duo, st);
+    if (choice == WIDE_TILES) return launch_gram<256, false>(job, hi, lo, kp, wide, st);
+    return launch_gram<128, false>(job, hi, lo, kp, square, st);
 }

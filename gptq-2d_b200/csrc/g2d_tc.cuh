@@ -161,6 +161,49 @@ __device__ __forceinline__ void umma_commit_duo(uint64_t *bar) {  // arrives at 
     asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(smem_u32(bar)), "h"((uint16_t)3) : "memory");
 }
 
+// For one CTA or two
+template <bool DUO>
+__device__ __forceinline__ void mma(uint32_t tmem_d, uint32_t a, uint32_t b, uint32_t idesc, uint32_t accumulate) {
+    if (DUO) umma_16_duo(tmem_d, umma_desc(a), umma_desc(b), idesc, accumulate);
+    else umma_16(tmem_d, umma_desc(a), umma_desc(b), idesc, accumulate);
+}
+template <bool DUO>
+__device__ __forceinline__ void commit(uint64_t *bar) {
+    if (DUO) umma_commit_duo(bar);
+    else umma_commit(bar);
+}
+template <bool DUO>
+__device__ __forceinline__ void tmem_alloc(uint32_t *slot, uint32_t cols) {  // one warp (of each CTA)
+    if (DUO) {
+        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(slot)), "r"(cols) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+    } else {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(slot)), "r"(cols) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+}
+template <bool DUO>
+__device__ __forceinline__ void tmem_free(uint32_t tmem, uint32_t cols) {
+    if (DUO) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(cols) : "memory");
+    else asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(cols) : "memory");
+}
+// a launch of clusters of two CTAs along x
+template <typename Job>
+inline int launch_duo(void (*kernel)(Job), dim3 grid, int threads, size_t smem, cudaStream_t stream, const Job &job) {
+    cudaLaunchConfig_t config{};
+    config.gridDim = grid;
+    config.blockDim = dim3((unsigned)threads);
+    config.dynamicSmemBytes = smem;
+    config.stream = stream;
+    cudaLaunchAttribute attribute{};
+    attribute.id = cudaLaunchAttributeClusterDimension;
+    attribute.val.clusterDim.x = 2;
+    attribute.val.clusterDim.y = attribute.val.clusterDim.z = 1;
+    config.attrs = &attribute;
+    config.numAttrs = 1;
+    return cudaLaunchKernelEx(&config, kernel, job) == cudaSuccess ? check_launch() : G2D_ERR_CUDA;
+}
+
 // All threads: barriers, tensor-memory allocation of `cols` columns (by warp 1); returns the accumulator's address.  DUO: of both CTAs.
 template <bool DUO = false>
 __device__ __forceinline__ uint32_t tc_ring_setup(TcRing &ring, uint32_t cols) {
@@ -173,15 +216,7 @@ __device__ __forceinline__ uint32_t tc_ring_setup(TcRing &ring, uint32_t cols) {
         ring.failed = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    if ((threadIdx.x >> 5) == 1) {
-        if (DUO) {
-            asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&ring.tmem_slot)), "r"(cols) : "memory");
-            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
-        } else {
-            asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&ring.tmem_slot)), "r"(cols) : "memory");
-            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-        }
-    }
+    if ((threadIdx.x >> 5) == 1) tmem_alloc<DUO>(&ring.tmem_slot, cols);
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     if (DUO) {
@@ -203,14 +238,13 @@ __device__ __forceinline__ bool tc_ring_teardown(TcRing &ring, uint32_t tmem, ui
             if ((threadIdx.x & 31) == 0) mbar_wait(&ring.accum, 0);
             __syncwarp();
         }
-        if (!DUO) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(cols) : "memory");
     }
     if (DUO) {
         // neither CTA leaves while the other's MMAs may read its shared memory or arrive at its barriers
         __syncwarp();
         cluster_sync();
-        if ((threadIdx.x >> 5) == 1) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(cols) : "memory");
     }
+    if ((threadIdx.x >> 5) == 1) tmem_free<DUO>(tmem, cols);
     return ring.failed != 0;
 }
 
@@ -282,19 +316,21 @@ struct PairRing {
 // A CTA takes several tiles, one after the other, so that a tile's loads and MMAs run while the results of the one before leave.
 // next(number, tile): the CTA's tile of that number, false past the last.  load(tile, chunk, destination, barrier): A_hi, A_lo,
 // B_hi, B_lo tiles one after the other.  finish(tile, q, lane, first column, totals, 4 KB of shared memory of the warp's own
-// behind the stages).  scale(tile, slice, q, column), optional: what a slice's sums are multiplied by, the same for 64 columns.
+// behind the stages).  DUO: by two CTAs of a cluster whose tiles differ in i0 only; load brings half of B's rows and counts at the barrier
+// of CTA 0.  scale(tile, slice, q, column), optional: what a slice's sums are multiplied by, the same for 64 columns.
 // Returns whether a wait ran out.
 struct PairTile {
     int i0, j0, chunks;
     int k0 = 0, which = 0;  // first k and a number of the caller's
 };
 struct PairNoScale {};
-template <int NT, int NSTAGE, int SLICE, typename Next, typename Load, typename Finish, typename Scale = PairNoScale>
+template <int NT, int NSTAGE, int SLICE, bool DUO = false, typename Next, typename Load, typename Finish, typename Scale = PairNoScale>
 __device__ __forceinline__ bool pair_gemm(PairRing<NSTAGE> &ring, uint32_t smem_base, Next next, Load load, Finish finish, Scale scale = Scale()) {
     constexpr bool SCALED = !std::is_same<Scale, PairNoScale>::value;
-    constexpr int B_BYTES = NT * KH * 2, STAGE = 2 * HTILE_BYTES + 2 * B_BYTES, MINE = NT / 2;
-    constexpr uint32_t COLS = 2 * NT, DESC = idesc_16(NT, 0);
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    constexpr int B_BYTES = NT * KH * 2 / (DUO ? 2 : 1), STAGE = 2 * HTILE_BYTES + 2 * B_BYTES, MINE = NT / 2;
+    constexpr uint32_t COLS = 2 * NT, DESC = idesc_16(NT, 0, DUO ? 2 * MT : MT);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, rank = DUO ? (int)cluster_rank() : 0;
+    const auto wait = [](uint64_t *bar, uint32_t parity, unsigned nap = 32) { return DUO ? mbar_wait_cluster(bar, parity, nap) : mbar_wait(bar, parity, nap); };
     if (threadIdx.x == 0) {
         for (int s = 0; s < NSTAGE; ++s) {
             mbar_init(&ring.full[s], 1);
@@ -302,17 +338,18 @@ __device__ __forceinline__ bool pair_gemm(PairRing<NSTAGE> &ring, uint32_t smem_
         }
         for (int s = 0; s < 2; ++s) {
             mbar_init(&ring.acc_full[s], 1);
-            mbar_init(&ring.acc_empty[s], 8);  // one arrival per reading warp
+            mbar_init(&ring.acc_empty[s], DUO ? 16 : 8);  // one arrival per reading warp, of both CTAs at the leader's
         }
         ring.failed = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    if (warp == 1) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&ring.tmem)), "r"(COLS) : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-    }
+    if (warp == 1) tmem_alloc<DUO>(&ring.tmem, COLS);
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
+    if (DUO) {
+        __syncwarp();
+        cluster_sync();
+    }
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = ring.tmem;
     // the roles count chunks and slices over all tiles of the CTA: stages and accumulators are used in turn throughout
@@ -323,14 +360,20 @@ __device__ __forceinline__ bool pair_gemm(PairRing<NSTAGE> &ring, uint32_t smem_
             for (int it = 0; !ring.failed && next(it, tile); ++it) {
                 for (int ch = 0; ch < tile.chunks; ++ch, ++c) {
                     const int stage = c % NSTAGE, round = c / NSTAGE;
-                    if (round > 0 && !mbar_wait(&ring.empty[stage], (round - 1) & 1)) { ring.failed = 1; break; }
-                    mbar_expect_tx(&ring.full[stage], STAGE);
+                    if (round > 0 && !wait(&ring.empty[stage], (round - 1) & 1)) { ring.failed = 1; break; }
+                    // DUO: both CTAs' bytes count at the leader's barrier (they may do so before it expects them: the phase waits for its arrival)
+                    if (rank == 0) mbar_expect_tx(&ring.full[stage], DUO ? 2 * STAGE : STAGE);
                     load(tile, ch, smem_base + stage * STAGE, &ring.full[stage]);
                 }
             }
+            if (DUO && !ring.failed) {
+                // the leader's commits arrive here as well: none may be under way when this CTA ends (those of the accumulators are awaited below)
+                for (int k = max(c - NSTAGE, 0); k < c; ++k)
+                    if (!wait(&ring.empty[k % NSTAGE], (k / NSTAGE) & 1)) ring.failed = 1;
+            }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
+        if (lane == 0 && rank == 0) {
             PairTile tile;
             int c = 0, slice = 0;
             for (int it = 0; !ring.failed && next(it, tile); ++it) {
@@ -338,21 +381,21 @@ __device__ __forceinline__ bool pair_gemm(PairRing<NSTAGE> &ring, uint32_t smem_
                     const int stage = c % NSTAGE, round = c / NSTAGE, buf = slice & 1;
                     const bool opens = ch % SLICE == 0, closes = ch % SLICE == SLICE - 1 || ch == tile.chunks - 1;
                     // the accumulator must have been read out by the warps of the slice two before
-                    if (opens && slice >= 2 && !mbar_wait(&ring.acc_empty[buf], ((slice >> 1) - 1) & 1)) { ring.failed = 1; break; }
-                    if (!mbar_wait(&ring.full[stage], round & 1)) { ring.failed = 1; break; }
+                    if (opens && slice >= 2 && !wait(&ring.acc_empty[buf], ((slice >> 1) - 1) & 1)) { ring.failed = 1; break; }
+                    if (!wait(&ring.full[stage], round & 1)) { ring.failed = 1; break; }
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     const uint32_t d = tmem + (uint32_t)(buf * NT);
                     const uint32_t a_hi = smem_base + stage * STAGE, a_lo = a_hi + HTILE_BYTES, b_hi = a_hi + 2 * HTILE_BYTES, b_lo = b_hi + B_BYTES;
 #pragma unroll
                     for (int ks = 0; ks < KH / 16; ++ks) {
                         const uint32_t off = ks * 32;  // 16 values = 32 bytes along the swizzled row
-                        umma_16(d, umma_desc(a_hi + off), umma_desc(b_hi + off), DESC, (opens && ks == 0) ? 0u : 1u);
-                        umma_16(d, umma_desc(a_lo + off), umma_desc(b_hi + off), DESC, 1u);
-                        umma_16(d, umma_desc(a_hi + off), umma_desc(b_lo + off), DESC, 1u);
+                        mma<DUO>(d, a_hi + off, b_hi + off, DESC, (opens && ks == 0) ? 0u : 1u);
+                        mma<DUO>(d, a_lo + off, b_hi + off, DESC, 1u);
+                        mma<DUO>(d, a_hi + off, b_lo + off, DESC, 1u);
                     }
-                    umma_commit(&ring.empty[stage]);  // arrives when the MMAs above have read the stage
+                    commit<DUO>(&ring.empty[stage]);  // arrives when the MMAs above have read the stage
                     if (closes) {
-                        umma_commit(&ring.acc_full[buf]);  // arrives when the slice is complete in tensor memory
+                        commit<DUO>(&ring.acc_full[buf]);  // arrives when the slice is complete in tensor memory
                         ++slice;
                     }
                 }
@@ -377,7 +420,7 @@ __device__ __forceinline__ bool pair_gemm(PairRing<NSTAGE> &ring, uint32_t smem_
 #pragma unroll
                     for (int g = 0; g < MINE / 64; ++g) factor[g] = scale(tile, s, q, c0 + g * 64);
                 }
-                const bool ok = mbar_wait(&ring.acc_full[buf], (slice >> 1) & 1, 64);
+                const bool ok = wait(&ring.acc_full[buf], (slice >> 1) & 1, 64);
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 if (!ok) ring.failed = 1;
                 go = __all_sync(0xffffffffu, ok && !ring.failed);  // warp-uniform: the tensor-memory loads are warp-wide
@@ -395,7 +438,10 @@ __device__ __forceinline__ bool pair_gemm(PairRing<NSTAGE> &ring, uint32_t smem_
                 // this warp has read the accumulator: hand it back to the MMA warp
                 asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
                 __syncwarp();
-                if (lane == 0) mbar_arrive(&ring.acc_empty[buf]);
+                if (lane == 0) {
+                    if (DUO) mbar_arrive_at(leaders(&ring.acc_empty[buf]));
+                    else mbar_arrive(&ring.acc_empty[buf]);
+                }
             }
             if (go) finish(tile, q, lane, c0, total, smem_base + (uint32_t)(NSTAGE * STAGE + (warp - 2) * BOX_BYTES));
         }
@@ -403,8 +449,12 @@ __device__ __forceinline__ bool pair_gemm(PairRing<NSTAGE> &ring, uint32_t smem_
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
-    if (warp == 1)
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(COLS) : "memory");
+    if (DUO) {
+        // neither CTA leaves while the other's MMAs may read its shared memory or arrive at its barriers
+        __syncwarp();
+        cluster_sync();
+    }
+    if (warp == 1) tmem_free<DUO>(tmem, COLS);
     return ring.failed != 0;
 }
 
@@ -413,6 +463,8 @@ template <int NT>
 __host__ __device__ inline int64_t lower_tiles(int64_t rows) {  // of the first `rows` tile rows
     return NT == 256 ? (rows / 2) * (rows / 2 + 1) + (rows % 2) * (rows / 2 + 1) : rows * (rows + 1) / 2;
 }
+// Tiles of 256 x 256: tile rows 2 a and 2 a + 1 together, a triangle of squares again.
+__host__ __device__ inline int64_t duo_tiles(int64_t row_pairs) { return lower_tiles<128>(row_pairs); }
 template <int NT>
 __device__ __forceinline__ void lower_tile(int64_t lin, int &I, int &J) {
     if (NT == 256) {  // rows 2 a and 2 a + 1 have a + 1 tiles each
@@ -430,9 +482,15 @@ __device__ __forceinline__ void lower_tile(int64_t lin, int &I, int &J) {
         J = (int)(lin - a * (a + 1) / 2);
     }
 }
-// A 128 x 256 tile takes 1.5 times as long as a 128 x 128 one (80 against 60 % of the tensor rate for twice the work), so the wide
-// tiles are for problems with enough of them: whole waves over the 148 SMs decide.
-inline bool wide_tiles_pay(int64_t wide, int64_t square) { return 3 * ceil_div(wide, (int64_t)148) <= 2 * ceil_div(square, (int64_t)148); }
+// Whole waves over the 148 SMs decide.  A 128 x 256 tile takes 1.5 times as long as a 128 x 128 one (80 against 60 % of the tensor rate for
+// twice the work); two CTAs take 1.25 times as long for 256 x 256, but such tiles fill a wave less well.  Gram of 8192 samples, in us, with
+// 128 x 128, 128 x 256 and 256 x 256: 169, 170, 200 at n = 2048 (1, 1 and 1 waves), 296, 237, 367 at 2944 (2, 1, 2), 410, 403, 373 at 3072
+// (3, 2, 2), 550, 433, 408 at 4096 (4, 2, 2), 809, 641, 750 at 5248 (6, 3, 4), 2000, 1690, 1540 at 8192 (15, 8, 8).
+enum TileChoice { SQUARE_TILES, WIDE_TILES, DUO_TILES };
+inline TileChoice tiles_that_pay(int64_t square, int64_t wide, int64_t duo = 0) {  // duo: 0 where two CTAs do not share a tile
+    const int64_t s = 4 * ceil_div(square, (int64_t)148), w = 6 * ceil_div(wide, (int64_t)148), d = 5 * ceil_div(duo, (int64_t)74);
+    return duo > 0 && d <= s && d <= w ? DUO_TILES : w <= s ? WIDE_TILES : SQUARE_TILES;
+}
 
 // ---- host side: tensor maps ----
 typedef CUresult (*EncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *,

@@ -123,6 +123,13 @@ def test_gram_at_edges(k, n, offset):
     assert ((h.double() - want).abs() <= bound).all() and torch.equal(h, h.T)
 
 
+# two CTAs per 256 x 256 tile: a second tile row of four channels or none, fewer chunks than stages and more, one tile per cluster and several,
+# and one CTA per 128 x 256 tile beside them (n = 2944)
+@pytest.mark.parametrize("k, n", [(64, 2180), (130, 2052), (600, 2816), (1030, 3072), (700, 2944), (449, 5000)])
+def test_gram_of_two_ctas_per_tile(k, n):
+    test_gram_at_edges(k, n, 0)
+
+
 # block rows of 64, groups of four and pairs of groups: one group, one pair, a pair cut short on either side, a last block row
 # that is nearly empty, and pairs whose sizes start in different halves of a pair
 @pytest.mark.parametrize("n, other", [(257, 64), (320, 1025), (513, 258), (769, 2049), (1025, 513), (1281, 1283), (3001, 700)])
