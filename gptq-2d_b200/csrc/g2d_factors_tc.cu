@@ -4,14 +4,14 @@
 // The inverse Lf = T^{-1} of the lower triangular Cholesky factor is built by doubling: at level b every aligned pair
 // of finished b x b diagonal blocks [A^{-1} 0; . B^{-1}] of Lf is completed by X = -B^{-1} (C A^{-1}) with
 // C = T[second half rows, first half columns].  From b = 128 on, both products of a level run here as tcgen05.mma
-// kind::f16 GEMMs over output tiles of 128 x 128 (256 x 128 for two CTAs) on three bf16 planes per operand (six products per k step, see
+// kind::f16 GEMMs over output tiles of 128 x 128 (256 x 256 for two CTAs) on three bf16 planes per operand (six products per k step, see
 // "Precision" below).  The MMA wants both operands K-major, so the first product is formed transposed,
 //     W^T[j][i] = sum_k Lf^T[j][k] T[i][k]        (k from the tile's first row j0 to the end of the first half)
 //     X[i][j]   = -sum_k Lf[i][k] W^T[j][k]       (k from the start of the second half through the tile's rows)
 // and every operand is kept as ready-made hi / mid / lo planes: Lf and its transpose (both written by the second
 // product's epilogue), and one plane triple whose lower triangle holds T and whose upper triangle receives W^T.
-// Same pipeline as the macro updates of the sweep: one warp issues TMA loads into a two-stage ring of 96 KB stages (three of 72 KB in
-// each of two CTAs), one warp issues the MMAs, four warps read the accumulators and store; every wait is bounded.
+// Same pipeline as the macro updates of the sweep: one warp issues TMA loads into a two-stage ring of 96 KB stages, one
+// warp issues the MMAs, four warps (eight in the kernel for two CTAs) read the accumulators and store; every wait is bounded.
 #include <cstring>
 
 #include "g2d_tc.cuh"
@@ -19,7 +19,7 @@
 namespace g2d {
 
 struct FactorMaps {
-    CUtensorMap out[3], outt[3], tw[3], tw_half[3];  // hi, mid, lo; tw_half: boxes of 64 rows
+    CUtensorMap out[3], outt[3], tw[3];  // hi, mid, lo
 };
 struct TrinvJob {
     FactorMaps maps[2];
@@ -46,17 +46,14 @@ constexpr int TRINV_STAGES = 2;
 constexpr int TRINV_STAGE_BYTES = 6 * HTILE_BYTES;         // A hi, mid, lo; B hi, mid, lo
 constexpr int TRINV_SLICE = 4;                             // chunks per slice: k = 256
 constexpr uint32_t TRINV_TMEM_COLS = 4 * MT;               // two alternating pairs of (main, correction) accumulators
-// Two CTAs of a cluster per 256 x 128 tile at the levels with large blocks.  Alone a CTA reads 256 rows of shared memory per MMA and fills
-// 768 per six of them, 1.5 times what the port gives in the time of the MMAs; two CTAs with half of B each read 192 and fill 576, and
-// a third stage has room.  The ranges of k of the two tiles differ by 128: where one has none its operand is filled with zeros (a load
-// from outside the matrix), and the last wave of a level is coarser, so small blocks lose: a whole preparation with two CTAs from b = 256 on
-// takes 647 us at 1024 and 1024 (636 alone), 2.62 ms at 4096 and 4096 (2.57), 7.66 ms at 8192 and 8192 (7.63), 92 ms at 8192 and 28672 (96.5);
-// from b = 2048 on 2.59, 7.62 and 93.5, from b = 4096 on 2.57, 7.60 and 92, from b = 8192 on 2.57, 7.63 and 93.7.
+constexpr uint32_t TRINV_DESC = idesc_16(MT, 1);           // bf16
+// Two CTAs of a cluster per 256 x 256 tile (trinv_duo_kernel) at the levels with large blocks.  Alone a CTA reads 256 rows of shared memory per MMA of
+// 64 cycles and fills 768 per six of them, 1.5 times what the port gives meanwhile; two CTAs read 256 each (384 with the other's half) per MMA of 128
+// cycles and fill 768 per six.  Tiles of the moment share their strips in L2.  Small blocks lose by the coarser tiles: a whole preparation
+// with two CTAs from b = 2048 on takes 1.85 ms at 2048 and 3000 (1.79 alone), 2.68 ms at 4096 and 4096 (2.59), 7.50 at 8192 and 8192 (7.67), 84.2 at
+// 8192 and 28672 (97); from b = 4096 on 1.79, 2.59, 7.47 and 84.6, from b = 8192 on 1.79, 2.59, 7.68 and 85.3.  (256 x 128 tiles with half of
+// the second operand each, three stages and alternating accumulators: 92 ms at 8192 and 28672.)
 constexpr int DUO_BLOCK = 4096;
-constexpr int DUO_STAGES = 3;
-constexpr int DUO_HALF = HTILE_BYTES / 2;                  // 64 rows of B
-constexpr int DUO_STAGE_BYTES = 3 * HTILE_BYTES + 3 * DUO_HALF;
-static_assert(DUO_STAGES <= STAGES, "the ring has a barrier per stage");
 
 // fp32 -> three bf16 values with a = hi + mid + lo exactly (8 significant bits each)
 __device__ __forceinline__ void split_bf16_3(float a, __nv_bfloat16 &hi, __nv_bfloat16 &mid, __nv_bfloat16 &lo) {
@@ -66,42 +63,80 @@ __device__ __forceinline__ void split_bf16_3(float a, __nv_bfloat16 &hi, __nv_bf
     lo = __float2bfloat16_rn(r - __bfloat162float(mid));
 }
 
-template <bool DUO>
+// A thread's row gi of a finished tile, columns n0 .. n0 + 127
+__device__ __forceinline__ void trinv_write(const FactorPlanes &P, int second, int64_t gi, int64_t n0, int64_t r2, const float (&total)[MT]) {
+    const int64_t n = P.n, ld = P.ld;
+    const bool vec = n % 4 == 0;  // rows of the float matrix are 16-byte multiples; those of the planes always are
+#pragma unroll
+    for (int cb = 0; cb < MT / 8; ++cb) {
+        const int64_t gj0 = n0 + cb * 8;
+        __align__(16) __nv_bfloat16 h[8];
+        __align__(16) __nv_bfloat16 c[8];
+        __align__(16) __nv_bfloat16 l[8];
+        if (!second) {
+            // W^T[gi][gj]: gi is inside the first half (always a row of the matrix), gj is cut at r2; a group of eight that
+            // reaches past it ends in the padding of its row (its extra products are zero)
+            if (gj0 < r2) {
+#pragma unroll
+                for (int e = 0; e < 8; ++e) split_bf16_3(total[cb * 8 + e], h[e], c[e], l[e]);
+                *reinterpret_cast<uint4 *>(P.tw_hi + gi * ld + gj0) = *reinterpret_cast<const uint4 *>(h);
+                *reinterpret_cast<uint4 *>(P.tw_mid + gi * ld + gj0) = *reinterpret_cast<const uint4 *>(c);
+                *reinterpret_cast<uint4 *>(P.tw_lo + gi * ld + gj0) = *reinterpret_cast<const uint4 *>(l);
+            }
+        } else if (gi < r2) {
+            // X[gi][gj] = -acc (gj is inside the first half): the inverse itself, its split, and the split of its transpose
+            // (coalesced across the lanes)
+            float *dst = P.out + gi * n + gj0;
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+                const float v = -total[cb * 8 + e];
+                split_bf16_3(v, h[e], c[e], l[e]);
+                P.outt_hi[(gj0 + e) * ld + gi] = h[e];
+                P.outt_mid[(gj0 + e) * ld + gi] = c[e];
+                P.outt_lo[(gj0 + e) * ld + gi] = l[e];
+                if (!vec) dst[e] = v;
+            }
+            if (vec) {
+                *reinterpret_cast<float4 *>(dst) = make_float4(-total[cb * 8], -total[cb * 8 + 1], -total[cb * 8 + 2], -total[cb * 8 + 3]);
+                *reinterpret_cast<float4 *>(dst + 4) = make_float4(-total[cb * 8 + 4], -total[cb * 8 + 5], -total[cb * 8 + 6], -total[cb * 8 + 7]);
+            }
+            *reinterpret_cast<uint4 *>(P.out_hi + gi * ld + gj0) = *reinterpret_cast<const uint4 *>(h);
+            *reinterpret_cast<uint4 *>(P.out_mid + gi * ld + gj0) = *reinterpret_cast<const uint4 *>(c);
+            *reinterpret_cast<uint4 *>(P.out_lo + gi * ld + gj0) = *reinterpret_cast<const uint4 *>(l);
+        }
+    }
+}
+
 __global__ void __launch_bounds__(TC_THREADS) trinv_tc_kernel(const __grid_constant__ TrinvJob job) {
-    constexpr int NSTAGE = DUO ? DUO_STAGES : TRINV_STAGES, STAGE = DUO ? DUO_STAGE_BYTES : TRINV_STAGE_BYTES, B_BYTES = DUO ? DUO_HALF : HTILE_BYTES;
-    constexpr int EDGE = DUO ? 2 * MT : MT;  // rows of the tile
-    constexpr uint32_t DESC = idesc_16(MT, 1, EDGE);  // bf16
     extern __shared__ unsigned char tc_smem_raw[];
     __shared__ __align__(8) TcRing ring;
     __shared__ __align__(8) uint64_t acc_full[2], acc_empty[2];
-    const int rank = DUO ? (int)cluster_rank() : 0, block_x = DUO ? (int)blockIdx.x >> 1 : (int)blockIdx.x;
-    const int z = block_x >= job.pairs ? 1 : 0;
-    const int64_t pair = (int64_t)block_x - (int64_t)z * job.pairs;
+    const int z = (int)blockIdx.x >= job.pairs ? 1 : 0;
+    const int64_t pair = (int64_t)blockIdx.x - (int64_t)z * job.pairs;
     const FactorPlanes P = z ? job.p[1] : job.p[0];
     const FactorMaps *maps = z ? &job.maps[1] : &job.maps[0];
     const int64_t n = P.n, b = job.b;
     const int64_t r0 = pair * 2 * b, r1 = r0 + b;  // first half rows [r0, r1), second half rows [r1, r2)
     if (r1 >= n) return;
     const int64_t r2 = min(r0 + 2 * b, n);
-    // output tile: rows m0.. of the A operand's matrix (tile_m0.. of both CTAs), columns n0.. of the B operand's
-    int64_t tile_m0, n0, k_lo, k_hi;
+    // output tile: rows m0.. of the A operand's matrix, columns n0.. of the B operand's
+    int64_t m0, n0, k_lo, k_hi;
     const CUtensorMap *a_maps;
     if (!job.second) {
-        tile_m0 = r0 + (int64_t)blockIdx.z * EDGE;  // j: long k ranges (small j) are scheduled first
+        m0 = r0 + (int64_t)blockIdx.z * MT;  // j: long k ranges (small j) are scheduled first
         n0 = r1 + (int64_t)blockIdx.y * MT;  // i
         if (n0 >= r2) return;
-        k_lo = tile_m0;
+        k_lo = m0;
         k_hi = r1;
         a_maps = maps->outt;
     } else {
-        tile_m0 = r1 + (int64_t)(job.tiles * MT / EDGE - 1 - (int)blockIdx.y) * EDGE;  // i: long k ranges (large i) first
-        if (tile_m0 >= r2) return;
+        m0 = r1 + (int64_t)(job.tiles - 1 - (int)blockIdx.y) * MT;  // i: long k ranges (large i) first
+        if (m0 >= r2) return;
         n0 = r0 + (int64_t)blockIdx.z * MT;  // j
         k_lo = r1;
-        k_hi = min(tile_m0 + EDGE, r2);
+        k_hi = min(m0 + MT, r2);
         a_maps = maps->out;
     }
-    const int64_t m0 = tile_m0 + rank * MT;
     const int chunks = (int)ceil_div(k_hi - k_lo, (int64_t)KH);  // a ragged tail reads zeros beyond the matrix
     const int slices = (chunks + TRINV_SLICE - 1) / TRINV_SLICE;
 
@@ -110,83 +145,62 @@ __global__ void __launch_bounds__(TC_THREADS) trinv_tc_kernel(const __grid_const
     if (threadIdx.x == 0) {
         for (int s2 = 0; s2 < 2; ++s2) {
             mbar_init(&acc_full[s2], 1);
-            mbar_init(&acc_empty[s2], DUO ? 8 : 4);  // one arrival per epilogue warp, of both CTAs at the leader's
+            mbar_init(&acc_empty[s2], 4);  // one arrival per epilogue warp
         }
     }
-    const uint32_t tmem = tc_ring_setup<DUO>(ring, TRINV_TMEM_COLS);  // fences the barrier initialisations and synchronises the CTA
-    const auto wait = [](uint64_t *bar, uint32_t parity, unsigned nap = 32) { return DUO ? mbar_wait_cluster(bar, parity, nap) : mbar_wait(bar, parity, nap); };
+    const uint32_t tmem = tc_ring_setup(ring, TRINV_TMEM_COLS);  // fences the barrier initialisations and synchronises the CTA
     if (warp == 0) {
         if (lane == 0) {
             for (int ch = 0; ch < chunks; ++ch) {
-                const int stage = ch % NSTAGE, round = ch / NSTAGE;
-                if (round > 0 && !wait(&ring.empty[stage], (round - 1) & 1)) {
+                const int stage = ch % TRINV_STAGES, round = ch / TRINV_STAGES;
+                if (round > 0 && !mbar_wait(&ring.empty[stage], (round - 1) & 1)) {
                     ring.failed = 1;
                     break;
                 }
                 const int k = (int)(k_lo + (int64_t)ch * KH);
-                const uint32_t dst = smem_base + stage * STAGE;
-                if constexpr (DUO) {
-                    // both CTAs' bytes count at the leader's barrier (they may do so before it expects them: the phase waits for its arrival)
-                    if (rank == 0) mbar_expect_tx(&ring.full[stage], 2 * STAGE);
-                    const bool none = job.second ? rank == 0 && k >= tile_m0 + MT : rank == 1 && k < tile_m0 + MT;
-                    const uint32_t bar = leaders(&ring.full[stage]);
-                    for (int part = 0; part < 3; ++part) {
-                        tma_load_2d_duo(dst + part * HTILE_BYTES, &a_maps[part], k, none ? (int)n : (int)m0, bar);
-                        tma_load_2d_duo(dst + 3 * HTILE_BYTES + part * DUO_HALF, &maps->tw_half[part], k, (int)n0 + rank * (MT / 2), bar);
-                    }
-                } else {
-                    mbar_expect_tx(&ring.full[stage], STAGE);
-                    for (int part = 0; part < 3; ++part) {
-                        tma_load_2d(dst + part * HTILE_BYTES, &a_maps[part], k, (int)m0, &ring.full[stage]);
-                        tma_load_2d(dst + (3 + part) * HTILE_BYTES, &maps->tw[part], k, (int)n0, &ring.full[stage]);
-                    }
+                const uint32_t dst = smem_base + stage * TRINV_STAGE_BYTES;
+                mbar_expect_tx(&ring.full[stage], TRINV_STAGE_BYTES);
+                for (int part = 0; part < 3; ++part) {
+                    tma_load_2d(dst + part * HTILE_BYTES, &a_maps[part], k, (int)m0, &ring.full[stage]);
+                    tma_load_2d(dst + (3 + part) * HTILE_BYTES, &maps->tw[part], k, (int)n0, &ring.full[stage]);
                 }
-            }
-            if (DUO && !ring.failed) {
-                // the leader's commits arrive here as well: none may be under way when this CTA ends
-                for (int ch = max(chunks - NSTAGE, 0); ch < chunks; ++ch)
-                    if (!wait(&ring.empty[ch % NSTAGE], (ch / NSTAGE) & 1)) ring.failed = 1;
-                if (!wait(&ring.accum, 0)) ring.failed = 1;
             }
         }
     } else if (warp == 1) {
-        if (lane == 0 && rank == 0) {
-            int ch = 0;
-            for (; ch < chunks; ++ch) {
-                const int stage = ch % NSTAGE, round = ch / NSTAGE;
+        if (lane == 0) {
+            for (int ch = 0; ch < chunks; ++ch) {
+                const int stage = ch % TRINV_STAGES, round = ch / TRINV_STAGES;
                 const int slice = ch / TRINV_SLICE, buf = slice & 1;
                 const bool opens = ch % TRINV_SLICE == 0, closes = ch % TRINV_SLICE == TRINV_SLICE - 1 || ch == chunks - 1;
                 // the accumulators must have been read out by the epilogue of the slice two before
-                if (opens && slice >= 2 && !wait(&acc_empty[buf], ((slice >> 1) - 1) & 1)) {
+                if (opens && slice >= 2 && !mbar_wait(&acc_empty[buf], ((slice >> 1) - 1) & 1)) {
                     ring.failed = 1;
                     break;
                 }
-                if (!wait(&ring.full[stage], round & 1)) {
+                if (!mbar_wait(&ring.full[stage], round & 1)) {
                     ring.failed = 1;
                     break;
                 }
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const uint32_t acc_main = tmem + (uint32_t)(buf * 2 * MT), acc_small = acc_main + MT;
-                const uint32_t base = smem_base + stage * STAGE;
+                const uint32_t base = smem_base + stage * TRINV_STAGE_BYTES;
                 const uint32_t a_hi = base, a_mid = base + HTILE_BYTES, a_lo = base + 2 * HTILE_BYTES;
-                const uint32_t b_hi = base + 3 * HTILE_BYTES, b_mid = b_hi + B_BYTES, b_lo = b_mid + B_BYTES;
+                const uint32_t b_hi = base + 3 * HTILE_BYTES, b_mid = base + 4 * HTILE_BYTES, b_lo = base + 5 * HTILE_BYTES;
 #pragma unroll
                 for (int ks = 0; ks < KH / 16; ++ks) {
                     const uint32_t off = ks * 32;  // 16 values = 32 bytes along the swizzled row
                     const uint32_t fresh = (opens && ks == 0) ? 0u : 1u;
-                    mma<DUO>(acc_main, a_hi + off, b_hi + off, DESC, fresh);
-                    mma<DUO>(acc_small, a_hi + off, b_mid + off, DESC, fresh);
-                    mma<DUO>(acc_small, a_mid + off, b_hi + off, DESC, 1u);
-                    mma<DUO>(acc_small, a_mid + off, b_mid + off, DESC, 1u);
-                    mma<DUO>(acc_small, a_hi + off, b_lo + off, DESC, 1u);
-                    mma<DUO>(acc_small, a_lo + off, b_hi + off, DESC, 1u);
+                    umma_16(acc_main, umma_desc(a_hi + off), umma_desc(b_hi + off), TRINV_DESC, fresh);
+                    umma_16(acc_small, umma_desc(a_hi + off), umma_desc(b_mid + off), TRINV_DESC, fresh);
+                    umma_16(acc_small, umma_desc(a_mid + off), umma_desc(b_hi + off), TRINV_DESC, 1u);
+                    umma_16(acc_small, umma_desc(a_mid + off), umma_desc(b_mid + off), TRINV_DESC, 1u);
+                    umma_16(acc_small, umma_desc(a_hi + off), umma_desc(b_lo + off), TRINV_DESC, 1u);
+                    umma_16(acc_small, umma_desc(a_lo + off), umma_desc(b_hi + off), TRINV_DESC, 1u);
                 }
-                commit<DUO>(&ring.empty[stage]);       // arrives when the MMAs above have read the stage
-                if (closes) commit<DUO>(&acc_full[buf]);    // arrives when the slice is complete in tensor memory
-                if (ch == chunks - 1) commit<DUO>(&ring.accum);  // and when all of them have completed
+                umma_commit(&ring.empty[stage]);            // arrives when the MMAs above have read the stage
+                if (closes) umma_commit(&acc_full[buf]);    // arrives when the slice is complete in tensor memory
             }
-            // on a time-out: what has been issued so far
-            if (ch < chunks) commit<DUO>(&ring.accum);
+            umma_commit(&ring.accum);                       // arrives when every MMA issued so far has completed
         }
     } else {
         // epilogue warps: lanes 32 q .. 32 q + 31 of tensor memory, q = warp % 4; one accumulator row per thread, whose
@@ -198,7 +212,7 @@ __global__ void __launch_bounds__(TC_THREADS) trinv_tc_kernel(const __grid_const
         bool go = true;
         for (int slice = 0; slice < slices && go; ++slice) {
             const int buf = slice & 1;
-            const bool ok = wait(&acc_full[buf], (slice >> 1) & 1, 64);
+            const bool ok = mbar_wait(&acc_full[buf], (slice >> 1) & 1, 64);
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             if (!ok) ring.failed = 1;
             go = __all_sync(0xffffffffu, ok && !ring.failed);  // warp-uniform: the tensor-memory loads are warp-wide
@@ -214,56 +228,181 @@ __global__ void __launch_bounds__(TC_THREADS) trinv_tc_kernel(const __grid_const
             // this warp has read the accumulators: hand them back to the MMA warp
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();
-            if (lane == 0) {
-                if (DUO) mbar_arrive_at(leaders(&acc_empty[buf]));
-                else mbar_arrive(&acc_empty[buf]);
-            }
+            if (lane == 0) mbar_arrive(&acc_empty[buf]);
         }
         if (go) {
-            const int64_t gi = m0 + q * 32 + lane, ld = P.ld;
-            const bool vec = n % 4 == 0;  // rows of the float matrix are 16-byte multiples; those of the planes always are
-#pragma unroll
-            for (int cb = 0; cb < MT / 8; ++cb) {
-                const int64_t gj0 = n0 + cb * 8;
-                __align__(16) __nv_bfloat16 h[8];
-                __align__(16) __nv_bfloat16 c[8];
-                __align__(16) __nv_bfloat16 l[8];
-                if (!job.second) {
-                    // W^T[gi][gj]: gi is inside the first half (always a row of the matrix), gj is cut at r2; a group of eight that
-                    // reaches past it ends in the padding of its row (its extra products are zero)
-                    if (gj0 < r2) {
-#pragma unroll
-                        for (int e = 0; e < 8; ++e) split_bf16_3(total[cb * 8 + e], h[e], c[e], l[e]);
-                        *reinterpret_cast<uint4 *>(P.tw_hi + gi * ld + gj0) = *reinterpret_cast<const uint4 *>(h);
-                        *reinterpret_cast<uint4 *>(P.tw_mid + gi * ld + gj0) = *reinterpret_cast<const uint4 *>(c);
-                        *reinterpret_cast<uint4 *>(P.tw_lo + gi * ld + gj0) = *reinterpret_cast<const uint4 *>(l);
-                    }
-                } else if (gi < r2) {
-                    // X[gi][gj] = -acc (gj is inside the first half): the inverse itself, its split, and the split of its transpose
-                    // (coalesced across the lanes)
-                    float *dst = P.out + gi * n + gj0;
-#pragma unroll
-                    for (int e = 0; e < 8; ++e) {
-                        const float v = -total[cb * 8 + e];
-                        split_bf16_3(v, h[e], c[e], l[e]);
-                        P.outt_hi[(gj0 + e) * ld + gi] = h[e];
-                        P.outt_mid[(gj0 + e) * ld + gi] = c[e];
-                        P.outt_lo[(gj0 + e) * ld + gi] = l[e];
-                        if (!vec) dst[e] = v;
-                    }
-                    if (vec) {
-                        *reinterpret_cast<float4 *>(dst) = make_float4(-total[cb * 8], -total[cb * 8 + 1], -total[cb * 8 + 2], -total[cb * 8 + 3]);
-                        *reinterpret_cast<float4 *>(dst + 4) = make_float4(-total[cb * 8 + 4], -total[cb * 8 + 5], -total[cb * 8 + 6], -total[cb * 8 + 7]);
-                    }
-                    *reinterpret_cast<uint4 *>(P.out_hi + gi * ld + gj0) = *reinterpret_cast<const uint4 *>(h);
-                    *reinterpret_cast<uint4 *>(P.out_mid + gi * ld + gj0) = *reinterpret_cast<const uint4 *>(c);
-                    *reinterpret_cast<uint4 *>(P.out_lo + gi * ld + gj0) = *reinterpret_cast<const uint4 *>(l);
-                }
-            }
+            trinv_write(P, job.second, m0 + q * 32 + lane, n0, r2, total);
         }
     }
-    const bool failed = tc_ring_teardown<DUO>(ring, tmem, TRINV_TMEM_COLS);
+    const bool failed = tc_ring_teardown(ring, tmem, TRINV_TMEM_COLS);
     if (threadIdx.x == 0 && failed && P.flag) atomicExch(P.flag, -1);
+}
+
+// As trinv_tc_kernel, by two CTAs of a cluster on a tile of 256 x 256: each has 128 rows of the first operand and of the second.  The main and the
+// correction accumulator fill tensor memory, so there is one pair of them: a chunk's large products come first, so that the reading warps take
+// the main accumulator of a slice while its last small products are multiplied, and the small one under the first large products
+// of the next.
+struct TrinvDuoRing {
+    uint64_t full[TRINV_STAGES], empty[TRINV_STAGES], acc_full[2], acc_empty[2];  // accumulators: main, correction
+    uint32_t tmem;
+    int failed;
+};
+constexpr int DUO_EDGE = 2 * MT, DUO_GROUP = 8;
+static_assert(DUO_BLOCK % (DUO_EDGE * DUO_GROUP) == 0, "whole groups");
+__global__ void __launch_bounds__(PAIR_THREADS, 1) trinv_duo_kernel(const __grid_constant__ TrinvJob job) {
+    constexpr uint32_t DESC = idesc_16(DUO_EDGE, 1, DUO_EDGE), COLS = 2 * DUO_EDGE;  // bf16
+    extern __shared__ unsigned char tc_smem_raw[];
+    __shared__ __align__(8) TrinvDuoRing ring;
+    const int rank = (int)cluster_rank();
+    const int z = (int)blockIdx.y >= job.pairs ? 1 : 0;
+    const int64_t pair = (int64_t)blockIdx.y - (int64_t)z * job.pairs;
+    const FactorPlanes P = z ? job.p[1] : job.p[0];
+    const FactorMaps *maps = z ? &job.maps[1] : &job.maps[0];
+    const int64_t n = P.n, b = job.b;
+    const int64_t r0 = pair * 2 * b, r1 = r0 + b;  // first half rows [r0, r1), second half rows [r1, r2)
+    if (r1 >= n) return;
+    const int64_t r2 = min(r0 + 2 * b, n);
+    // Groups of eight tile rows, column after column, so that the clusters of the moment share 8 and 9 strips in L2; long k ranges first.
+    const int64_t edge = b / DUO_EDGE, at = blockIdx.x >> 1, group = at / (DUO_GROUP * edge), within = at % (DUO_GROUP * edge);
+    const int64_t row = group * DUO_GROUP + within % DUO_GROUP, column = within / DUO_GROUP;  // edge is a multiple of DUO_GROUP
+    int64_t tile_m0, n0, k_lo, k_hi;
+    const CUtensorMap *a_maps;
+    if (!job.second) {
+        tile_m0 = r0 + row * DUO_EDGE;  // j
+        n0 = r1 + column * DUO_EDGE;    // i
+        if (n0 >= r2) return;
+        k_lo = tile_m0;
+        k_hi = r1;
+        a_maps = maps->outt;
+    } else {
+        tile_m0 = r1 + (edge - 1 - row) * DUO_EDGE;  // i
+        if (tile_m0 >= r2) return;
+        n0 = r0 + column * DUO_EDGE;  // j
+        k_lo = r1;
+        k_hi = min(tile_m0 + DUO_EDGE, r2);
+        a_maps = maps->out;
+    }
+    const int64_t m0 = tile_m0 + rank * MT;
+    const int chunks = (int)ceil_div(k_hi - k_lo, (int64_t)KH);  // a ragged tail reads zeros beyond the matrix
+    const int slices = (chunks + TRINV_SLICE - 1) / TRINV_SLICE;
+
+    const uint32_t smem_base = (smem_u32(tc_smem_raw) + 1023u) & ~1023u;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < TRINV_STAGES; ++s) {
+            mbar_init(&ring.full[s], 1);
+            mbar_init(&ring.empty[s], 1);
+        }
+        for (int s = 0; s < 2; ++s) {
+            mbar_init(&ring.acc_full[s], 1);
+            mbar_init(&ring.acc_empty[s], 16);  // one arrival per reading warp of both CTAs, at the leader's
+        }
+        ring.failed = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 1) tmem_alloc<true>(&ring.tmem, COLS);
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    __syncwarp();
+    cluster_sync();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t tmem = ring.tmem;
+    if (warp == 0) {
+        if (lane == 0) {
+            for (int ch = 0; ch < chunks; ++ch) {
+                const int stage = ch % TRINV_STAGES, round = ch / TRINV_STAGES;
+                if (round > 0 && !mbar_wait_cluster(&ring.empty[stage], (round - 1) & 1)) {
+                    ring.failed = 1;
+                    break;
+                }
+                const int k = (int)(k_lo + (int64_t)ch * KH);
+                const uint32_t dst = smem_base + stage * TRINV_STAGE_BYTES, bar = leaders(&ring.full[stage]);
+                // both CTAs' bytes count at the leader's barrier (they may do so before it expects them: the phase waits for its arrival)
+                if (rank == 0) mbar_expect_tx(&ring.full[stage], 2 * TRINV_STAGE_BYTES);
+                // the ranges of k of the two CTAs' rows differ by 128: outside its own a CTA's operand is zeros, loaded from outside the matrix
+                const bool none = job.second ? rank == 0 && k >= tile_m0 + MT : rank == 1 && k < tile_m0 + MT;
+                for (int part = 0; part < 3; ++part) {
+                    tma_load_2d_duo(dst + part * HTILE_BYTES, &a_maps[part], k, none ? (int)n : (int)m0, bar);
+                    tma_load_2d_duo(dst + (3 + part) * HTILE_BYTES, &maps->tw[part], k, (int)n0 + rank * MT, bar);
+                }
+            }
+            // the leader's commits arrive here as well: none may be under way when this CTA ends (those of the accumulators are awaited below)
+            for (int ch = max(chunks - TRINV_STAGES, 0); ch < chunks && !ring.failed; ++ch)
+                if (!mbar_wait_cluster(&ring.empty[ch % TRINV_STAGES], (ch / TRINV_STAGES) & 1)) ring.failed = 1;
+        }
+    } else if (warp == 1) {
+        if (lane == 0 && rank == 0) {
+            const uint32_t acc_main = tmem, acc_small = tmem + DUO_EDGE;
+            int slice = 0;
+            for (int ch = 0; ch < chunks; ++ch) {
+                const int stage = ch % TRINV_STAGES, round = ch / TRINV_STAGES;
+                const bool opens = ch % TRINV_SLICE == 0, closes = ch % TRINV_SLICE == TRINV_SLICE - 1 || ch == chunks - 1;
+                if (!mbar_wait_cluster(&ring.full[stage], round & 1)) { ring.failed = 1; break; }
+                // the accumulators must have been read out for the slice before
+                if (opens && slice > 0 && !mbar_wait_cluster(&ring.acc_empty[0], (slice - 1) & 1)) { ring.failed = 1; break; }
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                const uint32_t a_hi = smem_base + stage * TRINV_STAGE_BYTES, a_mid = a_hi + HTILE_BYTES, a_lo = a_hi + 2 * HTILE_BYTES;
+                const uint32_t b_hi = a_hi + 3 * HTILE_BYTES, b_mid = b_hi + HTILE_BYTES, b_lo = b_mid + HTILE_BYTES;
+#pragma unroll
+                for (int ks = 0; ks < KH / 16; ++ks) mma<true>(acc_main, a_hi + ks * 32, b_hi + ks * 32, DESC, (opens && ks == 0) ? 0u : 1u);
+                if (closes) commit<true>(&ring.acc_full[0]);
+                if (opens && slice > 0) {
+                    if (!mbar_wait_cluster(&ring.acc_empty[1], (slice - 1) & 1)) { ring.failed = 1; break; }
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                }
+#pragma unroll
+                for (int ks = 0; ks < KH / 16; ++ks) {
+                    const uint32_t off = ks * 32;  // 16 values = 32 bytes along the swizzled row
+                    mma<true>(acc_small, a_hi + off, b_mid + off, DESC, (opens && ks == 0) ? 0u : 1u);
+                    mma<true>(acc_small, a_mid + off, b_hi + off, DESC, 1u);
+                    mma<true>(acc_small, a_mid + off, b_mid + off, DESC, 1u);
+                    mma<true>(acc_small, a_hi + off, b_lo + off, DESC, 1u);
+                    mma<true>(acc_small, a_lo + off, b_hi + off, DESC, 1u);
+                }
+                commit<true>(&ring.empty[stage]);  // arrives when the MMAs above have read the stage
+                if (closes) {
+                    commit<true>(&ring.acc_full[1]);
+                    ++slice;
+                }
+            }
+            // on time-out, give what is in flight a bounded chance to land before its memory is released
+            if (ring.failed && slice > 0) mbar_wait(&ring.acc_full[1], (slice - 1) & 1);
+        }
+    } else {
+        // reading warps: lanes 32 q .. 32 q + 31 of tensor memory, q = warp % 4, and half of the columns; 128 running sums in registers
+        const int q = warp & 3, c0 = ((warp - 2) >> 2) * MT;
+        float total[MT];
+#pragma unroll
+        for (int x = 0; x < MT; ++x) total[x] = 0.f;
+        bool go = true;
+        for (int s = 0; s < 2 * slices && go; ++s) {
+            const int which = s & 1;
+            const bool ok = mbar_wait_cluster(&ring.acc_full[which], (s >> 1) & 1, 64);
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            if (!ok) ring.failed = 1;
+            go = __all_sync(0xffffffffu, ok && !ring.failed);  // warp-uniform: the tensor-memory loads are warp-wide
+            if (!go) break;
+#pragma unroll
+            for (int cb = 0; cb < MT / 16; ++cb) {  // 16 at a time, as in pair_gemm
+                uint32_t v[16];
+                tmem_load_16(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(which * DUO_EDGE + c0 + cb * 16), v);
+#pragma unroll
+                for (int x = 0; x < 16; ++x) total[cb * 16 + x] += __uint_as_float(v[x]);
+            }
+            // this warp has read the accumulator: hand it back to the MMA warp
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) mbar_arrive_at(leaders(&ring.acc_empty[which]));
+        }
+        if (go) trinv_write(P, job.second, m0 + q * 32 + lane, n0 + c0, r2, total);
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    // neither CTA leaves while the other's MMAs may read its shared memory or arrive at its barriers
+    __syncwarp();
+    cluster_sync();
+    if (warp == 1) tmem_free<true>(tmem, COLS);
+    if (threadIdx.x == 0 && ring.failed && P.flag) atomicExch(P.flag, -1);
 }
 
 // Operand planes after the 64-level of the doubling: T strictly below the diagonal into the lower triangle of tw, and the
@@ -310,17 +449,17 @@ static bool factor_maps(FactorMaps *maps, const FactorPlanes &p) {
     bool ok = true;
     for (int part = 0; part < 3; ++part)
         ok = ok && make_map_16(&maps->out[part], out[part], p.n, p.n, MT, true, p.ld) && make_map_16(&maps->outt[part], outt[part], p.n, p.n, MT, true, p.ld) &&
-             make_map_16(&maps->tw[part], tw[part], p.n, p.n, MT, true, p.ld) && make_map_16(&maps->tw_half[part], tw[part], p.n, p.n, MT / 2, true, p.ld);
+             make_map_16(&maps->tw[part], tw[part], p.n, p.n, MT, true, p.ld);
     return ok;
 }
 
 // Levels b = 128, 256, ... of the doubling for one or two problems whose 128 x 128 diagonal blocks are finished.
 int launch_trinv_tc(int count, const FactorPlanes *problems, cudaStream_t stream) {
     static PerDeviceOnce configured;
-    const size_t smem = (size_t)TRINV_STAGES * TRINV_STAGE_BYTES + 1024, duo_smem = (size_t)DUO_STAGES * DUO_STAGE_BYTES + 1024;
+    const size_t smem = (size_t)TRINV_STAGES * TRINV_STAGE_BYTES + 1024;
     if (configured.run([&] {
-            return cudaFuncSetAttribute(trinv_tc_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) == cudaSuccess &&
-                   cudaFuncSetAttribute(trinv_tc_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)duo_smem) == cudaSuccess;
+            return cudaFuncSetAttribute(trinv_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) == cudaSuccess &&
+                   cudaFuncSetAttribute(trinv_duo_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) == cudaSuccess;
         }) != G2D_OK)
         return G2D_ERR_CUDA;
     TrinvJob job;
@@ -334,17 +473,17 @@ int launch_trinv_tc(int count, const FactorPlanes *problems, cudaStream_t stream
     if (check_launch() != G2D_OK) return G2D_ERR_CUDA;
     for (int64_t b = MT; b < n_max; b *= 2) {
         const int64_t pairs = ceil_div(n_max, 2 * b), tiles = b / MT;
-        if (tiles > 65535 || 2 * pairs * count > 0x7fffffff) return G2D_ERR_TOO_LARGE;
+        if (tiles > 65535 || pairs * count > 0x7fffffff) return G2D_ERR_TOO_LARGE;
         job.pairs = (int)pairs;
         job.tiles = (int)tiles;
         job.b = b;
         for (int second = 0; second < 2; ++second) {
             job.second = second;
             if (b < DUO_BLOCK) {
-                trinv_tc_kernel<false><<<dim3((unsigned)(pairs * count), (unsigned)tiles, (unsigned)tiles), TC_THREADS, smem, stream>>>(job);
+                trinv_tc_kernel<<<dim3((unsigned)(pairs * count), (unsigned)tiles, (unsigned)tiles), TC_THREADS, smem, stream>>>(job);
             } else {
-                const dim3 grid((unsigned)(2 * pairs * count), (unsigned)(second ? tiles / 2 : tiles), (unsigned)(second ? tiles : tiles / 2));
-                if (launch_duo(trinv_tc_kernel<true>, grid, TC_THREADS, duo_smem, stream, job) != G2D_OK) return G2D_ERR_CUDA;
+                const int64_t edge = b / DUO_EDGE;
+                if (launch_duo(trinv_duo_kernel, dim3((unsigned)(2 * edge * edge), (unsigned)(pairs * count)), PAIR_THREADS, smem, stream, job) != G2D_OK) return G2D_ERR_CUDA;
             }
             if (check_launch() != G2D_OK) return G2D_ERR_CUDA;
         }

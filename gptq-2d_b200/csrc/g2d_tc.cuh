@@ -204,8 +204,7 @@ inline int launch_duo(void (*kernel)(Job), dim3 grid, int threads, size_t smem, 
     return cudaLaunchKernelEx(&config, kernel, job) == cudaSuccess ? check_launch() : G2D_ERR_CUDA;
 }
 
-// All threads: barriers, tensor-memory allocation of `cols` columns (by warp 1); returns the accumulator's address.  DUO: of both CTAs.
-template <bool DUO = false>
+// All threads: barriers, tensor-memory allocation of `cols` columns (by warp 1); returns the accumulator's address.
 __device__ __forceinline__ uint32_t tc_ring_setup(TcRing &ring, uint32_t cols) {
     if (threadIdx.x == 0) {
         for (int s = 0; s < STAGES; ++s) {
@@ -216,19 +215,14 @@ __device__ __forceinline__ uint32_t tc_ring_setup(TcRing &ring, uint32_t cols) {
         ring.failed = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    if ((threadIdx.x >> 5) == 1) tmem_alloc<DUO>(&ring.tmem_slot, cols);
+    if ((threadIdx.x >> 5) == 1) tmem_alloc<false>(&ring.tmem_slot, cols);
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
-    if (DUO) {
-        __syncwarp();
-        cluster_sync();
-    }
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     return ring.tmem_slot;
 }
 
 // All threads: release tensor memory; returns whether a wait ran out (meaningful in every thread).
-template <bool DUO = false>
 __device__ __forceinline__ bool tc_ring_teardown(TcRing &ring, uint32_t tmem, uint32_t cols) {
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
@@ -239,12 +233,7 @@ __device__ __forceinline__ bool tc_ring_teardown(TcRing &ring, uint32_t tmem, ui
             __syncwarp();
         }
     }
-    if (DUO) {
-        // neither CTA leaves while the other's MMAs may read its shared memory or arrive at its barriers
-        __syncwarp();
-        cluster_sync();
-    }
-    if ((threadIdx.x >> 5) == 1) tmem_free<DUO>(tmem, cols);
+    if ((threadIdx.x >> 5) == 1) tmem_free<false>(tmem, cols);
     return ring.failed != 0;
 }
 

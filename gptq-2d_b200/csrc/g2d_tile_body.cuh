@@ -239,12 +239,12 @@
         // the row lane, which received the C accumulator with the same shuffle, the completed C to the right: one shuffle
         // and fifteen multiply-adds per lane and stage.  (Half a warp per sub-tile with both feedbacks in one lane takes
         // two shuffles and thirty multiply-adds: 208 cycles per stage against about 100.)
-        // What bounds a stage is the chain from one rounding to the next (multiply-add, shuffle, the quantizer's dozen dependent
-        // operations: about 95 cycles); everything else has to fit into its gaps.  So every address of a stage is a lane's base
-        // plus a constant stride (lanes before their first or past their last entry read zero rows or values that they
-        // ignore, and store nothing), the operands of a stage are loaded one stage ahead, and there is no branch inside the
-        // four unrolled stages (one branch per stage costs 40 cycles): about 120 cycles per stage for one warp on its
-        // scheduler, 150 for two, against 168 with wrapped addresses and selects.
+        // What bounds a stage is the chain from one rounding to the next (multiply-add, shuffle of 26 cycles, the quantizer's
+        // dependent operations at 4.5 to 5.4 cycles each: about 72 cycles, 95 before affine_steps_fast); everything else has to fit into its
+        // gaps.  So every address of a stage is a lane's base plus a constant stride (lanes before their first or past their last entry
+        // read zero rows or values that they ignore, and store nothing), the operands of a stage are loaded one stage ahead, and there is
+        // no branch inside the four unrolled stages (one branch per stage costs 40 cycles): with the other warps' work beside it about 120 cycles
+        // per stage where one sub-tile is swept and 190 where four are.
         // The two roles run the same sequence of barriers from loops of their own, so that neither holds the other's registers.
         // Operands of the tensor-core updates: fp16 pairs of E (transposed) and of the completed C under the tile's scales, eight entries
         // per thread and store.  C along its rows; E transposed: a thread gathers eight rows of one column (consecutive threads take
