@@ -2,7 +2,7 @@
 // the SMs that the tiles leave free, carry out the near update of the anti-diagonal before.  The two do not depend on each other: the update's
 // targets start at S + 1.  Bound by the tiles' serial chain, about 24 us.  On streams of their own (g2d_tile_sweep.cu, g2d_band_tc.cu) a step took
 // 7 us of events between the two on top of it; in one launch that starts early, 1024 x 1024 takes 0.82 ms in place of 0.93, 2048 x 2048 1.69 in
-// place of 1.92, 8192 x 8192 11.0 in place of 11.7.  A warp issues an instruction every ninth cycle; 1.8 of
+// place of 1.92, 8192 x 8192 11.0 in place of 11.7.  A warp issues an instruction every ninth cycle; 2.0 of
 // those nine it waits for instructions to arrive, 2.3 at barriers (4096 x 4096): how long the kernel's text is, and where its parts lie,
 // shows in its time.
 #include "g2d_band_tc.cuh"
