@@ -145,11 +145,12 @@ __device__ __forceinline__ void chain_product(F (&acc)[4][4], int K, LA la, LB l
 
 // ---- step 1a: factor the diagonal block kb (bs x bs), M_kk = T_kk^T T_kk, and invert T_kk ----
 // One CTA of 256 threads; sixteen rows are factored at a time, the last ones first.  Warp 0 holds their columns 0 .. r0 + 15 in
-// registers, two per lane, and eliminates row after row: the pivot's column goes through shared memory to all lanes, the
+// registers, two per lane, and eliminates row after row: the columns of the pivots go through shared memory to all lanes one pivot ahead, the
 // pivot row is scaled and stored as a row of T.  Then all threads subtract the rows' Gram from what is left.  At the end four
 // warps invert the four 16 x 16 diagonal blocks of T by columns, and two doubling levels join them.  Bound by the chain of 64
-// pivots, about 190 cycles each.  At n = 1024 a step of 64 rows took 25 us with one barrier per pivot over the whole block
-// and exact divisions, 17 us now.
+// pivots.  A pivot took 290 cycles while its own column had to come through shared memory before its root, 20 thousand of the 37 thousand
+// cycles of a block at n = 8192; with every lane forming the next pivot itself the factors of 1024 and 1024 take 590 us in place of 637, 2048 and 3000
+// 1.63 ms in place of 1.78, 8192 and 8192 7.08 ms in place of 7.47.
 constexpr int DTH = 256;
 constexpr int DS = 16;          // rows factored at a time
 constexpr int DLDS = FB + 4;    // shared row stride: rows are 16-byte multiples
@@ -250,43 +251,61 @@ __global__ void __launch_bounds__(DTH) ldl_diag_kernel(LdlBatch<F> B, int step_d
 #pragma unroll 1
     for (int r0 = FB - DS; r0 >= 0; r0 -= DS) {
         if (warp == 0) {
-            const int owner = r0 & 16;       // first of the lanes that hold the rows' own columns, in the second set from 32 on
+            const int owner = r0 & 16;       // first of the lanes that hold the rows' own columns
             const bool second = r0 >= 32;    // columns 32 .. r0 + 15 are there
-            F v0[DS], v1[DS];                // register r: row r0 + r of columns lane and lane + 32 (by symmetry where it lies above the diagonal)
+            const int c0 = second ? lane + 32 : lane, c1 = c0 ^ 32;
+            F v0[DS], v1[DS];                // register r: row r0 + r of columns c0 (the set with the rows' own) and c1 (by symmetry where it lies above the diagonal)
 #pragma unroll
             for (int r = 0; r < DS; ++r) {
-                const int row = r0 + r, c1 = lane + 32;
-                v0[r] = row >= lane ? S[row * DLDS + lane] : S[lane * DLDS + row];
+                const int row = r0 + r;
+                v0[r] = row >= c0 ? S[row * DLDS + c0] : S[c0 * DLDS + row];
                 v1[r] = row >= c1 ? S[row * DLDS + c1] : S[c1 * DLDS + row];
             }
+            // Every lane has the pivot's column (w) and the one of the pivot after it (u, not yet updated with this one): a lane
+            // then forms the next pivot itself, and the way through shared memory, which brings the column after that, runs beside
+            // the pivot's root.
+            F w[DS], u[DS];
+            if ((lane | 1) == owner + DS - 1) {
+#pragma unroll
+                for (int r = 0; r < DS; ++r) column[lane & 1][r] = v0[r];
+            }
+            __syncwarp();
+#pragma unroll
+            for (int r = 0; r < DS; ++r) {
+                w[r] = column[1][r];
+                u[r] = column[0][r];
+            }
+            __syncwarp();
             int worst = FB + 1;
             // The row that is eliminated sits in the last register: a step moves the others up by one, so that all steps are the
-            // same instructions and fit the instruction cache.
+            // same instructions and fit the instruction cache.  (fma: left to the compiler, the last row's update can lie in another block of the
+            // program than its product, and is rounded twice.)
 #pragma unroll 2
             for (int j = DS - 1; j >= 0; --j) {
-                F *const col = column[j & 1];
-                if (lane == owner + j) {
-#pragma unroll
-                    for (int r = 0; r < DS; ++r) col[r] = second ? v1[r] : v0[r];
-                }
-                __syncwarp();
-                F w[DS];
-#pragma unroll
-                for (int r = 0; r < DS; ++r) w[r] = col[r];
                 F root, inv_root, inv;
                 pivot_roots(w[DS - 1], root, inv_root, inv);
                 worst = worst > FB && r0 + j < bs && !(w[DS - 1] > (F)0) ? r0 + j + 1 : worst;  // the first: its root makes the later ones NaN
-                const F f0 = v0[DS - 1] * inv, f1 = v1[DS - 1] * inv;
+                const F f0 = v0[DS - 1] * inv, f1 = v1[DS - 1] * inv, fu = u[DS - 1] * inv;
                 // what lies right of the diagonal is stored along and never read
                 F *const row = S + (r0 + j) * DLDS;
-                row[lane] = lane == r0 + j ? root : v0[DS - 1] * inv_root;
-                if (second) row[lane + 32] = lane + 32 == r0 + j ? root : v1[DS - 1] * inv_root;
+                row[c0] = c0 == r0 + j ? root : v0[DS - 1] * inv_root;
+                if (second) row[c1] = v1[DS - 1] * inv_root;
                 pivots[r0 + j] = inv_root;
+                F *const col = column[j & 1];
+#pragma unroll
+                for (int r = DS - 1; r > 0; --r) v0[r] = fma(-f0, w[r - 1], v0[r - 1]);
+                if (lane == owner + j - 2) {
+#pragma unroll
+                    for (int r = 0; r < DS; ++r) col[r] = v0[r];
+                }
+                __syncwarp();
 #pragma unroll
                 for (int r = DS - 1; r > 0; --r) {
-                    v0[r] = v0[r - 1] - f0 * w[r - 1];
-                    v1[r] = v1[r - 1] - f1 * w[r - 1];
+                    v1[r] = fma(-f1, w[r - 1], v1[r - 1]);
+                    w[r] = fma(-fu, w[r - 1], u[r - 1]);
                 }
+#pragma unroll
+                for (int r = 0; r < DS; ++r) u[r] = col[r];
             }
             if constexpr (sizeof(F) == sizeof(double)) {
                 __syncwarp();
