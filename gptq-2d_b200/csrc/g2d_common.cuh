@@ -60,7 +60,7 @@ __device__ __forceinline__ float affine_value_rcp(float y, float scale, float zp
 }
 // The stage loop's form, for bounds that are integers below 2^22 in size: then clamping and rounding commute, and a clamped value is
 // rounded half to even by adding and subtracting 1.5 * 2^23, eight cycles instead of the conversion unit's twenty-odd.
-// NaN stays NaN as with the comparisons above.  Returns code - zp, from which the chain goes on with one multiply-add, and in `clamped` what
+// NaN stays NaN as with the comparisons above.  Returns code - zp, whose product with the scale the chain goes on with, and in `clamped` what
 // affine_value_after needs to form the value away from the chain: the difference code + 1.5 * 2^23 - 1.5 * 2^23 has lost the sign of a zero
 // (a quotient of -0.3 rounds to -0).  ZERO: the zero point is +0, which leaves two additions out of the chain.
 template <bool ZERO>

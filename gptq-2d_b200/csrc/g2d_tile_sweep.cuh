@@ -205,21 +205,23 @@ __device__ __forceinline__ void sweep_sub_tile(const SubTile<F> tile, const int 
             F kc_next[SUB], pa_next[3];
             fetch(dg + (uint32_t)((j + 1) * DLD * (int)sizeof(F)), par + par_bytes, kc_next, pa_next);
             const F yv = acc[0] + other;
-            F result, carried;  // what is stored: the rounded value or what it follows from, and the completed C (row lanes) or the error (column lanes)
+            F z, result;  // the rounded value, and what is stored of it: itself or what write_rounded forms it from
             if constexpr (KIND == G2D_Q_AFFINE && DIVIDE >= 3) {
-                // E = z - (Y + C), and the completed C = C + E = z - Y, from the unrounded product of code and scale
-                carried = fmaf(affine_steps_fast<DIVIDE == 4>(yv, pa[0], pa[2], pa[1], qmin, qmax, result), pa[0], role ? -acc[0] : -yv);
+                z = mul_rn(affine_steps_fast<DIVIDE == 4>(yv, pa[0], pa[2], pa[1], qmin, qmax, result), pa[0]);
             } else {
                 if (KIND == G2D_Q_AFFINE) {
-                    result = DIVIDE == 2 ? affine_value(yv, pa[0], pa[2], qmin, qmax) : affine_value_rcp(yv, pa[0], pa[2], pa[1], qmin, qmax);
+                    z = DIVIDE == 2 ? affine_value(yv, pa[0], pa[2], qmin, qmax) : affine_value_rcp(yv, pa[0], pa[2], pa[1], qmin, qmax);
                 } else if (KIND == G2D_Q_FORCED) {
-                    result = pa[0];
+                    z = pa[0];
                 } else {
-                    result = rint_even(yv);
+                    z = rint_even(yv);
                 }
-                if (sizeof(F) == sizeof(float)) carried = result - (role ? acc[0] : yv);
-                else carried = (result - yv) + (role ? other : (F)0);  // the reference's order
+                result = z;
             }
+            // What is pushed: the error E of the float that is stored (column lanes), the completed C + E (row lanes), in the reference's order.  (Both
+            // from the unrounded product of code and scale are one multiply-add and two additions less on the chain, but leave up to half an ulp of
+            // Z out of the feedback, and an infinite C is then no NaN in what goes to the right.)
+            const F carried = (z - yv) + (role ? other : (F)0);
             const F v = ok ? carried : (F)0;     // lanes without an entry push zero
             // the push moves every accumulator down by one register on the way
             const F last = acc[0];

@@ -65,6 +65,35 @@ def test_stages_chosen_by_sub_tile(m, n, dtype):
     assert torch.equal(got, want) and torch.equal(torch.signbit(got), torch.signbit(want))
 
 
+@pytest.mark.parametrize("m, n", [(64, 64), (130, 190), (77, 333), (520, 901)])
+@pytest.mark.parametrize("offset", [0, 2 ** 18])
+def test_feedback_of_the_values_that_are_stored(m, n, offset):
+    """Scales in full precision, sub-tiles with zero points and without, factors that couple all entries: an ordinary sweep (short stages) commits
+    what a sweep that records its values before rounding does (long stages), those follow from the recorded values, and Z - X = L E U with
+    the errors of the stored floats.  Large zero points make half an ulp of Z a sixty-fourth of a code."""
+    import _abi
+    import gptq_2d as G
+
+    gen = torch.Generator(device="cuda").manual_seed(m + n)
+    rand = lambda *shape: torch.randn(*shape, generator=gen, device="cuda")
+    l, u = torch.tril(rand(m, m) * 0.3 / m ** 0.5, -1), torch.triu(rand(n, n) * 0.3 / n ** 0.5, 1)
+    scale = 0.1 + 0.05 * torch.rand(m, n, generator=gen, device="cuda")
+    some = torch.randint(0, 2, ((m + 15) // 16, (n + 15) // 16), generator=gen, device="cuda").repeat_interleave(16, 0).repeat_interleave(16, 1)[:m, :n]
+    zero = some * (offset + torch.randint(1, 8, (m, n), generator=gen, device="cuda")).float()
+    w = (4 * rand(m, n) - zero) * scale
+    ordinary = quantize(w, l, u, scale, zero)
+    y, _, _, batch_shape = G._prepare_output(w, l, u, False)
+    pre = torch.empty_like(y)
+    G._sweep_fused(y, l, u, batch_shape, dict(kind=_abi.Q_AFFINE, qmin=-8, qmax=7), (scale, zero), y_pre=pre)
+    assert torch.equal(ordinary, y)
+    assert torch.equal(y, (torch.clamp(torch.round(pre / scale + zero), -8, 7) - zero) * scale)
+    wide = torch.float64
+    e, lower, upper = y.to(wide) - pre.to(wide), l.to(wide) + torch.eye(m, device="cuda", dtype=wide), u.to(wide) + torch.eye(n, device="cuda", dtype=wide)
+    # m + n products and additions per entry, each rounded at the size of the sums that it joins
+    magnitude = lower.abs() @ e.abs() @ upper.abs() + w.abs()
+    assert ((y.to(wide) - w.to(wide) - lower @ e @ upper).abs() <= (m + n) * 2.0 ** -24 * magnitude).all()
+
+
 @pytest.mark.parametrize("raised", [0.0, 3.0, 40.0])
 def test_last_sub_tile_sets_the_scale(raised, monkeypatch):
     """Operand planes are made before the last sub-tile of a tile is swept, under the scale of the others: where that sub-tile has the largest

@@ -31,6 +31,22 @@ def test_double_quotients_beyond_the_range(value, scale):
     assert torch.equal(fused[~fed], generic[~fed])
 
 
+@pytest.mark.parametrize("m, n", [(16, 16), (40, 50), (130, 190)])
+def test_infinite_feedback_from_above(m, n, oracle):
+    """Below an infinite value the completed C, (Z - Y) + C, is NaN, and so is what the entries to the right receive, as in the oracle."""
+    import gptq_2d as G
+
+    rng = np.random.default_rng(m)
+    w, l, u = (rng.standard_normal(s).astype(np.float32) for s in ((m, n), (m, m), (n, n)))
+    l, u = np.tril(0.1 * l, -1), np.triu(0.1 * u, 1)
+    z = np.rint(w)
+    w[4, 9] = np.inf
+    want = oracle.sweep(w, l, u, kind=oracle.Q_FORCED, forced_z=z, return_y_pre=True)[1]
+    cuda = lambda a: torch.from_numpy(a).cuda()
+    got = G.gptq_2d_forced(cuda(w), cuda(l), cuda(u), cuda(z))[1].cpu().numpy()
+    assert np.isnan(want[5:, 10:]).all() and np.isnan(got[5:, 10:]).all()
+
+
 @pytest.mark.parametrize("qmin, qmax, zero", [(-8, 7, 0.0), (0, 15, 0.0), (-15, 0, 0.0), (0, 15, 8.0), (-8, 7, -0.0), (-8, 7, 3.0)])
 @pytest.mark.parametrize("m, n", [(64, 64), (100, 71), (200, 333)])
 @pytest.mark.parametrize("scale_sign", [1, -1])
