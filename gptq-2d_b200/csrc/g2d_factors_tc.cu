@@ -481,11 +481,11 @@ int launch_trinv_tc(int count, const FactorPlanes *problems, cudaStream_t stream
             job.second = second;
             if (b < DUO_BLOCK) {
                 trinv_tc_kernel<<<dim3((unsigned)(pairs * count), (unsigned)tiles, (unsigned)tiles), TC_THREADS, smem, stream>>>(job);
+                if (check_launch() != G2D_OK) return G2D_ERR_CUDA;
             } else {
                 const int64_t edge = b / DUO_EDGE;
                 if (launch_duo(trinv_duo_kernel, dim3((unsigned)(2 * edge * edge), (unsigned)(pairs * count)), PAIR_THREADS, smem, stream, job) != G2D_OK) return G2D_ERR_CUDA;
             }
-            if (check_launch() != G2D_OK) return G2D_ERR_CUDA;
         }
     }
     return G2D_OK;

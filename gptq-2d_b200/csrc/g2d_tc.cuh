@@ -187,7 +187,7 @@ __device__ __forceinline__ void tmem_free(uint32_t tmem, uint32_t cols) {
     if (DUO) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(cols) : "memory");
     else asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(cols) : "memory");
 }
-// a launch of clusters of two CTAs along x
+// a launch of clusters of two CTAs along x, counted here
 template <typename Job>
 inline int launch_duo(void (*kernel)(Job), dim3 grid, int threads, size_t smem, cudaStream_t stream, const Job &job) {
     cudaLaunchConfig_t config{};
