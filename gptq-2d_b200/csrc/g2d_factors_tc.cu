@@ -284,7 +284,13 @@ __global__ void __launch_bounds__(PAIR_THREADS, 1) trinv_duo_kernel(const __grid
     }
     const int64_t m0 = tile_m0 + rank * MT;
     const int chunks = (int)ceil_div(k_hi - k_lo, (int64_t)KH);  // a ragged tail reads zeros beyond the matrix
-    const int slices = (chunks + TRINV_SLICE - 1) / TRINV_SLICE;
+    // The ranges of k of the two CTAs' rows differ by 128: the first chunks of the first product belong to CTA 0's rows alone, the last ones of the
+    // second to CTA 1's.  A slice boundary lies where they part (the first slice is half a slice), and the other CTA leaves that
+    // slice out of its sums: zeros in place of its operand would carry NaN and infinities of the other operand into its rows.
+    constexpr int APART = MT / KH;
+    static_assert(TRINV_SLICE == 2 * APART && DUO_EDGE == TRINV_SLICE * KH, "a tile's ranges of k begin and end with half a slice");
+    const int slices = (chunks + APART + TRINV_SLICE - 1) / TRINV_SLICE;
+    const int not_mine = job.second ? (rank == 0 && k_hi > tile_m0 + MT ? slices - 1 : -1) : rank == 1 ? 0 : -1;
 
     const uint32_t smem_base = (smem_u32(tc_smem_raw) + 1023u) & ~1023u;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -319,10 +325,8 @@ __global__ void __launch_bounds__(PAIR_THREADS, 1) trinv_duo_kernel(const __grid
                 const uint32_t dst = smem_base + stage * TRINV_STAGE_BYTES, bar = leaders(&ring.full[stage]);
                 // both CTAs' bytes count at the leader's barrier (they may do so before it expects them: the phase waits for its arrival)
                 if (rank == 0) mbar_expect_tx(&ring.full[stage], 2 * TRINV_STAGE_BYTES);
-                // the ranges of k of the two CTAs' rows differ by 128: outside its own a CTA's operand is zeros, loaded from outside the matrix
-                const bool none = job.second ? rank == 0 && k >= tile_m0 + MT : rank == 1 && k < tile_m0 + MT;
                 for (int part = 0; part < 3; ++part) {
-                    tma_load_2d_duo(dst + part * HTILE_BYTES, &a_maps[part], k, none ? (int)n : (int)m0, bar);
+                    tma_load_2d_duo(dst + part * HTILE_BYTES, &a_maps[part], k, (int)m0, bar);
                     tma_load_2d_duo(dst + (3 + part) * HTILE_BYTES, &maps->tw[part], k, (int)n0 + rank * MT, bar);
                 }
             }
@@ -336,7 +340,7 @@ __global__ void __launch_bounds__(PAIR_THREADS, 1) trinv_duo_kernel(const __grid
             int slice = 0;
             for (int ch = 0; ch < chunks; ++ch) {
                 const int stage = ch % TRINV_STAGES, round = ch / TRINV_STAGES;
-                const bool opens = ch % TRINV_SLICE == 0, closes = ch % TRINV_SLICE == TRINV_SLICE - 1 || ch == chunks - 1;
+                const bool opens = ch == 0 || ch % TRINV_SLICE == APART, closes = ch % TRINV_SLICE == APART - 1 || ch == chunks - 1;
                 if (!mbar_wait_cluster(&ring.full[stage], round & 1)) { ring.failed = 1; break; }
                 // the accumulators must have been read out for the slice before
                 if (opens && slice > 0 && !mbar_wait_cluster(&ring.acc_empty[0], (slice - 1) & 1)) { ring.failed = 1; break; }
@@ -382,12 +386,14 @@ __global__ void __launch_bounds__(PAIR_THREADS, 1) trinv_duo_kernel(const __grid
             if (!ok) ring.failed = 1;
             go = __all_sync(0xffffffffu, ok && !ring.failed);  // warp-uniform: the tensor-memory loads are warp-wide
             if (!go) break;
+            if (s >> 1 != not_mine) {
 #pragma unroll
-            for (int cb = 0; cb < MT / 16; ++cb) {  // 16 at a time, as in pair_gemm
-                uint32_t v[16];
-                tmem_load_16(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(which * DUO_EDGE + c0 + cb * 16), v);
+                for (int cb = 0; cb < MT / 16; ++cb) {  // 16 at a time, as in pair_gemm
+                    uint32_t v[16];
+                    tmem_load_16(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(which * DUO_EDGE + c0 + cb * 16), v);
 #pragma unroll
-                for (int x = 0; x < 16; ++x) total[cb * 16 + x] += __uint_as_float(v[x]);
+                    for (int x = 0; x < 16; ++x) total[cb * 16 + x] += __uint_as_float(v[x]);
+                }
             }
             // this warp has read the accumulator: hand it back to the MMA warp
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");

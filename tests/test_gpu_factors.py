@@ -82,6 +82,19 @@ def test_large_blocks_against_float64(K, n):
     assert error.norm().item() < 2e-6 * l.norm().item()
 
 
+@pytest.mark.parametrize("n, i, k", [(12300, 5000, 100), (12300, 7000, 300), (12300, 9000, 4500), (8300, 8200, 100)])
+def test_products_of_large_blocks_keep_to_their_own_rows(K, n, i, k):
+    """NaN in column k of the Gram fails pivot k + 1 and fills the factor's columns up to k.  The products go by tiles of 128 rows, whose zeros it
+    meets too: columns of later tiles stay finite, also where two CTAs share a tile of 256."""
+    gram = 1e-3 * torch.randn(n, n, generator=torch.Generator(device="cuda").manual_seed(n), device="cuda")
+    gram = gram + gram.T + 2 * torch.eye(n, device="cuda")
+    gram[i, k] = gram[k, i] = float("nan")
+    l, _ = K.feedback_factors_from_grams(gram, gram)
+    assert l[k + 1:, :k + 1].isnan().all() and l[:, (k // 128 + 1) * 128:].isfinite().all()
+    with pytest.raises(torch.linalg.LinAlgError):
+        K.check_pending()
+
+
 def test_feedback_factors_and_errors(K):
     gen = torch.Generator(device="cuda").manual_seed(0)
     a = torch.randn(24, 24, generator=gen, device="cuda", dtype=torch.float64)
