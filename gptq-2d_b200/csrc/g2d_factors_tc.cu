@@ -47,13 +47,17 @@ constexpr int TRINV_STAGE_BYTES = 6 * HTILE_BYTES;         // A hi, mid, lo; B h
 constexpr int TRINV_SLICE = 4;                             // chunks per slice: k = 256
 constexpr uint32_t TRINV_TMEM_COLS = 4 * MT;               // two alternating pairs of (main, correction) accumulators
 constexpr uint32_t TRINV_DESC = idesc_16(MT, 1);           // bf16
-// Two CTAs of a cluster per 256 x 256 tile (trinv_duo_kernel) at the levels with large blocks.  Alone a CTA reads 256 rows of shared memory per MMA of
-// 64 cycles and fills 768 per six of them, 1.5 times what the port gives meanwhile; two CTAs read 256 each (384 with the other's half) per MMA of 128
-// cycles and fill 768 per six.  Tiles of the moment share their strips in L2.  Small blocks lose by the coarser tiles: a whole preparation
-// with two CTAs from b = 2048 on takes 1.85 ms at 2048 and 3000 (1.79 alone), 2.68 ms at 4096 and 4096 (2.59), 7.50 at 8192 and 8192 (7.67), 84.2 at
-// 8192 and 28672 (97); from b = 4096 on 1.79, 2.59, 7.47 and 84.6, from b = 8192 on 1.79, 2.59, 7.68 and 85.3.  (256 x 128 tiles with half of
-// the second operand each, three stages and alternating accumulators: 92 ms at 8192 and 28672.)
-constexpr int DUO_BLOCK = 4096;
+// Two CTAs of a cluster per 256 x 256 tile (trinv_duo_kernel) where blocks are large and their tiles many.  Alone a CTA reads 256 rows of shared memory per
+// MMA of 64 cycles and fills 768 per six of them, 1.5 times what the port gives meanwhile; two CTAs read 256 each (384 with the other's half) per MMA of 128
+// cycles and fill 768 per six.  Tiles of the moment share their strips in L2: factors of 8192 and 28672 97 ms alone, 84.6 with two CTAs from blocks
+// of 4096 on.  (256 x 128 tiles with half of the second operand each, three stages and alternating accumulators: 92 ms.)
+// But a cluster takes a third longer for its tile than a CTA for one of the four, and a level with few tiles lasts as long as its longest.
+// Whole preparations in ms, alone and with two CTAs at one level, by the tiles of 256 x 256 there: blocks of 4096, 16 tiles (n = 4352) 2.30 and
+// 2.38, 128 (6144) 3.41 and 3.47, 256 (8192) 5.03 and 5.05, 320 (6656 twice) 5.01 and 5.03, 384 (7168 twice) 5.71 and 5.70, 512 (8192 twice) 7.30
+// and 7.13; of 8192, 64 (8704) 5.63 and 5.73, 128 (9216) 6.11 and 6.13, 384 (11264) 8.69 and 8.68, 512 (12288) 10.32 and 10.24; of 16384, 64
+// (16640) 19.33 and 19.34, 256 (17408) 21.86 and 21.72.  So from five tiles of 4096 per cluster on, and of larger blocks as much work.  Blocks of
+// 2048 do not gain at any number: 512 tiles (16384 twice) 33.74 and 33.81.
+constexpr int DUO_BLOCK = 4096, DUO_TILES_EACH = 5;
 
 // fp32 -> three bf16 values with a = hi + mid + lo exactly (8 significant bits each)
 __device__ __forceinline__ void split_bf16_3(float a, __nv_bfloat16 &hi, __nv_bfloat16 &mid, __nv_bfloat16 &lo) {
@@ -459,6 +463,13 @@ static bool factor_maps(FactorMaps *maps, const FactorPlanes &p) {
     return ok;
 }
 
+// Tiles of 256 x 256 in a product of the level b: a pair's second half may end with the matrix, or be missing.
+static int64_t duo_tiles_of_level(int64_t n, int64_t b) {
+    int64_t tiles = 0;
+    for (int64_t r1 = b; r1 < n; r1 += 2 * b) tiles += b / DUO_EDGE * ceil_div(n - r1 < b ? n - r1 : b, (int64_t)DUO_EDGE);
+    return tiles;
+}
+
 // Levels b = 128, 256, ... of the doubling for one or two problems whose 128 x 128 diagonal blocks are finished.
 int launch_trinv_tc(int count, const FactorPlanes *problems, cudaStream_t stream) {
     static PerDeviceOnce configured;
@@ -483,9 +494,12 @@ int launch_trinv_tc(int count, const FactorPlanes *problems, cudaStream_t stream
         job.pairs = (int)pairs;
         job.tiles = (int)tiles;
         job.b = b;
+        int64_t duo = 0;
+        for (int z = 0; z < count; ++z) duo += duo_tiles_of_level(job.p[z].n, b);
+        const bool two_ctas = b >= DUO_BLOCK && duo * (b / DUO_BLOCK) >= DUO_TILES_EACH * 74;
         for (int second = 0; second < 2; ++second) {
             job.second = second;
-            if (b < DUO_BLOCK) {
+            if (!two_ctas) {
                 trinv_tc_kernel<<<dim3((unsigned)(pairs * count), (unsigned)tiles, (unsigned)tiles), TC_THREADS, smem, stream>>>(job);
                 if (check_launch() != G2D_OK) return G2D_ERR_CUDA;
             } else {

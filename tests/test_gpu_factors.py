@@ -82,6 +82,25 @@ def test_large_blocks_against_float64(K, n):
     assert error.norm().item() < 2e-6 * l.norm().item()
 
 
+@pytest.mark.parametrize("n, other", [(8071, 7900), (12289, 8192), (8300, 12300)])
+def test_pairs_with_many_large_blocks_against_float64(K, n, other):
+    """Sizes with enough tiles of large blocks for two CTAs per tile: ragged second halves, of one row, of a tile or less, a full pair beside one that
+    ends early.  The tolerances of the single factors above."""
+    grams = []
+    for k in (n, other):
+        gen = torch.Generator(device="cuda").manual_seed(k)
+        x = torch.randn(k + k // 2, k, generator=gen, device="cuda") * torch.exp(0.5 * torch.randn(k, generator=gen, device="cuda"))
+        grams.append(x.T @ x / x.size(0))
+        grams[-1].diagonal().add_(0.01 * grams[-1].diagonal().mean())
+    l, u = K.feedback_factors_from_grams(*grams, check=True)
+    for got, gram in ((l, grams[0]), (u.T, grams[1])):
+        want = K.ldl_of_inverse(gram.double(), 1)
+        check_structure(got, 1)
+        error = (got.double() - want).abs()
+        assert error.max().item() < 2e-5 * max(1.0, want.abs().max().item())
+        assert error.norm().item() < 2e-6 * want.norm().item()
+
+
 @pytest.mark.parametrize("n, i, k", [(12300, 5000, 100), (12300, 7000, 300), (12300, 9000, 4500), (8300, 8200, 100)])
 def test_products_of_large_blocks_keep_to_their_own_rows(K, n, i, k):
     """NaN in column k of the Gram fails pivot k + 1 and fills the factor's columns up to k.  The products go by tiles of 128 rows, whose zeros it
