@@ -248,6 +248,7 @@ __global__ void __launch_bounds__(TC_THREADS) trinv_tc_kernel(const __grid_const
 // of the next.
 struct TrinvDuoRing {
     uint64_t full[TRINV_STAGES], empty[TRINV_STAGES], acc_full[2], acc_empty[2];  // accumulators: main, correction
+    uint64_t drained;  // as in PairRing
     uint32_t tmem;
     int failed;
 };
@@ -307,6 +308,7 @@ __global__ void __launch_bounds__(PAIR_THREADS, 1) trinv_duo_kernel(const __grid
             mbar_init(&ring.acc_full[s], 1);
             mbar_init(&ring.acc_empty[s], 16);  // one arrival per reading warp of both CTAs, at the leader's
         }
+        mbar_init(&ring.drained, 1);
         ring.failed = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -319,7 +321,8 @@ __global__ void __launch_bounds__(PAIR_THREADS, 1) trinv_duo_kernel(const __grid
     const uint32_t tmem = ring.tmem;
     if (warp == 0) {
         if (lane == 0) {
-            for (int ch = 0; ch < chunks; ++ch) {
+            int ch = 0;
+            for (; ch < chunks; ++ch) {
                 const int stage = ch % TRINV_STAGES, round = ch / TRINV_STAGES;
                 if (round > 0 && !mbar_wait_cluster(&ring.empty[stage], (round - 1) & 1)) {
                     ring.failed = 1;
@@ -334,9 +337,12 @@ __global__ void __launch_bounds__(PAIR_THREADS, 1) trinv_duo_kernel(const __grid
                     tma_load_2d_duo(dst + (3 + part) * HTILE_BYTES, &maps->tw[part], k, (int)n0 + rank * MT, bar);
                 }
             }
+            // both CTAs' last loads have landed, or had their time to, before their shared memory is given back, whatever became of the MMAs
+            if (rank == 0)
+                for (int k = max(ch - TRINV_STAGES, 0); k < ch; ++k) mbar_wait_cluster(&ring.full[k % TRINV_STAGES], (k / TRINV_STAGES) & 1);
             // the leader's commits arrive here as well: none may be under way when this CTA ends (those of the accumulators are awaited below)
-            for (int ch = max(chunks - TRINV_STAGES, 0); ch < chunks && !ring.failed; ++ch)
-                if (!mbar_wait_cluster(&ring.empty[ch % TRINV_STAGES], (ch / TRINV_STAGES) & 1)) ring.failed = 1;
+            for (int k = max(chunks - TRINV_STAGES, 0); k < chunks && !ring.failed; ++k)
+                if (!mbar_wait_cluster(&ring.empty[k % TRINV_STAGES], (k / TRINV_STAGES) & 1)) ring.failed = 1;
         }
     } else if (warp == 1) {
         if (lane == 0 && rank == 0) {
@@ -373,8 +379,13 @@ __global__ void __launch_bounds__(PAIR_THREADS, 1) trinv_duo_kernel(const __grid
                     ++slice;
                 }
             }
-            // on time-out, give what is in flight a bounded chance to land before its memory is released
-            if (ring.failed && slice > 0) mbar_wait(&ring.acc_full[1], (slice - 1) & 1);
+            // every MMA that was issued completes, or has its time to, as in pair_gemm
+            if (ring.failed) {
+                commit<true>(&ring.drained);
+                mbar_wait_cluster(&ring.drained, 0);
+            } else {
+                mbar_wait_cluster(&ring.acc_full[1], (slice - 1) & 1);
+            }
         }
     } else {
         // reading warps: lanes 32 q .. 32 q + 31 of tensor memory, q = warp % 4, and half of the columns; 128 running sums in registers
@@ -409,6 +420,7 @@ __global__ void __launch_bounds__(PAIR_THREADS, 1) trinv_duo_kernel(const __grid
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     // neither CTA leaves while the other's MMAs may read its shared memory or arrive at its barriers
+    if (threadIdx.x == 0 && ring.failed) let_it_land();
     __syncwarp();
     cluster_sync();
     if (warp == 1) tmem_free<true>(tmem, COLS);

@@ -109,6 +109,7 @@ struct GramJob {
     int chunks;
     float alpha;
     int *flag;
+    long long wait_cycles;  // limit of the waits
 };
 
 template <int NT, bool DUO>
@@ -184,7 +185,7 @@ __global__ void __launch_bounds__(PAIR_THREADS, 1) gram_tc_kernel(const __grid_c
             }
         }
     };
-    const bool failed = pair_gemm<NT, NSTAGE, GRAM_SLICE, DUO>(ring, smem_base, next, load, finish);
+    const bool failed = pair_gemm<NT, NSTAGE, GRAM_SLICE, DUO>(ring, smem_base, next, load, finish, PairNoScale(), job.wait_cycles);
     if (threadIdx.x == 0 && failed && job.flag) atomicExch(job.flag, -1);
 }
 
@@ -220,8 +221,8 @@ extern "C" int g2d_gram_workspace_bytes(int64_t n, int64_t k, size_t *bytes) {
     return G2D_OK;
 }
 
-extern "C" int g2d_gram_accumulate(int64_t n, int64_t k, const float *x, float alpha, float *h, int32_t *status_flag, void *workspace,
-                                   size_t workspace_bytes, void *stream) {
+static int accumulate(int64_t n, int64_t k, const float *x, float alpha, float *h, int32_t *status_flag, void *workspace, size_t workspace_bytes, long long wait_cycles,
+                      void *stream) {
     if (n < 0 || k < 0) return G2D_ERR_BAD_ARGUMENT;
     if (n == 0 || k == 0) return G2D_OK;
     if (!x || !h || n % 4 != 0 || ((uintptr_t)h & 15) != 0 || ((uintptr_t)x & 3) != 0) return G2D_ERR_BAD_ARGUMENT;
@@ -255,9 +256,22 @@ extern "C" int g2d_gram_accumulate(int64_t n, int64_t k, const float *x, float a
     job.chunks = (int)ceil_div(kp, (int64_t)KH);
     job.alpha = alpha;
     job.flag = status_flag;
+    job.wait_cycles = wait_cycles;
     const int64_t square = lower_tiles<128>(rows), wide = lower_tiles<256>(rows), duo = duo_tiles(ceil_div(rows, (int64_t)2));
     const TileChoice choice = tiles_that_pay(square, wide, duo);
     if (choice == DUO_TILES) return launch_gram<256, true>(job, hi, lo, kp, duo, st);
     if (choice == WIDE_TILES) return launch_gram<256, false>(job, hi, lo, kp, wide, st);
     return launch_gram<128, false>(job, hi, lo, kp, square, st);
+}
+
+extern "C" int g2d_gram_accumulate(int64_t n, int64_t k, const float *x, float alpha, float *h, int32_t *status_flag, void *workspace,
+                                   size_t workspace_bytes, void *stream) {
+    return accumulate(n, k, x, alpha, h, status_flag, workspace, workspace_bytes, WAIT_CYCLES, stream);
+}
+
+// For tests: with a limit of its own on the waits inside the kernel.  One that runs out sets *status_flag to -1 and leaves H incomplete.
+extern "C" int g2d_gram_accumulate_limited(int64_t n, int64_t k, const float *x, float alpha, float *h, int32_t *status_flag, void *workspace,
+                                           size_t workspace_bytes, int64_t wait_cycles, void *stream) {
+    if (wait_cycles < 0 || wait_cycles > WAIT_CYCLES) return G2D_ERR_BAD_ARGUMENT;
+    return accumulate(n, k, x, alpha, h, status_flag, workspace, workspace_bytes, wait_cycles, stream);
 }

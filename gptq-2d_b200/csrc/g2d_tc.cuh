@@ -36,10 +36,10 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t *bar, uint32_t parity) {
 }
 // false on time-out.  Between polls the warp sleeps for `nap` nanoseconds: several CTAs of an update kernel share an SM, and the
 // warps that work should not lose issue slots to those that wait.
-__device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, unsigned nap = 32) {
+__device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, unsigned nap = 32, long long limit = WAIT_CYCLES) {
     const long long start = clock64();
     while (!mbar_try_wait(bar, parity)) {
-        if (clock64() - start > WAIT_CYCLES) return false;
+        if (clock64() - start > limit) return false;
         __nanosleep(nap);
     }
     return true;
@@ -127,7 +127,7 @@ __device__ __forceinline__ uint32_t leaders(uint64_t *bar) {  // the same barrie
 }
 __device__ __forceinline__ void mbar_arrive_at(uint32_t bar) { asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory"); }
 // as mbar_wait, for what a thread of the other CTA may have arrived at
-__device__ __forceinline__ bool mbar_wait_cluster(uint64_t *bar, uint32_t parity, unsigned nap = 32) {
+__device__ __forceinline__ bool mbar_wait_cluster(uint64_t *bar, uint32_t parity, unsigned nap = 32, long long limit = WAIT_CYCLES) {
     const long long start = clock64();
     for (;;) {
         uint32_t ok;
@@ -139,7 +139,7 @@ __device__ __forceinline__ bool mbar_wait_cluster(uint64_t *bar, uint32_t parity
             : "r"(smem_u32(bar)), "r"(parity)
             : "memory");
         if (ok) return true;
-        if (clock64() - start > WAIT_CYCLES) return false;
+        if (clock64() - start > limit) return false;
         __nanosleep(nap);
     }
 }
@@ -186,6 +186,12 @@ template <bool DUO>
 __device__ __forceinline__ void tmem_free(uint32_t tmem, uint32_t cols) {
     if (DUO) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(cols) : "memory");
     else asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(cols) : "memory");
+}
+// One thread, after a time-out in a pair of CTAs: a load of this CTA may count at a barrier that nobody awaits any more, and a commit be on its way
+// to the other CTA.  They land within microseconds; a millisecond on, the shared memory may be given back.
+__device__ __forceinline__ void let_it_land() {
+    const long long start = clock64();
+    while (clock64() - start < WAIT_CYCLES / 1000) __nanosleep(1000);
 }
 // a launch of clusters of two CTAs along x, counted here
 template <typename Job>
@@ -298,6 +304,7 @@ constexpr int PAIR_BOXES = 8 * BOX_BYTES;  // one per reading warp, where the re
 template <int NSTAGE>
 struct PairRing {
     uint64_t full[NSTAGE], empty[NSTAGE], acc_full[2], acc_empty[2];
+    uint64_t drained;  // after a time-out: every MMA that was issued has completed
     uint32_t tmem;
     int failed;
 };
@@ -307,19 +314,20 @@ struct PairRing {
 // B_hi, B_lo tiles one after the other.  finish(tile, q, lane, first column, totals, 4 KB of shared memory of the warp's own
 // behind the stages).  DUO: by two CTAs of a cluster whose tiles differ in i0 only; load brings half of B's rows and counts at the barrier
 // of CTA 0.  scale(tile, slice, q, column), optional: what a slice's sums are multiplied by, the same for 64 columns.
-// Returns whether a wait ran out.
+// Returns whether a wait ran out (of `limit` cycles; those that only let what is in flight come to its end have the usual limit).
 struct PairTile {
     int i0, j0, chunks;
     int k0 = 0, which = 0;  // first k and a number of the caller's
 };
 struct PairNoScale {};
 template <int NT, int NSTAGE, int SLICE, bool DUO = false, typename Next, typename Load, typename Finish, typename Scale = PairNoScale>
-__device__ __forceinline__ bool pair_gemm(PairRing<NSTAGE> &ring, uint32_t smem_base, Next next, Load load, Finish finish, Scale scale = Scale()) {
+__device__ __forceinline__ bool pair_gemm(PairRing<NSTAGE> &ring, uint32_t smem_base, Next next, Load load, Finish finish, Scale scale = Scale(), long long limit = WAIT_CYCLES) {
     constexpr bool SCALED = !std::is_same<Scale, PairNoScale>::value;
     constexpr int B_BYTES = NT * KH * 2 / (DUO ? 2 : 1), STAGE = 2 * HTILE_BYTES + 2 * B_BYTES, MINE = NT / 2;
     constexpr uint32_t COLS = 2 * NT, DESC = idesc_16(NT, 0, DUO ? 2 * MT : MT);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, rank = DUO ? (int)cluster_rank() : 0;
-    const auto wait = [](uint64_t *bar, uint32_t parity, unsigned nap = 32) { return DUO ? mbar_wait_cluster(bar, parity, nap) : mbar_wait(bar, parity, nap); };
+    const auto await = [](uint64_t *bar, uint32_t parity, unsigned nap, long long cycles) { return DUO ? mbar_wait_cluster(bar, parity, nap, cycles) : mbar_wait(bar, parity, nap, cycles); };
+    const auto wait = [&](uint64_t *bar, uint32_t parity, unsigned nap = 32) { return await(bar, parity, nap, limit); };
     if (threadIdx.x == 0) {
         for (int s = 0; s < NSTAGE; ++s) {
             mbar_init(&ring.full[s], 1);
@@ -329,6 +337,7 @@ __device__ __forceinline__ bool pair_gemm(PairRing<NSTAGE> &ring, uint32_t smem_
             mbar_init(&ring.acc_full[s], 1);
             mbar_init(&ring.acc_empty[s], DUO ? 16 : 8);  // one arrival per reading warp, of both CTAs at the leader's
         }
+        mbar_init(&ring.drained, 1);
         ring.failed = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -355,6 +364,9 @@ __device__ __forceinline__ bool pair_gemm(PairRing<NSTAGE> &ring, uint32_t smem_
                     load(tile, ch, smem_base + stage * STAGE, &ring.full[stage]);
                 }
             }
+            // the last loads (DUO: both CTAs') have landed, or had their time to, before their shared memory is given back, whatever became of the MMAs
+            if (rank == 0)
+                for (int k = max(c - NSTAGE, 0); k < c; ++k) await(&ring.full[k % NSTAGE], (k / NSTAGE) & 1, 32, WAIT_CYCLES);
             if (DUO && !ring.failed) {
                 // the leader's commits arrive here as well: none may be under way when this CTA ends (those of the accumulators are awaited below)
                 for (int k = max(c - NSTAGE, 0); k < c; ++k)
@@ -389,8 +401,14 @@ __device__ __forceinline__ bool pair_gemm(PairRing<NSTAGE> &ring, uint32_t smem_
                     }
                 }
             }
-            // on time-out, give what is in flight a bounded chance to land before its memory is released
-            if (ring.failed && slice > 0) mbar_wait(&ring.acc_full[(slice - 1) & 1], ((slice - 1) >> 1) & 1);
+            // every MMA that was issued completes, or has its time to, before what it reads and writes is given back: all of them closed a slice, but for
+            // those before a time-out
+            if (ring.failed) {
+                commit<DUO>(&ring.drained);
+                await(&ring.drained, 0, 32, WAIT_CYCLES);
+            } else if (slice > 0) {
+                await(&ring.acc_full[(slice - 1) & 1], ((slice - 1) >> 1) & 1, 32, WAIT_CYCLES);
+            }
         }
     } else {
         const int q = warp & 3, c0 = ((warp - 2) >> 2) * MINE;
@@ -440,6 +458,7 @@ __device__ __forceinline__ bool pair_gemm(PairRing<NSTAGE> &ring, uint32_t smem_
     __syncthreads();
     if (DUO) {
         // neither CTA leaves while the other's MMAs may read its shared memory or arrive at its barriers
+        if (threadIdx.x == 0 && ring.failed) let_it_land();
         __syncwarp();
         cluster_sync();
     }

@@ -291,6 +291,11 @@ int g2d_gram_workspace_bytes(int64_t n, int64_t k, size_t *bytes);
 int g2d_gram_accumulate(int64_t n, int64_t k, const float *x, float alpha, float *h, int32_t *status_flag,
                         void *workspace, size_t workspace_bytes, void *stream);
 
+/* The same under a limit of the caller's, in clock cycles (up to the usual 2e9), on the waits inside the kernel: a limit of 0 lets a test see
+ * one that ran out.  h is incomplete then. */
+int g2d_gram_accumulate_limited(int64_t n, int64_t k, const float *x, float alpha, float *h, int32_t *status_flag,
+                                void *workspace, size_t workspace_bytes, int64_t wait_cycles, void *stream);
+
 /* Packed integer codes of a rounded matrix z [m, n] and back.  The reference has no counterpart: it returns
  * dequantised floats and notes that the code can be recovered from them (quantizer_trellis.py:11-14; for the
  * affine quantizer, quantizer_int.py:63-83, code = rint(z / scale + zero point)).  Entry j of a row is the

@@ -42,3 +42,33 @@ def test_search_whose_waits_run_out(rows, T, K, V, tail):
     after = search(2_000_000_000)
     assert all(torch.equal(a, b) for a, b in zip(before, after)) and np.isfinite(before[0].cpu().numpy()).all()
     _abi.check_status(device)
+
+
+# tiles of one CTA and of two; fewer tiles than CTAs and more
+@pytest.mark.parametrize("n, k", [(128, 512), (2944, 300), (3072, 300), (4096, 1000)])
+def test_gram_whose_waits_run_out(n, k):
+    """Loads, products and their commits come to their end before a CTA leaves: the next call, into the same shared and tensor memory, is right."""
+    import _abi
+
+    lib = _abi.library()
+    gen = torch.Generator(device="cuda").manual_seed(n)
+    x = torch.randn(k, n, generator=gen, device="cuda")
+    size = ctypes.c_size_t()
+    _abi.check(lib.g2d_gram_workspace_bytes(n, k, ctypes.byref(size)), "g2d_gram_workspace_bytes")
+    workspace, status = torch.empty(size.value, dtype=torch.uint8, device="cuda"), torch.zeros(1, dtype=torch.int32, device="cuda")
+
+    def accumulate(wait_cycles):
+        h = torch.zeros(n, n, device="cuda")
+        status.zero_()
+        _abi.check(lib.g2d_gram_accumulate_limited(n, k, x.data_ptr(), 1.0, h.data_ptr(), status.data_ptr(), workspace.data_ptr(), size.value, wait_cycles,
+                                                   _abi.stream_of(x)), "g2d_gram_accumulate_limited")
+        return h
+
+    before = accumulate(2_000_000_000)
+    assert status.item() == 0
+    accumulate(0)
+    after = accumulate(2_000_000_000)  # enqueued behind it at once
+    assert status.item() == 0 and torch.equal(before, after)
+    accumulate(0)
+    assert status.item() == -1
+    assert lib.g2d_gram_accumulate_limited(n, k, x.data_ptr(), 1.0, before.data_ptr(), status.data_ptr(), workspace.data_ptr(), size.value, -1, _abi.stream_of(x)) == -1
