@@ -52,12 +52,13 @@ constexpr uint32_t TRINV_DESC = idesc_16(MT, 1);           // bf16
 // cycles and fill 768 per six.  Tiles of the moment share their strips in L2: factors of 8192 and 28672 97 ms alone, 84.6 with two CTAs from blocks
 // of 4096 on.  (256 x 128 tiles with half of the second operand each, three stages and alternating accumulators: 92 ms.)
 // But a cluster takes a third longer for its tile than a CTA for one of the four, and a level with few tiles lasts as long as its longest.
-// Whole preparations in ms, alone and with two CTAs at one level, by the tiles of 256 x 256 there: blocks of 4096, 16 tiles (n = 4352) 2.30 and
-// 2.38, 128 (6144) 3.41 and 3.47, 256 (8192) 5.03 and 5.05, 320 (6656 twice) 5.01 and 5.03, 384 (7168 twice) 5.71 and 5.70, 512 (8192 twice) 7.30
-// and 7.13; of 8192, 64 (8704) 5.63 and 5.73, 128 (9216) 6.11 and 6.13, 384 (11264) 8.69 and 8.68, 512 (12288) 10.32 and 10.24; of 16384, 64
-// (16640) 19.33 and 19.34, 256 (17408) 21.86 and 21.72.  So from five tiles of 4096 per cluster on, and of larger blocks as much work.  Blocks of
-// 2048 do not gain at any number: 512 tiles (16384 twice) 33.74 and 33.81.
-constexpr int DUO_BLOCK = 4096, DUO_TILES_EACH = 5;
+// Whole preparations in ms, alone and with two CTAs at one level, by a factor's tiles of 256 x 256 there, one factor and two of that size:
+// blocks of 4096, 16 tiles (n = 4352) 2.30 and 2.38, 2.70 and 2.76; 128 (6144) 3.41 and 3.47, 4.43 and 4.47; 192 (7168) 4.19 and 4.24, 5.71 and
+// 5.70; 224 (7680) 4.58 and 4.63, 6.49 and 6.41; 256 (8192) 5.03 and 5.05, 7.30 and 7.13.  Blocks of 8192, 32 tiles (8300) 5.48 and 5.59; 128
+// (9216) 6.11 and 6.13; 256 (10240) 7.43 and 7.44, 11.42 and 11.35; 512 (12288) 10.32 and 10.24, 17.53 and 17.26.  Of 16384, 64 (16640) 19.33
+// and 19.34; 256 (17408) 21.86 and 21.72.  So from three tiles per cluster on.  (By a factor's own tiles, not those of a launch: a factor has the
+// same bits alone and in a pair, and the two kernels differ in theirs.)  Blocks of 2048 do not gain: 16384 twice 33.74 and 33.81.
+constexpr int DUO_BLOCK = 4096, DUO_TILES_EACH = 3;
 
 // fp32 -> three bf16 values with a = hi + mid + lo exactly (8 significant bits each)
 __device__ __forceinline__ void split_bf16_3(float a, __nv_bfloat16 &hi, __nv_bfloat16 &mid, __nv_bfloat16 &lo) {
@@ -475,11 +476,12 @@ static bool factor_maps(FactorMaps *maps, const FactorPlanes &p) {
     return ok;
 }
 
-// Tiles of 256 x 256 in a product of the level b: a pair's second half may end with the matrix, or be missing.
-static int64_t duo_tiles_of_level(int64_t n, int64_t b) {
+// Whether a factor's products of the level b go to two CTAs per tile, by its tiles there: a pair's second half may end with the matrix, or be missing.
+static bool two_ctas_pay(int64_t n, int64_t b) {
+    if (b < DUO_BLOCK) return false;
     int64_t tiles = 0;
     for (int64_t r1 = b; r1 < n; r1 += 2 * b) tiles += b / DUO_EDGE * ceil_div(n - r1 < b ? n - r1 : b, (int64_t)DUO_EDGE);
-    return tiles;
+    return tiles >= DUO_TILES_EACH * 74;
 }
 
 // Levels b = 128, 256, ... of the doubling for one or two problems whose 128 x 128 diagonal blocks are finished.
@@ -491,32 +493,43 @@ int launch_trinv_tc(int count, const FactorPlanes *problems, cudaStream_t stream
                    cudaFuncSetAttribute(trinv_duo_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) == cudaSuccess;
         }) != G2D_OK)
         return G2D_ERR_CUDA;
-    TrinvJob job;
+    TrinvJob all;
     int64_t n_max = 0;
     for (int z = 0; z < 2; ++z) {
-        job.p[z] = problems[z < count ? z : 0];
-        if (!factor_maps(&job.maps[z], job.p[z])) return G2D_ERR_CUDA;
-        n_max = job.p[z].n > n_max ? job.p[z].n : n_max;
+        all.p[z] = problems[z < count ? z : 0];
+        if (!factor_maps(&all.maps[z], all.p[z])) return G2D_ERR_CUDA;
+        n_max = all.p[z].n > n_max ? all.p[z].n : n_max;
     }
-    trinv_split_kernel<<<dim3((unsigned)(n_max < 148 * 16 ? n_max : 148 * 16), count), 256, 0, stream>>>(job.p[0], job.p[1]);
+    trinv_split_kernel<<<dim3((unsigned)(n_max < 148 * 16 ? n_max : 148 * 16), count), 256, 0, stream>>>(all.p[0], all.p[1]);
     if (check_launch() != G2D_OK) return G2D_ERR_CUDA;
     for (int64_t b = MT; b < n_max; b *= 2) {
-        const int64_t pairs = ceil_div(n_max, 2 * b), tiles = b / MT;
-        if (tiles > 65535 || pairs * count > 0x7fffffff) return G2D_ERR_TOO_LARGE;
-        job.pairs = (int)pairs;
-        job.tiles = (int)tiles;
-        job.b = b;
-        int64_t duo = 0;
-        for (int z = 0; z < count; ++z) duo += duo_tiles_of_level(job.p[z].n, b);
-        const bool two_ctas = b >= DUO_BLOCK && duo * (b / DUO_BLOCK) >= DUO_TILES_EACH * 74;
-        for (int second = 0; second < 2; ++second) {
-            job.second = second;
-            if (!two_ctas) {
-                trinv_tc_kernel<<<dim3((unsigned)(pairs * count), (unsigned)tiles, (unsigned)tiles), TC_THREADS, smem, stream>>>(job);
-                if (check_launch() != G2D_OK) return G2D_ERR_CUDA;
-            } else {
-                const int64_t edge = b / DUO_EDGE;
-                if (launch_duo(trinv_duo_kernel, dim3((unsigned)(2 * edge * edge), (unsigned)(pairs * count)), PAIR_THREADS, smem, stream, job) != G2D_OK) return G2D_ERR_CUDA;
+        const int64_t tiles = b / MT, edge = b / DUO_EDGE;
+        if (tiles > 65535) return G2D_ERR_TOO_LARGE;
+        for (const bool two_ctas : {true, false}) {  // together what goes to the same kernel
+            TrinvJob job = all;
+            int mine = 0;
+            int64_t largest = 0;
+            for (int z = 0; z < count; ++z) {
+                if (all.p[z].n <= b || two_ctas_pay(all.p[z].n, b) != two_ctas) continue;
+                job.p[mine] = all.p[z];
+                job.maps[mine] = all.maps[z];
+                largest = all.p[z].n > largest ? all.p[z].n : largest;
+                ++mine;
+            }
+            if (mine == 0) continue;
+            const int64_t pairs = ceil_div(largest, 2 * b);
+            if (pairs * mine > 0x7fffffff) return G2D_ERR_TOO_LARGE;
+            job.pairs = (int)pairs;
+            job.tiles = (int)tiles;
+            job.b = b;
+            for (int second = 0; second < 2; ++second) {
+                job.second = second;
+                if (two_ctas) {
+                    if (launch_duo(trinv_duo_kernel, dim3((unsigned)(2 * edge * edge), (unsigned)(pairs * mine)), PAIR_THREADS, smem, stream, job) != G2D_OK) return G2D_ERR_CUDA;
+                } else {
+                    trinv_tc_kernel<<<dim3((unsigned)(pairs * mine), (unsigned)tiles, (unsigned)tiles), TC_THREADS, smem, stream>>>(job);
+                    if (check_launch() != G2D_OK) return G2D_ERR_CUDA;
+                }
             }
         }
     }

@@ -144,6 +144,12 @@ def test_pair_equals_two_single_calls(K, dtype, m, n, p, q):
     check_structure(u.T, q)
 
 
+# the inverse's large blocks: two CTAs per tile for both, for one, at one level only, for none
+@pytest.mark.parametrize("m, n", [(8192, 8192), (4300, 8192), (8300, 12300), (7680, 7000), (5000, 6000)])
+def test_large_pair_equals_two_single_calls(K, m, n):
+    test_pair_equals_two_single_calls(K, torch.float32, m, n, 1, 1)
+
+
 def test_pair_reports_the_failing_factor(K):
     good = torch.eye(130, device="cuda", dtype=torch.float64)
     with pytest.raises(torch.linalg.LinAlgError, match="H is not positive definite"):
