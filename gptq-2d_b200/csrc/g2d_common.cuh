@@ -368,4 +368,12 @@ int launch_stage_commit(const g2d_stage_desc &d, const F *z, int64_t s, cudaStre
 __device__ __forceinline__ void after_the_launch_before() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void let_the_next_launch_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
+// Clusters of CTAs: the CTA's number in its cluster, and a barrier of all threads of the cluster (by whole warps)
+__device__ __forceinline__ uint32_t cluster_rank() {
+    uint32_t r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ void cluster_sync() { asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+
 }  // namespace g2d

@@ -114,12 +114,6 @@ struct TcRing {
 
 // ---- two CTAs of a cluster on one product (cta_group::2): M = 256, 128 rows in each CTA, and half of B in each, so that a CTA fills and reads
 // shared memory for 192 rows where one on its own does for 256 of a 128 x 128 tile.  CTA 0 leads: it issues the MMAs for both. ----
-__device__ __forceinline__ uint32_t cluster_rank() {
-    uint32_t r;
-    asm volatile("mov.u32 %0, %cluster_ctarank;" : "=r"(r));
-    return r;
-}
-__device__ __forceinline__ void cluster_sync() { asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 __device__ __forceinline__ uint32_t leaders(uint64_t *bar) {  // the same barrier of CTA 0
     uint32_t r;
     asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(r) : "r"(smem_u32(bar)));
