@@ -67,7 +67,7 @@ def test_against_oracle_and_properties(K, oracle, n, size):
 
 @pytest.mark.parametrize("n", [4097, 4300, 8071, 8500])
 def test_large_blocks_against_float64(K, n):
-    """The products of two CTAs per tile (blocks of 4096 rows): second halves of one row, of a tile or less, ragged, and a last pair of blocks
+    """Blocks of 4096 rows with few tiles, which one CTA per tile takes: second halves of one row, of a tile or less, ragged, and a last pair of blocks
     without one.  Against float64; the tolerance is the one of the smaller factors above, for the largest entry and, by the root of their
     number below it, for the norm."""
     gen = torch.Generator(device="cuda").manual_seed(n)

@@ -32,19 +32,29 @@ def test_double_quotients_beyond_the_range(value, scale):
 
 
 @pytest.mark.parametrize("m, n", [(16, 16), (40, 50), (130, 190)])
-def test_infinite_feedback_from_above(m, n, oracle):
-    """Below an infinite value the completed C, (Z - Y) + C, is NaN, and so is what the entries to the right receive, as in the oracle."""
+@pytest.mark.parametrize("kind", ["forced", "divided"])
+def test_infinite_feedback_from_above(m, n, kind, oracle):
+    """Below an infinite value the completed C, (Z - Y) + C, is NaN, and so is what the entries to the right receive, as in the oracle: with values
+    committed as they are, and under scales that take the exact division (a clamped infinity is finite)."""
+    import _abi
     import gptq_2d as G
 
     rng = np.random.default_rng(m)
     w, l, u = (rng.standard_normal(s).astype(np.float32) for s in ((m, n), (m, m), (n, n)))
     l, u = np.tril(0.1 * l, -1), np.triu(0.1 * u, 1)
-    z = np.rint(w)
+    z, small = np.rint(w), np.float32(2.0 ** -70)
     w[4, 9] = np.inf
-    want = oracle.sweep(w, l, u, kind=oracle.Q_FORCED, forced_z=z, return_y_pre=True)[1]
     cuda = lambda a: torch.from_numpy(a).cuda()
-    got = G.gptq_2d_forced(cuda(w), cuda(l), cuda(u), cuda(z))[1].cpu().numpy()
-    assert np.isnan(want[5:, 10:]).all() and np.isnan(got[5:, 10:]).all()
+    if kind == "forced":
+        want = oracle.sweep(w, l, u, kind=oracle.Q_FORCED, forced_z=z, return_y_pre=True)[1]
+        got = G.gptq_2d_forced(cuda(w), cuda(l), cuda(u), cuda(z))[1]
+    else:
+        scale, zero = np.full((m, n), small), np.zeros((m, n), np.float32)
+        want = oracle.sweep(w * small, l, u, kind=oracle.Q_AFFINE, scale=scale, zero_point=zero, qmin=-8, qmax=7, return_y_pre=True)[1]
+        y, _, _, batch_shape = G._prepare_output(cuda(w * small), cuda(l), cuda(u), False)
+        got = torch.empty_like(y)
+        G._sweep_fused(y, cuda(l), cuda(u), batch_shape, dict(kind=_abi.Q_AFFINE, qmin=-8, qmax=7), (cuda(scale), cuda(zero)), y_pre=got)
+    assert np.isnan(want[5:, 10:]).all() and got[5:, 10:].isnan().all()
 
 
 @pytest.mark.parametrize("qmin, qmax, zero", [(-8, 7, 0.0), (0, 15, 0.0), (-15, 0, 0.0), (0, 15, 8.0), (-8, 7, -0.0), (-8, 7, 3.0)])
