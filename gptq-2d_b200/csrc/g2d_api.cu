@@ -337,10 +337,10 @@ constexpr double kFarBound = 1.5e8;  // entries from which on the far updates bo
 
 // Whether the tiles of an anti-diagonal and the near update of the one before are one launch (g2d_tile_sweep_step.cu).  The updating CTAs hold an SM
 // each: they keep far updates waiting where those bound the sweep, and too few SMs are left for them beside many tiles.  Apart -> together, in
-// ms, by the tiles of the longest anti-diagonal: 16, 1024 x 1024: 0.93 -> 0.82; 32, 2048 x 2048: 1.92 -> 1.69, 2048 x 65536: 83.8 -> 60.8; 64,
-// 4096 x 4096: 4.19 -> 3.66, 4096 x 28672: 31.2 -> 27.0; 112, 7168 x 20900: 33.8 -> 31.4; 128, 8192 x 8192: 11.67 -> 10.99, 8192 x 12160: 17.6 ->
-// 17.4, 8192 x 18200: 31.4 -> 30.9; 132, 8448 x 8448: 12.4 -> 11.8, 8448 x 12000: 18.0 -> 18.6; 136, 8704 x 12000: 18.6 -> 20.5; far updates as
-// the bound, 8192 x 28672: 55.9 -> 63.7.  Four sweeps on two streams, with a tile kernel of 28.5 us: 8192 x 8192 40.3 -> 39.2, 8192 x 14336 81.5 -> 78.7.
+// ms, by the tiles of the longest anti-diagonal: 16, 1024 x 1024: 0.95 -> 0.84; 32, 2048 x 2048: 1.96 -> 1.72, 2048 x 65536: 83.9 -> 62.0; 64,
+// 4096 x 4096: 4.26 -> 3.70, 4096 x 28672: 31.4 -> 27.5; 112, 7168 x 20900: 34.5 -> 32.5; 128, 8192 x 8192: 11.76 -> 11.07, 8192 x 12160: 17.8 ->
+// 17.5, 8192 x 18200: 31.9 -> 31.6; 132, 8448 x 8448: 12.5 -> 11.9, 8448 x 12000: 18.2 -> 19.5; 136, 8704 x 12000: 18.7 -> 20.7; far updates as
+// the bound, 8192 x 28672: 57.3 -> 64.3.  Four sweeps on two streams, with a tile kernel of 28.5 us: 8192 x 8192 40.3 -> 39.2, 8192 x 14336 81.5 -> 78.7.
 bool together(const SweepArgs<float> &a) {
     const int tiles = a.nI < a.nJ ? a.nI : a.nJ;
     return a.nI + a.nJ > 3 && tiles <= 128 && (double)a.m * (double)a.n < kFarBound;

@@ -11,8 +11,9 @@
 //
 // Bound: tensor pipe.  A 128 x 256 x 16 MMA of one CTA reads 12 KB of operands in 128 cycles and a chunk's 96 KB arrive in the 1536 cycles
 // of its MMAs: 160 of the port's 128 bytes per cycle, so 80 % of the tensor rate.  Two CTAs with half of B each read 8 KB and
-// fill 64 KB: 107 bytes per cycle.  8192 samples of 8192 channels: 4.61 ms with 128 x 128 tf32 tiles (60 % of half the rate, every slice added to
-// H in global memory), 1.69 ms with 128 x 256, 1.54 ms now; 2048 samples of 4096 channels 153 and 152 us.
+// fill 64 KB: 107 bytes per cycle.  8192 samples of 8192 channels, calls one after the other: 4.61 ms with 128 x 128 tf32 tiles (60 % of half the
+// rate, every slice added to H in global memory), 1.69 ms with 128 x 256, 1.54 ms now; with H cleared and the L2 emptied between calls 1.79 and
+// 1.70.  2048 samples of 4096 channels 153 and 152 us.
 #include "g2d_tc.cuh"
 
 namespace g2d {

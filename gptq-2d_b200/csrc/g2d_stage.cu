@@ -127,6 +127,7 @@ int launch_stage_commit(const g2d_stage_desc &d, const F *z, int64_t s, cudaStre
     const int threads = 128;
     int64_t blocks = ceil_div(total, threads);
     if (blocks > 65535 * 16) blocks = 65535 * 16;
+    // an ordinary launch: the kernel releases its successor early but has no wait of its own, so it must not be allowed to start ahead of its predecessor's end
     stage_error_kernel<F><<<(unsigned)blocks, threads, 0, stream>>>(stage_args<F>(d, z, s, s + 1, skew, z_stride));
     return check_launch();
 }

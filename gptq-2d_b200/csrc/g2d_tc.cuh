@@ -112,8 +112,8 @@ struct TcRing {
     int failed;
 };
 
-// ---- two CTAs of a cluster on one product (cta_group::2): M = 256, 128 rows in each CTA, and half of B in each, so that a CTA fills and reads
-// shared memory for 192 rows where one on its own does for 256 of a 128 x 128 tile.  CTA 0 leads: it issues the MMAs for both. ----
+// ---- two CTAs of a cluster on one product (cta_group::2): M = N = 256, 128 rows of A and of B in each CTA, so that a CTA fills shared memory with 256
+// rows for its 128 x 256 of the product, where one on its own fills it with 384.  CTA 0 leads: it issues the MMAs for both. ----
 __device__ __forceinline__ uint32_t leaders(uint64_t *bar) {  // the same barrier of CTA 0
     uint32_t r;
     asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(r) : "r"(smem_u32(bar)));

@@ -240,11 +240,11 @@
         // and fifteen multiply-adds per lane and stage.  (Half a warp per sub-tile with both feedbacks in one lane takes
         // two shuffles and thirty multiply-adds: 208 cycles per stage against about 100.)
         // What bounds a stage is the chain from one rounding to the next (multiply-add, shuffle of 26 cycles, the quantizer's
-        // dependent operations at 4.5 to 5.4 cycles each: about 72 cycles, 95 before affine_steps_fast); everything else has to fit into its
+        // dependent operations at 4.5 to 5.4 cycles each: about 82 cycles, 92 with a zero point, 95 before affine_steps_fast); everything else has to fit into its
         // gaps.  So every address of a stage is a lane's base plus a constant stride (lanes before their first or past their last entry
         // read zero rows or values that they ignore, and store nothing), the operands of a stage are loaded one stage ahead, and there is
-        // no branch inside the four unrolled stages (one branch per stage costs 40 cycles): with the other warps' work beside it about 120 cycles
-        // per stage where one sub-tile is swept and 190 where four are.
+        // no branch inside the four unrolled stages (one branch per stage costs 40 cycles): with the other warps' work beside it 123 to 143 cycles
+        // per stage where one or two sub-tiles are swept and 180 where four are.
         // The two roles run the same sequence of barriers from loops of their own, so that neither holds the other's registers.
         // Operands of the tensor-core updates: fp16 pairs of E (transposed) and of the completed C under the tile's scales, eight entries
         // per thread and store.  C along its rows; E transposed: a thread gathers eight rows of one column (consecutive threads take
@@ -281,8 +281,8 @@
                     t.pre = pre != nullptr ? pre + (i0 + r0) * n + j0 + b * SUB : nullptr;  // the caller's array: rows of n
                     t.pre_ld = n;
                     // 3 and 4 (float) and 1 (double) for the common case, without a branch in the stages; recording the pre-rounding
-                    // values is a matter of tests.  The zero points of symmetric codes are zeros: stages of 95 cycles with 4, 104 with 3 and 120
-                    // before there was either (one sweeping warp alone; four of them 136, 141 and 152).
+                    // values is a matter of tests.  The zero points of symmetric codes are zeros.  Cycles per stage with 4, 3 and 1, where one
+                    // sub-tile is swept and where four are: 134 and 180, 155 and 198, 164 and 217 (256 x 256).
                     const unsigned how = fast_div[w & 1][sub_a];
                     const bool exact = !(how & 1);
                     if (pre != nullptr) {

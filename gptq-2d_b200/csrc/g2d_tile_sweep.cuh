@@ -219,8 +219,8 @@ __device__ __forceinline__ void sweep_sub_tile(const SubTile<F> tile, const int 
                 result = z;
             }
             // What is pushed: the error E of the float that is stored (column lanes), the completed C + E (row lanes), in the reference's order.  (Both
-            // from the unrounded product of code and scale are one multiply-add and two additions less on the chain, but leave up to half an ulp of
-            // Z out of the feedback, and an infinite C is then no NaN in what goes to the right.)
+            // from the unrounded product of code and scale are one multiply-add where these are a product and two additions, 2 % of a small
+            // sweep, but leave up to half an ulp of Z out of the feedback, and an infinite C is then no NaN in what goes to the right.)
             const F carried = (z - yv) + (role ? other : (F)0);
             const F v = ok ? carried : (F)0;     // lanes without an entry push zero
             // the push moves every accumulator down by one register on the way

@@ -1,8 +1,8 @@
 // A step of the pipelined schedule in one launch (float, one matrix): the first CTAs sweep the tiles of the anti-diagonal S, and the others, on
 // the SMs that the tiles leave free, carry out the near update of the anti-diagonal before.  The two do not depend on each other: the update's
 // targets start at S + 1.  Bound by the tiles' serial chain, about 24 us.  On streams of their own (g2d_tile_sweep.cu, g2d_band_tc.cu) a step took
-// 7 us of events between the two on top of it; in one launch that starts early, 1024 x 1024 takes 0.82 ms in place of 0.93, 2048 x 2048 1.69 in
-// place of 1.92, 8192 x 8192 11.0 in place of 11.7.  A warp issues an instruction every ninth cycle; 2.0 of
+// 7 us of events between the two on top of it; in one launch that starts early, 1024 x 1024 takes 0.84 ms in place of 0.95, 2048 x 2048 1.72 in
+// place of 1.97, 8192 x 8192 11.1 in place of 11.8.  A warp issues an instruction every ninth cycle; 2.0 of
 // those nine it waits for instructions to arrive, 2.3 at barriers (4096 x 4096): how long the kernel's text is, and where its parts lie,
 // shows in its time.
 #include "g2d_band_tc.cuh"
@@ -34,8 +34,8 @@ static int launch_step_kind(const SweepArgs<float> &args, int S, const BandJob &
         return G2D_ERR_CUDA;
     const int i_lo = S - args.nJ + 1 > 0 ? S - args.nJ + 1 : 0, i_hi = S + 1 < args.nI ? S + 1 : args.nI, tiles = i_hi - i_lo;
     // Updating CTAs: as many as there are SMs left, but sixteen jobs each, which the ring takes in 5 to 12 us of the tiles' 25.  More of them keep SMs
-    // from the far updates (4 us of set-up and first loads each): 1, 8, 16 and 24 jobs at least, in us: 2048 x 2048 1694, 1678, 1684, 1732;
-    // 4096 x 4096 3672, 3635, 3615, 3719; 8192 x 8192 11047, 11010, 10971, 10935.
+    // from the far updates (4 us of set-up and first loads each): 1, 8, 16 and 24 jobs at least, in us: 2048 x 2048 1732, 1719, 1721, 1764;
+    // 4096 x 4096 3747, 3708, 3709, 3804; 8192 x 8192 11120, 11103, 11041, 10985.
     constexpr int JOBS_EACH = 16;
     const int jobs = 2 * job.longest * job.slots, free_sms = 148 - tiles, updating = (jobs + JOBS_EACH - 1) / JOBS_EACH;  // at most 128 tiles take this schedule
     if (free_sms < 1) return G2D_ERR_BAD_ARGUMENT;
