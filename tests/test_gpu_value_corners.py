@@ -77,6 +77,25 @@ def test_signs_of_zeros(qmin, qmax, zero, m, n, scale_sign):
     assert torch.equal(torch.signbit(z), torch.signbit(want))
 
 
+@pytest.mark.parametrize("m, n, q", [(64, 1024, 16), (96, 512, 32)])
+def test_infinite_coupling_of_groups(m, n, q, oracle):
+    """An infinite entry of U makes its receivers infinite and their groups' scales with them, so whole groups are NaN from there on, as in the oracle: a
+    flush forms no zero times infinity for sources outside a row's stages, which would leave NaN that a group's largest value passes over."""
+    import gptq_2d as G
+    import quantizer_int as Q
+
+    rng = np.random.default_rng(n)
+    w, l, u = (0.02 * rng.standard_normal(s).astype(np.float32) for s in ((m, n), (m, m), (n, n)))
+    block = np.arange(n) // q
+    l, u = np.tril(l, -1) + np.eye(m, dtype=np.float32), np.where(block[:, None] < block[None, :], u, np.float32(0)) + np.eye(n, dtype=np.float32)
+    u[n // 4, n // 2 + 3] = np.inf
+    want = oracle.sweep(w, l, u, kind=oracle.Q_ABSMAX, super_entry_shape=(1, q), qmin=-8, qmax=7, half=oracle.FP16)
+    cuda = lambda a: torch.from_numpy(a).cuda()
+    quantizer = functools.partial(Q.int_abs_max_quantizer_cuda, qmin=-8, qmax=7, dtype=torch.float16)
+    got = G.gptq_2d_super_entry(cuda(w), cuda(l), cuda(u), quantizer=quantizer, super_entry_shape=(1, q)).cpu().numpy()
+    assert np.isnan(want[:, n // 2:]).all() and np.array_equal(np.isnan(got), np.isnan(want))
+
+
 @pytest.mark.parametrize("n", [8, 9, 32])
 def test_packing_under_a_zero_point_that_is_nan(n):
     """Converts to 0 before it is clamped, in whole groups of eight as in ragged ones."""
